@@ -307,7 +307,10 @@ def work(case):
 
 
 def tolerance(case):
-    # Values pass through 2 to 72 bf16 residual additions and some ten bf16 roundings per layer: every rounding moves a
-    # value by up to 2^-9, and two summation orders end about 1 % apart (2-norm) behind 36 layers.  Largest single
-    # differences sit at five to six standard deviations of that.  Tokens are chosen by wide margins: equal.
-    return {"rel": 2e-2, "max": 0.25}
+    # A layer passes values through two bf16 residual additions and some ten more bf16 roundings.  Another order of
+    # summation flips some of them, and behind a few layers two correct runs round independently of one another:
+    # about 1e-2 (2-norm) for one layer, growing like the square root of the depth.  Measured with the grid cut to 131
+    # CTAs (another split of every sum): 0.003 behind 4 layers, 0.024 behind 36, largest single difference 0.19 of the
+    # root mean square among tens of millions.  A MoE router may flip a near-tie besides.  Tokens are chosen by wide
+    # margins: equal.
+    return {"rel": 3e-2 if case["kind"] == "moe" else min(3e-2, 1e-2 * math.sqrt(case["layers"])), "max": 0.4}
