@@ -14,7 +14,7 @@ CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libb200mk.so")
 # mk_kernel_tp.cu, mk_kernel_hier.cu and mk_kernel_moe.cu include mk_kernel.cu with other build switches (see its header)
 SOURCES = ["mk_kernel.cu", "mk_kernel_tp.cu", "mk_kernel_hier.cu", "mk_kernel_moe.cu", "mk_runtime.cpp", "mk_noalloc.cu"]
-HEADERS = ["mk_types.h", os.path.join("..", "..", "include", "b200mk.h")]
+HEADERS = ["mk_types.h", "mk_wide.cuh", os.path.join("..", "..", "include", "b200mk.h")]
 
 
 def _nvcc():

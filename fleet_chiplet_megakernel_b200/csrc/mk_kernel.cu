@@ -1,14 +1,13 @@
 // The persistent decode megakernel for sm_100a.
 //
-// One cooperative launch runs a whole generation.  Every SM hosts one CTA of
-// nine warps: warp 8 is a TMA producer that streams this CTA's share of every
-// linear layer's weights (128x64 bf16 tiles, 128-byte swizzle) into a ring of
-// shared-memory stages, running ahead of the eight consumer warps across op
-// boundaries (weights have no dependencies).  The consumer warps walk the
-// program: wait at a grid barrier where an op reads what other CTAs wrote, do
-// the op's share of work, go on.  Every wait in the kernel is bounded: on
-// expiry the waiter records a status and raises a sticky abort flag that all
-// other waits poll, and the kernel returns with an error code.
+// One cooperative launch runs a whole generation.  Every SM hosts one CTA: warp 8 is a TMA
+// producer that streams this CTA's share of every linear layer's weights (boxes of 64 k-elements,
+// 128-byte swizzle) into a ring of shared-memory stages, running ahead of the consumers across op
+// boundaries (weights have no dependencies); the eight consumer warps walk the program: wait at a
+// grid barrier where an op reads what other CTAs wrote, do the op's share of work, go on.  The wide
+// path (mk_wide.cuh) has two more roles, an activation producer and an MMA issuer.  Every wait in
+// the kernel is bounded: on expiry the waiter records a status and raises a sticky abort flag that
+// all other waits poll, and the kernel returns with an error code.
 //
 // Replaces the worker/scheduler loops of the reference runtime
 // (include/mirage/persistent_kernel/persistent_kernel.cuh:693-1854) and its
@@ -141,12 +140,10 @@ struct Ctx {
   uint32_t smem_addr;
   unsigned epoch;     // grid barriers passed
   unsigned cons_idx;  // weight stages consumed
-  unsigned xphase;    // per stage: parity of the next activation-box phase (only some ops use the boxes)
   bool arrived;       // this CTA has already arrived at the coming grid barrier
-  int attn_iter;      // iteration whose attention metadata is cached in shared memory
-  uint32_t tmem;      // base address of the CTA's tensor-memory columns
-  bool has_tmem;
-  unsigned done_phase;  // phases of the accumulator-ready mbarrier consumed so far
+  int attn_iter;      // row-owner path: iteration whose attention metadata is cached in shared memory; wide path: head geometry planned
+  uint32_t tmem;      // wide path: base address of the CTA's tensor-memory columns
+  unsigned acc_runs;  // wide path: accumulator runs finished
   int tid, lane, warp;
   int iter, cur_op;
   unsigned long long* dbg;  // inner-phase stamps of the traced op (thread 0), or null
@@ -163,19 +160,22 @@ struct Ctx {
   __device__ uint32_t empty_bar(int s) const { return smem_addr + p.bar_off + 8 * (p.num_stages + s); }
   __device__ uint32_t xfull_bar(int s) const { return smem_addr + p.bar_off + 8 * (2 * p.num_stages + s); }
   __device__ volatile int* flags() const { return (volatile int*)(smem + p.bar_off + 24 * p.num_stages); }
-  // behind the flags: the accumulator-ready mbarrier of the tcgen05 path and the word tcgen05.alloc writes
+  // behind the flags: the end-of-work mbarrier of the tcgen05 path and the word tcgen05.alloc writes
   __device__ uint32_t done_bar() const { return smem_addr + p.bar_off + 24 * p.num_stages + 64; }
   __device__ uint32_t tmem_slot() const { return smem_addr + p.bar_off + 24 * p.num_stages + 72; }
   // hierarchical grid barrier: arrivals of the cluster (used in its first CTA), release from the first CTA, its abort word
   __device__ uint32_t cl_arrive_bar() const { return smem_addr + p.bar_off + 24 * p.num_stages + 80; }
   __device__ uint32_t cl_open_bar() const { return smem_addr + p.bar_off + 24 * p.num_stages + 88; }
   __device__ uint32_t cl_dead_word() const { return smem_addr + p.bar_off + 24 * p.num_stages + 96; }
+  // wide path, per accumulator buffer: sums complete (tcgen05.commit), sums fetched (one arrival per finishing warp)
+  __device__ uint32_t acc_full_bar(unsigned b) const { return smem_addr + p.bar_off + 24 * p.num_stages + 104 + 8 * b; }
+  __device__ uint32_t acc_empty_bar(unsigned b) const { return smem_addr + p.bar_off + 24 * p.num_stages + 120 + 8 * b; }
   __device__ float* sums() const { return (float*)(smem + p.sums_off); }
   __device__ float* red() const { return (float*)(smem + p.red_off); }  // small scratch: reductions, lengths
 };
 // flags(): [0] go word written by consumers, read by the producer
 //          [1] stages issued by the producer   [2] broadcast slot   [3] dead flag of the op
-//          [4] linear ops whose barrier the consumers have passed   [5] activation stages issued
+//          [4] linear ops whose barrier the consumers have passed   [5] wide path: stages multiplied
 
 #define MK_STAMP(c, k)                                             \
   do {                                                            \
@@ -979,14 +979,8 @@ __device__ __noinline__ void stage_rows_ll(Ctx& c, const void* ll_in, int ld_in,
 }
 
 // ------------------------------------------------------------------------------------
-// linear layer: weight tiles from the TMA ring x activations from shared memory on the
-// warp-level tensor cores (mma.sync m16n8k16, bf16 in, fp32 accumulate)
+// linear layers: pieces shared by the row-owner path (below) and the wide path (mk_wide.cuh)
 // ------------------------------------------------------------------------------------
-// Each of the 8 consumer warps owns 16 of a tile's 128 weight rows (the A operand, read
-// with ldmatrix from the 128-byte-swizzled stage); up to 8 tokens form the N dimension
-// (the B operand, token rows read with ldmatrix from the staged activations).  Every
-// (row, token) sum lives in exactly one thread, so a run of tiles ends without any
-// cross-lane reduction.
 struct ArgBest {
   float v;
   int i;
@@ -1019,609 +1013,6 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 }
 
 
-// ntok tokens starting at tok0; sums at sums()[row * sums_stride + token]
-__device__ void linear_epilogue(Ctx& c, const OpDesc& op, int blk, int tok0, int ntok, float res0) {
-  const KParams& p = c.p;
-  const float* red = c.sums();
-  const int kRedStride = p.sums_stride;
-  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out);
-  if (op.flags & F_SILU_MUL) {
-    // rows 0..63 of the tile are gate columns, rows 64..127 the matching up columns; with F_SILU4 the
-    // weight is laid out for the row-owner path instead: units of 8 rows, [4 gate | 4 up]
-    const int half = op.n >> 1;
-    const bool by4 = (op.flags & F_SILU4) != 0;
-    if (ntok > 2 && (op.ld_out & 7) == 0 && (blk + 1) * 64 <= half) {
-      // a thread takes 8 consecutive output columns of one token: lanes of a warp read different tokens
-      // (no bank conflicts in the sums block) and store 16 bytes
-#pragma unroll 1
-      for (int u = c.tid; u < 8 * ntok; u += kNumConsumers) {
-        const int tb = u % ntok, cg = u / ntok;
-        float v[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int idx = cg * 8 + i;
-          const int row = by4 ? ((idx >> 2) << 3) + (idx & 3) : idx;
-          const float g = rbf(red[row * kRedStride + tb]);  // linear output is bf16 before the activation
-          const float up = rbf(red[(by4 ? row + 4 : row + 64) * kRedStride + tb]);
-          v[i] = rbf(__fdividef(g, 1.0f + __expf(-g))) * up;
-        }
-        *reinterpret_cast<uint4*>(out + (size_t)(tok0 + tb) * op.ld_out + blk * 64 + cg * 8) = pack8(v);
-      }
-      return;
-    }
-#pragma unroll 1
-    for (int e = c.tid; e < 64 * ntok; e += kNumConsumers) {
-      const int idx = e & 63, tb = e >> 6;
-      const int col = blk * 64 + idx;
-      const int row = by4 ? ((idx >> 2) << 3) + (idx & 3) : idx;
-      const int urow = by4 ? row + 4 : row + 64;
-      if (col < half) {
-        const float g = rbf(red[row * kRedStride + tb]);  // linear output is bf16 before the activation
-        const float u = rbf(red[urow * kRedStride + tb]);
-        const float s = rbf(__fdividef(g, 1.0f + __expf(-g)));
-        out[(size_t)(tok0 + tb) * op.ld_out + col] = __float2bfloat16_rn(s * u);
-      }
-    }
-    return;
-  }
-  const bool with_res = (op.flags & F_RESIDUAL) && (!(op.flags & F_RES_RANK0) || p.rank == 0);
-  const __nv_bfloat16* res = reinterpret_cast<const __nv_bfloat16*>(op.res);
-  const bool push = MK_XF(op, F_PUSH) != 0;
-  // Wide batches: a thread takes 8 consecutive output columns of one token (one 16-byte residual load, one
-  // 16-byte store), four such units per round with their loads issued together: one dependent 2-byte load
-  // per element made the block's finisher the slowest CTA of the op by far (at 64 tokens: 32 round trips).
-  // Lanes of a warp take different tokens, so the sums block is read without bank conflicts.
-  // (a pushing linear stores the eight sums of a unit as four 16-byte stores {value, number, value, number} per rank)
-  const bool vec = !MK_XF(op, F_GATHER_RES) && ntok > 2 && (push || (op.ld_out & 7) == 0) && (!with_res || (op.ld_res & 7) == 0) &&
-                   ((blk + 1) * kTileRows <= op.n);
-  if (vec) {
-    const int nunits = (kTileRows / 8) * ntok;
-#pragma unroll 1
-    for (int u0 = c.tid; u0 < nunits; u0 += 4 * kNumConsumers) {
-      uint4 rv[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int u = u0 + k * kNumConsumers;
-        rv[k] = make_uint4(0, 0, 0, 0);
-        if (with_res && u < nunits)
-          rv[k] = __ldcg(reinterpret_cast<const uint4*>(res + (size_t)(tok0 + u % ntok) * op.ld_res + blk * kTileRows + (u / ntok) * 8));
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int u = u0 + k * kNumConsumers;
-        if (u < nunits) {
-          const int tb = u % ntok, cg = u / ntok;
-          float r[8], v[8];
-          unpack8(rv[k], r);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            v[i] = red[(cg * 8 + i) * kRedStride + tb];
-            if (p.numerics == NUM_TORCH && !push) v[i] = rbf(v[i]);  // (pushed sums stay fp32: rounded once, after the ranks are added up)
-            v[i] += r[i];
-          }
-#if MK_WITH_XCHG
-          if (push) {
-            const unsigned seq = xchg_next(c);
-            const size_t w = xchg_word(seq, p.world, p.xchg_tokens, p.xchg_cols, p.rank, tok0 + tb, blk * kTileRows + cg * 8);
-#pragma unroll 1
-            for (int rk = 0; rk < p.world; ++rk) {
-              uint4* dstw = reinterpret_cast<uint4*>(reinterpret_cast<uint2*>(p.xchg[rk]) + w);
-#pragma unroll
-              for (int i = 0; i < 4; ++i) st_sys_v4(dstw + i, __float_as_uint(v[2 * i]), seq, __float_as_uint(v[2 * i + 1]), seq);
-            }
-            continue;
-          }
-#endif
-          *reinterpret_cast<uint4*>(out + (size_t)(tok0 + tb) * op.ld_out + blk * kTileRows + cg * 8) = pack8(v);
-        }
-      }
-    }
-  } else
-#pragma unroll 1
-  for (int e = c.tid; e < kTileRows * ntok; e += kNumConsumers) {
-    const int row = e & 127, tb = e >> 7;
-    const int tok = tok0 + tb, col = blk * kTileRows + row;
-    if (col < op.n) {
-      float v = red[row * kRedStride + tb];
-      if (p.numerics == NUM_TORCH && !push) v = rbf(v);  // (pushed partial sums stay fp32: they are rounded once, after the ranks are added up)
-      if (with_res) {
-        float r;
-        if (e < kNumConsumers) r = res0;
-        else if (MK_XF(op, F_GATHER_RES)) r = xchg_gather1(c, xchg_cur(c), tok, col);
-        else r = __bfloat162float(__ldcg(res + (size_t)tok * op.ld_res + col));
-        v += r;
-      }
-      if (push) xchg_push1(p, xchg_next(c), tok, col, v);
-      else out[(size_t)tok * op.ld_out + col] = __float2bfloat16_rn(v);
-    }
-  }
-  if (op.flags & F_ARGMAX) {
-    // one warp per token: the tile's 128 bf16 logits of the token, four per lane
-#pragma unroll 1
-    for (int tb = c.warp; tb < ntok; tb += kNumConsumerWarps) {
-      ArgBest b;
-      b.v = -INFINITY;
-      b.i = 0x7fffffff;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const int row = c.lane + 32 * q, col = blk * kTileRows + row;
-        if (col < op.n) {
-          ArgBest x;
-          x.v = rbf(red[row * kRedStride + tb]);
-          x.i = col;
-          b = arg_better(b, x);
-        }
-      }
-      b = warp_argmax(b);
-      if (c.lane == 0) {
-        op.amax_val[(size_t)(tok0 + tb) * op.amax_n + blk] = b.v;
-        op.amax_idx[(size_t)(tok0 + tb) * op.amax_n + blk] = b.i;
-      }
-    }
-  }
-}
-
-// Called by all consumers at the end of a run of tiles of one row block, after the
-// per-row sums of the run were left in sums()[row * sums_stride + token].
-//
-// When several CTAs hold k-ranges of the block, the CTA with the block's FIRST k-range
-// finishes it: that range is the tail of its own tile range, so it is the last piece to
-// be computed anyway.  The others publish their partial sums with a release and move on
-// without waiting for anything; the finisher waits (bounded) until they have all
-// arrived, adds the pieces in CTA order and runs the epilogue.
-__device__ __noinline__ void linear_finish_piece(Ctx& c, const OpDesc& op, int blk, int kt_first, int kt_last,
-                                                 bool first_of_cta, int tok0, int ntok, int group, float res0) {
-  const KParams& p = c.p;
-  float* red = c.sums();
-  const int kRedStride = p.sums_stride;
-  const int nvec4 = kTileRows * kRedStride / 4;  // float4 pieces of the sums block
-  consumer_sync();
-  const bool whole = (kt_first == 0) && (kt_last == op.nkt - 1);
-  if (!whole) {
-    const unsigned total = (unsigned)op.nblk * (unsigned)op.nkt;
-    const int G = (int)min(gridDim.x, total);  // CTAs that hold tiles of this op
-    const int GS = gridDim.x;
-    const size_t slot_elems = (size_t)kTileRows * kRedStride;
-    const int c_first = tile_owner((unsigned)blk * op.nkt, total, G);
-    const int c_last = tile_owner((unsigned)blk * op.nkt + op.nkt - 1, total, G);
-    unsigned* cnt = p.piece_count + (size_t)group * p.piece_stride + blk;
-    float4* red4 = reinterpret_cast<float4*>(red);
-    if ((int)blockIdx.x != c_first) {
-      float4* mine = reinterpret_cast<float4*>(
-          p.partial + (((size_t)group * GS + blockIdx.x) * 2 + (first_of_cta ? 0 : 1)) * slot_elems);
-#pragma unroll 1
-      for (int i = c.tid; i < nvec4; i += kNumConsumers) mine[i] = red4[i];
-      consumer_sync();  // thread 0's release covers what the CTA wrote before this sync
-      if (c.tid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
-      return;
-    }
-    const unsigned want = (unsigned)(c_last - c_first);
-    if (c.tid == 0) {
-      unsigned long long t0 = 0;
-      unsigned spins = 0;
-      while (ld_acquire_u32(cnt) < want) {
-        if (((++spins) & 1023u) == 0) {
-          if (aborted(c)) break;
-          const unsigned long long now = globaltimer();
-          if (t0 == 0) {
-            t0 = now;
-          } else if (now - t0 > 2 * c.p.timeout_ns) {
-            raise_abort(c, ST_TIMEOUT_PEER, blk, (int)ld_acquire_u32(cnt));
-            break;
-          }
-        }
-      }
-      *cnt = 0u;
-    }
-    consumer_sync();
-    __threadfence();
-    // all pieces' loads go out together: one L2 round trip instead of one per piece
-#pragma unroll 2
-    for (int i = c.tid; i < nvec4; i += kNumConsumers) {
-      float4 acc = red4[i];
-#pragma unroll 1
-      for (int c0 = c_first + 1; c0 <= c_last; c0 += 4) {
-        float4 v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int cc = c0 + u;
-          v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (cc <= c_last) {
-            const bool first = (tile_begin(cc, total, G) / op.nkt) == blk;
-            const float4* src = reinterpret_cast<const float4*>(
-                p.partial + (((size_t)group * GS + cc) * 2 + (first ? 0 : 1)) * slot_elems);
-            v[u] = __ldcg(src + i);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          acc.x += v[u].x;
-          acc.y += v[u].y;
-          acc.z += v[u].z;
-          acc.w += v[u].w;
-        }
-      }
-      red4[i] = acc;
-    }
-    consumer_sync();
-  }
-  linear_epilogue(c, op, blk, tok0, ntok, res0);
-  consumer_sync();
-}
-
-// Tokens one pass of a linear op covers (aux3, fixed by the host from the shared-memory
-// budget) and the passes its weight stream makes for T active tokens.
-__device__ __forceinline__ int linear_passes(const OpDesc& op, int T) { return (T + op.aux3 - 1) / op.aux3; }
-
-__device__ __noinline__ void linear_pass(Ctx& c, const OpDesc& op, int tok0, int T, int group, const uint4* pre_w) {
-  const KParams& p = c.p;
-  const int nkt = op.nkt;
-  const int kp = nkt * kTileK;
-  const int ntok = min(op.aux3, T - tok0);
-  MK_STAMP(c, 0);
-  stage_x(c, op.in, op.ld_in, op.k, kp, (op.flags & F_NORM_IN) ? op.norm_w : nullptr, tok0, ntok, T, pre_w,
-          MK_XF(op, F_GATHER_IN) != 0);
-  MK_STAMP(c, 1);
-
-  const unsigned total = (unsigned)op.nblk * (unsigned)nkt;
-  const int G = (int)min(gridDim.x, total);  // with fewer tiles than CTAs the rest idle
-  if ((int)blockIdx.x >= G) return;
-  const unsigned t0 = tile_begin(blockIdx.x, total, G);
-  const unsigned t1 = tile_begin(blockIdx.x + 1, total, G);
-  const int S = p.num_stages;
-  const int lane = c.lane, warp = c.warp;
-  // A operand: lane l addresses row 16*warp + (l & 7) + 8 * ((l >> 3) & 1), 16-byte chunk 2*kb + (l >> 4)
-  const int a_row = 16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8;
-  const uint32_t a_base = (uint32_t)(a_row * 128);
-  const uint32_t a_xor = (uint32_t)(a_row & 7);
-  const uint32_t a_hi = (uint32_t)(lane >> 4);
-  // B operand: lane l addresses token (l & 7), chunk 4*half + (l >> 3); absent tokens read the zero chunk
-  const int pitch_b = (kp + 8) * 2;
-  const bool b_real = (lane & 7) < ntok;
-  const uint32_t xs0 = c.smem_addr + p.x_off;
-  const uint32_t b_zero = xs0 + (uint32_t)(ntok * pitch_b);
-  const uint32_t b_row = xs0 + (uint32_t)((lane & 7) * pitch_b + (lane >> 3) * 16);
-  const uint32_t bar_full0 = c.full_bar(0), bar_empty0 = c.empty_bar(0);
-
-  // The residual element this thread adds first in the epilogue of a row block is requested
-  // when the block starts, a whole run of tiles ahead of its use.
-  const bool with_res = (op.flags & F_RESIDUAL) && (!(op.flags & F_RES_RANK0) || p.rank == 0);
-  const __nv_bfloat16* res_ptr = reinterpret_cast<const __nv_bfloat16*>(op.res) +
-                                 (size_t)(tok0 + (c.tid >> 7)) * op.ld_res + (c.tid & 127);
-  const bool res_tok = with_res && (c.tid >> 7) < ntok;
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  int blk = (int)(t0 / (unsigned)nkt);
-  int kt = (int)(t0 - (unsigned)blk * (unsigned)nkt);
-  int kt_first = kt;
-  bool first_of_cta = true;
-  int s = (int)(c.cons_idx % (unsigned)S);
-  uint32_t parity = (c.cons_idx / (unsigned)S) & 1u;
-  unsigned consumed = 0;
-  const bool arith = !(p.debug_flags & 1);
-  float res0 = 0.f;
-  bool new_blk = true;
-  for (unsigned tile = t0; tile < t1; ++tile) {
-    if (new_blk) {
-      new_blk = false;
-      res0 = 0.f;
-      if (res_tok && blk * kTileRows + (c.tid & 127) < op.n)
-        res0 = MK_XF(op, F_GATHER_RES) ? xchg_gather1(c, xchg_cur(c), tok0 + (c.tid >> 7), blk * kTileRows + (c.tid & 127))
-                                         : __bfloat162float(__ldcg(res_ptr + blk * kTileRows));
-    }
-    mbar_wait(c, bar_full0 + 8 * s, parity, ST_TIMEOUT_FULL);
-    if (tile == t0) MK_STAMP(c, 2);
-    const uint32_t st = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes + a_base;
-    if (arith) {
-#pragma unroll
-      for (int sub = 0; sub < kSubTiles; ++sub) {
-        uint32_t b[8];
-        const uint32_t bk = b_real ? b_row + (uint32_t)kt * (kTileK * 2) + (uint32_t)sub * (kBoxK * 2) : b_zero;
-        ldmatrix_x4(bk, b[0], b[1], b[2], b[3]);
-        ldmatrix_x4(b_real ? bk + 64 : b_zero, b[4], b[5], b[6], b[7]);
-#pragma unroll
-        for (int kb = 0; kb < 4; ++kb) {
-          uint32_t a0, a1, a2, a3;
-          ldmatrix_x4(st + (uint32_t)sub * kSubBytes + ((((uint32_t)(2 * kb) + a_hi) ^ a_xor) << 4), a0, a1, a2, a3);
-          mma_bf16(acc, a0, a1, a2, a3, b[2 * kb], b[2 * kb + 1]);
-        }
-      }
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(bar_empty0 + 8 * s);
-    ++consumed;
-    if (++s == S) {
-      s = 0;
-      parity ^= 1u;
-    }
-    const bool end_blk = (kt == nkt - 1);
-    if (tile == t1 - 1) MK_STAMP(c, 3);
-    if (end_blk || tile == t1 - 1) {
-      // thread (lane) holds rows 16*warp + lane/4 (+8) and tokens 2*(lane%4) (+1)
-      float* red = c.sums() + (16 * warp + (lane >> 2)) * p.sums_stride + 2 * (lane & 3);
-      red[0] = acc[0];
-      red[1] = acc[1];
-      red[8 * p.sums_stride] = acc[2];
-      red[8 * p.sums_stride + 1] = acc[3];
-      acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
-      linear_finish_piece(c, op, blk, kt_first, kt, first_of_cta, tok0, ntok, group, res0);
-      first_of_cta = false;
-      kt_first = 0;
-      if (tile == t1 - 1) MK_STAMP(c, 4);
-    }
-    if (end_blk) {
-      kt = 0;
-      blk += 1;
-      new_blk = true;
-    } else {
-      kt += 1;
-    }
-  }
-  c.cons_idx += consumed;
-}
-
-// Batches above 8 tokens: the input rows of a pass (16, 32 or 64 token rows x 128 k) come
-// with every weight stage as two more TMA boxes (issued by the activation producer once the
-// op's barrier has opened), 128-byte swizzled like the weights, and each warp multiplies its
-// 16 weight rows against NT n-tiles of 8 tokens.  The weights are streamed once per pass of
-// up to 64 tokens instead of once per 8.
-template <int NT>
-__device__ __noinline__ void linear_pass_wide(Ctx& c, const OpDesc& op, int tok0, int T, int group) {
-  const KParams& p = c.p;
-  const int nkt = op.nkt;
-  const int ntok = min(8 * NT, T - tok0);
-  const unsigned total = (unsigned)op.nblk * (unsigned)nkt;
-  const int G = (int)min(gridDim.x, total);
-  if ((int)blockIdx.x >= G) return;
-  const unsigned t0 = tile_begin(blockIdx.x, total, G);
-  const unsigned t1 = tile_begin(blockIdx.x + 1, total, G);
-  const int S = p.num_stages;
-  const int lane = c.lane, warp = c.warp;
-  const int a_row = 16 * warp + (lane & 7) + ((lane >> 3) & 1) * 8;
-  const uint32_t a_base = (uint32_t)(a_row * 128);
-  const uint32_t a_xor = (uint32_t)(a_row & 7);
-  const uint32_t a_hi = (uint32_t)(lane >> 4);
-  // B operand: lane l addresses token row 8*nt + (l & 7), 16-byte chunk 4*half + (l >> 3)
-  const uint32_t b_row = (uint32_t)((lane & 7) * 128);
-  const uint32_t b_xor = (uint32_t)(lane & 7);
-  const uint32_t b_hi = (uint32_t)(lane >> 3);
-  const uint32_t x_sub = (uint32_t)(8 * NT * 128);  // bytes of one activation box
-  const uint32_t bar_full0 = c.full_bar(0), bar_empty0 = c.empty_bar(0), bar_x0 = c.xfull_bar(0);
-  const bool with_res = (op.flags & F_RESIDUAL) && (!(op.flags & F_RES_RANK0) || p.rank == 0);
-  const __nv_bfloat16* res_ptr = reinterpret_cast<const __nv_bfloat16*>(op.res) +
-                                 (size_t)(tok0 + (c.tid >> 7)) * op.ld_res + (c.tid & 127);
-  const bool res_tok = with_res && (c.tid >> 7) < ntok;
-  float acc[NT][4];
-#pragma unroll
-  for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) acc[nt][i] = 0.f;
-  int blk = (int)(t0 / (unsigned)nkt);
-  int kt = (int)(t0 - (unsigned)blk * (unsigned)nkt);
-  int kt_first = kt;
-  bool first_of_cta = true;
-  int s = (int)(c.cons_idx % (unsigned)S);
-  uint32_t parity = (c.cons_idx / (unsigned)S) & 1u;
-  unsigned consumed = 0;
-  float res0 = 0.f;
-  bool new_blk = true;
-  for (unsigned tile = t0; tile < t1; ++tile) {
-    if (new_blk) {
-      new_blk = false;
-      res0 = 0.f;
-      if (res_tok && blk * kTileRows + (c.tid & 127) < op.n)
-        res0 = MK_XF(op, F_GATHER_RES) ? xchg_gather1(c, xchg_cur(c), tok0 + (c.tid >> 7), blk * kTileRows + (c.tid & 127))
-                                         : __bfloat162float(__ldcg(res_ptr + blk * kTileRows));
-    }
-    mbar_wait(c, bar_full0 + 8 * s, parity, ST_TIMEOUT_FULL);
-    mbar_wait(c, bar_x0 + 8 * s, (c.xphase >> s) & 1u, ST_TIMEOUT_FULL);
-    c.xphase ^= 1u << s;
-    const uint32_t st = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes;
-    const uint32_t xt = st + kStageBytes;
-#pragma unroll
-    for (int sub = 0; sub < kSubTiles; ++sub) {
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t a[2][4];
-#pragma unroll
-        for (int q = 0; q < 2; ++q)
-          ldmatrix_x4(st + a_base + (uint32_t)sub * kSubBytes + ((((uint32_t)(2 * (2 * half + q)) + a_hi) ^ a_xor) << 4),
-                      a[q][0], a[q][1], a[q][2], a[q][3]);
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-          uint32_t b0, b1, b2, b3;
-          ldmatrix_x4(xt + (uint32_t)sub * x_sub + (uint32_t)nt * 1024u + b_row + ((((uint32_t)(4 * half) + b_hi) ^ b_xor) << 4),
-                      b0, b1, b2, b3);
-          mma_bf16(acc[nt], a[0][0], a[0][1], a[0][2], a[0][3], b0, b1);
-          mma_bf16(acc[nt], a[1][0], a[1][1], a[1][2], a[1][3], b2, b3);
-        }
-      }
-    }
-    __syncwarp();
-    if (lane == 0) mbar_arrive(bar_empty0 + 8 * s);
-    ++consumed;
-    if (++s == S) {
-      s = 0;
-      parity ^= 1u;
-    }
-    const bool end_blk = (kt == nkt - 1);
-    if (end_blk || tile == t1 - 1) {
-      float* red = c.sums() + (16 * warp + (lane >> 2)) * p.sums_stride + 2 * (lane & 3);
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        red[8 * nt] = acc[nt][0];
-        red[8 * nt + 1] = acc[nt][1];
-        red[8 * p.sums_stride + 8 * nt] = acc[nt][2];
-        red[8 * p.sums_stride + 8 * nt + 1] = acc[nt][3];
-        acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.f;
-      }
-      linear_finish_piece(c, op, blk, kt_first, kt, first_of_cta, tok0, ntok, group, res0);
-      first_of_cta = false;
-      kt_first = 0;
-    }
-    if (end_blk) {
-      kt = 0;
-      blk += 1;
-      new_blk = true;
-    } else {
-      kt += 1;
-    }
-  }
-  c.cons_idx += consumed;
-}
-
-// ------------------------------------------------------------------------------------
-// Stream-K tiles on the 5th-generation tensor cores (17-64 tokens).  With mma.sync every warp
-// re-reads the activation boxes of a stage (at 64 tokens: 160 KB of ldmatrix traffic per
-// 32 KB weight tile, the SM's shared-memory bandwidth is the limit).  tcgen05.mma reads both
-// operands from shared memory once: A = the weight tile (M = 128 rows), B = the activation
-// box (N = 32 or 64 token rows), both K-major with the 128-byte swizzle TMA left them in;
-// D = 128 lanes x N columns of fp32 in tensor memory.  One thread issues the 8 MMAs of a
-// stage (2 boxes x 4 k-steps of 16) and commits them to the stage's "empty" mbarrier; when a
-// run of tiles ends, a commit to the "done" mbarrier tells all warps to fetch the
-// accumulators (tcgen05.ld, warp w reads lanes 32 * (w & 3) .. + 31) into the sums block,
-// from where the usual split-k finish and epilogue take over.
-// ------------------------------------------------------------------------------------
-__device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr) {
-  // start address >> 4 | leading offset (unused for swizzled K-major) 1 | stride between 8-row
-  // groups 1024 B >> 4 | descriptor version 1 | layout 2 = 128-byte swizzle
-  return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
-}
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
-  uint32_t r[16];
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-        "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-  for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-__device__ __noinline__ void linear_pass_umma(Ctx& c, const OpDesc& op, int tok0, int T, int group) {
-  const KParams& p = c.p;
-  const int nkt = op.nkt;
-  const int ntok = min(op.aux3, T - tok0);
-  const int N = p.x_rows;  // 32 or 64 token rows per activation box
-  const unsigned total = (unsigned)op.nblk * (unsigned)nkt;
-  const int G = (int)min(gridDim.x, total);
-  if ((int)blockIdx.x >= G) return;
-  const unsigned t0 = tile_begin(blockIdx.x, total, G);
-  const unsigned t1 = tile_begin(blockIdx.x + 1, total, G);
-  const int S = p.num_stages;
-  const int lane = c.lane, warp = c.warp;
-  const uint32_t x_sub = (uint32_t)N * 128u;  // bytes of one activation box
-  const uint32_t bar_full0 = c.full_bar(0), bar_empty0 = c.empty_bar(0), bar_x0 = c.xfull_bar(0);
-  // instruction descriptor: D = f32, A = B = bf16, both K-major, N >> 3, M >> 4
-  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((128u >> 4) << 24);
-  const bool with_res = (op.flags & F_RESIDUAL) && (!(op.flags & F_RES_RANK0) || p.rank == 0);
-  const __nv_bfloat16* res_ptr = reinterpret_cast<const __nv_bfloat16*>(op.res) +
-                                 (size_t)(tok0 + (c.tid >> 7)) * op.ld_res + (c.tid & 127);
-  const bool res_tok = with_res && (c.tid >> 7) < ntok;
-  int blk = (int)(t0 / (unsigned)nkt);
-  int kt = (int)(t0 - (unsigned)blk * (unsigned)nkt);
-  int kt_first = kt;
-  bool first_of_cta = true;
-  int s = (int)(c.cons_idx % (unsigned)S);
-  uint32_t parity = (c.cons_idx / (unsigned)S) & 1u;
-  unsigned consumed = 0;
-  float res0 = 0.f;
-  bool new_blk = true;
-  bool fresh = true;  // the next MMA starts a run: it overwrites the accumulators
-  for (unsigned tile = t0; tile < t1; ++tile) {
-    if (new_blk) {
-      new_blk = false;
-      res0 = 0.f;
-      if (res_tok && blk * kTileRows + (c.tid & 127) < op.n)
-        res0 = MK_XF(op, F_GATHER_RES) ? xchg_gather1(c, xchg_cur(c), tok0 + (c.tid >> 7), blk * kTileRows + (c.tid & 127))
-                                         : __bfloat162float(__ldcg(res_ptr + blk * kTileRows));
-    }
-    // every warp follows the ring (one arrival per warp and phase keeps the "empty" count
-    // exact); warp 0's arrival is the commit of the stage's MMAs
-    bool ok = mbar_wait(c, bar_full0 + 8 * s, parity, ST_TIMEOUT_FULL);
-    if (warp == 0) {
-      ok = mbar_wait(c, bar_x0 + 8 * s, (c.xphase >> s) & 1u, ST_TIMEOUT_FULL) && ok;
-      if (lane == 0) {
-        if (ok) {
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          const uint32_t st = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes;
-          const uint32_t xt = st + kStageBytes;
-#pragma unroll
-          for (int sub = 0; sub < kSubTiles; ++sub) {
-            const uint64_t ad = umma_smem_desc(st + (uint32_t)sub * kSubBytes);
-            const uint64_t bd = umma_smem_desc(xt + (uint32_t)sub * x_sub);
-#pragma unroll
-            for (int k16 = 0; k16 < 4; ++k16) {
-              // 16 k-elements = 32 bytes further inside the 128-byte swizzle span: +2 in the address field
-              umma_bf16(c.tmem, ad + (uint64_t)(2 * k16), bd + (uint64_t)(2 * k16), idesc, (fresh && sub == 0 && k16 == 0) ? 0u : 1u);
-            }
-          }
-          umma_commit(bar_empty0 + 8 * s);
-        } else {
-          mbar_arrive(bar_empty0 + 8 * s);  // aborting: keep the count exact, the body is skipped
-        }
-      }
-      __syncwarp();
-    } else if (lane == 0) {
-      mbar_arrive(bar_empty0 + 8 * s);
-    }
-    c.xphase ^= 1u << s;
-    fresh = false;
-    ++consumed;
-    if (++s == S) {
-      s = 0;
-      parity ^= 1u;
-    }
-    const bool end_blk = (kt == nkt - 1);
-    if (end_blk || tile == t1 - 1) {
-      // accumulators complete -> sums block [row][token]
-      if (warp == 0 && lane == 0) umma_commit(c.done_bar());
-      __syncwarp();
-      mbar_wait(c, c.done_bar(), c.done_phase & 1u, ST_TIMEOUT_FULL);
-      c.done_phase += 1;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      __syncwarp();
-      {
-        const int q = warp & 3, half = warp >> 2;  // lane quadrant, column half
-        const int row = 32 * q + lane;
-        const int ncol = N >> 1;  // columns of this warp: 16 or 32
-        float* dst = c.sums() + row * p.sums_stride + half * ncol;
-#pragma unroll 1
-        for (int c0 = 0; c0 < ncol; c0 += 16) {
-          float v[16];
-          tmem_ld16(c.tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(half * ncol + c0), v);
-#pragma unroll
-          for (int i = 0; i < 16; i += 4) *reinterpret_cast<float4*>(dst + c0 + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-        }
-      }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      linear_finish_piece(c, op, blk, kt_first, kt, first_of_cta, tok0, ntok, group, res0);
-      first_of_cta = false;
-      kt_first = 0;
-      fresh = true;
-    }
-    if (end_blk) {
-      kt = 0;
-      blk += 1;
-      new_blk = true;
-    } else {
-      kt += 1;
-    }
-  }
-  c.cons_idx += consumed;
-}
-
 // ------------------------------------------------------------------------------------
 // Row-owner linear (F_ROWS): for one or two tokens the cross-CTA finish of a k-split costs
 // more than the whole weight stream of a small layer, so every CTA takes whole output rows
@@ -1631,6 +1022,9 @@ __device__ __noinline__ void linear_pass_umma(Ctx& c, const OpDesc& op, int tok0
 // 512-wide stage, 16 weight rows on the M side of the mma and the tokens on the N side, and
 // the eight partial sums of an output meet in shared memory when the chunk ends.
 // ------------------------------------------------------------------------------------
+// Tokens one pass of a row-owner linear covers (aux3, fixed by the host from the shared-memory
+// budget) and the passes its weight stream makes for T active tokens.
+__device__ __forceinline__ int linear_passes(const OpDesc& op, int T) { return (T + op.aux3 - 1) / op.aux3; }
 __device__ __forceinline__ void rows_range(const OpDesc& op, int& row0, int& row1, bool& any) {
   const unsigned U = (unsigned)(op.n + kUnitRows - 1) / kUnitRows;
   const unsigned G = min((unsigned)gridDim.x, U);
@@ -1645,14 +1039,6 @@ __device__ __forceinline__ int rows_num_chunks(int row0, int row1) { return (row
 __device__ __forceinline__ int rows_chunk_begin(int row0, int row1, int nch, int ci) {
   return row0 + kUnitRows * (ci * ((row1 - row0) / kUnitRows) / nch);
 }
-// weight stages of this CTA in one pass of the op
-__device__ __forceinline__ unsigned rows_stage_count(const OpDesc& op) {
-  int row0, row1;
-  bool any;
-  rows_range(op, row0, row1, any);
-  return (unsigned)((row1 - row0 + kChunkRows - 1) / kChunkRows) * (unsigned)op.nkt;
-}
-
 __device__ __noinline__ void linear_pass_rows(Ctx& c, const OpDesc& op, int tok0, int T, const uint4* pre_w) {
   const KParams& p = c.p;
   const int nks = op.nkt;
@@ -1825,21 +1211,17 @@ __device__ __noinline__ void linear_pass_rows(Ctx& c, const OpDesc& op, int tok0
   c.cons_idx += consumed;
 }
 
-template <int PATH>
-__device__ void op_linear(Ctx& c, const OpDesc& op, int T) {
+__device__ void op_linear_rows(Ctx& c, const OpDesc& op, int T) {
   // the norm weights do not depend on other CTAs: fetched ahead of the barrier
   uint4 pre_w[4] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
-  bool pre = false;
-  if constexpr (PATH != PATH_UMMA) {
-    const int wpr0 = stage_warps_per_row(min(op.aux3, T));
-    const int kvec_pad = op.nkt * ((PATH == PATH_ROWS ? kRowsStageK : kTileK) >> 3);  // padded row, in 16-byte vectors
-    pre = (op.flags & F_NORM_IN) && kvec_pad <= 128 * wpr0;
-    if (pre) {
+  const int wpr0 = stage_warps_per_row(min(op.aux3, T));
+  const int kvec_pad = op.nkt * (kRowsStageK >> 3);  // padded row, in 16-byte vectors
+  const bool pre = (op.flags & F_NORM_IN) && kvec_pad <= 128 * wpr0;
+  if (pre) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int v = (c.warp % wpr0) * 32 + c.lane + 32 * wpr0 * i;
-        if (v < (op.k >> 3)) pre_w[i] = __ldg(reinterpret_cast<const uint4*>(op.norm_w) + v);
-      }
+    for (int i = 0; i < 4; ++i) {
+      const int v = (c.warp % wpr0) * 32 + c.lane + 32 * wpr0 * i;
+      if (v < (op.k >> 3)) pre_w[i] = __ldg(reinterpret_cast<const uint4*>(op.norm_w) + v);
     }
   }
 #if MK_WITH_XCHG
@@ -1853,24 +1235,11 @@ __device__ void op_linear(Ctx& c, const OpDesc& op, int T) {
     return;
   }
   c.lin_seq += 1;
-  if (c.tid == 0) c.flags()[4] = (int)c.lin_seq;  // the activation producer may now read this op's input
+  if (c.tid == 0) c.flags()[4] = (int)c.lin_seq;
   const int passes = linear_passes(op, T);
-  if constexpr (PATH == PATH_ROWS) {
-    for (int g = 0; g < passes; ++g) {
-      linear_pass_rows(c, op, g * op.aux3, T, (pre && g == 0) ? pre_w : nullptr);
-      if (g + 1 < passes) consumer_sync();  // (a pass leaves its last chunk's sums block without a sync of its own)
-    }
-  } else if constexpr (PATH == PATH_UMMA) {
-    for (int g = 0; g < passes; ++g) linear_pass_umma(c, op, g * op.aux3, T, g);
-  } else {
-    if (op.flags & F_XTILE) {
-      for (int g = 0; g < passes; ++g) {
-        if (c.p.x_rows == 8) linear_pass_wide<1>(c, op, g * op.aux3, T, g);
-        else linear_pass_wide<2>(c, op, g * op.aux3, T, g);
-      }
-    } else {
-      for (int g = 0; g < passes; ++g) linear_pass(c, op, g * op.aux3, T, g, (pre && g == 0) ? pre_w : nullptr);
-    }
+  for (int g = 0; g < passes; ++g) {
+    linear_pass_rows(c, op, g * op.aux3, T, (pre && g == 0) ? pre_w : nullptr);
+    if (g + 1 < passes) consumer_sync();  // (a pass leaves its last chunk's sums block without a sync of its own)
   }
   if (MK_XF(op, F_PUSH)) c.ar_seq += 1;  // every CTA counts the exchange, with or without rows of its own
 }
@@ -1944,7 +1313,6 @@ __device__ __noinline__ F8 head_norm_rope(F8 xin, uint4 wv, uint4 csv, uint4 snv
 struct AttnTask {
   int t, h, ch, L, p0, p1, nch, kv_base, new_page;
   bool valid;
-  uint4 wq, wk, cs, sn;
   uint4 kr[4], vr[4];
 };
 
@@ -1987,9 +1355,8 @@ __device__ __forceinline__ void attn_fetch_rows(const Ctx& c, const OpDesc& op, 
   }
 }
 
-// NORMW: also fetch the norm weights and the cos/sin row of the task's position (the single-task path fetches
-// them itself, next to the q/k rows: held from here on, they were spilled, and a spill waits for its load).
-template <bool NORMW = true, bool FETCH = true>
+// (The norm weights and the cos/sin row of the position are fetched later, next to the q/k rows: held from here on,
+// they were spilled, and a spill waits for its load.)
 __device__ __forceinline__ void attn_prepare(const Ctx& c, const OpDesc& op, const AttnPlan& pl, const int* lens, int task,
                                           int l16, AttnTask& a, int* pgc = nullptr, bool fill = false,
                                           int* geom = nullptr) {
@@ -2020,20 +1387,13 @@ __device__ __forceinline__ void attn_prepare(const Ctx& c, const OpDesc& op, con
       geom[5] = a.p0; geom[6] = a.p1; geom[7] = a.nch; geom[8] = a.kv_base;
     }
   }
-  if constexpr (NORMW) {
-    const int pos = min(a.L - 1, op.aux2 - 1);  // aux2 = rows of the cos/sin tables
-    a.wq = __ldg(reinterpret_cast<const uint4*>(op.q_norm_w) + l16);
-    a.wk = __ldg(reinterpret_cast<const uint4*>(op.k_norm_w) + l16);
-    a.cs = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.cos) + (size_t)pos * kHeadDim) + l16);
-    a.sn = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.sin) + (size_t)pos * kHeadDim) + l16);
-  }
   if (pgc != nullptr && !fill) {
     a.new_page = pgc[4];
   } else {
     a.new_page = (a.p1 == a.L) ? __ldcg(c.p.kv_indices + a.kv_base + ((a.L - 1) >> c.p.page_shift)) : 0;
     if (pgc != nullptr) pgc[4] = a.new_page;
   }
-  if constexpr (FETCH) attn_fetch_rows(c, op, pl, a, 0, l16, a.kr, a.vr, pgc, fill);
+  attn_fetch_rows(c, op, pl, a, 0, l16, a.kr, a.vr, pgc, fill);
 }
 
 // Merge of a (request, kv head)'s chunks by the CTA that arrived last: kept out of line, only a
@@ -2189,78 +1549,6 @@ __device__ __noinline__ void attn_merge_ll(Ctx& c, const uint2* base, __nv_bfloa
   }
 }
 
-// The half-warp's pass over its positions of the task: for up to four q heads of the kv-head
-// group, running (max, sum, output) per head.  Rows are consumed four at a time while the next
-// four are in flight; `a.kr/a.vr` hold the first batch (loaded ahead of the op's barrier).
-__device__ __forceinline__ void attn_rows(const Ctx& c, const OpDesc& op, const AttnPlan& pl, AttnTask& a, int l16, int hq,
-                                          const uint4* qv, uint4 knew, uint4 vnew, float sc, float* m, float* l,
-                                          float (*o)[8]) {
-  const int L = a.L;
-#pragma unroll
-  for (int h = 0; h < 4; ++h) {
-    m[h] = -INFINITY;
-    l[h] = 0.f;
-#pragma unroll
-    for (int i = 0; i < 8; ++i) o[h][i] = 0.f;
-  }
-  const int niter = (a.p1 - a.p0 + pl.ngroups - 1) / pl.ngroups;
-#pragma unroll 1
-  for (int it = 0; it < niter; it += 4) {
-    // the next four rows are requested before this batch is used
-    uint4 nk[4], nv[4];
-    const bool more = it + 4 < niter;
-    if (more) attn_fetch_rows(c, op, pl, a, it + 4, l16, nk, nv);
-    // The row loop stays rolled (this code runs once per layer out of a cold instruction
-    // cache; its size is its cost): the batch's rows are rotated through slot 0 instead of
-    // being indexed.
-#pragma unroll 1
-    for (int u = 0; u < 4; ++u) {
-      const int j = a.p0 + (it + u) * pl.ngroups + pl.gi;
-      const bool ok = j < a.p1;  // may differ between the two halves of a warp: no shuffle may depend on it
-      if (__any_sync(0xffffffffu, ok)) {
-        uint4 kr = a.kr[0], vr = a.vr[0];
-        if (ok && j == L - 1) {
-          kr = knew;
-          vr = vnew;
-        }
-        float kk[8], vf[8];
-        unpack8(kr, kk);
-        unpack8(vr, vf);
-#pragma unroll
-        for (int h = 0; h < 4; ++h) {
-          if (h < hq) {  // uniform
-            float qf[8];
-            unpack8(qv[h], qf);
-            float d = 0.f;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) d = fmaf(qf[i], kk[i], d);
-#pragma unroll
-            for (int x = 8; x > 0; x >>= 1) d += __shfl_xor_sync(0xffffffffu, d, x);
-            if (ok) {
-              const float sv = d * sc;
-              const float mn = fmaxf(m[h], sv);
-              const float alpha = exp2f(m[h] - mn), pr = exp2f(sv - mn);
-              l[h] = l[h] * alpha + pr;
-#pragma unroll
-              for (int i = 0; i < 8; ++i) o[h][i] = fmaf(pr, vf[i], o[h][i] * alpha);
-              m[h] = mn;
-            }
-          }
-        }
-      }
-      a.kr[0] = a.kr[1]; a.kr[1] = a.kr[2]; a.kr[2] = a.kr[3];
-      a.vr[0] = a.vr[1]; a.vr[1] = a.vr[2]; a.vr[2] = a.vr[3];
-    }
-    if (more) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        a.kr[u] = nk[u];
-        a.vr[u] = nv[u];
-      }
-    }
-  }
-}
-
 // The same pass for ONE q head per half-warp (the single-chunk-per-CTA path): running
 // (max, sum, output) of the half-warp's positions of the task.  Four rows are handled as one
 // batch: their dot products and the four shuffle trees run side by side, and the running
@@ -2410,282 +1698,7 @@ __device__ __noinline__ bool attn_barrier_then_append(Ctx& c, const OpDesc& op, 
   return c.dead;
 }
 
-// Larger batches: with more (request, kv head) pairs than CTAs and sequences short enough to
-// need no split, a CTA runs 2 or 4 pairs side by side instead of one after the other: its 8
-// warps form groups of 4 or 2, every group is a small copy of the CTA-wide scheme (its warps
-// split the positions, a half-warp serves all q heads of the pair, the group meets on a
-// named barrier of its own).  The fixed latencies of a pair (q path, row fetches, combine)
-// are then paid once per round of `groups` pairs.
-__device__ __forceinline__ void group_sync(int g, int nthreads) {
-  asm volatile("bar.sync %0, %1;" ::"r"(2 + g), "r"(nthreads) : "memory");
-}
-__device__ __noinline__ void attention_groups(Ctx& c, const OpDesc& op, const AttnPlan& pl0, const int* lens, int wpg, int T, bool chunked) {
-  const KParams& p = c.p;
-  const int G = gridDim.x;
-  AttnPlan pl = pl0;
-  const int ngrp = kNumConsumerWarps / wpg;
-  const int g = c.warp / wpg, lw = c.warp % wpg;
-  const int gthreads = wpg * 32, gtid = lw * 32 + c.lane;
-  const int l16 = c.lane & 15;
-  const int hq = pl.qpk;  // at most 4 here
-  pl.ngroups = 2 * wpg;
-  pl.gi = 2 * lw + (c.lane >> 4);
-  const float sc = 1.4426950408889634f * 0.08838834764831845f;  // log2(e) / sqrt(128)
-  const bool dbl_q = op.aux1 < 32, dbl_k = op.aux0 < 32;
-  // per group: q heads [4][16] + new k [16] (bf16 x 8 per entry); per warp: 4 heads x 128 floats, (max, sum) x 4
-  uint4* sm_q = reinterpret_cast<uint4*>(c.smem + p.x_off) + g * 80;
-  uint4* sm_k = sm_q + 64;
-  float* sm_o = reinterpret_cast<float*>(reinterpret_cast<uint4*>(c.smem + p.x_off) + 4 * 80) + c.warp * 4 * kHeadDim;
-  float* sm_ml = reinterpret_cast<float*>(reinterpret_cast<uint4*>(c.smem + p.x_off) + 4 * 80) + kNumConsumerWarps * 4 * kHeadDim;
-  bool first = true;
-  if (chunked) {
-    if (attn_barrier_then_append(c, op, pl, lens, T)) return;
-    first = false;
-  }
-#pragma unroll 1
-  for (int task = blockIdx.x + G * g;; task += G * ngrp) {
-    AttnTask a;
-    attn_prepare(c, op, pl, lens, task, l16, a);
-    if (first) {
-      first = false;
-      if (op.flags & F_SYNC_BEFORE) {  // op_barrier with the wait inlined: the prefetched rows stay in registers
-        grid_wait(c);
-        if (c.pr != nullptr && c.tid == 0) c.pr[1] = globaltimer();
-        c.dead = c.flags()[3] != 0;
-        if (c.dead) return;
-      } else if (op_barrier(c, op)) {
-        return;
-      }
-    }
-    if (task >= pl.ntasks) break;   // uniform within the group
-    if (!a.valid) continue;
-    const int L = a.L;
-    const __nv_bfloat16* row = reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)a.t * op.ld_in +
-                               (size_t)a.h * (pl.qpk + 2) * kHeadDim;
-    const uint4 vnew = __ldcg(reinterpret_cast<const uint4*>(row + (pl.qpk + 1) * kHeadDim) + l16);
-#pragma unroll 1
-    for (int h = lw; h < hq; h += wpg) {  // this warp's share of the q heads
-      F8 q;
-      unpack8(__ldcg(reinterpret_cast<const uint4*>(row + h * kHeadDim) + l16), q.v);
-      q = head_norm_rope(q, a.wq, a.cs, a.sn, l16, op.flags, p.numerics, dbl_q);
-      if (c.lane < 16) sm_q[h * 16 + l16] = pack8(q.v);
-    }
-    if (lw == wpg - 1) {  // the group's last warp also prepares the new k
-      F8 kf;
-      unpack8(__ldcg(reinterpret_cast<const uint4*>(row + pl.qpk * kHeadDim) + l16), kf.v);
-      kf = head_norm_rope(kf, a.wk, a.cs, a.sn, l16, op.flags, p.numerics, dbl_k);
-      const uint4 kn = pack8(kf.v);
-      if (c.lane < 16) {
-        sm_k[l16] = kn;
-        if (a.p1 == L && !chunked) {  // append the new token's K and V to the cache
-          const size_t dst = ((((size_t)a.new_page << p.page_shift) + ((L - 1) & (p.page_size - 1))) * pl.HKV + a.h) * kHeadDim;
-          reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(op.k_cache) + dst)[l16] = kn;
-          reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(op.v_cache) + dst)[l16] = vnew;
-        }
-      }
-    }
-    group_sync(g, gthreads);
-    uint4 qv[4];
-#pragma unroll
-    for (int h = 0; h < 4; ++h) qv[h] = (h < hq) ? sm_q[h * 16 + l16] : make_uint4(0, 0, 0, 0);
-    const uint4 knew = sm_k[l16];
-    float m[4], l[4], o[4][8];
-    attn_rows(c, op, pl, a, l16, hq, qv, knew, vnew, sc, m, l, o);
-    // the two halves of a warp by shuffle, then the group's warps through shared memory
-#pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      if (h < hq) {
-        const float m2 = __shfl_xor_sync(0xffffffffu, m[h], 16), l2 = __shfl_xor_sync(0xffffffffu, l[h], 16);
-        const float M = fmaxf(m[h], m2);
-        const float f1 = (m[h] == -INFINITY) ? 0.f : exp2f(m[h] - M), f2 = (m2 == -INFINITY) ? 0.f : exp2f(m2 - M);
-        const float lsum = f1 * l[h] + f2 * l2;
-        float r[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) r[i] = f1 * o[h][i] + f2 * __shfl_xor_sync(0xffffffffu, o[h][i], 16);
-        if (c.lane < 16) {
-          float* dst = sm_o + h * kHeadDim + l16 * 8;
-          reinterpret_cast<float4*>(dst)[0] = make_float4(r[0], r[1], r[2], r[3]);
-          reinterpret_cast<float4*>(dst)[1] = make_float4(r[4], r[5], r[6], r[7]);
-          if (l16 == 0) {
-            sm_ml[(c.warp * 4 + h) * 2] = M;
-            sm_ml[(c.warp * 4 + h) * 2 + 1] = lsum;
-          }
-        }
-      }
-    }
-    group_sync(g, gthreads);
-    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out) + (size_t)a.t * op.ld_out +
-                         (size_t)a.h * pl.qpk * kHeadDim;
-    const float* go = reinterpret_cast<const float*>(reinterpret_cast<const uint4*>(c.smem + p.x_off) + 4 * 80) +
-                      (size_t)(g * wpg) * 4 * kHeadDim;  // the group's first warp slot
-#pragma unroll 1
-    for (int e = gtid; e < hq * kHeadDim; e += gthreads) {
-      const int h = e >> 7, d = e & 127;
-      float M = -INFINITY;
-      for (int w = 0; w < wpg; ++w) M = fmaxf(M, sm_ml[((g * wpg + w) * 4 + h) * 2]);
-      float Ls = 0.f, O = 0.f;
-      for (int w = 0; w < wpg; ++w) {
-        const float mw = sm_ml[((g * wpg + w) * 4 + h) * 2];
-        const float f = (mw == -INFINITY) ? 0.f : exp2f(mw - M);
-        Ls += f * sm_ml[((g * wpg + w) * 4 + h) * 2 + 1];
-        O += f * go[(w * 4 + h) * kHeadDim + d];
-      }
-      out[e] = __float2bfloat16_rn(__fdividef(O, Ls));
-    }
-    group_sync(g, gthreads);  // the group's buffers are free again
-  }
-}
-
-// aux0 = kv heads, aux1 = q heads (q heads per kv head: 1, 2, 4 or 8).  Tokens: one per
-// request, token t == request slot t.
-// The pass of a task over its positions on the tensor cores (wider batches; up to four q heads per kv head).
-// One warp takes 16 positions at a time (tiles warp, warp + 8, ... of the task's range) for all q heads:
-//   S = Q K^T   mma.m16n8k16, M = the q heads (rows 4..15 are padding), N = 8 positions, K = 128 dims in 8 steps
-//   O += P V    M = the q heads, K = 16 positions, N = 128 dims in 16 tiles of 8
-// with the fragments loaded STRAIGHT from the cache rows, no shared-memory staging and no ldmatrix: a dot
-// product does not care in which order the dims are walked, so k step s of lane j of a quad stands for dims
-// 32 (s / 2) + 8 j + 4 (s % 2) + {0..3} (the quad reads 64 contiguous bytes of the K row of position lane / 4
-// per load), and output column n of tile t stands for dim 64 (t / 8) + 8 n + t % 8 (eight lanes read 128
-// contiguous bytes of a V row per load; two rows are paired up per register with byte permutes).  The scalar pass (attn_rows1) issued about twenty times the instructions per position.
-// Leaves (max, sum, output) of slot warp * qpk + head in shared memory for the combine.
-__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
-  uint32_t r;
-  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
-  return r;
-}
-// (rows 8..15 of the M side are padding: their two accumulators are scratch registers shared by all tiles)
-__device__ __forceinline__ void mma_bf16_top(float& c0, float& c1, float& z0, float& z1, uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-               : "+f"(c0), "+f"(c1), "+f"(z0), "+f"(z1)
-               : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
-}
-__device__ __noinline__ void attn_tc_rows(const Ctx& c, const OpDesc& op, const AttnPlan& pl, const AttnTask& a, const uint4* sm_q,
-                                          const uint4* sm_knew, const uint4* sm_vnew, float sc, float* sm_o, float* sm_m,
-                                          float* sm_l, const int* pgt, bool subst_new) {
-  const int lane = c.lane, g = lane >> 2, j = lane & 3;
-  const int psh = c.p.page_shift, pmask = c.p.page_size - 1;
-  const bool hv = g < pl.qpk;
-  uint32_t qa0[8], qa2[8];
-#pragma unroll
-  for (int s = 0; s < 8; ++s) {
-    const uint2 v = hv ? *reinterpret_cast<const uint2*>(reinterpret_cast<const char*>(sm_q) + g * 256 + (32 * (s >> 1) + 8 * j + 4 * (s & 1)) * 2)
-                       : make_uint2(0u, 0u);
-    qa0[s] = v.x;
-    qa2[s] = v.y;
-  }
-  float m = -INFINITY, l = 0.f;
-  float oacc[16][2], z0 = 0.f, z1 = 0.f;
-#pragma unroll
-  for (int t = 0; t < 16; ++t) oacc[t][0] = oacc[t][1] = 0.f;
-  const int base_slot = a.p0 >> psh;
-  const int ntiles = (a.p1 - a.p0 + 15) >> 4;
-  const char* kc = reinterpret_cast<const char*>(op.k_cache);
-  const char* vc = reinterpret_cast<const char*>(op.v_cache);
-#pragma unroll 1
-  for (int ti = c.warp; ti < ntiles; ti += kNumConsumerWarps) {
-    const int pos0 = a.p0 + 16 * ti;
-    // K: positions pos0 + g and pos0 + 8 + g, dims [32 j, 32 j + 32)
-    uint4 kr[2][4];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      const int pos = pos0 + 8 * u + g;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) kr[u][i] = make_uint4(0u, 0u, 0u, 0u);
-      if (pos < a.p1) {
-        if (subst_new && pos == a.L - 1) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) kr[u][i] = sm_knew[4 * i + j];
-        } else {
-          const int slot = (pos >> psh) - base_slot;
-          const int pg = slot < 32 ? pgt[slot] : __ldcg(c.p.kv_indices + a.kv_base + (pos >> psh));
-          const uint4* src = reinterpret_cast<const uint4*>(kc + ((((size_t)pg << psh) + (pos & pmask)) * pl.HKV + a.h) * (kHeadDim * 2)) + j;
-#pragma unroll
-          for (int i = 0; i < 4; ++i) kr[u][i] = __ldcg(src + 4 * i);  // a quad reads 64 contiguous bytes per load
-        }
-      }
-    }
-    // V: positions pos0 + 2 j + {0, 1} and pos0 + 8 + 2 j + {0, 1}, dims [16 g, 16 g + 16)
-    uint4 vr[4][2];
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int pos = pos0 + 2 * j + (r & 1) + 8 * (r >> 1);
-      vr[r][0] = vr[r][1] = make_uint4(0u, 0u, 0u, 0u);
-      if (pos < a.p1) {
-        if (subst_new && pos == a.L - 1) {
-          vr[r][0] = sm_vnew[g];
-          vr[r][1] = sm_vnew[8 + g];
-        } else {
-          const int slot = (pos >> psh) - base_slot;
-          const int pg = slot < 32 ? pgt[slot] : __ldcg(c.p.kv_indices + a.kv_base + (pos >> psh));
-          const uint4* src = reinterpret_cast<const uint4*>(vc + ((((size_t)pg << psh) + (pos & pmask)) * pl.HKV + a.h) * (kHeadDim * 2)) + g;
-          vr[r][0] = __ldcg(src);  // the eight lanes with this j read 128 contiguous bytes per load
-          vr[r][1] = __ldcg(src + 8);
-        }
-      }
-    }
-    // S = Q K^T for the two groups of 8 positions
-    float sv[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-    for (int s = 0; s < 8; ++s) {
-      const uint4& k0 = kr[0][s >> 1];
-      const uint4& k1 = kr[1][s >> 1];
-      mma_bf16_top(sv[0], sv[1], z0, z1, qa0[s], qa2[s], (s & 1) ? k0.z : k0.x, (s & 1) ? k0.w : k0.y);
-      mma_bf16_top(sv[2], sv[3], z0, z1, qa0[s], qa2[s], (s & 1) ? k1.z : k1.x, (s & 1) ? k1.w : k1.y);
-    }
-    // this lane: head g at positions pos0 + 2 j + {0, 1} (sv[0], sv[1]) and pos0 + 8 + 2 j + {0, 1} (sv[2], sv[3])
-    float tmax = -INFINITY;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int pos = pos0 + 2 * j + (i & 1) + 8 * (i >> 1);
-      sv[i] = pos < a.p1 ? sv[i] * sc : -INFINITY;
-      tmax = fmaxf(tmax, sv[i]);
-    }
-    tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
-    tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
-    const float mn = fmaxf(m, tmax);  // finite: the tile holds at least one position of the range
-    const float alpha = exp2f(m - mn);
-    float pr[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) pr[i] = exp2f(sv[i] - mn);
-    l = l * alpha + ((pr[0] + pr[1]) + (pr[2] + pr[3]));  // this lane's share of the row sum: the quad adds up at the end
-    m = mn;
-    const uint32_t pa0 = pack2(pr[0], pr[1]), pa2 = pack2(pr[2], pr[3]);
-#pragma unroll
-    for (int t = 0; t < 16; ++t) {
-      oacc[t][0] *= alpha;
-      oacc[t][1] *= alpha;
-      // dim 16 g + t of the four V rows: element t of the lane's 16, two rows per register
-      const uint4& a0 = vr[0][t >> 3];
-      const uint4& a1 = vr[1][t >> 3];
-      const uint4& a2 = vr[2][t >> 3];
-      const uint4& a3 = vr[3][t >> 3];
-      const int w = (t >> 1) & 3;
-      const uint32_t w0 = w == 0 ? a0.x : (w == 1 ? a0.y : (w == 2 ? a0.z : a0.w));
-      const uint32_t w1 = w == 0 ? a1.x : (w == 1 ? a1.y : (w == 2 ? a1.z : a1.w));
-      const uint32_t w2 = w == 0 ? a2.x : (w == 1 ? a2.y : (w == 2 ? a2.z : a2.w));
-      const uint32_t w3 = w == 0 ? a3.x : (w == 1 ? a3.y : (w == 2 ? a3.z : a3.w));
-      const uint32_t sel = (t & 1) ? 0x7632u : 0x5410u;
-      mma_bf16_top(oacc[t][0], oacc[t][1], z0, z1, pa0, pa2, prmt(w0, w1, sel), prmt(w2, w3, sel));
-    }
-  }
-  l += __shfl_xor_sync(0xffffffffu, l, 1);
-  l += __shfl_xor_sync(0xffffffffu, l, 2);
-  if (hv) {
-    const int w = c.warp * pl.qpk + g;
-    if (j == 0) {
-      sm_m[w] = m;
-      sm_l[w] = l;
-    }
-    float* dst = sm_o + w * kHeadDim + 16 * j;
-#pragma unroll
-    for (int t = 0; t < 16; ++t) {
-      dst[64 * (t >> 3) + (t & 7)] = oacc[t][0];
-      dst[64 * (t >> 3) + 8 + (t & 7)] = oacc[t][1];
-    }
-  }
-}
-
-template <int PATH>
+// aux0 = kv heads, aux1 = q heads (q heads per kv head: 1, 2, 4 or 8).  The row-owner path's attention: one or two tokens.
 __device__ __noinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
   const KParams& p = c.p;
   const int G = gridDim.x;
@@ -2733,7 +1746,6 @@ __device__ __noinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
   pl.qpk = op.aux1 / op.aux0;
   int* plan = pgs + 16;   // [0] chunk size, [1] chunks of the longest request, [2] tasks: the same in every layer of an iteration
   int* geom = plan + 3;   // [9]: the CTA's first task, see attn_prepare
-  bool all_short;         // no sequence of the iteration is longer than 256 tokens (bit 8 of plan[1])
   if (fill) {
     int Lmax = 1;
 #pragma unroll 1
@@ -2747,30 +1759,16 @@ __device__ __noinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
     pl.CS = bpc * 16;
     pl.nch_max = (nb_max + bpc - 1) / bpc;
     pl.ntasks = T * pl.HKV * pl.nch_max;
-    all_short = Lmax <= 256;
     if (c.tid == 0) {
       plan[0] = pl.CS;
-      plan[1] = pl.nch_max | (all_short ? 256 : 0);
+      plan[1] = pl.nch_max;
       plan[2] = pl.ntasks;
     }
   } else {
     pl.CS = plan[0];
-    pl.nch_max = plan[1] & 255;
-    all_short = (plan[1] & 256) != 0;
+    pl.nch_max = plan[1];
     pl.ntasks = plan[2];
   }
-  // More (request, kv head) pairs than CTAs, all of them short: several pairs side by side per CTA (the fixed
-  // cost of a pair, about 12 us, dominates; measured at 64 requests of 100 tokens: 48 us against 68 us one
-  // pair at a time).
-  if constexpr (PATH == PATH_UMMA) {
-    if (pl.nch_max == 1 && pl.ntasks > G && pl.qpk <= 4 && all_short) {
-      attention_groups(c, op, pl, lens, pl.ntasks > 2 * G ? 2 : 4, T, *multi != 0);
-      return;
-    }
-  }
-  // wider batches: the pass over the positions runs on the tensor cores (up to four q heads per kv head; measured
-  // at 16 requests: 20 us against 24 us at 100 tokens, 33 us against 83 us at 600; slower below 9 batched tokens)
-  const bool tc = PATH != PATH_ROWS && pl.qpk <= 4 && p.x_rows >= 16;
   const int l16 = c.lane & 15;
   // Half-warp hw serves q head (hw % qpk) of the kv-head group for the positions of group
   // (hw / qpk): one head per thread keeps the row loop and the combine small (this code runs
@@ -2778,18 +1776,16 @@ __device__ __noinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
   // same K/V rows, so their loads share a request.
   const int hw = 2 * c.warp + (c.lane >> 4);
   const int head = hw % pl.qpk;
-  pl.ngroups = tc ? kNumConsumerWarps : 16 / pl.qpk;  // slots per head in the combine: warps, or half-warp groups
+  pl.ngroups = 16 / pl.qpk;  // slots per head in the combine
   pl.gi = hw / pl.qpk;
   const int part_stride = pl.qpk * (kHeadDim + 2);
   const float sc = 1.4426950408889634f * 0.08838834764831845f;  // log2(e) / sqrt(128)
   uint4* sm_q = reinterpret_cast<uint4*>(c.smem + p.x_off);     // [8 heads][16 lanes]: q after norm and RoPE
   uint4* sm_k = sm_q + 8 * 16;                                  // [16 lanes]: the new k
-  uint4* sm_v = sm_k + 16;                                      // [16 lanes]: the new v (tensor-core pass)
-  const int nslots = tc ? kNumConsumerWarps * pl.qpk : 16;
-  float* sm_o = reinterpret_cast<float*>(sm_v + 16);            // [slots][128]: 16 half-warps, or warp x head
+  constexpr int nslots = 16;                                    // half-warps
+  float* sm_o = reinterpret_cast<float*>(sm_k + 16);            // [slots][128]
   float* sm_m = sm_o + nslots * kHeadDim;                       // [slots]
   float* sm_l = sm_m + nslots;
-  int* pgt = reinterpret_cast<int*>(sm_l + nslots);             // [32]: page numbers of the task's range (tensor-core pass)
   const bool dbl_q = op.aux1 < 32, dbl_k = op.aux0 < 32;
   const int kw = pl.qpk & 7;  // the warp that prepares the new k (warp 0 when all eight prepare q heads)
 
@@ -2805,10 +1801,7 @@ __device__ __noinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
 #pragma unroll 1
   for (int task = blockIdx.x;; task += G) {
     AttnTask a;
-    if constexpr (PATH == PATH_ROWS)
-      attn_prepare<false>(c, op, pl, lens, task, l16, a, (first && !chunked) ? pgc : nullptr, fill, (first && !chunked) ? geom : nullptr);
-    else
-      attn_prepare<false, false>(c, op, pl, lens, task, l16, a, nullptr, true, nullptr);
+    attn_prepare(c, op, pl, lens, task, l16, a, (first && !chunked) ? pgc : nullptr, fill, (first && !chunked) ? geom : nullptr);
     if (first) {
       // everything above is independent of this layer's QKV rows: fetched ahead of the barrier
       first = false;
@@ -2817,7 +1810,7 @@ __device__ __noinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
           const int slot = (a.p0 >> p.page_shift) + c.tid;
           if ((slot << p.page_shift) < a.p1) pgs[c.tid] = __ldcg(p.kv_indices + a.kv_base + slot);
         }
-        if constexpr (PATH == PATH_ROWS) attn_l2_ahead(c, op, pl, a, l16, fill ? nullptr : pgs);
+        attn_l2_ahead(c, op, pl, a, l16, fill ? nullptr : pgs);
       }
       MK_STAMP(c, 1);
       if (op.flags & F_SYNC_BEFORE) {  // op_barrier, with the wait inlined
@@ -2888,7 +1881,6 @@ __device__ __noinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
       const uint4 kn = pack8(kf.v);
       if (c.lane < 16) {
         sm_k[l16] = kn;
-        sm_v[l16] = vnew;
         if (a.p1 == L && !chunked) {  // the last chunk appends the new token's K and V to the cache
           const size_t dst = ((((size_t)a.new_page << p.page_shift) + ((L - 1) & (p.page_size - 1))) * pl.HKV + a.h) * kHeadDim;
           reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(op.k_cache) + dst)[l16] = kn;
@@ -2896,24 +1888,12 @@ __device__ __noinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
         }
       }
     }
-    if (PATH != PATH_ROWS && tc && c.tid < 32) {  // the page numbers of the task's range, for the tensor-core pass
-      const int slot = (a.p0 >> p.page_shift) + c.tid;
-      if ((slot << p.page_shift) < a.p1) pgt[c.tid] = __ldcg(p.kv_indices + a.kv_base + slot);
-    }
     consumer_sync();
     MK_STAMP(c, 2);
-    bool done_rows = false;
-    if constexpr (PATH != PATH_ROWS) {
-      if (tc) {
-        attn_tc_rows(c, op, pl, a, sm_q, sm_k, sm_v, sc, sm_o, sm_m, sm_l, pgt, !chunked);
-        done_rows = true;
-      }
-    }
-    if (!done_rows) {
+    {
       const uint4 qv = sm_q[head * 16 + l16];
       const uint4 knew = sm_k[l16];
       float m, l, o[8];
-      if constexpr (PATH != PATH_ROWS) attn_fetch_rows(c, op, pl, a, 0, l16, a.kr, a.vr);  // (nothing was fetched ahead)
       attn_rows1(c, op, pl, a, l16, qv, knew, vnew, sc, m, l, o, (task == (int)blockIdx.x && !chunked) ? pgs : nullptr);
       // every half-warp leaves its (max, sum, output) in shared memory; one pass over the output
       // elements then combines the position groups of each head
@@ -3000,6 +1980,8 @@ __device__ __noinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
     MK_STAMP(c, 7);
   }
 }
+
+#include "mk_wide.cuh"
 
 // ------------------------------------------------------------------------------------
 // small ops
@@ -3706,7 +2688,7 @@ struct TileCursor {
 // Open the CTA's range of linear op `oi`; false if the op is not linear or gives this CTA nothing.
 __device__ __forceinline__ bool cursor_open(const KParams& p, TileCursor& tc, int oi) {
   const OpDesc& op = p.ops[oi];
-  if (op.type != OP_LINEAR || (op.flags & F_ROWS)) return false;
+  if (op.type != OP_LINEAR) return false;
   const unsigned total = (unsigned)op.nblk * (unsigned)op.nkt;
   const int G = (int)min(gridDim.x, total);
   if ((int)blockIdx.x >= G) return false;
@@ -3825,7 +2807,7 @@ __device__ __noinline__ void producer_loop(Ctx& c) {
   TileCursor pc;
   pc.valid = false;
   int ahead = 0;
-  if (PATH != PATH_ROWS && p.prefetch_tiles > 0)
+  if (PATH == PATH_WIDE && p.prefetch_tiles > 0)
     for (int oi = 0; oi < p.num_ops && !pc.valid; ++oi) pc.valid = cursor_open(p, pc, oi);
   // Weights are read once per step: their lines are marked evict-first on the way through L2, so
   // that what the look-ahead has fetched (and the KV cache) is not pushed out by bytes already used.
@@ -3993,55 +2975,48 @@ __device__ __noinline__ void producer_loop(Ctx& c) {
       } else {
       TileCursor lc;
       if (!cursor_open(p, lc, oi)) continue;
-      const int passes = linear_passes(p.ops[oi], T);
-      const unsigned t0 = lc.tile;
-      for (int g = 0; g < passes && !dead; ++g) {
-        if (g > 0) cursor_open(p, lc, oi);
-        for (unsigned tile = t0; tile < lc.t1; ++tile) {
-          if (g == 0 && pc.valid) {
-            while (ahead < p.prefetch_tiles) {
-              tma_prefetch_2d(pc.tmap, pc.kt * kTileK, pc.blk * kTileRows);
-              tma_prefetch_2d(pc.tmap, pc.kt * kTileK + kBoxK, pc.blk * kTileRows);
-              cursor_advance_wrap(p, pc);
-              ++ahead;
-            }
-            --ahead;
+      for (; lc.tile < lc.t1; ++lc.tile) {
+        if (pc.valid) {
+          while (ahead < p.prefetch_tiles) {
+            tma_prefetch_2d(pc.tmap, pc.kt * kTileK, pc.blk * kTileRows);
+            tma_prefetch_2d(pc.tmap, pc.kt * kTileK + kBoxK, pc.blk * kTileRows);
+            cursor_advance_wrap(p, pc);
+            ++ahead;
           }
-          if (!mbar_wait(c, bar_empty0 + 8 * s, empty_parity, ST_TIMEOUT_EMPTY)) {
-            dead = true;
-            break;
-          }
-          const uint32_t full = bar_full0 + 8 * s;
-          const uint32_t dst = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes;
-          mbar_arrive_expect_tx(full, kStageBytes);
-          tma_load_2d_hint(dst, lc.tmap, full, lc.kt * kTileK, lc.blk * kTileRows, pol_stream);
-          tma_load_2d_hint(dst + kSubBytes, lc.tmap, full, lc.kt * kTileK + kBoxK, lc.blk * kTileRows, pol_stream);
-          issued += 1;
-          fl[1] = (int)issued;
-          if (++s == S) {
-            s = 0;
-            empty_parity ^= 1u;
-          }
-          if (++lc.kt == lc.nkt) {
-            lc.kt = 0;
-            lc.blk += 1;
-          }
+          --ahead;
+        }
+        if (!mbar_wait(c, bar_empty0 + 8 * s, empty_parity, ST_TIMEOUT_EMPTY)) {
+          dead = true;
+          break;
+        }
+        const uint32_t full = bar_full0 + 8 * s;
+        const uint32_t dst = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes;
+        mbar_arrive_expect_tx(full, kStageBytes);
+        tma_load_2d_hint(dst, lc.tmap, full, lc.kt * kTileK, lc.blk * kTileRows, pol_stream);
+        tma_load_2d_hint(dst + kSubBytes, lc.tmap, full, lc.kt * kTileK + kBoxK, lc.blk * kTileRows, pol_stream);
+        issued += 1;
+        fl[1] = (int)issued;
+        if (++s == S) {
+          s = 0;
+          empty_parity ^= 1u;
+        }
+        if (++lc.kt == lc.nkt) {
+          lc.kt = 0;
+          lc.blk += 1;
         }
       }
-      }  // stream-K paths
+      }  // wide path
     }
     if (dead || p.mode == MODE_ONEPASS) break;
   }
   fl[1] = (int)issued;
 }
 
-// The activation producer (warp 9, one lane).  For wide-batch linear ops it walks the same
-// tile sequence as the weight producer and adds the input boxes to every stage, but only
-// after the consumers have passed the op's barrier: unlike weights, activations are the
-// previous op's output.
+// The activation producer of the wide path (warp 9, one lane).  It walks the same tile sequence
+// as the weight producer and adds the input boxes to every stage, but only after the consumers
+// have passed the op's barrier: unlike weights, activations are the previous op's output.
 __device__ __noinline__ void xproducer_loop(Ctx& c) {
   const KParams& p = c.p;
-  if (p.x_rows == 0) return;
   const int S = p.num_stages;
   volatile int* fl = c.flags();
   int s = 0;
@@ -4052,50 +3027,21 @@ __device__ __noinline__ void xproducer_loop(Ctx& c) {
   const uint32_t x_sub = (uint32_t)p.x_rows * 128u;
   for (int iter = 1;; ++iter) {
     int go;
-    {
-      unsigned long long t0 = 0;
-      int spins = 0;
-      while (true) {
-        go = fl[0];
-        if (go < 0 || (go >> 8) >= iter) break;
-        __nanosleep(40);
-        if (((++spins) & 255) == 0) {
-          if (aborted(c)) { go = -1; break; }
-          const unsigned long long now = globaltimer();
-          if (t0 == 0) t0 = now;
-          if (now - t0 > 4 * c.p.timeout_ns) { go = -1; break; }
-        }
-      }
-    }
-    if (go < 0) break;
-    const int T = go & 255;
+    if (!wait_go(c, fl, iter, go)) break;
     bool dead = false;
     for (int oi = 0; oi < p.num_ops && !dead; ++oi) {
       const OpDesc& op = p.ops[oi];
       if (op.type != OP_LINEAR) continue;
       lin_seq += 1;
-      if (op.flags & F_ROWS) {
-        const unsigned n = rows_stage_count(op) * (unsigned)linear_passes(op, T);
-        for (unsigned i = 0; i < n; ++i)
-          if (++s == S) { s = 0; empty_parity ^= 1u; }
-        continue;
-      }
       TileCursor lc;
       if (!cursor_open(p, lc, oi)) continue;
-      if (!(op.flags & F_XTILE)) {
-        // stages of this op carry no activation boxes, but they advance the ring
-        const unsigned n = (lc.t1 - lc.tile) * (unsigned)linear_passes(op, T);
-        for (unsigned i = 0; i < n; ++i)
-          if (++s == S) { s = 0; empty_parity ^= 1u; }
-        continue;
-      }
       // wait until the consumers have passed this op's barrier
       {
         unsigned long long t0 = 0;
         int spins = 0;
         while ((unsigned)fl[4] < lin_seq) {
           if (fl[0] < 0) { dead = true; break; }
-          __nanosleep(64);  // a hot spin would take issue slots from the consumer warps of this scheduler
+          __nanosleep(32);  // a hot spin would take issue slots from the consumer warps of this scheduler
           if (((++spins) & 1023) == 0) {
             if (aborted(c)) { dead = true; break; }
             const unsigned long long now = globaltimer();
@@ -4105,25 +3051,21 @@ __device__ __noinline__ void xproducer_loop(Ctx& c) {
         }
       }
       if (dead) break;
-      const int passes = linear_passes(op, T);
-      const unsigned t0 = lc.tile;
-      for (int g = 0; g < passes && !dead; ++g) {
-        if (g > 0) cursor_open(p, lc, oi);
-        for (unsigned tile = t0; tile < lc.t1; ++tile) {
-          if (!mbar_wait(c, bar_empty0 + 8 * s, empty_parity, ST_TIMEOUT_EMPTY)) {
-            dead = true;
-            break;
-          }
-          const uint32_t full = bar_x0 + 8 * s;
-          const uint32_t dst = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes + kStageBytes;
-          mbar_arrive_expect_tx(full, 2 * x_sub);
-          tma_load_2d(dst, op.tmap_x, full, lc.kt * kTileK, g * op.aux3);
-          tma_load_2d(dst + x_sub, op.tmap_x, full, lc.kt * kTileK + kBoxK, g * op.aux3);
-          issued_mask |= 1u << s;
-          xphase ^= 1u << s;
-          if (++s == S) { s = 0; empty_parity ^= 1u; }
-          if (++lc.kt == lc.nkt) { lc.kt = 0; lc.blk += 1; }
+      asm volatile("fence.proxy.async;" ::: "memory");  // the rows were written with plain stores, TMA reads them
+      for (; lc.tile < lc.t1; ++lc.tile) {
+        if (!mbar_wait(c, bar_empty0 + 8 * s, empty_parity, ST_TIMEOUT_EMPTY)) {
+          dead = true;
+          break;
         }
+        const uint32_t full = bar_x0 + 8 * s;
+        const uint32_t dst = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes + kStageBytes;
+        mbar_arrive_expect_tx(full, 2 * x_sub);
+        tma_load_2d(dst, op.tmap_x, full, lc.kt * kTileK, 0);
+        tma_load_2d(dst + x_sub, op.tmap_x, full, lc.kt * kTileK + kBoxK, 0);
+        issued_mask |= 1u << s;
+        xphase ^= 1u << s;
+        if (++s == S) { s = 0; empty_parity ^= 1u; }
+        if (++lc.kt == lc.nkt) { lc.kt = 0; lc.blk += 1; }
       }
     }
     if (dead || p.mode == MODE_ONEPASS) break;
@@ -4137,7 +3079,7 @@ __device__ __noinline__ void xproducer_loop(Ctx& c) {
 // the kernel
 // ------------------------------------------------------------------------------------
 template <int PATH>
-__global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_constant__ KParams p) {
+__global__ void __launch_bounds__(PATH == PATH_WIDE ? kWideThreads : kNumThreads, 1) megakernel(const __grid_constant__ KParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   Ctx c(p);
   // 128-byte-swizzled TMA stages need a 1024-byte-aligned base; the host budgets the slack
@@ -4153,12 +3095,10 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
   if (c.cl_size > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(c.cl_rank));
 #endif
   c.cons_idx = 0;
-  c.xphase = 0;
   c.arrived = false;
   c.attn_iter = -1;
   c.tmem = 0u;
-  c.has_tmem = false;
-  c.done_phase = 0;
+  c.acc_runs = 0;
   c.tid = threadIdx.x;
   c.lane = threadIdx.x & 31;
   c.warp = threadIdx.x >> 5;
@@ -4173,10 +3113,14 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
   if (threadIdx.x == 0) {
     for (int s = 0; s < p.num_stages; ++s) {
       mbar_init(c.full_bar(s), 1);
-      mbar_init(c.empty_bar(s), kNumConsumerWarps);
+      mbar_init(c.empty_bar(s), PATH == PATH_WIDE ? 1 : kNumConsumerWarps);  // the commit of the stage's MMAs, or every consumer warp
       mbar_init(c.xfull_bar(s), 1);
     }
     mbar_init(c.done_bar(), 1);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(c.acc_full_bar(b), 1);
+      mbar_init(c.acc_empty_bar(b), kNumConsumerWarps);
+    }
 #if MK_HIER_BARRIER
     mbar_init(c.cl_arrive_bar(), c.cl_size);
     mbar_init(c.cl_open_bar(), 1);
@@ -4197,19 +3141,18 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
 #endif
-  // Tensor memory for the tcgen05 linears (32 or 64 token rows per box): x_rows columns of fp32
-  // accumulators, allocated once by warp 0 and freed by it when the CTA leaves.
-  constexpr bool use_tmem = PATH == PATH_UMMA;
+  // Tensor memory for the tcgen05 linears: two buffers of x_rows columns of fp32 accumulators,
+  // allocated once by warp 0 and freed by it when the CTA leaves.
+  constexpr bool use_tmem = PATH == PATH_WIDE;
   if (use_tmem) {
     if (c.warp == 0) {
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(c.tmem_slot()), "r"((uint32_t)p.x_rows) : "memory");
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(c.tmem_slot()), "r"(2u * (uint32_t)p.x_rows) : "memory");
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     c.tmem = *reinterpret_cast<volatile uint32_t*>(c.smem + p.bar_off + 24 * p.num_stages + 72);
-    c.has_tmem = true;
   }
 
   if (c.warp == kNumConsumerWarps) {
@@ -4220,6 +3163,11 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
       rows_prefetch_loop(c);
     } else {
       if (c.lane == 0) xproducer_loop(c);
+    }
+    __syncwarp();
+  } else if (PATH == PATH_WIDE && c.warp == kNumConsumerWarps + 2) {
+    if constexpr (PATH == PATH_WIDE) {
+      if (c.lane == 0) mma_loop(c);
     }
     __syncwarp();
   } else {
@@ -4283,12 +3231,15 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
       if (T <= 0) break;
       if (T > 255) T = 255;
       if (c.tid == 0) fl[0] = (iter << 8) | T;
+      if constexpr (PATH == PATH_WIDE) {
+        if (p.has_attn) wide_fill_tokens(c, T);
+      }
 
       // The op descriptors are read from a two-slot copy in shared memory: the next op's
       // descriptor is fetched asynchronously while the current op runs, so that no op starts
       // with a round trip to L2 for its own parameters.
       constexpr int kDescVecs = (int)(sizeof(OpDesc) / 16);
-      OpDesc* sdesc = reinterpret_cast<OpDesc*>(c.smem + p.bar_off + 512);
+      OpDesc* sdesc = reinterpret_cast<OpDesc*>(c.smem + p.desc_off);
       if (c.tid < kDescVecs)
         reinterpret_cast<uint4*>(&sdesc[0])[c.tid] = __ldg(reinterpret_cast<const uint4*>(&p.ops[0]) + c.tid);
       for (int oi = 0; oi < p.num_ops; ++oi) {
@@ -4315,9 +3266,13 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
         switch (op.type) {
           case OP_EMBED: if (!op_barrier(c, op)) op_embed(c, op, T); break;
           case OP_RMSNORM: op_rmsnorm(c, op, T); break;
-          case OP_LINEAR: op_linear<PATH>(c, op, T); break;
+          case OP_LINEAR:
+            if constexpr (PATH == PATH_WIDE) op_linear_wide(c, op, T);
+            else op_linear_rows(c, op, T);
+            break;
           case OP_ATTN:
-            op_attention<PATH>(c, op, T);
+            if constexpr (PATH == PATH_WIDE) op_attention_wide(c, op, T);
+            else op_attention(c, op, T);
             break;
           case OP_SILU_MUL: if (!op_barrier(c, op)) op_silu_mul(c, op, T); break;
           case OP_ARGMAX_PARTIAL: if (!op_barrier(c, op)) op_argmax_partial(c, op, T); break;
@@ -4350,20 +3305,14 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
   // no CTA may exit with a bulk copy still writing its shared memory
   if (threadIdx.x == 0) {
     const unsigned issued = (unsigned)fl[1];
-    for (unsigned i = c.cons_idx; i < issued; ++i)
+    for (unsigned i = PATH == PATH_WIDE ? (unsigned)fl[5] : c.cons_idx; i < issued; ++i)
       mbar_wait(c, c.full_bar(i % p.num_stages), (i / p.num_stages) & 1, ST_TIMEOUT_FULL);
   }
   __syncthreads();
   if (use_tmem && c.warp == 0) {
-    // every tensor-core operation of this CTA has completed before its columns are given back:
-    // one more commit collects whatever an aborted pass left in flight (bounded wait)
-    if (c.lane == 0) {
-      umma_commit(c.done_bar());
-      mbar_wait(c, c.done_bar(), c.done_phase & 1u, ST_TIMEOUT_FULL);
-    }
-    __syncwarp();
+    // (the MMA issuer has waited for everything it had in flight)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(c.tmem), "r"((uint32_t)p.x_rows) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(c.tmem), "r"(2u * (uint32_t)p.x_rows) : "memory");
   }
 #if MK_HIER_BARRIER
   if (c.cl_size > 1) {  // a peer may still be storing into this CTA's shared memory
@@ -4409,8 +3358,7 @@ __global__ void init_state_kernel(KParams p) {
 extern "C" const void* MK_CAT(mk_kernel_variant_, MK_VARIANT)(int path) {
   switch (path) {
     case mk::PATH_ROWS: return (const void*)mk::MK_VARIANT::megakernel<mk::PATH_ROWS>;
-    case mk::PATH_UMMA: return (const void*)mk::MK_VARIANT::megakernel<mk::PATH_UMMA>;
-    default: return (const void*)mk::MK_VARIANT::megakernel<mk::PATH_TILES>;
+    default: return (const void*)mk::MK_VARIANT::megakernel<mk::PATH_WIDE>;
   }
 }
 #else
@@ -4421,6 +3369,7 @@ extern "C" const void* mk_kernel_variant_tp(int path);
 extern "C" const void* mk_kernel_variant_hier(int path);
 extern "C" const void* mk_kernel_variant_moe(int path);
 namespace {
+int mk_kernel_threads(int path) { return path == mk::PATH_WIDE ? mk::kWideThreads : mk::kNumThreads; }
 // the build of the kernel a launch needs: tensor-parallel exchange code only when there are peers,
 // the hierarchical barrier only when the launch uses clusters
 const void* kernel_for(const mk::KParams* p) {
@@ -4429,8 +3378,7 @@ const void* kernel_for(const mk::KParams* p) {
   if (p->world > 1) return mk_kernel_variant_tp(p->path);
   switch (p->path) {
     case mk::PATH_ROWS: return (const void*)mk::MK_VARIANT::megakernel<mk::PATH_ROWS>;
-    case mk::PATH_UMMA: return (const void*)mk::MK_VARIANT::megakernel<mk::PATH_UMMA>;
-    default: return (const void*)mk::MK_VARIANT::megakernel<mk::PATH_TILES>;
+    default: return (const void*)mk::MK_VARIANT::megakernel<mk::PATH_WIDE>;
   }
 }
 }  // namespace
@@ -4439,7 +3387,7 @@ extern "C" int mk_kernel_max_ctas_per_sm(const mk::KParams* p, int smem_bytes) {
   int n = 0;
   const void* k = kernel_for(p);
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) return -1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, mk::kNumThreads, smem_bytes) != cudaSuccess) return -1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, mk_kernel_threads(p->path), smem_bytes) != cudaSuccess) return -1;
   return n;
 }
 
@@ -4449,7 +3397,7 @@ extern "C" int mk_kernel_max_clusters(int path, int smem_bytes, int cluster, int
   if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) return -1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(mk::kNumThreads);
+  cfg.blockDim = dim3(mk_kernel_threads(path));
   cfg.dynamicSmemBytes = (size_t)smem_bytes;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeClusterDimension;
@@ -4472,13 +3420,13 @@ extern "C" int mk_kernel_launch(const mk::KParams* p, int grid, int smem_bytes, 
   if (e != cudaSuccess) return (int)e;
   void* args[] = {(void*)p};
   if (p->cluster <= 1) {
-    e = cudaLaunchCooperativeKernel(k, dim3(grid), dim3(mk::kNumThreads), args, (size_t)smem_bytes, (cudaStream_t)stream);
+    e = cudaLaunchCooperativeKernel(k, dim3(grid), dim3(mk_kernel_threads(p->path)), args, (size_t)smem_bytes, (cudaStream_t)stream);
     return (int)e;
   }
   // co-resident grid of thread-block clusters
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(mk::kNumThreads);
+  cfg.blockDim = dim3(mk_kernel_threads(p->path));
   cfg.dynamicSmemBytes = (size_t)smem_bytes;
   cfg.stream = (cudaStream_t)stream;
   cudaLaunchAttribute at[2];

@@ -38,6 +38,8 @@ constexpr int kRowsSumsBytes = mk::kNumConsumerWarps * mk::kChunkRows * 2 * 4;  
 // token rows a row-owner CTA may keep resident beside three 32 KB weight stages
 constexpr int kRowsXBudget = kFastSmem - 2048 - kRedBytes - kRowsSumsBytes - 3 * mk::kStageBytes;
 constexpr int kAttnMaxChunks = 32;
+constexpr int kWideMaxStages = 5;  // ring stages of the wide path, shared memory permitting
+constexpr int kGateUpUnit = 4;     // fused gate/up weights are laid out [4 gate | 4 up] per 8-row unit
 constexpr int kMaxStepTimes = 16384;
 
 size_t dtype_size(int dt) {
@@ -59,7 +61,7 @@ struct Tensor {
   bool user = false;        // attached by the caller: contents are observable
   std::vector<int> src;     // shuffle/fuse sources
   int groups = 0;
-  int interleave = 0;  // > 0: two sources laid out as [g rows of src0 | g rows of src1] repeating (g = 64 or 4)
+  int interleave = 0;  // > 0: two sources laid out as [g rows of src0 | g rows of src1] repeating
   int readers = 0;
   int64_t numel() const {
     int64_t n = 1;
@@ -89,6 +91,7 @@ struct PlanOp {
   int n = 0, k = 0, aux0 = 0, aux1 = 0, aux2 = 0, aux3 = 0;
   int amax_n = 0;
   int ll_in_op = -1, ll_res_op = -1;  // tagged activations: the ops that produce the input / the residual
+  bool only_next_reads_out = false;   // nothing but the next op reads what this one writes (and the caller cannot see it)
   std::string note;
 };
 
@@ -130,7 +133,6 @@ struct mk_handle {
   int nprog = 0;
   int cur_prog = 0;          // program the next kernel of a launch uses
   int plan_tokens = 0;       // widest iteration the plan being built must serve
-  int force_interleave = 0;  // gate/up weight layout fixed by the primary program (4 or 64), 0 = the plan's own choice
   std::string err;
   void* meta[10] = {};
   int64_t total_requests = 0;
@@ -331,9 +333,6 @@ int plan_graph(mk_handle* h) {
     if (h->plan_tokens * (kpad + 8) * 2 + 16 > kRowsXBudget) rows_mode = false;
   }
   h->rows_mode = rows_mode;
-  // layout of fused gate/up weights: [4 gate | 4 up] per 8-row unit for the row-owner path, [64 | 64] per tile
-  // otherwise; a second program over the same weights takes the primary program's layout
-  const int gu_interleave = h->force_interleave ? h->force_interleave : (rows_mode ? 4 : 64);
   const int nops_all = (int)h->nops.size();
   // True when the value layer `i` writes into tensor `tid` is read by layer i+1 only:
   // walk the layers in execution order (wrapping into the next iteration) until the
@@ -535,8 +534,7 @@ int plan_graph(mk_handle* h) {
             prev.flags |= mk::F_SILU_MUL;
             prev.out = tmp;
             prev.note += prev.note.empty() ? "silu_mul fused" : ", silu_mul fused";
-            h->tensors[prev.w].interleave = gu_interleave;
-            if (gu_interleave == 4 && !rows_mode) prev.flags |= mk::F_SILU4;
+            h->tensors[prev.w].interleave = kGateUpUnit;
             fused_up = true;
           }
         }
@@ -561,8 +559,7 @@ int plan_graph(mk_handle* h) {
           return h->fail(MK_E_UNSUPPORTED, "%s: the weight must come from shuffle_tensors([gate, up]) and the output width be a multiple of 64", nm.c_str());
         po.flags |= mk::F_SILU_MUL;
         po.note = "silu_mul fused";
-        h->tensors[w].interleave = gu_interleave;
-        if (gu_interleave == 4 && !rows_mode) po.flags |= mk::F_SILU4;
+        h->tensors[w].interleave = kGateUpUnit;
       }
       po.type = mk::OP_LINEAR;
       if (rows_mode) po.flags |= mk::F_ROWS;
@@ -611,8 +608,7 @@ int plan_graph(mk_handle* h) {
           po.flags |= mk::F_SILU_MUL;
           po.out = sm.t[1];
           po.note += po.note.empty() ? "silu_mul fused" : ", silu_mul fused";
-          h->tensors[w].interleave = gu_interleave;
-        if (gu_interleave == 4 && !rows_mode) po.flags |= mk::F_SILU4;
+          h->tensors[w].interleave = kGateUpUnit;
           ++i;
         }
       }
@@ -828,6 +824,7 @@ int plan_graph(mk_handle* h) {
     } else {
       return h->fail(MK_E_UNSUPPORTED, "unknown layer '%s'", nm.c_str());
     }
+    if (po.type == mk::OP_LINEAR) po.only_next_reads_out = only_next_reads(i, po.out);
     if (pending_norm_out >= 0 && po.type != 0) {
       return h->fail(MK_E_STATE, "internal: a fused rmsnorm lost its linear");
     }
@@ -1104,7 +1101,7 @@ int mk_comm_connect(mk_handle* h, const unsigned char* handles, int n) {
 }
 
 // Shape class of an iteration width: which path and activation-box height the linears get.
-static int width_class(int tokens) { return tokens <= 2 ? 2 : (tokens <= 8 ? 8 : (tokens <= 16 ? 16 : (tokens <= 32 ? 32 : 64))); }
+static int width_class(int tokens) { return tokens <= 2 ? 2 : (tokens <= 16 ? 16 : (tokens <= 32 ? 32 : (tokens <= 64 ? 64 : 128))); }
 // Two programs when prompt chunks make some iterations wider than the decode iterations can be and the
 // two widths put the linears on different paths (otherwise one program planned for the wider one serves all).
 static bool two_programs(const mk_config& c) {
@@ -1122,7 +1119,6 @@ int mk_plan(mk_handle* h) {
   if (c.page_size < 1 || c.max_num_pages < 1 || c.max_seq_length < 2) return h->fail(MK_E_INVALID, "bad paging/sequence limits");
   if (c.page_size & (c.page_size - 1)) return h->fail(MK_E_UNSUPPORTED, "page_size must be a power of two (got %d)", c.page_size);
   if (c.world_size < 1 || c.rank < 0 || c.rank >= c.world_size) return h->fail(MK_E_INVALID, "bad rank/world_size");
-  h->force_interleave = 0;
   h->plan_tokens = two_programs(c) ? c.max_num_batched_requests : c.max_num_batched_tokens;
   return plan_graph(h);
 }
@@ -1196,64 +1192,87 @@ int mk_barrier_target_reached(uint32_t counter, uint32_t epoch, uint32_t arrival
   return (int)(counter - epoch * arrivals_per_barrier) >= 0 ? 1 : 0;
 }
 
+// What the wide path makes of a plan.  A fused input norm becomes an op of its own in front of the linear (the input
+// rows arrive by TMA), and where an attention op follows its QKV linear directly, nothing else can see that linear's
+// output and a row block of it is a head, the linear's epilogue applies QK-norm and RoPE and appends K and V
+// (F_QKV_PREP / F_QKV_READY).
+static int lower_wide(mk_handle* h) {
+  for (size_t i = 0; i < h->plan.size(); ++i) {
+    if (h->plan[i].type != mk::OP_LINEAR || !(h->plan[i].flags & mk::F_NORM_IN)) continue;
+    if (h->plan_tokens > 8) return h->fail(MK_E_UNSUPPORTED, "rmsnorm_linear is only built for up to 8 batched tokens");
+    PlanOp nrm;
+    PlanOp& lin = h->plan[i];
+    const int tmp = plan_temp_tensor(h, "__normed_" + std::to_string(lin.k), h->cfg.max_num_batched_tokens, lin.k);
+    if (tmp < 0) return tmp;
+    if (!h->tensors[tmp].ptr)
+      if (int e = h->dmalloc(&h->tensors[tmp].ptr, h->tensors[tmp].alloc_bytes())) return e;
+    nrm.type = mk::OP_RMSNORM;
+    nrm.flags = (lin.flags & (mk::F_SYNC_BEFORE | mk::F_GATHER_IN));
+    nrm.in = lin.in; nrm.w = lin.norm_w; nrm.out = tmp;
+    nrm.n = lin.k;
+    nrm.note = "from a fused input norm";
+    lin.in = tmp;
+    lin.norm_w = -1;
+    lin.flags = (lin.flags & ~(mk::F_NORM_IN | mk::F_GATHER_IN)) | mk::F_SYNC_BEFORE;
+    h->plan.insert(h->plan.begin() + i, nrm);
+    ++i;
+  }
+  for (size_t i = 1; i < h->plan.size(); ++i) {
+    PlanOp &at = h->plan[i], &lin = h->plan[i - 1];
+    if (at.type != mk::OP_ATTN || lin.type != mk::OP_LINEAR || lin.out != at.in || !lin.only_next_reads_out) continue;
+    if (lin.flags & (mk::F_RESIDUAL | mk::F_SILU_MUL | mk::F_ARGMAX | mk::F_PUSH)) continue;
+    if (!h->cfg.fuse || lin.n != (at.aux1 + 2 * at.aux0) * mk::kHeadDim) continue;
+    lin.flags |= mk::F_QKV_PREP;
+    at.flags |= mk::F_QKV_READY;
+    lin.note += lin.note.empty() ? "QK-norm, RoPE and KV append in the epilogue" : ", QK-norm, RoPE and KV append in the epilogue";
+  }
+  return 0;
+}
+
 // Everything of mk_compile that depends on the width a program is planned for (h->plan_tokens): the
 // shared-memory carve-up, scratch, tensor maps, op descriptors and kernel parameters of the plan in
 // h->plan.  `first`: also allocates the scheduler state the programs of a handle share.
 static int compile_program(mk_handle* h, bool first) {
   const mk_config& cfg = h->cfg;
   cudaError_t ce;
+  if (!h->rows_mode)
+    if (int e = lower_wide(h)) return e;
   // 2. shared-memory carve-up: [weight ring: stages x (32 KB of weights + two activation
-  // boxes of x_rows token rows)][x region: rows staged by the consumers for a fused input
-  // norm, attention scratch][sums block of a tile: 128 x x_rows floats][small scratch]
-  // [barriers, flags].  Above 8 tokens nothing is staged by the consumers and the sums
-  // block shares the x region.
-  const bool wide = h->plan_tokens > mk::kMaxTokGroup;
+  // boxes of x_rows token rows)][x region: resident token rows (row-owner path), attention
+  // scratch][row-owner path: sums block][small scratch][barriers, flags, op descriptors].
   const int nt = h->plan_tokens;
   const bool rows_mode = h->rows_mode;  // row-owner linears: resident token rows, no activation boxes
-  const int x_rows = rows_mode ? 0 : (nt <= 8 ? 8 : (nt <= 16 ? 16 : (nt <= 32 ? 32 : 64)));
+  const int x_rows = rows_mode ? 0 : (nt <= 16 ? 16 : (nt <= 32 ? 32 : (nt <= 64 ? 64 : 128)));
   const int stage_bytes = mk::kStageBytes + 2 * x_rows * 128;
-  const int sums_bytes = rows_mode ? kRowsSumsBytes : mk::kTileRows * x_rows * 4;
-  const int sums_sep = wide ? 0 : sums_bytes;
-  const int tb_max = std::min(mk::kMaxTokGroup, nt);
-  const int fixed0 = 1024 /*alignment slack*/ + sums_sep + kRedBytes + 1024 /*barriers, flags*/;
+  const int sums_bytes = rows_mode ? kRowsSumsBytes : 0;
+  const int red_bytes = rows_mode ? kRedBytes : mk::kWideRedBytes;
+  const int bar_bytes = rows_mode ? 1024 : 2048;  // barriers and flags, then the two op descriptors
+  const int fixed0 = 1024 /*alignment slack*/ + sums_bytes + red_bytes + bar_bytes;
   // Measured on B200: a CTA whose shared memory (plus the 1 KB the system adds) stays within
   // the 164 KB carve-out leaves 92 KB of the SM's unified array to L1, and the whole kernel
   // runs about 8 % faster than with the next carve-out (196 KB, 60 KB of L1).
   const int want_stages = cfg.max_stages > 0 ? std::min(cfg.max_stages, 16) : 4;
   // (row-owner mode prefers two resident token rows and three stages to one row and four)
-  int x_budget = rows_mode ? kRowsXBudget : kFastSmem - fixed0 - want_stages * stage_bytes;
-  int x_bytes = std::max(cfg.max_num_pages * 4, wide ? sums_bytes : 0);
-  int max_nblk = 1, n_linear = 0, min_tpp = rows_mode ? 2 : x_rows;
-  bool has_moe = false;
-  const int kpad_to = rows_mode ? mk::kRowsStageK : mk::kTileK;  // the staged rows are padded to whole stages
-  for (int attempt = 0; attempt < 2; ++attempt) {
-    bool fits = true;
-    for (PlanOp& p : h->plan) {
-      if (p.type != mk::OP_LINEAR || !(p.flags & (mk::F_NORM_IN | mk::F_ROWS))) continue;
-      const int kp = (p.k + kpad_to - 1) / kpad_to * kpad_to;
-      if ((x_budget - 16) / ((kp + 8) * 2) < 1) fits = false;
+  int x_budget = kRowsXBudget;
+  int x_bytes = cfg.max_num_pages * 4;
+  int max_nblk = 1, n_linear = 0;
+  bool has_moe = false, has_attn = false;
+  if (rows_mode)
+    for (const PlanOp& p : h->plan) {
+      if (p.type != mk::OP_LINEAR) continue;
+      const int kp = (p.k + mk::kRowsStageK - 1) / mk::kRowsStageK * mk::kRowsStageK;
+      if ((x_budget - 16) / ((kp + 8) * 2) < 1) x_budget = kMaxSmem - fixed0 - 3 * stage_bytes;  // a wide fused norm: give up the small carve-out
     }
-    if (fits) break;
-    x_budget = kMaxSmem - fixed0 - 3 * stage_bytes;  // a wide fused norm: give up the small carve-out
-  }
   for (PlanOp& p : h->plan) {
     if (p.type == mk::OP_LINEAR) {
       max_nblk = std::max(max_nblk, (p.n + mk::kTileRows - 1) / mk::kTileRows);
       ++n_linear;
-      if (wide && (p.flags & mk::F_NORM_IN)) return h->fail(MK_E_UNSUPPORTED, "rmsnorm_linear is only built for up to 8 batched tokens");
-      if (!(p.flags & (mk::F_NORM_IN | mk::F_ROWS))) {
-        // no fused norm: the input is read straight from the previous task's output, as
-        // activation boxes that ride with the weight stages
-        p.flags |= mk::F_XTILE;
-        p.aux3 = x_rows;
-        continue;
-      }
-      const int kp = (p.k + kpad_to - 1) / kpad_to * kpad_to;
+      if (!rows_mode) continue;  // the input arrives as activation boxes that ride with the weight stages
+      const int kp = (p.k + mk::kRowsStageK - 1) / mk::kRowsStageK * mk::kRowsStageK;
       const int row_bytes = (kp + 8) * 2;
-      int tpp = std::min(rows_mode ? std::min(2, nt) : tb_max, (x_budget - 16) / row_bytes);
+      int tpp = std::min(std::min(2, nt), (x_budget - 16) / row_bytes);
       if (tpp < 1) return h->fail(MK_E_UNSUPPORTED, "K=%d is too wide for a fused input norm", p.k);
       p.aux3 = tpp;
-      min_tpp = std::min(min_tpp, tpp);
       x_bytes = std::max(x_bytes, tpp * row_bytes + 16);
     } else if (p.type == mk::OP_MOE_LINEAR) {
       // a CTA stages the input rows of the pairs its share of the virtual row space (pairs x n rows) touches
@@ -1272,13 +1291,11 @@ static int compile_program(mk_handle* h, bool first) {
     } else if (p.type == mk::OP_RMSNORM) {
       x_bytes = std::max(x_bytes, ((p.n + 63) / 64 * 64 + 8) * 2 + 16);
     } else if (p.type == mk::OP_ATTN) {
-      // q heads and the new k (bf16), four combine slots of 4 heads x 128 floats, (max, sum) pairs, merge scratch
-      x_bytes = std::max(x_bytes, 9 * 256 + 4 * 4 * (mk::kHeadDim + 2) * 4 + 2 * kAttnMaxChunks * 8 * 4 + 64 + 256);
-      // above 16 tokens several (request, kv head) pairs run side by side in a CTA: q/k per group
-      // (4 x 1280 B) and one combine slot per warp (8 x 4 heads x 128 floats + (max, sum) pairs)
-      if (x_rows >= 32) x_bytes = std::max(x_bytes, 4 * 1280 + 8 * 4 * mk::kHeadDim * 4 + 8 * 4 * 2 * 4);
-      // the tensor-core pass of the wider paths: q heads, new k and v, (warp x head) combine slots, page numbers
-      if (!rows_mode) x_bytes = std::max(x_bytes, 10 * 256 + 8 * 4 * (mk::kHeadDim + 2) * 4 + 128 + 256);
+      has_attn = true;
+      // row-owner path: q heads and the new k (bf16), combine slots of 16 half-warps x 128 floats, (max, sum) pairs, merge scratch
+      if (rows_mode) x_bytes = std::max(x_bytes, 9 * 256 + 4 * 4 * (mk::kHeadDim + 2) * 4 + 2 * kAttnMaxChunks * 8 * 4 + 64 + 256);
+      // wide path: 2 KB per warp (q rows, then combine slots), (max, sum) pairs; the QKV epilogue transposes through the same 16 KB
+      else x_bytes = std::max(x_bytes, 16384 + mk::kNumConsumerWarps * 16 * 8);
     }
   }
   if (has_moe) x_bytes += 512;  // the expert ids of the pairs, for the producer (routing folded into the expert linear)
@@ -1287,7 +1304,8 @@ static int compile_program(mk_handle* h, bool first) {
   const int s_fast = (kFastSmem - fixed) / stage_bytes, s_max = (kMaxSmem - fixed) / stage_bytes;
   int stages;
   if (cfg.max_stages > 0) stages = std::min(s_max, want_stages);  // an explicit request wins
-  else stages = std::min(s_fast, 4) >= 3 ? std::min(s_fast, 4) : std::min(s_max, 4);
+  else if (rows_mode) stages = std::min(s_fast, 4) >= 3 ? std::min(s_fast, 4) : std::min(s_max, 4);
+  else stages = std::min(s_max, kWideMaxStages);
   if (stages < 2) return h->fail(MK_E_UNSUPPORTED, "activations need %d bytes of shared memory: no room for the weight ring", x_bytes);
   mk::KParams& kp = h->kp;
   memset(&kp, 0, sizeof(kp));
@@ -1296,12 +1314,14 @@ static int compile_program(mk_handle* h, bool first) {
   kp.x_rows = x_rows;
   kp.x_off = stages * stage_bytes;
   kp.x_bytes = x_bytes;
-  kp.sums_off = wide ? kp.x_off : kp.x_off + x_bytes;
-  kp.sums_stride = rows_mode ? 2 : x_rows;
-  kp.red_off = kp.x_off + x_bytes + sums_sep;
-  kp.bar_off = kp.red_off + kRedBytes;
-  h->smem_bytes = kp.bar_off + 1024 + 1024;
-  kp.path = rows_mode ? mk::PATH_ROWS : (x_rows >= 32 ? mk::PATH_UMMA : mk::PATH_TILES);
+  kp.sums_off = kp.x_off + x_bytes;
+  kp.sums_stride = 2;
+  kp.red_off = kp.x_off + x_bytes + sums_bytes;
+  kp.bar_off = kp.red_off + red_bytes;
+  kp.desc_off = kp.bar_off + bar_bytes / 2;
+  h->smem_bytes = kp.bar_off + bar_bytes + 1024;
+  kp.path = rows_mode ? mk::PATH_ROWS : mk::PATH_WIDE;
+  kp.has_attn = has_attn ? 1 : 0;
   kp.rank = cfg.rank;
   kp.world = cfg.world_size;
   kp.cluster = 1;
@@ -1329,6 +1349,11 @@ static int compile_program(mk_handle* h, bool first) {
     PlanOp& po = h->plan[i];
     if (po.type == mk::OP_LINEAR && (po.flags & mk::F_ROWS) && (po.flags & mk::F_ARGMAX)) {
       po.amax_n = std::min(h->grid, (po.n + mk::kUnitRows - 1) / mk::kUnitRows);
+      if (i + 1 < h->plan.size() && h->plan[i + 1].type == mk::OP_ARGMAX_REDUCE) h->plan[i + 1].amax_n = po.amax_n;
+    }
+    // wide LM head: one partial per CTA and row quarter of its tiles
+    if (po.type == mk::OP_LINEAR && !(po.flags & mk::F_ROWS) && (po.flags & mk::F_ARGMAX)) {
+      po.amax_n = h->grid * 4;
       if (i + 1 < h->plan.size() && h->plan[i + 1].type == mk::OP_ARGMAX_REDUCE) h->plan[i + 1].amax_n = po.amax_n;
     }
   }
@@ -1445,21 +1470,24 @@ static int compile_program(mk_handle* h, bool first) {
 
   // 3. scratch and state
   const int G = h->grid;
-  const int groups = (h->plan_tokens + min_tpp - 1) / min_tpp;
   void* p = nullptr;
-  if (int e = h->dmalloc(&p, (size_t)groups * G * 2 * mk::kTileRows * kp.sums_stride * 4)) return e;
+  if (int e = h->dmalloc(&p, (size_t)G * mk::kTileRows * x_rows * 4)) return e;
   kp.partial = (float*)p;
-  const size_t piece_count_bytes = (size_t)groups * max_nblk * 4;
-  h->piece_count_bytes = piece_count_bytes;
+  h->piece_count_bytes = rows_mode ? 4 : (size_t)max_nblk * mk::kNumConsumerWarps * 4;
   if (int e = h->dmalloc(&p, h->piece_count_bytes)) return e;
   kp.piece_count = (unsigned*)p;
-  kp.piece_stride = max_nblk;
   int max_hkv = 1, max_qpk = 2;
   for (const PlanOp& po : h->plan)
     if (po.type == mk::OP_ATTN) {
       max_hkv = std::max(max_hkv, po.aux0);
       max_qpk = std::max(max_qpk, po.aux1 / po.aux0);
     }
+  int max_q = 1;
+  for (const PlanOp& po : h->plan)
+    if (po.type == mk::OP_ATTN) max_q = std::max(max_q, po.aux1);
+  void* q_rows = nullptr;
+  if (!rows_mode && has_attn)
+    if (int e = h->dmalloc(&q_rows, (size_t)h->plan_tokens * max_q * mk::kHeadDim * 2)) return e;
   kp.attn_max_chunks = kAttnMaxChunks;
   if (int e = h->dmalloc(&p, (size_t)h->plan_tokens * max_hkv * kAttnMaxChunks * max_qpk * (mk::kHeadDim + 2) * 4)) return e;
   kp.attn_part = (float*)p;
@@ -1586,7 +1614,7 @@ static int compile_program(mk_handle* h, bool first) {
       if (r != CUDA_SUCCESS) return h->fail(MK_E_CUDA, "cuTensorMapEncodeTiled failed (%d) for %s [%d x %d]", (int)r, w.name.c_str(), po.n, po.k);
       map_of[i] = (int)maps.size();
       maps.push_back(m);
-      if (po.flags & mk::F_XTILE) {
+      {
         const Tensor& x = h->tensors[po.in];
         CUtensorMap mx;
         cuuint64_t xdim[2] = {(cuuint64_t)po.k, (cuuint64_t)x.dims[0]};
@@ -1644,12 +1672,25 @@ static int compile_program(mk_handle* h, bool first) {
       d.ld_in = (int)ti.strides[ti.ndim - 2];
       d.ld_out = (int)to.strides[to.ndim - 2];
     } else if (po.type == mk::OP_ATTN) {
-      d.k_cache = tp(po.kc);
-      d.v_cache = tp(po.vc);
-      d.q_norm_w = tp(po.qn);
-      d.k_norm_w = tp(po.kn);
-      d.cos = tp(po.cos);
-      d.sin = tp(po.sin);
+      auto attn_operands = [&](mk::OpDesc& x) {
+        x.k_cache = tp(po.kc);
+        x.v_cache = tp(po.vc);
+        x.q_norm_w = tp(po.qn);
+        x.k_norm_w = tp(po.kn);
+        x.cos = tp(po.cos);
+        x.sin = tp(po.sin);
+        if (rows_mode) return;
+        // wide path: the normalised, rotated q rows
+        x.out2 = q_rows;
+        x.ld_out2 = max_q * mk::kHeadDim;
+        x.aux3 = po.flags & (mk::F_QK_NORM | mk::F_ROPE);
+      };
+      attn_operands(d);
+      if (po.flags & mk::F_QKV_READY) {
+        mk::OpDesc& lin = descs[i - 1];
+        attn_operands(lin);
+        lin.aux0 = po.aux0; lin.aux1 = po.aux1; lin.aux2 = po.aux2;
+      }
     } else if (po.type == mk::OP_ARGMAX_PARTIAL) {
       void* q = nullptr;
       if (int e = h->dmalloc(&q, (size_t)h->plan_tokens * po.amax_n * 4)) return e;
@@ -1772,7 +1813,6 @@ int mk_compile(mk_handle* h) {
   h->nprog = 1;
   if (two) {
     h->plan_tokens = cfg.max_num_batched_tokens;
-    h->force_interleave = h->prog[0].rows_mode ? 4 : 64;
     if (int e = plan_graph(h)) return e;   // (same fusion decisions where they do not depend on the width)
     if (int e = compile_program(h, false)) return e;
     h->prog[1].plan = h->plan; h->prog[1].rows_mode = h->rows_mode; h->prog[1].max_tokens = h->plan_tokens;
@@ -1780,7 +1820,6 @@ int mk_compile(mk_handle* h) {
     h->prog[1].max_nblk = h->max_nblk;
     h->prog[1].attn_count_bytes = h->attn_count_bytes; h->prog[1].piece_count_bytes = h->piece_count_bytes;
     h->prog[1].ll_buf = h->ll_buf; h->prog[1].ll_bytes = h->ll_bytes;
-    h->force_interleave = 0;
     h->nprog = 2;
     h->prog[0].kp.tok_lo = 1;
     h->prog[0].kp.tok_hi = h->prog[0].max_tokens;

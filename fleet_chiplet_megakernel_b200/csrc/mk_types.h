@@ -21,8 +21,10 @@ constexpr int kSubBytes = kTileRows * kBoxK * 2;  // 16 KB
 constexpr int kStageBytes = kSubBytes * kSubTiles;
 constexpr int kNumConsumerWarps = 8;
 constexpr int kNumConsumers = kNumConsumerWarps * 32;
-constexpr int kNumThreads = kNumConsumers + 64;  // + the weight producer warp and the activation producer warp
-constexpr int kMaxTokGroup = 8;                  // tokens per pass of a linear op (one mma n-tile)
+// + the weight producer warp, the activation producer (or L2 look-ahead) warp and, on the wide path, the MMA issuer warp
+constexpr int kNumThreads = kNumConsumers + 64;
+constexpr int kWideThreads = kNumConsumers + 96;
+constexpr int kWideRedBytes = 4096;              // scratch of the wide path: reductions and the iteration's token table
 constexpr int kHeadDim = 128;
 // Row-owner linear (one or two batched tokens): a CTA owns a contiguous range of 8-row units
 // and walks it in chunks of up to 32 rows; a stage holds a chunk's rows for 512 k-elements
@@ -51,13 +53,14 @@ enum OpFlags : int {
   F_CTA0_ONLY = 1 << 1,     // only CTA 0 executes the body
   F_NORM_IN = 1 << 2,       // linear: RMSNorm fused on the input rows
   F_RESIDUAL = 1 << 3,      // linear: + residual
-  F_SILU_MUL = 1 << 4,      // linear: rows are [64 gate | 64 up] per tile, epilogue SiLU(gate)*up
+  F_SILU_MUL = 1 << 4,      // linear: rows are [4 gate | 4 up] per 8-row unit, epilogue SiLU(gate)*up
   F_ARGMAX = 1 << 5,        // linear: per-tile (max, index) of the bf16 logits
   F_QK_NORM = 1 << 6,       // attention
   F_ROPE = 1 << 7,          // attention
-  F_WRITE_NORM = 1 << 8,    // linear with F_NORM_IN: CTA 0 also stores the normalised rows
   F_RES_RANK0 = 1 << 9,     // residual only contributed when rank == 0 (row-parallel TP)
-  F_XTILE = 1 << 10,        // linear: input rows arrive per stage by TMA as activation boxes
+  F_QKV_PREP = 1 << 8,      // wide QKV linear: the epilogue applies QK-norm and RoPE, stores q to the attention's scratch rows (out2)
+                            // and k / v to the cache (aux0/aux1: kv/q heads, aux2: cos/sin rows, aux3: F_QK_NORM | F_ROPE)
+  F_QKV_READY = 1 << 10,    // wide attention: the linear before it has F_QKV_PREP
   F_ROWS = 1 << 11,         // linear: every CTA owns whole output rows (no split over k between CTAs)
   // tensor parallelism: the allreduce behind a row-parallel linear folded into its neighbours
   F_PUSH = 1 << 12,         // linear: the epilogue stores its fp32 sums into every rank's exchange slots instead of `out`
@@ -65,7 +68,6 @@ enum OpFlags : int {
   F_GATHER_RES = 1 << 14,   // linear: the residual is the rank-order sum of the latest exchange's slots
   F_MOE_PAIR_IN = 1 << 17,  // MoE linear: the input has one row per (token, slot) pair (the down projection), not one per token
   F_XRANK = 1 << 16,        // argmax reduce: the per-rank (value, index) pairs of a vocabulary-sharded LM head are exchanged and the global best is taken
-  F_SILU4 = 1 << 15,        // linear with F_SILU_MUL on the tile paths: rows are [4 gate | 4 up] per 8-row unit (the row-owner layout)
   // Tagged activations (row-owner path): a producer also stores its bf16 outputs as 8-byte words
   // {two adjacent columns, tag of the producing op in this iteration}; a consumer polls the words
   // it needs instead of waiting at a grid barrier, so data and "ready" arrive in one load.
@@ -91,9 +93,8 @@ enum Mode : int { MODE_OFFLINE = 0, MODE_ONEPASS = 1 };
 // path runs: the whole step executes out of the instruction cache once per layer, and code
 // that is merely present (other paths' loops) measurably slowed the batch-1 step down.
 enum Path : int {
-  PATH_ROWS = 0,   // 1-2 tokens: row-owner linears, resident token rows, L2 look-ahead
-  PATH_TILES = 1,  // 3-16 tokens (and graphs the row-owner path cannot take): stream-K tiles, mma.sync
-  PATH_UMMA = 2,   // 17-64 tokens: stream-K tiles, tcgen05.mma, grouped attention
+  PATH_ROWS = 0,  // 1-2 tokens: row-owner linears, resident token rows, L2 look-ahead
+  PATH_WIDE = 1,  // 3-128 tokens (and graphs the row-owner path cannot take): stream-K tiles, tcgen05.mma
 };
 
 enum Status : int {
@@ -191,10 +192,9 @@ struct KParams {
   int max_step_times;
   int max_iters;      // 0 = unlimited
   unsigned long long timeout_ns;
-  // split-k scratch shared by all linear ops
-  float* partial;         // [groups][grid][2][128*kMaxTokGroup]
-  unsigned* piece_count;  // [groups][max nblk]
-  int piece_stride;       // max nblk
+  // split-k scratch shared by all linear ops of the wide path
+  float* partial;         // [grid][x_rows / 4][128 rows] float4: a CTA's sums of the block that an earlier CTA finishes
+  unsigned* piece_count;  // [max nblk][8 warps]: shares published
   // attention scratch
   float* attn_part;       // [tokens][kv heads][max chunks][qpk*(128+2)]
   unsigned* attn_count;   // [tokens][kv heads]
@@ -216,17 +216,19 @@ struct KParams {
   unsigned long long* prof;
   int trace_op;     // op whose inner phases are stamped: prof[(num_ops + 1) * grid * 4 + cta * 16 + k]; -1 none
   int debug_flags;  // bit 0: linear tasks skip the arithmetic
+  int has_attn;        // (wide path) the program holds attention ops: the token table is filled every iteration
   int prefetch_tiles;  // weight tiles per CTA requested into L2 ahead of the ring (0 = off)
   int has_moe;         // the program holds mixture-of-experts ops: the host launches the build of the kernel that has them
   // shared-memory carve-up (bytes from the 1024-aligned base)
   int num_stages;
   int stage_bytes;  // weights (kStageBytes) + the activation boxes of a wide-batch stage
-  int x_rows;       // token rows of an activation box (0: activations are staged by the consumers)
+  int x_rows;       // token rows of an activation box (wide path: 16, 32, 64 or 128; row-owner path: 0)
   int sums_off;     // per-(row, token) sums of a run of tiles: [128][sums_stride] floats
   int sums_stride;
   int x_off, x_bytes;
   int red_off;
   int bar_off;
+  int desc_off;     // two op descriptors
 };
 
 // Exchange sequence arithmetic (shared with the host-side checks).  Exchange k (1-based) of a launch

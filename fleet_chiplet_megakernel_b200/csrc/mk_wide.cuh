@@ -1,0 +1,905 @@
+// The wide path of the megakernel: iterations of 3 to 128 tokens (batches, prompt chunks).
+//
+// Linears are stream-K tiles on the 5th-generation tensor cores.  Four roles per CTA work side by side:
+//   warp 8   weight producer      TMA boxes of 128 rows x 64 k into the ring (producer_loop)
+//   warp 9   activation producer  the matching boxes of x_rows token rows x 64 k (xproducer_loop)
+//   warp 10  MMA issuer           tcgen05.mma over a stage's boxes, accumulators in tensor memory (mma_loop)
+//   warps 0-7                     finish: accumulators -> split-k exchange -> epilogue (linear_wide)
+// The accumulators are double-buffered, so the MMAs of the next row block run while the finishing warps
+// are still busy with the last one.
+//
+// Included by mk_kernel.cu inside its namespace.
+
+// ------------------------------------------------------------------------------------
+// tcgen05
+// ------------------------------------------------------------------------------------
+__device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr) {
+  // start address >> 4 | leading offset (unused for swizzled K-major) 1 | stride between 8-row
+  // groups 1024 B >> 4 | descriptor version 1 | layout 2 = 128-byte swizzle
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// NC (8, 16 or 32) accumulator columns of this warp's 32 lanes; the caller waits with tmem_wait_ld
+template <int NC>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[NC]) {
+  if constexpr (NC == 8) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+                 : "r"(taddr)
+                 : "memory");
+  } else if constexpr (NC == 16) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr)
+        : "memory");
+  } else {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+        "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
+          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+  }
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
+// This CTA's range of a stream-K linear's tiles (row block major, k minor); false: nothing for it.
+__device__ __forceinline__ bool wide_range(const OpDesc& op, unsigned& total, int& G, unsigned& t0, unsigned& t1) {
+  total = (unsigned)op.nblk * (unsigned)op.nkt;
+  G = (int)min(gridDim.x, total);  // with fewer tiles than CTAs the rest idle
+  if ((int)blockIdx.x >= G) return false;
+  t0 = tile_begin(blockIdx.x, total, G);
+  t1 = tile_begin(blockIdx.x + 1, total, G);
+  return t0 < t1;
+}
+
+// ------------------------------------------------------------------------------------
+// token table of the iteration, in the scratch region behind the reduction words
+// ------------------------------------------------------------------------------------
+// pos[t]: position of token t in its sequence; slot[t]: cache row (page * page size + offset) of that position;
+// kvb[t]: first entry of its request in the page table; grp[g]: query groups of the attention (first token |
+// tokens << 8 | their count in plan[]).
+constexpr int kWideTab = 128;  // the host admits at most 128 batched tokens
+struct WideTab {
+  int pos[kWideTab], slot[kWideTab], kvb[kWideTab], req[kWideTab], grp[kWideTab];
+  int plan[8];
+  int scan[8];
+};
+static_assert(256 + sizeof(WideTab) <= kWideRedBytes, "the token table fits the scratch region");
+__device__ __forceinline__ WideTab& wide_tab(const Ctx& c) { return *reinterpret_cast<WideTab*>(c.smem + c.p.red_off + 256); }
+
+// Filled once per iteration, by all consumers.  Token t of request r (qo_indptr[r] <= t < qo_indptr[r + 1]) sits at
+// position kv_len(r) - (tokens of r behind it) - 1.
+__device__ __noinline__ void wide_fill_tokens(Ctx& c, int T) {
+  const KParams& p = c.p;
+  WideTab& tab = wide_tab(c);
+  T = min(T, kWideTab);
+#pragma unroll 1
+  for (int r = c.tid; r < p.max_reqs; r += kNumConsumers) {
+    const int q0 = __ldcg(p.qo_indptr + r), q1 = min(__ldcg(p.qo_indptr + r + 1), T);
+    if (q1 > q0) {
+      const int first = __ldcg(p.kv_indptr + r), last = __ldcg(p.kv_indptr + r + 1);
+      const int kvlen = (last - first - 1) * p.page_size + __ldcg(p.kv_last_page_len + r);
+      for (int t = q0; t < q1; ++t) {
+        tab.pos[t] = kvlen - (q1 - t);
+        tab.kvb[t] = first;
+        tab.req[t] = r;
+      }
+    }
+  }
+  consumer_sync();
+#pragma unroll 1
+  for (int t = c.tid; t < T; t += kNumConsumers) {
+    const int pos = tab.pos[t];
+    tab.slot[t] = pos >= 0 ? (__ldcg(p.kv_indices + tab.kvb[t] + (pos >> p.page_shift)) << p.page_shift) + (pos & (p.page_size - 1)) : -1;
+  }
+  c.attn_iter = -1;
+  consumer_sync();
+}
+
+// ------------------------------------------------------------------------------------
+// the MMA issuer (one lane of warp 10)
+// ------------------------------------------------------------------------------------
+// Waits for the consumers to publish iteration `iter`; false: the launch ends.
+__device__ __forceinline__ bool wait_go(const Ctx& c, volatile int* fl, int iter, int& go) {
+  unsigned long long t0 = 0;
+  int spins = 0;
+  while (true) {
+    go = fl[0];
+    if (go < 0 || (go >> 8) >= iter) return go >= 0;
+    __nanosleep(40);
+    if (((++spins) & 255) == 0) {
+      if (aborted(c)) return false;
+      const unsigned long long now = globaltimer();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > 4 * c.p.timeout_ns) return false;
+    }
+  }
+}
+
+__device__ __noinline__ void mma_loop(Ctx& c) {
+  const KParams& p = c.p;
+  const int S = p.num_stages, N = p.x_rows;
+  volatile int* fl = c.flags();
+  const uint32_t bar_full0 = c.full_bar(0), bar_empty0 = c.empty_bar(0), bar_x0 = c.xfull_bar(0);
+  const uint32_t x_sub = (uint32_t)N * 128u;  // bytes of one activation box
+  // instruction descriptor: D = f32, A = B = bf16, both K-major, N >> 3, M >> 4
+  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((128u >> 4) << 24);
+  int s = 0;
+  uint32_t parity = 0;
+  unsigned consumed = 0, runs = 0;  // stages multiplied; accumulator runs started
+  bool dead = false;
+  for (int iter = 1; !dead; ++iter) {
+    int go;
+    if (!wait_go(c, fl, iter, go)) break;
+    for (int oi = 0; oi < p.num_ops && !dead; ++oi) {
+      const OpDesc& op = p.ops[oi];
+      if (op.type != OP_LINEAR) continue;
+      unsigned total, t0, t1;
+      int G;
+      if (!wide_range(op, total, G, t0, t1)) continue;
+      const int nkt = op.nkt;
+      int kt = (int)(t0 % (unsigned)nkt);
+      bool fresh = true;
+      for (unsigned tile = t0; tile < t1; ++tile) {
+        const uint32_t d = c.tmem + (runs & 1u) * (uint32_t)N;
+        if (fresh && !mbar_wait(c, c.acc_empty_bar(runs & 1), ((runs >> 1) & 1u) ^ 1u, ST_TIMEOUT_EMPTY)) { dead = true; break; }
+        if (!mbar_wait(c, bar_full0 + 8 * s, parity, ST_TIMEOUT_FULL) || !mbar_wait(c, bar_x0 + 8 * s, parity, ST_TIMEOUT_FULL)) { dead = true; break; }
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t st = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes;
+        const uint32_t xt = st + kStageBytes;
+#pragma unroll
+        for (int sub = 0; sub < kSubTiles; ++sub) {
+          const uint64_t ad = umma_smem_desc(st + (uint32_t)sub * kSubBytes);
+          const uint64_t bd = umma_smem_desc(xt + (uint32_t)sub * x_sub);
+#pragma unroll
+          for (int k16 = 0; k16 < 4; ++k16)  // 16 k-elements = 32 bytes further inside the swizzle span: +2 in the address field
+            umma_bf16(d, ad + (uint64_t)(2 * k16), bd + (uint64_t)(2 * k16), idesc, (fresh && sub == 0 && k16 == 0) ? 0u : 1u);
+        }
+        umma_commit(bar_empty0 + 8 * s);
+        fresh = false;
+        ++consumed;
+        if (++s == S) {
+          s = 0;
+          parity ^= 1u;
+        }
+        if (++kt == nkt || tile + 1 == t1) {  // the run ends: its accumulators belong to the finishing warps
+          umma_commit(c.acc_full_bar(runs & 1));
+          ++runs;
+          fresh = true;
+          kt = 0;
+        }
+      }
+    }
+    if (p.mode == MODE_ONEPASS) break;
+  }
+  // nothing of this thread may be in flight when the tensor memory is given back
+  umma_commit(c.done_bar());
+  mbar_wait(c, c.done_bar(), 0u, ST_TIMEOUT_FULL);
+  fl[5] = (int)consumed;
+}
+
+// ------------------------------------------------------------------------------------
+// finishing a run of tiles
+// ------------------------------------------------------------------------------------
+// Warp w reads accumulator lanes 32 (w & 3) .. + 31 (weight rows of the tile) and one half of the token columns;
+// a thread holds one output row for up to 32 tokens in registers, from tensor memory to the store.
+//
+// When several CTAs hold k-ranges of a row block, the CTA with the block's FIRST k-range finishes it (that range
+// is the tail of its own tile range, so it is computed last anyway).  The others store their sums as float4 of
+// four tokens, [token / 4][row], and every warp publishes its share with a release of its own; the matching warp of
+// the finisher waits for exactly those, fetches all of them in one round of loads and adds them up in CTA order.
+// No CTA-wide sync and no shared memory on the way: with both, at 64 tokens, the slowest CTA of an O projection
+// needed 30 us (5 us of streaming), most of it here.
+__device__ __forceinline__ uint32_t order_bf16(float v) {  // monotone 16-bit key of a bf16 value; 0 only for NaN
+  const uint32_t b = __float_as_uint(v + 0.f) >> 16;       // (-0 counts as +0)
+  const uint32_t k = (b & 0x8000u) ? (~b & 0xffffu) : (b | 0x8000u);
+  return v != v ? 0u : k;
+}
+__device__ __forceinline__ float unorder_bf16(uint32_t k) {
+  const uint32_t b = (k & 0x8000u) ? (k & 0x7fffu) : (~k & 0xffffu);
+  return __uint_as_float(b << 16);
+}
+// running best logit per token of a warp's rows: lane i holds token column c0 + i
+struct WideBest {
+  uint32_t key[2];
+  int idx[2];
+};
+
+// The q/k/v head vector of a token, 8 dims per lane of a half-warp: RMSNorm + RoPE for q and k, then q goes to the
+// attention's scratch rows and k / v to their cache row.  `part`: q head (< qpk), qpk = k, qpk + 1 = v.
+__device__ __forceinline__ void wide_store_head(const Ctx& c, const OpDesc& op, uint4 raw, int tok, int h, int part, bool live, int l16) {
+  const KParams& p = c.p;
+  const int HKV = op.aux0, qpk = op.aux1 / op.aux0;
+  const WideTab& tab = wide_tab(c);
+  uint4 y = raw;
+  if (__any_sync(0xffffffffu, part <= qpk)) {  // (the halves of a warp may hold different parts: the shuffles below want both)
+    const int pos = min(max(tab.pos[tok], 0), op.aux2 - 1);  // aux2 = rows of the cos/sin tables
+    const uint4 w = __ldg(reinterpret_cast<const uint4*>(part < qpk ? op.q_norm_w : op.k_norm_w) + l16);
+    const uint4 cs = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.cos) + (size_t)pos * kHeadDim) + l16);
+    const uint4 sn = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.sin) + (size_t)pos * kHeadDim) + l16);
+    F8 f;
+    unpack8(raw, f.v);
+    f = head_norm_rope(f, w, cs, sn, l16, op.aux3, p.numerics, part < qpk ? op.aux1 < 32 : op.aux0 < 32);
+    if (part <= qpk) y = pack8(f.v);
+  }
+  if (!live) return;
+  if (part < qpk) {
+    reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(op.out2) + (size_t)tok * op.ld_out2 + (size_t)(h * qpk + part) * kHeadDim)[l16] = y;
+  } else {
+    const int slot = tab.slot[tok];
+    if (slot < 0) return;
+    __nv_bfloat16* cache = reinterpret_cast<__nv_bfloat16*>(part == qpk ? op.k_cache : op.v_cache);
+    reinterpret_cast<uint4*>(cache + ((size_t)slot * HKV + h) * kHeadDim)[l16] = y;
+  }
+}
+
+template <int NC>
+__device__ __forceinline__ void wide_epilogue(Ctx& c, const OpDesc& op, int blk, int row, int tok0, int nlive, const float (&v)[NC],
+                                              const uint32_t (&res)[NC / 2], WideBest& best, int cc) {
+  const KParams& p = c.p;
+  const int col = blk * kTileRows + row;
+  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out);
+  if (op.flags & F_SILU_MUL) {
+    // weight rows are units of [4 gate | 4 up]: lanes l and l ^ 4 hold the two halves of four output columns.  Of
+    // every pair of tokens the gate lane finishes the even one, the up lane the odd one.
+    const bool up = (row & 4) != 0;
+    const int ocol = blk * 64 + (row >> 3) * 4 + (row & 3);
+    const bool okc = ocol < (op.n >> 1);
+#pragma unroll
+    for (int i = 0; i < NC; i += 2) {
+      const float mine0 = rbf(v[i]), mine1 = rbf(v[i + 1]);  // the linear output is bf16 before the activation
+      const float other = __shfl_xor_sync(0xffffffffu, up ? mine0 : mine1, 4);
+      const float g = up ? other : mine0, u = up ? mine1 : other;
+      const float y = rbf(__fdividef(g, 1.0f + __expf(-g))) * u;
+      const int t = i + (up ? 1 : 0);
+      if (okc && t < nlive) out[(size_t)(tok0 + t) * op.ld_out + ocol] = __float2bfloat16_rn(y);
+    }
+    return;
+  }
+  if (op.flags & F_QKV_PREP) {
+    // a row block is one head vector of every token: transposed through shared memory (32 token rows per column
+    // half), then a half-warp per token.  The four warps of a half meet on a named barrier of their own.
+    const int half = c.warp >> 2, q = c.warp & 3, l16 = c.lane & 15;
+    const int qpk = op.aux1 / op.aux0;
+    __nv_bfloat16* buf = reinterpret_cast<__nv_bfloat16*>(c.smem + p.x_off) + half * 32 * kHeadDim;
+#pragma unroll
+    for (int i = 0; i < NC; ++i) buf[i * kHeadDim + row] = __float2bfloat16_rn(v[i]);
+    asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
+#pragma unroll 1
+    for (int t = q * 2 + (c.lane >> 4); t < NC; t += 8)
+      wide_store_head(c, op, reinterpret_cast<const uint4*>(buf + t * kHeadDim)[l16], tok0 + (t < nlive ? t : 0), blk / (qpk + 2), blk % (qpk + 2),
+                      t < nlive, l16);
+    asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
+    return;
+  }
+  const bool okc = col < op.n;
+  const bool push = MK_XF(op, F_PUSH) != 0;
+  const bool with_res = (op.flags & F_RESIDUAL) && (!(op.flags & F_RES_RANK0) || p.rank == 0);
+  const bool rnd = p.numerics == NUM_TORCH && !push;  // (pushed partial sums stay fp32: rounded once, after the ranks are added up)
+#pragma unroll
+  for (int i = 0; i < NC; ++i) {
+    float y = v[i];
+    if (with_res) {
+      float r = (i & 1) ? bf_hi(res[i >> 1]) : bf_lo(res[i >> 1]);
+      if (MK_XF(op, F_GATHER_RES) && okc && i < nlive) r = xchg_gather1(c, xchg_cur(c), tok0 + i, col);
+      y = (rnd ? rbf(y) : y) + r;
+    }
+    if (okc && i < nlive) {
+      if (push) xchg_push1(p, xchg_next(c), tok0 + i, col, y);
+      else out[(size_t)(tok0 + i) * op.ld_out + col] = __float2bfloat16_rn(y);
+    }
+  }
+  if (op.flags & F_ARGMAX) {
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      // larger value wins, ties go to the lower index: one 32-bit maximum over the warp's rows
+      const uint32_t k = okc ? (order_bf16(rbf(v[i])) << 16) | (uint32_t)(0xffff - row) : 0u;
+      const uint32_t m = __reduce_max_sync(0xffffffffu, k);
+      if (c.lane == i && (m >> 16) > best.key[cc]) {  // (blocks come in ascending order: an equal value keeps the lower index)
+        best.key[cc] = m >> 16;
+        best.idx[cc] = blk * kTileRows + 0xffff - (int)(m & 0xffffu);
+      }
+    }
+  }
+}
+
+// A finisher's warp waits until the `want` other pieces of its block have published their share (bounded).
+__device__ __forceinline__ void wide_wait_pieces(const Ctx& c, unsigned* cnt, unsigned want, int blk) {
+  if (c.lane == 0) {
+    unsigned long long t0 = 0;
+    unsigned spins = 0;
+    while (ld_acquire_u32(cnt) < want) {
+      if (((++spins) & 1023u) == 0) {
+        if (aborted(c)) break;
+        const unsigned long long now = globaltimer();
+        if (t0 == 0) {
+          t0 = now;
+        } else if (now - t0 > 2 * c.p.timeout_ns) {
+          raise_abort(c, ST_TIMEOUT_PEER, blk, (int)ld_acquire_u32(cnt));
+          break;
+        }
+      }
+    }
+    *cnt = 0u;  // (its next use lies behind a grid barrier)
+  }
+  __syncwarp();
+}
+
+// NC: token columns of a thread per round: x_rows / 2, at most 32 (128 token rows: two rounds)
+template <int NC>
+__device__ __noinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
+  const KParams& p = c.p;
+  const int N = p.x_rows, nkt = op.nkt;
+  const int q = c.warp & 3, half = c.warp >> 2, row = 32 * q + c.lane;
+  const int nround = N > 2 * NC ? 2 : 1;
+  WideBest best;
+  best.key[0] = best.key[1] = 0u;
+  best.idx[0] = best.idx[1] = 0x7fffffff;
+  unsigned total, t0, t1;
+  int G;
+  if (wide_range(op, total, G, t0, t1)) {
+    const bool with_res = (op.flags & F_RESIDUAL) && !MK_XF(op, F_GATHER_RES) && (!(op.flags & F_RES_RANK0) || p.rank == 0);
+    const size_t slot_vec = (size_t)kTileRows * N / 4;  // float4 of a CTA's partial sums
+#pragma unroll 1
+    for (unsigned tile = t0; tile < t1;) {
+      const int blk = (int)(tile / (unsigned)nkt);
+      const unsigned blk0 = (unsigned)blk * (unsigned)nkt, blk1 = blk0 + (unsigned)nkt;
+      const bool finisher = tile == blk0;  // (only the first run of a range can belong to another CTA's block)
+      const int c_last = tile_owner(blk1 - 1, total, G);
+      unsigned* cnt = p.piece_count + (size_t)blk * kNumConsumerWarps + c.warp;
+      const uint32_t acc = c.tmem + (c.acc_runs & 1u) * (uint32_t)N + ((uint32_t)(32 * q) << 16);
+#pragma unroll 1
+      for (int cc = 0; cc < nround; ++cc) {
+        const int col0 = half * (N >> 1) + cc * NC;   // first token column of this thread's round
+        const int nlive = min(NC, T - col0);          // may be negative: nothing but padding
+        // the residual does not depend on the sums: requested first
+        uint32_t res[NC / 2];
+#pragma unroll
+        for (int i = 0; i < NC / 2; ++i) res[i] = 0u;
+        if (with_res && finisher && blk * kTileRows + row < op.n) {
+          const unsigned short* rp = reinterpret_cast<const unsigned short*>(op.res) + (size_t)col0 * op.ld_res + blk * kTileRows + row;
+#pragma unroll
+          for (int i = 0; i < NC / 2; ++i) {
+            uint32_t lo = 0u, hi = 0u;
+            if (2 * i < nlive) lo = __ldcg(rp + (size_t)(2 * i) * op.ld_res);
+            if (2 * i + 1 < nlive) hi = __ldcg(rp + (size_t)(2 * i + 1) * op.ld_res);
+            res[i] = lo | (hi << 16);
+          }
+        }
+        if (cc == 0) {
+          mbar_wait(c, c.acc_full_bar(c.acc_runs & 1), (c.acc_runs >> 1) & 1u, ST_TIMEOUT_FULL);
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        }
+        __syncwarp();
+        uint32_t raw[NC];
+        tmem_ld<NC>(acc + (uint32_t)col0, raw);
+        tmem_wait_ld();
+        if (cc == nround - 1) {  // the accumulators may be overwritten
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (c.lane == 0) mbar_arrive(c.acc_empty_bar(c.acc_runs & 1));
+        }
+        float v[NC];
+#pragma unroll
+        for (int i = 0; i < NC; ++i) v[i] = __uint_as_float(raw[i]);
+        if (!finisher) {
+          float4* mine = reinterpret_cast<float4*>(p.partial) + (size_t)blockIdx.x * slot_vec + (size_t)(col0 >> 2) * kTileRows + row;
+#pragma unroll
+          for (int i = 0; i < NC / 4; ++i)
+            if (4 * i < nlive) mine[(size_t)i * kTileRows] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+          if (cc == nround - 1) {
+            __syncwarp();  // lane 0's release covers what the warp wrote before
+            if (c.lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
+          }
+          continue;
+        }
+        if (c_last > (int)blockIdx.x) {
+          if (cc == 0) wide_wait_pieces(c, cnt, (unsigned)(c_last - (int)blockIdx.x), blk);
+          const float4* src0 = reinterpret_cast<const float4*>(p.partial) + (size_t)(col0 >> 2) * kTileRows + row;
+#pragma unroll 1
+          for (int cta = (int)blockIdx.x + 1; cta <= c_last; ++cta) {
+            const float4* src = src0 + (size_t)cta * slot_vec;
+            float4 w[NC / 4];
+#pragma unroll
+            for (int i = 0; i < NC / 4; ++i) w[i] = 4 * i < nlive ? __ldcg(src + (size_t)i * kTileRows) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int i = 0; i < NC / 4; ++i) {
+              v[4 * i] += w[i].x;
+              v[4 * i + 1] += w[i].y;
+              v[4 * i + 2] += w[i].z;
+              v[4 * i + 3] += w[i].w;
+            }
+          }
+        }
+        wide_epilogue<NC>(c, op, blk, row, col0, nlive, v, res, best, cc);
+      }
+      c.acc_runs += 1;
+      tile = min(blk1, t1);
+    }
+  }
+  if (op.flags & F_ARGMAX) {  // one (max, index) partial per token, CTA and row quarter
+#pragma unroll
+    for (int cc = 0; cc < 2; ++cc) {
+      const int t = half * (N >> 1) + cc * NC + c.lane;
+      if (cc < nround && c.lane < NC && t < T) {
+        const size_t o = (size_t)t * op.amax_n + blockIdx.x * 4 + q;
+        op.amax_val[o] = best.key[cc] != 0u ? unorder_bf16(best.key[cc]) : -INFINITY;
+        op.amax_idx[o] = best.idx[cc];
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ void op_linear_wide(Ctx& c, const OpDesc& op, int T) {
+  if (op_barrier(c, op)) return;
+  c.lin_seq += 1;
+  if (c.tid == 0) c.flags()[4] = (int)c.lin_seq;  // the activation producer may now read this op's input
+  if (c.p.x_rows == 16) linear_wide<8>(c, op, T);
+  else if (c.p.x_rows == 32) linear_wide<16>(c, op, T);
+  else linear_wide<32>(c, op, T);
+  if (MK_XF(op, F_PUSH)) c.ar_seq += 1;  // every CTA counts the exchange, with or without rows of its own
+}
+
+// ------------------------------------------------------------------------------------
+// attention: paged GQA on the warp-level tensor cores
+// ------------------------------------------------------------------------------------
+// When this runs, the new tokens' K/V rows are in the cache and the normalised, rotated q rows in the op's scratch
+// (stored by the QKV linear's epilogue, F_QKV_PREP, or by attn_prepare_rows below).
+//
+// A query group is up to 16 / qpk consecutive tokens of one request: with the q heads of a kv head they fill the 16
+// rows of an mma, so a prompt chunk reads a K/V row once per group instead of once per token (a decoding request is
+// a group of one).  A task is (query group, kv head[, chunk of positions]); W = 1, 2, 4 or 8 warps share a task and
+// take its 16-position tiles in turn:
+//   S = Q K^T   mma.m16n8k16, M = the group's rows, N = 8 positions, K = 128 dims in 8 steps
+//   O += P V    M = the rows, K = 16 positions, N = 128 dims in 16 tiles of 8
+// with the fragments loaded straight from the cache rows, no staging and no ldmatrix: a dot product does not care in
+// which order the dims are walked, so k step s of lane j of a quad stands for dims 32 (s / 2) + 8 j + 4 (s % 2) +
+// {0..3} (the quad reads 64 contiguous bytes of a K row per load), and output column n of tile t stands for dim
+// 64 (t / 8) + 8 n + t % 8 (eight lanes read 128 contiguous bytes of a V row per load; two rows are paired up per
+// register with byte permutes).  P enters as the sum of two bf16 values, so that it keeps 16 bits.
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
+}
+
+struct WideTask {
+  int t0, nt, h, ch, nch;  // first token, tokens, kv head, chunk, chunks
+  int p0, p1, L0, kvb;     // positions [p0, p1) of this chunk; length the first token sees; page-table base
+};
+
+// Query groups, warps per task and chunking of the iteration: the same in every layer, worked out by the first
+// attention op (key: the head geometry).
+__device__ __noinline__ void wide_plan_attention(Ctx& c, const OpDesc& op, int T) {
+  const KParams& p = c.p;
+  WideTab& tab = wide_tab(c);
+  const int HKV = op.aux0, qpk = op.aux1 / op.aux0, tpg = 16 / qpk;
+  T = min(T, kWideTab);
+  // a token opens a group when it is the first of its request or tpg tokens behind the last opening
+  int lmax = 1;
+  bool opens = false;
+  int first = 0, len = 0;
+  if (c.tid < T) {
+    const int r = tab.req[c.tid];
+    first = __ldcg(p.qo_indptr + r);
+    const int q1 = min(__ldcg(p.qo_indptr + r + 1), T);
+    opens = (c.tid - first) % tpg == 0;
+    len = min(tpg, q1 - c.tid);
+    lmax = tab.pos[c.tid] + 1;
+  }
+  const unsigned bal = __ballot_sync(0xffffffffu, opens);
+  const int wmax = __reduce_max_sync(0xffffffffu, lmax);
+  if (c.lane == 0 && c.warp < 4) {
+    tab.scan[c.warp] = __popc(bal);
+    tab.scan[4 + c.warp] = wmax;
+  }
+  consumer_sync();
+  if (opens) {
+    int g = __popc(bal & ((1u << c.lane) - 1u));
+    for (int w = 0; w < c.warp; ++w) g += tab.scan[w];
+    tab.grp[g] = c.tid | (len << 8);
+  }
+  if (c.tid == 0) {
+    const int ng = tab.scan[0] + tab.scan[1] + tab.scan[2] + tab.scan[3];
+    const int L = max(max(tab.scan[4], tab.scan[5]), max(tab.scan[6], tab.scan[7]));
+    const int G = gridDim.x, pairs = ng * HKV, tiles = (L + 15) >> 4;
+    const bool full = tpg > 1 && ng < T;  // some group holds several tokens: up to 16 rows
+    // Warps per task: as many as the grid has for one round of tasks, no more than the longest sequence has tiles.
+    // Groups of several tokens need 4 KB of shared memory for their q rows: at least two warps.
+    int W = full ? 2 : 1;
+    while (W < 8 && pairs * (2 * W) <= G * kNumConsumerWarps && W < tiles) W *= 2;
+    // Few pairs and long sequences: a CTA per chunk of at least 8 tiles, as many chunks as one round of CTAs holds.
+    int nch = 1;
+    if (W == 8) nch = max(1, min(min(G / pairs, tiles / 8), p.attn_max_chunks));
+    const int tpc = (tiles + nch - 1) / nch;  // tiles per chunk
+    nch = (tiles + tpc - 1) / tpc;
+    tab.plan[0] = ng;
+    tab.plan[1] = W;
+    tab.plan[2] = nch;
+    tab.plan[3] = tpc * 16;
+    tab.plan[4] = full ? 1 : 0;
+  }
+  consumer_sync();
+}
+
+// q and k head vectors of the new tokens, where no linear's epilogue has done it: a half-warp per head vector.
+__device__ __noinline__ void attn_prepare_rows(Ctx& c, const OpDesc& op, int T) {
+  const int HKV = op.aux0, qpk = op.aux1 / op.aux0, parts = qpk + 2;
+  const int total = T * HKV * parts, l16 = c.lane & 15;
+#pragma unroll 1
+  for (int i0 = (blockIdx.x * kNumConsumerWarps + c.warp) * 2; i0 < total; i0 += gridDim.x * kNumConsumerWarps * 2) {
+    const int i = min(i0 + (c.lane >> 4), total - 1);
+    const int tok = i / (HKV * parts), e = i % (HKV * parts);
+    const __nv_bfloat16* src = reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)tok * op.ld_in + (size_t)e * kHeadDim;
+    wide_store_head(c, op, __ldcg(reinterpret_cast<const uint4*>(src) + l16), tok, e / parts, e % parts, i0 + (c.lane >> 4) < total, l16);
+  }
+}
+
+// mma of the group's rows; FULL: rows 8..15 are in use, else their accumulators are scratch shared by all tiles
+template <bool FULL>
+__device__ __forceinline__ void wide_mma(float (&d)[FULL ? 4 : 2], float& z0, float& z1, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1) {
+  if constexpr (FULL) {
+    mma_bf16(d, a0, a1, a2, a3, b0, b1);
+  } else {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(z0), "+f"(z1)
+                 : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
+  }
+}
+
+// cache rows of a 16-position tile; positions at or beyond p1 read as zero
+__device__ __forceinline__ int wide_page(const Ctx& c, const WideTask& a, int pos) {
+  return pos < a.p1 ? __ldcg(c.p.kv_indices + a.kvb + (pos >> c.p.page_shift)) : 0;
+}
+__device__ __forceinline__ void wide_load_k(const Ctx& c, const OpDesc& op, const WideTask& a, int pos0, int pg, uint4 (&kr)[2][4]) {
+  const int psh = c.p.page_shift, pmask = c.p.page_size - 1, g = c.lane >> 2, j = c.lane & 3;
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const int pos = pos0 + 8 * u + g;
+    if (psh < 4) pg = wide_page(c, a, pos);  // (pages of 16 positions or more: one page per tile, looked up ahead)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) kr[u][i] = make_uint4(0u, 0u, 0u, 0u);
+    if (pos < a.p1) {
+      const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(op.k_cache) +
+                                                        ((((size_t)pg << psh) + (pos & pmask)) * op.aux0 + a.h) * (kHeadDim * 2)) + j;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) kr[u][i] = __ldcg(src + 4 * i);
+    }
+  }
+}
+__device__ __forceinline__ void wide_load_v(const Ctx& c, const OpDesc& op, const WideTask& a, int pos0, int pg, uint4 (&vr)[4][2]) {
+  const int psh = c.p.page_shift, pmask = c.p.page_size - 1, g = c.lane >> 2, j = c.lane & 3;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int pos = pos0 + 2 * j + (r & 1) + 8 * (r >> 1);
+    if (psh < 4) pg = wide_page(c, a, pos);
+    vr[r][0] = vr[r][1] = make_uint4(0u, 0u, 0u, 0u);
+    if (pos < a.p1) {
+      const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(op.v_cache) +
+                                                        ((((size_t)pg << psh) + (pos & pmask)) * op.aux0 + a.h) * (kHeadDim * 2)) + g;
+      vr[r][0] = __ldcg(src);
+      vr[r][1] = __ldcg(src + 8);
+    }
+  }
+}
+// bf16 pair of two floats and the pair of what rounding left over
+__device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
+  hi = pack2(a, b);
+  lo = pack2(a - bf_lo(hi), b - bf_hi(hi));
+}
+
+// One task by W warps.  `reg`: the group's shared memory (W x 2 KB), `ml`: [warps of the CTA][16] (max, sum) pairs.
+template <bool FULL>
+__device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTask& a, int W, int gi, uint8_t* reg, float2* ml) {
+  constexpr int NR = FULL ? 4 : 2;  // accumulator registers of a tile in use
+  const KParams& p = c.p;
+  const int lane = c.lane, g = lane >> 2, j = lane & 3;
+  const int HKV = op.aux0, qpk = op.aux1 / HKV, rows = a.nt * qpk;
+  const int sub = c.warp & (W - 1), gtid = sub * 32 + lane, nthr = W * 32;
+  const float sc = 1.4426950408889634f * 0.08838834764831845f;  // log2(e) / sqrt(128)
+  const int psh = p.page_shift;
+  const int ntiles = (a.p1 - a.p0 + 15) >> 4;
+  uint4 kr[2][4], vr[4][2];
+  int ti = sub;
+  int pg = 0;
+  if (ti < ntiles && psh >= 4) pg = wide_page(c, a, a.p0 + 16 * ti);
+  // q rows -> shared memory, [row][256 B]; rows past the group's are zero.  64-byte halves trade places in odd rows and
+  // 8-byte halves in rows with bit 1 set: the 8-byte fragment reads of four rows then cover all banks.
+  {
+    const __nv_bfloat16* q0 = reinterpret_cast<const __nv_bfloat16*>(op.out2) + (size_t)a.t0 * op.ld_out2 + (size_t)a.h * qpk * kHeadDim;
+    uint4* sq = reinterpret_cast<uint4*>(reg);
+#pragma unroll 1
+    for (int i = gtid; i < (FULL ? 16 : 8) * 16; i += nthr) {
+      const int r = i >> 4;
+      uint4 v = r < rows ? __ldcg(reinterpret_cast<const uint4*>(q0 + (size_t)(r / qpk) * op.ld_out2 + (r % qpk) * kHeadDim) + (i & 15)) : make_uint4(0, 0, 0, 0);
+      if (r & 2) v = make_uint4(v.z, v.w, v.x, v.y);
+      sq[r * 16 + ((i & 15) ^ ((r & 1) << 2))] = v;
+    }
+  }
+  if (ti < ntiles) {
+    wide_load_k(c, op, a, a.p0 + 16 * ti, pg, kr);
+    wide_load_v(c, op, a, a.p0 + 16 * ti, pg, vr);
+  }
+  int pgn = (psh >= 4 && ti + W < ntiles) ? wide_page(c, a, a.p0 + 16 * (ti + W)) : 0;
+  if (W > 1) asm volatile("bar.sync %0, %1;" ::"r"(2 + gi), "r"(nthr) : "memory");
+  else __syncwarp();
+  const char* sq = reinterpret_cast<const char*>(reg) + g * 256 + 16 * j;
+  const int swz = ((g & 1) << 6) | ((g & 2) << 2);
+  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+  float oacc[16][NR], z0 = 0.f, z1 = 0.f;
+#pragma unroll
+  for (int t = 0; t < 16; ++t)
+#pragma unroll
+    for (int i = 0; i < NR; ++i) oacc[t][i] = 0.f;
+  // length this lane's rows see: row r belongs to token r / qpk of the group
+  const int Lr[2] = {a.L0 + g / qpk, a.L0 + (g + 8) / qpk};
+#pragma unroll 1
+  for (; ti < ntiles; ti += W) {
+    const int pos0 = a.p0 + 16 * ti;
+    const bool more = ti + W < ntiles;
+    float s0[NR], s1[NR];
+#pragma unroll
+    for (int i = 0; i < NR; ++i) s0[i] = s1[i] = 0.f;
+#pragma unroll
+    for (int s = 0; s < 8; ++s) {
+      const char* qs = sq + ((64 * (s >> 1) + 8 * (s & 1)) ^ swz);
+      const uint2 qa = *reinterpret_cast<const uint2*>(qs);
+      uint2 qb = make_uint2(0u, 0u);
+      if constexpr (FULL) qb = *reinterpret_cast<const uint2*>(qs + 8 * 256);
+      const uint4 &k0 = kr[0][s >> 1], &k1 = kr[1][s >> 1];
+      wide_mma<FULL>(s0, z0, z1, qa.x, qb.x, qa.y, qb.y, (s & 1) ? k0.z : k0.x, (s & 1) ? k0.w : k0.y);
+      wide_mma<FULL>(s1, z0, z1, qa.x, qb.x, qa.y, qb.y, (s & 1) ? k1.z : k1.x, (s & 1) ? k1.w : k1.y);
+    }
+    if (more) wide_load_k(c, op, a, pos0 + 16 * W, pgn, kr);  // K of the next tile flies during the rest of this one
+    // rows g (and g + 8), positions pos0 + 2 j + {0, 1} (s0) and pos0 + 8 + 2 j + {0, 1} (s1)
+    uint32_t ph[4] = {0u, 0u, 0u, 0u}, pl[4] = {0u, 0u, 0u, 0u};
+    float alpha[2];
+#pragma unroll
+    for (int u = 0; u < NR / 2; ++u) {
+      float sv[4] = {s0[2 * u], s0[2 * u + 1], s1[2 * u], s1[2 * u + 1]};
+      const int last = min(Lr[u], a.p1);
+      float tmax = -INFINITY;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        sv[i] = pos0 + 2 * j + (i & 1) + 8 * (i >> 1) < last ? sv[i] * sc : -INFINITY;
+        tmax = fmaxf(tmax, sv[i]);
+      }
+      tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
+      tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
+      const float mn = fmaxf(m[u], tmax);
+      const float ms = mn == -INFINITY ? 0.f : mn;  // (a causal row may see nothing of a tile)
+      alpha[u] = exp2f(m[u] - ms);
+      m[u] = mn;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sv[i] = exp2f(sv[i] - ms);
+      l[u] = l[u] * alpha[u] + ((sv[0] + sv[1]) + (sv[2] + sv[3]));  // this lane's share: the quad adds up at the end
+      split2(sv[0], sv[1], ph[u], pl[u]);
+      split2(sv[2], sv[3], ph[2 + u], pl[2 + u]);
+    }
+#pragma unroll
+    for (int t = 0; t < 16; ++t) {
+#pragma unroll
+      for (int i = 0; i < NR; ++i) oacc[t][i] *= alpha[i >> 1];
+      // dim 16 g + t of the four V rows: element t of the lane's 16, two rows per register
+      const uint4 &a0 = vr[0][t >> 3], &a1 = vr[1][t >> 3], &a2 = vr[2][t >> 3], &a3 = vr[3][t >> 3];
+      const int w = (t >> 1) & 3;
+      const uint32_t w0 = w == 0 ? a0.x : (w == 1 ? a0.y : (w == 2 ? a0.z : a0.w));
+      const uint32_t w1 = w == 0 ? a1.x : (w == 1 ? a1.y : (w == 2 ? a1.z : a1.w));
+      const uint32_t w2 = w == 0 ? a2.x : (w == 1 ? a2.y : (w == 2 ? a2.z : a2.w));
+      const uint32_t w3 = w == 0 ? a3.x : (w == 1 ? a3.y : (w == 2 ? a3.z : a3.w));
+      const uint32_t sel = (t & 1) ? 0x7632u : 0x5410u;
+      const uint32_t b0 = prmt(w0, w1, sel), b1 = prmt(w2, w3, sel);
+      wide_mma<FULL>(oacc[t], z0, z1, ph[0], ph[1], ph[2], ph[3], b0, b1);
+      wide_mma<FULL>(oacc[t], z0, z1, pl[0], pl[1], pl[2], pl[3], b0, b1);
+    }
+    if (more) {
+      wide_load_v(c, op, a, pos0 + 16 * W, pgn, vr);
+      if (psh >= 4) pgn = ti + 2 * W < ntiles ? wide_page(c, a, pos0 + 32 * W) : 0;
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < NR / 2; ++u) {
+    l[u] += __shfl_xor_sync(0xffffffffu, l[u], 1);
+    l[u] += __shfl_xor_sync(0xffffffffu, l[u], 2);
+  }
+  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out) + (size_t)a.t0 * op.ld_out + (size_t)a.h * qpk * kHeadDim;
+  if (W == 1 && a.nch == 1) {
+    // this lane holds, per row, dims 64 x + 16 j + {0..7} (oacc[8 x + i][0]) and the eight behind them (oacc[8 x + i][1])
+#pragma unroll
+    for (int u = 0; u < NR / 2; ++u) {
+      const int r = g + 8 * u;
+      if (r < rows) {
+        const float inv = __fdividef(1.0f, l[u]);
+        __nv_bfloat16* dst = out + (size_t)(r / qpk) * op.ld_out + (r % qpk) * kHeadDim + 16 * j;
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+          for (int y = 0; y < 2; ++y) {
+            float f[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) f[i] = oacc[8 * x + i][2 * u + y] * inv;
+            *reinterpret_cast<uint4*>(dst + 64 * x + 8 * y) = pack8(f);
+          }
+      }
+    }
+    __syncwarp();
+    return;
+  }
+  // The warps of the task meet in shared memory, four rows at a time (the slots take the place of the q rows).
+  const uint32_t nbar = (uint32_t)(2 + gi);
+  if (j == 0) {
+#pragma unroll
+    for (int u = 0; u < NR / 2; ++u) ml[c.warp * 16 + g + 8 * u] = make_float2(m[u], l[u]);
+  }
+  float* slot0 = reinterpret_cast<float*>(reg);
+  float* part = p.attn_part + ((size_t)a.t0 * HKV * p.attn_max_chunks * qpk + (size_t)(a.h * p.attn_max_chunks + a.ch) * rows) * (kHeadDim + 2);
+#pragma unroll
+  for (int rb = 0; rb < (FULL ? 4 : 2); ++rb) {
+    if (4 * rb >= rows) break;
+    asm volatile("bar.sync %0, %1;" ::"r"(nbar), "r"(nthr) : "memory");
+    if ((g >> 2) == (rb & 1)) {
+      float* dst = slot0 + (size_t)sub * 4 * kHeadDim + (g & 3) * kHeadDim + 16 * j;
+      const int u = rb >> 1;
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+          for (int i = 0; i < 8; i += 4)
+            *reinterpret_cast<float4*>(dst + 64 * x + 8 * y + i) =
+                make_float4(oacc[8 * x + i][2 * u + y], oacc[8 * x + i + 1][2 * u + y], oacc[8 * x + i + 2][2 * u + y], oacc[8 * x + i + 3][2 * u + y]);
+    }
+    asm volatile("bar.sync %0, %1;" ::"r"(nbar), "r"(nthr) : "memory");
+#pragma unroll 1
+    for (int e = gtid; e < 4 * 32; e += nthr) {  // (row of the round, four dims)
+      const int r = 4 * rb + (e >> 5), d = (e & 31) * 4;
+      if (r >= rows) continue;
+      const float2* mlr = ml + (c.warp - sub) * 16 + r;
+      float M = -INFINITY;
+      for (int w = 0; w < W; ++w) M = fmaxf(M, mlr[w * 16].x);
+      const float Ms = M == -INFINITY ? 0.f : M;
+      float L = 0.f;
+      float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+      for (int w = 0; w < W; ++w) {
+        const float2 v = mlr[w * 16];
+        const float f = exp2f(v.x - Ms);
+        const float4 o4 = *reinterpret_cast<const float4*>(slot0 + (size_t)w * 4 * kHeadDim + (e >> 5) * kHeadDim + d);
+        L = fmaf(f, v.y, L);
+        O.x = fmaf(f, o4.x, O.x);
+        O.y = fmaf(f, o4.y, O.y);
+        O.z = fmaf(f, o4.z, O.z);
+        O.w = fmaf(f, o4.w, O.w);
+      }
+      if (a.nch == 1) {
+        const float inv = __fdividef(1.0f, L);
+        *reinterpret_cast<uint2*>(out + (size_t)(r / qpk) * op.ld_out + (r % qpk) * kHeadDim + d) =
+            make_uint2(pack2(O.x * inv, O.y * inv), pack2(O.z * inv, O.w * inv));
+      } else {
+        *reinterpret_cast<float2*>(part + r * kHeadDim + d) = make_float2(O.x, O.y);
+        *reinterpret_cast<float2*>(part + r * kHeadDim + d + 2) = make_float2(O.z, O.w);
+        if (d == 0) {
+          part[rows * kHeadDim + r] = M;
+          part[rows * kHeadDim + rows + r] = L;
+        }
+      }
+    }
+  }
+  if (a.nch == 1) {
+    asm volatile("bar.sync %0, %1;" ::"r"(nbar), "r"(nthr) : "memory");  // the group's memory is free again
+    return;
+  }
+  // several chunks (then W == 8, the whole CTA): the one that arrives last merges them
+  consumer_sync();  // the CTA's partial is complete; thread 0's release below publishes all of it
+  unsigned* cnt = p.attn_count + (size_t)a.t0 * HKV + a.h;
+  volatile int* fl = c.flags();
+  if (c.tid == 0) {
+    unsigned old;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(cnt) : "memory");
+    fl[2] = (old == (unsigned)(a.nch - 1)) ? 1 : 0;
+  }
+  consumer_sync();
+  if (fl[2] != 0) {
+    const int stride = rows * (kHeadDim + 2);
+    const float* base = part - (size_t)a.ch * stride;
+#pragma unroll 1
+    for (int e = c.tid; e < rows * 64; e += kNumConsumers) {
+      const int r = e >> 6, d = (e & 63) * 2;
+      float M = -INFINITY, L = 0.f;
+      float2 O = make_float2(0.f, 0.f);
+#pragma unroll 1
+      for (int c0 = 0; c0 < a.nch; c0 += 8) {
+        float2 v[8];
+        float mm[8], ll[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const bool ok = c0 + u < a.nch;
+          const float* b = base + (size_t)(ok ? c0 + u : c0) * stride;
+          v[u] = __ldcg(reinterpret_cast<const float2*>(b + r * kHeadDim + d));
+          mm[u] = ok ? __ldcg(b + rows * kHeadDim + r) : -INFINITY;
+          ll[u] = ok ? __ldcg(b + rows * kHeadDim + rows + r) : 0.f;
+        }
+        float Mb = M;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) Mb = fmaxf(Mb, mm[u]);
+        const float Ms = Mb == -INFINITY ? 0.f : Mb;
+        const float f0 = exp2f(M - Ms);
+        O.x *= f0;
+        O.y *= f0;
+        L *= f0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const float f = exp2f(mm[u] - Ms);
+          O.x = fmaf(f, v[u].x, O.x);
+          O.y = fmaf(f, v[u].y, O.y);
+          L = fmaf(f, ll[u], L);
+        }
+        M = Mb;
+      }
+      const float inv = __fdividef(1.0f, L);
+      *reinterpret_cast<uint32_t*>(out + (size_t)(r / qpk) * op.ld_out + (r % qpk) * kHeadDim + d) = pack2(O.x * inv, O.y * inv);
+    }
+    if (c.tid == 0) *cnt = 0u;
+  }
+  consumer_sync();
+}
+
+__device__ __noinline__ void op_attention_wide(Ctx& c, const OpDesc& op, int T) {
+  const KParams& p = c.p;
+  if (op_barrier(c, op)) return;
+  if (p.debug_flags & 2) return;  // measurement aid: the op keeps its barrier and does nothing else
+  const int key = op.aux0 * 256 + op.aux1;
+  if (c.attn_iter != key) {
+    wide_plan_attention(c, op, T);
+    c.attn_iter = key;
+  }
+  if (!(op.flags & F_QKV_READY)) {
+    attn_prepare_rows(c, op, T);
+    grid_sync(c);  // every token's K/V row is in the cache before any is read
+    c.dead = c.flags()[3] != 0;
+    if (c.dead) return;
+  }
+  const WideTab& tab = wide_tab(c);
+  const int HKV = op.aux0;
+  const int W = tab.plan[1], nch = tab.plan[2], CS = tab.plan[3];
+  const bool full = tab.plan[4] != 0;
+  const int ntasks = tab.plan[0] * HKV * nch, per = kNumConsumerWarps / W;
+  const int gi = c.warp / W;
+  uint8_t* reg = c.smem + p.x_off + (size_t)gi * W * 2048;
+  float2* ml = reinterpret_cast<float2*>(c.smem + p.x_off + 16384);
+#pragma unroll 1
+  for (int task = blockIdx.x + gridDim.x * gi; task < ntasks; task += gridDim.x * per) {
+    WideTask a;
+    a.ch = task % nch;
+    const int pr = task / nch;
+    a.h = pr % HKV;
+    const int e = tab.grp[pr / HKV];
+    a.t0 = e & 255;
+    a.nt = e >> 8;
+    a.L0 = tab.pos[a.t0] + 1;
+    a.kvb = tab.kvb[a.t0];
+    const int L = a.L0 + a.nt - 1;
+    a.p0 = a.ch * CS;
+    a.p1 = min(L, a.p0 + CS);
+    a.nch = (L + CS - 1) / CS;
+    if (a.p0 >= L || a.L0 <= 0) continue;  // (uniform within the task's warps)
+    if (full) wide_attend<true>(c, op, a, W, gi, reg, ml);
+    else wide_attend<false>(c, op, a, W, gi, reg, ml);
+  }
+}
