@@ -31,9 +31,11 @@ extern "C" int mk_kernel_init_state(const mk::KParams* p, void* stream);
 
 namespace {
 
-constexpr int kMaxSmem = 232448;  // 227 KB opt-in limit per CTA on sm_100
+constexpr int kParamSmem = 768;  // static shared memory of the kernel: its copy of KParams
+static_assert(sizeof(mk::KParams) <= kParamSmem, "the kernel's parameter copy");
+constexpr int kMaxSmem = 232448 - kParamSmem;  // 227 KB opt-in limit per CTA on sm_100
 constexpr int kRedBytes = 2048;    // small scratch (reductions, argmax, sequence lengths)
-constexpr int kFastSmem = 166912;  // 164 KB carve-out minus the 1 KB the system reserves per CTA
+constexpr int kFastSmem = 166912 - kParamSmem;  // 164 KB carve-out minus the 1 KB the system reserves per CTA
 constexpr int kRowsSumsBytes = mk::kNumConsumerWarps * mk::kChunkRows * 2 * 4;  // [warp][32 rows][2 tokens] floats
 // token rows a row-owner CTA may keep resident beside three 32 KB weight stages
 constexpr int kRowsXBudget = kFastSmem - 2048 - kRedBytes - kRowsSumsBytes - 3 * mk::kStageBytes;
@@ -1351,9 +1353,10 @@ static int compile_program(mk_handle* h, bool first) {
       po.amax_n = std::min(h->grid, (po.n + mk::kUnitRows - 1) / mk::kUnitRows);
       if (i + 1 < h->plan.size() && h->plan[i + 1].type == mk::OP_ARGMAX_REDUCE) h->plan[i + 1].amax_n = po.amax_n;
     }
-    // wide LM head: one partial per CTA and row quarter of its tiles
+    // wide LM head: one partial per CTA that holds tiles and row quarter
     if (po.type == mk::OP_LINEAR && !(po.flags & mk::F_ROWS) && (po.flags & mk::F_ARGMAX)) {
-      po.amax_n = h->grid * 4;
+      const int64_t tiles = (int64_t)((po.n + mk::kTileRows - 1) / mk::kTileRows) * ((po.k + mk::kTileK - 1) / mk::kTileK);
+      po.amax_n = (int)std::min<int64_t>(h->grid, tiles) * 4;
       if (i + 1 < h->plan.size() && h->plan[i + 1].type == mk::OP_ARGMAX_REDUCE) h->plan[i + 1].amax_n = po.amax_n;
     }
   }

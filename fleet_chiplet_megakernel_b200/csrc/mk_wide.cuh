@@ -385,6 +385,7 @@ __device__ __noinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
           mbar_wait(c, c.acc_full_bar(c.acc_runs & 1), (c.acc_runs >> 1) & 1u, ST_TIMEOUT_FULL);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
+        if (tile == t0) MK_STAMP(c, 0);
         __syncwarp();
         uint32_t raw[NC];
         tmem_ld<NC>(acc + (uint32_t)col0, raw);
@@ -406,27 +407,40 @@ __device__ __noinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
             __syncwarp();  // lane 0's release covers what the warp wrote before
             if (c.lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
           }
+          if (tile == t0) MK_STAMP(c, 1);
           continue;
         }
+        MK_STAMP(c, 2);
         if (c_last > (int)blockIdx.x) {
           if (cc == 0) wide_wait_pieces(c, cnt, (unsigned)(c_last - (int)blockIdx.x), blk);
+          MK_STAMP(c, 3);
           const float4* src0 = reinterpret_cast<const float4*>(p.partial) + (size_t)(col0 >> 2) * kTileRows + row;
+          // Several pieces in flight per round (registers allowing): a block of a small layer has up to `nkt` of them, and a
+          // round trip each (0.45 us) was most of its finish (7 of 15 us in a 1024 x 3072 layer).  Added in CTA order all the same.
+          constexpr int PB = NC == 8 ? 8 : (NC == 16 ? 4 : 2);
 #pragma unroll 1
-          for (int cta = (int)blockIdx.x + 1; cta <= c_last; ++cta) {
-            const float4* src = src0 + (size_t)cta * slot_vec;
-            float4 w[NC / 4];
+          for (int cta = (int)blockIdx.x + 1; cta <= c_last; cta += PB) {
+            float4 w[PB][NC / 4];
 #pragma unroll
-            for (int i = 0; i < NC / 4; ++i) w[i] = 4 * i < nlive ? __ldcg(src + (size_t)i * kTileRows) : make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int u = 0; u < PB; ++u)
 #pragma unroll
-            for (int i = 0; i < NC / 4; ++i) {
-              v[4 * i] += w[i].x;
-              v[4 * i + 1] += w[i].y;
-              v[4 * i + 2] += w[i].z;
-              v[4 * i + 3] += w[i].w;
-            }
+              for (int i = 0; i < NC / 4; ++i)
+                w[u][i] = (cta + u <= c_last && 4 * i < nlive) ? __ldcg(src0 + (size_t)(cta + u) * slot_vec + (size_t)i * kTileRows)
+                                                               : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int u = 0; u < PB; ++u)
+#pragma unroll
+              for (int i = 0; i < NC / 4; ++i) {
+                v[4 * i] += w[u][i].x;
+                v[4 * i + 1] += w[u][i].y;
+                v[4 * i + 2] += w[u][i].z;
+                v[4 * i + 3] += w[u][i].w;
+              }
           }
         }
+        MK_STAMP(c, 4);
         wide_epilogue<NC>(c, op, blk, row, col0, nlive, v, res, best, cc);
+        MK_STAMP(c, 5);
       }
       c.acc_runs += 1;
       tile = min(blk1, t1);
@@ -436,7 +450,7 @@ __device__ __noinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
 #pragma unroll
     for (int cc = 0; cc < 2; ++cc) {
       const int t = half * (N >> 1) + cc * NC + c.lane;
-      if (cc < nround && c.lane < NC && t < T) {
+      if (cc < nround && c.lane < NC && t < T && (int)blockIdx.x < G) {
         const size_t o = (size_t)t * op.amax_n + blockIdx.x * 4 + q;
         op.amax_val[o] = best.key[cc] != 0u ? unorder_bf16(best.key[cc]) : -INFINITY;
         op.amax_idx[o] = best.idx[cc];
@@ -550,52 +564,45 @@ __device__ __noinline__ void attn_prepare_rows(Ctx& c, const OpDesc& op, int T) 
   }
 }
 
-// mma of the group's rows; FULL: rows 8..15 are in use, else their accumulators are scratch shared by all tiles
+// mma of the group's rows; FULL: rows 8..15 are in use, else what they give is dropped
 template <bool FULL>
-__device__ __forceinline__ void wide_mma(float (&d)[FULL ? 4 : 2], float& z0, float& z1, uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+__device__ __forceinline__ void wide_mma(float (&d)[FULL ? 4 : 2], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1) {
   if constexpr (FULL) {
     mma_bf16(d, a0, a1, a2, a3, b0, b1);
   } else {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-                 : "+f"(d[0]), "+f"(d[1]), "+f"(z0), "+f"(z1)
-                 : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1));
+    float x0, x1;  // rows 8..15: nothing (shared accumulators in their place would chain every mma to the one before)
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%10,%10};"
+        : "+f"(d[0]), "+f"(d[1]), "=f"(x0), "=f"(x1)
+        : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1), "f"(0.f));
   }
 }
 
-// cache rows of a 16-position tile; positions at or beyond p1 read as zero
+// Cache rows of a 16-position tile.  Positions at or beyond p1 read row p1 - 1 instead: their probabilities are zero.
 __device__ __forceinline__ int wide_page(const Ctx& c, const WideTask& a, int pos) {
-  return pos < a.p1 ? __ldcg(c.p.kv_indices + a.kvb + (pos >> c.p.page_shift)) : 0;
+  return __ldcg(c.p.kv_indices + a.kvb + (min(pos, a.p1 - 1) >> c.p.page_shift));
+}
+// this lane's 16-byte column (vector `col` of the head) of the cache row of position `pos`
+__device__ __forceinline__ const uint4* wide_row(const Ctx& c, const WideTask& a, const void* cache, int HKV, int pos, int pg, int col) {
+  pos = min(pos, a.p1 - 1);
+  if (c.p.page_shift < 4) pg = wide_page(c, a, pos);  // (pages of 16 positions or more: one page per tile, looked up ahead)
+  const int r = (pg << c.p.page_shift) + (pos & (c.p.page_size - 1));
+  return reinterpret_cast<const uint4*>(cache) + ((size_t)r * HKV + a.h) * (kHeadDim / 8) + col;
 }
 __device__ __forceinline__ void wide_load_k(const Ctx& c, const OpDesc& op, const WideTask& a, int pos0, int pg, uint4 (&kr)[2][4]) {
-  const int psh = c.p.page_shift, pmask = c.p.page_size - 1, g = c.lane >> 2, j = c.lane & 3;
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
-    const int pos = pos0 + 8 * u + g;
-    if (psh < 4) pg = wide_page(c, a, pos);  // (pages of 16 positions or more: one page per tile, looked up ahead)
+    const uint4* src = wide_row(c, a, op.k_cache, op.aux0, pos0 + 8 * u + (c.lane >> 2), pg, c.lane & 3);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) kr[u][i] = make_uint4(0u, 0u, 0u, 0u);
-    if (pos < a.p1) {
-      const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(op.k_cache) +
-                                                        ((((size_t)pg << psh) + (pos & pmask)) * op.aux0 + a.h) * (kHeadDim * 2)) + j;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) kr[u][i] = __ldcg(src + 4 * i);
-    }
+    for (int i = 0; i < 4; ++i) kr[u][i] = __ldcg(src + 4 * i);
   }
 }
 __device__ __forceinline__ void wide_load_v(const Ctx& c, const OpDesc& op, const WideTask& a, int pos0, int pg, uint4 (&vr)[4][2]) {
-  const int psh = c.p.page_shift, pmask = c.p.page_size - 1, g = c.lane >> 2, j = c.lane & 3;
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    const int pos = pos0 + 2 * j + (r & 1) + 8 * (r >> 1);
-    if (psh < 4) pg = wide_page(c, a, pos);
-    vr[r][0] = vr[r][1] = make_uint4(0u, 0u, 0u, 0u);
-    if (pos < a.p1) {
-      const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const char*>(op.v_cache) +
-                                                        ((((size_t)pg << psh) + (pos & pmask)) * op.aux0 + a.h) * (kHeadDim * 2)) + g;
-      vr[r][0] = __ldcg(src);
-      vr[r][1] = __ldcg(src + 8);
-    }
+    const uint4* src = wide_row(c, a, op.v_cache, op.aux0, pos0 + 2 * (c.lane & 3) + (r & 1) + 8 * (r >> 1), pg, c.lane >> 2);
+    vr[r][0] = __ldcg(src);
+    vr[r][1] = __ldcg(src + 8);
   }
 }
 // bf16 pair of two floats and the pair of what rounding left over
@@ -620,29 +627,39 @@ __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTas
   int pg = 0;
   if (ti < ntiles && psh >= 4) pg = wide_page(c, a, a.p0 + 16 * ti);
   // q rows -> shared memory, [row][256 B]; rows past the group's are zero.  64-byte halves trade places in odd rows and
-  // 8-byte halves in rows with bit 1 set: the 8-byte fragment reads of four rows then cover all banks.
+  // 8-byte halves in rows with bit 1 set: the 8-byte fragment reads of four rows then cover all banks.  All loads of a
+  // thread (at most four), then the first K and V rows, then the stores: one round trip instead of one per row (with
+  // the clamped row loads, the op's start took 5.4 us instead of 7.7 at eight requests of 300 tokens).
   {
+    constexpr int NQ = (FULL ? 16 : 8) * 16;
+    const int qsh = 31 - __clz(qpk);  // (1, 2, 4 or 8 q heads per kv head)
     const __nv_bfloat16* q0 = reinterpret_cast<const __nv_bfloat16*>(op.out2) + (size_t)a.t0 * op.ld_out2 + (size_t)a.h * qpk * kHeadDim;
     uint4* sq = reinterpret_cast<uint4*>(reg);
-#pragma unroll 1
-    for (int i = gtid; i < (FULL ? 16 : 8) * 16; i += nthr) {
-      const int r = i >> 4;
-      uint4 v = r < rows ? __ldcg(reinterpret_cast<const uint4*>(q0 + (size_t)(r / qpk) * op.ld_out2 + (r % qpk) * kHeadDim) + (i & 15)) : make_uint4(0, 0, 0, 0);
-      if (r & 2) v = make_uint4(v.z, v.w, v.x, v.y);
-      sq[r * 16 + ((i & 15) ^ ((r & 1) << 2))] = v;
+    uint4 qv[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const int i = gtid + x * nthr, r = i >> 4;
+      qv[x] = make_uint4(0, 0, 0, 0);
+      if (i < NQ && r < rows) qv[x] = __ldcg(reinterpret_cast<const uint4*>(q0 + (size_t)(r >> qsh) * op.ld_out2 + (r & (qpk - 1)) * kHeadDim) + (i & 15));
     }
-  }
-  if (ti < ntiles) {
-    wide_load_k(c, op, a, a.p0 + 16 * ti, pg, kr);
-    wide_load_v(c, op, a, a.p0 + 16 * ti, pg, vr);
+    if (ti < ntiles) {
+      wide_load_k(c, op, a, a.p0 + 16 * ti, pg, kr);
+      wide_load_v(c, op, a, a.p0 + 16 * ti, pg, vr);
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const int i = gtid + x * nthr, r = i >> 4;
+      if (i < NQ) sq[r * 16 + ((i & 15) ^ ((r & 1) << 2))] = (r & 2) ? make_uint4(qv[x].z, qv[x].w, qv[x].x, qv[x].y) : qv[x];
+    }
   }
   int pgn = (psh >= 4 && ti + W < ntiles) ? wide_page(c, a, a.p0 + 16 * (ti + W)) : 0;
   if (W > 1) asm volatile("bar.sync %0, %1;" ::"r"(2 + gi), "r"(nthr) : "memory");
   else __syncwarp();
+  MK_STAMP(c, 1);
   const char* sq = reinterpret_cast<const char*>(reg) + g * 256 + 16 * j;
   const int swz = ((g & 1) << 6) | ((g & 2) << 2);
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
-  float oacc[16][NR], z0 = 0.f, z1 = 0.f;
+  float oacc[16][NR];
 #pragma unroll
   for (int t = 0; t < 16; ++t)
 #pragma unroll
@@ -663,8 +680,8 @@ __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTas
       uint2 qb = make_uint2(0u, 0u);
       if constexpr (FULL) qb = *reinterpret_cast<const uint2*>(qs + 8 * 256);
       const uint4 &k0 = kr[0][s >> 1], &k1 = kr[1][s >> 1];
-      wide_mma<FULL>(s0, z0, z1, qa.x, qb.x, qa.y, qb.y, (s & 1) ? k0.z : k0.x, (s & 1) ? k0.w : k0.y);
-      wide_mma<FULL>(s1, z0, z1, qa.x, qb.x, qa.y, qb.y, (s & 1) ? k1.z : k1.x, (s & 1) ? k1.w : k1.y);
+      wide_mma<FULL>(s0, qa.x, qb.x, qa.y, qb.y, (s & 1) ? k0.z : k0.x, (s & 1) ? k0.w : k0.y);
+      wide_mma<FULL>(s1, qa.x, qb.x, qa.y, qb.y, (s & 1) ? k1.z : k1.x, (s & 1) ? k1.w : k1.y);
     }
     if (more) wide_load_k(c, op, a, pos0 + 16 * W, pgn, kr);  // K of the next tile flies during the rest of this one
     // rows g (and g + 8), positions pos0 + 2 j + {0, 1} (s0) and pos0 + 8 + 2 j + {0, 1} (s1)
@@ -705,8 +722,8 @@ __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTas
       const uint32_t w3 = w == 0 ? a3.x : (w == 1 ? a3.y : (w == 2 ? a3.z : a3.w));
       const uint32_t sel = (t & 1) ? 0x7632u : 0x5410u;
       const uint32_t b0 = prmt(w0, w1, sel), b1 = prmt(w2, w3, sel);
-      wide_mma<FULL>(oacc[t], z0, z1, ph[0], ph[1], ph[2], ph[3], b0, b1);
-      wide_mma<FULL>(oacc[t], z0, z1, pl[0], pl[1], pl[2], pl[3], b0, b1);
+      wide_mma<FULL>(oacc[t], ph[0], ph[1], ph[2], ph[3], b0, b1);
+      wide_mma<FULL>(oacc[t], pl[0], pl[1], pl[2], pl[3], b0, b1);
     }
     if (more) {
       wide_load_v(c, op, a, pos0 + 16 * W, pgn, vr);
@@ -718,6 +735,7 @@ __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTas
     l[u] += __shfl_xor_sync(0xffffffffu, l[u], 1);
     l[u] += __shfl_xor_sync(0xffffffffu, l[u], 2);
   }
+  MK_STAMP(c, 2);
   __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out) + (size_t)a.t0 * op.ld_out + (size_t)a.h * qpk * kHeadDim;
   if (W == 1 && a.nch == 1) {
     // this lane holds, per row, dims 64 x + 16 j + {0..7} (oacc[8 x + i][0]) and the eight behind them (oacc[8 x + i][1])
@@ -801,6 +819,7 @@ __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTas
       }
     }
   }
+  MK_STAMP(c, 3);
   if (a.nch == 1) {
     asm volatile("bar.sync %0, %1;" ::"r"(nbar), "r"(nthr) : "memory");  // the group's memory is free again
     return;
@@ -875,6 +894,7 @@ __device__ __noinline__ void op_attention_wide(Ctx& c, const OpDesc& op, int T) 
     c.dead = c.flags()[3] != 0;
     if (c.dead) return;
   }
+  MK_STAMP(c, 0);
   const WideTab& tab = wide_tab(c);
   const int HKV = op.aux0;
   const int W = tab.plan[1], nch = tab.plan[2], CS = tab.plan[3];
