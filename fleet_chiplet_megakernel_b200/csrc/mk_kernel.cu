@@ -96,6 +96,12 @@ __device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const void* tmap,
       ::"r"(dst), "l"(tmap), "r"(bar), "r"(x), "r"(y), "l"(pol)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_3d_hint(uint32_t dst, const void* tmap, uint32_t bar, int x, int y, int z, uint64_t pol) {
+  asm volatile(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5}], [%2], %6;" ::"r"(dst),
+      "l"(tmap), "r"(bar), "r"(x), "r"(y), "r"(z), "l"(pol)
+      : "memory");
+}
 __device__ __forceinline__ void tma_prefetch_2d(const void* tmap, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(tmap), "r"(x), "r"(y) : "memory");
 }
@@ -1044,6 +1050,10 @@ __device__ __noinline__ void linear_pass_rows(Ctx& c, const OpDesc& op, int tok0
   const int nks = op.nkt;
   const int kp = nks * kRowsStageK;
   const int ntok = min(op.aux3, T - tok0);
+  int row0, row1;
+  bool any;
+  rows_range(op, row0, row1, any);
+  if (!any) return;  // (nor may it poll for tagged words that no output of its own protects from being overwritten)
   MK_STAMP(c, 0);
   if (op.flags & F_LL_IN) {
     if (op.flags & F_NORM_IN) stage_x_ll(c, op.ll_in, op.ld_in, op.k, kp, op.norm_w, tok0, ntok, T, pre_w, ll_tag_of(c, op.ll_in_op));
@@ -1052,10 +1062,6 @@ __device__ __noinline__ void linear_pass_rows(Ctx& c, const OpDesc& op, int tok0
   else stage_x(c, op.in, op.ld_in, op.k, kp, (op.flags & F_NORM_IN) ? op.norm_w : nullptr, tok0, ntok, T, pre_w,
                MK_XF(op, F_GATHER_IN) != 0);
   MK_STAMP(c, 1);
-  int row0, row1;
-  bool any;
-  rows_range(op, row0, row1, any);
-  if (!any) return;
   const int S = p.num_stages;
   const int lane = c.lane, warp = c.warp;
   const bool arith = !(p.debug_flags & 1);
@@ -2190,54 +2196,95 @@ __device__ void op_argmax_reduce(Ctx& c, const OpDesc& op, int T) {
 // routing tables [T, top-k] (fp32 weight, expert id).  One warp per token: fp32 softmax over the experts,
 // k rounds of (largest probability, lowest index), weights renormalised over the k picked
 // (transformers' Qwen3MoeTopKRouter with norm_topk_prob; reference task: topk_softmax_sm100.cuh:61-290).
-// One token, by one warp: `w_out` / `idx_out` (may be null) receive the k weights and expert ids.
-__device__ __noinline__ void moe_route_token(Ctx& c, const __nv_bfloat16* logits, int E, int K, float* w_out, int* idx_out, int* idx_out2) {
-  float v[8];  // up to 256 experts: 8 per lane
+// One token, by one warp: `w_out` / `idx_out` and `w_out2` / `idx_out2` (may be null) receive the k weights and expert
+// ids.  `words` not null: the logits arrive as tagged words.  A round is two warp-wide integer reductions (a
+// probability's bits grow with it), not five levels of shuffles of (value, index).
+__device__ __noinline__ void moe_route_token(Ctx& c, const __nv_bfloat16* logits, const uint2* words, unsigned tag, int E, int K, float* w_out,
+                                             int* idx_out, float* w_out2, int* idx_out2) {
+  float v[8];  // up to 256 experts, 8 per lane: v[i] is expert 2 * (lane + 32 * (i / 2)) + i % 2
+  if (words != nullptr) {
+    unsigned long long t0 = 0;
+    unsigned spins = 0;
+    uint2 q[4];
+    while (true) {
+      bool here = true;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        q[j] = make_uint2(0u, tag);
+        if (2 * (c.lane + 32 * j) < E) q[j] = ld_gpu_v2(words + c.lane + 32 * j);
+        here = here && q[j].y == tag;
+      }
+      if (here) break;
+      if (((++spins) & 63u) == 0) {
+        if (aborted(c)) break;
+        const unsigned long long now = globaltimer();
+        if (t0 == 0) {
+          t0 = now;
+        } else if (now - t0 > 2 * c.p.timeout_ns) {
+          raise_abort(c, ST_TIMEOUT_DATA, (int)tag, (int)q[0].y);
+          break;
+        }
+      }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = (i & 1) ? bf_hi(q[i >> 1].x) : bf_lo(q[i >> 1].x);
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int e = 2 * (c.lane + 32 * (i >> 1)) + (i & 1);
+      v[i] = e < E ? __bfloat162float(__ldcg(logits + e)) : 0.f;
+    }
+  }
   float mx = -INFINITY;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int e = c.lane + 32 * i;
-    v[i] = e < E ? __bfloat162float(__ldcg(logits + e)) : -INFINITY;
-    mx = fmaxf(mx, v[i]);
-  }
+  for (int i = 0; i < 8; ++i)
+    if (2 * (c.lane + 32 * (i >> 1)) + (i & 1) < E) mx = fmaxf(mx, v[i]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   float sum = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    v[i] = (c.lane + 32 * i) < E ? expf(v[i] - mx) : 0.f;
+    v[i] = 2 * (c.lane + 32 * (i >> 1)) + (i & 1) < E ? expf(v[i] - mx) : 0.f;
     sum += v[i];
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   const float inv = 1.0f / sum;
+  uint32_t key[8];  // bits of the probability + 1; 0: not an expert, taken, or not a number
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float pr = v[i] * inv;
+    key[i] = (2 * (c.lane + 32 * (i >> 1)) + (i & 1) < E && pr >= 0.f) ? __float_as_uint(pr) + 1u : 0u;
+  }
   float picked_sum = 0.f, my_w = 0.f;
   int my_e = 0;
 #pragma unroll 1
   for (int k = 0; k < K; ++k) {
-    ArgBest b;
-    b.v = -INFINITY;
-    b.i = 0x7fffffff;
+    uint32_t best = 0u;
+    int bi = 0x7fffffff;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      ArgBest x;
-      x.v = v[i] * inv;
-      x.i = c.lane + 32 * i;
-      if (x.i < E && v[i] >= 0.f) b = arg_better(b, x);
-    }
-    b = warp_argmax(b);
-    picked_sum += b.v;
+    for (int i = 0; i < 8; ++i)
+      if (key[i] > best) {  // (a lane's experts come in ascending order: the first of equals is the lowest)
+        best = key[i];
+        bi = 2 * (c.lane + 32 * (i >> 1)) + (i & 1);
+      }
+    const uint32_t m = __reduce_max_sync(0xffffffffu, best);
+    const int e = __reduce_min_sync(0xffffffffu, best == m && m != 0u ? bi : 0x7fffffff);
+    const float pv = m != 0u ? __uint_as_float(m - 1u) : -INFINITY;
+    picked_sum += pv;
     if (c.lane == k) {
-      my_w = b.v;
-      my_e = b.i;
+      my_w = pv;
+      my_e = e;
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      if (c.lane + 32 * i == b.i) v[i] = -1.f;  // taken
+      if (2 * (c.lane + 32 * (i >> 1)) + (i & 1) == e) key[i] = 0u;  // taken
   }
   if (c.lane < K) {
     if (w_out != nullptr) w_out[c.lane] = my_w / picked_sum;
     if (idx_out != nullptr) idx_out[c.lane] = my_e;
+    if (w_out2 != nullptr) w_out2[c.lane] = my_w / picked_sum;
     if (idx_out2 != nullptr) idx_out2[c.lane] = my_e;
   }
 }
@@ -2246,7 +2293,7 @@ __device__ __noinline__ void op_moe_route(Ctx& c, const OpDesc& op, int T) {
   const __nv_bfloat16* in = reinterpret_cast<const __nv_bfloat16*>(op.in);
 #pragma unroll 1
   for (int t = blockIdx.x * kNumConsumerWarps + c.warp; t < T; t += gridDim.x * kNumConsumerWarps)
-    moe_route_token(c, in + (size_t)t * op.ld_in, E, K, op.amax_val + (size_t)t * K, op.amax_idx + (size_t)t * K, nullptr);
+    moe_route_token(c, in + (size_t)t * op.ld_in, nullptr, 0u, E, K, op.amax_val + (size_t)t * K, op.amax_idx + (size_t)t * K, nullptr, nullptr);
 }
 
 // The CTA's share of the virtual row space of a MoE linear and its walk: pairs x n rows, contiguous ranges
@@ -2267,46 +2314,104 @@ __device__ __forceinline__ MoeWalk moe_walk(const OpDesc& op, int pairs) {
   return w;
 }
 
+// This CTA's copy of the routing, behind the staged rows: expert ids [T, top-k], then the weights (at most 64 each).
+__device__ __forceinline__ int* moe_route_ids(const Ctx& c) { return reinterpret_cast<int*>(c.smem + c.p.x_off + c.p.x_bytes - 512); }
+__device__ __forceinline__ float* moe_route_weights(const Ctx& c) { return reinterpret_cast<float*>(moe_route_ids(c) + 64); }
+
+// `rows` tagged rows of K columns -> shared memory rows of pitch kp + 8, zero padded, by all consumers: four 8-column
+// pieces of a thread in flight, then whatever has not arrived is polled.
+__device__ __noinline__ void stage_ll_pairs(Ctx& c, const uint2* base, int ld, int rows, int K, int kp, unsigned tag) {
+  uint4* xs = reinterpret_cast<uint4*>(c.smem + c.p.x_off);
+  const int pitch = (kp >> 3) + 1, nvec = kp >> 3, kvec = K >> 3, total = rows * nvec;
+  if (c.tid == 0) xs[rows * pitch] = make_uint4(0, 0, 0, 0);  // the chunk absent columns of the mma point at
+#pragma unroll 1
+  for (int i0 = c.tid; i0 < total; i0 += 4 * kNumConsumers) {
+    uint4 qa[4], qb[4];
+    const uint4* src[4];
+    int dst[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * kNumConsumers, r = i / nvec, v = i - r * nvec;
+      const bool ok = i < total && v < kvec;
+      dst[u] = i < total ? r * pitch + v : -1;
+      src[u] = ok ? reinterpret_cast<const uint4*>(base + (size_t)r * (size_t)(ld >> 1)) + 2 * v : nullptr;
+      qa[u] = ok ? ld_gpu_v4(src[u]) : make_uint4(0, 0, 0, 0);
+      qb[u] = ok ? ld_gpu_v4(src[u] + 1) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (dst[u] >= 0) xs[dst[u]] = src[u] != nullptr ? ll_take8(c, src[u], qa[u], qb[u], tag) : make_uint4(0, 0, 0, 0);
+  }
+  consumer_sync();
+}
+
 __device__ __noinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, int T);
 
 // aux0 = top-k, aux1 = experts, n = rows per expert, k = K.  w: [experts * n, K] bf16 (tmap_w: the four maps of
 // the row-owner path over that 2-D view).  in: [T, K] (one row per token) or, with F_MOE_PAIR_IN, [T * top-k, K];
 // out: [T * top-k, n].  amax_idx: the routing table.
+// F_SILU_MUL (gate/up): n = 2 * inter, and a chunk of R virtual rows holds R / 2 gate rows and the R / 2 up rows that
+// belong to them (tmap_w: maps over [2 * experts, inter, K], one box fetches both halves), so the epilogue also has
+// SiLU(gate) * up -> out2 [T * top-k, inter]; the activation layer behind it has nothing left to do.
+// F_LL_IN (gate/up): no barrier.  The rows (ll_in) and the router logits (ll_res) arrive as tagged words; the rows are
+// staged and normalised while the router linear is still at work.
 __device__ __noinline__ void op_moe_linear(Ctx& c, const OpDesc& op, int T) {
   const KParams& p = c.p;
-  if (op_barrier(c, op)) return;
-  const int topk = op.aux0;
-  if (op.flags & F_MOE_ROUTE) {
-    // The routing folded into this op: warp t of EVERY CTA routes token t from the router logits (one or two
-    // tokens) and leaves the expert ids in shared memory for this CTA's producer; CTA 0 also stores the
-    // runtime's tables, which the later ops of the layer read behind their barriers.
-    int* rt = reinterpret_cast<int*>(c.smem + p.x_off + p.x_bytes - 512);
-    if (c.warp < T)
-      moe_route_token(c, reinterpret_cast<const __nv_bfloat16*>(op.res) + (size_t)c.warp * op.ld_res, op.aux1, topk,
-                      blockIdx.x == 0 ? op.amax_val + (size_t)c.warp * topk : nullptr,
-                      blockIdx.x == 0 ? op.amax_idx + (size_t)c.warp * topk : nullptr, rt + c.warp * topk);
-    consumer_sync();
-    __threadfence_block();
+  const bool ll = (op.flags & F_LL_IN) != 0;
+  if (ll) {  // (no look at the abort flag either: the polls and the stage waits watch it)
+    if (c.pr != nullptr && c.tid == 0) c.pr[1] = globaltimer();
+  } else if (op_barrier(c, op)) {
+    return;
   }
-  c.lin_seq += 1;
-  if (c.tid == 0) c.flags()[4] = (int)c.lin_seq;  // the routing is visible: the producer may pick this op's expert rows
+  const int topk = op.aux0;
   if (op.flags & F_MOE_COMBINE) {
+    c.lin_seq += 1;
+    if (c.tid == 0) c.flags()[4] = (int)c.lin_seq;  // the routing is visible: the producer may pick this op's expert rows
     op_moe_down_combine(c, op, T);
     return;
   }
   const int pairs = T * topk;
   const MoeWalk wk = moe_walk(op, pairs);
-  if (!wk.any || wk.row0 >= wk.row1) return;
+  const bool work = wk.any && wk.row0 < wk.row1;  // (always, with F_LL_IN: the host sees to it)
   const int nks = op.nkt;
   const int kp = nks * kRowsStageK;
-  const bool pair_in = (op.flags & F_MOE_PAIR_IN) != 0;
-  const int p_first = wk.row0 / wk.n, p_last = (wk.row1 - 1) / wk.n;
+  const bool pair_in = (op.flags & F_MOE_PAIR_IN) != 0, silu = (op.flags & F_SILU_MUL) != 0;
+  const int p_first = work ? wk.row0 / wk.n : 0, p_last = work ? (wk.row1 - 1) / wk.n : 0;
   // input rows this CTA needs: those of its pairs (the down projection) or of their tokens
   const int in_first = pair_in ? p_first : p_first / topk;
   const int in_last = pair_in ? p_last : p_last / topk;
   const int nrows = in_last - in_first + 1;  // at most 8 (the host admits MoE graphs for one or two tokens)
-  stage_x(c, reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)in_first * op.ld_in, op.ld_in, op.k, kp,
-          (op.flags & F_NORM_IN) ? op.norm_w : nullptr, 0, nrows, nrows, nullptr);
+  if (ll) {
+    // the norm weights do not depend on other CTAs: requested before the rows are awaited
+    uint4 pre_w[4];
+    const int wpr = stage_warps_per_row(nrows);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int v = (c.warp % wpr) * 32 + c.lane + 32 * wpr * i;
+      pre_w[i] = v < (op.k >> 3) ? __ldg(reinterpret_cast<const uint4*>(op.norm_w) + v) : make_uint4(0, 0, 0, 0);
+    }
+    stage_x_ll(c, op.ll_in, op.ld_in, op.k, kp, op.norm_w, in_first, nrows, T, pre_w, ll_tag_of(c, op.ll_in_op));
+  }
+  if (op.flags & F_MOE_ROUTE) {
+    // The routing folded into this op: warp t of EVERY CTA routes token t from the router logits (one or two
+    // tokens) and leaves the expert ids and weights in shared memory, for this CTA's producer and for the down
+    // projection; without F_LL_IN CTA 0 also stores the runtime's tables, which the later ops of the layer read
+    // behind their barriers.
+    const bool table = !ll && blockIdx.x == 0;
+    if (c.warp < T)
+      moe_route_token(c, reinterpret_cast<const __nv_bfloat16*>(op.res) + (size_t)c.warp * op.ld_res,
+                      ll ? ll_row(op.ll_res, op.ld_res, c.warp) : nullptr, ll ? ll_tag_of(c, op.ll_res_op) : 0u, op.aux1, topk,
+                      table ? op.amax_val + (size_t)c.warp * topk : nullptr, table ? op.amax_idx + (size_t)c.warp * topk : nullptr,
+                      moe_route_weights(c) + c.warp * topk, moe_route_ids(c) + c.warp * topk);
+    consumer_sync();
+    __threadfence_block();
+  }
+  c.lin_seq += 1;
+  if (c.tid == 0) c.flags()[4] = (int)c.lin_seq;  // the routing is visible: the producer may pick this op's expert rows
+  if (!work) return;
+  if (!ll)
+    stage_x(c, reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)in_first * op.ld_in, op.ld_in, op.k, kp,
+            (op.flags & F_NORM_IN) ? op.norm_w : nullptr, 0, nrows, nrows, nullptr);
   const int S = p.num_stages;
   const int lane = c.lane, warp = c.warp;
   const int pitch_b = (kp + 8) * 2;
@@ -2322,6 +2427,7 @@ __device__ __noinline__ void op_moe_linear(Ctx& c, const OpDesc& op, int T) {
   const int e_row = c.tid & 31;
   int s = (int)(c.cons_idx % (unsigned)S);
   uint32_t parity = (c.cons_idx / (unsigned)S) & 1u;
+  int half = 0;
   unsigned consumed = 0;
 #pragma unroll 1
   for (int pr = p_first; pr <= p_last; ++pr) {
@@ -2367,23 +2473,42 @@ __device__ __noinline__ void op_moe_linear(Ctx& c, const OpDesc& op, int T) {
           parity ^= 1u;
         }
       }
-      // column 0 of the accumulators (lanes with (lane & 3) == 0): rows 16t + (lane >> 2) and + 8
+      // column 0 of the accumulators (lanes with (lane & 3) == 0): rows 16t + (lane >> 2) and + 8.  Consecutive chunks
+      // take turns in the two token slots of the sums block: one CTA-wide sync per chunk.
+      half ^= 1;
       if ((lane & 3) == 0) {
 #pragma unroll
         for (int t = 0; t < 2; ++t) {
-          float* d = sums + ((warp * kChunkRows + 16 * t + (lane >> 2)) * TP);
+          float* d = sums + ((warp * kChunkRows + 16 * t + (lane >> 2)) * TP) + half;
           d[0] = acc[2 * t][0] + acc[2 * t + 1][0];
           d[8 * TP] = acc[2 * t][2] + acc[2 * t + 1][2];
         }
       }
       consumer_sync();
-      if (c.tid < 32 && e_row < R) {
+      if (c.warp == 0) {
         float v = 0.f;
+        if (e_row < R) {
 #pragma unroll
-        for (int w = 0; w < kNumConsumerWarps; ++w) v += sums[(w * kChunkRows + e_row) * TP];
-        out[(size_t)pr * op.ld_out + (r0 - pr * wk.n) + e_row] = __float2bfloat16_rn(v);
+          for (int w = 0; w < kNumConsumerWarps; ++w) v += sums[(w * kChunkRows + e_row) * TP + half];
+        }
+        const int rp = r0 - pr * wk.n;  // the chunk's first row within the pair
+        if (silu) {
+          const int h2 = R >> 1, inter = wk.n >> 1;
+          const float g = rbf(v), u = rbf(__shfl_sync(0xffffffffu, v, (e_row + h2) & 31));
+          const int col = (rp >> 1) + (e_row < h2 ? e_row : e_row - h2);
+          if (e_row < R) out[(size_t)pr * op.ld_out + (e_row < h2 ? 0 : inter) + col] = __float2bfloat16_rn(v);
+          const __nv_bfloat16 y = __float2bfloat16_rn(rbf(g / (1.0f + expf(-g))) * u);
+          const uint32_t lo = (uint32_t)__bfloat16_as_ushort(y), hi = __shfl_down_sync(0xffffffffu, lo, 1);
+          if (e_row < h2) {
+            reinterpret_cast<__nv_bfloat16*>(op.out2)[(size_t)pr * op.ld_out2 + col] = y;
+            if ((op.flags & F_LL_OUT) && !(e_row & 1))  // (columns come in groups of four: the pair sits in two neighbouring lanes)
+              st_gpu_v2(reinterpret_cast<uint2*>(op.ll_out) + (size_t)pr * (size_t)(op.ld_out2 >> 1) + (col >> 1), lo | (hi << 16),
+                        ll_tag_of(c, c.cur_op));
+          }
+        } else if (e_row < R) {
+          out[(size_t)pr * op.ld_out + rp + e_row] = __float2bfloat16_rn(v);
+        }
       }
-      consumer_sync();
     }
   }
   c.cons_idx += consumed;
@@ -2416,6 +2541,7 @@ __device__ __noinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, int T
   const int TP = p.sums_stride;  // 2
   float* sums = c.sums();
   const bool torch_num = p.numerics == NUM_TORCH;
+  const bool ll = (op.flags & F_LL_IN) != 0;  // the slots' rows as tagged words, the routing from this CTA's shared memory
   const __nv_bfloat16* res = reinterpret_cast<const __nv_bfloat16*>(op.res);
   __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out);
   const int e_row = c.tid & 31;
@@ -2425,7 +2551,8 @@ __device__ __noinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, int T
   const int nch = rows_num_chunks(row0, row1);
 #pragma unroll 1
   for (int t = 0; t < T; ++t) {
-    stage_x(c, reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)t * topk * op.ld_in, op.ld_in, op.k, kp, nullptr, 0, topk, topk, nullptr);
+    if (ll) stage_ll_pairs(c, reinterpret_cast<const uint2*>(op.ll_in) + (size_t)t * topk * (size_t)(op.ld_in >> 1), op.ld_in, topk, op.k, kp, ll_tag_of(c, op.ll_in_op));
+    else stage_x(c, reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)t * topk * op.ld_in, op.ld_in, op.k, kp, nullptr, 0, topk, topk, nullptr);
 #pragma unroll 1
     for (int ci = 0; ci < nch; ++ci) {
       const int r0 = rows_chunk_begin(row0, row1, nch, ci);
@@ -2434,7 +2561,9 @@ __device__ __noinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, int T
       const uint32_t box_bytes = (uint32_t)R * 128u;
       float comb = 0.f;  // (threads 0..R-1: the running weighted sum of output row r0 + tid)
       float rr = 0.f;
-      if (c.tid < R && res != nullptr) rr = __bfloat162float(__ldcg(res + (size_t)t * op.ld_res + r0 + e_row));
+      if (c.tid < R && res != nullptr)
+        rr = (op.flags & F_LL_RES) ? ll_gather1(c, ll_row(op.ll_res, op.ld_res, t), r0 + e_row, ll_tag_of(c, op.ll_res_op))
+                                   : __bfloat162float(__ldcg(res + (size_t)t * op.ld_res + r0 + e_row));
 #pragma unroll 1
       for (int sl = 0; sl < topk; ++sl) {
         const bool a_real = (lane & 7) == 0;
@@ -2484,14 +2613,21 @@ __device__ __noinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, int T
 #pragma unroll
           for (int w = 0; w < kNumConsumerWarps; ++w) v += sums[(w * kChunkRows + e_row) * TP + half];
           const float f = rbf(v);  // the down projection's output is bf16
-          const float wgt = __ldcg(op.amax_val + (size_t)t * topk + sl);
+          const float wgt = ll ? moe_route_weights(c)[t * topk + sl] : __ldcg(op.amax_val + (size_t)t * topk + sl);
           comb = torch_num ? rbf(comb + rbf(f * wgt)) : fmaf(f, wgt, comb);
         }
       }
-      if (c.tid < R) {
+      if (c.warp == 0) {
         float v = comb;
         if (res != nullptr) v = (torch_num ? rbf(v) : v) + rr;
-        out[(size_t)t * op.ld_out + r0 + e_row] = __float2bfloat16_rn(v);
+        if (e_row < R) out[(size_t)t * op.ld_out + r0 + e_row] = __float2bfloat16_rn(v);
+        if (op.flags & F_LL_OUT) {  // rows come in units of 8: the pair (row, row + 1) sits in two neighbouring lanes
+          const uint32_t lo = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v));
+          const uint32_t hi = __shfl_down_sync(0xffffffffu, lo, 1);
+          if (e_row < R && !(e_row & 1))
+            st_gpu_v2(reinterpret_cast<uint2*>(op.ll_out) + (size_t)t * (size_t)(op.ld_out >> 1) + ((r0 + e_row) >> 1), lo | (hi << 16),
+                      ll_tag_of(c, c.cur_op));
+        }
       }
       consumer_sync();  // (the next chunk's or token's first slot writes the half the last slot may still be read from)
     }
@@ -2861,9 +2997,12 @@ __device__ __noinline__ void producer_loop(Ctx& c) {
       if constexpr (PATH == PATH_ROWS) {
 #if MK_WITH_MOE
         if (rop.type == OP_MOE_LINEAR) {
-          // the expert of a pair is only known once the consumers have passed this op's barrier
+          // the expert of a pair is only known once the consumers have routed the tokens (or passed the op's barrier);
+          // a down projection without a barrier takes the experts of the gate/up linear before it: no wait
           lin_seq += 1;
-          {
+          const bool routed = (rop.flags & F_MOE_ROUTE) != 0 || (rop.flags & (F_MOE_COMBINE | F_LL_IN)) == (F_MOE_COMBINE | F_LL_IN);
+          const volatile int* route = moe_route_ids(c);
+          if (!((rop.flags & F_MOE_COMBINE) && routed)) {
             unsigned long long t0 = 0;
             int spins = 0;
             while ((unsigned)fl[4] < lin_seq) {
@@ -2894,7 +3033,7 @@ __device__ __noinline__ void producer_loop(Ctx& c) {
                 const void* tmap = reinterpret_cast<const unsigned char*>(rop.tmap_w) + ((R >> 3) - 1) * 128;
                 const uint32_t box_bytes = (uint32_t)R * 128u;
                 for (int sl = 0; sl < topk && !dead; ++sl) {
-                  const int wrow = __ldcg(rop.amax_idx + t * topk + sl) * rop.n + r0;
+                  const int wrow = (routed ? route[t * topk + sl] : __ldcg(rop.amax_idx + t * topk + sl)) * rop.n + r0;
                   for (int ks = 0; ks < rop.nkt; ++ks) {
                     if (!mbar_wait(c, bar_empty0 + 8 * s, empty_parity, ST_TIMEOUT_EMPTY)) {
                       dead = true;
@@ -2921,8 +3060,8 @@ __device__ __noinline__ void producer_loop(Ctx& c) {
           if (!wk.any || wk.row0 >= wk.row1) continue;
           const int p_first = wk.row0 / wk.n, p_last = (wk.row1 - 1) / wk.n;
           for (int pr = p_first; pr <= p_last && !dead; ++pr) {
-            const int expert = (rop.flags & F_MOE_ROUTE) ? reinterpret_cast<volatile int*>(c.smem + p.x_off + p.x_bytes - 512)[pr]
-                                                         : __ldcg(rop.amax_idx + pr);
+            const int expert = routed ? route[pr] : __ldcg(rop.amax_idx + pr);
+            const bool silu = (rop.flags & F_SILU_MUL) != 0;
             const int seg0 = max(wk.row0, pr * wk.n), seg1 = min(wk.row1, (pr + 1) * wk.n);
             const int nch = rows_num_chunks(seg0, seg1);
             for (int ci = 0; ci < nch && !dead; ++ci) {
@@ -2941,7 +3080,8 @@ __device__ __noinline__ void producer_loop(Ctx& c) {
                 mbar_arrive_expect_tx(full, 8u * box_bytes);
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                  tma_load_2d_hint(dst + (uint32_t)j * box_bytes, tmap, full, ks * kRowsStageK + j * kBoxK, wrow, pol_stream);
+                  if (silu) tma_load_3d_hint(dst + (uint32_t)j * box_bytes, tmap, full, ks * kRowsStageK + j * kBoxK, (r0 - pr * wk.n) >> 1, 2 * expert, pol_stream);
+                  else tma_load_2d_hint(dst + (uint32_t)j * box_bytes, tmap, full, ks * kRowsStageK + j * kBoxK, wrow, pol_stream);
                 issued += 1;
                 fl[1] = (int)issued;
                 if (++s == S) {
@@ -3298,7 +3438,12 @@ __global__ void __launch_bounds__(PATH == PATH_WIDE ? kWideThreads : kNumThreads
             if constexpr (PATH == PATH_WIDE) op_attention_wide(c, op, T);
             else op_attention(c, op, T);
             break;
-          case OP_SILU_MUL: if (!op_barrier(c, op)) op_silu_mul(c, op, T); break;
+          case OP_SILU_MUL:
+#if MK_WITH_MOE
+            if (op.flags & F_FOLDED) break;  // the expert linear before it has done it
+#endif
+            if (!op_barrier(c, op)) op_silu_mul(c, op, T);
+            break;
           case OP_ARGMAX_PARTIAL: if (!op_barrier(c, op)) op_argmax_partial(c, op, T); break;
           case OP_ARGMAX_REDUCE: if (!op_barrier(c, op)) op_argmax_reduce(c, op, T); break;
           case OP_ALLREDUCE: op_allreduce(c, op, T); break;

@@ -91,6 +91,7 @@ struct PlanOp {
   int in = -1, w = -1, norm_w = -1, res = -1, out = -1;
   int kc = -1, vc = -1, qn = -1, kn = -1, cos = -1, sin = -1;
   int n = 0, k = 0, aux0 = 0, aux1 = 0, aux2 = 0, aux3 = 0;
+  int out2 = -1;              // MoE gate/up with F_SILU_MUL: the activation layer's output
   int amax_n = 0;
   int ll_in_op = -1, ll_res_op = -1;  // tagged activations: the ops that produce the input / the residual
   bool only_next_reads_out = false;   // nothing but the next op reads what this one writes (and the caller cannot see it)
@@ -795,6 +796,19 @@ int plan_graph(mk_handle* h) {
       const Tensor &in = h->tensors[op.t[0]], &out = h->tensors[op.t[1]];
       if (in.ndim != 3 || out.ndim != 3 || in.dims[2] != 2 * out.dims[2] || out.dims[2] % 8 || in.dtype != MK_BF16)
         return h->fail(MK_E_INVALID, "moe_silu_mul: input [T, k, 2 * inter], output [T, k, inter], bf16");
+      // right behind the gate/up linear of the experts: its epilogue has both halves of a column and stores this
+      // layer's output as well (the linear's own output stays what it was)
+      if (fuse && rows_mode && !h->plan.empty()) {
+        PlanOp& prev = h->plan.back();
+        if (prev.type == mk::OP_MOE_LINEAR && !(prev.flags & mk::F_MOE_PAIR_IN) && prev.out == op.t[0] && prev.n == 2 * out.dims[2] &&
+            out.dims[2] % 4 == 0 && in.dims[1] == out.dims[1] && out.dtype == MK_BF16 && out.strides[2] == 1) {
+          prev.flags |= mk::F_SILU_MUL;
+          prev.out2 = op.t[1];
+          prev.note += prev.note.empty() ? "silu_mul in the epilogue" : ", silu_mul in the epilogue";
+          po.flags |= mk::F_FOLDED;
+          po.note = "done by the linear before it";
+        }
+      }
       po.type = mk::OP_SILU_MUL;
       po.in = op.t[0]; po.out = op.t[1];
       po.n = (int)out.dims[2];
@@ -1371,7 +1385,9 @@ static int compile_program(mk_handle* h, bool first) {
   // own producer, or must be older than a barrier that is kept.
   std::map<int, size_t> ll_off;  // tensor -> byte offset of its words in the program's arena
   size_t ll_bytes = 0;
-  if (rows_mode && !has_moe && kp.cluster == 1 && !(cfg.debug_flags & 16)) {
+  for (PlanOp& po : h->plan)
+    if (po.flags & mk::F_FOLDED) po.flags &= ~mk::F_SYNC_BEFORE;
+  if (rows_mode && kp.cluster == 1 && !(cfg.debug_flags & 16)) {
     auto ll_tensor = [&](int id) {
       if (!ll_off.count(id)) {
         const Tensor& t = h->tensors[id];
@@ -1380,6 +1396,13 @@ static int compile_program(mk_handle* h, bool first) {
       }
     };
     auto row_linear = [&](const PlanOp& q) { return q.type == mk::OP_LINEAR && (q.flags & mk::F_ROWS) && q.n % 8 == 0; };
+    // the experts' down projection with the weighted sum folded in owns whole output rows too
+    auto moe_down = [&](const PlanOp& q) { return q.type == mk::OP_MOE_LINEAR && (q.flags & mk::F_MOE_COMBINE) && q.n % 8 == 0; };
+    auto last_writer = [&](size_t before, int id) {
+      for (int q = (int)before - 1; q >= 0; --q)
+        if (h->plan[q].out == id) return q;
+      return -1;
+    };
     auto plain_2d = [&](int id) {
       if (id < 0) return false;
       const Tensor& t = h->tensors[id];
@@ -1412,10 +1435,39 @@ static int compile_program(mk_handle* h, bool first) {
         cur.flags = (cur.flags & ~mk::F_GATHER_RES) | mk::F_LL_RES;
         cur.ll_res_op = reduced_by[cur.res];
       }
+      if (cur.type == mk::OP_MOE_LINEAR && !(cur.flags & mk::F_MOE_PAIR_IN)) {
+        // The MoE layer: router linear -> gate/up linear (routes, activates) -> [activation, folded] -> down projection
+        // (weighted sum).  The gate/up linear reads the rows the router linear has read (tagged by their producer) and
+        // the logits; the down projection reads the activations and takes the routing from its own CTA's gate/up pass.
+        // Every CTA must hold gate/up rows even at one token: its outputs are what keeps the words it polls in place.
+        const int want = mk::F_SYNC_BEFORE | mk::F_NORM_IN | mk::F_MOE_ROUTE | mk::F_SILU_MUL;
+        if ((cur.flags & want) != want || i + 2 >= h->plan.size()) continue;
+        PlanOp &act = h->plan[i + 1], &down = h->plan[i + 2];
+        const int rows_op = last_writer(i, cur.in);
+        const int nvec = (cur.k + mk::kRowsStageK - 1) / mk::kRowsStageK * (mk::kRowsStageK / 8);
+        if (!row_linear(prev) || prev.out != cur.res || !plain_2d(cur.res) || cur.aux1 % 2 != 0 || prev.n != cur.aux1) continue;
+        if (rows_op < 0 || !plain_2d(cur.in) || prev.in != cur.in || !(prev.flags & mk::F_LL_IN) || prev.ll_in_op != rows_op) continue;
+        if (nvec > 128 * (h->plan_tokens <= 1 ? 8 : 4) || (int64_t)cur.aux0 * (cur.n / 8) < h->grid) continue;
+        if (!(act.flags & mk::F_FOLDED) || act.out != cur.out2 || !moe_down(down) || down.in != cur.out2 || down.aux0 != cur.aux0) continue;
+        const Tensor& ta = h->tensors[cur.out2];
+        if (ta.ndim != 3 || ta.strides[1] % 8 != 0 || ta.strides[0] != ta.dims[1] * ta.strides[1]) continue;
+        const int res_op = down.res >= 0 ? last_writer(i + 2, down.res) : -1;
+        if (res_op < 0 || !(h->plan[res_op].flags & mk::F_LL_OUT) || !plain_2d(down.res) || !plain_2d(down.out)) continue;
+        cur.flags = (cur.flags & ~mk::F_SYNC_BEFORE) | mk::F_LL_IN | mk::F_LL_RES | mk::F_LL_OUT;
+        cur.ll_in_op = rows_op;
+        cur.ll_res_op = (int)i - 1;
+        prev.flags |= mk::F_LL_OUT;
+        ll_tensor(cur.res);
+        ll_tensor(cur.out2);
+        down.flags = (down.flags & ~mk::F_SYNC_BEFORE) | mk::F_LL_IN | mk::F_LL_RES;
+        down.ll_in_op = (int)i;
+        down.ll_res_op = res_op;
+        continue;
+      }
       if (!(cur.flags & mk::F_SYNC_BEFORE) || cur.in < 0 || cur.in != prev.out || !plain_2d(cur.in)) continue;
       bool ok = false;
       if (row_linear(cur) && !(cur.flags & mk::F_GATHER_IN)) {
-        ok = ((row_linear(prev) && !(prev.flags & (mk::F_PUSH | mk::F_ARGMAX))) || prev.type == mk::OP_ATTN) && stage_ok(cur);
+        ok = ((row_linear(prev) && !(prev.flags & (mk::F_PUSH | mk::F_ARGMAX))) || prev.type == mk::OP_ATTN || moe_down(prev)) && stage_ok(cur);
       } else if (cur.type == mk::OP_ATTN) {
         ok = row_linear(prev) && !(prev.flags & (mk::F_PUSH | mk::F_ARGMAX | mk::F_SILU_MUL));
       }
@@ -1566,7 +1618,8 @@ static int compile_program(mk_handle* h, bool first) {
     d.ll_in_op = po.ll_in_op;
     d.ll_res_op = po.ll_res_op;
     if (po.flags & mk::F_LL_IN) d.ll_in = (char*)h->ll_buf + ll_off.at(po.in);
-    if (po.flags & mk::F_LL_OUT) d.ll_out = (char*)h->ll_buf + ll_off.at(po.out);
+    if (po.flags & mk::F_LL_OUT) d.ll_out = (char*)h->ll_buf + ll_off.at(po.out2 >= 0 ? po.out2 : po.out);
+    d.out2 = tp(po.out2);
     if (po.flags & mk::F_LL_RES) d.ll_res = (char*)h->ll_buf + ll_off.at(po.res);
     if (po.type == mk::OP_EMBED) {
       d.ld_res = ld(po.w);
@@ -1649,15 +1702,19 @@ static int compile_program(mk_handle* h, bool first) {
       d.nkt = (po.k + mk::kRowsStageK - 1) / mk::kRowsStageK;
       d.amax_idx = route_idx;
       d.amax_val = route_w;
+      const bool silu = (po.flags & mk::F_SILU_MUL) != 0;
+      if (silu) d.ld_out2 = (int)h->tensors[po.out2].strides[1];
       if (((uintptr_t)w.ptr) & 15) return h->fail(MK_E_INVALID, "weight %s is not 16-byte aligned", w.name.c_str());
       map_of[i] = (int)maps.size();
       for (int rows = mk::kUnitRows; rows <= mk::kChunkRows; rows += mk::kUnitRows) {
         CUtensorMap m;
-        cuuint64_t gdim[2] = {(cuuint64_t)po.k, (cuuint64_t)((int64_t)po.aux1 * po.n)};
-        cuuint64_t gstr[1] = {(cuuint64_t)po.k * 2};
-        cuuint32_t box[2] = {(cuuint32_t)mk::kBoxK, (cuuint32_t)rows};
-        cuuint32_t estr[2] = {1, 1};
-        CUresult r = encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, w.ptr, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+        // with the activation in the epilogue, [2 * experts, n / 2, K]: a box is half its rows of gate and half of up
+        const int half = po.n / 2;
+        cuuint64_t gdim[3] = {(cuuint64_t)po.k, silu ? (cuuint64_t)half : (cuuint64_t)((int64_t)po.aux1 * po.n), (cuuint64_t)(2 * po.aux1)};
+        cuuint64_t gstr[2] = {(cuuint64_t)po.k * 2, (cuuint64_t)half * po.k * 2};
+        cuuint32_t box[3] = {(cuuint32_t)mk::kBoxK, silu ? (cuuint32_t)rows / 2 : (cuuint32_t)rows, 2};
+        cuuint32_t estr[3] = {1, 1, 1};
+        CUresult r = encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, silu ? 3 : 2, w.ptr, gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return h->fail(MK_E_CUDA, "cuTensorMapEncodeTiled failed (%d) for %s", (int)r, w.name.c_str());
         maps.push_back(m);

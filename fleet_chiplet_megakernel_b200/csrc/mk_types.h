@@ -53,7 +53,7 @@ enum OpFlags : int {
   F_CTA0_ONLY = 1 << 1,     // only CTA 0 executes the body
   F_NORM_IN = 1 << 2,       // linear: RMSNorm fused on the input rows
   F_RESIDUAL = 1 << 3,      // linear: + residual
-  F_SILU_MUL = 1 << 4,      // linear: rows are [4 gate | 4 up] per 8-row unit, epilogue SiLU(gate)*up
+  F_SILU_MUL = 1 << 4,      // linear: rows are [4 gate | 4 up] per 8-row unit, epilogue SiLU(gate)*up (MoE gate/up: a chunk is [gate | up] halves, also -> out2)
   F_ARGMAX = 1 << 5,        // linear: per-tile (max, index) of the bf16 logits
   F_QK_NORM = 1 << 6,       // attention
   F_ROPE = 1 << 7,          // attention
@@ -78,6 +78,7 @@ enum OpFlags : int {
                             // (weights amax_val, + res), out: [T, n]; no per-slot output, no separate weighted-sum op
   F_MOE_ROUTE = 1 << 22,    // MoE gate/up linear: the op first routes the tokens itself (res: router logits [T, experts]); every CTA
                             // keeps the expert ids in shared memory for its producer, CTA 0 also stores the runtime's tables
+  F_FOLDED = 1 << 24,       // silu_mul behind a MoE gate/up linear with F_SILU_MUL: nothing left to do, no barrier
   F_XRED = 1 << 21,         // linear with F_LL_IN under tensor parallelism: the op first adds up its slice of the latest exchange
                             // over the ranks and stores it as tagged words (ll_in, tagged as its own output), then reads them all
 };
