@@ -261,6 +261,15 @@ __host__ __device__ inline unsigned tile_begin(unsigned c, unsigned total, unsig
 __host__ __device__ inline int tile_owner(unsigned tile, unsigned total, unsigned grid) {
   return (int)(((tile + 1u) * grid - 1u) / total);
 }
+// CTAs that share a wide linear of nblk row blocks x nkt k tiles.  With activation boxes of 64 rows and more, where a
+// block's tiles are few (the ring already holds `stages` of them when the op opens), a CTA takes whole blocks: the
+// exchange of split sums moves 32 KB and more per piece.  Measured, 6 layers, 48 requests of 20 tokens: 582 -> 548 us at
+// 512 hidden, 679 -> 654 at 1024; at 8 requests (boxes of 16 rows) the lone CTA's stream costs more: 502 -> 526 at 1024.
+__host__ __device__ inline int wide_ctas(int grid, int nblk, int nkt, int stages, int x_rows) {
+  if (x_rows >= 64 && nkt <= stages + 4 && nblk <= grid) return nblk;
+  const unsigned total = (unsigned)nblk * (unsigned)nkt;
+  return total < (unsigned)grid ? (int)total : grid;  // with fewer tiles than CTAs the rest idle
+}
 
 static_assert(sizeof(OpDesc) % 16 == 0 && sizeof(OpDesc) <= 256, "OpDesc is copied to shared memory in 16-byte pieces");
 

@@ -58,9 +58,9 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[NC]) {
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // This CTA's range of a stream-K linear's tiles (row block major, k minor); false: nothing for it.
-__device__ __forceinline__ bool wide_range(const OpDesc& op, unsigned& total, int& G, unsigned& t0, unsigned& t1) {
+__device__ __forceinline__ bool wide_range(const KParams& p, const OpDesc& op, unsigned& total, int& G, unsigned& t0, unsigned& t1) {
   total = (unsigned)op.nblk * (unsigned)op.nkt;
-  G = (int)min(gridDim.x, total);  // with fewer tiles than CTAs the rest idle
+  G = wide_ctas((int)gridDim.x, op.nblk, op.nkt, p.num_stages, p.x_rows);  // (the rest idle)
   if ((int)blockIdx.x >= G) return false;
   t0 = tile_begin(blockIdx.x, total, G);
   t1 = tile_begin(blockIdx.x + 1, total, G);
@@ -151,7 +151,7 @@ __device__ __noinline__ void mma_loop(Ctx& c) {
       if (op.type != OP_LINEAR) continue;
       unsigned total, t0, t1;
       int G;
-      if (!wide_range(op, total, G, t0, t1)) continue;
+      if (!wide_range(p, op, total, G, t0, t1)) continue;
       const int nkt = op.nkt;
       int kt = (int)(t0 % (unsigned)nkt);
       bool fresh = true;
@@ -352,7 +352,7 @@ __device__ __noinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
   best.idx[0] = best.idx[1] = 0x7fffffff;
   unsigned total, t0, t1;
   int G;
-  if (wide_range(op, total, G, t0, t1)) {
+  if (wide_range(p, op, total, G, t0, t1)) {
     const bool with_res = (op.flags & F_RESIDUAL) && !MK_XF(op, F_GATHER_RES) && (!(op.flags & F_RES_RANK0) || p.rank == 0);
     const size_t slot_vec = (size_t)kTileRows * N / 4;  // float4 of a CTA's partial sums
 #pragma unroll 1
