@@ -2197,11 +2197,12 @@ __device__ void op_argmax_reduce(Ctx& c, const OpDesc& op, int T) {
 // k rounds of (largest probability, lowest index), weights renormalised over the k picked
 // (transformers' Qwen3MoeTopKRouter with norm_topk_prob; reference task: topk_softmax_sm100.cuh:61-290).
 // One token, by one warp: `w_out` / `idx_out` and `w_out2` / `idx_out2` (may be null) receive the k weights and expert
-// ids.  `words` not null: the logits arrive as tagged words.  A round is two warp-wide integer reductions (a
-// probability's bits grow with it), not five levels of shuffles of (value, index).
+// ids.  `words` not null: the logits arrive as tagged words.  Lane l holds experts l, l + 32, ...: the softmax's sum runs
+// over them in that order, however the logits arrive.  A round is two warp-wide integer reductions (a probability's
+// bits grow with it), not five levels of shuffles of (value, index).
 __device__ __noinline__ void moe_route_token(Ctx& c, const __nv_bfloat16* logits, const uint2* words, unsigned tag, int E, int K, float* w_out,
                                              int* idx_out, float* w_out2, int* idx_out2) {
-  float v[8];  // up to 256 experts, 8 per lane: v[i] is expert 2 * (lane + 32 * (i / 2)) + i % 2
+  float v[8];  // up to 256 experts, 8 per lane
   if (words != nullptr) {
     unsigned long long t0 = 0;
     unsigned spins = 0;
@@ -2227,25 +2228,26 @@ __device__ __noinline__ void moe_route_token(Ctx& c, const __nv_bfloat16* logits
       }
     }
     __syncwarp();
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = (i & 1) ? bf_hi(q[i >> 1].x) : bf_lo(q[i >> 1].x);
-  } else {
+    // word w holds experts 2 w and 2 w + 1 and sits in lane w % 32: expert l + 32 i is a half of word l / 2 + 16 i
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const int e = 2 * (c.lane + 32 * (i >> 1)) + (i & 1);
-      v[i] = e < E ? __bfloat162float(__ldcg(logits + e)) : 0.f;
+      const uint32_t x = __shfl_sync(0xffffffffu, q[i >> 1].x, (c.lane >> 1) + 16 * (i & 1));
+      v[i] = (c.lane & 1) ? bf_hi(x) : bf_lo(x);
     }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = c.lane + 32 * i < E ? __bfloat162float(__ldcg(logits + c.lane + 32 * i)) : 0.f;
   }
   float mx = -INFINITY;
 #pragma unroll
   for (int i = 0; i < 8; ++i)
-    if (2 * (c.lane + 32 * (i >> 1)) + (i & 1) < E) mx = fmaxf(mx, v[i]);
+    if (c.lane + 32 * i < E) mx = fmaxf(mx, v[i]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   float sum = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
-    v[i] = 2 * (c.lane + 32 * (i >> 1)) + (i & 1) < E ? expf(v[i] - mx) : 0.f;
+    v[i] = c.lane + 32 * i < E ? expf(v[i] - mx) : 0.f;
     sum += v[i];
   }
 #pragma unroll
@@ -2255,7 +2257,7 @@ __device__ __noinline__ void moe_route_token(Ctx& c, const __nv_bfloat16* logits
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const float pr = v[i] * inv;
-    key[i] = (2 * (c.lane + 32 * (i >> 1)) + (i & 1) < E && pr >= 0.f) ? __float_as_uint(pr) + 1u : 0u;
+    key[i] = (c.lane + 32 * i < E && pr >= 0.f) ? __float_as_uint(pr) + 1u : 0u;
   }
   float picked_sum = 0.f, my_w = 0.f;
   int my_e = 0;
@@ -2267,7 +2269,7 @@ __device__ __noinline__ void moe_route_token(Ctx& c, const __nv_bfloat16* logits
     for (int i = 0; i < 8; ++i)
       if (key[i] > best) {  // (a lane's experts come in ascending order: the first of equals is the lowest)
         best = key[i];
-        bi = 2 * (c.lane + 32 * (i >> 1)) + (i & 1);
+        bi = c.lane + 32 * i;
       }
     const uint32_t m = __reduce_max_sync(0xffffffffu, best);
     const int e = __reduce_min_sync(0xffffffffu, best == m && m != 0u ? bi : 0x7fffffff);
@@ -2279,7 +2281,7 @@ __device__ __noinline__ void moe_route_token(Ctx& c, const __nv_bfloat16* logits
     }
 #pragma unroll
     for (int i = 0; i < 8; ++i)
-      if (2 * (c.lane + 32 * (i >> 1)) + (i & 1) == e) key[i] = 0u;  // taken
+      if (c.lane + 32 * i == e) key[i] = 0u;  // taken
   }
   if (c.lane < K) {
     if (w_out != nullptr) w_out[c.lane] = my_w / picked_sum;

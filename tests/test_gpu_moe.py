@@ -87,6 +87,50 @@ def test_moe_block_matches_oracle(T, E, K, H, I, fuse):
     k.finalize()
 
 
+def _routing_weights(logits, K):
+    """Softmax and renormalised top-k weights in fp32, summed as documented: lane l of 32 adds up experts l, l + 32, ...,
+    then the lanes meet in a butterfly; the picked probabilities are added in the order they are picked."""
+    v = torch.exp(logits.float() - logits.float().amax(-1, keepdim=True))
+    T, E = v.shape
+    s = torch.zeros(T, 32, device=v.device)
+    for i in range(0, E, 32):
+        s = s + v[:, i:i + 32]
+    lane = torch.arange(32, device=v.device)
+    for o in (16, 8, 4, 2, 1):
+        s = s + s[:, lane ^ o]
+    pr = v * (1.0 / s[:, :1])
+    val, idx = torch.sort(pr, dim=-1, descending=True, stable=True)
+    picked = torch.zeros(T, device=v.device)
+    for k in range(K):
+        picked = picked + val[:, k]
+    return val[:, :K] / picked[:, None], idx[:, :K]
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3])
+def test_routing_weights_keep_their_bits(seed):
+    """The weights are fp32 sums in a fixed order.  Their last bit is made visible by a residual that cancels the layer's
+    output to its first bf16: what is left is 2^-9 of the terms, so a weight off by one unit flips about 1 % of the values."""
+    T, E, K, H, I = 2, 128, 8, 2048, 64
+    x, router = _rand((T, H), 80 + seed), _rand((E, H), 90 + seed, 1.0 / H ** 0.5)
+    w13, w2 = _rand((E, 2 * I, H), 73, 0.05), _rand((E, H, I), 74, 0.05)
+    res = torch.zeros(T, H, dtype=BF)
+    for cancelled in (False, True):
+        k, meta, _ = onepass_kernel(T, fuse=False)
+        od = torch.zeros(T, H, dtype=BF, device="cuda")
+        gate_out, _, _, out = _moe_block(k, T, E, K, H, I, x, router, w13, w2, res, od)
+        k.compile()
+        k()
+        rows, logits = k.read_tensor(out).cuda().view(T, K, H).double(), k.read_tensor(gate_out).cuda()
+        wgt, _ = _routing_weights(logits, K)
+        acc = torch.zeros(T, H, device="cuda")
+        for s in range(K):  # fused multiply-adds: exact in float64, then one rounding
+            acc = (rows[:, s] * wgt[:, s, None].double() + acc.double()).float()
+        want = (acc + res.cuda().float()).to(BF)
+        assert torch.equal(od, want), int((od != want).sum())
+        res = -od.cpu()
+        k.finalize()
+
+
 def _geom(g):
     return mk.Qwen3MoeGeometry(hidden=g.hidden, n_q=g.n_q, n_kv=g.n_kv, head_dim=g.head_dim, experts=g.experts, top_k=g.top_k,
                                moe_mlp=g.moe_mlp, layers=g.layers, vocab=g.vocab, rope_theta=g.rope_theta)
