@@ -617,6 +617,87 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t&
   lo = pack2(a - bf_lo(mid), b - bf_hi(mid));
 }
 
+// A task whose output is not finite, once more.  An mma multiplies every row by every V row of its tile: by P = 0 where a
+// causal row does not see the position or the tile runs past the end, and by three parts of P of either sign elsewhere, so
+// 0 x inf would carry an infinite value of a prompt chunk's last token into the tokens before it.  Here a row takes the
+// positions it sees and no others, in scalar fp32: a warp per row, a lane per position for the scores and four dims per
+// lane for the sums.  (The check sits on the outputs: 36 layers at 8 requests 5.83 -> 5.86 ms; on the accumulators, with
+// the sums redone in place, 5.90.)
+__device__ __noinline__ void wide_attend_exact(const Ctx& c, const OpDesc& op, const WideTask& a, int W, __nv_bfloat16* out, float* part) {
+  const KParams& p = c.p;
+  const int HKV = op.aux0, qpk = op.aux1 / HKV, rows = a.nt * qpk, lane = c.lane;
+  const float sc = 1.4426950408889634f * 0.08838834764831845f;  // log2(e) / sqrt(128)
+#pragma unroll 1
+  for (int r = c.warp & (W - 1); r < rows; r += W) {
+    const int tok = r / qpk, head = r % qpk, last = min(a.L0 + tok, a.p1);
+    const uint4* q = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.out2) + (size_t)(a.t0 + tok) * op.ld_out2 +
+                                                    (size_t)(a.h * qpk + head) * kHeadDim);
+    float M = -INFINITY, L = 0.f, O[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 1
+    for (int pass = 0; pass < 2; ++pass) {  // the maximum, then the sums
+#pragma unroll 1
+      for (int pos0 = a.p0; pos0 < last; pos0 += 32) {
+        const int pos = min(pos0 + lane, last - 1);
+        const int slot = (__ldcg(p.kv_indices + a.kvb + (pos >> p.page_shift)) << p.page_shift) + (pos & (p.page_size - 1));
+        const uint4* k = reinterpret_cast<const uint4*>(op.k_cache) + ((size_t)slot * HKV + a.h) * (kHeadDim / 8);
+        float s = 0.f;
+#pragma unroll 4
+        for (int i = 0; i < kHeadDim / 8; ++i) {
+          float qf[8], kf[8];
+          unpack8(__ldcg(q + i), qf);
+          unpack8(__ldcg(k + i), kf);
+#pragma unroll
+          for (int e = 0; e < 8; ++e) s = fmaf(qf[e], kf[e], s);
+        }
+        s = pos0 + lane < last ? s * sc : -INFINITY;
+        if (pass == 0) {
+          M = fmaxf(M, s);
+          continue;
+        }
+        const float pr = exp2f(s - (M == -INFINITY ? 0.f : M));
+        L += pr;
+#pragma unroll 4
+        for (int i = 0; i < min(32, last - pos0); ++i) {
+          const int vs = __shfl_sync(0xffffffffu, slot, i);
+          const float pi = __shfl_sync(0xffffffffu, pr, i);
+          const uint2 v = __ldcg(reinterpret_cast<const uint2*>(op.v_cache) + ((size_t)vs * HKV + a.h) * (kHeadDim / 4) + lane);
+          O[0] = fmaf(pi, bf_lo(v.x), O[0]);
+          O[1] = fmaf(pi, bf_hi(v.x), O[1]);
+          O[2] = fmaf(pi, bf_lo(v.y), O[2]);
+          O[3] = fmaf(pi, bf_hi(v.y), O[3]);
+        }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        if (pass == 0) M = fmaxf(M, __shfl_xor_sync(0xffffffffu, M, o));
+        else L += __shfl_xor_sync(0xffffffffu, L, o);
+      }
+    }
+    if (a.nch == 1) {
+      const float inv = __fdividef(1.0f, L);
+      *reinterpret_cast<uint2*>(out + (size_t)tok * op.ld_out + head * kHeadDim + 4 * lane) =
+          make_uint2(pack2(O[0] * inv, O[1] * inv), pack2(O[2] * inv, O[3] * inv));
+    } else {
+      *reinterpret_cast<float2*>(part + r * kHeadDim + 4 * lane) = make_float2(O[0], O[1]);
+      *reinterpret_cast<float2*>(part + r * kHeadDim + 4 * lane + 2) = make_float2(O[2], O[3]);
+      if (lane == 0) {
+        part[rows * kHeadDim + r] = M;
+        part[rows * kHeadDim + rows + r] = L;
+      }
+    }
+  }
+}
+// bar.sync that also tells every thread whether any thread's `pred` holds
+__device__ __forceinline__ bool bar_any(int id, int nthr, bool pred) {
+  uint32_t r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %3, 0;\n\tbar.red.or.pred q, %1, %2, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
+      : "=r"(r)
+      : "r"(id), "r"(nthr), "r"((uint32_t)pred)
+      : "memory");
+  return r != 0u;
+}
+
 // One task by W warps.  `reg`: the group's shared memory (W x 2 KB), `ml`: [warps of the CTA][16] (max, sum) pairs.
 template <bool FULL>
 __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTask& a, int W, int gi, uint8_t* reg, float2* ml) {
@@ -749,6 +830,7 @@ __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTas
   }
   MK_STAMP(c, 2);
   __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out) + (size_t)a.t0 * op.ld_out + (size_t)a.h * qpk * kHeadDim;
+  float chk = 0.f;  // stays zero while the outputs are finite
   if (W == 1 && a.nch == 1) {
     // this lane holds, per row, dims 64 x + 16 j + {0..7} (oacc[8 x + i][0]) and the eight behind them (oacc[8 x + i][1])
 #pragma unroll
@@ -763,12 +845,16 @@ __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTas
           for (int y = 0; y < 2; ++y) {
             float f[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) f[i] = oacc[8 * x + i][2 * u + y] * inv;
+            for (int i = 0; i < 8; ++i) {
+              f[i] = oacc[8 * x + i][2 * u + y] * inv;
+              chk = fmaf(f[i], 0.f, chk);
+            }
             *reinterpret_cast<uint4*>(dst + 64 * x + 8 * y) = pack8(f);
           }
       }
     }
     __syncwarp();
+    if (__any_sync(0xffffffffu, chk != 0.f)) wide_attend_exact(c, op, a, W, out, nullptr);
     return;
   }
   // The warps of the task meet in shared memory, four rows at a time (the slots take the place of the q rows).
@@ -817,6 +903,7 @@ __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTas
         O.z = fmaf(f, o4.z, O.z);
         O.w = fmaf(f, o4.w, O.w);
       }
+      chk = fmaf(O.x, 0.f, fmaf(O.y, 0.f, fmaf(O.z, 0.f, fmaf(O.w, 0.f, chk))));
       if (a.nch == 1) {
         const float inv = __fdividef(1.0f, L);
         *reinterpret_cast<uint2*>(out + (size_t)(r / qpk) * op.ld_out + (r % qpk) * kHeadDim + d) =
@@ -832,12 +919,13 @@ __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTas
     }
   }
   MK_STAMP(c, 3);
-  if (a.nch == 1) {
-    asm volatile("bar.sync %0, %1;" ::"r"(nbar), "r"(nthr) : "memory");  // the group's memory is free again
-    return;
+  if (bar_any((int)nbar, nthr, chk != 0.f)) {  // (the group's memory is free again)
+    wide_attend_exact(c, op, a, W, out, part);
+    asm volatile("bar.sync %0, %1;" ::"r"(nbar), "r"(nthr) : "memory");
   }
-  // several chunks (then W == 8, the whole CTA): the one that arrives last merges them
-  consumer_sync();  // the CTA's partial is complete; thread 0's release below publishes all of it
+  if (a.nch == 1) return;
+  // several chunks (then W == 8, the whole CTA): the one that arrives last merges them.  The CTA's partial is complete
+  // behind the sync above; thread 0's release publishes all of it.
   unsigned* cnt = p.attn_count + (size_t)a.t0 * HKV + a.h;
   volatile int* fl = c.flags();
   if (c.tid == 0) {
@@ -862,7 +950,7 @@ __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTas
         for (int u = 0; u < 8; ++u) {
           const bool ok = c0 + u < a.nch;
           const float* b = base + (size_t)(ok ? c0 + u : c0) * stride;
-          v[u] = __ldcg(reinterpret_cast<const float2*>(b + r * kHeadDim + d));
+          v[u] = ok ? __ldcg(reinterpret_cast<const float2*>(b + r * kHeadDim + d)) : make_float2(0.f, 0.f);
           mm[u] = ok ? __ldcg(b + rows * kHeadDim + r) : -INFINITY;
           ll[u] = ok ? __ldcg(b + rows * kHeadDim + rows + r) : 0.f;
         }

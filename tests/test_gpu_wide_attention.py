@@ -100,3 +100,25 @@ def test_probabilities_keep_fp32(requests, n_q, n_kv):
             total += ref.numel()
     print(f"{wrong} of {total} outputs are not the nearest bf16")
     assert wrong <= 1e-3 * total, (wrong, total)
+
+
+@pytest.mark.parametrize("requests,n_q,n_kv", [([(40, 4), (3, 9), (20, 1)], 4, 1), ([(200, 5), (33, 1), (0, 7)], 16, 8), ([(600, 6)], 16, 2),
+                                               ([(50, 1), (37, 1), (300, 1)], 16, 4)])
+def test_infinite_values_reach_only_the_rows_that_see_them(requests, n_q, n_kv):
+    """Infinities in V: of new tokens (later tokens of a chunk only may show them) and of a cached row (all tokens show them,
+    as the infinity that the sum gives, not as 0 x inf)."""
+    def edit(a):
+        rows = a.qkv.view(a.qkv.shape[0], n_kv, n_q // n_kv + 2, D)
+        for r, (_, n) in enumerate(requests):
+            rows[a.starts[r] + n - 1, :, -1, 5] = math.inf  # the last new token of each request
+            rows[a.starts[r] + n // 2, 0, -1, 7] = -math.inf
+        p = a.pages[0][0]
+        a.vc[p, 2, :, 100] = math.inf  # position 2 of the first request
+    a = Attention(requests, n_q, n_kv, 16, seed=5, edit=edit)
+    for r, (_, n) in enumerate(requests):
+        for i in range(n):
+            ref, got = a.reference(r, i), a.out[a.starts[r] + i].double()
+            assert torch.equal(ref.isnan(), got.isnan()) and torch.equal(ref.isinf(), got.isinf()), f"request {r} token {i}"
+            assert torch.equal(ref[ref.isinf()], got[ref.isinf()])
+            fin = ref.isfinite()
+            assert float((got[fin] - ref[fin]).abs().max()) <= 1e-2 * float(ref[fin].abs().max())
