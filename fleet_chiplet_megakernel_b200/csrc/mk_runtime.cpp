@@ -40,9 +40,22 @@ constexpr int kRowsSumsBytes = mk::kNumConsumerWarps * mk::kChunkRows * 2 * 4;  
 // token rows a row-owner CTA may keep resident beside three 32 KB weight stages
 constexpr int kRowsXBudget = kFastSmem - 2048 - kRedBytes - kRowsSumsBytes - 3 * mk::kStageBytes;
 constexpr int kAttnMaxChunks = 32;
-constexpr int kWideMaxStages = 5;  // ring stages of the wide path, shared memory permitting
 constexpr int kGateUpUnit = 4;     // fused gate/up weights are laid out [4 gate | 4 up] per 8-row unit
 constexpr int kMaxStepTimes = 16384;
+
+// The wide path's shared memory.  Ring: stages of 32 KB of weights and two activation boxes of x_rows token rows.  As many
+// stages as leave the CTA within the 164 KB carve-out (3 up to 32 token rows, 2 beyond): what the carve-out takes is L1,
+// and the kernel's own state, spills and metadata live there.  Measured with 5, 4, 3 and 2 stages, us per step of 6 layers:
+// 512 hidden, 4 requests 423, 364, 328, 310 (409 on the path of up to 16 tokens that kept to 164 KB); 1152 hidden, 8
+// requests of 300 tokens 557, 489, 461, 439; 4096 hidden, 8 of 300 1047, 986, 961, 1004, 32 requests 1117, 1063, 1034,
+// 1084; 64 requests (48 KB stages, 4, 3 and 2 of them) 1340, 1285, 1290; 128 prompt tokens (64 KB, 3 and 2) 1805, 1735.
+constexpr int kWideFixed = 1024 /*alignment slack*/ + mk::kWideRedBytes + 2048 /*barriers and flags, op descriptors*/;
+int wide_x_rows(int tokens) { return tokens <= 16 ? 16 : (tokens <= 32 ? 32 : (tokens <= 64 ? 64 : 128)); }
+int wide_stage_bytes(int tokens) { return mk::kStageBytes + 2 * wide_x_rows(tokens) * 128; }
+int wide_stages(int tokens, int x_bytes) {
+  const int fast = (kFastSmem - kWideFixed - x_bytes) / wide_stage_bytes(tokens);
+  return fast >= 2 ? fast : std::min(2, (kMaxSmem - kWideFixed - x_bytes) / wide_stage_bytes(tokens));
+}
 
 size_t dtype_size(int dt) {
   switch (dt) {
@@ -1203,6 +1216,13 @@ int mk_debug_exchange_sequence(uint32_t total_before, uint32_t k, int world, int
   return 0;
 }
 
+int mk_debug_wide_ring(int tokens, int x_bytes, int* smem_out) {
+  if (tokens < 1 || tokens > 128 || x_bytes < 0) return MK_E_INVALID;
+  const int stages = wide_stages(tokens, x_bytes);
+  if (smem_out) *smem_out = stages * wide_stage_bytes(tokens) + kWideFixed + x_bytes + kParamSmem;
+  return stages;
+}
+
 int mk_barrier_target_reached(uint32_t counter, uint32_t epoch, uint32_t arrivals_per_barrier) {
   // the comparison the device's grid barrier makes (modulo 2^32)
   return (int)(counter - epoch * arrivals_per_barrier) >= 0 ? 1 : 0;
@@ -1258,12 +1278,12 @@ static int compile_program(mk_handle* h, bool first) {
   // scratch][row-owner path: sums block][small scratch][barriers, flags, op descriptors].
   const int nt = h->plan_tokens;
   const bool rows_mode = h->rows_mode;  // row-owner linears: resident token rows, no activation boxes
-  const int x_rows = rows_mode ? 0 : (nt <= 16 ? 16 : (nt <= 32 ? 32 : (nt <= 64 ? 64 : 128)));
-  const int stage_bytes = mk::kStageBytes + 2 * x_rows * 128;
+  const int x_rows = rows_mode ? 0 : wide_x_rows(nt);
+  const int stage_bytes = rows_mode ? mk::kStageBytes : wide_stage_bytes(nt);
   const int sums_bytes = rows_mode ? kRowsSumsBytes : 0;
   const int red_bytes = rows_mode ? kRedBytes : mk::kWideRedBytes;
   const int bar_bytes = rows_mode ? 1024 : 2048;  // barriers and flags, then the two op descriptors
-  const int fixed0 = 1024 /*alignment slack*/ + sums_bytes + red_bytes + bar_bytes;
+  const int fixed0 = rows_mode ? 1024 /*alignment slack*/ + sums_bytes + red_bytes + bar_bytes : kWideFixed;
   // Measured on B200: a CTA whose shared memory (plus the 1 KB the system adds) stays within
   // the 164 KB carve-out leaves 92 KB of the SM's unified array to L1, and the whole kernel
   // runs about 8 % faster than with the next carve-out (196 KB, 60 KB of L1).
@@ -1321,7 +1341,7 @@ static int compile_program(mk_handle* h, bool first) {
   int stages;
   if (cfg.max_stages > 0) stages = std::min(s_max, want_stages);  // an explicit request wins
   else if (rows_mode) stages = std::min(s_fast, 4) >= 3 ? std::min(s_fast, 4) : std::min(s_max, 4);
-  else stages = std::min(s_max, kWideMaxStages);
+  else stages = wide_stages(nt, x_bytes);
   if (stages < 2) return h->fail(MK_E_UNSUPPORTED, "activations need %d bytes of shared memory: no room for the weight ring", x_bytes);
   mk::KParams& kp = h->kp;
   memset(&kp, 0, sizeof(kp));
@@ -1369,7 +1389,7 @@ static int compile_program(mk_handle* h, bool first) {
     }
     // wide LM head: one partial per CTA that holds tiles and row quarter
     if (po.type == mk::OP_LINEAR && !(po.flags & mk::F_ROWS) && (po.flags & mk::F_ARGMAX)) {
-      po.amax_n = mk::wide_ctas(h->grid, (po.n + mk::kTileRows - 1) / mk::kTileRows, (po.k + mk::kTileK - 1) / mk::kTileK, stages, x_rows) * 4;
+      po.amax_n = mk::wide_ctas(h->grid, (po.n + mk::kTileRows - 1) / mk::kTileRows, (po.k + mk::kTileK - 1) / mk::kTileK, x_rows) * 4;
       if (i + 1 < h->plan.size() && h->plan[i + 1].type == mk::OP_ARGMAX_REDUCE) h->plan[i + 1].amax_n = po.amax_n;
     }
   }

@@ -261,12 +261,14 @@ __host__ __device__ inline unsigned tile_begin(unsigned c, unsigned total, unsig
 __host__ __device__ inline int tile_owner(unsigned tile, unsigned total, unsigned grid) {
   return (int)(((tile + 1u) * grid - 1u) / total);
 }
-// CTAs that share a wide linear of nblk row blocks x nkt k tiles.  With activation boxes of 64 rows and more, where a
-// block's tiles are few (the ring already holds `stages` of them when the op opens), a CTA takes whole blocks: the
-// exchange of split sums moves 32 KB and more per piece.  Measured, 6 layers, 48 requests of 20 tokens: 582 -> 548 us at
-// 512 hidden, 679 -> 654 at 1024; at 8 requests (boxes of 16 rows) the lone CTA's stream costs more: 502 -> 526 at 1024.
-__host__ __device__ inline int wide_ctas(int grid, int nblk, int nkt, int stages, int x_rows) {
-  if (x_rows >= 64 && nkt <= stages + 4 && nblk <= grid) return nblk;
+// CTAs that share a wide linear of nblk row blocks x nkt k tiles.  With activation boxes of 64 rows and more, a CTA takes
+// whole blocks where a block's tiles are few: the exchange of split sums moves 32 KB and more per piece.  Measured, us per
+// step of 6 layers with the line at 6, 8, 9 and 16 k tiles: 1024 hidden, 64 requests 643, 621, 621, 622, 128 prompt tokens
+// 1016, 908, 910, 907; 1152 hidden 748, 742, 744, 745 and 1042, 1003, 965, 967; 2048 hidden (16 k tiles) 909, 910, 909,
+// 947 and 1232, 1232, 1236, 1213.  At 8 requests (boxes of 16 rows) the lone CTA's stream costs more: 502 -> 526 at 1024.
+constexpr int kWholeTiles = 9;
+__host__ __device__ inline int wide_ctas(int grid, int nblk, int nkt, int x_rows) {
+  if (x_rows >= 64 && nkt <= kWholeTiles && nblk <= grid) return nblk;
   const unsigned total = (unsigned)nblk * (unsigned)nkt;
   return total < (unsigned)grid ? (int)total : grid;  // with fewer tiles than CTAs the rest idle
 }

@@ -163,6 +163,9 @@ int mk_debug_partition(int64_t nblk, int64_t nkt, int grid, int64_t* begin_out /
  * the numbers a slot may still hold from earlier uses would be taken for "arrived" (must be 0). */
 int mk_debug_exchange_sequence(uint32_t total_before, uint32_t k, int world, int tokens, int cols, uint32_t* seq_out,
                                int64_t* first_word_out, int* stale_arrived_out);
+/* Weight stages of the wide path's ring for iterations of up to `tokens` tokens, with x_bytes of activation scratch, and
+ * the shared memory of a CTA (used by the host-side tests). */
+int mk_debug_wide_ring(int tokens, int x_bytes, int* smem_out);
 int mk_barrier_target_reached(uint32_t counter, uint32_t epoch, uint32_t arrivals_per_barrier);
 void* mk_tensor_ptr(mk_handle* h, int tensor_id);      /* device address after compile (runtime-owned ones too) */
 int mk_tensor_read(mk_handle* h, int tensor_id, void* host_buf, int64_t bytes); /* copy a tensor's bytes to the host */

@@ -14,10 +14,10 @@ def _rand(shape, seed, scale=1.0):
     return (torch.randn(shape, generator=torch.Generator().manual_seed(seed)) * scale).to(BF)
 
 
-# k tiles of 128: 1, 8 and 9 (around the line between whole blocks and split ones at 64 rows of activations: the ring's
-# stages + 4), 24 with one block (24 pieces) and with three; the tolerance is bf16_close's of the other linear tests
+# k tiles of 128: 1, 8, 9 and 10 (around the line between whole blocks and split ones at 64 and 128 rows of activations:
+# nine), 24 with one block (24 pieces) and with three; the tolerance is bf16_close's of the other linear tests
 @pytest.mark.parametrize("T", [3, 17, 33, 64, 65, 128])
-@pytest.mark.parametrize("N,K", [(200, 128), (1024, 1024), (1160, 1096), (128, 3072), (384, 3072)])
+@pytest.mark.parametrize("N,K", [(200, 128), (1024, 1024), (1160, 1096), (384, 1176), (128, 3072), (384, 3072)])
 def test_wide_linear_matches_oracle(T, N, K):
     x, w, r = _rand((T, K), 1), _rand((N, K), 2, 0.05), _rand((T, N), 3)
     k, meta, _ = onepass_kernel(T)
