@@ -2762,8 +2762,8 @@ __device__ __noinline__ int bookkeep_prepare(Ctx& c) {
   const KParams& p = c.p;
   const int R = p.max_reqs;
   int head = p.sched[0], tail = p.sched[1];
-  int* old_idx = reinterpret_cast<int*>(c.smem + p.x_off);
   const int n_old = p.kv_indptr[R];
+  int* old_idx = n_old <= p.page_entries ? reinterpret_cast<int*>(c.smem + p.x_off) : p.page_scratch;
   for (int i = 0; i < n_old; ++i) old_idx[i] = p.kv_indices[i];
   int nreq = 0, ntok = 0, npages = 0;
   for (int i = 0; i < R; ++i) {

@@ -1290,7 +1290,7 @@ static int compile_program(mk_handle* h, bool first) {
   const int want_stages = cfg.max_stages > 0 ? std::min(cfg.max_stages, 16) : 4;
   // (row-owner mode prefers two resident token rows and three stages to one row and four)
   int x_budget = kRowsXBudget;
-  int x_bytes = cfg.max_num_pages * 4;
+  int x_bytes = 0;
   int max_nblk = 1, n_linear = 0;
   bool has_moe = false, has_attn = false;
   if (rows_mode)
@@ -1343,8 +1343,15 @@ static int compile_program(mk_handle* h, bool first) {
   else if (rows_mode) stages = std::min(s_fast, 4) >= 3 ? std::min(s_fast, 4) : std::min(s_max, 4);
   else stages = wide_stages(nt, x_bytes);
   if (stages < 2) return h->fail(MK_E_UNSUPPORTED, "activations need %d bytes of shared memory: no room for the weight ring", x_bytes);
+  // The page table is rewritten through shared memory as far as it fits into what the ring leaves of the carve-out
+  // (a larger pool costs no stage and no L1), through global memory beyond.
+  const int used = fixed + stages * stage_bytes;
+  const int spare = (used <= kFastSmem ? kFastSmem : kMaxSmem) - used;
+  const int64_t table = (int64_t)cfg.max_num_pages * 4;
+  if (table > x_bytes) x_bytes += (int)std::min<int64_t>(spare / 1024 * 1024, (table - x_bytes + 1023) / 1024 * 1024);
   mk::KParams& kp = h->kp;
   memset(&kp, 0, sizeof(kp));
+  kp.page_entries = (x_bytes - (has_moe ? 512 : 0)) / 4;  // (the expert ids keep their place at the end)
   kp.num_stages = stages;
   kp.stage_bytes = stage_bytes;
   kp.x_rows = x_rows;
@@ -1573,6 +1580,8 @@ static int compile_program(mk_handle* h, bool first) {
     kp.request_ids = (int*)p;
     if (int e = h->dmalloc(&p, (size_t)cfg.max_num_pages * 4)) return e;
     kp.page_queue = (int*)p;
+    if (int e = h->dmalloc(&p, (size_t)cfg.max_num_pages * 4)) return e;
+    kp.page_scratch = (int*)p;
     if (int e = h->dmalloc(&p, 256)) return e;
     kp.sched = (int*)p;
     kp.grid_bar = (unsigned*)p + 16;
@@ -1586,6 +1595,7 @@ static int compile_program(mk_handle* h, bool first) {
     const mk::KParams& k0 = h->prog[0].kp;
     kp.request_ids = k0.request_ids;
     kp.page_queue = k0.page_queue;
+    kp.page_scratch = k0.page_scratch;
     kp.sched = k0.sched;
     kp.grid_bar = k0.grid_bar;
     kp.ctrl = k0.ctrl;

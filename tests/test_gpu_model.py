@@ -518,3 +518,24 @@ def test_mpk_wrapper_generates_what_the_decoder_generates():
     out = m.run(p)
     m.finalize()
     assert out[0].cpu().tolist() == base[0]
+
+
+@pytest.mark.parametrize("pool,budget", [(30000, 128), (30000, 64), (8100, 8), (30000, 1)])
+def test_large_page_pools(pool, budget):
+    """Pools whose page table does not fit into shared memory beside the ring, and tables in use that do not: one-position
+    pages and up to 7600 of them, against 64-position pages (the same arithmetic, whatever the pages: bit for bit)."""
+    geom, R = O.TINY, 1 if budget == 1 else 8
+    w = _cuda(O.make_weights(geom, 0, norm_jitter=0.25))
+    prompts = [O.make_prompt(geom, 940 - 3 * r if budget > 8 else 30, r) for r in range(R)]
+    P = max(len(p) for p in prompts)
+    n_new = 10 if budget > 8 else 960 - P
+    got = []
+    for page, pages in ((1, pool), (64, None)):
+        dec = mk.Qwen3Decoder(_geom(geom), w, max_seq_length=P + n_new, max_requests=R, page_size=page, max_num_pages=pages,
+                              max_num_batched_tokens=budget, numerics="mpk", keep_logits=True)
+        dec.set_prompts(prompts)
+        dec.run()
+        got.append(([dec.generated(r).cpu() for r in range(R)], dec.logits[:R].cpu()))
+        dec.finalize()
+    assert all(torch.equal(a, b) for a, b in zip(got[0][0], got[1][0]))
+    assert torch.equal(got[0][1], got[1][1])
