@@ -963,7 +963,8 @@ mk_handle* mk_create(const mk_config* cfg) {
   h->cfg = *cfg;
   if (h->cfg.timeout_ms <= 0) h->cfg.timeout_ms = 4000;
   if ((h->cfg.debug_flags & 15) != 0)
-    fprintf(stderr, "b200mk: debug_flags=0x%x: measurement mode, the kernel skips arithmetic and its results are WRONG\n",
+    fprintf(stderr, "b200mk: debug_flags=0x%x: measurement mode, the kernel skips arithmetic (bit 0: linears at one or two tokens; bit 1: attention) "
+            "and its results are WRONG\n",
             h->cfg.debug_flags);
   return h;
 }

@@ -218,7 +218,8 @@ struct KParams {
   // k = 0 op reached, 1 barrier passed, 2 op done; op == num_ops is the iteration prologue
   unsigned long long* prof;
   int trace_op;     // op whose inner phases are stamped: prof[(num_ops + 1) * grid * 4 + cta * 16 + k]; -1 none
-  int debug_flags;  // bit 0: linear tasks skip the arithmetic
+  int debug_flags;  // bit 0: linear tasks of the row-owner path skip the arithmetic (the wide path's MMA issuer does not look
+                    // at it: the look cost 0.4 % of a step); bit 1: attention tasks keep their barrier and do nothing else
   int has_attn;        // (wide path) the program holds attention ops: the token table is filled every iteration
   int prefetch_tiles;  // weight tiles per CTA requested into L2 ahead of the ring (0 = off)
   int has_moe;         // the program holds mixture-of-experts ops: the host launches the build of the kernel that has them
