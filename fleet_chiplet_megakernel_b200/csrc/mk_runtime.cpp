@@ -1241,10 +1241,10 @@ static int lower_wide(mk_handle* h) {
     PlanOp& lin = h->plan[i];
     const int tmp = plan_temp_tensor(h, "__normed_" + std::to_string(lin.k), h->cfg.max_num_batched_tokens, lin.k);
     if (tmp < 0) return tmp;
-    if (!h->tensors[tmp].ptr)
-      if (int e = h->dmalloc(&h->tensors[tmp].ptr, h->tensors[tmp].alloc_bytes())) return e;
     nrm.type = mk::OP_RMSNORM;
     nrm.flags = (lin.flags & (mk::F_SYNC_BEFORE | mk::F_GATHER_IN));
+    // (rows gathered from the ranks need no barrier, but the op before may still be reading an earlier norm's rows there)
+    if (i > 0 && h->plan[i - 1].in == tmp) nrm.flags |= mk::F_SYNC_BEFORE;
     nrm.in = lin.in; nrm.w = lin.norm_w; nrm.out = tmp;
     nrm.n = lin.k;
     nrm.note = "from a fused input norm";
@@ -1266,14 +1266,29 @@ static int lower_wide(mk_handle* h) {
   return 0;
 }
 
+int mk_debug_describe_wide(mk_handle* h, char* buf, int n) {
+  if (!h) return MK_E_INVALID;
+  if (h->compiled) return h->fail(MK_E_STATE, "already compiled");
+  if (int e = mk_plan(h)) return e;
+  if (h->rows_mode) return h->fail(MK_E_STATE, "the row-owner path takes this plan");
+  if (int e = lower_wide(h)) return e;
+  const int ops = mk_describe(h, buf, n);
+  h->planned = false;
+  return ops;
+}
+
 // Everything of mk_compile that depends on the width a program is planned for (h->plan_tokens): the
 // shared-memory carve-up, scratch, tensor maps, op descriptors and kernel parameters of the plan in
 // h->plan.  `first`: also allocates the scheduler state the programs of a handle share.
 static int compile_program(mk_handle* h, bool first) {
   const mk_config& cfg = h->cfg;
   cudaError_t ce;
-  if (!h->rows_mode)
+  if (!h->rows_mode) {
     if (int e = lower_wide(h)) return e;
+    for (auto& t : h->tensors)
+      if (t.owned && !t.ptr)
+        if (int e = h->dmalloc(&t.ptr, t.alloc_bytes())) return e;
+  }
   // 2. shared-memory carve-up: [weight ring: stages x (32 KB of weights + two activation
   // boxes of x_rows token rows)][x region: resident token rows (row-owner path), attention
   // scratch][row-owner path: sums block][small scratch][barriers, flags, op descriptors].

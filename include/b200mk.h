@@ -163,6 +163,8 @@ int mk_debug_partition(int64_t nblk, int64_t nkt, int grid, int64_t* begin_out /
  * the numbers a slot may still hold from earlier uses would be taken for "arrived" (must be 0). */
 int mk_debug_exchange_sequence(uint32_t total_before, uint32_t k, int world, int tokens, int cols, uint32_t* seq_out,
                                int64_t* first_word_out, int* stale_arrived_out);
+/* mk_describe of the plan as the wide path runs it (host only, before mk_compile; used by the host-side tests). */
+int mk_debug_describe_wide(mk_handle* h, char* buf, int n);
 /* Weight stages of the wide path's ring for iterations of up to `tokens` tokens, with x_bytes of activation scratch, and
  * the shared memory of a CTA (used by the host-side tests). */
 int mk_debug_wide_ring(int tokens, int x_bytes, int* smem_out);

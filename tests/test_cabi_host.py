@@ -392,3 +392,32 @@ def test_wide_ring_leaves_the_l1_its_share(native_lib, tokens):
     assert stages >= 2 and smem.value + 1024 <= 164 * 1024
     stages = native_lib.mk_debug_wide_ring(tokens, 64 * 1024, C.byref(smem))  # (a norm of 32768 columns)
     assert stages >= 2 and smem.value <= 227 * 1024
+
+
+@pytest.mark.parametrize("widths,barrier", [((512, 512), True), ((512, 1024), False)])
+def test_norm_rows_are_not_overwritten_while_the_linear_before_reads_them(widths, barrier):
+    """Two fused norm linears with an allreduce between them, on the wide path: each norm becomes an op that stores its rows,
+    into the same rows where the widths are equal.  The second takes its input word by word, without a barrier, but the
+    linear before it may still be reading the first one's rows."""
+    T, (k0, k1) = 4, widths
+    k = mk.PersistentKernel(mode="online_notoken", world_size=2, mpi_rank=0, num_workers=0, num_local_schedulers=0, num_remote_schedulers=0,
+                            max_seq_length=64, max_num_batched_requests=T, max_num_batched_tokens=T, max_num_pages=8, page_size=16,
+                            meta_tensors=_meta(T, T, 64, 8), profiler_tensor=None, trace_name="", spec_decode_config=None, use_cutlass_kernel=True)
+    held = []
+
+    def attach(name, *shape):
+        held.append(torch.zeros(shape, dtype=torch.bfloat16))
+        return k.attach_input(held[-1], name)
+
+    part, buf, red = k.new_tensor(dims=(T, k1), name="part"), k.new_tensor(dims=(2, T, k1), name="buf"), k.new_tensor(dims=(T, k1), name="red")
+    k.rmsnorm_linear_layer(input=attach("x", T, k0), weight_norm=attach("n0", k0), weight_linear=attach("w0", k1, k0), output=part,
+                           grid_dim=(8, 1, 1), block_dim=(128, 1, 1))
+    k.allreduce_layer(input=part, buffer=buf, output=red, grid_dim=(8, 1, 1), block_dim=(128, 1, 1))
+    k.rmsnorm_linear_layer(input=red, weight_norm=attach("n1", k1), weight_linear=attach("w1", 256, k1), output=attach("y", T, 256),
+                           grid_dim=(4, 1, 1), block_dim=(128, 1, 1))
+    buf_ = C.create_string_buffer(1 << 16)
+    assert k._lib.mk_debug_describe_wide(k._h, buf_, 1 << 16) == 4
+    ops = buf_.value.decode().strip().splitlines()
+    assert [ln.split()[1] for ln in ops] == ["rmsnorm", "linear", "rmsnorm", "linear"]
+    sync = [int(ln.split("flags=")[1].split()[0], 16) & 1 for ln in ops]
+    assert sync == [0, 1, 1 if barrier else 0, 1], ops

@@ -122,3 +122,92 @@ def test_infinite_values_reach_only_the_rows_that_see_them(requests, n_q, n_kv):
             assert torch.equal(ref[ref.isinf()], got[ref.isinf()])
             fin = ref.isfinite()
             assert float((got[fin] - ref[fin]).abs().max()) <= 1e-2 * float(ref[fin].abs().max())
+
+
+# One and several new tokens behind none, some and many cached ones; 1, 2, 4 and 8 q heads per kv head (8 to 1 token of a
+# request share a group); pages below 8 positions (looked up row by row), of 8 and of 64.  The last three are few and long:
+# several chunks per pair, with groups across chunk borders (chunks of 144 positions in the second last, 128 and 160 beside it).
+REQUESTS = {
+    "mixed": [(0, 1), (250, 7), (1000, 17), (0, 7)],
+    "long chunk": [(1000, 64), (0, 7), (250, 1)],
+    "wide": [(3 + 5 * r, 1 + r % 4) for r in range(40)],
+    "128 new": [(40, 128)],
+    "one long": [(1000, 7)],
+    "straddle": [(1000, 3), (142, 5), (286, 4), (126, 5), (430, 3)],
+    "one short chunk": [(253, 6), (120, 17)],
+}
+
+
+@pytest.mark.parametrize("page", [4, 8, 64])
+@pytest.mark.parametrize("n_q,n_kv", [(4, 4), (8, 4), (8, 2), (16, 2)])
+@pytest.mark.parametrize("requests", sorted(REQUESTS))
+def test_new_tokens_behind_cached_ones(requests, n_q, n_kv, page):
+    a = Attention(REQUESTS[requests], n_q, n_kv, page, seed=21)
+    kc, vc = a.kc.clone(), a.vc.clone()
+    new = torch.zeros(kc.shape[:2], dtype=torch.bool)
+    for r, (_, n) in enumerate(a.requests):
+        for i in range(n):
+            pos, t, _, k, v = a.token(r, i)
+            kc[a.pages[r][pos // page], pos % page], vc[a.pages[r][pos // page], pos % page] = k, v
+            new[a.pages[r][pos // page], pos % page] = True
+            ref, got = a.reference(r, i), a.out[t].double()
+            # bf16 outputs (2^-9) of bf16 inputs that are the same on both sides: 1e-2 of the largest, as for every attention test
+            assert float((got - ref).abs().max()) <= 1e-2 * float(ref.abs().max()), f"request {r} token {i}"
+    # The new rows, and no other.  V is copied; K is rounded to bf16 behind the norm and behind the rotation, so where the
+    # fp32 sum of squares rounds otherwise (2^-22) a value within that of a rounding border may come out one step (2^-8 of
+    # the pair it is rotated with) off: at most 2^-13 of the values per rounding.
+    got = a.kcd.cpu()
+    assert torch.equal(a.vcd.cpu(), vc) and torch.equal(got[~new], kc[~new])
+    off = (got[new].float() - kc[new].float()).abs()
+    assert float((off / kc[new].float().abs().amax(-1, keepdim=True)).max()) <= 2 ** -7
+    assert int((off > 0).sum()) <= 2 + 2 ** -11 * off.numel()
+
+
+@pytest.mark.parametrize("requests,n_q,n_kv", [([(0, 3)], 4, 2), ([(30, 17)], 8, 8), ([(5, 40), (100, 1)], 16, 2), ([(7 * r, 2) for r in range(35)], 8, 2),
+                                               ([(64, 128)], 8, 4)])
+def test_qkv_epilogue_gives_the_bits_of_the_separate_preparation(requests, n_q, n_kv):
+    """QKV linear and attention: the linear's epilogue normalises, rotates and appends (fuse), or the attention op does."""
+    H, page = 640, 16
+    R, T = len(requests), sum(n for _, n in requests)
+    lens = [c + n for c, n in requests]
+    pages = [math.ceil(n / page) for n in lens]
+    dev = torch.device("cuda")
+    x, w = _rand((T, H), 31).to(dev), _rand(((n_q + 2 * n_kv) * D, H), 32, 0.05).to(dev)
+    qn, kn = (1 + 0.2 * _rand((D,), 33).float()).to(BF).to(dev), (1 + 0.2 * _rand((D,), 34).float()).to(BF).to(dev)
+    cos, sin = (c.to(dev) for c in O.rope_tables(O.Geometry(n_q=n_q, n_kv=n_kv), max(lens) + 1))
+    cache = _rand((2, sum(pages), page, n_kv, D), 35)
+    got = []
+    for fuse in (True, False):
+        i32 = lambda v: torch.tensor(v, dtype=torch.int32, device=dev)  # noqa: E731
+        indptr, starts = [0], [0]
+        for (_, n), p in zip(requests, pages):
+            indptr.append(indptr[-1] + p)
+            starts.append(starts[-1] + n)
+        meta = {
+            "step": i32([0] * R), "tokens": torch.zeros(R, max(lens) + 1, dtype=torch.int64, device=dev),
+            "input_tokens": torch.zeros(T, 1, dtype=torch.int64, device=dev), "output_tokens": torch.zeros(T, 1, dtype=torch.int64, device=dev),
+            "num_new_tokens": i32([1] * R), "prompt_lengths": i32([1] * R), "qo_indptr_buffer": i32(starts),
+            "paged_kv_indptr_buffer": i32(indptr), "paged_kv_indices_buffer": i32(list(range(sum(pages)))[::-1]),
+            "paged_kv_last_page_len_buffer": i32([n - (p - 1) * page for n, p in zip(lens, pages)]),
+        }
+        kc, vc = cache[0].to(dev), cache[1].to(dev)
+        out = torch.zeros(T, n_q * D, dtype=BF, device=dev)
+        k = mk.PersistentKernel(
+            mode="online_notoken", world_size=1, mpi_rank=0, num_workers=0, num_local_schedulers=0, num_remote_schedulers=0,
+            max_seq_length=max(lens) + 1, max_num_batched_requests=R, max_num_batched_tokens=T, max_num_pages=sum(pages), page_size=page,
+            meta_tensors=meta, numerics="torch", fuse=fuse)
+        qkv = k.new_tensor(dims=(T, (n_q + 2 * n_kv) * D), name="qkv")
+        k.linear_layer(input=k.attach_input(x, "x"), weight=k.attach_input(w, "w"), output=qkv, grid_dim=(n_q + 2 * n_kv, 1, 1), block_dim=(128, 1, 1))
+        k.paged_attention_layer(
+            input=qkv, k_cache=k.attach_input(kc, "kc"), v_cache=k.attach_input(vc, "vc"), q_norm=k.attach_input(qn, "qn"),
+            k_norm=k.attach_input(kn, "kn"), cos_pos_embed=k.attach_input(cos, "cos"), sin_pos_embed=k.attach_input(sin, "sin"),
+            output=k.attach_input(out, "o"), grid_dim=(R, n_kv, 1), block_dim=(128, 1, 1))
+        k.compile()
+        assert ("KV append in the epilogue" in k.describe()) == fuse
+        k()
+        torch.cuda.synchronize()
+        k.finalize()
+        got.append((out, kc, vc))
+    assert not torch.equal(got[0][1].cpu(), cache[0])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)

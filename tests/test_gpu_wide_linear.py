@@ -3,6 +3,7 @@ tiles at 33 tokens and more), pieces fetched in one batch and in several, ragged
 import pytest
 import torch
 
+import fleet_chiplet_megakernel_b200 as mk
 from oracle import qwen3_oracle as O
 from tests.helpers import onepass_kernel, bf16_close
 
@@ -31,4 +32,63 @@ def test_wide_linear_matches_oracle(T, N, K):
         k()
         bf16_close(od, O.mpk_linear(x, w), 1e-2, f"linear {T}x{N}x{K}")
         bf16_close(rd, O.mpk_linear(x, w, residual=r), 1e-2, f"with residual {T}x{N}x{K}")
+    k.finalize()
+
+
+@pytest.mark.parametrize("T", [3, 17, 33, 64, 65, 128])
+@pytest.mark.parametrize("K,inter", [(512, 1024), (1160, 192), (3072, 64)])
+def test_wide_gate_up_matches_oracle(T, K, inter):
+    x, wg, wu = _rand((T, K), 4), _rand((inter, K), 5, 0.05), _rand((inter, K), 6, 0.05)
+    k, meta, _ = onepass_kernel(T)
+    od = torch.zeros(T, inter, dtype=BF, device="cuda")
+    wgu = k.shuffle_tensors([k.attach_input(wg.cuda(), "wg"), k.attach_input(wu.cuda(), "wu")], 0, inter // 64, "wgu")
+    mid = k.new_tensor(dims=(T, 2 * inter), name="mid")
+    k.linear_layer(input=k.attach_input(x.cuda(), "x"), weight=wgu, output=mid, grid_dim=(2 * inter // 64, 1, 1), block_dim=(128, 1, 1))
+    k.silu_mul_layer(input=mid, output=k.attach_input(od, "o"), grid_dim=(inter // 64, 1, 1), block_dim=(128, 1, 1))
+    assert "silu_mul fused" in k.plan()
+    k.compile()
+    k()
+    bf16_close(od, O.mpk_silu_mul(O.mpk_linear(x, wg), O.mpk_linear(x, wu)), 1e-2, f"gate/up {T}x{inter}x{K}")
+    k.finalize()
+
+
+@pytest.mark.parametrize("T", [3, 17, 64, 65, 128])
+def test_wide_lm_head_picks_the_lowest_index_of_ties(T):
+    """The argmax in the epilogue of the LM head, on whole numbers (every sum and its bf16 rounding is exact): two equal best
+    rows within a warp's rows, within a block, in two blocks and far apart; logits that are all negative; logits that are
+    all zero, of either sign."""
+    V, K = 20008, 512
+    gen = torch.Generator().manual_seed(3)
+    w = torch.randint(-1, 2, (V, K), generator=gen).float()
+    x = torch.randint(0, 2, (T, K), generator=gen).float() * 2 - 1
+    w[:, 0], x[:, 0] = 1.0, 0.0
+    tied = 0
+    for t in range(T):
+        a = (t * 151 + 7) % (V - 9000)
+        if t % 6 < 4:
+            for row in (a, a + (5, 70, 128, 8000)[t % 6]):
+                w[row, 1:] = x[t, 1:]
+        elif t % 6 == 4:
+            x[t, 0] = -600.0
+        else:
+            x[t] = 0.0
+            x[t, ::2] = -0.0
+    logits = (x.double() @ w.double().T).to(BF).float()
+    best = logits.max(-1, keepdim=True).values
+    want = [int((logits[t] == best[t]).nonzero()[0]) for t in range(T)]
+    tied = sum(int((logits[t] == best[t]).sum()) > 1 for t in range(T))
+    assert tied > T // 2 and (T < 6 or float(best.min()) < 0)
+    k, meta, _ = onepass_kernel(T)
+    lg = torch.zeros(T, V, dtype=BF, device="cuda")
+    lgt = k.attach_input(lg, "argmax_in")
+    pv, pi = k.new_tensor(dims=(T, 8), name="pv"), k.new_tensor(dims=(T, 8), dtype=mk.int64, name="pi")
+    k.linear_layer(input=k.attach_input(x.to(BF).cuda(), "x"), weight=k.attach_input(w.to(BF).cuda(), "w"), output=lgt, grid_dim=(8, 1, 1),
+                   block_dim=(128, 1, 1))
+    k.argmax_partial_layer(input=lgt, output=(pv, pi), grid_dim=(8, 1, 1), block_dim=(128, 1, 1))
+    k.argmax_reduce_layer(input=(pv, pi), output=k.attach_input(meta["output_tokens"], "tok"), grid_dim=(1, 1, 1), block_dim=(128, 1, 1))
+    assert "argmax partials fused" in k.plan()
+    k.compile()
+    k()
+    assert torch.equal(lg.float().cpu(), logits)
+    assert meta["output_tokens"][:, 0].tolist() == want
     k.finalize()
