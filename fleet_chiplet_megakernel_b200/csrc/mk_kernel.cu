@@ -2843,7 +2843,7 @@ __device__ __forceinline__ bool cursor_open(const KParams& p, TileCursor& tc, in
   const OpDesc& op = p.ops[oi];
   if (op.type != OP_LINEAR) return false;
   const unsigned total = (unsigned)op.nblk * (unsigned)op.nkt;
-  const int G = wide_ctas((int)gridDim.x, op.nblk, op.nkt, p.x_rows);
+  const int G = wide_ctas((int)gridDim.x, op.nblk, op.nkt);
   if ((int)blockIdx.x >= G) return false;
   tc.oi = oi;
   tc.tile = tile_begin(blockIdx.x, total, G);

@@ -1412,7 +1412,7 @@ static int compile_program(mk_handle* h, bool first) {
     }
     // wide LM head: one partial per CTA that holds tiles and row quarter
     if (po.type == mk::OP_LINEAR && !(po.flags & mk::F_ROWS) && (po.flags & mk::F_ARGMAX)) {
-      po.amax_n = mk::wide_ctas(h->grid, (po.n + mk::kTileRows - 1) / mk::kTileRows, (po.k + mk::kTileK - 1) / mk::kTileK, x_rows) * 4;
+      po.amax_n = mk::wide_ctas(h->grid, (po.n + mk::kTileRows - 1) / mk::kTileRows, (po.k + mk::kTileK - 1) / mk::kTileK) * 4;
       if (i + 1 < h->plan.size() && h->plan[i + 1].type == mk::OP_ARGMAX_REDUCE) h->plan[i + 1].amax_n = po.amax_n;
     }
   }

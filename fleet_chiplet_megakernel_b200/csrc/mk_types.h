@@ -264,16 +264,14 @@ __host__ __device__ inline unsigned tile_begin(unsigned c, unsigned total, unsig
 __host__ __device__ inline int tile_owner(unsigned tile, unsigned total, unsigned grid) {
   return (int)(((tile + 1u) * grid - 1u) / total);
 }
-// CTAs that share a wide linear of nblk row blocks x nkt k tiles.  With activation boxes of 64 rows and more, a CTA takes
-// whole blocks where a block's tiles are few: the exchange of split sums moves 32 KB and more per piece.  Measured, us per
-// step of 6 layers with the line at 6, 8, 9 and 16 k tiles: 1024 hidden, 64 requests 643, 621, 621, 622, 128 prompt tokens
-// 1016, 908, 910, 907; 1152 hidden 748, 742, 744, 745 and 1042, 1003, 965, 967; 2048 hidden (16 k tiles) 909, 910, 909,
-// 947 and 1232, 1232, 1236, 1213.  At 8 requests (boxes of 16 rows) the lone CTA's stream costs more: 502 -> 526 at 1024.
-constexpr int kWholeTiles = 9;
-__host__ __device__ inline int wide_ctas(int grid, int nblk, int nkt, int x_rows) {
-  if (x_rows >= 64 && nkt <= kWholeTiles && nblk <= grid) return nblk;
+// CTAs that share a wide linear of nblk row blocks x nkt k tiles: all of them, a tile each where there are fewer tiles.
+// (A CTA per whole block, without an exchange of sums, from 33 tokens and up to nine tiles a block, was taken back: an mma
+// chain truncates what it adds up, and over 8 tiles it misrounds 0.059 % of the outputs; split over CTAs and added in fp32
+// 0.010 %.  It gave 6 layers at 64 requests 517 instead of 538 us at 512 hidden, 621 to 628 instead of 637 and, with eight
+// kv heads, 743 instead of 726 at 1024; with the tiles of a whole block added one by one in registers 540, 646 and 768.)
+__host__ __device__ inline int wide_ctas(int grid, int nblk, int nkt) {
   const unsigned total = (unsigned)nblk * (unsigned)nkt;
-  return total < (unsigned)grid ? (int)total : grid;  // with fewer tiles than CTAs the rest idle
+  return total < (unsigned)grid ? (int)total : grid;
 }
 
 static_assert(sizeof(OpDesc) % 16 == 0 && sizeof(OpDesc) <= 256, "OpDesc is copied to shared memory in 16-byte pieces");

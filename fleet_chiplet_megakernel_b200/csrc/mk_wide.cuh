@@ -60,7 +60,7 @@ __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.
 // This CTA's range of a stream-K linear's tiles (row block major, k minor); false: nothing for it.
 __device__ __forceinline__ bool wide_range(const KParams& p, const OpDesc& op, unsigned& total, int& G, unsigned& t0, unsigned& t1) {
   total = (unsigned)op.nblk * (unsigned)op.nkt;
-  G = wide_ctas((int)gridDim.x, op.nblk, op.nkt, p.x_rows);  // (the rest idle)
+  G = wide_ctas((int)gridDim.x, op.nblk, op.nkt);  // (the rest idle)
   if ((int)blockIdx.x >= G) return false;
   t0 = tile_begin(blockIdx.x, total, G);
   t1 = tile_begin(blockIdx.x + 1, total, G);
