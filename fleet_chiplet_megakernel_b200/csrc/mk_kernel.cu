@@ -2011,6 +2011,26 @@ __device__ void op_embed(Ctx& c, const OpDesc& op, int T) {
   }
 }
 
+// A row that is too wide for shared memory: read once for its sum of squares (in stage_x's order) and once to be scaled.
+__device__ __noinline__ void rmsnorm_wide_row(Ctx& c, const OpDesc& op, int tok) {
+  const bool torch_num = c.p.numerics == NUM_TORCH;
+  const int kvec = op.n >> 3;
+  const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)tok * op.ld_in);
+  uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(op.out) + (size_t)tok * op.ld_out);
+  float* red = c.red();
+  float ss = 0.f;
+#pragma unroll 4
+  for (int v = c.tid; v < kvec; v += kNumConsumers) ss = sumsq8(__ldcg(src + v), torch_num, ss);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (c.lane == 0) red[c.warp] = ss;
+  consumer_sync();
+  const float r = row_rms_scale(red, 0, kNumConsumerWarps, op.n, torch_num);
+#pragma unroll 4
+  for (int v = c.tid; v < kvec; v += kNumConsumers) dst[v] = scale8(__ldcg(src + v), __ldg(reinterpret_cast<const uint4*>(op.w) + v), r, torch_num);
+  consumer_sync();
+}
+
 __device__ void op_rmsnorm(Ctx& c, const OpDesc& op, int T) {
   const int kp = ((op.n + 63) / 64) * 64;
   // the norm weights do not depend on other CTAs: a CTA that has a row fetches them ahead of the barrier
@@ -2025,6 +2045,10 @@ __device__ void op_rmsnorm(Ctx& c, const OpDesc& op, int T) {
   }
   if (op_barrier(c, op)) return;
   for (int tok = blockIdx.x; tok < T; tok += gridDim.x) {
+    if (op.n > kNormStagedCols && !MK_XF(op, F_GATHER_IN)) {
+      rmsnorm_wide_row(c, op, tok);
+      continue;
+    }
     // (the sums are also stored into the gathered tensor's own rows when the host asked for it: aux0)
     if (MK_XF(op, F_GATHER_IN)) stage_x(c, nullptr, op.ld_in, op.n, kp, op.w, tok, 1, tok + 1, pre ? pre_w : nullptr, true,
                                          (op.aux0 && pre) ? const_cast<void*>(op.in) : nullptr);

@@ -1341,7 +1341,7 @@ static int compile_program(mk_handle* h, bool first) {
       if (spans * (kp + 8) * 2 + 16 > x_budget) return h->fail(MK_E_UNSUPPORTED, "moe linear: K=%d is too wide", p.k);
       x_bytes = std::max(x_bytes, spans * (kp + 8) * 2 + 16);
     } else if (p.type == mk::OP_RMSNORM) {
-      x_bytes = std::max(x_bytes, ((p.n + 63) / 64 * 64 + 8) * 2 + 16);
+      if (p.n <= mk::kNormStagedCols || (p.flags & mk::F_GATHER_IN)) x_bytes = std::max(x_bytes, ((p.n + 63) / 64 * 64 + 8) * 2 + 16);
     } else if (p.type == mk::OP_ATTN) {
       has_attn = true;
       // row-owner path: q heads and the new k (bf16), combine slots of 16 half-warps x 128 floats, (max, sum) pairs, merge scratch

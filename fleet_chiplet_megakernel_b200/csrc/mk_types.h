@@ -26,6 +26,9 @@ constexpr int kNumThreads = kNumConsumers + 64;
 constexpr int kWideThreads = kNumConsumers + 96;
 constexpr int kWideRedBytes = 4096;              // scratch of the wide path: reductions and the iteration's token table
 constexpr int kHeadDim = 128;
+// Columns a stand-alone norm stages in shared memory (48 KB).  Wider rows are read twice instead: at 65 tokens and more,
+// where a ring stage is 64 KB, two stages would leave no room for rows of more than 46000 columns.
+constexpr int kNormStagedCols = 24576;
 // Row-owner linear (one or two batched tokens): a CTA owns a contiguous range of 8-row units
 // and walks it in chunks of up to 32 rows; a stage holds a chunk's rows for 512 k-elements
 // as eight TMA boxes of 64 k-elements (32 KB for a full chunk).

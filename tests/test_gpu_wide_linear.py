@@ -114,3 +114,20 @@ def test_sums_of_few_tiles_keep_fp32(T, N, K):
         k.finalize()
     print(f"{wrong} of {total} outputs are not the nearest bf16")
     assert wrong <= 3 + 2.5e-4 * total, (wrong, total)
+
+
+@pytest.mark.parametrize("numerics", ["mpk", "torch"])
+@pytest.mark.parametrize("T,K", [(3, 24576), (3, 24584), (70, 24584), (100, 49152), (8, 65536)])
+def test_norm_of_rows_wider_than_shared_memory(T, K, numerics):
+    """Around and beyond the 24576 columns that are staged in shared memory."""
+    x, wn = _rand((T, K), 9, 3.0), (1 + 0.3 * _rand((K,), 10).float()).to(BF)
+    k, meta, _ = onepass_kernel(T, numerics=numerics)
+    od = torch.zeros(T, K, dtype=BF, device="cuda")
+    k.rmsnorm_layer(input=k.attach_input(x.cuda(), "x"), weight=k.attach_input(wn.cuda(), "wn"), output=k.attach_input(od, "o"),
+                    grid_dim=(T, 1, 1), block_dim=(128, 1, 1))
+    k.compile()
+    k()
+    # "mpk": one rounding (8e-3 as for the other norms).  "torch": the scale itself is bf16, and a row whose mean lies at a
+    # rounding border may get the next one: 2^-7, and 2^-8 for each of the two products.
+    bf16_close(od, O.mpk_rmsnorm(x, wn) if numerics == "mpk" else O.ref_rmsnorm(x, wn), 8e-3 if numerics == "mpk" else 2 ** -6, "rmsnorm")
+    k.finalize()
