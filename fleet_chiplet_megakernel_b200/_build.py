@@ -8,12 +8,15 @@ import os
 import shutil
 import subprocess
 import sys
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libb200mk.so")
-# mk_kernel_tp.cu, mk_kernel_hier.cu and mk_kernel_moe.cu include mk_kernel.cu with other build switches (see its header)
-SOURCES = ["mk_kernel.cu", "mk_kernel_tp.cu", "mk_kernel_hier.cu", "mk_kernel_moe.cu", "mk_runtime.cpp", "mk_noalloc.cu"]
+# mk_kernel_tp.cu, mk_kernel_hier.cu and mk_kernel_moe.cu include mk_kernel.cu with other build switches (see its header); each
+# is compiled once per linear path (MK_NC, see mk_launch.cu)
+SOURCES = {"mk_kernel.cu": (0, 8, 16, 32), "mk_kernel_tp.cu": (0, 8, 16, 32), "mk_kernel_hier.cu": (0, 8, 16, 32), "mk_kernel_moe.cu": (0, 8),
+           "mk_launch.cu": None, "mk_runtime.cpp": None, "mk_noalloc.cu": None}
 HEADERS = ["mk_types.h", "mk_wide.cuh", os.path.join("..", "..", "include", "b200mk.h")]
 
 
@@ -28,7 +31,7 @@ def needs_build():
     if not os.path.exists(LIB):
         return True
     t = os.path.getmtime(LIB)
-    deps = [os.path.join(CSRC, s) for s in SOURCES + HEADERS]
+    deps = [os.path.join(CSRC, s) for s in list(SOURCES) + HEADERS]
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
@@ -40,22 +43,22 @@ def build(force=False, verbose=False):
         flags = ["-Xptxas", "-v"] + flags
     objdir = os.path.join(HERE, "build")
     os.makedirs(objdir, exist_ok=True)
-    # one nvcc per source, side by side (the three builds of the kernel dominate), then one link
-    procs = []
-    for src in SOURCES:
-        obj = os.path.join(objdir, os.path.splitext(src)[0] + ".o")
-        cmd = [_nvcc()] + flags + ["-c", os.path.join(CSRC, src), "-o", obj]
-        if verbose:
-            print(" ".join(cmd))
-        procs.append((cmd, obj, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
-    objs = []
-    for cmd, obj, pr in procs:
-        out, _ = pr.communicate()
-        if verbose or pr.returncode != 0:
-            sys.stdout.write(out)
-        if pr.returncode != 0:
-            raise subprocess.CalledProcessError(pr.returncode, cmd)
-        objs.append(obj)
+    jobs = []
+    for src, instances in SOURCES.items():
+        stem = os.path.splitext(src)[0]
+        for nc in instances or (None,):
+            obj = os.path.join(objdir, stem + ("" if nc is None else f"_{nc}") + ".o")
+            define = [] if nc is None else [f"-DMK_NC={nc}"]
+            jobs.append(([_nvcc()] + flags + define + ["-c", os.path.join(CSRC, src), "-o", obj], obj))
+    # one nvcc per object, as many side by side as there are cores, then one link
+    with ThreadPoolExecutor(max_workers=os.cpu_count() or 4) as pool:
+        done = list(pool.map(lambda job: subprocess.run(job[0], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True), jobs))
+    for (cmd, _), r in zip(jobs, done):
+        if verbose or r.returncode != 0:
+            sys.stdout.write(" ".join(cmd) + "\n" + r.stdout)
+        if r.returncode != 0:
+            raise subprocess.CalledProcessError(r.returncode, cmd)
+    objs = [obj for _, obj in jobs]
     subprocess.check_call([_nvcc(), "-shared", "-o", LIB] + objs)
     return LIB
 

@@ -18,16 +18,27 @@
 
 #include "mk_types.h"
 
-// This file is compiled three times into one library (see the wrappers mk_kernel_tp.cu and
-// mk_kernel_hier.cu): the persistent kernel runs every op body once per layer out of a cold
-// instruction cache, and code that is merely present in an op (a branch for another
-// configuration, the registers it pins) measurably slows the batch-1 step down.  So the
-// single-GPU kernels carry no tensor-parallel exchange code (+2.8 % when present) and only the
-// kernels launched in thread-block clusters carry the hierarchical grid barrier (+2.0 %).
-//   MK_VARIANT        inner namespace of this compilation: base | tp | hier
+// This file is compiled several times into one library (see the wrappers mk_kernel_tp.cu,
+// mk_kernel_hier.cu and mk_kernel_moe.cu, and mk_launch.cu): the persistent kernel runs every op body
+// once per layer, and code that is merely present in an op (a branch for another configuration, the
+// registers it pins) measurably slows a step down.  So the single-GPU kernels carry no tensor-parallel
+// exchange code (+2.8 % when present), only the kernels launched in thread-block clusters carry the
+// hierarchical grid barrier (+2.0 %), and each instance holds one linear path.
+//
+// There are no calls in an instance: with one, its per-thread context lives in local memory, calls save
+// and restore registers there, and the register split of the warp roles (kConsumerRegs) has no effect.
+// A block then had 200 to 320 KB of local memory beside an L1 of 28 to 92 KB.  Without calls it has
+// none.  Measured against the same code with out-of-line functions, 12 layers of 8B width, us per step: one
+// request 1283 -> 1109, two 1468 -> 1166, eight of 300 tokens 1707 -> 1477, 32 of 100 1878 -> 1588, 64 of 100 2340 -> 1942;
+// four layers 1024 wide, one request 172 -> 134.
+//   MK_NC             linear path: 0 the row-owner path, 8, 16 or 32 the wide path (token columns of a finishing thread)
+//   MK_VARIANT        inner namespace of this compilation: base | tp | hier | moe
 //   MK_WITH_XCHG      1: linear epilogues can push to / input staging can gather from the ranks' exchange regions
 //   MK_HIER_BARRIER   1: cluster-first grid barrier (the kernel must be launched with a cluster dimension)
 //   MK_WITH_MOE       1: the mixture-of-experts ops (routing, per-expert row-owner linears, weighted combine)
+#ifndef MK_NC
+#define MK_NC 0
+#endif
 #ifndef MK_VARIANT
 #define MK_VARIANT base
 #endif
@@ -162,6 +173,14 @@ struct Ctx {
   uint32_t cl_rank, cl_size;  // this CTA's rank in its thread-block cluster, CTAs per cluster
 #endif
   __device__ Ctx(const KParams& p_) : p(p_) {}
+  // Every op starts from values the compiler cannot trace to the kernel's start: else it works out what depends on the
+  // thread's index for all ops ahead of the op loop, and spills it there.
+  __device__ __forceinline__ void opaque() {
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+    lane = tid & 31;
+    warp = tid >> 5;
+    asm volatile("" : "+l"(smem), "+r"(smem_addr), "+r"(tmem));
+  }
   __device__ uint32_t full_bar(int s) const { return smem_addr + p.bar_off + 8 * s; }
   __device__ uint32_t empty_bar(int s) const { return smem_addr + p.bar_off + 8 * (p.num_stages + s); }
   __device__ uint32_t xfull_bar(int s) const { return smem_addr + p.bar_off + 8 * (2 * p.num_stages + s); }
@@ -188,17 +207,20 @@ struct Ctx {
     if ((c).dbg != nullptr && (c).tid == 0) (c).dbg[k] = globaltimer(); \
   } while (0)
 
-__device__ __noinline__ void raise_abort(const Ctx& c, int code, int d0, int d1) {
-  if (atomicCAS(c.p.abort_flag, 0, 1) == 0) {
-    c.p.status[0] = code;
-    c.p.status[1] = blockIdx.x;
-    c.p.status[2] = c.cur_op;
-    c.p.status[3] = c.iter;
-    c.p.status[4] = d0;
-    c.p.status[5] = d1;
-    c.p.status[6] = threadIdx.x;
+__device__ __forceinline__ void raise_abort_at(const KParams* p, int iter, int op, int code, int d0, int d1) {
+  if (atomicCAS(p->abort_flag, 0, 1) == 0) {
+    p->status[0] = code;
+    p->status[1] = blockIdx.x;
+    p->status[2] = op;
+    p->status[3] = iter;
+    p->status[4] = d0;
+    p->status[5] = d1;
+    p->status[6] = threadIdx.x;
     __threadfence();
   }
+}
+__device__ __forceinline__ void raise_abort(const Ctx& c, int code, int d0, int d1) {
+  raise_abort_at(&c.p, c.iter, c.cur_op, code, d0, d1);
 }
 __device__ __forceinline__ bool aborted(const Ctx& c) { return *(volatile int*)c.p.abort_flag != 0; }
 
@@ -208,18 +230,18 @@ __device__ __forceinline__ bool aborted(const Ctx& c) { return *(volatile int*)c
 // Time limits are tiered so that the record names the root cause: a wait on another GPU gives
 // up after timeout_ns, waits on other CTAs or on the producer after twice that, the producers'
 // own waits (on the consumers) after four times.
-__device__ __noinline__ bool mbar_wait_slow(const Ctx& c, uint32_t bar, uint32_t parity, int code) {
+__device__ __forceinline__ bool mbar_wait_slow(const KParams* p, int iter, int op, uint32_t bar, uint32_t parity, int code) {
   unsigned long long t0 = 0;
   unsigned polls = 0;
   while (true) {
     if (mbar_try_wait(bar, parity)) return true;
     if (((++polls) & 4095u) == 0) {
-      if (aborted(c)) return false;
+      if (*(volatile int*)p->abort_flag != 0) return false;
       const unsigned long long now = globaltimer();
       if (t0 == 0) {
         t0 = now;
-      } else if (now - t0 > c.p.timeout_ns * (code == ST_TIMEOUT_EMPTY ? 4ull : 2ull)) {
-        raise_abort(c, code, (int)bar, (int)parity);
+      } else if (now - t0 > p->timeout_ns * (code == ST_TIMEOUT_EMPTY ? 4ull : 2ull)) {
+        raise_abort_at(p, iter, op, code, (int)bar, (int)parity);
         return false;
       }
     }
@@ -230,7 +252,7 @@ __device__ __forceinline__ bool mbar_wait(const Ctx& c, uint32_t bar, uint32_t p
 #pragma unroll 1
   for (int i = 0; i < 256; ++i)
     if (mbar_try_wait(bar, parity)) return true;
-  return mbar_wait_slow(c, bar, parity, code);
+  return mbar_wait_slow(&c.p, c.iter, c.cur_op, bar, parity, code);
 }
 
 // Grid-wide barrier of the consumer warps.  The counter only grows within a launch: barrier
@@ -272,7 +294,7 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint32_t bar, uint32_t par
   return ok != 0;
 }
 // Bounded wait on an mbarrier that CTAs of the same cluster arrive on.
-__device__ __noinline__ bool cluster_bar_wait(const Ctx& c, uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ bool cluster_bar_wait(const Ctx& c, uint32_t bar, uint32_t parity) {
   unsigned long long t0 = 0;
   unsigned polls = 0;
   while (true) {
@@ -390,7 +412,7 @@ __device__ __forceinline__ void grid_wait(Ctx& c) {
   consumer_sync();
 }
 #endif  // MK_HIER_BARRIER
-__device__ __noinline__ void grid_sync(Ctx& c) {
+__device__ __forceinline__ void grid_sync(Ctx& c) {
   if (!c.arrived) grid_arrive(c);
   grid_wait(c);
 }
@@ -460,7 +482,7 @@ __device__ __forceinline__ void xchg_push1(const KParams& p, unsigned seq, int t
   for (int r = 0; r < p.world; ++r) st_sys_v2(reinterpret_cast<uint2*>(p.xchg[r]) + w, __float_as_uint(v), seq);
 }
 // A word of a rank that is not there yet: poll it (bounded).  Returns false after raising the abort flag.
-__device__ __noinline__ bool xchg_wait_word(const Ctx& c, const uint2* w, unsigned seq, int src) {
+__device__ __forceinline__ bool xchg_wait_word(const Ctx& c, const uint2* w, unsigned seq, int src) {
   unsigned long long t0 = 0;
   unsigned spins = 0;
   while (true) {
@@ -478,7 +500,7 @@ __device__ __noinline__ bool xchg_wait_word(const Ctx& c, const uint2* w, unsign
   }
 }
 // 8 consecutive columns (col a multiple of 8) of token row `tok`: the sum over ranks as bf16 x 8
-__device__ __noinline__ uint4 xchg_gather8(const Ctx& c, unsigned seq, int tok, int col) {
+__device__ __forceinline__ uint4 xchg_gather8(const Ctx& c, unsigned seq, int tok, int col) {
   const KParams& p = c.p;
   float acc[8];
 #pragma unroll
@@ -504,7 +526,7 @@ __device__ __noinline__ uint4 xchg_gather8(const Ctx& c, unsigned seq, int tok, 
   return pack8(acc);
 }
 // one column: the bf16-rounded sum over ranks, as a float
-__device__ __noinline__ float xchg_gather1(const Ctx& c, unsigned seq, int tok, int col) {
+__device__ __forceinline__ float xchg_gather1(const Ctx& c, unsigned seq, int tok, int col) {
   const KParams& p = c.p;
   float acc = 0.f;
 #pragma unroll 1
@@ -546,53 +568,58 @@ __device__ __forceinline__ void st_gpu_v2(uint2* p, uint32_t a, uint32_t b) {
 __device__ __forceinline__ bool ll_ok(const uint4& a, const uint4& b, unsigned tag) {
   return a.y == tag && a.w == tag && b.y == tag && b.w == tag;
 }
-// Eight columns whose words have not all arrived: poll them (bounded).  Zeros after the abort flag went up.
-__device__ __noinline__ uint4 ll_wait8(const Ctx& c, const uint4* src, unsigned tag) {
-  unsigned long long t0 = 0;
+// The bound of a poll: true (after raising the abort flag) when the wait has to end without its data.
+struct PollLimit {
   unsigned spins = 0;
-  while (true) {
-    const uint4 a = ld_gpu_v4(src), b = ld_gpu_v4(src + 1);
-    if (ll_ok(a, b, tag)) return make_uint4(a.x, a.z, b.x, b.z);
-    if (((++spins) & 63u) == 0) {
-      if (aborted(c)) return make_uint4(0, 0, 0, 0);
-      const unsigned long long now = globaltimer();
-      if (t0 == 0) {
-        t0 = now;
-      } else if (now - t0 > 2 * c.p.timeout_ns) {
-        raise_abort(c, ST_TIMEOUT_DATA, (int)tag, (int)a.y);
-        return make_uint4(0, 0, 0, 0);
-      }
+  unsigned long long t0 = 0;
+  __device__ __forceinline__ bool expired(const Ctx& c, unsigned tag, unsigned got) {
+    if (((++spins) & 63u) != 0) return false;
+    if (aborted(c)) return true;
+    const unsigned long long now = globaltimer();
+    if (t0 == 0) {
+      t0 = now;
+    } else if (now - t0 > 2 * c.p.timeout_ns) {
+      raise_abort(c, ST_TIMEOUT_DATA, (int)tag, (int)got);
+      return true;
     }
+    return false;
   }
-}
-__device__ __forceinline__ uint4 ll_take8(const Ctx& c, const uint4* src, const uint4& a, const uint4& b, unsigned tag) {
-  return ll_ok(a, b, tag) ? make_uint4(a.x, a.z, b.x, b.z) : ll_wait8(c, src, tag);
-}
-// eight columns from column `col` (a multiple of 8) of the row that starts at word `row`
-__device__ __forceinline__ uint4 ll_gather8(const Ctx& c, const uint2* row, int col, unsigned tag) {
-  const uint4* src = reinterpret_cast<const uint4*>(row + (col >> 1));
-  const uint4 a = ld_gpu_v4(src), b = ld_gpu_v4(src + 1);
-  return ll_take8(c, src, a, b, tag);
+};
+// N vectors of eight columns: vector i from src + 2 at[i] where at[i] >= 0, else zeros.  All loads first, then whatever
+// has not arrived is loaded again, all of it per trip: one loop, where a poll per vector was as many copies of its code
+// (inlined) or as many calls.
+template <int N>
+__device__ __forceinline__ void ll_take(const Ctx& c, const uint4* src, const int (&at)[N], unsigned tag, uint4 (&out)[N]) {
+  uint4 a[N], b[N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const unsigned t = at[i] >= 0 ? ~tag : tag;  // (nothing to wait for: zeros that carry the tag)
+    a[i] = b[i] = make_uint4(0u, t, 0u, t);
+  }
+  PollLimit limit;
+  while (true) {
+#pragma unroll
+    for (int i = 0; i < N; ++i)
+      if (!ll_ok(a[i], b[i], tag)) {
+        a[i] = ld_gpu_v4(src + 2 * at[i]);
+        b[i] = ld_gpu_v4(src + 2 * at[i] + 1);
+      }
+    bool here = true;
+#pragma unroll
+    for (int i = 0; i < N; ++i) here = here && ll_ok(a[i], b[i], tag);
+    if (here || limit.expired(c, tag, a[0].y)) break;
+  }
+#pragma unroll
+  for (int i = 0; i < N; ++i) out[i] = make_uint4(a[i].x, a[i].z, b[i].x, b[i].z);
 }
 // one column, as a float
-__device__ __noinline__ float ll_gather1(const Ctx& c, const uint2* row, int col, unsigned tag) {
+__device__ __forceinline__ float ll_gather1(const Ctx& c, const uint2* row, int col, unsigned tag) {
   const uint2* w = row + (col >> 1);
-  unsigned long long t0 = 0;
-  unsigned spins = 0;
-  while (true) {
-    const uint2 q = ld_gpu_v2(w);
-    if (q.y == tag) return (col & 1) ? bf_hi(q.x) : bf_lo(q.x);
-    if (((++spins) & 63u) == 0) {
-      if (aborted(c)) return 0.f;
-      const unsigned long long now = globaltimer();
-      if (t0 == 0) {
-        t0 = now;
-      } else if (now - t0 > 2 * c.p.timeout_ns) {
-        raise_abort(c, ST_TIMEOUT_DATA, (int)tag, (int)q.y);
-        return 0.f;
-      }
-    }
-  }
+  PollLimit limit;
+  uint2 q;
+  do q = ld_gpu_v2(w);
+  while (q.y != tag && !limit.expired(c, tag, q.y));
+  return (col & 1) ? bf_hi(q.x) : bf_lo(q.x);
 }
 __device__ __forceinline__ const uint2* ll_row(const void* base, int ld, int tok) {
   return reinterpret_cast<const uint2*>(base) + (size_t)tok * (size_t)(ld >> 1);
@@ -606,7 +633,7 @@ __device__ __forceinline__ unsigned ll_tag_of(const Ctx& c, int op) { return ll_
 // its own slice of the columns, in rank order in fp32 with one bf16 rounding (the same value on every
 // rank), and stores it as tagged words; all CTAs then stage the row from those words like any other
 // tagged input: two round trips whatever the number of ranks.
-__device__ __noinline__ void xchg_reduce_slice(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void xchg_reduce_slice(Ctx& c, const OpDesc& op, int T) {
   const KParams& p = c.p;
   const int pairs = op.k >> 1;
   const int p0 = (int)((long long)blockIdx.x * pairs / gridDim.x), p1 = (int)((long long)(blockIdx.x + 1) * pairs / gridDim.x);
@@ -643,7 +670,7 @@ __device__ __noinline__ void xchg_reduce_slice(Ctx& c, const OpDesc& op, int T) 
 #endif
 
 // ------------------------------------------------------------------------------------
-__device__ __noinline__ float torch_rsqrt_bf16(float var, bool dbl);
+__device__ __forceinline__ float torch_rsqrt_bf16(float var, bool dbl);
 
 // activations -> shared memory, with the optional fused RMSNorm
 // ------------------------------------------------------------------------------------
@@ -792,7 +819,7 @@ __device__ __forceinline__ void stage_row_regs(Ctx& c, const uint4* src, uint4* 
 }
 
 // `gather`: the rows are not read from `in` but summed over the ranks' slots of the latest exchange.
-__device__ __noinline__ void stage_x(Ctx& c, const void* in, int ld_in, int K, int kp, const void* norm_w, int tok0,
+__device__ __forceinline__ void stage_x(Ctx& c, const void* in, int ld_in, int K, int kp, const void* norm_w, int tok0,
                                      int rows, int T, const uint4* pre_w, bool gather = false, void* sums_out = nullptr) {
   if (!MK_WITH_XCHG) gather = false;  // (compiled out of the single-GPU build)
   uint4* xs = reinterpret_cast<uint4*>(c.smem + c.p.x_off);
@@ -867,7 +894,7 @@ __device__ __noinline__ void stage_x(Ctx& c, const void* in, int ld_in, int K, i
 // its first tile.  Lane l takes the 16-byte chunk (l & 7) of the slices of stages (l >> 3) + 4 i.
 // (The same scheme with the norm fused in was 0.36 ms per step SLOWER: its unrolled scaling code
 // is several KB that every op would run once, out of a cold instruction cache.)
-__device__ __noinline__ void stage_x_rows(Ctx& c, const void* in, int ld_in, int K, int kp, int tok0, int rows, int T) {
+__device__ __forceinline__ void stage_x_rows(Ctx& c, const void* in, int ld_in, int K, int kp, int tok0, int rows, int T) {
   constexpr int kMaxV = 6;  // 24 stages / 4 per round
   uint4* xs = reinterpret_cast<uint4*>(c.smem + c.p.x_off);
   const int pitch = (kp >> 3) + 1;  // uint4 per row
@@ -905,19 +932,11 @@ __device__ __forceinline__ void stage_ll_regs(Ctx& c, const uint4* ll, uint4* ds
   const int kvec = K >> 3;
   const bool torch_num = c.p.numerics == NUM_TORCH;
   float* red = c.red();
-  uint4 qa[NV], qb[NV], raw[NV];
+  uint4 raw[NV];
+  int at[NV];
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int v = v0 + vstep * i;
-    const bool ok = valid && v < kvec;
-    qa[i] = ok ? ld_gpu_v4(ll + 2 * v) : make_uint4(0, 0, 0, 0);
-    qb[i] = ok ? ld_gpu_v4(ll + 2 * v + 1) : make_uint4(0, 0, 0, 0);
-  }
-#pragma unroll
-  for (int i = 0; i < NV; ++i) {
-    const int v = v0 + vstep * i;
-    raw[i] = (valid && v < kvec) ? ll_take8(c, ll + 2 * v, qa[i], qb[i], tag) : make_uint4(0, 0, 0, 0);
-  }
+  for (int i = 0; i < NV; ++i) at[i] = valid && v0 + vstep * i < kvec ? v0 + vstep * i : -1;
+  ll_take(c, ll, at, tag, raw);
   float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < NV; ++i) ss = sumsq8(raw[i], torch_num, ss);
@@ -936,7 +955,7 @@ __device__ __forceinline__ void stage_ll_regs(Ctx& c, const uint4* ll, uint4* ds
   consumer_sync();
 }
 // fused norm; the host only plans it for rows of at most four vectors per lane
-__device__ __noinline__ void stage_x_ll(Ctx& c, const void* ll_in, int ld_in, int K, int kp, const void* norm_w, int tok0,
+__device__ __forceinline__ void stage_x_ll(Ctx& c, const void* ll_in, int ld_in, int K, int kp, const void* norm_w, int tok0,
                                         int rows, int T, const uint4* pre_w, unsigned tag) {
   uint4* xs = reinterpret_cast<uint4*>(c.smem + c.p.x_off);
   const int pitch = (kp >> 3) + 1;
@@ -955,7 +974,7 @@ __device__ __noinline__ void stage_x_ll(Ctx& c, const void* ll_in, int ld_in, in
   else stage_ll_regs<4>(c, ll, dst, pre_w, wv, K, nvec, v0, vstep, active, valid, tb * wpr, wpr, tag);
 }
 // no norm: every warp stages the k slices it multiplies (see stage_x_rows)
-__device__ __noinline__ void stage_rows_ll(Ctx& c, const void* ll_in, int ld_in, int K, int kp, int tok0, int rows, int T, unsigned tag) {
+__device__ __forceinline__ void stage_rows_ll(Ctx& c, const void* ll_in, int ld_in, int K, int kp, int tok0, int rows, int T, unsigned tag) {
   constexpr int kMaxV = 6;
   uint4* xs = reinterpret_cast<uint4*>(c.smem + c.p.x_off);
   const int pitch = (kp >> 3) + 1;
@@ -967,19 +986,14 @@ __device__ __noinline__ void stage_rows_ll(Ctx& c, const void* ll_in, int ld_in,
   for (int t = 0; t < rows; ++t) {
     const bool live = tok0 + t < T;
     const uint4* ll = reinterpret_cast<const uint4*>(ll_row(ll_in, ld_in, live ? tok0 + t : 0));
-    uint4 qa[kMaxV], qb[kMaxV];
+    uint4 raw[kMaxV];
+    int at[kMaxV];
 #pragma unroll
-    for (int i = 0; i < kMaxV; ++i) {
-      const int v = v0 + i * vstep;
-      const bool ok = live && v < kvec;
-      qa[i] = ok ? ld_gpu_v4(ll + 2 * v) : make_uint4(0, 0, 0, 0);
-      qb[i] = ok ? ld_gpu_v4(ll + 2 * v + 1) : make_uint4(0, 0, 0, 0);
-    }
+    for (int i = 0; i < kMaxV; ++i) at[i] = live && v0 + i * vstep < kvec ? v0 + i * vstep : -1;
+    ll_take(c, ll, at, tag, raw);
 #pragma unroll
-    for (int i = 0; i < kMaxV; ++i) {
-      const int v = v0 + i * vstep;
-      if (v < nvec) xs[t * pitch + v] = (live && v < kvec) ? ll_take8(c, ll + 2 * v, qa[i], qb[i], tag) : make_uint4(0, 0, 0, 0);
-    }
+    for (int i = 0; i < kMaxV; ++i)
+      if (v0 + i * vstep < nvec) xs[t * pitch + v0 + i * vstep] = raw[i];
   }
   __syncwarp();
 }
@@ -1045,7 +1059,7 @@ __device__ __forceinline__ int rows_num_chunks(int row0, int row1) { return (row
 __device__ __forceinline__ int rows_chunk_begin(int row0, int row1, int nch, int ci) {
   return row0 + kUnitRows * (ci * ((row1 - row0) / kUnitRows) / nch);
 }
-__device__ __noinline__ void linear_pass_rows(Ctx& c, const OpDesc& op, int tok0, int T, const uint4* pre_w) {
+__device__ __forceinline__ void linear_pass_rows(Ctx& c, const OpDesc& op, int tok0, int T, const uint4* pre_w) {
   const KParams& p = c.p;
   const int nks = op.nkt;
   const int kp = nks * kRowsStageK;
@@ -1217,7 +1231,7 @@ __device__ __noinline__ void linear_pass_rows(Ctx& c, const OpDesc& op, int tok0
   c.cons_idx += consumed;
 }
 
-__device__ void op_linear_rows(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void op_linear_rows(Ctx& c, const OpDesc& op, int T) {
   // the norm weights do not depend on other CTAs: fetched ahead of the barrier
   uint4 pre_w[4] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
   const int wpr0 = stage_warps_per_row(min(op.aux3, T));
@@ -1262,7 +1276,7 @@ __device__ void op_linear_rows(Ctx& c, const OpDesc& op, int T) {
 
 // bf16 reciprocal square root the way the reference PyTorch model's CPU kernels round it:
 // `dbl` = scalar loop (sqrt rounded to bf16 before the reciprocal), else vector loop.
-__device__ __noinline__ float torch_rsqrt_bf16(float var, bool dbl) {
+__device__ __forceinline__ float torch_rsqrt_bf16(float var, bool dbl) {
   return dbl ? rbf(1.0f / rbf(sqrtf(var))) : rbf(1.0f / sqrtf(var));
 }
 
@@ -1271,7 +1285,7 @@ __device__ __noinline__ float torch_rsqrt_bf16(float var, bool dbl) {
 struct F8 {
   float v[8];
 };
-__device__ __noinline__ F8 head_norm_rope(F8 xin, uint4 wv, uint4 csv, uint4 snv, int l16, int flags, int numerics,
+__device__ __forceinline__ F8 head_norm_rope(F8 xin, uint4 wv, uint4 csv, uint4 snv, int l16, int flags, int numerics,
                                           bool dbl) {
   float* x = xin.v;
   if (flags & F_QK_NORM) {
@@ -1406,7 +1420,7 @@ __device__ __forceinline__ void attn_prepare(const Ctx& c, const OpDesc& op, con
 // handful of CTAs per layer ever run it.  One round of loads: every thread fetches, for its
 // output elements, the chunks' values together with their (max, sum) pairs and rescales as it
 // goes, eight chunks at a time (more loads in flight per thread measured slower).
-__device__ __noinline__ void attn_merge(Ctx& c, const float* base, __nv_bfloat16* out, int nch, int qpk, int part_stride,
+__device__ __forceinline__ void attn_merge(Ctx& c, const float* base, __nv_bfloat16* out, int nch, int qpk, int part_stride,
                                         uint2* ll_out, unsigned tag) {
   const int nout = qpk * kHeadDim;
   constexpr int kMergeBatch = 8;
@@ -1473,25 +1487,7 @@ __device__ __noinline__ void attn_merge(Ctx& c, const float* base, __nv_bfloat16
 // words of all chunks it needs: no atomic round trip, no last arriver doing all of it, one output per
 // thread.  (A CTA stores its own partial before it waits for any other, and the chunks of one pair are
 // consecutive tasks, so a wait never depends on a later task of the waiting CTA.)
-__device__ __noinline__ float ll_wait_word(const Ctx& c, const uint2* w, unsigned tag) {
-  unsigned long long t0 = 0;
-  unsigned spins = 0;
-  while (true) {
-    const uint2 q = ld_gpu_v2(w);
-    if (q.y == tag) return __uint_as_float(q.x);
-    if (((++spins) & 63u) == 0) {
-      if (aborted(c)) return 0.f;
-      const unsigned long long now = globaltimer();
-      if (t0 == 0) {
-        t0 = now;
-      } else if (now - t0 > 2 * c.p.timeout_ns) {
-        raise_abort(c, ST_TIMEOUT_DATA, (int)tag, (int)q.y);
-        return 0.f;
-      }
-    }
-  }
-}
-__device__ __noinline__ void attn_merge_ll(Ctx& c, const uint2* base, __nv_bfloat16* out, uint2* ll_out, int nch, int ch, int qpk,
+__device__ __forceinline__ void attn_merge_ll(Ctx& c, const uint2* base, __nv_bfloat16* out, uint2* ll_out, int nch, int ch, int qpk,
                                            int part_stride, unsigned tag) {
   const int nout = qpk * kHeadDim;
   const int S = (((nout + nch - 1) / nch) + 1) & ~1;  // outputs per chunk CTA, even: a bf16 pair never straddles two slices
@@ -1511,25 +1507,30 @@ __device__ __noinline__ void attn_merge_ll(Ctx& c, const uint2* base, __nv_bfloa
         uint2 qv[kBatch], qm[kBatch], ql[kBatch];
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
-          const bool ok = c0 + u < nch;
-          const size_t off = (size_t)(ok ? c0 + u : c0) * part_stride;
-          qv[u] = ld_gpu_v2(pv + off);
-          qm[u] = ld_gpu_v2(pm + off);
-          ql[u] = ld_gpu_v2(pm + off + qpk);
+          const unsigned t = c0 + u < nch ? ~tag : tag;
+          qv[u] = ql[u] = make_uint2(0u, t);
+          qm[u] = make_uint2(0xff800000u, t);  // (-inf)
+        }
+        PollLimit limit;
+        while (true) {
+          bool here = true;
+#pragma unroll
+          for (int u = 0; u < kBatch; ++u) {
+            const size_t off = (size_t)(c0 + u) * part_stride;
+            if (qv[u].y != tag) qv[u] = ld_gpu_v2(pv + off);
+            if (qm[u].y != tag) qm[u] = ld_gpu_v2(pm + off);
+            if (ql[u].y != tag) ql[u] = ld_gpu_v2(pm + off + qpk);
+          }
+#pragma unroll
+          for (int u = 0; u < kBatch; ++u) here = here && qv[u].y == tag && qm[u].y == tag && ql[u].y == tag;
+          if (here || limit.expired(c, tag, qv[0].y)) break;
         }
         float v[kBatch], mm[kBatch], ll[kBatch];
 #pragma unroll
         for (int u = 0; u < kBatch; ++u) {
-          const bool ok = c0 + u < nch;
-          const size_t off = (size_t)(ok ? c0 + u : c0) * part_stride;
-          v[u] = qv[u].y == tag ? __uint_as_float(qv[u].x) : ll_wait_word(c, pv + off, tag);
-          mm[u] = qm[u].y == tag ? __uint_as_float(qm[u].x) : ll_wait_word(c, pm + off, tag);
-          ll[u] = ql[u].y == tag ? __uint_as_float(ql[u].x) : ll_wait_word(c, pm + off + qpk, tag);
-          if (!ok) {
-            v[u] = 0.f;
-            mm[u] = -INFINITY;
-            ll[u] = 0.f;
-          }
+          v[u] = __uint_as_float(qv[u].x);
+          mm[u] = __uint_as_float(qm[u].x);
+          ll[u] = __uint_as_float(ql[u].x);
         }
         float Mb = M;
 #pragma unroll
@@ -1660,7 +1661,7 @@ __device__ __forceinline__ void attn_l2_ahead(const Ctx& c, const OpDesc& op, co
 // the token's own position in the cache; a second grid barrier makes all of them visible.  Returns true
 // when the launch is aborting.  (Both halves of a warp compute the same pair: the shuffles in
 // head_norm_rope use the full mask.)
-__device__ __noinline__ bool attn_barrier_then_append(Ctx& c, const OpDesc& op, const AttnPlan& pl, const int* lens, int T) {
+__device__ __forceinline__ bool attn_barrier_then_append(Ctx& c, const OpDesc& op, const AttnPlan& pl, const int* lens, int T) {
   const KParams& p = c.p;
   if (op.flags & F_SYNC_BEFORE) {
     grid_wait(c);
@@ -1705,7 +1706,7 @@ __device__ __noinline__ bool attn_barrier_then_append(Ctx& c, const OpDesc& op, 
 }
 
 // aux0 = kv heads, aux1 = q heads (q heads per kv head: 1, 2, 4 or 8).  The row-owner path's attention: one or two tokens.
-__device__ __noinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
   const KParams& p = c.p;
   const int G = gridDim.x;
   MK_STAMP(c, 0);
@@ -1851,23 +1852,13 @@ __device__ __noinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
       ncs = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.cos) + (size_t)pos * kHeadDim) + l16);
       nsn = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.sin) + (size_t)pos * kHeadDim) + l16);
     }
-    if (ll_in) {  // all loads first, then whatever has not arrived is polled
-      const uint4* sv = reinterpret_cast<const uint4*>(llr + (((pl.qpk + 1) * kHeadDim + l16 * 8) >> 1));
-      const uint4* sq = reinterpret_cast<const uint4*>(llr + ((c.warp * kHeadDim + l16 * 8) >> 1));
-      const uint4* sk = reinterpret_cast<const uint4*>(llr + ((pl.qpk * kHeadDim + l16 * 8) >> 1));
-      const uint4 v0 = ld_gpu_v4(sv), v1 = ld_gpu_v4(sv + 1);
-      uint4 q0 = v0, q1 = v1, k0 = v0, k1 = v1;
-      if (do_q) {
-        q0 = ld_gpu_v4(sq);
-        q1 = ld_gpu_v4(sq + 1);
-      }
-      if (do_k) {
-        k0 = ld_gpu_v4(sk);
-        k1 = ld_gpu_v4(sk + 1);
-      }
-      vnew = ll_take8(c, sv, v0, v1, tag_in);
-      if (do_q) xq = ll_take8(c, sq, q0, q1, tag_in);
-      if (do_k) xk = ll_take8(c, sk, k0, k1, tag_in);
+    if (ll_in) {
+      const int at[3] = {(pl.qpk + 1) * (kHeadDim / 8) + l16, do_q ? c.warp * (kHeadDim / 8) + l16 : -1, do_k ? pl.qpk * (kHeadDim / 8) + l16 : -1};
+      uint4 got[3];
+      ll_take(c, reinterpret_cast<const uint4*>(llr), at, tag_in, got);
+      vnew = got[0];
+      xq = got[1];
+      xk = got[2];
     } else {
       vnew = __ldcg(reinterpret_cast<const uint4*>(row + (pl.qpk + 1) * kHeadDim) + l16);
       if (do_q) xq = __ldcg(reinterpret_cast<const uint4*>(row + c.warp * kHeadDim) + l16);
@@ -1993,7 +1984,7 @@ __device__ __noinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
 // small ops
 // ------------------------------------------------------------------------------------
 // aux0 = embedding rows
-__device__ void op_embed(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void op_embed(Ctx& c, const OpDesc& op, int T) {
   const int nseg = (op.n + 2047) / 2048;
   const long long* ids = reinterpret_cast<const long long*>(op.in);
   for (int u = blockIdx.x; u < T * nseg; u += gridDim.x) {
@@ -2012,7 +2003,7 @@ __device__ void op_embed(Ctx& c, const OpDesc& op, int T) {
 }
 
 // A row that is too wide for shared memory: read once for its sum of squares (in stage_x's order) and once to be scaled.
-__device__ __noinline__ void rmsnorm_wide_row(Ctx& c, const OpDesc& op, int tok) {
+__device__ __forceinline__ void rmsnorm_wide_row(Ctx& c, const OpDesc& op, int tok) {
   const bool torch_num = c.p.numerics == NUM_TORCH;
   const int kvec = op.n >> 3;
   const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)tok * op.ld_in);
@@ -2031,7 +2022,7 @@ __device__ __noinline__ void rmsnorm_wide_row(Ctx& c, const OpDesc& op, int tok)
   consumer_sync();
 }
 
-__device__ void op_rmsnorm(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void op_rmsnorm(Ctx& c, const OpDesc& op, int T) {
   const int kp = ((op.n + 63) / 64) * 64;
   // the norm weights do not depend on other CTAs: a CTA that has a row fetches them ahead of the barrier
   uint4 pre_w[4] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
@@ -2062,7 +2053,7 @@ __device__ void op_rmsnorm(Ctx& c, const OpDesc& op, int T) {
 }
 
 // aux0 = columns per [gate | up] block of the input
-__device__ void op_silu_mul(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void op_silu_mul(Ctx& c, const OpDesc& op, int T) {
   const int bk = op.aux0;
   const int nvec = op.n >> 3;
   const __nv_bfloat16* in = reinterpret_cast<const __nv_bfloat16*>(op.in);
@@ -2081,7 +2072,7 @@ __device__ void op_silu_mul(Ctx& c, const OpDesc& op, int T) {
   }
 }
 
-__device__ ArgBest block_argmax(Ctx& c, ArgBest b) {
+__device__ __forceinline__ ArgBest block_argmax(Ctx& c, ArgBest b) {
   float* scratch = c.red() + 32;
   b = warp_argmax(b);
   if (c.lane == 0) {
@@ -2103,7 +2094,7 @@ __device__ ArgBest block_argmax(Ctx& c, ArgBest b) {
 }
 
 // logits [T][n] -> amax_n partial (value, index) pairs per token
-__device__ void op_argmax_partial(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void op_argmax_partial(Ctx& c, const OpDesc& op, int T) {
   const int np = op.amax_n;
   const int chunk = (op.n + np - 1) / np;
   const __nv_bfloat16* in = reinterpret_cast<const __nv_bfloat16*>(op.in);
@@ -2183,7 +2174,7 @@ __device__ __forceinline__ ArgBest argmax_scan(const OpDesc& op, int tok, int i0
 // Up to 8 tokens CTA 0 reduces them all, a warp per token: it also runs the bookkeeping that reads the result, so
 // nothing has to cross CTAs.  (All warps on one token after the other took 12 us for 8 tokens.)  Larger batches are
 // spread over the grid (one token per CTA at a time) and pay one more grid barrier so that CTA 0 sees every token.
-__device__ void op_argmax_reduce(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void op_argmax_reduce(Ctx& c, const OpDesc& op, int T) {
   const bool spread = T > kNumConsumerWarps;
   if (spread) {
     for (int tok = blockIdx.x; tok < T; tok += gridDim.x) {
@@ -2225,7 +2216,7 @@ __device__ void op_argmax_reduce(Ctx& c, const OpDesc& op, int T) {
 // over them in that order, however the logits arrive (a word holds two neighbouring experts, so two lanes poll it; polled
 // once and handed over by shuffles, the layer's gate/up op took 22.9 instead of 22.0 us).  A round is two warp-wide
 // integer reductions (a probability's bits grow with it), not five levels of shuffles of (value, index).
-__device__ __noinline__ void moe_route_token(Ctx& c, const __nv_bfloat16* logits, const uint2* words, unsigned tag, int E, int K, float* w_out,
+__device__ __forceinline__ void moe_route_token(Ctx& c, const __nv_bfloat16* logits, const uint2* words, unsigned tag, int E, int K, float* w_out,
                                              int* idx_out, float* w_out2, int* idx_out2) {
   float v[8];  // up to 256 experts, 8 per lane
   if (words != nullptr) {
@@ -2311,7 +2302,7 @@ __device__ __noinline__ void moe_route_token(Ctx& c, const __nv_bfloat16* logits
     if (idx_out2 != nullptr) idx_out2[c.lane] = my_e;
   }
 }
-__device__ __noinline__ void op_moe_route(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void op_moe_route(Ctx& c, const OpDesc& op, int T) {
   const int E = op.aux1, K = op.aux0;
   const __nv_bfloat16* in = reinterpret_cast<const __nv_bfloat16*>(op.in);
 #pragma unroll 1
@@ -2343,32 +2334,29 @@ __device__ __forceinline__ float* moe_route_weights(const Ctx& c) { return reint
 
 // `rows` tagged rows of K columns -> shared memory rows of pitch kp + 8, zero padded, by all consumers: four 8-column
 // pieces of a thread in flight, then whatever has not arrived is polled.
-__device__ __noinline__ void stage_ll_pairs(Ctx& c, const uint2* base, int ld, int rows, int K, int kp, unsigned tag) {
+__device__ __forceinline__ void stage_ll_pairs(Ctx& c, const uint2* base, int ld, int rows, int K, int kp, unsigned tag) {
   uint4* xs = reinterpret_cast<uint4*>(c.smem + c.p.x_off);
   const int pitch = (kp >> 3) + 1, nvec = kp >> 3, kvec = K >> 3, total = rows * nvec;
   if (c.tid == 0) xs[rows * pitch] = make_uint4(0, 0, 0, 0);  // the chunk absent columns of the mma point at
 #pragma unroll 1
   for (int i0 = c.tid; i0 < total; i0 += 4 * kNumConsumers) {
-    uint4 qa[4], qb[4];
-    const uint4* src[4];
-    int dst[4];
+    uint4 got[4];
+    int at[4], dst[4];  // (in 16-byte vectors of eight columns: a row of words is ld / 8 of them)
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int i = i0 + u * kNumConsumers, r = i / nvec, v = i - r * nvec;
-      const bool ok = i < total && v < kvec;
       dst[u] = i < total ? r * pitch + v : -1;
-      src[u] = ok ? reinterpret_cast<const uint4*>(base + (size_t)r * (size_t)(ld >> 1)) + 2 * v : nullptr;
-      qa[u] = ok ? ld_gpu_v4(src[u]) : make_uint4(0, 0, 0, 0);
-      qb[u] = ok ? ld_gpu_v4(src[u] + 1) : make_uint4(0, 0, 0, 0);
+      at[u] = i < total && v < kvec ? r * (ld >> 3) + v : -1;
     }
+    ll_take(c, reinterpret_cast<const uint4*>(base), at, tag, got);
 #pragma unroll
     for (int u = 0; u < 4; ++u)
-      if (dst[u] >= 0) xs[dst[u]] = src[u] != nullptr ? ll_take8(c, src[u], qa[u], qb[u], tag) : make_uint4(0, 0, 0, 0);
+      if (dst[u] >= 0) xs[dst[u]] = got[u];
   }
   consumer_sync();
 }
 
-__device__ __noinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, int T);
+__device__ __forceinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, int T);
 
 // aux0 = top-k, aux1 = experts, n = rows per expert, k = K.  w: [experts * n, K] bf16 (tmap_w: the four maps of
 // the row-owner path over that 2-D view).  in: [T, K] (one row per token) or, with F_MOE_PAIR_IN, [T * top-k, K];
@@ -2378,7 +2366,7 @@ __device__ __noinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, int T
 // SiLU(gate) * up -> out2 [T * top-k, inter]; the activation layer behind it has nothing left to do.
 // F_LL_IN (gate/up): no barrier.  The rows (ll_in) and the router logits (ll_res) arrive as tagged words; the rows are
 // staged and normalised while the router linear is still at work.
-__device__ __noinline__ void op_moe_linear(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void op_moe_linear(Ctx& c, const OpDesc& op, int T) {
   const KParams& p = c.p;
   const bool ll = (op.flags & F_LL_IN) != 0;
   if (ll) {  // (no look at the abort flag either: the polls and the stage waits watch it)
@@ -2543,7 +2531,7 @@ __device__ __noinline__ void op_moe_linear(Ctx& c, const OpDesc& op, int T) {
 // like the linear's output would be, and adds them up slot by slot exactly as the stand-alone weighted sum does
 // (bf16 roundings of the PyTorch model, or fp32 fused multiply-adds), + residual.  The per-slot sums of the warps
 // alternate between the two token slots of the sums block, so that one CTA-wide sync per slot is enough.
-__device__ __noinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, int T) {
   const KParams& p = c.p;
   const int topk = op.aux0;
   int row0, row1;
@@ -2661,7 +2649,7 @@ __device__ __noinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, int T
 // aux0 = top-k.  in: [T * top-k, n] bf16, amax_val: routing weights [T, top-k], res: [T, n] (may be null), out: [T, n].
 // out[t] = bf16( sum over the token's slots of weight * in[pair] ) + residual  (reference task mul_sum_add_sm100.cuh:17-48;
 // the PyTorch model adds the slots up in bf16 and the residual in bf16)
-__device__ void op_moe_combine(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void op_moe_combine(Ctx& c, const OpDesc& op, int T) {
   const int topk = op.aux0;
   const int nvec = op.n >> 3;
   const __nv_bfloat16* in = reinterpret_cast<const __nv_bfloat16*>(op.in);
@@ -2702,7 +2690,7 @@ __device__ void op_moe_combine(Ctx& c, const OpDesc& op, int T) {
 // cannot fold the exchange into the producing linear's epilogue and the consumers' input staging
 // (F_PUSH / F_GATHER_*).  Same exchange words as there: every unit of 8 columns is pushed to all
 // ranks and then gathered from this rank's own region by the same thread.
-__device__ __noinline__ void op_allreduce(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void op_allreduce(Ctx& c, const OpDesc& op, int T) {
   const KParams& p = c.p;
   if (op_barrier(c, op)) return;
   const int world = op.aux0;
@@ -2746,8 +2734,7 @@ __device__ __noinline__ void op_allreduce(Ctx& c, const OpDesc& op, int T) {
 // that a launch bounded by max_iters still appends its last tokens before it ends.
 // Part 1, after an iteration: append the sampled tokens, advance step[], retire
 // finished requests and return their pages.
-__device__ __noinline__ void bookkeep_finish(Ctx& c) {
-  const KParams& p = c.p;
+__device__ __forceinline__ void bookkeep_finish(const KParams& p) {
   const int R = p.max_reqs;
   int tail = p.sched[1];
   for (int i = 0; i < R; ++i) {
@@ -2779,12 +2766,11 @@ __device__ __noinline__ void bookkeep_finish(Ctx& c) {
 
 // Part 2, before an iteration: compact the surviving requests, give each one more
 // token and the page it needs, admit new requests.  Returns the active tokens.
-__device__ __noinline__ int bookkeep_prepare(Ctx& c) {
-  const KParams& p = c.p;
+__device__ __forceinline__ int bookkeep_prepare(const KParams& p, int* table, int iter) {
   const int R = p.max_reqs;
   int head = p.sched[0], tail = p.sched[1];
   const int n_old = p.kv_indptr[R];
-  int* old_idx = n_old <= p.page_entries ? reinterpret_cast<int*>(c.smem + p.x_off) : p.page_scratch;
+  int* old_idx = n_old <= p.page_entries ? table : p.page_scratch;
   for (int i = 0; i < n_old; ++i) old_idx[i] = p.kv_indices[i];
   int nreq = 0, ntok = 0, npages = 0;
   for (int i = 0; i < R; ++i) {
@@ -2808,7 +2794,7 @@ __device__ __noinline__ int bookkeep_prepare(Ctx& c) {
     for (int j = 0; j < have; ++j) p.kv_indices[npages + j] = old_idx[k0 + j];
     for (int j = have; j < need; ++j) {
       if (tail - head <= 0) {
-        raise_abort(c, ST_OUT_OF_PAGES, rid, need);
+        raise_abort_at(&p, iter, -1, ST_OUT_OF_PAGES, rid, need);
         return 0;
       }
       p.kv_indices[npages + j] = p.page_queue[head % p.max_pages];
@@ -2933,7 +2919,7 @@ __device__ __forceinline__ void rows_cursor_next(const KParams& p, RowsCursor& r
 // activation-producer warp: the stages the ring will load next are requested into L2 line by
 // line with plain prefetch instructions, so that HBM keeps streaming while the consumers sit
 // in a barrier or stage their inputs, and the ring refills from L2 when they come back.
-__device__ __noinline__ void rows_prefetch_loop(Ctx& c) {
+__device__ __forceinline__ void rows_prefetch_loop(Ctx& c) {
   const KParams& p = c.p;
   if (p.prefetch_tiles <= 0) return;
   const unsigned W = (unsigned)p.prefetch_tiles;
@@ -2968,7 +2954,7 @@ __device__ __noinline__ void rows_prefetch_loop(Ctx& c) {
 }
 
 template <int PATH>
-__device__ __noinline__ void producer_loop(Ctx& c) {
+__device__ __forceinline__ void producer_loop(Ctx& c) {
   const KParams& p = c.p;
   const int S = p.num_stages;
   volatile int* fl = c.flags();
@@ -3196,7 +3182,7 @@ __device__ __noinline__ void producer_loop(Ctx& c) {
 // The activation producer of the wide path (warp 9, one lane).  It walks the same tile sequence
 // as the weight producer and adds the input boxes to every stage, but only after the consumers
 // have passed the op's barrier: unlike weights, activations are the previous op's output.
-__device__ __noinline__ void xproducer_loop(Ctx& c) {
+__device__ __forceinline__ void xproducer_loop(Ctx& c) {
   const KParams& p = c.p;
   const int S = p.num_stages;
   volatile int* fl = c.flags();
@@ -3259,8 +3245,8 @@ __device__ __noinline__ void xproducer_loop(Ctx& c) {
 // ------------------------------------------------------------------------------------
 // the kernel
 // ------------------------------------------------------------------------------------
-template <int PATH>
-__global__ void __launch_bounds__(PATH == PATH_WIDE ? kWideThreads : kNumThreads, 1) megakernel(const __grid_constant__ KParams p) {
+template <int PATH, int NC>
+__global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_constant__ KParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // The parameters are read from shared memory: behind a reference they are generic loads, and the L1 left beside the
   // ring (28 KB on the wide path) does not hold them from op to op.  Measured, 12 layers of 8B width: 1.765 -> 1.720 ms
@@ -3342,22 +3328,24 @@ __global__ void __launch_bounds__(PATH == PATH_WIDE ? kWideThreads : kNumThreads
     c.tmem = *reinterpret_cast<volatile uint32_t*>(c.smem + p.bar_off + 24 * p.num_stages + 72);
   }
 
-  if (c.warp == kNumConsumerWarps) {
-    if (c.lane == 0) producer_loop<PATH>(c);
-    __syncwarp();
-  } else if (c.warp == kNumConsumerWarps + 1) {
-    if constexpr (PATH == PATH_ROWS) {
-      rows_prefetch_loop(c);
-    } else {
-      if (c.lane == 0) xproducer_loop(c);
-    }
-    __syncwarp();
-  } else if (PATH == PATH_WIDE && c.warp == kNumConsumerWarps + 2) {
-    if constexpr (PATH == PATH_WIDE) {
-      if (c.lane == 0) mma_loop(c);
+  if (c.warp >= kNumConsumerWarps) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kServiceRegs));
+    if (c.warp == kNumConsumerWarps) {
+      if (c.lane == 0) producer_loop<PATH>(c);
+    } else if (c.warp == kNumConsumerWarps + 1) {
+      if constexpr (PATH == PATH_ROWS) {
+        rows_prefetch_loop(c);
+      } else {
+        if (c.lane == 0) xproducer_loop(c);
+      }
+    } else if (PATH == PATH_WIDE && c.warp == kNumConsumerWarps + 2) {
+      if constexpr (PATH == PATH_WIDE) {
+        if (c.lane == 0) mma_loop(c);
+      }
     }
     __syncwarp();
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConsumerRegs));
     for (int iter = 1;; ++iter) {
       c.iter = iter;
       c.cur_op = -1;
@@ -3379,10 +3367,10 @@ __global__ void __launch_bounds__(PATH == PATH_WIDE ? kWideThreads : kNumThreads
                 p.sched[5] = 0;
               } else {
                 // sched[4] != 0: the last iteration's outputs have not been appended yet
-                if (p.sched[4] != 0) bookkeep_finish(c);
+                if (p.sched[4] != 0) bookkeep_finish(c.p);
                 p.sched[4] = 0;
                 if (p.max_iters == 0 || git <= p.max_iters) {
-                  n = bookkeep_prepare(c);
+                  n = bookkeep_prepare(c.p, reinterpret_cast<int*>(c.smem + p.x_off), iter);
                   if (n > 0) p.sched[4] = 1;
                 }
               }
@@ -3440,6 +3428,7 @@ __global__ void __launch_bounds__(PATH == PATH_WIDE ? kWideThreads : kNumThreads
           asm volatile("cp.async.commit_group;" ::: "memory");
         }
         c.cur_op = oi;
+        c.opaque();
         unsigned long long* pr = prof ? prof + ((size_t)oi * gridDim.x + blockIdx.x) * 4 : nullptr;
         c.dbg = (prof && oi == p.trace_op) ? prof + ((size_t)(p.num_ops + 1) * gridDim.x) * 4 + (size_t)blockIdx.x * 16 : nullptr;
         if (pr && c.tid == 0) pr[0] = globaltimer();
@@ -3454,7 +3443,7 @@ __global__ void __launch_bounds__(PATH == PATH_WIDE ? kWideThreads : kNumThreads
           case OP_EMBED: if (!op_barrier(c, op)) op_embed(c, op, T); break;
           case OP_RMSNORM: op_rmsnorm(c, op, T); break;
           case OP_LINEAR:
-            if constexpr (PATH == PATH_WIDE) op_linear_wide(c, op, T);
+            if constexpr (PATH == PATH_WIDE) op_linear_wide<NC>(c, op, T);
             else op_linear_rows(c, op, T);
             break;
           case OP_ATTN:
@@ -3515,127 +3504,10 @@ __global__ void __launch_bounds__(PATH == PATH_WIDE ? kWideThreads : kNumThreads
 }
 
 }  // namespace MK_VARIANT
-
-#ifndef MK_VARIANT_SECONDARY
-__global__ void init_state_kernel(KParams p) {
-  const int tid = threadIdx.x + blockIdx.x * blockDim.x;
-  const int nth = blockDim.x * gridDim.x;
-  for (int i = tid; i < p.total_requests; i += nth) p.step[i] = 0;
-  for (int i = tid; i < p.max_reqs; i += nth) p.request_ids[i] = -1;
-  for (int i = tid; i <= p.max_reqs; i += nth) {
-    p.qo_indptr[i] = 0;
-    p.kv_indptr[i] = 0;
-  }
-  for (int i = tid; i < p.max_pages; i += nth) p.page_queue[i] = i;
-  if (tid == 0) {
-    p.sched[0] = 0;
-    p.sched[1] = p.max_pages;
-    p.sched[2] = 0;
-    p.sched[3] = 0;
-    p.sched[4] = 0;
-    p.sched[5] = 0;
-    p.sched[6] = 0;
-    p.sched[7] = 0;
-  }
-}
-
-#endif
 }  // namespace mk
 
-#define MK_CAT2(a, b) a##b
-#define MK_CAT(a, b) MK_CAT2(a, b)
-
-#ifdef MK_VARIANT_SECONDARY
-// a secondary build only exports its kernel instances
-extern "C" const void* MK_CAT(mk_kernel_variant_, MK_VARIANT)(int path) {
-  switch (path) {
-    case mk::PATH_ROWS: return (const void*)mk::MK_VARIANT::megakernel<mk::PATH_ROWS>;
-    default: return (const void*)mk::MK_VARIANT::megakernel<mk::PATH_WIDE>;
-  }
+#define MK_CAT3_(a, b, c) a##b##_##c
+#define MK_CAT3(a, b, c) MK_CAT3_(a, b, c)
+extern "C" const void* MK_CAT3(mk_instance_, MK_VARIANT, MK_NC)() {
+  return (const void*)mk::MK_VARIANT::megakernel<MK_NC == 0 ? mk::PATH_ROWS : mk::PATH_WIDE, MK_NC>;
 }
-#else
-// ------------------------------------------------------------------------------------
-// host-side launch helpers (called by the runtime in mk_runtime.cpp)
-// ------------------------------------------------------------------------------------
-extern "C" const void* mk_kernel_variant_tp(int path);
-extern "C" const void* mk_kernel_variant_hier(int path);
-extern "C" const void* mk_kernel_variant_moe(int path);
-namespace {
-int mk_kernel_threads(int path) { return path == mk::PATH_WIDE ? mk::kWideThreads : mk::kNumThreads; }
-// the build of the kernel a launch needs: tensor-parallel exchange code only when there are peers,
-// the hierarchical barrier only when the launch uses clusters
-const void* kernel_for(const mk::KParams* p) {
-  if (p->has_moe) return mk_kernel_variant_moe(p->path);
-  if (p->cluster > 1) return mk_kernel_variant_hier(p->path);
-  if (p->world > 1) return mk_kernel_variant_tp(p->path);
-  switch (p->path) {
-    case mk::PATH_ROWS: return (const void*)mk::MK_VARIANT::megakernel<mk::PATH_ROWS>;
-    default: return (const void*)mk::MK_VARIANT::megakernel<mk::PATH_WIDE>;
-  }
-}
-}  // namespace
-
-extern "C" int mk_kernel_max_ctas_per_sm(const mk::KParams* p, int smem_bytes) {
-  int n = 0;
-  const void* k = kernel_for(p);
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) return -1;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, mk_kernel_threads(p->path), smem_bytes) != cudaSuccess) return -1;
-  return n;
-}
-
-// Clusters of `cluster` CTAs that can be resident at once (the hierarchical barrier needs all of them).
-extern "C" int mk_kernel_max_clusters(int path, int smem_bytes, int cluster, int grid) {
-  const void* k = mk_kernel_variant_hier(path);
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) return -1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(mk_kernel_threads(path));
-  cfg.dynamicSmemBytes = (size_t)smem_bytes;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = cluster;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess) {
-    cudaGetLastError();
-    return -1;
-  }
-  return n;
-}
-
-extern "C" int mk_kernel_launch(const mk::KParams* p, int grid, int smem_bytes, void* stream) {
-  const void* k = kernel_for(p);
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
-  if (e != cudaSuccess) return (int)e;
-  void* args[] = {(void*)p};
-  if (p->cluster <= 1) {
-    e = cudaLaunchCooperativeKernel(k, dim3(grid), dim3(mk_kernel_threads(p->path)), args, (size_t)smem_bytes, (cudaStream_t)stream);
-    return (int)e;
-  }
-  // co-resident grid of thread-block clusters
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(mk_kernel_threads(p->path));
-  cfg.dynamicSmemBytes = (size_t)smem_bytes;
-  cfg.stream = (cudaStream_t)stream;
-  cudaLaunchAttribute at[2];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = p->cluster;
-  at[0].val.clusterDim.y = 1;
-  at[0].val.clusterDim.z = 1;
-  at[1].id = cudaLaunchAttributeCooperative;
-  at[1].val.cooperative = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 2;
-  e = cudaLaunchKernelExC(&cfg, k, args);
-  return (int)e;
-}
-
-extern "C" int mk_kernel_init_state(const mk::KParams* p, void* stream) {
-  mk::init_state_kernel<<<4, 256, 0, (cudaStream_t)stream>>>(*p);
-  return (int)cudaGetLastError();
-}
-#endif  // MK_VARIANT_SECONDARY

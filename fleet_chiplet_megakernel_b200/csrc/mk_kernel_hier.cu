@@ -3,5 +3,4 @@
 // in mk_kernel.cu.
 #define MK_VARIANT hier
 #define MK_HIER_BARRIER 1
-#define MK_VARIANT_SECONDARY 1
 #include "mk_kernel.cu"

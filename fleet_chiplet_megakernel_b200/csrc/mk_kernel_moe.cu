@@ -3,5 +3,4 @@
 // variants in mk_kernel.cu.
 #define MK_VARIANT moe
 #define MK_WITH_MOE 1
-#define MK_VARIANT_SECONDARY 1
 #include "mk_kernel.cu"

@@ -3,5 +3,4 @@
 // them).  Launched whenever world_size > 1; see the note on build variants in mk_kernel.cu.
 #define MK_VARIANT tp
 #define MK_WITH_XCHG 1
-#define MK_VARIANT_SECONDARY 1
 #include "mk_kernel.cu"

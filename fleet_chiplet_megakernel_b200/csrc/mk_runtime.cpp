@@ -25,7 +25,7 @@
 #include "mk_types.h"
 
 extern "C" int mk_kernel_max_ctas_per_sm(const mk::KParams* p, int smem_bytes);
-extern "C" int mk_kernel_max_clusters(int path, int smem_bytes, int cluster, int grid);
+extern "C" int mk_kernel_max_clusters(int path, int x_rows, int smem_bytes, int cluster, int grid);
 extern "C" int mk_kernel_launch(const mk::KParams* p, int grid, int smem_bytes, void* stream);
 extern "C" int mk_kernel_init_state(const mk::KParams* p, void* stream);
 
@@ -1300,9 +1300,6 @@ static int compile_program(mk_handle* h, bool first) {
   const int red_bytes = rows_mode ? kRedBytes : mk::kWideRedBytes;
   const int bar_bytes = rows_mode ? 1024 : 2048;  // barriers and flags, then the two op descriptors
   const int fixed0 = rows_mode ? 1024 /*alignment slack*/ + sums_bytes + red_bytes + bar_bytes : kWideFixed;
-  // Measured on B200: a CTA whose shared memory (plus the 1 KB the system adds) stays within
-  // the 164 KB carve-out leaves 92 KB of the SM's unified array to L1, and the whole kernel
-  // runs about 8 % faster than with the next carve-out (196 KB, 60 KB of L1).
   const int want_stages = cfg.max_stages > 0 ? std::min(cfg.max_stages, 16) : 4;
   // (row-owner mode prefers two resident token rows and three stages to one row and four)
   int x_budget = kRowsXBudget;
@@ -1353,10 +1350,12 @@ static int compile_program(mk_handle* h, bool first) {
   if (has_moe) x_bytes += 512;  // the expert ids of the pairs, for the producer (routing folded into the expert linear)
   x_bytes = (x_bytes + 1023) / 1024 * 1024;
   const int fixed = fixed0 + x_bytes;
-  const int s_fast = (kFastSmem - fixed) / stage_bytes, s_max = (kMaxSmem - fixed) / stage_bytes;
+  const int s_max = (kMaxSmem - fixed) / stage_bytes;
   int stages;
   if (cfg.max_stages > 0) stages = std::min(s_max, want_stages);  // an explicit request wins
-  else if (rows_mode) stages = std::min(s_fast, 4) >= 3 ? std::min(s_fast, 4) : std::min(s_max, 4);
+  // Row-owner path: five stages where they fit beside the resident rows.  12 layers of 8B width, us per step with 4 and 5
+  // stages: one request 1119 and 1109; two requests, 3, 4 and 5: 1238, 1172, 1166.
+  else if (rows_mode) stages = std::min(s_max, 5);
   else stages = wide_stages(nt, x_bytes);
   if (stages < 2) return h->fail(MK_E_UNSUPPORTED, "activations need %d bytes of shared memory: no room for the weight ring", x_bytes);
   // The page table is rewritten through shared memory as far as it fits into what the ring leaves of the carve-out
@@ -1393,7 +1392,7 @@ static int compile_program(mk_handle* h, bool first) {
   if (cfg.cluster_size == 2 || cfg.cluster_size == 4) {
     if (cfg.world_size > 1) return h->fail(MK_E_UNSUPPORTED, "the cluster-first grid barrier is only built for single-GPU launches");
     const int cs = cfg.cluster_size;
-    const int fit = mk_kernel_max_clusters(kp.path, h->smem_bytes, cs, h->grid / cs * cs);
+    const int fit = mk_kernel_max_clusters(kp.path, x_rows, h->smem_bytes, cs, h->grid / cs * cs);
     if (fit >= 1) {
       kp.cluster = cs;
       h->grid = std::min(h->grid / cs, fit) * cs;

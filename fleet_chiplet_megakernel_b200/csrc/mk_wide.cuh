@@ -84,7 +84,7 @@ __device__ __forceinline__ WideTab& wide_tab(const Ctx& c) { return *reinterpret
 
 // Filled once per iteration, by all consumers.  Token t of request r (qo_indptr[r] <= t < qo_indptr[r + 1]) sits at
 // position kv_len(r) - (tokens of r behind it) - 1.
-__device__ __noinline__ void wide_fill_tokens(Ctx& c, int T) {
+__device__ __forceinline__ void wide_fill_tokens(Ctx& c, int T) {
   const KParams& p = c.p;
   WideTab& tab = wide_tab(c);
   T = min(T, kWideTab);
@@ -131,7 +131,7 @@ __device__ __forceinline__ bool wait_go(const Ctx& c, volatile int* fl, int iter
   }
 }
 
-__device__ __noinline__ void mma_loop(Ctx& c) {
+__device__ __forceinline__ void mma_loop(Ctx& c) {
   const KParams& p = c.p;
   const int S = p.num_stages, N = p.x_rows;
   volatile int* fl = c.flags();
@@ -310,9 +310,16 @@ __device__ __forceinline__ void wide_epilogue(Ctx& c, const OpDesc& op, int blk,
       // larger value wins, ties go to the lower index: one 32-bit maximum over the warp's rows
       const uint32_t k = okc ? (order_bf16(rbf(v[i])) << 16) | (uint32_t)(0xffff - row) : 0u;
       const uint32_t m = __reduce_max_sync(0xffffffffu, k);
-      if (c.lane == i && (m >> 16) > best.key[cc]) {  // (blocks come in ascending order: an equal value keeps the lower index)
-        best.key[cc] = m >> 16;
-        best.idx[cc] = blk * kTileRows + 0xffff - (int)(m & 0xffffu);
+      // (blocks come in ascending order: an equal value keeps the lower index; indexed by cc, the pairs would live in local memory)
+      if (c.lane == i && (m >> 16) > (cc == 0 ? best.key[0] : best.key[1])) {
+        const int at = blk * kTileRows + 0xffff - (int)(m & 0xffffu);
+        if (cc == 0) {
+          best.key[0] = m >> 16;
+          best.idx[0] = at;
+        } else {
+          best.key[1] = m >> 16;
+          best.idx[1] = at;
+        }
       }
     }
   }
@@ -342,7 +349,7 @@ __device__ __forceinline__ void wide_wait_pieces(const Ctx& c, unsigned* cnt, un
 
 // NC: token columns of a thread per round: x_rows / 2, at most 32 (128 token rows: two rounds)
 template <int NC>
-__device__ __noinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
   const KParams& p = c.p;
   const int N = p.x_rows, nkt = op.nkt;
   const int q = c.warp & 3, half = c.warp >> 2, row = 32 * q + c.lane;
@@ -459,13 +466,12 @@ __device__ __noinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
   }
 }
 
+template <int NC>
 __device__ __forceinline__ void op_linear_wide(Ctx& c, const OpDesc& op, int T) {
   if (op_barrier(c, op)) return;
   c.lin_seq += 1;
   if (c.tid == 0) c.flags()[4] = (int)c.lin_seq;  // the activation producer may now read this op's input
-  if (c.p.x_rows == 16) linear_wide<8>(c, op, T);
-  else if (c.p.x_rows == 32) linear_wide<16>(c, op, T);
-  else linear_wide<32>(c, op, T);
+  linear_wide<NC>(c, op, T);
   if (MK_XF(op, F_PUSH)) c.ar_seq += 1;  // every CTA counts the exchange, with or without rows of its own
 }
 
@@ -475,20 +481,22 @@ __device__ __forceinline__ void op_linear_wide(Ctx& c, const OpDesc& op, int T) 
 // When this runs, the new tokens' K/V rows are in the cache and the normalised, rotated q rows in the op's scratch
 // (stored by the QKV linear's epilogue, F_QKV_PREP, or by attn_prepare_rows below).
 //
-// A query group is up to 16 / qpk consecutive tokens of one request: with the q heads of a kv head they fill the 16
-// rows of an mma, so a prompt chunk reads a K/V row once per group instead of once per token (a decoding request is
-// a group of one).  A task is (query group, kv head[, chunk of positions]); W = 1, 2, 4 or 8 warps share a task and
-// take its 16-position tiles in turn:
-//   S = Q K^T   mma.m16n8k16, M = the group's rows, N = 8 positions, K = 128 dims in 8 steps
-//   O += P V    M = the rows, K = 16 positions, N = 128 dims in 16 tiles of 8
+// A query group is up to 8 / qpk consecutive tokens of one request: with the q heads of a kv head they fill eight rows, so
+// a prompt chunk reads a K/V row once per group instead of once per token (a decoding request is a group of one).  A task
+// is (query group, kv head[, chunk of positions]); W = 1, 2, 4 or 8 warps share a task and take its 16-position tiles in
+// turn:
+//   S = Q K^T       mma.m16n8k16, M = the group's rows (eight of 16), N = 8 positions, K = 128 dims in 8 steps
+//   O^T += V^T P^T  M = 16 dims in 8 tiles, N = the rows, K = 16 positions: the scores are its B operand as they are
 // with the fragments loaded straight from the cache rows, no staging and no ldmatrix: a dot product does not care in
 // which order the dims are walked, so k step s of lane j of a quad stands for dims 32 (s / 2) + 8 j + 4 (s % 2) +
-// {0..3} (the quad reads 64 contiguous bytes of a K row per load), and output column n of tile t stands for dim
-// 64 (t / 8) + 8 n + t % 8 (eight lanes read 128 contiguous bytes of a V row per load; two rows are paired up per
+// {0..3} (the quad reads 64 contiguous bytes of a K row per load), and rows n and n + 8 of dim tile t stand for dims
+// 8 n + t and 64 + 8 n + t (eight lanes read 128 contiguous bytes of a V row per load; two rows are paired up per
 // register with byte permutes).  P enters as the sum of three bf16 values (24 bits: what fp32 holds), and a score is
 // the sum of two chains of four mma (a chain truncates what it adds up).  Outputs that are not the bf16 nearest to a
 // float64 softmax, 4 to 40 requests: 0.038 %, the same as with scalar fp32; with one chain 0.040 %, with P as two bf16
 // values 0.2 %, as one 10 to 34 %.  Two more mma per tile column cost nothing that could be measured.
+// (Groups of 16 rows, with the rows on M in both products, took 64 registers of sums, half of them idle in decoding, and
+// did not fit beside the other kind of group without 280 bytes of spills per thread.)
 __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
   uint32_t r;
   asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
@@ -502,10 +510,10 @@ struct WideTask {
 
 // Query groups, warps per task and chunking of the iteration: the same in every layer, worked out by the first
 // attention op (key: the head geometry).
-__device__ __noinline__ void wide_plan_attention(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void wide_plan_attention(Ctx& c, const OpDesc& op, int T) {
   const KParams& p = c.p;
   WideTab& tab = wide_tab(c);
-  const int HKV = op.aux0, qpk = op.aux1 / op.aux0, tpg = 16 / qpk;
+  const int HKV = op.aux0, qpk = op.aux1 / op.aux0, tpg = 8 / qpk;
   T = min(T, kWideTab);
   // a token opens a group when it is the first of its request or tpg tokens behind the last opening
   int lmax = 1;
@@ -535,10 +543,8 @@ __device__ __noinline__ void wide_plan_attention(Ctx& c, const OpDesc& op, int T
     const int ng = tab.scan[0] + tab.scan[1] + tab.scan[2] + tab.scan[3];
     const int L = max(max(tab.scan[4], tab.scan[5]), max(tab.scan[6], tab.scan[7]));
     const int G = gridDim.x, pairs = ng * HKV, tiles = (L + 15) >> 4;
-    const bool full = tpg > 1 && ng < T;  // some group holds several tokens: up to 16 rows
     // Warps per task: as many as the grid has for one round of tasks, no more than the longest sequence has tiles.
-    // Groups of several tokens need 4 KB of shared memory for their q rows: at least two warps.
-    int W = full ? 2 : 1;
+    int W = 1;
     while (W < 8 && pairs * (2 * W) <= G * kNumConsumerWarps && W < tiles) W *= 2;
     // Few pairs and long sequences: a CTA per chunk of at least 8 tiles, as many chunks as one round of CTAs holds.
     int nch = 1;
@@ -549,13 +555,12 @@ __device__ __noinline__ void wide_plan_attention(Ctx& c, const OpDesc& op, int T
     tab.plan[1] = W;
     tab.plan[2] = nch;
     tab.plan[3] = tpc * 16;
-    tab.plan[4] = full ? 1 : 0;
   }
   consumer_sync();
 }
 
 // q and k head vectors of the new tokens, where no linear's epilogue has done it: a half-warp per head vector.
-__device__ __noinline__ void attn_prepare_rows(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void attn_prepare_rows(Ctx& c, const OpDesc& op, int T) {
   const int HKV = op.aux0, qpk = op.aux1 / op.aux0, parts = qpk + 2;
   const int total = T * HKV * parts, l16 = c.lane & 15;
 #pragma unroll 1
@@ -567,18 +572,13 @@ __device__ __noinline__ void attn_prepare_rows(Ctx& c, const OpDesc& op, int T) 
   }
 }
 
-// mma of the group's rows; FULL: rows 8..15 are in use, else what they give is dropped
-template <bool FULL>
-__device__ __forceinline__ void wide_mma(float (&d)[FULL ? 4 : 2], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-  if constexpr (FULL) {
-    mma_bf16(d, a0, a1, a2, a3, b0, b1);
-  } else {
-    float x0, x1;  // rows 8..15: nothing (shared accumulators in their place would chain every mma to the one before)
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%10,%10};"
-        : "+f"(d[0]), "+f"(d[1]), "=f"(x0), "=f"(x1)
-        : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1), "f"(0.f));
-  }
+// A group has eight rows: rows 8..15 of the score mma's M side are nothing (shared accumulators in their place would chain
+// every mma to the one before).
+__device__ __forceinline__ void wide_mma_qk(float (&d)[2], uint32_t a0, uint32_t a2, uint32_t b0, uint32_t b1) {
+  float x0, x1;
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%10,%10};"
+      : "+f"(d[0]), "+f"(d[1]), "=f"(x0), "=f"(x1)
+      : "r"(a0), "r"(0u), "r"(a2), "r"(0u), "r"(b0), "r"(b1), "f"(0.f));
 }
 
 // Cache rows of a 16-position tile.  Positions at or beyond p1 read row p1 - 1 instead: their probabilities are zero.
@@ -623,12 +623,11 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t&
 // positions it sees and no others, in scalar fp32: a warp per row, a lane per position for the scores and four dims per
 // lane for the sums.  (The check sits on the outputs: 36 layers at 8 requests 5.83 -> 5.86 ms; on the accumulators, with
 // the sums redone in place, 5.90.)
-__device__ __noinline__ void wide_attend_exact(const Ctx& c, const OpDesc& op, const WideTask& a, int W, __nv_bfloat16* out, float* part) {
-  const KParams& p = c.p;
-  const int HKV = op.aux0, qpk = op.aux1 / HKV, rows = a.nt * qpk, lane = c.lane;
+__device__ __forceinline__ void wide_attend_exact(const KParams& p, const OpDesc& op, const WideTask a, int W, __nv_bfloat16* out, float* part) {
+  const int HKV = op.aux0, qpk = op.aux1 / HKV, rows = a.nt * qpk, lane = threadIdx.x & 31;
   const float sc = 1.4426950408889634f * 0.08838834764831845f;  // log2(e) / sqrt(128)
 #pragma unroll 1
-  for (int r = c.warp & (W - 1); r < rows; r += W) {
+  for (int r = (threadIdx.x >> 5) & (W - 1); r < rows; r += W) {
     const int tok = r / qpk, head = r % qpk, last = min(a.L0 + tok, a.p1);
     const uint4* q = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.out2) + (size_t)(a.t0 + tok) * op.ld_out2 +
                                                     (size_t)(a.h * qpk + head) * kHeadDim);
@@ -698,10 +697,8 @@ __device__ __forceinline__ bool bar_any(int id, int nthr, bool pred) {
   return r != 0u;
 }
 
-// One task by W warps.  `reg`: the group's shared memory (W x 2 KB), `ml`: [warps of the CTA][16] (max, sum) pairs.
-template <bool FULL>
-__device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTask& a, int W, int gi, uint8_t* reg, float2* ml) {
-  constexpr int NR = FULL ? 4 : 2;  // accumulator registers of a tile in use
+// One task by W warps.  `reg`: the group's shared memory (W x 2 KB), `ml`: [warps of the CTA][8] (max, sum) pairs.
+__device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTask& a, int W, int gi, uint8_t* reg, float2* ml) {
   const KParams& p = c.p;
   const int lane = c.lane, g = lane >> 2, j = lane & 3;
   const int HKV = op.aux0, qpk = op.aux1 / HKV, rows = a.nt * qpk;
@@ -718,7 +715,7 @@ __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTas
   // thread (at most four), then the first K and V rows, then the stores: one round trip instead of one per row (with
   // the clamped row loads, the op's start took 5.4 us instead of 7.7 at eight requests of 300 tokens).
   {
-    constexpr int NQ = (FULL ? 16 : 8) * 16;
+    constexpr int NQ = 8 * 16;
     const int qsh = 31 - __clz(qpk);  // (1, 2, 4 or 8 q heads per kv head)
     const __nv_bfloat16* q0 = reinterpret_cast<const __nv_bfloat16*>(op.out2) + (size_t)a.t0 * op.ld_out2 + (size_t)a.h * qpk * kHeadDim;
     uint4* sq = reinterpret_cast<uint4*>(reg);
@@ -745,156 +742,134 @@ __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTas
   MK_STAMP(c, 1);
   const char* sq = reinterpret_cast<const char*>(reg) + g * 256 + 16 * j;
   const int swz = ((g & 1) << 6) | ((g & 2) << 2);
-  float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
-  float oacc[16][NR];
+  float m = -INFINITY, l = 0.f;  // of row g
+  float oacc[8][4];  // tile t of 16 dims: {dim 8 g + t of rows 2 j and 2 j + 1, dim 64 + 8 g + t of the same}
 #pragma unroll
-  for (int t = 0; t < 16; ++t)
+  for (int t = 0; t < 8; ++t)
 #pragma unroll
-    for (int i = 0; i < NR; ++i) oacc[t][i] = 0.f;
-  // length this lane's rows see: row r belongs to token r / qpk of the group
-  const int Lr[2] = {a.L0 + g / qpk, a.L0 + (g + 8) / qpk};
+    for (int i = 0; i < 4; ++i) oacc[t][i] = 0.f;
+  const int last = min(a.L0 + g / qpk, a.p1);  // positions row g sees: it belongs to token g / qpk of the group
 #pragma unroll 1
   for (; ti < ntiles; ti += W) {
     const int pos0 = a.p0 + 16 * ti;
     const bool more = ti + W < ntiles;
-    float s0[NR], s1[NR], z0[NR], z1[NR];
-#pragma unroll
-    for (int i = 0; i < NR; ++i) s0[i] = s1[i] = z0[i] = z1[i] = 0.f;
+    float s0[2] = {0.f, 0.f}, s1[2] = {0.f, 0.f}, z0[2] = {0.f, 0.f}, z1[2] = {0.f, 0.f};
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
-      const char* qs = sq + ((64 * (s >> 1) + 8 * (s & 1)) ^ swz);
-      const uint2 qa = *reinterpret_cast<const uint2*>(qs);
-      uint2 qb = make_uint2(0u, 0u);
-      if constexpr (FULL) qb = *reinterpret_cast<const uint2*>(qs + 8 * 256);
+      const uint2 qa = *reinterpret_cast<const uint2*>(sq + ((64 * (s >> 1) + 8 * (s & 1)) ^ swz));
       const uint4 &k0 = kr[0][s >> 1], &k1 = kr[1][s >> 1];
-      wide_mma<FULL>((s & 1) ? z0 : s0, qa.x, qb.x, qa.y, qb.y, (s & 1) ? k0.z : k0.x, (s & 1) ? k0.w : k0.y);
-      wide_mma<FULL>((s & 1) ? z1 : s1, qa.x, qb.x, qa.y, qb.y, (s & 1) ? k1.z : k1.x, (s & 1) ? k1.w : k1.y);
-    }
-#pragma unroll
-    for (int i = 0; i < NR; ++i) {
-      s0[i] += z0[i];
-      s1[i] += z1[i];
+      wide_mma_qk((s & 1) ? z0 : s0, qa.x, qa.y, (s & 1) ? k0.z : k0.x, (s & 1) ? k0.w : k0.y);
+      wide_mma_qk((s & 1) ? z1 : s1, qa.x, qa.y, (s & 1) ? k1.z : k1.x, (s & 1) ? k1.w : k1.y);
     }
     if (more) wide_load_k(c, op, a, pos0 + 16 * W, pgn, kr);  // K of the next tile flies during the rest of this one
-    // rows g (and g + 8), positions pos0 + 2 j + {0, 1} (s0) and pos0 + 8 + 2 j + {0, 1} (s1)
-    uint32_t ph[4] = {0u, 0u, 0u, 0u}, pm[4] = {0u, 0u, 0u, 0u}, pl[4] = {0u, 0u, 0u, 0u};
-    float alpha[2];
+    // row g, positions pos0 + 2 j + {0, 1} and pos0 + 8 + 2 j + {0, 1}
+    float sv[4] = {s0[0] + z0[0], s0[1] + z0[1], s1[0] + z1[0], s1[1] + z1[1]};
+    float tmax = -INFINITY;
 #pragma unroll
-    for (int u = 0; u < NR / 2; ++u) {
-      float sv[4] = {s0[2 * u], s0[2 * u + 1], s1[2 * u], s1[2 * u + 1]};
-      const int last = min(Lr[u], a.p1);
-      float tmax = -INFINITY;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        sv[i] = pos0 + 2 * j + (i & 1) + 8 * (i >> 1) < last ? sv[i] * sc : -INFINITY;
-        tmax = fmaxf(tmax, sv[i]);
-      }
-      tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
-      tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
-      const float mn = fmaxf(m[u], tmax);
-      const float ms = mn == -INFINITY ? 0.f : mn;  // (a causal row may see nothing of a tile)
-      alpha[u] = exp2f(m[u] - ms);
-      m[u] = mn;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) sv[i] = exp2f(sv[i] - ms);
-      l[u] = l[u] * alpha[u] + ((sv[0] + sv[1]) + (sv[2] + sv[3]));  // this lane's share: the quad adds up at the end
-      split3(sv[0], sv[1], ph[u], pm[u], pl[u]);
-      split3(sv[2], sv[3], ph[2 + u], pm[2 + u], pl[2 + u]);
+    for (int i = 0; i < 4; ++i) {
+      sv[i] = pos0 + 2 * j + (i & 1) + 8 * (i >> 1) < last ? sv[i] * sc : -INFINITY;
+      tmax = fmaxf(tmax, sv[i]);
     }
+    tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 1));
+    tmax = fmaxf(tmax, __shfl_xor_sync(0xffffffffu, tmax, 2));
+    const float mn = fmaxf(m, tmax);
+    const float ms = mn == -INFINITY ? 0.f : mn;  // (a causal row may see nothing of a tile)
+    const float alpha = exp2f(m - ms);
+    m = mn;
 #pragma unroll
-    for (int t = 0; t < 16; ++t) {
+    for (int i = 0; i < 4; ++i) sv[i] = exp2f(sv[i] - ms);
+    l = l * alpha + ((sv[0] + sv[1]) + (sv[2] + sv[3]));  // this lane's share: the quad adds up at the end
+    uint32_t ph[2], pm[2], pl[2];  // as they are, the B operand of O^T = V^T P^T
+    split3(sv[0], sv[1], ph[0], pm[0], pl[0]);
+    split3(sv[2], sv[3], ph[1], pm[1], pl[1]);
+    const float al0 = __shfl_sync(0xffffffffu, alpha, 8 * j), al1 = __shfl_sync(0xffffffffu, alpha, 8 * j + 4);  // rows 2 j, 2 j + 1
 #pragma unroll
-      for (int i = 0; i < NR; ++i) oacc[t][i] *= alpha[i >> 1];
-      // dim 16 g + t of the four V rows: element t of the lane's 16, two rows per register
-      const uint4 &a0 = vr[0][t >> 3], &a1 = vr[1][t >> 3], &a2 = vr[2][t >> 3], &a3 = vr[3][t >> 3];
-      const int w = (t >> 1) & 3;
-      const uint32_t w0 = w == 0 ? a0.x : (w == 1 ? a0.y : (w == 2 ? a0.z : a0.w));
-      const uint32_t w1 = w == 0 ? a1.x : (w == 1 ? a1.y : (w == 2 ? a1.z : a1.w));
-      const uint32_t w2 = w == 0 ? a2.x : (w == 1 ? a2.y : (w == 2 ? a2.z : a2.w));
-      const uint32_t w3 = w == 0 ? a3.x : (w == 1 ? a3.y : (w == 2 ? a3.z : a3.w));
+    for (int t = 0; t < 8; ++t) {
+      oacc[t][0] *= al0;
+      oacc[t][1] *= al1;
+      oacc[t][2] *= al0;
+      oacc[t][3] *= al1;
+      // element t of the lane's two vectors of four V rows, two rows per register
+      uint32_t e[4][2];
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int x = 0; x < 2; ++x) e[r][x] = t < 2 ? vr[r][x].x : (t < 4 ? vr[r][x].y : (t < 6 ? vr[r][x].z : vr[r][x].w));
       const uint32_t sel = (t & 1) ? 0x7632u : 0x5410u;
-      const uint32_t b0 = prmt(w0, w1, sel), b1 = prmt(w2, w3, sel);
-      wide_mma<FULL>(oacc[t], ph[0], ph[1], ph[2], ph[3], b0, b1);
-      wide_mma<FULL>(oacc[t], pm[0], pm[1], pm[2], pm[3], b0, b1);
-      wide_mma<FULL>(oacc[t], pl[0], pl[1], pl[2], pl[3], b0, b1);
+      const uint32_t a0 = prmt(e[0][0], e[1][0], sel), a1 = prmt(e[0][1], e[1][1], sel);
+      const uint32_t a2 = prmt(e[2][0], e[3][0], sel), a3 = prmt(e[2][1], e[3][1], sel);
+      mma_bf16(oacc[t], a0, a1, a2, a3, ph[0], ph[1]);
+      mma_bf16(oacc[t], a0, a1, a2, a3, pm[0], pm[1]);
+      mma_bf16(oacc[t], a0, a1, a2, a3, pl[0], pl[1]);
     }
     if (more) {
       wide_load_v(c, op, a, pos0 + 16 * W, pgn, vr);
       if (psh >= 4) pgn = ti + 2 * W < ntiles ? wide_page(c, a, pos0 + 32 * W) : 0;
     }
   }
-#pragma unroll
-  for (int u = 0; u < NR / 2; ++u) {
-    l[u] += __shfl_xor_sync(0xffffffffu, l[u], 1);
-    l[u] += __shfl_xor_sync(0xffffffffu, l[u], 2);
-  }
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
   MK_STAMP(c, 2);
   __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out) + (size_t)a.t0 * op.ld_out + (size_t)a.h * qpk * kHeadDim;
   float chk = 0.f;  // stays zero while the outputs are finite
   if (W == 1 && a.nch == 1) {
-    // this lane holds, per row, dims 64 x + 16 j + {0..7} (oacc[8 x + i][0]) and the eight behind them (oacc[8 x + i][1])
 #pragma unroll
-    for (int u = 0; u < NR / 2; ++u) {
-      const int r = g + 8 * u;
+    for (int y = 0; y < 2; ++y) {
+      const float lr = __shfl_sync(0xffffffffu, l, 8 * j + 4 * y);
+      const int r = 2 * j + y;
       if (r < rows) {
-        const float inv = __fdividef(1.0f, l[u]);
-        __nv_bfloat16* dst = out + (size_t)(r / qpk) * op.ld_out + (r % qpk) * kHeadDim + 16 * j;
+        const float inv = __fdividef(1.0f, lr);
+        __nv_bfloat16* dst = out + (size_t)(r / qpk) * op.ld_out + (r % qpk) * kHeadDim + 8 * g;
 #pragma unroll
-        for (int x = 0; x < 2; ++x)
+        for (int x = 0; x < 2; ++x) {
+          float f[8];
 #pragma unroll
-          for (int y = 0; y < 2; ++y) {
-            float f[8];
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              f[i] = oacc[8 * x + i][2 * u + y] * inv;
-              chk = fmaf(f[i], 0.f, chk);
-            }
-            *reinterpret_cast<uint4*>(dst + 64 * x + 8 * y) = pack8(f);
+          for (int i = 0; i < 8; ++i) {
+            f[i] = oacc[i][2 * x + y] * inv;
+            chk = fmaf(f[i], 0.f, chk);
           }
+          *reinterpret_cast<uint4*>(dst + 64 * x) = pack8(f);
+        }
       }
     }
     __syncwarp();
-    if (__any_sync(0xffffffffu, chk != 0.f)) wide_attend_exact(c, op, a, W, out, nullptr);
+    if (__any_sync(0xffffffffu, chk != 0.f)) wide_attend_exact(c.p, op, a, W, out, nullptr);
     return;
   }
   // The warps of the task meet in shared memory, four rows at a time (the slots take the place of the q rows).
   const uint32_t nbar = (uint32_t)(2 + gi);
-  if (j == 0) {
-#pragma unroll
-    for (int u = 0; u < NR / 2; ++u) ml[c.warp * 16 + g + 8 * u] = make_float2(m[u], l[u]);
-  }
+  if (j == 0) ml[c.warp * 8 + g] = make_float2(m, l);
   float* slot0 = reinterpret_cast<float*>(reg);
   float* part = p.attn_part + ((size_t)a.t0 * HKV * p.attn_max_chunks * qpk + (size_t)(a.h * p.attn_max_chunks + a.ch) * rows) * (kHeadDim + 2);
 #pragma unroll
-  for (int rb = 0; rb < (FULL ? 4 : 2); ++rb) {
+  for (int rb = 0; rb < 2; ++rb) {
     if (4 * rb >= rows) break;
     asm volatile("bar.sync %0, %1;" ::"r"(nbar), "r"(nthr) : "memory");
-    if ((g >> 2) == (rb & 1)) {
-      float* dst = slot0 + (size_t)sub * 4 * kHeadDim + (g & 3) * kHeadDim + 16 * j;
-      const int u = rb >> 1;
+    if ((j >> 1) == rb) {
+      float* dst = slot0 + (size_t)sub * 4 * kHeadDim + 2 * (j & 1) * kHeadDim + 8 * g;
 #pragma unroll
-      for (int x = 0; x < 2; ++x)
+      for (int y = 0; y < 2; ++y)
 #pragma unroll
-        for (int y = 0; y < 2; ++y)
+        for (int x = 0; x < 2; ++x)
 #pragma unroll
           for (int i = 0; i < 8; i += 4)
-            *reinterpret_cast<float4*>(dst + 64 * x + 8 * y + i) =
-                make_float4(oacc[8 * x + i][2 * u + y], oacc[8 * x + i + 1][2 * u + y], oacc[8 * x + i + 2][2 * u + y], oacc[8 * x + i + 3][2 * u + y]);
+            *reinterpret_cast<float4*>(dst + y * kHeadDim + 64 * x + i) =
+                make_float4(oacc[i][2 * x + y], oacc[i + 1][2 * x + y], oacc[i + 2][2 * x + y], oacc[i + 3][2 * x + y]);
     }
     asm volatile("bar.sync %0, %1;" ::"r"(nbar), "r"(nthr) : "memory");
 #pragma unroll 1
     for (int e = gtid; e < 4 * 32; e += nthr) {  // (row of the round, four dims)
       const int r = 4 * rb + (e >> 5), d = (e & 31) * 4;
       if (r >= rows) continue;
-      const float2* mlr = ml + (c.warp - sub) * 16 + r;
+      const float2* mlr = ml + (c.warp - sub) * 8 + r;
       float M = -INFINITY;
-      for (int w = 0; w < W; ++w) M = fmaxf(M, mlr[w * 16].x);
+      for (int w = 0; w < W; ++w) M = fmaxf(M, mlr[w * 8].x);
       const float Ms = M == -INFINITY ? 0.f : M;
       float L = 0.f;
       float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
       for (int w = 0; w < W; ++w) {
-        const float2 v = mlr[w * 16];
+        const float2 v = mlr[w * 8];
         const float f = exp2f(v.x - Ms);
         const float4 o4 = *reinterpret_cast<const float4*>(slot0 + (size_t)w * 4 * kHeadDim + (e >> 5) * kHeadDim + d);
         L = fmaf(f, v.y, L);
@@ -920,7 +895,7 @@ __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTas
   }
   MK_STAMP(c, 3);
   if (bar_any((int)nbar, nthr, chk != 0.f)) {  // (the group's memory is free again)
-    wide_attend_exact(c, op, a, W, out, part);
+    wide_attend_exact(c.p, op, a, W, out, part);
     asm volatile("bar.sync %0, %1;" ::"r"(nbar), "r"(nthr) : "memory");
   }
   if (a.nch == 1) return;
@@ -979,7 +954,7 @@ __device__ __noinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTas
   consumer_sync();
 }
 
-__device__ __noinline__ void op_attention_wide(Ctx& c, const OpDesc& op, int T) {
+__device__ __forceinline__ void op_attention_wide(Ctx& c, const OpDesc& op, int T) {
   const KParams& p = c.p;
   if (op_barrier(c, op)) return;
   if (p.debug_flags & 2) return;  // measurement aid: the op keeps its barrier and does nothing else
@@ -998,7 +973,6 @@ __device__ __noinline__ void op_attention_wide(Ctx& c, const OpDesc& op, int T) 
   const WideTab& tab = wide_tab(c);
   const int HKV = op.aux0;
   const int W = tab.plan[1], nch = tab.plan[2], CS = tab.plan[3];
-  const bool full = tab.plan[4] != 0;
   const int ntasks = tab.plan[0] * HKV * nch, per = kNumConsumerWarps / W;
   const int gi = c.warp / W;
   uint8_t* reg = c.smem + p.x_off + (size_t)gi * W * 2048;
@@ -1019,7 +993,6 @@ __device__ __noinline__ void op_attention_wide(Ctx& c, const OpDesc& op, int T) 
     a.p1 = min(L, a.p0 + CS);
     a.nch = (L + CS - 1) / CS;
     if (a.p0 >= L || a.L0 <= 0) continue;  // (uniform within the task's warps)
-    if (full) wide_attend<true>(c, op, a, W, gi, reg, ml);
-    else wide_attend<false>(c, op, a, W, gi, reg, ml);
+    wide_attend(c, op, a, W, gi, reg, ml);
   }
 }
