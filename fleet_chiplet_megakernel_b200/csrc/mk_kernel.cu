@@ -565,6 +565,11 @@ __device__ __forceinline__ uint2 ld_gpu_v2(const uint2* p) {
 __device__ __forceinline__ void st_gpu_v2(uint2* p, uint32_t a, uint32_t b) {
   asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1,%2};" ::"l"(p), "r"(a), "r"(b) : "memory");
 }
+// two words at once: a vector of 64-bit scalars, each of them single-copy atomic
+__device__ __forceinline__ void st_gpu_words(uint4* p, uint32_t a, uint32_t b, uint32_t tag) {
+  const unsigned long long x = (unsigned long long)tag << 32 | a, y = (unsigned long long)tag << 32 | b;
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1,%2};" ::"l"(p), "l"(x), "l"(y) : "memory");
+}
 __device__ __forceinline__ bool ll_ok(const uint4& a, const uint4& b, unsigned tag) {
   return a.y == tag && a.w == tag && b.y == tag && b.w == tag;
 }

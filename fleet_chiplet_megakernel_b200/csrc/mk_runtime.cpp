@@ -1557,18 +1557,24 @@ static int compile_program(mk_handle* h, bool first) {
     ll_part_off = ll_bytes;
     ll_bytes += ((size_t)h->plan_tokens * hkv * kAttnMaxChunks * qpk * (mk::kHeadDim + 2) * 8 + 255) / 256 * 256;
   }
+  const size_t partial_off = ll_bytes;  // wide path up to 32 token rows: the split sums of a CTA, as tagged words
+  const bool words = !rows_mode && x_rows <= 32;
+  if (words) ll_bytes += (size_t)h->grid * mk::kTileRows * x_rows * 8;
   h->ll_buf = nullptr;
   h->ll_bytes = ll_bytes;
   if (ll_bytes > 0) {
     if (int e = h->dmalloc(&h->ll_buf, ll_bytes)) return e;
   }
+  kp.partial = words ? (uint4*)((char*)h->ll_buf + partial_off) : nullptr;
   kp.attn_part_ll = ll_part ? (uint2*)((char*)h->ll_buf + ll_part_off) : nullptr;
 
   // 3. scratch and state
   const int G = h->grid;
   void* p = nullptr;
-  if (int e = h->dmalloc(&p, (size_t)G * mk::kTileRows * x_rows * 4)) return e;
-  kp.partial = (float*)p;
+  if (!rows_mode && !words) {
+    if (int e = h->dmalloc(&p, (size_t)G * mk::kTileRows * x_rows * 4)) return e;
+    kp.partial = (uint4*)p;
+  }
   h->piece_count_bytes = rows_mode ? 4 : (size_t)max_nblk * mk::kNumConsumerWarps * 4;
   if (int e = h->dmalloc(&p, h->piece_count_bytes)) return e;
   kp.piece_count = (unsigned*)p;

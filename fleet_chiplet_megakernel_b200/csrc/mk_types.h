@@ -202,8 +202,9 @@ struct KParams {
   int max_iters;      // 0 = unlimited
   unsigned long long timeout_ns;
   // split-k scratch shared by all linear ops of the wide path
-  float* partial;         // [grid][x_rows / 4][128 rows] float4: a CTA's sums of the block that an earlier CTA finishes
-  unsigned* piece_count;  // [max nblk][8 warps]: shares published
+  uint4* partial;         // [grid][...][128 rows]: a CTA's sums of the block that an earlier CTA finishes.  Up to 32 token rows
+                          // [x_rows / 2] words {sum, tag, sum of the next token, tag}, beyond [x_rows / 4] float4
+  unsigned* piece_count;  // [max nblk][8 warps]: shares published (beyond 32 token rows)
   // attention scratch
   float* attn_part;       // [tokens][kv heads][max chunks][qpk*(128+2)]
   unsigned* attn_count;   // [tokens][kv heads]

@@ -200,11 +200,16 @@ __device__ __forceinline__ void mma_loop(Ctx& c) {
 // a thread holds one output row for up to 32 tokens in registers, from tensor memory to the store.
 //
 // When several CTAs hold k-ranges of a row block, the CTA with the block's FIRST k-range finishes it (that range
-// is the tail of its own tile range, so it is computed last anyway).  The others store their sums as float4 of
-// four tokens, [token / 4][row], and every warp publishes its share with a release of its own; the matching warp of
-// the finisher waits for exactly those, fetches all of them in one round of loads and adds them up in CTA order.
-// No CTA-wide sync and no shared memory on the way: with both, at 64 tokens, the slowest CTA of an O projection
-// needed 30 us (5 us of streaming), most of it here.
+// is the tail of its own tile range, so it is computed last anyway); a thread adds the other pieces of its output row up in
+// CTA order.  No CTA-wide sync and no shared memory on the way.
+//  * Up to 32 token rows the others store their sums as words that carry a tag, two tokens per 16 bytes, [token / 2][row],
+//    and the finisher polls them, several pieces at once: data and "ready" arrive in one load, with no release behind the
+//    stores, no counter and no second round trip.  The tag differs in every op of every iteration, the words are cleared
+//    before every launch, and a CTA's slot is written again only behind a grid barrier.
+//  * Beyond, twice the bytes cost more than the round trip: plain float4 of four tokens, [token / 4][row]; every warp
+//    publishes its share with a release of its own and the matching warp of the finisher waits for exactly those.
+// Both measured, us per step of 12 layers of 8B width (words, counters): 8 requests 1433, 1473; 32 1572, 1588; 64 1989,
+// 1942; 100 2488, 2377; 8 requests of 2048 hidden 855, 910; four layers of 1024 hidden, 4 requests 197, 209.
 __device__ __forceinline__ uint32_t order_bf16(float v) {  // monotone 16-bit key of a bf16 value; 0 only for NaN
   const uint32_t b = __float_as_uint(v + 0.f) >> 16;       // (-0 counts as +0)
   const uint32_t k = (b & 0x8000u) ? (~b & 0xffffu) : (b | 0x8000u);
@@ -361,7 +366,9 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
   int G;
   if (wide_range(p, op, total, G, t0, t1)) {
     const bool with_res = (op.flags & F_RESIDUAL) && !MK_XF(op, F_GATHER_RES) && (!(op.flags & F_RES_RANK0) || p.rank == 0);
-    const size_t slot_vec = (size_t)kTileRows * N / 4;  // float4 of a CTA's partial sums
+    constexpr bool kWords = NC < 32;
+    const size_t slot_vec = (size_t)kTileRows * N / (kWords ? 2 : 4);  // 16-byte vectors of a CTA's sums
+    const unsigned tag = ll_tag_of(c, c.cur_op);
 #pragma unroll 1
     for (unsigned tile = t0; tile < t1;) {
       const int blk = (int)(tile / (unsigned)nkt);
@@ -406,45 +413,89 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
 #pragma unroll
         for (int i = 0; i < NC; ++i) v[i] = __uint_as_float(raw[i]);
         if (!finisher) {
-          float4* mine = reinterpret_cast<float4*>(p.partial) + (size_t)blockIdx.x * slot_vec + (size_t)(col0 >> 2) * kTileRows + row;
+          if constexpr (kWords) {
+            uint4* mine = p.partial + (size_t)blockIdx.x * slot_vec + (size_t)(col0 >> 1) * kTileRows + row;
 #pragma unroll
-          for (int i = 0; i < NC / 4; ++i)
-            if (4 * i < nlive) mine[(size_t)i * kTileRows] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-          if (cc == nround - 1) {
-            __syncwarp();  // lane 0's release covers what the warp wrote before
-            if (c.lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
+            for (int i = 0; i < NC / 2; ++i)
+              if (2 * i < nlive) st_gpu_words(mine + (size_t)i * kTileRows, __float_as_uint(v[2 * i]), __float_as_uint(v[2 * i + 1]), tag);
+          } else {
+            float4* mine = reinterpret_cast<float4*>(p.partial) + (size_t)blockIdx.x * slot_vec + (size_t)(col0 >> 2) * kTileRows + row;
+#pragma unroll
+            for (int i = 0; i < NC / 4; ++i)
+              if (4 * i < nlive) mine[(size_t)i * kTileRows] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            if (cc == nround - 1) {
+              __syncwarp();  // lane 0's release covers what the warp wrote before
+              if (c.lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
+            }
           }
           if (tile == t0) MK_STAMP(c, 1);
           continue;
         }
         MK_STAMP(c, 2);
         if (c_last > (int)blockIdx.x) {
-          if (cc == 0) wide_wait_pieces(c, cnt, (unsigned)(c_last - (int)blockIdx.x), blk);
-          MK_STAMP(c, 3);
-          const float4* src0 = reinterpret_cast<const float4*>(p.partial) + (size_t)(col0 >> 2) * kTileRows + row;
-          // Several pieces in flight per round (registers allowing): a block of a small layer has up to `nkt` of them, and a
-          // round trip each (0.45 us) was most of its finish (7 of 15 us in a 1024 x 3072 layer).  Added in CTA order all the same.
-          constexpr int PB = NC == 8 ? 8 : (NC == 16 ? 4 : 2);
+          if constexpr (kWords) {
+            const uint4* src0 = p.partial + (size_t)(col0 >> 1) * kTileRows + row;
+            // Several pieces in flight per round (registers allowing): a block of a small layer has up to `nkt` of them.
+            constexpr int PB = NC == 8 ? 4 : 2;
 #pragma unroll 1
-          for (int cta = (int)blockIdx.x + 1; cta <= c_last; cta += PB) {
-            float4 w[PB][NC / 4];
+            for (int cta = (int)blockIdx.x + 1; cta <= c_last; cta += PB) {
+              uint4 w[PB][NC / 2];
 #pragma unroll
-            for (int u = 0; u < PB; ++u)
+              for (int u = 0; u < PB; ++u)
 #pragma unroll
-              for (int i = 0; i < NC / 4; ++i)
-                w[u][i] = (cta + u <= c_last && 4 * i < nlive) ? __ldcg(src0 + (size_t)(cta + u) * slot_vec + (size_t)i * kTileRows)
-                                                               : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (int i = 0; i < NC / 2; ++i) {
+                  const unsigned t = (cta + u <= c_last && 2 * i < nlive) ? ~tag : tag;  // (nothing to wait for: zeros)
+                  w[u][i] = make_uint4(0u, t, 0u, t);
+                }
+              PollLimit limit;
+              while (true) {
 #pragma unroll
-            for (int u = 0; u < PB; ++u)
+                for (int u = 0; u < PB; ++u)
 #pragma unroll
-              for (int i = 0; i < NC / 4; ++i) {
-                v[4 * i] += w[u][i].x;
-                v[4 * i + 1] += w[u][i].y;
-                v[4 * i + 2] += w[u][i].z;
-                v[4 * i + 3] += w[u][i].w;
+                  for (int i = 0; i < NC / 2; ++i)
+                    if (w[u][i].y != tag || w[u][i].w != tag) w[u][i] = ld_gpu_v4(src0 + (size_t)(cta + u) * slot_vec + (size_t)i * kTileRows);
+                bool here = true;
+#pragma unroll
+                for (int u = 0; u < PB; ++u)
+#pragma unroll
+                  for (int i = 0; i < NC / 2; ++i) here = here && w[u][i].y == tag && w[u][i].w == tag;
+                if (here || limit.expired(c, tag, w[0][0].y)) break;
               }
+#pragma unroll
+              for (int u = 0; u < PB; ++u)
+#pragma unroll
+                for (int i = 0; i < NC / 2; ++i) {
+                  v[2 * i] += __uint_as_float(w[u][i].x);
+                  v[2 * i + 1] += __uint_as_float(w[u][i].z);
+                }
+            }
+          } else {
+            if (cc == 0) wide_wait_pieces(c, cnt, (unsigned)(c_last - (int)blockIdx.x), blk);
+            const float4* src0 = reinterpret_cast<const float4*>(p.partial) + (size_t)(col0 >> 2) * kTileRows + row;
+            constexpr int PB = 2;  // pieces in flight per round
+#pragma unroll 1
+            for (int cta = (int)blockIdx.x + 1; cta <= c_last; cta += PB) {
+              float4 w[PB][NC / 4];
+#pragma unroll
+              for (int u = 0; u < PB; ++u)
+#pragma unroll
+                for (int i = 0; i < NC / 4; ++i)
+                  w[u][i] = (cta + u <= c_last && 4 * i < nlive) ? __ldcg(src0 + (size_t)(cta + u) * slot_vec + (size_t)i * kTileRows)
+                                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+              for (int u = 0; u < PB; ++u)
+#pragma unroll
+                for (int i = 0; i < NC / 4; ++i) {
+                  v[4 * i] += w[u][i].x;
+                  v[4 * i + 1] += w[u][i].y;
+                  v[4 * i + 2] += w[u][i].z;
+                  v[4 * i + 3] += w[u][i].w;
+                }
+            }
           }
+          MK_STAMP(c, 3);
         }
+        __syncwarp();  // (lanes leave the poll at different times; the epilogue shuffles)
         MK_STAMP(c, 4);
         wide_epilogue<NC>(c, op, blk, row, col0, nlive, v, res, best, cc);
         MK_STAMP(c, 5);
