@@ -122,6 +122,9 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
   return v;
 }
+__device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
 __device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
   unsigned v;
   asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -195,12 +198,15 @@ struct Ctx {
   // wide path, per accumulator buffer: sums complete (tcgen05.commit), sums fetched (one arrival per finishing warp)
   __device__ uint32_t acc_full_bar(unsigned b) const { return smem_addr + p.bar_off + 24 * p.num_stages + 104 + 8 * b; }
   __device__ uint32_t acc_empty_bar(unsigned b) const { return smem_addr + p.bar_off + 24 * p.num_stages + 120 + 8 * b; }
+  // wide path, per stage: the raw rows of a box that still has to be normalised
+  __device__ uint32_t xraw_bar(int s) const { return smem_addr + p.bar_off + 24 * p.num_stages + 136 + 8 * s; }
   __device__ float* sums() const { return (float*)(smem + p.sums_off); }
   __device__ float* red() const { return (float*)(smem + p.red_off); }  // small scratch: reductions, lengths
 };
 // flags(): [0] go word written by consumers, read by the producer
 //          [1] stages issued by the producer   [2] broadcast slot   [3] dead flag of the op
 //          [4] linear ops whose barrier the consumers have passed   [5] wide path: stages multiplied
+//          [6] wide path: linear ops whose row scales are in the token table
 
 #define MK_STAMP(c, k)                                             \
   do {                                                            \
@@ -3194,8 +3200,10 @@ __device__ __forceinline__ void xproducer_loop(Ctx& c) {
   int s = 0;
   uint32_t empty_parity = 1;
   unsigned lin_seq = 0;
-  unsigned issued_mask = 0, xphase = 0;  // per stage: boxes issued; parity of the stage's next box phase
-  const uint32_t bar_x0 = c.xfull_bar(0), bar_empty0 = c.empty_bar(0);
+  // per stage: parity of its next use, whether its latest box is a plain one; raw boxes (for the norm warp) issued and
+  // parity of the next one
+  unsigned xuse = 0, last_plain = 0, issued_raw = 0, raw_phase = 0;
+  const uint32_t bar_x0 = c.xfull_bar(0), bar_raw0 = c.xraw_bar(0), bar_empty0 = c.empty_bar(0);
   const uint32_t x_sub = (uint32_t)p.x_rows * 128u;
   for (int iter = 1;; ++iter) {
     int go;
@@ -3207,35 +3215,32 @@ __device__ __forceinline__ void xproducer_loop(Ctx& c) {
       lin_seq += 1;
       TileCursor lc;
       if (!cursor_open(p, lc, oi)) continue;
-      // wait until the consumers have passed this op's barrier
-      {
-        unsigned long long t0 = 0;
-        int spins = 0;
-        while ((unsigned)fl[4] < lin_seq) {
-          if (fl[0] < 0) { dead = true; break; }
-          __nanosleep(32);  // a hot spin would take issue slots from the consumer warps of this scheduler
-          if (((++spins) & 1023) == 0) {
-            if (aborted(c)) { dead = true; break; }
-            const unsigned long long now = globaltimer();
-            if (t0 == 0) t0 = now;
-            if (now - t0 > 4 * c.p.timeout_ns) { dead = true; break; }
-          }
-        }
+      const bool raw = (op.flags & F_NORM_IN) != 0;
+      const void* tmap = op.tmap_x;
+      asm volatile("prefetch.tensormap [%0];" ::"l"(tmap) : "memory");
+      if (!wait_lin(c, fl, 4, lin_seq)) {  // the consumers have passed this op's barrier
+        dead = true;
+        break;
       }
-      if (dead) break;
       asm volatile("fence.proxy.async;" ::: "memory");  // the rows were written with plain stores, TMA reads them
       for (; lc.tile < lc.t1; ++lc.tile) {
         if (!mbar_wait(c, bar_empty0 + 8 * s, empty_parity, ST_TIMEOUT_EMPTY)) {
           dead = true;
           break;
         }
-        const uint32_t full = bar_x0 + 8 * s;
+        const uint32_t full = (raw ? bar_raw0 : bar_x0) + 8 * s;
         const uint32_t dst = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes + kStageBytes;
         mbar_arrive_expect_tx(full, 2 * x_sub);
-        tma_load_2d(dst, op.tmap_x, full, lc.kt * kTileK, 0);
-        tma_load_2d(dst + x_sub, op.tmap_x, full, lc.kt * kTileK + kBoxK, 0);
-        issued_mask |= 1u << s;
-        xphase ^= 1u << s;
+        tma_load_2d(dst, tmap, full, lc.kt * kTileK, 0);
+        tma_load_2d(dst + x_sub, tmap, full, lc.kt * kTileK + kBoxK, 0);
+        xuse ^= 1u << s;
+        if (raw) {
+          issued_raw |= 1u << s;
+          raw_phase ^= 1u << s;
+          last_plain &= ~(1u << s);
+        } else {
+          last_plain |= 1u << s;
+        }
         if (++s == S) { s = 0; empty_parity ^= 1u; }
         if (++lc.kt == lc.nkt) { lc.kt = 0; lc.blk += 1; }
       }
@@ -3243,8 +3248,10 @@ __device__ __forceinline__ void xproducer_loop(Ctx& c) {
     if (dead || p.mode == MODE_ONEPASS) break;
   }
   // no copy of this thread may still be in flight when the CTA exits
-  for (int i = 0; i < S; ++i)
-    if (issued_mask & (1u << i)) mbar_wait(c, bar_x0 + 8 * i, ((xphase >> i) & 1u) ^ 1u, ST_TIMEOUT_FULL);
+  for (int i = 0; i < S; ++i) {
+    if (issued_raw & (1u << i)) mbar_wait(c, bar_raw0 + 8 * i, ((raw_phase >> i) & 1u) ^ 1u, ST_TIMEOUT_FULL);
+    if (last_plain & (1u << i)) mbar_wait(c, bar_x0 + 8 * i, ((xuse >> i) & 1u) ^ 1u, ST_TIMEOUT_FULL);
+  }
 }
 
 // ------------------------------------------------------------------------------------
@@ -3293,6 +3300,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
       mbar_init(c.full_bar(s), 1);
       mbar_init(c.empty_bar(s), PATH == PATH_WIDE ? 1 : kNumConsumerWarps);  // the commit of the stage's MMAs, or every consumer warp
       mbar_init(c.xfull_bar(s), 1);
+      if (PATH == PATH_WIDE) mbar_init(c.xraw_bar(s), 1);
     }
     mbar_init(c.done_bar(), 1);
     for (int b = 0; b < 2; ++b) {
@@ -3309,6 +3317,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
     fl[3] = 0;
     fl[4] = 0;
     fl[5] = 0;
+    fl[6] = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -3347,6 +3356,8 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
       if constexpr (PATH == PATH_WIDE) {
         if (c.lane == 0) mma_loop(c);
       }
+    } else {
+      if constexpr (PATH == PATH_WIDE && 2 * NC <= kNormBoxRows) norm_loop(c);
     }
     __syncwarp();
   } else {

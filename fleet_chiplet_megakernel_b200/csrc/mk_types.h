@@ -22,13 +22,14 @@ constexpr int kStageBytes = kSubBytes * kSubTiles;
 constexpr int kNumConsumerWarps = 8;
 constexpr int kNumConsumers = kNumConsumerWarps * 32;
 // + a warpgroup of service warps: the weight producer, the activation producer (or L2 look-ahead) and, on the wide path, the
-// MMA issuer; the last one idles.  The block starts with 168 registers a thread; the service warps hand theirs to the
+// MMA issuer; on the wide path, the norm warp.  The block starts with 168 registers a thread; the service warps hand theirs to the
 // consumers (their sum is what the block was launched with).
 constexpr int kNumThreads = kNumConsumers + 128;
 constexpr int kServiceRegs = 56, kConsumerRegs = 224;
 static_assert(128 * kServiceRegs + kNumConsumers * kConsumerRegs == kNumThreads * 168, "a register split beyond the block's own would wait for good");
 constexpr int kWideRedBytes = 4096;              // scratch of the wide path: reductions and the iteration's token table
 constexpr int kHeadDim = 128;
+constexpr int kNormBoxRows = 32;                 // widest activation box that the norm is applied to in shared memory
 // Columns a stand-alone norm stages in shared memory (48 KB).  Wider rows are read twice instead: at 65 tokens and more,
 // where a ring stage is 64 KB, two stages would leave no room for rows of more than 46000 columns.
 constexpr int kNormStagedCols = 24576;
@@ -57,12 +58,14 @@ enum OpType : int {
 enum OpFlags : int {
   F_SYNC_BEFORE = 1 << 0,   // grid barrier before the op
   F_CTA0_ONLY = 1 << 1,     // only CTA 0 executes the body
-  F_NORM_IN = 1 << 2,       // linear: RMSNorm fused on the input rows
+  F_NORM_IN = 1 << 2,       // linear: RMSNorm fused on the input rows (wide path: applied to the activation boxes in shared memory, the row
+                            // sums of squares come from the linear before, F_ROW_SUMS: ll_in, ll_in_op of them per token)
   F_RESIDUAL = 1 << 3,      // linear: + residual
   F_SILU_MUL = 1 << 4,      // linear: rows are [4 gate | 4 up] per 8-row unit, epilogue SiLU(gate)*up (MoE gate/up: a chunk is [gate | up] halves, also -> out2)
   F_ARGMAX = 1 << 5,        // linear: per-tile (max, index) of the bf16 logits
   F_QK_NORM = 1 << 6,       // attention
   F_ROPE = 1 << 7,          // attention
+  F_ROW_SUMS = 1 << 25,     // wide linear: the epilogue also stores, per token, the sum of squares of every 32 output columns (ll_out, ll_res_op of them per token)
   F_RES_RANK0 = 1 << 9,     // residual only contributed when rank == 0 (row-parallel TP)
   F_QKV_PREP = 1 << 8,      // wide QKV linear: the epilogue applies QK-norm and RoPE, stores q to the attention's scratch rows (out2)
                             // and k / v to the cache (aux0/aux1: kv/q heads, aux2: cos/sin rows, aux3: F_QK_NORM | F_ROPE)

@@ -1,9 +1,10 @@
 // The wide path of the megakernel: iterations of 3 to 128 tokens (batches, prompt chunks).
 //
-// Linears are stream-K tiles on the 5th-generation tensor cores.  Four roles per CTA work side by side:
+// Linears are stream-K tiles on the 5th-generation tensor cores.  Five roles per CTA work side by side:
 //   warp 8   weight producer      TMA boxes of 128 rows x 64 k into the ring (producer_loop)
 //   warp 9   activation producer  the matching boxes of x_rows token rows x 64 k (xproducer_loop)
 //   warp 10  MMA issuer           tcgen05.mma over a stage's boxes, accumulators in tensor memory (mma_loop)
+//   warp 11  norm warp            RMSNorm of the activation boxes, up to 32 token rows (norm_loop)
 //   warps 0-7                     finish: accumulators -> split-k exchange -> epilogue (linear_wide)
 // The accumulators are double-buffered, so the MMAs of the next row block run while the finishing warps
 // are still busy with the last one.
@@ -78,6 +79,8 @@ struct WideTab {
   int pos[kWideTab], slot[kWideTab], kvb[kWideTab], req[kWideTab], grp[kWideTab];
   int plan[8];
   int scan[8];
+  // of the linear op at hand: what its input norm multiplies a token's row with (fp32, or a pair of bf16), even tokens first
+  alignas(16) uint32_t scale[kNormBoxRows];
 };
 static_assert(256 + sizeof(WideTab) <= kWideRedBytes, "the token table fits the scratch region");
 __device__ __forceinline__ WideTab& wide_tab(const Ctx& c) { return *reinterpret_cast<WideTab*>(c.smem + c.p.red_off + 256); }
@@ -129,6 +132,23 @@ __device__ __forceinline__ bool wait_go(const Ctx& c, volatile int* fl, int iter
       if (now - t0 > 4 * c.p.timeout_ns) return false;
     }
   }
+}
+
+// Waits until the consumers have counted linear op `seq` in flag word `word`; false: the launch ends.
+__device__ __forceinline__ bool wait_lin(const Ctx& c, volatile int* fl, int word, unsigned seq) {
+  unsigned long long t0 = 0;
+  int spins = 0;
+  while ((unsigned)fl[word] < seq) {
+    if (fl[0] < 0) return false;
+    __nanosleep(32);  // a hot spin would take issue slots from the consumer warps of this scheduler
+    if (((++spins) & 1023) == 0) {
+      if (aborted(c)) return false;
+      const unsigned long long now = globaltimer();
+      if (t0 == 0) t0 = now;
+      if (now - t0 > 4 * c.p.timeout_ns) return false;
+    }
+  }
+  return true;
 }
 
 __device__ __forceinline__ void mma_loop(Ctx& c) {
@@ -191,6 +211,149 @@ __device__ __forceinline__ void mma_loop(Ctx& c) {
   umma_commit(c.done_bar());
   mbar_wait(c, c.done_bar(), 0u, ST_TIMEOUT_FULL);
   fl[5] = (int)consumed;
+}
+
+// ------------------------------------------------------------------------------------
+// the input norm of a linear (F_NORM_IN)
+// ------------------------------------------------------------------------------------
+// A norm between two linears has no op of its own up to kNormBoxRows token rows: as one it is a barrier, a round trip and
+// 3.6 us per norm at 8 requests of 8B width.  The linear before it stores the sums of squares of its output
+// rows (F_ROW_SUMS), the consumers turn them into a scale per token at the start of the linear behind it while the first
+// raw boxes are on their way, and warp 11 normalises every box in place: w * bf16(x * r) or x * (r * w), the arithmetic of
+// the norm op.  Measured, us per step of 12 layers: 8B width, 4 requests 1343 -> 1285, 8 of 300 tokens 1442 -> 1381, 32 of
+// 100 1566 -> 1505; 2048 hidden, 8 requests 862 -> 806; four layers of 1024 hidden, 4 requests 202 -> 187.
+__device__ __forceinline__ uint32_t hmul2_bf16(uint32_t a, uint32_t b) {  // both products rounded to bf16: exact in fp32 before that
+  uint32_t d;
+  asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  return d;
+}
+// Scales of the iteration's tokens, by the consumers.  Warp w takes tokens w, w + 8, ...; op.ll_in: [token][ll_in_op] sums.
+__device__ __forceinline__ void wide_row_scales(Ctx& c, const OpDesc& op, int T) {
+  const bool torch_num = c.p.numerics == NUM_TORCH;
+  const int parts = op.ll_in_op, nvec = parts >> 2;
+  uint32_t* scale = wide_tab(c).scale;
+  float ss[kNormBoxRows / kNumConsumerWarps];
+#pragma unroll
+  for (int i = 0; i < kNormBoxRows / kNumConsumerWarps; ++i) ss[i] = 0.f;
+#pragma unroll 1
+  for (int v = c.lane; v < nvec; v += 32) {
+    float4 q[kNormBoxRows / kNumConsumerWarps];
+#pragma unroll
+    for (int i = 0; i < kNormBoxRows / kNumConsumerWarps; ++i) {
+      const int t = c.warp + kNumConsumerWarps * i;
+      q[i] = t < T ? __ldcg(reinterpret_cast<const float4*>(reinterpret_cast<const float*>(op.ll_in) + (size_t)t * parts) + v) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int i = 0; i < kNormBoxRows / kNumConsumerWarps; ++i) ss[i] += (q[i].x + q[i].y) + (q[i].z + q[i].w);
+  }
+#pragma unroll
+  for (int i = 0; i < kNormBoxRows / kNumConsumerWarps; ++i)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss[i] += __shfl_xor_sync(0xffffffffu, ss[i], o);
+  // lane i finishes token w + 8 i (as row_rms_scale does for a staged row)
+  float mine = ss[0];
+#pragma unroll
+  for (int i = 1; i < kNormBoxRows / kNumConsumerWarps; ++i) mine = c.lane == i ? ss[i] : mine;
+  const int t = c.warp + kNumConsumerWarps * c.lane;
+  if (t < T && c.lane < kNormBoxRows / kNumConsumerWarps) {
+    const float r = torch_num ? torch_rsqrt_bf16(rbf(mine / (float)op.k), true) : rsqrtf(mine / (float)op.k + 1e-6f);
+    scale[(t & 1) * (kNormBoxRows / 2) + (t >> 1)] = torch_num ? pack2(r, r) : __float_as_uint(r);
+  }
+  consumer_sync();
+  if (c.tid == 0) {
+    __threadfence_block();
+    c.flags()[6] = (int)c.lin_seq;  // the norm warp may read them
+  }
+}
+
+// The norm warp (warp 11).  Lane l holds 16-byte column l & 15 of a stage's two boxes for token rows (l >> 4), + 2, ...
+__device__ __forceinline__ void norm_loop(Ctx& c) {
+  const KParams& p = c.p;
+  const int S = p.num_stages;
+  volatile int* fl = c.flags();
+  const bool torch_num = p.numerics == NUM_TORCH;
+  const uint32_t x_sub = (uint32_t)p.x_rows * 128u;
+  const int col = c.lane & 15, row0 = c.lane >> 4;
+  const uint32_t scale = smem_u32(wide_tab(c).scale) + (uint32_t)row0 * (kNormBoxRows / 2) * 4u;
+  const uint32_t sub = kStageBytes + (uint32_t)(col >> 3) * x_sub + (uint32_t)row0 * 128u;
+  uint32_t at[4];  // rows row0, + 2, + 4 and + 6 of eight, in the swizzled box
+#pragma unroll
+  for (int u = 0; u < 4; ++u) at[u] = (uint32_t)(2 * u) * 128u + (uint32_t)(((col & 7) ^ (row0 + 2 * u)) << 4);
+  int s = 0;
+  unsigned raw_phase = 0;  // per stage: parity of its next raw box
+  unsigned lin_seq = 0;
+  bool dead = false;
+  for (int iter = 1; !dead; ++iter) {
+    int go;
+    if (!wait_go(c, fl, iter, go)) break;
+    const int T = go & 255;
+    for (int oi = 0; oi < p.num_ops && !dead; ++oi) {
+      const OpDesc& op = p.ops[oi];
+      if (op.type != OP_LINEAR) continue;
+      lin_seq += 1;
+      unsigned total, t0, t1;
+      int G;
+      if (!wide_range(p, op, total, G, t0, t1)) continue;
+      if (!(op.flags & F_NORM_IN)) {  // (its boxes take the stages in turn all the same)
+        s = (int)(((unsigned)s + (t1 - t0)) % (unsigned)S);
+        continue;
+      }
+      // the weights of the first stages: they depend on nobody
+      const uint4* nw = reinterpret_cast<const uint4*>(op.norm_w) + col;
+      const int kvec = op.k >> 3, nkt = op.nkt;
+      int kt = (int)(t0 % (unsigned)nkt);
+      auto weights = [&](int k) { return k * 16 + col < kvec ? __ldg(nw + k * 16) : make_uint4(0u, 0u, 0u, 0u); };
+      uint4 w = weights(kt);
+      if (!wait_lin(c, fl, 6, lin_seq)) { dead = true; break; }
+      __threadfence_block();
+      for (unsigned tile = t0; tile < t1; ++tile) {
+        kt = kt + 1 == nkt ? 0 : kt + 1;
+        const uint4 w_next = weights(kt);
+        if (!mbar_wait(c, c.xraw_bar(s), (raw_phase >> s) & 1u, ST_TIMEOUT_FULL)) { dead = true; break; }
+        uint32_t box = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes + sub, sc = scale;
+        if (torch_num) {
+          // four rows at a time (rows past T, still inside the box, are nobody's): one by one, boxes of 32 rows took longer
+          // than their weight stage (1888 us per step)
+#pragma unroll 1
+          for (int t = 0; t < T; t += 8) {
+            uint4 x[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] = lds128(box + at[u]);
+            const uint4 r = lds128(sc);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const uint32_t ru = u == 0 ? r.x : (u == 1 ? r.y : (u == 2 ? r.z : r.w));
+              sts128(box + at[u], make_uint4(hmul2_bf16(w.x, hmul2_bf16(x[u].x, ru)), hmul2_bf16(w.y, hmul2_bf16(x[u].y, ru)),
+                                             hmul2_bf16(w.z, hmul2_bf16(x[u].z, ru)), hmul2_bf16(w.w, hmul2_bf16(x[u].w, ru))));
+            }
+            box += 1024;
+            sc += 16;
+          }
+        } else {
+#pragma unroll 1
+          for (int t = 0; t < T; t += 8) {
+            const uint4 r = lds128(sc);
+#pragma unroll
+            for (int u = 0; u < 4; u += 2) {
+              const uint4 x0 = lds128(box + at[u]), x1 = lds128(box + at[u + 1]);
+              sts128(box + at[u], scale8(x0, w, __uint_as_float(u == 0 ? r.x : r.z), false));
+              sts128(box + at[u + 1], scale8(x1, w, __uint_as_float(u == 0 ? r.y : r.w), false));
+              if (t + 4 >= T) break;  // (rows t + 4 .. t + 7 are nobody's)
+            }
+            box += 1024;
+            sc += 16;
+          }
+        }
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads the rows through the async proxy
+        __syncwarp();
+        if (c.lane == 0) mbar_arrive(c.xfull_bar(s));
+        raw_phase ^= 1u << s;
+        if (++s == S) s = 0;
+        w = w_next;
+      }
+    }
+    if (p.mode == MODE_ONEPASS) break;
+  }
 }
 
 // ------------------------------------------------------------------------------------
@@ -295,6 +458,7 @@ __device__ __forceinline__ void wide_epilogue(Ctx& c, const OpDesc& op, int blk,
   const bool okc = col < op.n;
   const bool push = MK_XF(op, F_PUSH) != 0;
   const bool with_res = (op.flags & F_RESIDUAL) && (!(op.flags & F_RES_RANK0) || p.rank == 0);
+  float sq[2 * NC <= kNormBoxRows ? NC : 1];
   const bool rnd = p.numerics == NUM_TORCH && !push;  // (pushed partial sums stay fp32: rounded once, after the ranks are added up)
 #pragma unroll
   for (int i = 0; i < NC; ++i) {
@@ -307,6 +471,30 @@ __device__ __forceinline__ void wide_epilogue(Ctx& c, const OpDesc& op, int blk,
     if (okc && i < nlive) {
       if (push) xchg_push1(p, xchg_next(c), tok0 + i, col, y);
       else out[(size_t)(tok0 + i) * op.ld_out + col] = __float2bfloat16_rn(y);
+    }
+    if constexpr (2 * NC <= kNormBoxRows) {
+      y = okc ? rbf(y) : 0.f;
+      sq[i] = p.numerics == NUM_TORCH ? rbf(y * y) : y * y;
+    }
+  }
+  if constexpr (2 * NC <= kNormBoxRows) {
+    if (op.flags & F_ROW_SUMS) {
+      // NC sums over the warp's 32 rows: halves change places until a lane is left with one token, then the rest is added up
+      int tok = 0;
+#pragma unroll
+      for (int n = NC, o = 16; n > 1; n >>= 1, o >>= 1) {
+        const bool upper = (c.lane & o) != 0;
+#pragma unroll
+        for (int i = 0; i < n / 2; ++i) {
+          const float give = upper ? sq[i] : sq[i + n / 2];
+          sq[i] = (upper ? sq[i + n / 2] : sq[i]) + __shfl_xor_sync(0xffffffffu, give, o);
+        }
+        if (upper) tok += n / 2;
+      }
+#pragma unroll
+      for (int o = 16 / NC; o > 0; o >>= 1) sq[0] += __shfl_xor_sync(0xffffffffu, sq[0], o);
+      if ((c.lane & (32 / NC - 1)) == 0 && tok < nlive)
+        reinterpret_cast<float*>(op.ll_out)[(size_t)(tok0 + tok) * (size_t)op.ll_res_op + blk * 4 + (row >> 5)] = sq[0];
     }
   }
   if (op.flags & F_ARGMAX) {
@@ -522,6 +710,9 @@ __device__ __forceinline__ void op_linear_wide(Ctx& c, const OpDesc& op, int T) 
   if (op_barrier(c, op)) return;
   c.lin_seq += 1;
   if (c.tid == 0) c.flags()[4] = (int)c.lin_seq;  // the activation producer may now read this op's input
+  if constexpr (2 * NC <= kNormBoxRows) {
+    if (op.flags & F_NORM_IN) wide_row_scales(c, op, T);
+  }
   linear_wide<NC>(c, op, T);
   if (MK_XF(op, F_PUSH)) c.ar_seq += 1;  // every CTA counts the exchange, with or without rows of its own
 }

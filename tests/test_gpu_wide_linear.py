@@ -131,3 +131,38 @@ def test_norm_of_rows_wider_than_shared_memory(T, K, numerics):
     # rounding border may get the next one: 2^-7, and 2^-8 for each of the two products.
     bf16_close(od, O.mpk_rmsnorm(x, wn) if numerics == "mpk" else O.ref_rmsnorm(x, wn), 8e-3 if numerics == "mpk" else 2 ** -6, "rmsnorm")
     k.finalize()
+
+
+@pytest.mark.parametrize("numerics", ["mpk", "torch"])
+@pytest.mark.parametrize("T,N,K,M", [(3, 512, 512, 256), (8, 1160, 384, 200), (16, 4096, 128, 136), (17, 1024, 1096, 640), (32, 136, 256, 2056), (33, 512, 512, 256)])
+def test_norm_in_the_activation_boxes(T, N, K, M, numerics):
+    """linear + residual -> RMSNorm -> linear -> RMSNorm -> linear: up to 32 tokens (8 with fp32 products) the norms are
+    applied to the boxes of the linear behind them, from sums of squares of the linear before (which itself may have had its
+    rows normalised that way)."""
+    x, r = _rand((T, K), 21), _rand((T, N), 22, 2.0)
+    w1, w2, w3 = _rand((N, K), 23, 0.05), _rand((M, N), 24, 0.05), _rand((N, M), 25, 0.05)
+    n1, n2 = (1 + 0.3 * _rand((N,), 26).float()).to(BF), (1 + 0.3 * _rand((M,), 27).float()).to(BF)
+    k, meta, _ = onepass_kernel(T, numerics=numerics)
+    h1, h2 = k.new_tensor(dims=(T, N), name="h1"), k.new_tensor(dims=(T, M), name="h2")
+    a1, a2 = k.new_tensor(dims=(T, N), name="a1"), k.new_tensor(dims=(T, M), name="a2")
+    od = torch.zeros(T, N, dtype=BF, device="cuda")
+    at = lambda name, t: k.attach_input(t.cuda(), name)
+    grid = dict(grid_dim=(8, 1, 1), block_dim=(128, 1, 1))
+    k.linear_with_residual_layer(input=at("x", x), weight=at("w1", w1), residual=at("r", r), output=h1, **grid)
+    k.rmsnorm_layer(input=h1, weight=at("n1", n1), output=a1, **grid)
+    k.linear_layer(input=a1, weight=at("w2", w2), output=h2, **grid)
+    k.rmsnorm_layer(input=h2, weight=at("n2", n2), output=a2, **grid)
+    k.linear_layer(input=a2, weight=at("w3", w3), output=k.attach_input(od, "o"), **grid)
+    k.compile()
+    assert k.describe().count("rmsnorm in the activation boxes") == (2 if T <= (8 if numerics == "mpk" else 32) else 0)
+    norm = O.mpk_rmsnorm if numerics == "mpk" else O.ref_rmsnorm
+    rows = (x.float() @ w1.float().T).to(BF)  # "torch": rounded before the residual is added
+    ref = O.mpk_linear(x, w1, residual=r) if numerics == "mpk" else (rows.float() + r.float()).to(BF)
+    ref = O.mpk_linear(norm(O.mpk_linear(norm(ref, n1), w2), n2), w3)
+    for _ in range(2):
+        k()
+        # Two norms and three linears, each rounded to bf16.  A value at a rounding border may fall the other way behind every one
+        # of them (2^-8 of it), independently over the terms of the next sum; "torch": a row's bf16 scale may take the
+        # neighbouring value besides (2^-7 of the whole row).  Four roundings and two scales of at most 2^-8 and 2^-7.
+        bf16_close(od, ref, 1e-2 if numerics == "mpk" else 2 ** -6 + 1e-2, f"{T}x{N}x{K}x{M}")
+    k.finalize()
