@@ -2047,6 +2047,30 @@ __device__ __forceinline__ void op_rmsnorm(Ctx& c, const OpDesc& op, int T) {
   }
   if (op_barrier(c, op)) return;
   for (int tok = blockIdx.x; tok < T; tok += gridDim.x) {
+    if (pre && !MK_XF(op, F_GATHER_IN)) {
+      // up to 8192 columns: the row stays in registers from the load to the store
+      const bool torch_num = c.p.numerics == NUM_TORCH;
+      const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)tok * op.ld_in);
+      uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(op.out) + (size_t)tok * op.ld_out);
+      const int kvec = op.n >> 3;
+      uint4 raw[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) raw[i] = c.tid + kNumConsumers * i < kvec ? __ldcg(src + c.tid + kNumConsumers * i) : make_uint4(0, 0, 0, 0);
+      float ss = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) ss = sumsq8(raw[i], torch_num, ss);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      float* red = c.red();
+      if (c.lane == 0) red[c.warp] = ss;
+      consumer_sync();
+      const float r = row_rms_scale(red, 0, kNumConsumerWarps, op.n, torch_num);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (c.tid + kNumConsumers * i < kvec) dst[c.tid + kNumConsumers * i] = scale8(raw[i], pre_w[i], r, torch_num);
+      consumer_sync();
+      continue;
+    }
     if (op.n > kNormStagedCols && !MK_XF(op, F_GATHER_IN)) {
       rmsnorm_wide_row(c, op, tok);
       continue;

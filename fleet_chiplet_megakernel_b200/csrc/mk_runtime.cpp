@@ -44,11 +44,10 @@ constexpr int kGateUpUnit = 4;     // fused gate/up weights are laid out [4 gate
 constexpr int kMaxStepTimes = 16384;
 
 // The wide path's shared memory.  Ring: stages of 32 KB of weights and two activation boxes of x_rows token rows.  As many
-// stages as leave the CTA within the 164 KB carve-out (3 up to 32 token rows, 2 beyond): what the carve-out takes is L1,
-// and the kernel's own state, spills and metadata live there.  Measured with 5, 4, 3 and 2 stages, us per step of 6 layers:
-// 512 hidden, 4 requests 423, 364, 328, 310 (409 on the path of up to 16 tokens that kept to 164 KB); 1152 hidden, 8
-// requests of 300 tokens 557, 489, 461, 439; 4096 hidden, 8 of 300 1047, 986, 961, 1004, 32 requests 1117, 1063, 1034,
-// 1084; 64 requests (48 KB stages, 4, 3 and 2 of them) 1340, 1285, 1290; 128 prompt tokens (64 KB, 3 and 2) 1805, 1735.
+// stages as leave the CTA within the 164 KB carve-out (4 up to 16 token rows, 3 up to 64, 2 beyond; the attention's scratch
+// is 9 KB for that reason).  12 layers of 8B width, us per step: 8 requests with 3, 4 and 5 stages 1477, 1453, 1454; 32
+// requests 1588, 1562, 1566; 64 requests with 2, 3 and 4 1942, 1823, 1826; 2048 hidden, 8 requests with 3, 4 and 5 910, 893,
+// 904; more only pays from 65 token rows on (2 and 3: 2377 and 2243).
 constexpr int kWideFixed = 1024 /*alignment slack*/ + mk::kWideRedBytes + 2048 /*barriers and flags, op descriptors*/;
 int wide_x_rows(int tokens) { return tokens <= 16 ? 16 : (tokens <= 32 ? 32 : (tokens <= 64 ? 64 : 128)); }
 int wide_stage_bytes(int tokens) { return mk::kStageBytes + 2 * wide_x_rows(tokens) * 128; }
@@ -1360,13 +1359,14 @@ static int compile_program(mk_handle* h, bool first) {
       if (spans * (kp + 8) * 2 + 16 > x_budget) return h->fail(MK_E_UNSUPPORTED, "moe linear: K=%d is too wide", p.k);
       x_bytes = std::max(x_bytes, spans * (kp + 8) * 2 + 16);
     } else if (p.type == mk::OP_RMSNORM) {
-      if (p.n <= mk::kNormStagedCols || (p.flags & mk::F_GATHER_IN)) x_bytes = std::max(x_bytes, ((p.n + 63) / 64 * 64 + 8) * 2 + 16);
+      // (rows of up to 8192 columns that are not gathered from the ranks stay in registers)
+      if ((p.n > 8192 && p.n <= mk::kNormStagedCols) || (p.flags & mk::F_GATHER_IN)) x_bytes = std::max(x_bytes, ((p.n + 63) / 64 * 64 + 8) * 2 + 16);
     } else if (p.type == mk::OP_ATTN) {
       has_attn = true;
       // row-owner path: q heads and the new k (bf16), combine slots of 16 half-warps x 128 floats, (max, sum) pairs, merge scratch
       if (rows_mode) x_bytes = std::max(x_bytes, 9 * 256 + 4 * 4 * (mk::kHeadDim + 2) * 4 + 2 * kAttnMaxChunks * 8 * 4 + 64 + 256);
-      // wide path: 2 KB per warp (q rows, then combine slots), (max, sum) pairs; the QKV epilogue transposes through the same 16 KB
-      else x_bytes = std::max(x_bytes, 16384 + mk::kNumConsumerWarps * 16 * 8);
+      // wide path: 1 KB per warp to combine their sums, (max, sum) pairs; the QKV epilogue transposes through the same 8 KB
+      else x_bytes = std::max(x_bytes, 8192 + mk::kNumConsumerWarps * 8 * 8);
     }
   }
   if (has_moe) x_bytes += 512;  // the expert ids of the pairs, for the producer (routing folded into the expert linear)

@@ -77,6 +77,7 @@ __device__ __forceinline__ bool wide_range(const KParams& p, const OpDesc& op, u
 constexpr int kWideTab = 128;  // the host admits at most 128 batched tokens
 struct WideTab {
   int pos[kWideTab], slot[kWideTab], kvb[kWideTab], req[kWideTab], grp[kWideTab];
+  int fresh[kWideTab];  // first position of the token's request whose K/V row is written in this iteration
   int plan[8];
   int scan[8];
   // of the linear op at hand: what its input norm multiplies a token's row with (fp32, or a pair of bf16), even tokens first
@@ -101,6 +102,7 @@ __device__ __forceinline__ void wide_fill_tokens(Ctx& c, int T) {
         tab.pos[t] = kvlen - (q1 - t);
         tab.kvb[t] = first;
         tab.req[t] = r;
+        tab.fresh[t] = kvlen - (q1 - q0);
       }
     }
   }
@@ -440,19 +442,23 @@ __device__ __forceinline__ void wide_epilogue(Ctx& c, const OpDesc& op, int blk,
     return;
   }
   if (op.flags & F_QKV_PREP) {
-    // a row block is one head vector of every token: transposed through shared memory (32 token rows per column
-    // half), then a half-warp per token.  The four warps of a half meet on a named barrier of their own.
+    // a row block is one head vector of every token: transposed through shared memory (16 token rows per column
+    // half and round), then a half-warp per token.  The four warps of a half meet on a named barrier of their own.
     const int half = c.warp >> 2, q = c.warp & 3, l16 = c.lane & 15;
     const int qpk = op.aux1 / op.aux0;
-    __nv_bfloat16* buf = reinterpret_cast<__nv_bfloat16*>(c.smem + p.x_off) + half * 32 * kHeadDim;
+    constexpr int kRound = NC < 16 ? NC : 16;
+    __nv_bfloat16* buf = reinterpret_cast<__nv_bfloat16*>(c.smem + p.x_off) + half * kRound * kHeadDim;
 #pragma unroll
-    for (int i = 0; i < NC; ++i) buf[i * kHeadDim + row] = __float2bfloat16_rn(v[i]);
-    asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
+    for (int c0 = 0; c0 < NC; c0 += kRound) {
+#pragma unroll
+      for (int i = 0; i < kRound; ++i) buf[i * kHeadDim + row] = __float2bfloat16_rn(v[c0 + i]);
+      asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
 #pragma unroll 1
-    for (int t = q * 2 + (c.lane >> 4); t < NC; t += 8)
-      wide_store_head(c, op, reinterpret_cast<const uint4*>(buf + t * kHeadDim)[l16], tok0 + (t < nlive ? t : 0), blk / (qpk + 2), blk % (qpk + 2),
-                      t < nlive, l16);
-    asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
+      for (int t = q * 2 + (c.lane >> 4); t < kRound; t += 8)
+        wide_store_head(c, op, reinterpret_cast<const uint4*>(buf + t * kHeadDim)[l16], tok0 + (c0 + t < nlive ? c0 + t : 0), blk / (qpk + 2),
+                        blk % (qpk + 2), c0 + t < nlive, l16);
+      asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory");
+    }
     return;
   }
   const bool okc = col < op.n;
@@ -748,6 +754,7 @@ __device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
 struct WideTask {
   int t0, nt, h, ch, nch;  // first token, tokens, kv head, chunk, chunks
   int p0, p1, L0, kvb;     // positions [p0, p1) of this chunk; length the first token sees; page-table base
+  int fresh;               // first position whose row this iteration writes
 };
 
 // Query groups, warps per task and chunking of the iteration: the same in every layer, worked out by the first
@@ -939,8 +946,10 @@ __device__ __forceinline__ bool bar_any(int id, int nthr, bool pred) {
   return r != 0u;
 }
 
-// One task by W warps.  `reg`: the group's shared memory (W x 2 KB), `ml`: [warps of the CTA][8] (max, sum) pairs.
-__device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTask& a, int W, int gi, uint8_t* reg, float2* ml) {
+// One task by W warps.  `reg`: the group's shared memory (W KB), `ml`: [warps of the CTA][8] (max, sum) pairs.  `loaded`: the
+// first tile's K and V rows are in kr and vr already, but for the rows that this iteration writes.
+__device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTask& a, int W, int gi, uint8_t* reg, float2* ml, bool loaded,
+                                            uint4 (&kr)[2][4], uint4 (&vr)[4][2]) {
   const KParams& p = c.p;
   const int lane = c.lane, g = lane >> 2, j = lane & 3;
   const int HKV = op.aux0, qpk = op.aux1 / HKV, rows = a.nt * qpk;
@@ -948,42 +957,21 @@ __device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const Wide
   const float sc = 1.4426950408889634f * 0.08838834764831845f;  // log2(e) / sqrt(128)
   const int psh = p.page_shift;
   const int ntiles = (a.p1 - a.p0 + 15) >> 4;
-  uint4 kr[2][4], vr[4][2];
   int ti = sub;
-  int pg = 0;
-  if (ti < ntiles && psh >= 4) pg = wide_page(c, a, a.p0 + 16 * ti);
-  // q rows -> shared memory, [row][256 B]; rows past the group's are zero.  64-byte halves trade places in odd rows and
-  // 8-byte halves in rows with bit 1 set: the 8-byte fragment reads of four rows then cover all banks.  All loads of a
-  // thread (at most four), then the first K and V rows, then the stores: one round trip instead of one per row (with
-  // the clamped row loads, the op's start took 5.4 us instead of 7.7 at eight requests of 300 tokens).
+  // Row g of the q rows as A fragments: 8 dims from 32 i + 8 j are k steps 2 i and 2 i + 1; rows past the group's are zero.
+  uint4 qf[4];
   {
-    constexpr int NQ = 8 * 16;
-    const int qsh = 31 - __clz(qpk);  // (1, 2, 4 or 8 q heads per kv head)
-    const __nv_bfloat16* q0 = reinterpret_cast<const __nv_bfloat16*>(op.out2) + (size_t)a.t0 * op.ld_out2 + (size_t)a.h * qpk * kHeadDim;
-    uint4* sq = reinterpret_cast<uint4*>(reg);
-    uint4 qv[4];
+    const __nv_bfloat16* q0 = reinterpret_cast<const __nv_bfloat16*>(op.out2) + (size_t)(a.t0 + g / qpk) * op.ld_out2 + (size_t)(a.h * qpk + g % qpk) * kHeadDim + 8 * j;
 #pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      const int i = gtid + x * nthr, r = i >> 4;
-      qv[x] = make_uint4(0, 0, 0, 0);
-      if (i < NQ && r < rows) qv[x] = __ldcg(reinterpret_cast<const uint4*>(q0 + (size_t)(r >> qsh) * op.ld_out2 + (r & (qpk - 1)) * kHeadDim) + (i & 15));
-    }
-    if (ti < ntiles) {
-      wide_load_k(c, op, a, a.p0 + 16 * ti, pg, kr);
-      wide_load_v(c, op, a, a.p0 + 16 * ti, pg, vr);
-    }
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      const int i = gtid + x * nthr, r = i >> 4;
-      if (i < NQ) sq[r * 16 + ((i & 15) ^ ((r & 1) << 2))] = (r & 2) ? make_uint4(qv[x].z, qv[x].w, qv[x].x, qv[x].y) : qv[x];
-    }
+    for (int i = 0; i < 4; ++i) qf[i] = g < rows ? __ldcg(reinterpret_cast<const uint4*>(q0 + 32 * i)) : make_uint4(0, 0, 0, 0);
+  }
+  if (ti < ntiles && (!loaded || a.p0 + 16 * ti + 15 >= a.fresh)) {
+    const int pg = psh >= 4 ? wide_page(c, a, a.p0 + 16 * ti) : 0;
+    wide_load_k(c, op, a, a.p0 + 16 * ti, pg, kr);
+    wide_load_v(c, op, a, a.p0 + 16 * ti, pg, vr);
   }
   int pgn = (psh >= 4 && ti + W < ntiles) ? wide_page(c, a, a.p0 + 16 * (ti + W)) : 0;
-  if (W > 1) asm volatile("bar.sync %0, %1;" ::"r"(2 + gi), "r"(nthr) : "memory");
-  else __syncwarp();
   MK_STAMP(c, 1);
-  const char* sq = reinterpret_cast<const char*>(reg) + g * 256 + 16 * j;
-  const int swz = ((g & 1) << 6) | ((g & 2) << 2);
   float m = -INFINITY, l = 0.f;  // of row g
   float oacc[8][4];  // tile t of 16 dims: {dim 8 g + t of rows 2 j and 2 j + 1, dim 64 + 8 g + t of the same}
 #pragma unroll
@@ -998,7 +986,7 @@ __device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const Wide
     float s0[2] = {0.f, 0.f}, s1[2] = {0.f, 0.f}, z0[2] = {0.f, 0.f}, z1[2] = {0.f, 0.f};
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
-      const uint2 qa = *reinterpret_cast<const uint2*>(sq + ((64 * (s >> 1) + 8 * (s & 1)) ^ swz));
+      const uint2 qa = (s & 1) ? make_uint2(qf[s >> 1].z, qf[s >> 1].w) : make_uint2(qf[s >> 1].x, qf[s >> 1].y);
       const uint4 &k0 = kr[0][s >> 1], &k1 = kr[1][s >> 1];
       wide_mma_qk((s & 1) ? z0 : s0, qa.x, qa.y, (s & 1) ? k0.z : k0.x, (s & 1) ? k0.w : k0.y);
       wide_mma_qk((s & 1) ? z1 : s1, qa.x, qa.y, (s & 1) ? k1.z : k1.x, (s & 1) ? k1.w : k1.y);
@@ -1078,43 +1066,66 @@ __device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const Wide
     if (__any_sync(0xffffffffu, chk != 0.f)) wide_attend_exact(c.p, op, a, W, out, nullptr);
     return;
   }
-  // The warps of the task meet in shared memory, four rows at a time (the slots take the place of the q rows).
+  // The warps of the task meet in shared memory, four rows at a time: the upper half leaves its sums in W / 2 slots, the
+  // lower half adds its own to them, in place, and all finish the rows from there.
   const uint32_t nbar = (uint32_t)(2 + gi);
+  const int H = W >> 1;
   if (j == 0) ml[c.warp * 8 + g] = make_float2(m, l);
   float* slot0 = reinterpret_cast<float*>(reg);
   float* part = p.attn_part + ((size_t)a.t0 * HKV * p.attn_max_chunks * qpk + (size_t)(a.h * p.attn_max_chunks + a.ch) * rows) * (kHeadDim + 2);
 #pragma unroll
   for (int rb = 0; rb < 2; ++rb) {
     if (4 * rb >= rows) break;
-    asm volatile("bar.sync %0, %1;" ::"r"(nbar), "r"(nthr) : "memory");
-    if ((j >> 1) == rb) {
-      float* dst = slot0 + (size_t)sub * 4 * kHeadDim + 2 * (j & 1) * kHeadDim + 8 * g;
+    if (rb > 0) asm volatile("bar.sync %0, %1;" ::"r"(nbar), "r"(nthr) : "memory");  // (the slots are free again)
+    const bool mine = (j >> 1) == rb;  // this lane holds rows 2 j and 2 j + 1
+    float* own = slot0 + (size_t)(sub & (H - 1)) * 4 * kHeadDim + 2 * (j & 1) * kHeadDim + 8 * g;
+    if (mine && sub >= H) {
 #pragma unroll
       for (int y = 0; y < 2; ++y)
 #pragma unroll
         for (int x = 0; x < 2; ++x)
 #pragma unroll
           for (int i = 0; i < 8; i += 4)
-            *reinterpret_cast<float4*>(dst + y * kHeadDim + 64 * x + i) =
+            *reinterpret_cast<float4*>(own + y * kHeadDim + 64 * x + i) =
                 make_float4(oacc[i][2 * x + y], oacc[i + 1][2 * x + y], oacc[i + 2][2 * x + y], oacc[i + 3][2 * x + y]);
+    }
+    asm volatile("bar.sync %0, %1;" ::"r"(nbar), "r"(nthr) : "memory");
+    const float2* mlt = ml + (c.warp - sub) * 8;  // the task's pairs
+    if (mine && sub < H) {
+#pragma unroll
+      for (int y = 0; y < 2; ++y) {
+        const float m0 = mlt[sub * 8 + 2 * j + y].x, m1 = mlt[(sub + H) * 8 + 2 * j + y].x;
+        const float M = fmaxf(m0, m1), Ms = M == -INFINITY ? 0.f : M;
+        const float f0 = exp2f(m0 - Ms), f1 = exp2f(m1 - Ms);
+#pragma unroll
+        for (int x = 0; x < 2; ++x)
+#pragma unroll
+          for (int i = 0; i < 8; i += 4) {
+            float4* q = reinterpret_cast<float4*>(own + y * kHeadDim + 64 * x + i);
+            const float4 o = *q;
+            *q = make_float4(fmaf(f1, o.x, f0 * oacc[i][2 * x + y]), fmaf(f1, o.y, f0 * oacc[i + 1][2 * x + y]),
+                             fmaf(f1, o.z, f0 * oacc[i + 2][2 * x + y]), fmaf(f1, o.w, f0 * oacc[i + 3][2 * x + y]));
+          }
+      }
     }
     asm volatile("bar.sync %0, %1;" ::"r"(nbar), "r"(nthr) : "memory");
 #pragma unroll 1
     for (int e = gtid; e < 4 * 32; e += nthr) {  // (row of the round, four dims)
       const int r = 4 * rb + (e >> 5), d = (e & 31) * 4;
       if (r >= rows) continue;
-      const float2* mlr = ml + (c.warp - sub) * 8 + r;
+      const float2* mlr = mlt + r;
       float M = -INFINITY;
       for (int w = 0; w < W; ++w) M = fmaxf(M, mlr[w * 8].x);
       const float Ms = M == -INFINITY ? 0.f : M;
       float L = 0.f;
       float4 O = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
-      for (int w = 0; w < W; ++w) {
-        const float2 v = mlr[w * 8];
-        const float f = exp2f(v.x - Ms);
+      for (int w = 0; w < H; ++w) {
+        const float2 v0 = mlr[w * 8], v1 = mlr[(w + H) * 8];
+        L = fmaf(exp2f(v0.x - Ms), v0.y, L);
+        L = fmaf(exp2f(v1.x - Ms), v1.y, L);
+        const float f = exp2f(fmaxf(v0.x, v1.x) - Ms);
         const float4 o4 = *reinterpret_cast<const float4*>(slot0 + (size_t)w * 4 * kHeadDim + (e >> 5) * kHeadDim + d);
-        L = fmaf(f, v.y, L);
         O.x = fmaf(f, o4.x, O.x);
         O.y = fmaf(f, o4.y, O.y);
         O.z = fmaf(f, o4.z, O.z);
@@ -1198,43 +1209,64 @@ __device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const Wide
 
 __device__ __forceinline__ void op_attention_wide(Ctx& c, const OpDesc& op, int T) {
   const KParams& p = c.p;
-  if (op_barrier(c, op)) return;
-  if (p.debug_flags & 2) return;  // measurement aid: the op keeps its barrier and does nothing else
+  // What does not depend on the QKV linear before the op is done ahead of its barrier: the plan, and the K and V rows of this warp's
+  // first tile.  Rows that this iteration writes are loaded again behind the barrier (the others then hit L2).
+  // (The arrival comes first: behind the page look-up it held the others up, 3 % of a step of a small model.)
+  if (op.flags & F_SYNC_BEFORE) grid_arrive(c);
   const int key = op.aux0 * 256 + op.aux1;
   if (c.attn_iter != key) {
     wide_plan_attention(c, op, T);
     c.attn_iter = key;
   }
-  if (!(op.flags & F_QKV_READY)) {
-    attn_prepare_rows(c, op, T);
-    grid_sync(c);  // every token's K/V row is in the cache before any is read
-    c.dead = c.flags()[3] != 0;
-    if (c.dead) return;
-  }
-  MK_STAMP(c, 0);
   const WideTab& tab = wide_tab(c);
   const int HKV = op.aux0;
   const int W = tab.plan[1], nch = tab.plan[2], CS = tab.plan[3];
   const int ntasks = tab.plan[0] * HKV * nch, per = kNumConsumerWarps / W;
   const int gi = c.warp / W;
-  uint8_t* reg = c.smem + p.x_off + (size_t)gi * W * 2048;
-  float2* ml = reinterpret_cast<float2*>(c.smem + p.x_off + 16384);
+  uint8_t* reg = c.smem + p.x_off + (size_t)gi * W * 1024;
+  float2* ml = reinterpret_cast<float2*>(c.smem + p.x_off + 8192);
+  uint4 kr[2][4], vr[4][2];
+  bool loaded = false;
 #pragma unroll 1
-  for (int task = blockIdx.x + gridDim.x * gi; task < ntasks; task += gridDim.x * per) {
+  for (int task = blockIdx.x + gridDim.x * gi, first = 1;; task += gridDim.x * per, first = 0) {
     WideTask a;
-    a.ch = task % nch;
-    const int pr = task / nch;
-    a.h = pr % HKV;
-    const int e = tab.grp[pr / HKV];
-    a.t0 = e & 255;
-    a.nt = e >> 8;
-    a.L0 = tab.pos[a.t0] + 1;
-    a.kvb = tab.kvb[a.t0];
-    const int L = a.L0 + a.nt - 1;
-    a.p0 = a.ch * CS;
-    a.p1 = min(L, a.p0 + CS);
-    a.nch = (L + CS - 1) / CS;
-    if (a.p0 >= L || a.L0 <= 0) continue;  // (uniform within the task's warps)
-    wide_attend(c, op, a, W, gi, reg, ml);
+    a.p0 = a.p1 = a.fresh = 0;
+    bool live = task < ntasks;
+    if (live) {
+      a.ch = task % nch;
+      const int pr = task / nch;
+      a.h = pr % HKV;
+      const int e = tab.grp[pr / HKV];
+      a.t0 = e & 255;
+      a.nt = e >> 8;
+      a.L0 = tab.pos[a.t0] + 1;
+      a.kvb = tab.kvb[a.t0];
+      a.fresh = tab.fresh[a.t0];
+      const int L = a.L0 + a.nt - 1;
+      a.p0 = a.ch * CS;
+      a.p1 = min(L, a.p0 + CS);
+      a.nch = (L + CS - 1) / CS;
+      live = a.p0 < L && a.L0 > 0;  // (uniform within the task's warps)
+    }
+    if (first) {
+      const int pos0 = a.p0 + 16 * (c.warp & (W - 1));
+      if (live && pos0 < min(a.p1, a.fresh) && !(p.debug_flags & 2)) {
+        const int pg = p.page_shift >= 4 ? wide_page(c, a, pos0) : 0;
+        wide_load_k(c, op, a, pos0, pg, kr);
+        wide_load_v(c, op, a, pos0, pg, vr);
+        loaded = true;
+      }
+      if (op_barrier(c, op)) return;
+      if (p.debug_flags & 2) return;  // measurement aid: the op keeps its barrier and does nothing else
+      if (!(op.flags & F_QKV_READY)) {
+        attn_prepare_rows(c, op, T);
+        grid_sync(c);  // every token's K/V row is in the cache before any is read
+        c.dead = c.flags()[3] != 0;
+        if (c.dead) return;
+      }
+      MK_STAMP(c, 0);
+    }
+    if (task >= ntasks) break;
+    if (live) wide_attend(c, op, a, W, gi, reg, ml, first && loaded, kr, vr);
   }
 }
