@@ -1278,13 +1278,6 @@ __device__ __forceinline__ void op_linear_rows(Ctx& c, const OpDesc& op, int T) 
 // ------------------------------------------------------------------------------------
 // attention: QK-norm + RoPE + KV append + paged split-KV GQA decode + merge
 // ------------------------------------------------------------------------------------
-// Work split inside a CTA: warp w serves q head (w % qpk) of the task's kv-head group and
-// position group (w / qpk); its two half-warps take alternate positions.  One head
-// vector is spread over the 16 lanes of a half-warp, 8 dims each, so a cached K or V
-// row of 256 bytes is one 16-byte load per lane.  The code is kept small on purpose:
-// the megakernel switches between task bodies thousands of times per step and every
-// switch refills the instruction cache.
-
 // bf16 reciprocal square root the way the reference PyTorch model's CPU kernels round it:
 // `dbl` = scalar loop (sqrt rounded to bf16 before the reciprocal), else vector loop.
 __device__ __forceinline__ float torch_rsqrt_bf16(float var, bool dbl) {
@@ -1337,95 +1330,11 @@ __device__ __forceinline__ F8 head_norm_rope(F8 xin, uint4 wv, uint4 csv, uint4 
   return xin;
 }
 
-// Everything a (token, kv head, chunk) task needs that does not depend on the QKV
-// rows of this layer: lengths, page numbers, norm weights, cos/sin, and the first
-// four cached K/V rows of this half-warp.  Loaded before the op's grid barrier for
-// the CTA's first task, so that only the q path is left on the critical path.
-struct AttnTask {
-  int t, h, ch, L, p0, p1, nch, kv_base, new_page;
-  bool valid;
-  uint4 kr[4], vr[4];
-};
-
+// Tiles of 16 positions that one CTA of the row-owner path takes alone, see op_attention.  Beyond, the chunks' merge (two round
+// trips) costs less than a third round of tiles.  12 layers of 8B width, one request, us per step with 8, 16, 24 and 32:
+// 1120, 1112, 1112, 1112 at 200 positions, 1118, 1118, 1135, 1135 at 300, 1124, 1126, 1125, 1163 at 440.
+constexpr int kAttnSoloTiles = 16;
 constexpr int kAttnLensMax = 128;  // requests (the host admits at most 128 batched tokens)
-
-struct AttnPlan {
-  int HKV, qpk, CS, nch_max, ntasks;
-  int gi, ngroups;  // this half-warp's position group and the number of groups
-};
-
-// rows of positions p0 + (it0 + u) * ngroups + gi, u = 0..3
-// `pgc`: this half-warp's four cached page numbers (the metadata of an iteration is the same
-// for all layers, so only the first attention op of an iteration looks them up: `fill`).
-// `pgs`: when not null, the page numbers of page slots (a.p0 >> page_shift) + 0..15 of the request,
-// cached in shared memory (the row loop would otherwise wait for a page look-up before every load).
-__device__ __forceinline__ void attn_fetch_rows(const Ctx& c, const OpDesc& op, const AttnPlan& pl, const AttnTask& a,
-                                                int it0, int l16, uint4* kr, uint4* vr, int* pgc = nullptr,
-                                                bool fill = false, const int* pgs = nullptr) {
-  const int psh = c.p.page_shift, pmask = c.p.page_size - 1;
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const int j = a.p0 + (it0 + u) * pl.ngroups + pl.gi;
-    kr[u] = make_uint4(0, 0, 0, 0);
-    vr[u] = make_uint4(0, 0, 0, 0);
-    if (j < a.p1 && j != a.L - 1) {
-      int pg;
-      const int slot = (j >> psh) - (a.p0 >> psh);
-      if (pgc != nullptr && !fill) {
-        pg = pgc[u];
-      } else if (pgs != nullptr && slot < 16) {
-        pg = pgs[slot];
-      } else {
-        pg = __ldcg(c.p.kv_indices + a.kv_base + (j >> psh));
-        if (pgc != nullptr) pgc[u] = pg;  // all 16 lanes store the same number
-      }
-      const size_t src = ((((size_t)pg << psh) + (j & pmask)) * pl.HKV + a.h) * kHeadDim;
-      kr[u] = __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.k_cache) + src) + l16);
-      vr[u] = __ldcg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.v_cache) + src) + l16);
-    }
-  }
-}
-
-// (The norm weights and the cos/sin row of the position are fetched later, next to the q/k rows: held from here on,
-// they were spilled, and a spill waits for its load.)
-__device__ __forceinline__ void attn_prepare(const Ctx& c, const OpDesc& op, const AttnPlan& pl, const int* lens, int task,
-                                          int l16, AttnTask& a, int* pgc = nullptr, bool fill = false,
-                                          int* geom = nullptr) {
-  // `geom`: the task's geometry as the iteration's first attention op worked it out
-  // ([0] valid, then t, h, ch, L, p0, p1, nch, kv_base): the other layers skip the divisions.
-  if (geom != nullptr && !fill) {
-    a.valid = geom[0] != 0;
-    if (!a.valid) return;
-    a.t = geom[1]; a.h = geom[2]; a.ch = geom[3]; a.L = geom[4];
-    a.p0 = geom[5]; a.p1 = geom[6]; a.nch = geom[7]; a.kv_base = geom[8];
-  } else {
-    a.valid = false;
-    if (geom != nullptr && c.tid == 0) geom[0] = 0;
-    if (task >= pl.ntasks) return;
-    a.ch = task % pl.nch_max;
-    a.h = (task / pl.nch_max) % pl.HKV;
-    a.t = task / (pl.nch_max * pl.HKV);
-    a.L = lens[a.t];
-    a.p0 = a.ch * pl.CS;
-    if (a.p0 >= a.L || a.L <= 0) return;
-    a.valid = true;
-    a.p1 = min(a.L, a.p0 + pl.CS);
-    a.nch = (a.L + pl.CS - 1) / pl.CS;
-    a.kv_base = lens[kAttnLensMax + a.t];
-    if (geom != nullptr && c.tid == 0) {
-      geom[0] = 1;
-      geom[1] = a.t; geom[2] = a.h; geom[3] = a.ch; geom[4] = a.L;
-      geom[5] = a.p0; geom[6] = a.p1; geom[7] = a.nch; geom[8] = a.kv_base;
-    }
-  }
-  if (pgc != nullptr && !fill) {
-    a.new_page = pgc[4];
-  } else {
-    a.new_page = (a.p1 == a.L) ? __ldcg(c.p.kv_indices + a.kv_base + ((a.L - 1) >> c.p.page_shift)) : 0;
-    if (pgc != nullptr) pgc[4] = a.new_page;
-  }
-  attn_fetch_rows(c, op, pl, a, 0, l16, a.kr, a.vr, pgc, fill);
-}
 
 // Merge of a (request, kv head)'s chunks by the CTA that arrived last: kept out of line, only a
 // handful of CTAs per layer ever run it.  One round of loads: every thread fetches, for its
@@ -1567,113 +1476,14 @@ __device__ __forceinline__ void attn_merge_ll(Ctx& c, const uint2* base, __nv_bf
   }
 }
 
-// The same pass for ONE q head per half-warp (the single-chunk-per-CTA path): running
-// (max, sum, output) of the half-warp's positions of the task.  Four rows are handled as one
-// batch: their dot products and the four shuffle trees run side by side, and the running
-// maximum is updated once per batch, so the dependent chain of a batch is about as long as
-// that of a single row.  `pgs`: see attn_fetch_rows.
-__device__ __forceinline__ void attn_rows1(const Ctx& c, const OpDesc& op, const AttnPlan& pl, AttnTask& a, int l16,
-                                           uint4 qv, uint4 knew, uint4 vnew, float sc, float& m, float& l, float* o,
-                                           const int* pgs) {
-  const int L = a.L;
-  m = -INFINITY;
-  l = 0.f;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) o[i] = 0.f;
-  float qf[8];
-  unpack8(qv, qf);
-  const int niter = (a.p1 - a.p0 + pl.ngroups - 1) / pl.ngroups;
-#pragma unroll 1
-  for (int it = 0; it < niter; it += 4) {
-    uint4 nk[4], nv[4];  // the next four rows are requested before this batch is used
-    const bool more = it + 4 < niter;
-    if (more) attn_fetch_rows(c, op, pl, a, it + 4, l16, nk, nv, nullptr, false, pgs);
-    float sv[4];
-    bool ok[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = a.p0 + (it + u) * pl.ngroups + pl.gi;
-      ok[u] = j < a.p1;  // may differ between the two halves of a warp: the shuffles below do not depend on it
-      if (ok[u] && j == L - 1) {
-        a.kr[u] = knew;
-        a.vr[u] = vnew;
-      }
-      float kk[8];
-      unpack8(a.kr[u], kk);
-      float d = 0.f;
-#pragma unroll
-      for (int i = 0; i < 8; ++i) d = fmaf(qf[i], kk[i], d);
-      sv[u] = d;
-    }
-#pragma unroll
-    for (int x = 8; x > 0; x >>= 1) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) sv[u] += __shfl_xor_sync(0xffffffffu, sv[u], x);
-    }
-    float mn = m;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      sv[u] = ok[u] ? sv[u] * sc : -INFINITY;
-      mn = fmaxf(mn, sv[u]);
-    }
-    if (mn != -INFINITY) {  // (a batch without a position of this half-warp leaves everything as it is)
-      const float alpha = exp2f(m - mn);
-      float pr[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) pr[u] = exp2f(sv[u] - mn);
-      l = l * alpha + ((pr[0] + pr[1]) + (pr[2] + pr[3]));
-#pragma unroll
-      for (int i = 0; i < 8; ++i) o[i] *= alpha;
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        float vf[8];
-        unpack8(a.vr[u], vf);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = fmaf(pr[u], vf[i], o[i]);
-      }
-      m = mn;
-    }
-    if (more) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        a.kr[u] = nk[u];
-        a.vr[u] = nv[u];
-      }
-    }
-  }
-}
-
-// Rows of the task beyond the first four per half-warp (those are loaded into registers) are
-// requested into L2 ahead of the op's barrier, one row per lane, so that the row loop's own
-// loads find them there.
-__device__ __forceinline__ void attn_l2_ahead(const Ctx& c, const OpDesc& op, const AttnPlan& pl, const AttnTask& a, int l16,
-                                              const int* pgs) {
-  const int psh = c.p.page_shift, pmask = c.p.page_size - 1;
-  const int niter = (a.p1 - a.p0 + pl.ngroups - 1) / pl.ngroups;
-#pragma unroll 1
-  for (int r = 4 + l16; r < niter; r += 16) {
-    const int j = a.p0 + r * pl.ngroups + pl.gi;
-    if (j < a.p1 && j != a.L - 1) {
-      const int slot = (j >> psh) - (a.p0 >> psh);
-      const int pg = (pgs != nullptr && slot < 16) ? pgs[slot] : __ldcg(c.p.kv_indices + a.kv_base + (j >> psh));
-      const size_t src = ((((size_t)pg << psh) + (j & pmask)) * pl.HKV + a.h) * kHeadDim;
-      const __nv_bfloat16* kp = reinterpret_cast<const __nv_bfloat16*>(op.k_cache) + src;
-      const __nv_bfloat16* vp = reinterpret_cast<const __nv_bfloat16*>(op.v_cache) + src;
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(kp));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(kp + 64));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(vp));
-      asm volatile("prefetch.global.L2 [%0];" ::"l"(vp + 64));
-    }
-  }
-}
-
 // Prompt chunks (several tokens of one request in an iteration).  Waits for the op's barrier, then one
 // warp per (token, kv head) pair normalises and rotates the token's new K and stores it, with its V, at
 // the token's own position in the cache; a second grid barrier makes all of them visible.  Returns true
 // when the launch is aborting.  (Both halves of a warp compute the same pair: the shuffles in
 // head_norm_rope use the full mask.)
-__device__ __forceinline__ bool attn_barrier_then_append(Ctx& c, const OpDesc& op, const AttnPlan& pl, const int* lens, int T) {
+__device__ __forceinline__ bool attn_barrier_then_append(Ctx& c, const OpDesc& op, const int* lens, int T) {
   const KParams& p = c.p;
+  const int HKV = op.aux0, qpk = op.aux1 / op.aux0;
   if (op.flags & F_SYNC_BEFORE) {
     grid_wait(c);
     if (c.pr != nullptr && c.tid == 0) c.pr[1] = globaltimer();
@@ -1692,21 +1502,21 @@ __device__ __forceinline__ bool attn_barrier_then_append(Ctx& c, const OpDesc& o
   const bool dbl_k = op.aux0 < 32;
   const uint4 wk = __ldg(reinterpret_cast<const uint4*>(op.k_norm_w) + l16);
 #pragma unroll 1
-  for (int pair = blockIdx.x * kNumConsumerWarps + c.warp; pair < T * pl.HKV; pair += gridDim.x * kNumConsumerWarps) {
-    const int t = pair / pl.HKV, h = pair % pl.HKV;
+  for (int pair = blockIdx.x * kNumConsumerWarps + c.warp; pair < T * HKV; pair += gridDim.x * kNumConsumerWarps) {
+    const int t = pair / HKV, h = pair % HKV;
     const int L = lens[t];
     if (L <= 0) continue;
     const int pos = min(L - 1, op.aux2 - 1);
     const uint4 cs = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.cos) + (size_t)pos * kHeadDim) + l16);
     const uint4 sn = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.sin) + (size_t)pos * kHeadDim) + l16);
-    const __nv_bfloat16* row = reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)t * op.ld_in + (size_t)h * (pl.qpk + 2) * kHeadDim;
-    const uint4 vnew = __ldcg(reinterpret_cast<const uint4*>(row + (pl.qpk + 1) * kHeadDim) + l16);
+    const __nv_bfloat16* row = reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)t * op.ld_in + (size_t)h * (qpk + 2) * kHeadDim;
+    const uint4 vnew = __ldcg(reinterpret_cast<const uint4*>(row + (qpk + 1) * kHeadDim) + l16);
     F8 kf;
-    unpack8(__ldcg(reinterpret_cast<const uint4*>(row + pl.qpk * kHeadDim) + l16), kf.v);
+    unpack8(__ldcg(reinterpret_cast<const uint4*>(row + qpk * kHeadDim) + l16), kf.v);
     kf = head_norm_rope(kf, wk, cs, sn, l16, op.flags, p.numerics, dbl_k);
     const int pg = __ldcg(p.kv_indices + lens[kAttnLensMax + t] + ((L - 1) >> p.page_shift));
     if (c.lane < 16) {
-      const size_t dst = ((((size_t)pg << p.page_shift) + ((L - 1) & (p.page_size - 1))) * pl.HKV + h) * kHeadDim;
+      const size_t dst = ((((size_t)pg << p.page_shift) + ((L - 1) & (p.page_size - 1))) * HKV + h) * kHeadDim;
       reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(op.k_cache) + dst)[l16] = pack8(kf.v);
       reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(op.v_cache) + dst)[l16] = vnew;
     }
@@ -1716,7 +1526,15 @@ __device__ __forceinline__ bool attn_barrier_then_append(Ctx& c, const OpDesc& o
   return c.dead;
 }
 
+#include "mk_wide.cuh"
+
 // aux0 = kv heads, aux1 = q heads (q heads per kv head: 1, 2, 4 or 8).  The row-owner path's attention: one or two tokens.
+// Latency is all: a task is (token, kv head[, chunk of positions]), done by a whole CTA, whose warps take 16-position tiles in
+// turn on the tensor cores (attend_tiles).  The K and V rows of a warp's first tile are requested before the q rows are awaited; q
+// heads and the new K are normalised and rotated once per CTA, into shared memory, and the new token's K and V rows are taken
+// from there.  (In scalar fp32, a q head per half-warp, a CTA took 16 positions a round at four q heads per kv head: from 17
+// positions on the task was split over CTAs and merged across them, 4 us.  12 layers of 8B width, one request, us per step: 1103 ->
+// 1088 behind 80 positions, 1199 -> 1132 behind 1000; 8 MoE layers 640 -> 593; 4 layers 1024 wide 134 -> 128.)
 __device__ __forceinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
   const KParams& p = c.p;
   const int G = gridDim.x;
@@ -1727,23 +1545,19 @@ __device__ __forceinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
   }
   // arrive at the op's barrier first: everything up to the wait below is independent of other CTAs
   if (op.flags & F_SYNC_BEFORE) grid_arrive(c);
-  // Per-iteration cache in the scratch region (nothing else touches these bytes): sequence
-  // lengths incl. the new token [128], page-table offsets [128], then per half-warp the page
-  // numbers of its first four rows and of the new token [16][8].  The metadata only changes
-  // between iterations, so the first attention op of an iteration fills it and the other
-  // layers start their K/V row loads without any dependent look-up.
+  const int HKV = op.aux0, qpk = op.aux1 / op.aux0;
+  // Per-iteration cache in the scratch region (nothing else touches these bytes): sequence lengths incl. the new token [128],
+  // page-table offsets [128], whether some request has several tokens, then the plan.
   int* lens = reinterpret_cast<int*>(c.red() + 64);
-  int* pgc = lens + 2 * kAttnLensMax + (c.tid >> 4) * 8;
-  int* pgs = lens + 2 * kAttnLensMax + 16 * 8;  // [16]: page numbers of the first task's chunk, from its first page on
+  int* multi = lens + 2 * kAttnLensMax;
+  int* plan = multi + 1;  // [0] chunk size, [1] chunks of the longest request: the same in every layer of an iteration
   const int key = (c.iter << 8) ^ (op.aux0 * 16 + op.aux1);  // iteration and head geometry
-  const bool fill = c.attn_iter != key;
-  c.attn_iter = key;
-  int* multi = pgs + 16 + 3 + 9;  // [1]: some request has several tokens in this iteration (a prompt chunk)
-  if (fill) {
+  if (c.attn_iter != key) {
+    c.attn_iter = key;
     if (c.tid == 0) *multi = 0;
     consumer_sync();
     // Token t of request r (qo_indptr[r] <= t < qo_indptr[r + 1]) sits at position kv_len(r) - (tokens of r behind
-    // it) - 1: its sequence length, itself included, is what the tasks below call L.
+    // it) - 1: its sequence length, itself included, is what the tasks below call L0.
 #pragma unroll 1
     for (int r = c.tid; r < p.max_reqs; r += kNumConsumers) {
       const int q0 = __ldcg(p.qo_indptr + r), q1 = min(__ldcg(p.qo_indptr + r + 1), T);
@@ -1758,78 +1572,71 @@ __device__ __forceinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
       }
     }
     consumer_sync();
-  }
-  AttnPlan pl;
-  pl.HKV = op.aux0;
-  pl.qpk = op.aux1 / op.aux0;
-  int* plan = pgs + 16;   // [0] chunk size, [1] chunks of the longest request, [2] tasks: the same in every layer of an iteration
-  int* geom = plan + 3;   // [9]: the CTA's first task, see attn_prepare
-  if (fill) {
-    int Lmax = 1;
-#pragma unroll 1
-    for (int r = 0; r < T; ++r) Lmax = max(Lmax, lens[r]);
-    const int nb_max = (Lmax + 15) >> 4;
-    int bpc = (T * pl.HKV * nb_max + G - 1) / G;  // 16-position blocks per chunk: one round of tasks
-    bpc = max(bpc, (nb_max + p.attn_max_chunks - 1) / p.attn_max_chunks);
-    bpc = max(bpc, 1);
-    // one round of tasks: a chunk count that leaves a few CTAs a second task doubles the op's time
-    while (T * pl.HKV <= G && T * pl.HKV * ((nb_max + bpc - 1) / bpc) > G) ++bpc;
-    pl.CS = bpc * 16;
-    pl.nch_max = (nb_max + bpc - 1) / bpc;
-    pl.ntasks = T * pl.HKV * pl.nch_max;
     if (c.tid == 0) {
-      plan[0] = pl.CS;
-      plan[1] = pl.nch_max;
-      plan[2] = pl.ntasks;
+      int tiles = 1;
+      for (int t = 0; t < T; ++t) tiles = max(tiles, (lens[t] + 15) >> 4);
+      // One CTA per (token, kv head) up to kAttnSoloTiles tiles; beyond, chunks of at least 8 tiles (a tile per warp), as many as one
+      // round of CTAs holds.
+      int nch = tiles <= kAttnSoloTiles ? 1 : max(1, min(min(G / (T * HKV), (tiles + 7) / 8), p.attn_max_chunks));
+      const int tpc = (tiles + nch - 1) / nch;
+      plan[0] = tpc * 16;
+      plan[1] = (tiles + tpc - 1) / tpc;
     }
-  } else {
-    pl.CS = plan[0];
-    pl.nch_max = plan[1];
-    pl.ntasks = plan[2];
+    consumer_sync();
   }
-  const int l16 = c.lane & 15;
-  // Half-warp hw serves q head (hw % qpk) of the kv-head group for the positions of group
-  // (hw / qpk): one head per thread keeps the row loop and the combine small (this code runs
-  // once per layer out of a cold instruction cache), and the two halves of a warp read the
-  // same K/V rows, so their loads share a request.
-  const int hw = 2 * c.warp + (c.lane >> 4);
-  const int head = hw % pl.qpk;
-  pl.ngroups = 16 / pl.qpk;  // slots per head in the combine
-  pl.gi = hw / pl.qpk;
-  const int part_stride = pl.qpk * (kHeadDim + 2);
-  const float sc = 1.4426950408889634f * 0.08838834764831845f;  // log2(e) / sqrt(128)
-  uint4* sm_q = reinterpret_cast<uint4*>(c.smem + p.x_off);     // [8 heads][16 lanes]: q after norm and RoPE
-  uint4* sm_k = sm_q + 8 * 16;                                  // [16 lanes]: the new k
-  constexpr int nslots = 16;                                    // half-warps
-  float* sm_o = reinterpret_cast<float*>(sm_k + 16);            // [slots][128]
-  float* sm_m = sm_o + nslots * kHeadDim;                       // [slots]
-  float* sm_l = sm_m + nslots;
-  const bool dbl_q = op.aux1 < 32, dbl_k = op.aux0 < 32;
-  const int kw = pl.qpk & 7;  // the warp that prepares the new k (warp 0 when all eight prepare q heads)
-
-  bool first = true;
   const bool chunked = *multi != 0;
+  const int CS = plan[0], nch = plan[1], ntasks = T * HKV * nch;
+  const int l16 = c.lane & 15, g = c.lane >> 2, j = c.lane & 3;
+  // x region: combine slots [4][4 rows][128] fp32, (max, sum) pairs [8][8], the new token's K and V rows, q rows of pitch 272 bytes
+  uint8_t* xr = c.smem + p.x_off;
+  float2* ml = reinterpret_cast<float2*>(xr + 8192);
+  uint4* sm_k = reinterpret_cast<uint4*>(xr + 8192 + 512);  // [16] K, [16] V
+  __nv_bfloat16* sm_q = reinterpret_cast<__nv_bfloat16*>(xr + 8192 + 512 + 512);
+  constexpr int kQPitch = 136;
+  const bool dbl_q = op.aux1 < 32, dbl_k = op.aux0 < 32;
+  const int kw = qpk & 7;  // the warp that prepares the new k (warp 0 when all eight prepare q heads)
+  const int part_stride = qpk * (kHeadDim + 2);
+  const unsigned tag_in = ll_tag_of(c, op.ll_in_op), tag = ll_tag_of(c, c.cur_op);
   if (chunked) {
     // A prompt chunk: its tokens attend to each other's K/V, which only exist once every token's K has been
     // normalised, rotated and appended.  So this iteration appends first, for all tokens, behind the op's
     // own barrier, and meets at one more grid barrier before any row is read (nothing is fetched early).
-    if (attn_barrier_then_append(c, op, pl, lens, T)) return;
-    first = false;
+    if (attn_barrier_then_append(c, op, lens, T)) return;
   }
+  bool first = !chunked;
 #pragma unroll 1
   for (int task = blockIdx.x;; task += G) {
-    AttnTask a;
-    attn_prepare(c, op, pl, lens, task, l16, a, (first && !chunked) ? pgc : nullptr, fill, (first && !chunked) ? geom : nullptr);
+    WideTask a;
+    a.p0 = a.p1 = a.fresh = a.L0 = 0;
+    int ti = c.warp, ntiles = 0, pgn = 0, new_page = 0;
+    uint4 kr[2][4], vr[4][2];
+    bool live = task < ntasks;
+    if (live) {
+      a.ch = task % nch;
+      a.h = (task / nch) % HKV;
+      a.t0 = task / (nch * HKV);
+      a.nt = 1;
+      a.L0 = lens[a.t0];
+      a.kvb = lens[kAttnLensMax + a.t0];
+      a.p0 = a.ch * CS;
+      a.p1 = min(a.L0, a.p0 + CS);
+      a.nch = (a.L0 + CS - 1) / CS;
+      a.fresh = chunked ? a.L0 + 16 : a.L0 - 1;  // (a prompt chunk's rows are all in the cache)
+      live = a.L0 > 0 && a.p0 < a.L0;
+    }
+    if (live) {
+      ntiles = (a.p1 - a.p0 + 15) >> 4;
+      if (ti < ntiles) {
+        const int pg = p.page_shift >= 4 ? wide_page(c, a, a.p0 + 16 * ti) : 0;
+        wide_load_k(c, op, a, a.p0 + 16 * ti, pg, kr);
+        wide_load_v(c, op, a, a.p0 + 16 * ti, pg, vr);
+        if (p.page_shift >= 4 && ti + kNumConsumerWarps < ntiles) pgn = wide_page(c, a, a.p0 + 16 * (ti + kNumConsumerWarps));
+      }
+      if (a.p1 == a.L0) new_page = __ldcg(p.kv_indices + a.kvb + ((a.L0 - 1) >> p.page_shift));
+    }
     if (first) {
       // everything above is independent of this layer's QKV rows: fetched ahead of the barrier
       first = false;
-      if (a.valid) {
-        if (fill && c.tid < 16) {  // (read only after the barrier's CTA-wide sync)
-          const int slot = (a.p0 >> p.page_shift) + c.tid;
-          if ((slot << p.page_shift) < a.p1) pgs[c.tid] = __ldcg(p.kv_indices + a.kv_base + slot);
-        }
-        attn_l2_ahead(c, op, pl, a, l16, fill ? nullptr : pgs);
-      }
       MK_STAMP(c, 1);
       if (op.flags & F_SYNC_BEFORE) {  // op_barrier, with the wait inlined
         grid_wait(c);
@@ -1844,132 +1651,119 @@ __device__ __forceinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
         return;
       }
     }
-    if (task >= pl.ntasks) break;
-    if (!a.valid) continue;
-    const int L = a.L;
-    const __nv_bfloat16* row = reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)a.t * op.ld_in +
-                               (size_t)a.h * (pl.qpk + 2) * kHeadDim;
-    // tagged input: the task polls the words of its own kv-head group only (a prompt chunk has had its barrier)
-    const bool ll_in = (op.flags & F_LL_IN) && !chunked;
-    const uint2* llr = ll_row(op.ll_in, op.ld_in, a.t) + ((a.h * (pl.qpk + 2) * kHeadDim) >> 1);
-    const unsigned tag_in = ll_tag_of(c, op.ll_in_op);
-    const bool do_q = c.warp < pl.qpk, do_k = c.warp == kw;
-    uint4 vnew, xq = make_uint4(0, 0, 0, 0), xk = make_uint4(0, 0, 0, 0);
-    // norm weights and the cos/sin row of the position, for the warps that prepare a head
-    uint4 nw = make_uint4(0, 0, 0, 0), ncs = nw, nsn = nw;
+    if (task >= ntasks) break;
+    if (!live) continue;
+    const __nv_bfloat16* row = reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)a.t0 * op.ld_in + (size_t)a.h * (qpk + 2) * kHeadDim;
+    const bool do_q = c.warp < qpk, do_k = c.warp == kw;
     if (do_q || do_k) {
-      const int pos = min(L - 1, op.aux2 - 1);  // aux2 = rows of the cos/sin tables
-      nw = __ldg(reinterpret_cast<const uint4*>(do_q ? op.q_norm_w : op.k_norm_w) + l16);
-      ncs = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.cos) + (size_t)pos * kHeadDim) + l16);
-      nsn = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.sin) + (size_t)pos * kHeadDim) + l16);
-    }
-    if (ll_in) {
-      const int at[3] = {(pl.qpk + 1) * (kHeadDim / 8) + l16, do_q ? c.warp * (kHeadDim / 8) + l16 : -1, do_k ? pl.qpk * (kHeadDim / 8) + l16 : -1};
-      uint4 got[3];
-      ll_take(c, reinterpret_cast<const uint4*>(llr), at, tag_in, got);
-      vnew = got[0];
-      xq = got[1];
-      xk = got[2];
-    } else {
-      vnew = __ldcg(reinterpret_cast<const uint4*>(row + (pl.qpk + 1) * kHeadDim) + l16);
-      if (do_q) xq = __ldcg(reinterpret_cast<const uint4*>(row + c.warp * kHeadDim) + l16);
-      if (do_k) xk = __ldcg(reinterpret_cast<const uint4*>(row + pl.qpk * kHeadDim) + l16);
-    }
-    // norm + RoPE once per CTA: warp w < qpk prepares q head w, one warp the new k
-    if (do_q) {
-      F8 q;
-      unpack8(xq, q.v);
-      q = head_norm_rope(q, nw, ncs, nsn, l16, op.flags, p.numerics, dbl_q);
-      if (c.lane < 16) sm_q[c.warp * 16 + l16] = pack8(q.v);  // exact: the values are bf16 already
-    }
-    if (do_k) {
-      F8 kf;
-      unpack8(xk, kf.v);
-      kf = head_norm_rope(kf, do_q ? __ldg(reinterpret_cast<const uint4*>(op.k_norm_w) + l16) : nw, ncs, nsn, l16, op.flags, p.numerics, dbl_k);
-      const uint4 kn = pack8(kf.v);
-      if (c.lane < 16) {
-        sm_k[l16] = kn;
-        if (a.p1 == L && !chunked) {  // the last chunk appends the new token's K and V to the cache
-          const size_t dst = ((((size_t)a.new_page << p.page_shift) + ((L - 1) & (p.page_size - 1))) * pl.HKV + a.h) * kHeadDim;
-          reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(op.k_cache) + dst)[l16] = kn;
-          reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(op.v_cache) + dst)[l16] = vnew;
+      uint4 vnew, xq = make_uint4(0, 0, 0, 0), xk = make_uint4(0, 0, 0, 0);
+      // norm weights and the cos/sin row of the position, beside the rows themselves
+      const int pos = min(a.L0 - 1, op.aux2 - 1);  // aux2 = rows of the cos/sin tables
+      const uint4 nw = __ldg(reinterpret_cast<const uint4*>(do_q ? op.q_norm_w : op.k_norm_w) + l16);
+      const uint4 ncs = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.cos) + (size_t)pos * kHeadDim) + l16);
+      const uint4 nsn = __ldg(reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.sin) + (size_t)pos * kHeadDim) + l16);
+      if ((op.flags & F_LL_IN) && !chunked) {  // (a prompt chunk has had its barrier)
+        const int at[3] = {do_k ? (qpk + 1) * (kHeadDim / 8) + l16 : -1, do_q ? c.warp * (kHeadDim / 8) + l16 : -1, do_k ? qpk * (kHeadDim / 8) + l16 : -1};
+        uint4 got[3];
+        ll_take(c, reinterpret_cast<const uint4*>(ll_row(op.ll_in, op.ld_in, a.t0) + ((a.h * (qpk + 2) * kHeadDim) >> 1)), at, tag_in, got);
+        __syncwarp();
+        vnew = got[0];
+        xq = got[1];
+        xk = got[2];
+      } else {
+        vnew = __ldcg(reinterpret_cast<const uint4*>(row + (qpk + 1) * kHeadDim) + l16);
+        if (do_q) xq = __ldcg(reinterpret_cast<const uint4*>(row + c.warp * kHeadDim) + l16);
+        if (do_k) xk = __ldcg(reinterpret_cast<const uint4*>(row + qpk * kHeadDim) + l16);
+      }
+      if (do_q) {
+        F8 q;
+        unpack8(xq, q.v);
+        q = head_norm_rope(q, nw, ncs, nsn, l16, op.flags, p.numerics, dbl_q);
+        if (c.lane < 16) reinterpret_cast<uint4*>(sm_q + c.warp * kQPitch)[l16] = pack8(q.v);  // exact: the values are bf16 already
+      }
+      if (do_k) {
+        F8 kf;
+        unpack8(xk, kf.v);
+        kf = head_norm_rope(kf, do_q ? __ldg(reinterpret_cast<const uint4*>(op.k_norm_w) + l16) : nw, ncs, nsn, l16, op.flags, p.numerics, dbl_k);
+        const uint4 kn = pack8(kf.v);
+        if (c.lane < 16) {
+          sm_k[l16] = kn;
+          sm_k[16 + l16] = vnew;
+          if (a.p1 == a.L0 && !chunked) {  // the last chunk appends the new token's K and V to the cache
+            const size_t dst = ((((size_t)new_page << p.page_shift) + ((a.L0 - 1) & (p.page_size - 1))) * HKV + a.h) * kHeadDim;
+            reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(op.k_cache) + dst)[l16] = kn;
+            reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(op.v_cache) + dst)[l16] = vnew;
+          }
         }
       }
     }
     consumer_sync();
     MK_STAMP(c, 2);
-    {
-      const uint4 qv = sm_q[head * 16 + l16];
-      const uint4 knew = sm_k[l16];
-      float m, l, o[8];
-      attn_rows1(c, op, pl, a, l16, qv, knew, vnew, sc, m, l, o, (task == (int)blockIdx.x && !chunked) ? pgs : nullptr);
-      // every half-warp leaves its (max, sum, output) in shared memory; one pass over the output
-      // elements then combines the position groups of each head
-      float* dst = sm_o + hw * kHeadDim + l16 * 8;
-      reinterpret_cast<float4*>(dst)[0] = make_float4(o[0], o[1], o[2], o[3]);
-      reinterpret_cast<float4*>(dst)[1] = make_float4(o[4], o[5], o[6], o[7]);
-      if (l16 == 0) {
-        sm_m[hw] = m;
-        sm_l[hw] = l;
-      }
-    }
+    uint4 qf[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) qf[i] = g < qpk ? *reinterpret_cast<const uint4*>(sm_q + g * kQPitch + 32 * i + 8 * j) : make_uint4(0, 0, 0, 0);
+    float m, l, oacc[8][4];
+    attend_tiles<true>(c, op, a, kNumConsumerWarps, ti, pgn, qf, kr, vr, sm_k, m, l, oacc);
     MK_STAMP(c, 3);
-    consumer_sync();
-    float* part = p.attn_part + (((size_t)a.t * pl.HKV + a.h) * p.attn_max_chunks + a.ch) * part_stride;
+    // a thread ends up with at most one (row, four dims) per batch of four rows: kept until the task is known to be finite
+    // (words that others poll cannot be taken back)
+    float4 keep[2] = {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)};
+    float keep_m[2] = {0.f, 0.f}, keep_l[2] = {1.f, 1.f};
+    float chk = 0.f;
+    attend_combine(c, kNumConsumerWarps, 0, qpk, xr, ml, m, l, oacc, [&](int rb, int, int, const float4& O, float M, float L) {
+      keep[rb] = O;
+      keep_m[rb] = M;
+      keep_l[rb] = L;
+      chk = fmaf(O.x, 0.f, fmaf(O.y, 0.f, fmaf(O.z, 0.f, fmaf(O.w, 0.f, chk))));
+    });
+    float* part = p.attn_part + (((size_t)a.t0 * HKV + a.h) * p.attn_max_chunks + a.ch) * part_stride;
     // tagged partials (see attn_merge_ll) when the op's output is tagged and the host gave them room
     const bool ll_part = (op.flags & F_LL_OUT) && p.attn_part_ll != nullptr;
-    uint2* partw = p.attn_part_ll + (((size_t)a.t * pl.HKV + a.h) * p.attn_max_chunks + a.ch) * part_stride;
-    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out) + (size_t)a.t * op.ld_out +
-                         (size_t)a.h * pl.qpk * kHeadDim;
-    uint2* ll_out = (op.flags & F_LL_OUT) ? reinterpret_cast<uint2*>(op.ll_out) + (size_t)a.t * (size_t)(op.ld_out >> 1) +
-                                                ((a.h * pl.qpk * kHeadDim) >> 1)
+    uint2* partw = p.attn_part_ll + (((size_t)a.t0 * HKV + a.h) * p.attn_max_chunks + a.ch) * part_stride;
+    __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out) + (size_t)a.t0 * op.ld_out + (size_t)a.h * qpk * kHeadDim;
+    uint2* ll_out = (op.flags & F_LL_OUT) ? reinterpret_cast<uint2*>(op.ll_out) + (size_t)a.t0 * (size_t)(op.ld_out >> 1) + ((a.h * qpk * kHeadDim) >> 1)
                                           : nullptr;
-#pragma unroll 1
-    for (int e = c.tid; e < pl.qpk * kHeadDim; e += kNumConsumers) {
-      const int eh = e >> 7, d = e & 127;
-      float M = -INFINITY;
-#pragma unroll 4
-      for (int g = 0; g < pl.ngroups; ++g) M = fmaxf(M, sm_m[g * pl.qpk + eh]);
-      float Ls = 0.f, O = 0.f;
-#pragma unroll 4  // (four reads of shared memory in flight: 0.5 % of a batch-1 step against the rolled loop)
-      for (int g = 0; g < pl.ngroups; ++g) {
-        const int w = g * pl.qpk + eh;
-        const float mw = sm_m[w];
-        const float f = (mw == -INFINITY) ? 0.f : exp2f(mw - M);
-        Ls += f * sm_l[w];
-        O += f * sm_o[w * kHeadDim + d];
-      }
+    auto store = [&](int r, int d, const float4& O, float M, float L) {
       if (a.nch == 1) {
-        const __nv_bfloat16 y = __float2bfloat16_rn(__fdividef(O, Ls));
-        out[e] = y;
-        if (op.flags & F_LL_OUT) {  // (whole warps run this loop: its bound is a multiple of 128)
-          const uint32_t lo = (uint32_t)__bfloat16_as_ushort(y);
-          const uint32_t hi = __shfl_down_sync(0xffffffffu, lo, 1);
-          if (!(e & 1)) st_gpu_v2(ll_out + (e >> 1), lo | (hi << 16), ll_tag_of(c, c.cur_op));
-        }
+        const float inv = __fdividef(1.0f, L);
+        const uint2 y = make_uint2(pack2(O.x * inv, O.y * inv), pack2(O.z * inv, O.w * inv));
+        *reinterpret_cast<uint2*>(out + r * kHeadDim + d) = y;
+        if (ll_out != nullptr) st_gpu_words(reinterpret_cast<uint4*>(ll_out + ((r * kHeadDim + d) >> 1)), y.x, y.y, tag);
       } else if (ll_part) {
-        st_gpu_v2(partw + e, __float_as_uint(O), ll_tag_of(c, c.cur_op));
+        uint4* dst = reinterpret_cast<uint4*>(partw + r * kHeadDim + d);
+        st_gpu_words(dst, __float_as_uint(O.x), __float_as_uint(O.y), tag);
+        st_gpu_words(dst + 1, __float_as_uint(O.z), __float_as_uint(O.w), tag);
         if (d == 0) {
-          st_gpu_v2(partw + pl.qpk * kHeadDim + eh, __float_as_uint(M), ll_tag_of(c, c.cur_op));
-          st_gpu_v2(partw + pl.qpk * kHeadDim + pl.qpk + eh, __float_as_uint(Ls), ll_tag_of(c, c.cur_op));
+          st_gpu_v2(partw + qpk * kHeadDim + r, __float_as_uint(M), tag);
+          st_gpu_v2(partw + qpk * kHeadDim + qpk + r, __float_as_uint(L), tag);
         }
       } else {
-        part[e] = O;
+        *reinterpret_cast<float2*>(part + r * kHeadDim + d) = make_float2(O.x, O.y);
+        *reinterpret_cast<float2*>(part + r * kHeadDim + d + 2) = make_float2(O.z, O.w);
         if (d == 0) {
-          part[pl.qpk * kHeadDim + eh] = M;
-          part[pl.qpk * kHeadDim + pl.qpk + eh] = Ls;
+          part[qpk * kHeadDim + r] = M;
+          part[qpk * kHeadDim + qpk + r] = L;
         }
+      }
+    };
+    if (bar_any(2, kNumConsumers, chk != 0.f)) {
+      attend_exact(p, op, a, kNumConsumerWarps, sm_q, (size_t)0, kQPitch, store);
+    } else if (c.tid < 128) {
+#pragma unroll
+      for (int rb = 0; rb < 2; ++rb) {
+        const int r = 4 * rb + (c.tid >> 5), d = (c.tid & 31) * 4;
+        if (r < qpk) store(r, d, keep[rb], keep_m[rb], keep_l[rb]);
       }
     }
     MK_STAMP(c, 4);
     if (a.nch > 1 && ll_part) {
-      attn_merge_ll(c, partw - (size_t)a.ch * part_stride, out, ll_out, a.nch, a.ch, pl.qpk, part_stride, ll_tag_of(c, c.cur_op));
+      attn_merge_ll(c, partw - (size_t)a.ch * part_stride, out, ll_out, a.nch, a.ch, qpk, part_stride, tag);
     } else if (a.nch > 1) {
       consumer_sync();  // the CTA's partial is complete; thread 0's release below publishes all of it
       MK_STAMP(c, 5);
       volatile int* fl = c.flags();
-      unsigned* cnt = p.attn_count + (size_t)a.t * pl.HKV + a.h;
-      const float* base = p.attn_part + (((size_t)a.t * pl.HKV + a.h) * p.attn_max_chunks) * part_stride;
+      unsigned* cnt = p.attn_count + (size_t)a.t0 * HKV + a.h;
+      const float* base = p.attn_part + (((size_t)a.t0 * HKV + a.h) * p.attn_max_chunks) * part_stride;
       if (c.tid == 0) {
         unsigned old;
         asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(old) : "l"(cnt) : "memory");
@@ -1980,7 +1774,7 @@ __device__ __forceinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
       // The chunk that arrives last merges all of them.  (A fixed merger per kv head, polling the
       // counter, measured slower: the last arriver knows at once that it is the last.)
       if (fl[2] != 0) {
-        attn_merge(c, base, out, a.nch, pl.qpk, part_stride, ll_out, ll_tag_of(c, c.cur_op));
+        attn_merge(c, base, out, a.nch, qpk, part_stride, ll_out, tag);
         if (c.tid == 0) *cnt = 0u;
       }
     }
@@ -1989,7 +1783,6 @@ __device__ __forceinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
   }
 }
 
-#include "mk_wide.cuh"
 
 // ------------------------------------------------------------------------------------
 // small ops

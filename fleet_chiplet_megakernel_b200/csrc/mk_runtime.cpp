@@ -1363,8 +1363,8 @@ static int compile_program(mk_handle* h, bool first) {
       if ((p.n > 8192 && p.n <= mk::kNormStagedCols) || (p.flags & mk::F_GATHER_IN)) x_bytes = std::max(x_bytes, ((p.n + 63) / 64 * 64 + 8) * 2 + 16);
     } else if (p.type == mk::OP_ATTN) {
       has_attn = true;
-      // row-owner path: q heads and the new k (bf16), combine slots of 16 half-warps x 128 floats, (max, sum) pairs, merge scratch
-      if (rows_mode) x_bytes = std::max(x_bytes, 9 * 256 + 4 * 4 * (mk::kHeadDim + 2) * 4 + 2 * kAttnMaxChunks * 8 * 4 + 64 + 256);
+      // row-owner path: combine slots, (max, sum) pairs, the new K and V rows, eight q rows
+      if (rows_mode) x_bytes = std::max(x_bytes, 8192 + 512 + 512 + 8 * 272);
       // wide path: 1 KB per warp to combine their sums, (max, sum) pairs; the QKV epilogue transposes through the same 8 KB
       else x_bytes = std::max(x_bytes, 8192 + mk::kNumConsumerWarps * 8 * 8);
     }

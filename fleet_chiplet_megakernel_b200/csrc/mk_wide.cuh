@@ -870,16 +870,17 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t&
 // causal row does not see the position or the tile runs past the end, and by three parts of P of either sign elsewhere, so
 // 0 x inf would carry an infinite value of a prompt chunk's last token into the tokens before it.  Here a row takes the
 // positions it sees and no others, in scalar fp32: a warp per row, a lane per position for the scores and four dims per
-// lane for the sums.  (The check sits on the outputs: 36 layers at 8 requests 5.83 -> 5.86 ms; on the accumulators, with
-// the sums redone in place, 5.90.)
-__device__ __forceinline__ void wide_attend_exact(const KParams& p, const OpDesc& op, const WideTask a, int W, __nv_bfloat16* out, float* part) {
+// lane for the sums.  `q0`: the task's q rows, `ld` apart from token to token (read past L1: other CTAs may have written
+// them); emit(row, dims 4 lane .. + 3, sums, max, sum of exponentials).  (The check sits on the outputs: 36 layers at 8
+// requests 5.83 -> 5.86 ms when it was added; on the accumulators, with the sums redone in place, 5.90.)
+template <class Emit>
+__device__ __forceinline__ void attend_exact(const KParams& p, const OpDesc& op, const WideTask& a, int W, const __nv_bfloat16* q0, size_t ld, int ldh, Emit emit) {
   const int HKV = op.aux0, qpk = op.aux1 / HKV, rows = a.nt * qpk, lane = threadIdx.x & 31;
   const float sc = 1.4426950408889634f * 0.08838834764831845f;  // log2(e) / sqrt(128)
 #pragma unroll 1
   for (int r = (threadIdx.x >> 5) & (W - 1); r < rows; r += W) {
     const int tok = r / qpk, head = r % qpk, last = min(a.L0 + tok, a.p1);
-    const uint4* q = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(op.out2) + (size_t)(a.t0 + tok) * op.ld_out2 +
-                                                    (size_t)(a.h * qpk + head) * kHeadDim);
+    const volatile uint32_t* q = reinterpret_cast<const volatile uint32_t*>(q0 + (size_t)tok * ld + (size_t)head * ldh);
     float M = -INFINITY, L = 0.f, O[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {  // the maximum, then the sums
@@ -887,15 +888,16 @@ __device__ __forceinline__ void wide_attend_exact(const KParams& p, const OpDesc
       for (int pos0 = a.p0; pos0 < last; pos0 += 32) {
         const int pos = min(pos0 + lane, last - 1);
         const int slot = (__ldcg(p.kv_indices + a.kvb + (pos >> p.page_shift)) << p.page_shift) + (pos & (p.page_size - 1));
-        const uint4* k = reinterpret_cast<const uint4*>(op.k_cache) + ((size_t)slot * HKV + a.h) * (kHeadDim / 8);
+        const uint2* k = reinterpret_cast<const uint2*>(op.k_cache) + ((size_t)slot * HKV + a.h) * (kHeadDim / 4);
         float s = 0.f;
-#pragma unroll 4
-        for (int i = 0; i < kHeadDim / 8; ++i) {
-          float qf[8], kf[8];
-          unpack8(__ldcg(q + i), qf);
-          unpack8(__ldcg(k + i), kf);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) s = fmaf(qf[e], kf[e], s);
+#pragma unroll 1
+        for (int i = 0; i < kHeadDim / 4; ++i) {
+          const uint32_t qa = q[2 * i], qb = q[2 * i + 1];
+          const uint2 kk = __ldcg(k + i);
+          s = fmaf(bf_lo(qa), bf_lo(kk.x), s);
+          s = fmaf(bf_hi(qa), bf_hi(kk.x), s);
+          s = fmaf(bf_lo(qb), bf_lo(kk.y), s);
+          s = fmaf(bf_hi(qb), bf_hi(kk.y), s);
         }
         s = pos0 + lane < last ? s * sc : -INFINITY;
         if (pass == 0) {
@@ -904,7 +906,7 @@ __device__ __forceinline__ void wide_attend_exact(const KParams& p, const OpDesc
         }
         const float pr = exp2f(s - (M == -INFINITY ? 0.f : M));
         L += pr;
-#pragma unroll 4
+#pragma unroll 1
         for (int i = 0; i < min(32, last - pos0); ++i) {
           const int vs = __shfl_sync(0xffffffffu, slot, i);
           const float pi = __shfl_sync(0xffffffffu, pr, i);
@@ -921,18 +923,7 @@ __device__ __forceinline__ void wide_attend_exact(const KParams& p, const OpDesc
         else L += __shfl_xor_sync(0xffffffffu, L, o);
       }
     }
-    if (a.nch == 1) {
-      const float inv = __fdividef(1.0f, L);
-      *reinterpret_cast<uint2*>(out + (size_t)tok * op.ld_out + head * kHeadDim + 4 * lane) =
-          make_uint2(pack2(O[0] * inv, O[1] * inv), pack2(O[2] * inv, O[3] * inv));
-    } else {
-      *reinterpret_cast<float2*>(part + r * kHeadDim + 4 * lane) = make_float2(O[0], O[1]);
-      *reinterpret_cast<float2*>(part + r * kHeadDim + 4 * lane + 2) = make_float2(O[2], O[3]);
-      if (lane == 0) {
-        part[rows * kHeadDim + r] = M;
-        part[rows * kHeadDim + rows + r] = L;
-      }
-    }
+    emit(r, 4 * lane, make_float4(O[0], O[1], O[2], O[3]), M, L);
   }
 }
 // bar.sync that also tells every thread whether any thread's `pred` holds
@@ -946,34 +937,18 @@ __device__ __forceinline__ bool bar_any(int id, int nthr, bool pred) {
   return r != 0u;
 }
 
-// One task by W warps.  `reg`: the group's shared memory (W KB), `ml`: [warps of the CTA][8] (max, sum) pairs.  `loaded`: the
-// first tile's K and V rows are in kr and vr already, but for the rows that this iteration writes.
-__device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTask& a, int W, int gi, uint8_t* reg, float2* ml, bool loaded,
-                                            uint4 (&kr)[2][4], uint4 (&vr)[4][2]) {
-  const KParams& p = c.p;
+// The tiles ti, ti + W, ... of a task by one warp: (max, sum) of row g and, per tile t of 16 dims, oacc[t] = {dim 8 g + t of rows 2 j and
+// 2 j + 1, dim 64 + 8 g + t of the same}.  The first tile's rows are in kr and vr, pgn is the page of the second.  FRESH: K and V of
+// the positions from a.fresh on are the two rows at fresh_kv (the new token's, in shared memory), not the cache's.
+template <bool FRESH>
+__device__ __forceinline__ void attend_tiles(const Ctx& c, const OpDesc& op, const WideTask& a, int W, int ti, int pgn, const uint4 (&qf)[4],
+                                             uint4 (&kr)[2][4], uint4 (&vr)[4][2], const uint4* fresh_kv, float& m, float& l, float (&oacc)[8][4]) {
   const int lane = c.lane, g = lane >> 2, j = lane & 3;
-  const int HKV = op.aux0, qpk = op.aux1 / HKV, rows = a.nt * qpk;
-  const int sub = c.warp & (W - 1), gtid = sub * 32 + lane, nthr = W * 32;
-  const float sc = 1.4426950408889634f * 0.08838834764831845f;  // log2(e) / sqrt(128)
-  const int psh = p.page_shift;
+  const int qpk = op.aux1 / op.aux0, psh = c.p.page_shift;
   const int ntiles = (a.p1 - a.p0 + 15) >> 4;
-  int ti = sub;
-  // Row g of the q rows as A fragments: 8 dims from 32 i + 8 j are k steps 2 i and 2 i + 1; rows past the group's are zero.
-  uint4 qf[4];
-  {
-    const __nv_bfloat16* q0 = reinterpret_cast<const __nv_bfloat16*>(op.out2) + (size_t)(a.t0 + g / qpk) * op.ld_out2 + (size_t)(a.h * qpk + g % qpk) * kHeadDim + 8 * j;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) qf[i] = g < rows ? __ldcg(reinterpret_cast<const uint4*>(q0 + 32 * i)) : make_uint4(0, 0, 0, 0);
-  }
-  if (ti < ntiles && (!loaded || a.p0 + 16 * ti + 15 >= a.fresh)) {
-    const int pg = psh >= 4 ? wide_page(c, a, a.p0 + 16 * ti) : 0;
-    wide_load_k(c, op, a, a.p0 + 16 * ti, pg, kr);
-    wide_load_v(c, op, a, a.p0 + 16 * ti, pg, vr);
-  }
-  int pgn = (psh >= 4 && ti + W < ntiles) ? wide_page(c, a, a.p0 + 16 * (ti + W)) : 0;
-  MK_STAMP(c, 1);
-  float m = -INFINITY, l = 0.f;  // of row g
-  float oacc[8][4];  // tile t of 16 dims: {dim 8 g + t of rows 2 j and 2 j + 1, dim 64 + 8 g + t of the same}
+  const float sc = 1.4426950408889634f * 0.08838834764831845f;  // log2(e) / sqrt(128)
+  m = -INFINITY;
+  l = 0.f;
 #pragma unroll
   for (int t = 0; t < 8; ++t)
 #pragma unroll
@@ -983,6 +958,21 @@ __device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const Wide
   for (; ti < ntiles; ti += W) {
     const int pos0 = a.p0 + 16 * ti;
     const bool more = ti + W < ntiles;
+    if constexpr (FRESH) {
+      if (pos0 + 15 >= a.fresh) {  // rows from a.fresh on (and what a position past the end is clamped to) come from shared memory
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          if (min(pos0 + 8 * u + g, a.p1 - 1) >= a.fresh)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) kr[u][i] = fresh_kv[j + 4 * i];
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          if (min(pos0 + 2 * j + (r & 1) + 8 * (r >> 1), a.p1 - 1) >= a.fresh) {
+            vr[r][0] = fresh_kv[16 + g];
+            vr[r][1] = fresh_kv[24 + g];
+          }
+      }
+    }
     float s0[2] = {0.f, 0.f}, s1[2] = {0.f, 0.f}, z0[2] = {0.f, 0.f}, z1[2] = {0.f, 0.f};
 #pragma unroll
     for (int s = 0; s < 8; ++s) {
@@ -1039,40 +1029,20 @@ __device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const Wide
   }
   l += __shfl_xor_sync(0xffffffffu, l, 1);
   l += __shfl_xor_sync(0xffffffffu, l, 2);
-  MK_STAMP(c, 2);
-  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out) + (size_t)a.t0 * op.ld_out + (size_t)a.h * qpk * kHeadDim;
-  float chk = 0.f;  // stays zero while the outputs are finite
-  if (W == 1 && a.nch == 1) {
-#pragma unroll
-    for (int y = 0; y < 2; ++y) {
-      const float lr = __shfl_sync(0xffffffffu, l, 8 * j + 4 * y);
-      const int r = 2 * j + y;
-      if (r < rows) {
-        const float inv = __fdividef(1.0f, lr);
-        __nv_bfloat16* dst = out + (size_t)(r / qpk) * op.ld_out + (r % qpk) * kHeadDim + 8 * g;
-#pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          float f[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            f[i] = oacc[i][2 * x + y] * inv;
-            chk = fmaf(f[i], 0.f, chk);
-          }
-          *reinterpret_cast<uint4*>(dst + 64 * x) = pack8(f);
-        }
-      }
-    }
-    __syncwarp();
-    if (__any_sync(0xffffffffu, chk != 0.f)) wide_attend_exact(c.p, op, a, W, out, nullptr);
-    return;
-  }
+}
+
+// emit(batch, row, dims d .. d + 3, sums, max, sum of exponentials) for every output of the task
+template <class Emit>
+__device__ __forceinline__ void attend_combine(const Ctx& c, int W, int gi, int rows, uint8_t* reg, float2* ml, float m, float l, const float (&oacc)[8][4],
+                                               Emit emit) {
+  const int lane = c.lane, g = lane >> 2, j = lane & 3;
+  const int sub = c.warp & (W - 1), gtid = sub * 32 + lane, nthr = W * 32;
   // The warps of the task meet in shared memory, four rows at a time: the upper half leaves its sums in W / 2 slots, the
   // lower half adds its own to them, in place, and all finish the rows from there.
   const uint32_t nbar = (uint32_t)(2 + gi);
   const int H = W >> 1;
   if (j == 0) ml[c.warp * 8 + g] = make_float2(m, l);
   float* slot0 = reinterpret_cast<float*>(reg);
-  float* part = p.attn_part + ((size_t)a.t0 * HKV * p.attn_max_chunks * qpk + (size_t)(a.h * p.attn_max_chunks + a.ch) * rows) * (kHeadDim + 2);
 #pragma unroll
   for (int rb = 0; rb < 2; ++rb) {
     if (4 * rb >= rows) break;
@@ -1131,24 +1101,89 @@ __device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const Wide
         O.z = fmaf(f, o4.z, O.z);
         O.w = fmaf(f, o4.w, O.w);
       }
-      chk = fmaf(O.x, 0.f, fmaf(O.y, 0.f, fmaf(O.z, 0.f, fmaf(O.w, 0.f, chk))));
-      if (a.nch == 1) {
-        const float inv = __fdividef(1.0f, L);
-        *reinterpret_cast<uint2*>(out + (size_t)(r / qpk) * op.ld_out + (r % qpk) * kHeadDim + d) =
-            make_uint2(pack2(O.x * inv, O.y * inv), pack2(O.z * inv, O.w * inv));
-      } else {
-        *reinterpret_cast<float2*>(part + r * kHeadDim + d) = make_float2(O.x, O.y);
-        *reinterpret_cast<float2*>(part + r * kHeadDim + d + 2) = make_float2(O.z, O.w);
-        if (d == 0) {
-          part[rows * kHeadDim + r] = M;
-          part[rows * kHeadDim + rows + r] = L;
+      emit(rb, r, d, O, M, L);
+    }
+  }
+}
+
+// One task by W warps.  `reg`: the group's shared memory (W KB), `ml`: [warps of the CTA][8] (max, sum) pairs.  `loaded`: the
+// first tile's K and V rows are in kr and vr already, but for the rows that this iteration writes.
+__device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTask& a, int W, int gi, uint8_t* reg, float2* ml, bool loaded,
+                                            uint4 (&kr)[2][4], uint4 (&vr)[4][2]) {
+  const KParams& p = c.p;
+  const int lane = c.lane, g = lane >> 2, j = lane & 3;
+  const int HKV = op.aux0, qpk = op.aux1 / HKV, rows = a.nt * qpk;
+  const int sub = c.warp & (W - 1), nthr = W * 32;
+  const int psh = p.page_shift;
+  const int ntiles = (a.p1 - a.p0 + 15) >> 4;
+  int ti = sub;
+  // Row g of the q rows as A fragments: 8 dims from 32 i + 8 j are k steps 2 i and 2 i + 1; rows past the group's are zero.
+  uint4 qf[4];
+  {
+    const __nv_bfloat16* q0 = reinterpret_cast<const __nv_bfloat16*>(op.out2) + (size_t)(a.t0 + g / qpk) * op.ld_out2 + (size_t)(a.h * qpk + g % qpk) * kHeadDim + 8 * j;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) qf[i] = g < rows ? __ldcg(reinterpret_cast<const uint4*>(q0 + 32 * i)) : make_uint4(0, 0, 0, 0);
+  }
+  if (ti < ntiles && (!loaded || a.p0 + 16 * ti + 15 >= a.fresh)) {
+    const int pg = psh >= 4 ? wide_page(c, a, a.p0 + 16 * ti) : 0;
+    wide_load_k(c, op, a, a.p0 + 16 * ti, pg, kr);
+    wide_load_v(c, op, a, a.p0 + 16 * ti, pg, vr);
+  }
+  int pgn = (psh >= 4 && ti + W < ntiles) ? wide_page(c, a, a.p0 + 16 * (ti + W)) : 0;
+  MK_STAMP(c, 1);
+  float m, l, oacc[8][4];
+  attend_tiles<false>(c, op, a, W, ti, pgn, qf, kr, vr, nullptr, m, l, oacc);
+  MK_STAMP(c, 2);
+  __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out) + (size_t)a.t0 * op.ld_out + (size_t)a.h * qpk * kHeadDim;
+  float* part = p.attn_part + ((size_t)a.t0 * HKV * p.attn_max_chunks * qpk + (size_t)(a.h * p.attn_max_chunks + a.ch) * rows) * (kHeadDim + 2);
+  const __nv_bfloat16* q = reinterpret_cast<const __nv_bfloat16*>(op.out2) + (size_t)a.t0 * op.ld_out2 + (size_t)a.h * qpk * kHeadDim;
+  auto store = [&](int r, int d, const float4& O, float M, float L) {
+    if (a.nch == 1) {
+      const float inv = __fdividef(1.0f, L);
+      *reinterpret_cast<uint2*>(out + (size_t)(r / qpk) * op.ld_out + (r % qpk) * kHeadDim + d) =
+          make_uint2(pack2(O.x * inv, O.y * inv), pack2(O.z * inv, O.w * inv));
+    } else {
+      *reinterpret_cast<float2*>(part + r * kHeadDim + d) = make_float2(O.x, O.y);
+      *reinterpret_cast<float2*>(part + r * kHeadDim + d + 2) = make_float2(O.z, O.w);
+      if (d == 0) {
+        part[rows * kHeadDim + r] = M;
+        part[rows * kHeadDim + rows + r] = L;
+      }
+    }
+  };
+  float chk = 0.f;  // stays zero while the outputs are finite
+  if (W == 1 && a.nch == 1) {
+#pragma unroll
+    for (int y = 0; y < 2; ++y) {
+      const float lr = __shfl_sync(0xffffffffu, l, 8 * j + 4 * y);
+      const int r = 2 * j + y;
+      if (r < rows) {
+        const float inv = __fdividef(1.0f, lr);
+        __nv_bfloat16* dst = out + (size_t)(r / qpk) * op.ld_out + (r % qpk) * kHeadDim + 8 * g;
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          float f[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            f[i] = oacc[i][2 * x + y] * inv;
+            chk = fmaf(f[i], 0.f, chk);
+          }
+          *reinterpret_cast<uint4*>(dst + 64 * x) = pack8(f);
         }
       }
     }
+    __syncwarp();
+    if (__any_sync(0xffffffffu, chk != 0.f)) attend_exact(p, op, a, W, q, op.ld_out2, kHeadDim, store);
+    return;
   }
+  const uint32_t nbar = (uint32_t)(2 + gi);
+  attend_combine(c, W, gi, rows, reg, ml, m, l, oacc, [&](int, int r, int d, const float4& O, float M, float L) {
+    chk = fmaf(O.x, 0.f, fmaf(O.y, 0.f, fmaf(O.z, 0.f, fmaf(O.w, 0.f, chk))));
+    store(r, d, O, M, L);
+  });
   MK_STAMP(c, 3);
   if (bar_any((int)nbar, nthr, chk != 0.f)) {  // (the group's memory is free again)
-    wide_attend_exact(c.p, op, a, W, out, part);
+    attend_exact(p, op, a, W, q, op.ld_out2, kHeadDim, store);
     asm volatile("bar.sync %0, %1;" ::"r"(nbar), "r"(nthr) : "memory");
   }
   if (a.nch == 1) return;

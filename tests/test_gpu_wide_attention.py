@@ -211,3 +211,41 @@ def test_qkv_epilogue_gives_the_bits_of_the_separate_preparation(requests, n_q, 
     assert not torch.equal(got[0][1].cpu(), cache[0])
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+# The row-owner path (one or two new tokens): lengths at the borders of a tile (16), of a round of eight tiles (128), of what one
+# CTA takes alone (256) and of chunks beyond; two requests of different lengths; two tokens of one request; 1 to 8 q heads per kv head.
+@pytest.mark.parametrize("page", [4, 64])
+@pytest.mark.parametrize("n_q,n_kv", [(4, 4), (8, 4), (32, 8), (16, 2)])
+@pytest.mark.parametrize("requests", [[(0, 1)], [(15, 1)], [(16, 1)], [(127, 1)], [(128, 1)], [(255, 1)], [(256, 1)], [(1000, 1)], [(5, 1), (271, 1)],
+                                      [(700, 1), (384, 1)], [(40, 2)], [(300, 2)]])
+def test_one_or_two_tokens(requests, n_q, n_kv, page):
+    a = Attention(requests, n_q, n_kv, page, seed=41)
+    wrong = total = 0
+    for r, (_, n) in enumerate(a.requests):
+        for i in range(n):
+            ref, got = a.reference(r, i), a.out[a.starts[r] + i].double()
+            assert float((got - ref).abs().max()) <= 1e-2 * float(ref.abs().max()), f"request {r} token {i}"
+            wrong, total = wrong + int((got != ref.to(BF).double()).sum()), total + ref.numel()
+            pos, _, _, k, v = a.token(r, i)
+            at = (a.pages[r][pos // page], pos % page)
+            assert torch.equal(a.vcd[at].cpu(), v)
+            assert float((a.kcd[at].cpu().float() - k.float()).abs().max()) <= 2 ** -7 * float(k.float().abs().max())
+    assert wrong <= 4 + 1e-3 * total, (wrong, total)  # (fp32 probabilities, as above)
+
+
+@pytest.mark.parametrize("requests,n_q,n_kv", [([(40, 1)], 16, 4), ([(300, 1), (7, 1)], 16, 8), ([(600, 1)], 16, 2), ([(50, 2)], 8, 2)])
+def test_infinite_values_of_one_or_two_tokens(requests, n_q, n_kv):
+    def edit(a):
+        rows = a.qkv.view(a.qkv.shape[0], n_kv, n_q // n_kv + 2, D)
+        rows[-1, :, -1, 5] = math.inf  # the last new token
+        p = a.pages[0][0]
+        a.vc[p, 2, :, 100] = -math.inf  # position 2 of the first request
+    a = Attention(requests, n_q, n_kv, 16, seed=6, edit=edit)
+    for r, (_, n) in enumerate(requests):
+        for i in range(n):
+            ref, got = a.reference(r, i), a.out[a.starts[r] + i].double()
+            assert torch.equal(ref.isnan(), got.isnan()) and torch.equal(ref.isinf(), got.isinf()), f"request {r} token {i}"
+            assert torch.equal(ref[ref.isinf()], got[ref.isinf()])
+            fin = ref.isfinite()
+            assert float((got[fin] - ref[fin]).abs().max()) <= 1e-2 * float(ref[fin].abs().max())
