@@ -421,3 +421,46 @@ def test_norm_rows_are_not_overwritten_while_the_linear_before_reads_them(widths
     assert [ln.split()[1] for ln in ops] == ["rmsnorm", "linear", "rmsnorm", "linear"]
     sync = [int(ln.split("flags=")[1].split()[0], 16) & 1 for ln in ops]
     assert sync == [0, 1, 1 if barrier else 0, 1], ops
+
+
+@pytest.mark.parametrize("tokens,numerics,form,folded", [
+    (3, "torch", "plain", True), (32, "torch", "plain", True), (33, "torch", "plain", False), (8, "mpk", "plain", True), (9, "mpk", "plain", False),
+    (4, "torch", "user input", False), (4, "torch", "user output", False), (4, "torch", "second reader", False), (4, "torch", "in place", False),
+    (4, "torch", "no linear before", False), (4, "torch", "residual of the rows", True)])
+def test_norms_folded_into_activation_boxes(tokens, numerics, form, folded):
+    """linear -> RMSNorm -> linear on the wide path: the norm goes into the second linear's boxes only where nobody else can see
+    the normalised rows and the rows that are read meanwhile are the runtime's own."""
+    n = 256
+    k = mk.PersistentKernel(mode="online_notoken", world_size=1, mpi_rank=0, num_workers=0, num_local_schedulers=0, num_remote_schedulers=0,
+                            max_seq_length=64, max_num_batched_requests=tokens, max_num_batched_tokens=tokens, max_num_pages=tokens, page_size=64,
+                            meta_tensors=_meta(tokens, tokens, 64, tokens), profiler_tensor=None, trace_name="", spec_decode_config=None,
+                            use_cutlass_kernel=True, numerics=numerics)
+    held = []
+
+    def attach(name, *shape):
+        held.append(torch.zeros(shape, dtype=torch.bfloat16))
+        return k.attach_input(held[-1], name)
+
+    def own(name):
+        return k.new_tensor(dims=(tokens, n), name=name)
+
+    grid = dict(grid_dim=(4, 1, 1), block_dim=(128, 1, 1))
+    h = attach("h", tokens, n) if form == "user input" else own("h")
+    a = attach("a", tokens, n) if form == "user output" else own("a")
+    y = h if form == "in place" else attach("y", tokens, n)
+    if form == "no linear before":
+        k.rmsnorm_layer(input=attach("x", tokens, n), weight=attach("n0", n), output=h, **grid)
+    else:
+        k.linear_layer(input=attach("x", tokens, n), weight=attach("w0", n, n), output=h, **grid)
+    k.rmsnorm_layer(input=h, weight=attach("n1", n), output=a, **grid)
+    if form == "residual of the rows":
+        k.linear_with_residual_layer(input=a, weight=attach("w1", n, n), residual=h, output=y, **grid)
+    else:
+        k.linear_layer(input=a, weight=attach("w1", n, n), output=y, **grid)
+    if form == "second reader":
+        k.linear_layer(input=a, weight=attach("w2", n, n), output=attach("z", tokens, n), **grid)
+    text = C.create_string_buffer(1 << 16)
+    ops = k._lib.mk_debug_describe_wide(k._h, text, 1 << 16)
+    assert ops == (4 if form == "second reader" else 3) - int(folded), text.value.decode()
+    assert ("rmsnorm in the activation boxes" in text.value.decode()) == folded
+    k.finalize()
