@@ -5,7 +5,7 @@
 // 128-byte swizzle) into a ring of shared-memory stages, running ahead of the consumers across op
 // boundaries (weights have no dependencies); the eight consumer warps walk the program: wait at a
 // grid barrier where an op reads what other CTAs wrote, do the op's share of work, go on.  The wide
-// path (mk_wide.cuh) has two more roles, an activation producer and an MMA issuer.  Every wait in
+// path (mk_wide.cuh) has three more roles, an activation producer, an MMA issuer and a norm warp.  Every wait in
 // the kernel is bounded: on expiry the waiter records a status and raises a sticky abort flag that
 // all other waits poll, and the kernel returns with an error code.
 //

@@ -22,7 +22,7 @@ constexpr int kStageBytes = kSubBytes * kSubTiles;
 constexpr int kNumConsumerWarps = 8;
 constexpr int kNumConsumers = kNumConsumerWarps * 32;
 // + a warpgroup of service warps: the weight producer, the activation producer (or L2 look-ahead) and, on the wide path, the
-// MMA issuer; on the wide path, the norm warp.  The block starts with 168 registers a thread; the service warps hand theirs to the
+// MMA issuer and the norm warp.  The block starts with 168 registers a thread; the service warps hand theirs to the
 // consumers (their sum is what the block was launched with).
 constexpr int kNumThreads = kNumConsumers + 128;
 constexpr int kServiceRegs = 56, kConsumerRegs = 224;
