@@ -129,8 +129,8 @@ struct Program {
   int smem_bytes = 0;
   int64_t weight_bytes = 0;
   int max_nblk = 1;
-  size_t attn_count_bytes = 0, piece_count_bytes = 0;  // arrival counters, cleared before every kernel launch
-  void* ll_buf = nullptr;  // tagged activation words of the program, cleared before every kernel launch
+  void* ll_buf = nullptr;  // tagged words of the program, then its arrival counters: cleared before every kernel launch
+  size_t clear_bytes = 0;
   size_t ll_bytes = 0;
 };
 
@@ -169,8 +169,8 @@ struct mk_handle {
   unsigned xchg_total = 0;      // cross-rank exchanges executed by all completed launches (all ranks advance alike)
   bool in_flight = false;       // launched and not yet waited for
   bool poisoned = false;        // a tensor-parallel launch aborted: the ranks' exchange sequences may differ
-  size_t attn_count_bytes = 0;  // the attention chunk counters, cleared before every launch
-  size_t piece_count_bytes = 0; // the split-k arrival counters, cleared before every launch
+  size_t clear_bytes = 0;       // of ll_buf: the words and the arrival counters behind them
+  void* launch_stream = nullptr;
   void* ll_buf = nullptr;       // tagged activation words of the program being compiled
   size_t ll_bytes = 0;
 
@@ -1584,9 +1584,15 @@ static int compile_program(mk_handle* h, bool first) {
   if (words) ll_bytes += (size_t)h->grid * mk::kTileRows * x_rows * 8;
   h->ll_buf = nullptr;
   h->ll_bytes = ll_bytes;
-  if (ll_bytes > 0) {
-    if (int e = h->dmalloc(&h->ll_buf, ll_bytes)) return e;
-  }
+  // behind the words: the counters of the attention chunks and of the split-k pieces
+  int count_hkv = 1;
+  for (const PlanOp& po : h->plan)
+    if (po.type == mk::OP_ATTN) count_hkv = std::max(count_hkv, po.aux0);
+  const size_t count_off = (ll_bytes + 255) / 256 * 256, attn_counts = (size_t)h->plan_tokens * count_hkv;
+  h->clear_bytes = count_off + (attn_counts + (rows_mode ? 1 : (size_t)max_nblk * mk::kNumConsumerWarps)) * 4;
+  if (int e = h->dmalloc(&h->ll_buf, h->clear_bytes)) return e;
+  kp.attn_count = (unsigned*)((char*)h->ll_buf + count_off);
+  kp.piece_count = kp.attn_count + attn_counts;
   kp.partial = words ? (uint4*)((char*)h->ll_buf + partial_off) : nullptr;
   kp.attn_part_ll = ll_part ? (uint2*)((char*)h->ll_buf + ll_part_off) : nullptr;
 
@@ -1597,9 +1603,6 @@ static int compile_program(mk_handle* h, bool first) {
     if (int e = h->dmalloc(&p, (size_t)G * mk::kTileRows * x_rows * 4)) return e;
     kp.partial = (uint4*)p;
   }
-  h->piece_count_bytes = rows_mode ? 4 : (size_t)max_nblk * mk::kNumConsumerWarps * 4;
-  if (int e = h->dmalloc(&p, h->piece_count_bytes)) return e;
-  kp.piece_count = (unsigned*)p;
   int max_hkv = 1, max_qpk = 2;
   for (const PlanOp& po : h->plan)
     if (po.type == mk::OP_ATTN) {
@@ -1615,9 +1618,6 @@ static int compile_program(mk_handle* h, bool first) {
   kp.attn_max_chunks = kAttnMaxChunks;
   if (int e = h->dmalloc(&p, (size_t)h->plan_tokens * max_hkv * kAttnMaxChunks * max_qpk * (mk::kHeadDim + 2) * 4)) return e;
   kp.attn_part = (float*)p;
-  h->attn_count_bytes = (size_t)h->plan_tokens * max_hkv * 4;
-  if (int e = h->dmalloc(&p, h->attn_count_bytes)) return e;
-  kp.attn_count = (unsigned*)p;
   if (first) {
     if (int e = h->dmalloc(&p, (size_t)cfg.max_num_batched_requests * 4)) return e;
     kp.request_ids = (int*)p;
@@ -1963,8 +1963,7 @@ int mk_compile(mk_handle* h) {
   h->prog[0].plan = h->plan; h->prog[0].rows_mode = h->rows_mode; h->prog[0].max_tokens = h->plan_tokens;
   h->prog[0].kp = h->kp; h->prog[0].smem_bytes = h->smem_bytes; h->prog[0].weight_bytes = h->weight_bytes;
   h->prog[0].max_nblk = h->max_nblk;
-  h->prog[0].attn_count_bytes = h->attn_count_bytes; h->prog[0].piece_count_bytes = h->piece_count_bytes;
-  h->prog[0].ll_buf = h->ll_buf; h->prog[0].ll_bytes = h->ll_bytes;
+  h->prog[0].ll_buf = h->ll_buf; h->prog[0].ll_bytes = h->ll_bytes; h->prog[0].clear_bytes = h->clear_bytes;
   h->nprog = 1;
   if (two) {
     h->plan_tokens = cfg.max_num_batched_tokens;
@@ -1973,8 +1972,7 @@ int mk_compile(mk_handle* h) {
     h->prog[1].plan = h->plan; h->prog[1].rows_mode = h->rows_mode; h->prog[1].max_tokens = h->plan_tokens;
     h->prog[1].kp = h->kp; h->prog[1].smem_bytes = h->smem_bytes; h->prog[1].weight_bytes = h->weight_bytes;
     h->prog[1].max_nblk = h->max_nblk;
-    h->prog[1].attn_count_bytes = h->attn_count_bytes; h->prog[1].piece_count_bytes = h->piece_count_bytes;
-    h->prog[1].ll_buf = h->ll_buf; h->prog[1].ll_bytes = h->ll_bytes;
+      h->prog[1].ll_buf = h->ll_buf; h->prog[1].ll_bytes = h->ll_bytes; h->prog[1].clear_bytes = h->clear_bytes;
     h->nprog = 2;
     h->prog[0].kp.tok_lo = 1;
     h->prog[0].kp.tok_hi = h->prog[0].max_tokens;
@@ -2008,11 +2006,12 @@ int mk_init_requests(mk_handle* h, void* stream) {
 
 // One kernel of a generation call: the program's counters and the launch state are reset, then the
 // persistent kernel of that program is launched.
-static int launch_program(mk_handle* h, int idx, void* stream) {
+static int launch_program(mk_handle* h, int idx, void* stream, bool first) {
   Program& P = h->prog[idx];
   cudaStream_t s = (cudaStream_t)stream;
   // grid barrier, control word, abort flag and status live in one 256-byte block behind sched[0..15]
-  cudaError_t ce = cudaMemsetAsync((char*)P.kp.sched + 64, 0, 192, s);
+  // (a generation call starts with no iteration handed over and none completed: sched[5..7] too)
+  cudaError_t ce = cudaMemsetAsync(P.kp.sched + (first ? 5 : 16), 0, first ? 236 : 192, s);
   if (ce != cudaSuccess) return h->cuda_fail(ce, "state reset");
   if (P.kp.bar_epoch0 != 0) {
     // (tests) the counter starts where barrier number bar_epoch0 has just been passed
@@ -2020,20 +2019,15 @@ static int launch_program(mk_handle* h, int idx, void* stream) {
     ce = cudaMemcpyAsync(P.kp.grid_bar, &start, 4, cudaMemcpyHostToDevice, s);
     if (ce != cudaSuccess) return h->cuda_fail(ce, "state reset");
   }
-  // a launch that aborted may have left the arrival counters of its attention chunks and of its
-  // split-k pieces half-way: a finisher that gave up clears its counter while late pieces still add to it
-  ce = cudaMemsetAsync(P.kp.attn_count, 0, P.attn_count_bytes, s);
+  // Tags restart with every kernel: no word of an earlier one may look valid.  And a launch that aborted may have left
+  // arrival counters half-way: a finisher that gave up clears its counter while late pieces still add to it.
+  ce = cudaMemsetAsync(P.ll_buf, 0, P.clear_bytes, s);
   if (ce != cudaSuccess) return h->cuda_fail(ce, "state reset");
-  ce = cudaMemsetAsync(P.kp.piece_count, 0, P.piece_count_bytes, s);
-  if (ce != cudaSuccess) return h->cuda_fail(ce, "state reset");
-  if (P.ll_bytes > 0) {  // tags restart with every kernel: no word of an earlier one may look valid
-    ce = cudaMemsetAsync(P.ll_buf, 0, P.ll_bytes, s);
-    if (ce != cudaSuccess) return h->cuda_fail(ce, "state reset");
-  }
   // exchange sequence numbers continue where the last kernel stopped (mk_wait adds what it executed)
   P.kp.xchg_seq_base = h->xchg_total;
   int e = mk_kernel_launch(&P.kp, h->grid, P.smem_bytes, stream);
   if (e) return h->cuda_fail((cudaError_t)e, "cooperative launch");
+  h->launch_stream = stream;
   return 0;
 }
 
@@ -2044,10 +2038,7 @@ int mk_launch_async(mk_handle* h, void* stream) {
   if (h->poisoned)
     return h->fail(MK_E_STATE, "an earlier tensor-parallel launch aborted: the ranks' exchange sequence numbers may "
                                "differ; finalize this handle on every rank and build a new one");
-  // a generation call starts with no iteration handed over and none completed (sched[5..7])
-  cudaError_t ce = cudaMemsetAsync(h->prog[0].kp.sched + 5, 0, 12, (cudaStream_t)stream);
-  if (ce != cudaSuccess) return h->cuda_fail(ce, "state reset");
-  if (int e = launch_program(h, h->cur_prog, stream)) return e;
+  if (int e = launch_program(h, h->cur_prog, stream, true)) return e;
   h->launched = true;
   h->in_flight = true;
   return 0;
@@ -2057,18 +2048,20 @@ int mk_wait(mk_handle* h, void* stream) {
   if (!h) return MK_E_INVALID;
   if (!h->launched) return h->fail(MK_E_STATE, "nothing launched");
   while (true) {
-    cudaError_t ce = cudaStreamSynchronize((cudaStream_t)stream);
+    // sched[0..15], then barrier counter, abort flag, control words and status.  The copy is enqueued behind the kernel, not
+    // started when it has ended (unless the caller waits on another stream than the launch's).
+    int state[64];
+    cudaError_t ce = cudaSuccess;
+    if (stream == h->launch_stream) ce = cudaMemcpyAsync(state, h->prog[0].kp.sched, sizeof(state), cudaMemcpyDeviceToHost, (cudaStream_t)stream);
+    if (ce == cudaSuccess) ce = cudaStreamSynchronize((cudaStream_t)stream);
     h->in_flight = false;
     if (ce != cudaSuccess) return h->cuda_fail(ce, "megakernel");
-    int st[24];
-    ce = cudaMemcpy(st, h->prog[0].kp.abort_flag, sizeof(int) * 24, cudaMemcpyDeviceToHost);
-    if (ce != cudaSuccess) return h->cuda_fail(ce, "status readback");
-    if (h->cfg.world_size > 1) {
-      int done = 0;
-      ce = cudaMemcpy(&done, h->prog[0].kp.sched + 6, 4, cudaMemcpyDeviceToHost);
+    if (stream != h->launch_stream) {
+      ce = cudaMemcpy(state, h->prog[0].kp.sched, sizeof(state), cudaMemcpyDeviceToHost);
       if (ce != cudaSuccess) return h->cuda_fail(ce, "status readback");
-      h->xchg_total += (unsigned)done;
     }
+    const int* st = state + 17;  // the abort flag and what sits behind it
+    if (h->cfg.world_size > 1) h->xchg_total += (unsigned)state[6];
     if (st[0] != 0) {
       static const char* names[] = {"ok", "grid barrier timed out", "weight stage never arrived", "weight ring never drained",
                                     "producer never got the next iteration", "peer never arrived", "token id out of range",
@@ -2084,7 +2077,7 @@ int mk_wait(mk_handle* h, void* stream) {
     // handle's other program and ended; that program takes over on the same stream
     if (st[3] != -2 || h->nprog < 2) return 0;
     h->cur_prog ^= 1;
-    if (int e = launch_program(h, h->cur_prog, stream)) return e;
+    if (int e = launch_program(h, h->cur_prog, stream, false)) return e;
     h->in_flight = true;
   }
 }
