@@ -4,7 +4,9 @@
 CUDA sources for sm_100a into ``libb200mk.so`` next to this file.  The built
 library is what the package loads; there is no fallback when it is missing.
 """
+import json
 import os
+import re
 import shutil
 import subprocess
 import sys
@@ -13,6 +15,8 @@ from concurrent.futures import ThreadPoolExecutor
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libb200mk.so")
+OBJDIR = os.path.join(HERE, "build")
+REPORT = os.path.join(OBJDIR, "instances.json")  # what ptxas made of every kernel instance
 # mk_kernel_tp.cu, mk_kernel_hier.cu and mk_kernel_moe.cu include mk_kernel.cu with other build switches (see its header); each
 # is compiled once per linear path (MK_NC, see mk_launch.cu)
 SOURCES = {"mk_kernel.cu": (0, 8, 16, 32), "mk_kernel_tp.cu": (0, 8, 16, 32), "mk_kernel_hier.cu": (0, 8, 16, 32), "mk_kernel_moe.cu": (0, 8),
@@ -35,29 +39,51 @@ def needs_build():
     return any(os.path.getmtime(d) > t for d in deps if os.path.exists(d))
 
 
+def resources(ptxas):
+    """Registers, stack and spills (bytes) a thread of the megakernel, from the output of ``ptxas -v``; None without one."""
+    entry = re.search(r"Compiling entry function '\w*megakernel\w*'.*?(?=Compiling entry function|\Z)", ptxas, re.S)
+    if entry is None:
+        return None
+    stack, stores, loads = map(int, re.search(r"(\d+) bytes stack frame, (\d+) bytes spill stores, (\d+) bytes spill loads", entry[0]).groups())
+    return {"registers": int(re.search(r"Used (\d+) registers", entry[0])[1]), "stack": stack, "spill_stores": stores, "spill_loads": loads}
+
+
+def check_registers(instances):
+    """The warp roles share out kLaunchRegs registers a thread (mk_types.h): an instance with fewer would wait for them for good."""
+    with open(os.path.join(CSRC, "mk_types.h")) as f:
+        need = int(re.search(r"kLaunchRegs = (\d+)", f.read())[1])
+    few = {name: r["registers"] for name, r in instances.items() if r["registers"] < need}
+    if few:
+        raise RuntimeError(f"kernel instances with fewer than {need} registers a thread: {few}")
+
+
 def build(force=False, verbose=False):
     if not force and not needs_build():
         return LIB
-    flags = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
-    if verbose:
-        flags = ["-Xptxas", "-v"] + flags
-    objdir = os.path.join(HERE, "build")
-    os.makedirs(objdir, exist_ok=True)
+    flags = ["-Xptxas", "-v", "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17", "-Xcompiler", "-fPIC"]
+    os.makedirs(OBJDIR, exist_ok=True)
     jobs = []
     for src, instances in SOURCES.items():
         stem = os.path.splitext(src)[0]
         for nc in instances or (None,):
-            obj = os.path.join(objdir, stem + ("" if nc is None else f"_{nc}") + ".o")
+            obj = os.path.join(OBJDIR, stem + ("" if nc is None else f"_{nc}") + ".o")
             define = [] if nc is None else [f"-DMK_NC={nc}"]
             jobs.append(([_nvcc()] + flags + define + ["-c", os.path.join(CSRC, src), "-o", obj], obj))
     # one nvcc per object, as many side by side as there are cores, then one link
     with ThreadPoolExecutor(max_workers=os.cpu_count() or 4) as pool:
         done = list(pool.map(lambda job: subprocess.run(job[0], stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True), jobs))
-    for (cmd, _), r in zip(jobs, done):
+    instances = {}
+    for (cmd, obj), r in zip(jobs, done):
         if verbose or r.returncode != 0:
             sys.stdout.write(" ".join(cmd) + "\n" + r.stdout)
         if r.returncode != 0:
             raise subprocess.CalledProcessError(r.returncode, cmd)
+        name = os.path.splitext(os.path.basename(obj))[0]
+        if name.startswith("mk_kernel"):
+            instances[name] = resources(r.stdout)
+    check_registers(instances)
+    with open(REPORT, "w") as f:
+        json.dump(instances, f, indent=1)
     objs = [obj for _, obj in jobs]
     subprocess.check_call([_nvcc(), "-shared", "-o", LIB] + objs)
     return LIB

@@ -1,6 +1,8 @@
 // Launching the megakernel: picks the instance of the kernel a program runs, and the kernel that resets the scheduler state.
 #include <cuda_runtime.h>
 
+#include <atomic>
+
 #include "mk_types.h"
 
 // mk_kernel.cu is compiled once per build (see its header) and per linear path: the row-owner path (0), and the wide path
@@ -50,33 +52,39 @@ const Instance kInstances[4][4] = {
     {mk_instance_hier_0, mk_instance_hier_8, mk_instance_hier_16, mk_instance_hier_32},
     {mk_instance_moe_0, mk_instance_moe_8, nullptr, nullptr},  // (MoE programs serve one or two tokens)
 };
-const void* instance(Build b, int path, int x_rows) {
-  const Instance f = kInstances[b][path == mk::PATH_ROWS ? 0 : (x_rows <= 16 ? 1 : (x_rows <= 32 ? 2 : 3))];
-  return f ? f() : nullptr;
-}
-// the build a launch needs: tensor-parallel exchange code only when there are peers, the hierarchical barrier only when the
-// launch uses clusters, the MoE ops only when the program has them
-const void* kernel_for(const mk::KParams* p) {
-  return instance(p->has_moe ? MOE : (p->cluster > 1 ? HIER : (p->world > 1 ? TP : BASE)), p->path, p->x_rows);
+// The kernel that a launch with these parameters runs: tensor-parallel exchange code only when there are peers, the
+// hierarchical barrier only when the launch uses clusters, the MoE ops only when the program has them.  Null where there is no
+// such instance, or where it has fewer registers than the warp roles split among them: its setmaxnreg.inc would wait for good,
+// the one wait of the kernel that nothing bounds.  (What an instance was compiled to does not change: asked once per process.)
+const void* kernel_for(const mk::KParams* p, int cluster) {
+  static std::atomic<int> fits[4][4];  // 0 not asked yet, 1 yes, -1 no
+  const Build b = p->has_moe ? MOE : (cluster > 1 ? HIER : (p->world > 1 ? TP : BASE));
+  const int i = p->path == mk::PATH_ROWS ? 0 : (p->x_rows <= 16 ? 1 : (p->x_rows <= 32 ? 2 : 3));
+  if (!kInstances[b][i]) return nullptr;
+  const void* k = kInstances[b][i]();
+  int ok = fits[b][i].load(std::memory_order_relaxed);
+  if (ok == 0) {
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, k) != cudaSuccess) return nullptr;  // (no device, or not this one: asked again)
+    ok = fa.numRegs >= mk::kLaunchRegs ? 1 : -1;
+    fits[b][i].store(ok, std::memory_order_relaxed);
+  }
+  return ok > 0 ? k : nullptr;
 }
 }  // namespace
 
 extern "C" int mk_kernel_max_ctas_per_sm(const mk::KParams* p, int smem_bytes) {
   int n = 0;
-  const void* k = kernel_for(p);
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) return -1;
-  // the register split of the warp roles draws on what the block is launched with: an instance with less must not run
-  cudaFuncAttributes fa;
-  if (cudaFuncGetAttributes(&fa, k) != cudaSuccess) return -1;
-  if (fa.numRegs * mk::kNumThreads < 128 * mk::kServiceRegs + mk::kNumConsumers * mk::kConsumerRegs) return -1;
+  const void* k = kernel_for(p, p->cluster);
+  if (!k || cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) return -1;
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, mk::kNumThreads, smem_bytes) != cudaSuccess) return -1;
   return n;
 }
 
 // Clusters of `cluster` CTAs that can be resident at once (the hierarchical barrier needs all of them).
-extern "C" int mk_kernel_max_clusters(int path, int x_rows, int smem_bytes, int cluster, int grid) {
-  const void* k = instance(HIER, path, x_rows);
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) return -1;
+extern "C" int mk_kernel_max_clusters(const mk::KParams* p, int smem_bytes, int cluster, int grid) {
+  const void* k = kernel_for(p, cluster);
+  if (!k || cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess) return -1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(mk::kNumThreads);
@@ -97,7 +105,8 @@ extern "C" int mk_kernel_max_clusters(int path, int x_rows, int smem_bytes, int 
 }
 
 extern "C" int mk_kernel_launch(const mk::KParams* p, int grid, int smem_bytes, void* stream) {
-  const void* k = kernel_for(p);
+  const void* k = kernel_for(p, p->cluster);
+  if (!k) return (int)cudaErrorInvalidDeviceFunction;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes);
   if (e != cudaSuccess) return (int)e;
   void* args[] = {(void*)p};

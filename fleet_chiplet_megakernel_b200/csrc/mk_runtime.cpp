@@ -25,7 +25,7 @@
 #include "mk_types.h"
 
 extern "C" int mk_kernel_max_ctas_per_sm(const mk::KParams* p, int smem_bytes);
-extern "C" int mk_kernel_max_clusters(int path, int x_rows, int smem_bytes, int cluster, int grid);
+extern "C" int mk_kernel_max_clusters(const mk::KParams* p, int smem_bytes, int cluster, int grid);
 extern "C" int mk_kernel_launch(const mk::KParams* p, int grid, int smem_bytes, void* stream);
 extern "C" int mk_kernel_init_state(const mk::KParams* p, void* stream);
 
@@ -1405,8 +1405,9 @@ static int compile_program(mk_handle* h, bool first) {
   kp.rank = cfg.rank;
   kp.world = cfg.world_size;
   kp.cluster = 1;
+  kp.has_moe = has_moe ? 1 : 0;  // (with path, x_rows, world and cluster: what picks the kernel that the next line asks about)
   const int per_sm = mk_kernel_max_ctas_per_sm(&kp, h->smem_bytes);
-  if (per_sm < 1) return h->fail(MK_E_CUDA, "the megakernel does not fit on an SM with %d bytes of shared memory", h->smem_bytes);
+  if (per_sm < 1) return h->fail(MK_E_CUDA, "the megakernel does not fit on an SM with %d bytes of shared memory, or was built with too few registers", h->smem_bytes);
   h->grid = h->num_sms;
   if (cfg.num_workers > 0) h->grid = std::min(h->grid, cfg.num_workers);
   // Grid barrier shape: hierarchical (cluster-first) when asked for and every cluster of the grid
@@ -1414,7 +1415,7 @@ static int compile_program(mk_handle* h, bool first) {
   if (cfg.cluster_size == 2 || cfg.cluster_size == 4) {
     if (cfg.world_size > 1) return h->fail(MK_E_UNSUPPORTED, "the cluster-first grid barrier is only built for single-GPU launches");
     const int cs = cfg.cluster_size;
-    const int fit = mk_kernel_max_clusters(kp.path, x_rows, h->smem_bytes, cs, h->grid / cs * cs);
+    const int fit = mk_kernel_max_clusters(&kp, h->smem_bytes, cs, h->grid / cs * cs);
     if (fit >= 1) {
       kp.cluster = cs;
       h->grid = std::min(h->grid / cs, fit) * cs;
@@ -1911,7 +1912,6 @@ static int compile_program(mk_handle* h, bool first) {
   // L2 look-ahead of the weight stream, in 32 KB stages: on by default (512 KB per CTA, the
   // measured optimum with evict-first weight loads) for a row-owner program whose ops all keep their grid
   // barriers, off elsewhere (it measured slower there); prefetch_kb > 0 sets it, < 0 turns it off
-  kp.has_moe = has_moe ? 1 : 0;
   // (no look-ahead with expert layers: which weights come next is only known after routing)
   // (with tagged activations the gaps between the ops are short and the look-ahead only competes with the ring:
   // measured 3.51 against 3.56 ms per step at context 100 and 3.84 against 3.97 at context 600 with it off)

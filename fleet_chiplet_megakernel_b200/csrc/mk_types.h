@@ -22,11 +22,11 @@ constexpr int kStageBytes = kSubBytes * kSubTiles;
 constexpr int kNumConsumerWarps = 8;
 constexpr int kNumConsumers = kNumConsumerWarps * 32;
 // + a warpgroup of service warps: the weight producer, the activation producer (or L2 look-ahead) and, on the wide path, the
-// MMA issuer and the norm warp.  The block starts with 168 registers a thread; the service warps hand theirs to the
-// consumers (their sum is what the block was launched with).
+// MMA issuer and the norm warp.  The block starts with kLaunchRegs registers a thread; the service warps hand theirs to the
+// consumers (their sum is what the block was launched with; an instance that is compiled to fewer is not launched).
 constexpr int kNumThreads = kNumConsumers + 128;
-constexpr int kServiceRegs = 56, kConsumerRegs = 224;
-static_assert(128 * kServiceRegs + kNumConsumers * kConsumerRegs == kNumThreads * 168, "a register split beyond the block's own would wait for good");
+constexpr int kServiceRegs = 56, kConsumerRegs = 224, kLaunchRegs = 168;
+static_assert(128 * kServiceRegs + kNumConsumers * kConsumerRegs == kNumThreads * kLaunchRegs, "a register split beyond the block's own would wait for good");
 constexpr int kWideRedBytes = 4096;              // scratch of the wide path: reductions and the iteration's token table
 constexpr int kHeadDim = 128;
 constexpr int kNormBoxRows = 32;                 // widest activation box that the norm is applied to in shared memory
