@@ -18,8 +18,8 @@ LIB = os.path.join(HERE, "libb200mk.so")
 OBJDIR = os.path.join(HERE, "build")
 REPORT = os.path.join(OBJDIR, "instances.json")  # what ptxas made of every kernel instance
 # mk_kernel_tp.cu, mk_kernel_hier.cu and mk_kernel_moe.cu include mk_kernel.cu with other build switches (see its header); each
-# is compiled once per linear path (MK_NC, see mk_launch.cu)
-SOURCES = {"mk_kernel.cu": (0, 8, 16, 32), "mk_kernel_tp.cu": (0, 8, 16, 32), "mk_kernel_hier.cu": (0, 8, 16, 32), "mk_kernel_moe.cu": (0, 8),
+# is compiled once per linear path that its programs take (MK_NC, see mk_launch.cu)
+SOURCES = {"mk_kernel.cu": (0, 8, 16, 32), "mk_kernel_tp.cu": (0, 8, 16, 32), "mk_kernel_hier.cu": (0, 8, 16, 32), "mk_kernel_moe.cu": (0,),
            "mk_launch.cu": None, "mk_runtime.cpp": None, "mk_noalloc.cu": None}
 HEADERS = ["mk_types.h", "mk_wide.cuh", os.path.join("..", "..", "include", "b200mk.h")]
 

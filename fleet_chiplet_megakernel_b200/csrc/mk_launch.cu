@@ -10,14 +10,12 @@
 // that a process loads the one it runs.
 #define MK_DECLARE(v) \
   extern "C" const void* mk_instance_##v##_0(); \
-  extern "C" const void* mk_instance_##v##_8();
-MK_DECLARE(base) MK_DECLARE(tp) MK_DECLARE(hier) MK_DECLARE(moe)
-#undef MK_DECLARE
-#define MK_DECLARE(v) \
+  extern "C" const void* mk_instance_##v##_8(); \
   extern "C" const void* mk_instance_##v##_16(); \
   extern "C" const void* mk_instance_##v##_32();
 MK_DECLARE(base) MK_DECLARE(tp) MK_DECLARE(hier)
 #undef MK_DECLARE
+extern "C" const void* mk_instance_moe_0();
 
 namespace mk {
 __global__ void init_state_kernel(KParams p) {
@@ -50,7 +48,7 @@ const Instance kInstances[4][4] = {
     {mk_instance_base_0, mk_instance_base_8, mk_instance_base_16, mk_instance_base_32},
     {mk_instance_tp_0, mk_instance_tp_8, mk_instance_tp_16, mk_instance_tp_32},
     {mk_instance_hier_0, mk_instance_hier_8, mk_instance_hier_16, mk_instance_hier_32},
-    {mk_instance_moe_0, mk_instance_moe_8, nullptr, nullptr},  // (MoE programs serve one or two tokens)
+    {mk_instance_moe_0, nullptr, nullptr, nullptr},  // (MoE layers are planned for one or two tokens only: row-owner path)
 };
 // The kernel that a launch with these parameters runs: tensor-parallel exchange code only when there are peers, the
 // hierarchical barrier only when the launch uses clusters, the MoE ops only when the program has them.  Null where there is no

@@ -16,7 +16,7 @@ static char insts[16];
 static int regs[16], asked, launched;
 #define INST(name, i) extern "C" const void* mk_instance_##name() { return insts + i; }
 INST(base_0, 0) INST(base_8, 1) INST(base_16, 2) INST(base_32, 3) INST(tp_0, 4) INST(tp_8, 5) INST(tp_16, 6) INST(tp_32, 7)
-INST(hier_0, 8) INST(hier_8, 9) INST(hier_16, 10) INST(hier_32, 11) INST(moe_0, 12) INST(moe_8, 13)
+INST(hier_0, 8) INST(hier_8, 9) INST(hier_16, 10) INST(hier_32, 11) INST(moe_0, 12)
 static int index_of(const void* k) { return k >= insts && k < insts + 16 ? (int)((const char*)k - insts) : -1; }
 extern "C" {
 int mk_kernel_max_ctas_per_sm(const mk::KParams*, int);
@@ -97,10 +97,11 @@ def test_an_instance_with_too_few_registers_is_not_launched(fake, launch, inst):
 
 
 def test_a_launch_without_an_instance_is_an_error(fake):
-    """Mixture-of-experts programs serve one or two tokens: there is no instance for wider boxes."""
+    """Mixture-of-experts programs serve one or two tokens: there is no instance of the wide path."""
     out, ret = (C.c_int * 3)(), (C.c_int * 3)()
-    fake("none").probe(-1, 1, 1, 1, 0, 64, out, ret)
-    assert list(out) == [-1, -1, -1] and ret[0] == -1 and ret[2] != 0
+    for x_rows in (16, 32, 64, 128):
+        fake(f"none{x_rows}").probe(-1, 1, 1, 1, 0, x_rows, out, ret)
+        assert list(out) == [-1, -1, -1] and ret[0] == -1 and ret[2] != 0
 
 
 PTXAS = """ptxas info    : 0 bytes gmem
@@ -124,7 +125,7 @@ def test_the_build_refuses_an_instance_with_too_few_registers():
     _build.check_registers({"mk_kernel_16": dict(r, registers=168)})
 
 
-def test_every_built_instance_has_the_registers_of_the_split():
+def test_every_built_instance_has_the_registers_of_the_split(native_lib):
     if not os.path.exists(_build.REPORT):
         pytest.skip("the library was built elsewhere")
     with open(_build.REPORT) as f:
