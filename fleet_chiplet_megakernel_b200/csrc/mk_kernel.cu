@@ -465,34 +465,40 @@ __device__ __forceinline__ float block_sum(Ctx& c, float v) {
 // bulk or tensor copy ever touches a peer's memory.  The halves of a region alternate between
 // consecutive exchanges: a rank can only push exchange s+2 after it has read all of s+1 from
 // every peer, which those peers push after their last read of s.
-__device__ __forceinline__ uint4 ld_sys_v4(const uint4* p) {
-  uint4 v;
-  asm volatile("ld.relaxed.sys.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-  return v;
+// Words travel as what they are, 64-bit scalars {value, number}: only those are single-copy atomic.  (Of a vector of 32-bit scalars
+// the memory model lets the number be newer than the value beside it.)
+__device__ __forceinline__ uint4 split_words(unsigned long long a, unsigned long long b) {
+  return make_uint4((uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32));
 }
-__device__ __forceinline__ uint2 ld_sys_v2(const uint2* p) {
-  uint2 v;
-  asm volatile("ld.relaxed.sys.global.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
-  return v;
+__device__ __forceinline__ unsigned long long join_word(uint32_t value, uint32_t number) { return (unsigned long long)number << 32 | value; }
+__device__ __forceinline__ uint4 ld_sys_words(const uint4* p) {
+  unsigned long long a, b;
+  asm volatile("ld.relaxed.sys.global.v2.b64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+  return split_words(a, b);
 }
-__device__ __forceinline__ void st_sys_v2(uint2* p, uint32_t a, uint32_t b) {
-  asm volatile("st.relaxed.sys.global.v2.u32 [%0], {%1,%2};" ::"l"(p), "r"(a), "r"(b) : "memory");
+__device__ __forceinline__ uint2 ld_sys_word(const uint2* p) {
+  unsigned long long a;
+  asm volatile("ld.relaxed.sys.global.b64 %0, [%1];" : "=l"(a) : "l"(p) : "memory");
+  return make_uint2((uint32_t)a, (uint32_t)(a >> 32));
 }
-__device__ __forceinline__ void st_sys_v4(uint4* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.relaxed.sys.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+__device__ __forceinline__ void st_sys_word(uint2* p, uint32_t value, uint32_t number) {
+  asm volatile("st.relaxed.sys.global.b64 [%0], %1;" ::"l"(p), "l"(join_word(value, number)) : "memory");
+}
+__device__ __forceinline__ void st_sys_words(uint4* p, uint32_t a, uint32_t b, uint32_t number) {
+  asm volatile("st.relaxed.sys.global.v2.b64 [%0], {%1,%2};" ::"l"(p), "l"(join_word(a, number)), "l"(join_word(b, number)) : "memory");
 }
 // one value of exchange `seq` into every rank's region
 __device__ __forceinline__ void xchg_push1(const KParams& p, unsigned seq, int tok, int col, float v) {
   const size_t w = xchg_word(seq, p.world, p.xchg_tokens, p.xchg_cols, p.rank, tok, col);
 #pragma unroll 1
-  for (int r = 0; r < p.world; ++r) st_sys_v2(reinterpret_cast<uint2*>(p.xchg[r]) + w, __float_as_uint(v), seq);
+  for (int r = 0; r < p.world; ++r) st_sys_word(reinterpret_cast<uint2*>(p.xchg[r]) + w, __float_as_uint(v), seq);
 }
 // A word of a rank that is not there yet: poll it (bounded).  Returns false after raising the abort flag.
 __device__ __forceinline__ bool xchg_wait_word(const Ctx& c, const uint2* w, unsigned seq, int src) {
   unsigned long long t0 = 0;
   unsigned spins = 0;
   while (true) {
-    if (xchg_arrived(ld_sys_v2(w).y, seq)) return true;
+    if (xchg_arrived(ld_sys_word(w).y, seq)) return true;
     if (((++spins) & 63u) == 0) {
       if (aborted(c)) return false;
       const unsigned long long now = globaltimer();
@@ -517,13 +523,13 @@ __device__ __forceinline__ uint4 xchg_gather8(const Ctx& c, unsigned seq, int to
                                                       xchg_word(seq, p.world, p.xchg_tokens, p.xchg_cols, r, tok, col));
     uint4 q[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) q[i] = ld_sys_v4(src + i);
+    for (int i = 0; i < 4; ++i) q[i] = ld_sys_words(src + i);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       if (!xchg_arrived(q[i].y, seq) || !xchg_arrived(q[i].w, seq)) {
         const uint2* w2 = reinterpret_cast<const uint2*>(src + i);
         if (!xchg_wait_word(c, w2, seq, r) || !xchg_wait_word(c, w2 + 1, seq, r)) return make_uint4(0, 0, 0, 0);
-        q[i] = ld_sys_v4(src + i);
+        q[i] = ld_sys_words(src + i);
       }
       acc[2 * i] += __uint_as_float(q[i].x);
       acc[2 * i + 1] += __uint_as_float(q[i].z);
@@ -538,10 +544,10 @@ __device__ __forceinline__ float xchg_gather1(const Ctx& c, unsigned seq, int to
 #pragma unroll 1
   for (int r = 0; r < p.world; ++r) {
     const uint2* w = reinterpret_cast<const uint2*>(p.xchg[p.rank]) + xchg_word(seq, p.world, p.xchg_tokens, p.xchg_cols, r, tok, col);
-    uint2 q = ld_sys_v2(w);
+    uint2 q = ld_sys_word(w);
     if (!xchg_arrived(q.y, seq)) {
       if (!xchg_wait_word(c, w, seq, r)) return 0.f;
-      q = ld_sys_v2(w);
+      q = ld_sys_word(w);
     }
     acc += __uint_as_float(q.x);
   }
@@ -558,23 +564,22 @@ __device__ __forceinline__ unsigned xchg_next(const Ctx& c) { return xchg_seq(c.
 // round trip, it simply polls the words it is going to read anyway.  Eight columns are four words,
 // read as two 16-byte loads.
 // ------------------------------------------------------------------------------------
-__device__ __forceinline__ uint4 ld_gpu_v4(const uint4* p) {
-  uint4 v;
-  asm volatile("ld.relaxed.gpu.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
-  return v;
+__device__ __forceinline__ uint4 ld_gpu_words(const uint4* p) {
+  unsigned long long a, b;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
+  return split_words(a, b);
 }
-__device__ __forceinline__ uint2 ld_gpu_v2(const uint2* p) {
-  uint2 v;
-  asm volatile("ld.relaxed.gpu.global.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
-  return v;
+__device__ __forceinline__ uint2 ld_gpu_word(const uint2* p) {
+  unsigned long long a;
+  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(a) : "l"(p) : "memory");
+  return make_uint2((uint32_t)a, (uint32_t)(a >> 32));
 }
-__device__ __forceinline__ void st_gpu_v2(uint2* p, uint32_t a, uint32_t b) {
-  asm volatile("st.relaxed.gpu.global.v2.u32 [%0], {%1,%2};" ::"l"(p), "r"(a), "r"(b) : "memory");
+__device__ __forceinline__ void st_gpu_word(uint2* p, uint32_t value, uint32_t tag) {
+  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(join_word(value, tag)) : "memory");
 }
 // two words at once: a vector of 64-bit scalars, each of them single-copy atomic
 __device__ __forceinline__ void st_gpu_words(uint4* p, uint32_t a, uint32_t b, uint32_t tag) {
-  const unsigned long long x = (unsigned long long)tag << 32 | a, y = (unsigned long long)tag << 32 | b;
-  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1,%2};" ::"l"(p), "l"(x), "l"(y) : "memory");
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1,%2};" ::"l"(p), "l"(join_word(a, tag)), "l"(join_word(b, tag)) : "memory");
 }
 __device__ __forceinline__ bool ll_ok(const uint4& a, const uint4& b, unsigned tag) {
   return a.y == tag && a.w == tag && b.y == tag && b.w == tag;
@@ -612,8 +617,8 @@ __device__ __forceinline__ void ll_take(const Ctx& c, const uint4* src, const in
 #pragma unroll
     for (int i = 0; i < N; ++i)
       if (!ll_ok(a[i], b[i], tag)) {
-        a[i] = ld_gpu_v4(src + 2 * at[i]);
-        b[i] = ld_gpu_v4(src + 2 * at[i] + 1);
+        a[i] = ld_gpu_words(src + 2 * at[i]);
+        b[i] = ld_gpu_words(src + 2 * at[i] + 1);
       }
     bool here = true;
 #pragma unroll
@@ -628,7 +633,7 @@ __device__ __forceinline__ float ll_gather1(const Ctx& c, const uint2* row, int 
   const uint2* w = row + (col >> 1);
   PollLimit limit;
   uint2 q;
-  do q = ld_gpu_v2(w);
+  do q = ld_gpu_word(w);
   while (q.y != tag && !limit.expired(c, tag, q.y));
   return (col & 1) ? bf_hi(q.x) : bf_lo(q.x);
 }
@@ -659,7 +664,7 @@ __device__ __forceinline__ void xchg_reduce_slice(Ctx& c, const OpDesc& op, int 
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
       if (r < p.world)
-        q[r] = ld_sys_v4(reinterpret_cast<const uint4*>(reinterpret_cast<const uint2*>(p.xchg[p.rank]) +
+        q[r] = ld_sys_words(reinterpret_cast<const uint4*>(reinterpret_cast<const uint2*>(p.xchg[p.rank]) +
                                                         xchg_word(seq, p.world, p.xchg_tokens, p.xchg_cols, r, tok, 2 * pr)));
     }
     float a0 = 0.f, a1 = 0.f;
@@ -669,13 +674,13 @@ __device__ __forceinline__ void xchg_reduce_slice(Ctx& c, const OpDesc& op, int 
         if (!xchg_arrived(q[r].y, seq) || !xchg_arrived(q[r].w, seq)) {
           const uint2* w2 = reinterpret_cast<const uint2*>(p.xchg[p.rank]) + xchg_word(seq, p.world, p.xchg_tokens, p.xchg_cols, r, tok, 2 * pr);
           if (!xchg_wait_word(c, w2, seq, r) || !xchg_wait_word(c, w2 + 1, seq, r)) return;
-          q[r] = ld_sys_v4(reinterpret_cast<const uint4*>(w2));
+          q[r] = ld_sys_words(reinterpret_cast<const uint4*>(w2));
         }
         a0 += __uint_as_float(q[r].x);
         a1 += __uint_as_float(q[r].z);
       }
     }
-    st_gpu_v2(dst + (size_t)tok * (size_t)(op.ld_in >> 1) + pr, pack2(a0, a1), tag);
+    st_gpu_word(dst + (size_t)tok * (size_t)(op.ld_in >> 1) + pr, pack2(a0, a1), tag);
   }
 }
 #endif
@@ -774,7 +779,7 @@ __device__ __forceinline__ void stage_row_regs(Ctx& c, const uint4* src, uint4* 
           src4[i] = reinterpret_cast<const uint4*>(reinterpret_cast<const uint2*>(p.xchg[p.rank]) +
                                                    xchg_word(seq, p.world, p.xchg_tokens, p.xchg_cols, r, tok, v * 8));
 #pragma unroll
-          for (int k = 0; k < 4; ++k) q[i][k] = (valid && v0 + vstep * i < kvec) ? ld_sys_v4(src4[i] + k) : make_uint4(0u, seq, 0u, seq);
+          for (int k = 0; k < 4; ++k) q[i][k] = (valid && v0 + vstep * i < kvec) ? ld_sys_words(src4[i] + k) : make_uint4(0u, seq, 0u, seq);
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
@@ -783,7 +788,7 @@ __device__ __forceinline__ void stage_row_regs(Ctx& c, const uint4* src, uint4* 
           for (int k = 0; k < 4; ++k) {
             if (!xchg_arrived(q[i][k].y, seq) || !xchg_arrived(q[i][k].w, seq)) {
               const uint2* w2 = reinterpret_cast<const uint2*>(src4[i] + k);
-              if (xchg_wait_word(c, w2, seq, r) && xchg_wait_word(c, w2 + 1, seq, r)) q[i][k] = ld_sys_v4(src4[i] + k);
+              if (xchg_wait_word(c, w2, seq, r) && xchg_wait_word(c, w2 + 1, seq, r)) q[i][k] = ld_sys_words(src4[i] + k);
             }
             acc[i][2 * k] += __uint_as_float(q[i][k].x);
             acc[i][2 * k + 1] += __uint_as_float(q[i][k].z);
@@ -1205,7 +1210,7 @@ __device__ __forceinline__ void linear_pass_rows(Ctx& c, const OpDesc& op, int t
         const uint32_t lo = (uint32_t)__bfloat16_as_ushort(y);
         const uint32_t hi = __shfl_down_sync(0xffffffffu, lo, 1);
         if (mine && !(e_row & 1))
-          st_gpu_v2(reinterpret_cast<uint2*>(op.ll_out) + (size_t)(tok0 + e_tok) * (size_t)(op.ld_out >> 1) + (col >> 1), lo | (hi << 16),
+          st_gpu_word(reinterpret_cast<uint2*>(op.ll_out) + (size_t)(tok0 + e_tok) * (size_t)(op.ld_out >> 1) + (col >> 1), lo | (hi << 16),
                     ll_tag_of(c, c.cur_op));
       }
     } else {
@@ -1221,7 +1226,7 @@ __device__ __forceinline__ void linear_pass_rows(Ctx& c, const OpDesc& op, int t
         const uint32_t lo = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v));
         const uint32_t hi = __shfl_down_sync(0xffffffffu, lo, 1);
         if (e_live && !(e_row & 1))
-          st_gpu_v2(reinterpret_cast<uint2*>(op.ll_out) + (size_t)(tok0 + e_tok) * (size_t)(op.ld_out >> 1) + ((r0 + e_row) >> 1),
+          st_gpu_word(reinterpret_cast<uint2*>(op.ll_out) + (size_t)(tok0 + e_tok) * (size_t)(op.ld_out >> 1) + ((r0 + e_row) >> 1),
                     lo | (hi << 16), ll_tag_of(c, c.cur_op));
       }
       if (op.flags & F_ARGMAX) {
@@ -1395,8 +1400,8 @@ __device__ __forceinline__ void attn_merge(Ctx& c, const float* base, __nv_bfloa
       const uint32_t lo = (uint32_t)__bfloat16_as_ushort(y), lo2 = (uint32_t)__bfloat16_as_ushort(y2);
       const uint32_t hi = __shfl_down_sync(0xffffffffu, lo, 1), hi2 = __shfl_down_sync(0xffffffffu, lo2, 1);
       if (!(e & 1)) {
-        st_gpu_v2(ll_out + (e >> 1), lo | (hi << 16), tag);
-        if (two) st_gpu_v2(ll_out + (e2 >> 1), lo2 | (hi2 << 16), tag);
+        st_gpu_word(ll_out + (e >> 1), lo | (hi << 16), tag);
+        if (two) st_gpu_word(ll_out + (e2 >> 1), lo2 | (hi2 << 16), tag);
       }
     }
   }
@@ -1437,9 +1442,9 @@ __device__ __forceinline__ void attn_merge_ll(Ctx& c, const uint2* base, __nv_bf
 #pragma unroll
           for (int u = 0; u < kBatch; ++u) {
             const size_t off = (size_t)(c0 + u) * part_stride;
-            if (qv[u].y != tag) qv[u] = ld_gpu_v2(pv + off);
-            if (qm[u].y != tag) qm[u] = ld_gpu_v2(pm + off);
-            if (ql[u].y != tag) ql[u] = ld_gpu_v2(pm + off + qpk);
+            if (qv[u].y != tag) qv[u] = ld_gpu_word(pv + off);
+            if (qm[u].y != tag) qm[u] = ld_gpu_word(pm + off);
+            if (ql[u].y != tag) ql[u] = ld_gpu_word(pm + off + qpk);
           }
 #pragma unroll
           for (int u = 0; u < kBatch; ++u) here = here && qv[u].y == tag && qm[u].y == tag && ql[u].y == tag;
@@ -1472,7 +1477,7 @@ __device__ __forceinline__ void attn_merge_ll(Ctx& c, const uint2* base, __nv_bf
     if (act) out[e] = yb;
     const uint32_t lo = (uint32_t)__bfloat16_as_ushort(yb);
     const uint32_t hi = __shfl_down_sync(0xffffffffu, lo, 1);
-    if (act && ll_out != nullptr && !(e & 1)) st_gpu_v2(ll_out + (e >> 1), lo | (hi << 16), tag);
+    if (act && ll_out != nullptr && !(e & 1)) st_gpu_word(ll_out + (e >> 1), lo | (hi << 16), tag);
   }
 }
 
@@ -1734,8 +1739,8 @@ __device__ __forceinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
         st_gpu_words(dst, __float_as_uint(O.x), __float_as_uint(O.y), tag);
         st_gpu_words(dst + 1, __float_as_uint(O.z), __float_as_uint(O.w), tag);
         if (d == 0) {
-          st_gpu_v2(partw + qpk * kHeadDim + r, __float_as_uint(M), tag);
-          st_gpu_v2(partw + qpk * kHeadDim + qpk + r, __float_as_uint(L), tag);
+          st_gpu_word(partw + qpk * kHeadDim + r, __float_as_uint(M), tag);
+          st_gpu_word(partw + qpk * kHeadDim + qpk + r, __float_as_uint(L), tag);
         }
       } else {
         *reinterpret_cast<float2*>(part + r * kHeadDim + d) = make_float2(O.x, O.y);
@@ -1959,8 +1964,8 @@ __device__ __forceinline__ void argmax_store(Ctx& c, const OpDesc& op, int tok, 
     const size_t mine = (size_t)p.xchg_amax_word + ((size_t)p.rank * p.xchg_tokens + tok) * 2;
     for (int r = 0; r < p.world; ++r) {
       uint2* w = reinterpret_cast<uint2*>(p.xchg[r]) + mine;
-      st_sys_v2(w, __float_as_uint(b.v), seq);
-      st_sys_v2(w + 1, (uint32_t)b.i, seq);
+      st_sys_word(w, __float_as_uint(b.v), seq);
+      st_sys_word(w + 1, (uint32_t)b.i, seq);
     }
     ArgBest g;
     g.v = -INFINITY;
@@ -1969,8 +1974,8 @@ __device__ __forceinline__ void argmax_store(Ctx& c, const OpDesc& op, int tok, 
       const uint2* w = reinterpret_cast<const uint2*>(p.xchg[p.rank]) + (size_t)p.xchg_amax_word + ((size_t)r * p.xchg_tokens + tok) * 2;
       if (!xchg_wait_word(c, w, seq, r) || !xchg_wait_word(c, w + 1, seq, r)) break;
       ArgBest x;
-      x.v = __uint_as_float(ld_sys_v2(w).x);
-      x.i = (int)ld_sys_v2(w + 1).x;
+      x.v = __uint_as_float(ld_sys_word(w).x);
+      x.i = (int)ld_sys_word(w + 1).x;
       g = arg_better(g, x);
     }
     b = g;
@@ -2056,7 +2061,7 @@ __device__ __forceinline__ void moe_route_token(Ctx& c, const __nv_bfloat16* log
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         q[j] = make_uint2(0u, tag);
-        if (c.lane + 32 * j < E) q[j] = ld_gpu_v2(words + (c.lane >> 1) + 16 * j);
+        if (c.lane + 32 * j < E) q[j] = ld_gpu_word(words + (c.lane >> 1) + 16 * j);
         here = here && q[j].y == tag;
       }
       if (here) break;
@@ -2341,7 +2346,7 @@ __device__ __forceinline__ void op_moe_linear(Ctx& c, const OpDesc& op, int T) {
           if (e_row < h2) {
             reinterpret_cast<__nv_bfloat16*>(op.out2)[(size_t)pr * op.ld_out2 + col] = y;
             if ((op.flags & F_LL_OUT) && !(e_row & 1))  // (columns come in groups of four: the pair sits in two neighbouring lanes)
-              st_gpu_v2(reinterpret_cast<uint2*>(op.ll_out) + (size_t)pr * (size_t)(op.ld_out2 >> 1) + (col >> 1), lo | (hi << 16),
+              st_gpu_word(reinterpret_cast<uint2*>(op.ll_out) + (size_t)pr * (size_t)(op.ld_out2 >> 1) + (col >> 1), lo | (hi << 16),
                         ll_tag_of(c, c.cur_op));
           }
         } else if (e_row < R) {
@@ -2464,7 +2469,7 @@ __device__ __forceinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, in
           const uint32_t lo = (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(v));
           const uint32_t hi = __shfl_down_sync(0xffffffffu, lo, 1);
           if (e_row < R && !(e_row & 1))
-            st_gpu_v2(reinterpret_cast<uint2*>(op.ll_out) + (size_t)t * (size_t)(op.ld_out >> 1) + ((r0 + e_row) >> 1), lo | (hi << 16),
+            st_gpu_word(reinterpret_cast<uint2*>(op.ll_out) + (size_t)t * (size_t)(op.ld_out >> 1) + ((r0 + e_row) >> 1), lo | (hi << 16),
                       ll_tag_of(c, c.cur_op));
         }
       }
@@ -2544,7 +2549,7 @@ __device__ __forceinline__ void op_allreduce(Ctx& c, const OpDesc& op, int T) {
     for (int r = 0; r < world; ++r) {
       uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<uint2*>(p.xchg[r]) + w);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) st_sys_v4(dst + i, __float_as_uint(f[2 * i]), seq, __float_as_uint(f[2 * i + 1]), seq);
+      for (int i = 0; i < 4; ++i) st_sys_words(dst + i, __float_as_uint(f[2 * i]), __float_as_uint(f[2 * i + 1]), seq);
     }
     reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(op.out) + (size_t)row * op.ld_out)[v] = xchg_gather8(c, seq, row, v * 8);
   }

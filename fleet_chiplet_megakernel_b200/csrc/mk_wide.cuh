@@ -647,7 +647,7 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
                 for (int u = 0; u < PB; ++u)
 #pragma unroll
                   for (int i = 0; i < NC / 2; ++i)
-                    if (w[u][i].y != tag || w[u][i].w != tag) w[u][i] = ld_gpu_v4(src0 + (size_t)(cta + u) * slot_vec + (size_t)i * kTileRows);
+                    if (w[u][i].y != tag || w[u][i].w != tag) w[u][i] = ld_gpu_words(src0 + (size_t)(cta + u) * slot_vec + (size_t)i * kTileRows);
                 bool here = true;
 #pragma unroll
                 for (int u = 0; u < PB; ++u)

@@ -464,3 +464,14 @@ def test_norms_folded_into_activation_boxes(tokens, numerics, form, folded):
     assert ops == (4 if form == "second reader" else 3) - int(folded), text.value.decode()
     assert ("rmsnorm in the activation boxes" in text.value.decode()) == folded
     k.finalize()
+
+
+def test_tagged_words_move_as_64_bit_scalars():
+    """A word that carries the awaited number carries its value: the two halves travel in one 64-bit scalar, which is single-copy
+    atomic.  The elements of a vector of 32-bit scalars may be of different ages."""
+    csrc = os.path.join(os.path.dirname(mk.__file__), "csrc")
+    found = set()
+    for name in ("mk_kernel.cu", "mk_wide.cuh"):
+        with open(os.path.join(csrc, name)) as f:
+            found |= set(re.findall(r"\b(?:ld|st)\.relaxed\.(?:gpu|sys)\.global\.[\w.]+", f.read()))
+    assert found and all(re.fullmatch(r"(ld|st)\.relaxed\.(gpu|sys)\.global\.(v2\.)?b64", form) for form in found), found
