@@ -53,6 +53,7 @@ SIGNATURES = {
     "mk_debug_exchange_sequence": (C.c_int, [C.c_uint32, C.c_uint32, C.c_int, C.c_int, C.c_int, C.POINTER(C.c_uint32),
                                              C.POINTER(C.c_int64), C.POINTER(C.c_int)]),
     "mk_debug_describe_wide": (C.c_int, [C.c_void_p, C.c_char_p, C.c_int]),
+    "mk_debug_page_entries": (C.c_int, [C.c_int, C.c_int]),
     "mk_debug_wide_ring": (C.c_int, [C.c_int, C.c_int, C.POINTER(C.c_int)]),
     "mk_barrier_target_reached": (C.c_int, [C.c_uint32, C.c_uint32, C.c_uint32]),
     "mk_tensor_ptr": (C.c_void_p, [C.c_void_p, C.c_int]),

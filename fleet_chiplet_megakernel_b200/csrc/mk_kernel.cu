@@ -3208,7 +3208,9 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
                 if (p.sched[4] != 0) bookkeep_finish(c.p);
                 p.sched[4] = 0;
                 if (p.max_iters == 0 || git <= p.max_iters) {
-                  n = bookkeep_prepare(c.p, reinterpret_cast<int*>(c.smem + p.x_off), iter);
+                  // (the page table goes through the weight ring: no stage is under way between two iterations)
+                  n = bookkeep_prepare(c.p, reinterpret_cast<int*>(c.smem), iter);
+                  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // TMA writes there next
                   if (n > 0) p.sched[4] = 1;
                 }
               }

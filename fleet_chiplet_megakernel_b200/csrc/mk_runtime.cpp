@@ -56,6 +56,14 @@ int wide_stages(int tokens, int x_bytes) {
   return fast >= 2 ? fast : std::min(2, (kMaxSmem - kWideFixed - x_bytes) / wide_stage_bytes(tokens));
 }
 
+// Row-owner path: five stages where they fit beside the resident rows.  12 layers of 8B width, us per step with 4 and 5 stages:
+// one request 1119 and 1109; two requests, 3, 4 and 5: 1238, 1172, 1166.
+constexpr int kRowsFixed = 1024 /*alignment slack*/ + kRowsSumsBytes + kRedBytes + 1024 /*barriers and flags, op descriptors*/;
+int rows_stages(int x_bytes) { return std::min((kMaxSmem - kRowsFixed - x_bytes) / mk::kStageBytes, 5); }
+// Page numbers that the scheduler can keep in shared memory while it rewrites the page table: between two iterations the weight
+// ring in front of the x region is empty, so the table has both (MoE programs keep expert ids in the last 512 bytes).
+int page_entries(int ring_bytes, int x_bytes, bool moe) { return (ring_bytes + x_bytes - (moe ? 512 : 0)) / 4; }
+
 size_t dtype_size(int dt) {
   switch (dt) {
     case MK_BF16: case MK_F16: return 2;
@@ -1223,6 +1231,12 @@ int mk_debug_wide_ring(int tokens, int x_bytes, int* smem_out) {
   return stages;
 }
 
+int mk_debug_page_entries(int tokens, int x_bytes) {
+  if (tokens < 1 || tokens > 128 || x_bytes < 0) return MK_E_INVALID;
+  const bool rows = tokens <= 2;
+  return page_entries(rows ? rows_stages(x_bytes) * mk::kStageBytes : wide_stages(tokens, x_bytes) * wide_stage_bytes(tokens), x_bytes, false);
+}
+
 int mk_barrier_target_reached(uint32_t counter, uint32_t epoch, uint32_t arrivals_per_barrier) {
   // the comparison the device's grid barrier makes (modulo 2^32)
   return (int)(counter - epoch * arrivals_per_barrier) >= 0 ? 1 : 0;
@@ -1320,7 +1334,7 @@ static int compile_program(mk_handle* h, bool first) {
   const int sums_bytes = rows_mode ? kRowsSumsBytes : 0;
   const int red_bytes = rows_mode ? kRedBytes : mk::kWideRedBytes;
   const int bar_bytes = rows_mode ? 1024 : 2048;  // barriers and flags, then the two op descriptors
-  const int fixed0 = rows_mode ? 1024 /*alignment slack*/ + sums_bytes + red_bytes + bar_bytes : kWideFixed;
+  const int fixed0 = rows_mode ? kRowsFixed : kWideFixed;
   const int want_stages = cfg.max_stages > 0 ? std::min(cfg.max_stages, 16) : 4;
   // (row-owner mode prefers two resident token rows and three stages to one row and four)
   int x_budget = kRowsXBudget;
@@ -1371,24 +1385,13 @@ static int compile_program(mk_handle* h, bool first) {
   }
   if (has_moe) x_bytes += 512;  // the expert ids of the pairs, for the producer (routing folded into the expert linear)
   x_bytes = (x_bytes + 1023) / 1024 * 1024;
-  const int fixed = fixed0 + x_bytes;
-  const int s_max = (kMaxSmem - fixed) / stage_bytes;
   int stages;
-  if (cfg.max_stages > 0) stages = std::min(s_max, want_stages);  // an explicit request wins
-  // Row-owner path: five stages where they fit beside the resident rows.  12 layers of 8B width, us per step with 4 and 5
-  // stages: one request 1119 and 1109; two requests, 3, 4 and 5: 1238, 1172, 1166.
-  else if (rows_mode) stages = std::min(s_max, 5);
-  else stages = wide_stages(nt, x_bytes);
+  if (cfg.max_stages > 0) stages = std::min((kMaxSmem - fixed0 - x_bytes) / stage_bytes, want_stages);  // an explicit request wins
+  else stages = rows_mode ? rows_stages(x_bytes) : wide_stages(nt, x_bytes);
   if (stages < 2) return h->fail(MK_E_UNSUPPORTED, "activations need %d bytes of shared memory: no room for the weight ring", x_bytes);
-  // The page table is rewritten through shared memory as far as it fits into what the ring leaves of the carve-out
-  // (a larger pool costs no stage and no L1), through global memory beyond.
-  const int used = fixed + stages * stage_bytes;
-  const int spare = (used <= kFastSmem ? kFastSmem : kMaxSmem) - used;
-  const int64_t table = (int64_t)cfg.max_num_pages * 4;
-  if (table > x_bytes) x_bytes += (int)std::min<int64_t>(spare / 1024 * 1024, (table - x_bytes + 1023) / 1024 * 1024);
   mk::KParams& kp = h->kp;
   memset(&kp, 0, sizeof(kp));
-  kp.page_entries = (x_bytes - (has_moe ? 512 : 0)) / 4;  // (the expert ids keep their place at the end)
+  kp.page_entries = page_entries(stages * stage_bytes, x_bytes, has_moe);
   kp.num_stages = stages;
   kp.stage_bytes = stage_bytes;
   kp.x_rows = x_rows;

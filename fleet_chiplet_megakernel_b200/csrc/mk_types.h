@@ -188,7 +188,7 @@ struct KParams {
   int* request_ids;   // [max_reqs]
   int* page_queue;    // ring of free pages [max_pages]
   int* page_scratch;  // [max_pages] copy of the page table while it is rewritten, where it is longer than ...
-  int page_entries;   // ... the entries that the x region of shared memory holds
+  int page_entries;   // ... the entries that the weight ring and the x region of shared memory hold
   int* sched;         // [0]=page head [1]=page tail [2]=next request id [3]=iterations done
                       // [4]=outputs of the last iteration not appended yet
                       // [5]=tokens of an iteration that is prepared but was handed to the other program

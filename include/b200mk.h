@@ -168,6 +168,9 @@ int mk_debug_describe_wide(mk_handle* h, char* buf, int n);
 /* Weight stages of the wide path's ring for iterations of up to `tokens` tokens, with x_bytes of activation scratch, and
  * the shared memory of a CTA (used by the host-side tests). */
 int mk_debug_wide_ring(int tokens, int x_bytes, int* smem_out);
+/* Entries of the page table that the scheduler rewrites through shared memory, for iterations of up to `tokens` tokens with
+ * x_bytes of activation scratch (used by the host-side tests). */
+int mk_debug_page_entries(int tokens, int x_bytes);
 int mk_barrier_target_reached(uint32_t counter, uint32_t epoch, uint32_t arrivals_per_barrier);
 void* mk_tensor_ptr(mk_handle* h, int tensor_id);      /* device address after compile (runtime-owned ones too) */
 int mk_tensor_read(mk_handle* h, int tensor_id, void* host_buf, int64_t bytes); /* copy a tensor's bytes to the host */

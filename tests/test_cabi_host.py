@@ -394,6 +394,12 @@ def test_wide_ring_leaves_the_l1_its_share(native_lib, tokens):
     assert stages >= 2 and smem.value <= 227 * 1024
 
 
+@pytest.mark.parametrize("tokens", [1, 2, 3, 16, 17, 32, 33, 64, 65, 128])
+def test_page_tables_are_rewritten_through_shared_memory(native_lib, tokens):
+    """64 requests of 8192 tokens on 16-position pages are 32768 page numbers; deeper or shallower rings leave room for as many."""
+    assert native_lib.mk_debug_page_entries(tokens, 8192 + 8 * 8 * 8) >= 32768
+
+
 @pytest.mark.parametrize("widths,barrier", [((512, 512), True), ((512, 1024), False)])
 def test_norm_rows_are_not_overwritten_while_the_linear_before_reads_them(widths, barrier):
     """Two fused norm linears with an allreduce between them, on the wide path: each norm becomes an op that stores its rows,

@@ -539,3 +539,22 @@ def test_large_page_pools(pool, budget):
         dec.finalize()
     assert all(torch.equal(a, b) for a, b in zip(got[0][0], got[1][0]))
     assert torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("requests,length,budget", [(64, 620, 128), (5, 8000, 64)])
+def test_page_tables_wider_than_the_ring(requests, length, budget):
+    """Tables in use that do not fit into shared memory where the weight ring was, either (some 39000 entries): rewritten through
+    global memory, with the results of 64-position pages, bit for bit."""
+    geom, n_new = O.TINY, 6
+    w = _cuda(O.make_weights(geom, 0, norm_jitter=0.25))
+    prompts = [O.make_prompt(geom, length - n_new, r) for r in range(requests)]
+    got = []
+    for page, pages in ((1, requests * length + 64), (64, None)):
+        dec = mk.Qwen3Decoder(_geom(geom), w, max_seq_length=length, max_requests=requests, page_size=page, max_num_pages=pages,
+                              max_num_batched_tokens=budget, numerics="mpk", keep_logits=True)
+        dec.set_prompts(prompts)
+        dec.run()
+        got.append(([dec.generated(r).cpu() for r in range(requests)], dec.logits[:requests].cpu()))
+        dec.finalize()
+    assert all(torch.equal(a, b) for a, b in zip(got[0][0], got[1][0]))
+    assert torch.equal(got[0][1], got[1][1])
