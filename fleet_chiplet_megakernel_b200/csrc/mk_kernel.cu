@@ -467,25 +467,28 @@ __device__ __forceinline__ float block_sum(Ctx& c, float v) {
 // every peer, which those peers push after their last read of s.
 // Words travel as what they are, 64-bit scalars {value, number}: only those are single-copy atomic.  (Of a vector of 32-bit scalars
 // the memory model lets the number be newer than the value beside it.)
-__device__ __forceinline__ uint4 split_words(unsigned long long a, unsigned long long b) {
-  return make_uint4((uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32));
-}
-__device__ __forceinline__ unsigned long long join_word(uint32_t value, uint32_t number) { return (unsigned long long)number << 32 | value; }
 __device__ __forceinline__ uint4 ld_sys_words(const uint4* p) {
-  unsigned long long a, b;
-  asm volatile("ld.relaxed.sys.global.v2.b64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
-  return split_words(a, b);
+  uint4 v;
+  asm volatile(
+      "{\n\t.reg .b64 a, b;\n\tld.relaxed.sys.global.v2.b64 {a,b}, [%4];\n\tmov.b64 {%0,%1}, a;\n\tmov.b64 {%2,%3}, b;\n\t}"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p)
+      : "memory");
+  return v;
 }
 __device__ __forceinline__ uint2 ld_sys_word(const uint2* p) {
-  unsigned long long a;
-  asm volatile("ld.relaxed.sys.global.b64 %0, [%1];" : "=l"(a) : "l"(p) : "memory");
-  return make_uint2((uint32_t)a, (uint32_t)(a >> 32));
+  uint2 v;
+  asm volatile("{\n\t.reg .b64 a;\n\tld.relaxed.sys.global.b64 a, [%2];\n\tmov.b64 {%0,%1}, a;\n\t}" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  return v;
 }
 __device__ __forceinline__ void st_sys_word(uint2* p, uint32_t value, uint32_t number) {
-  asm volatile("st.relaxed.sys.global.b64 [%0], %1;" ::"l"(p), "l"(join_word(value, number)) : "memory");
+  asm volatile("{\n\t.reg .b64 a;\n\tmov.b64 a, {%1,%2};\n\tst.relaxed.sys.global.b64 [%0], a;\n\t}" ::"l"(p), "r"(value), "r"(number) : "memory");
 }
+// two words at once, of the same number
 __device__ __forceinline__ void st_sys_words(uint4* p, uint32_t a, uint32_t b, uint32_t number) {
-  asm volatile("st.relaxed.sys.global.v2.b64 [%0], {%1,%2};" ::"l"(p), "l"(join_word(a, number)), "l"(join_word(b, number)) : "memory");
+  asm volatile(
+      "{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%1,%3};\n\tmov.b64 b, {%2,%3};\n\tst.relaxed.sys.global.v2.b64 [%0], {a,b};\n\t}" ::"l"(p), "r"(a), "r"(b), "r"(number)
+      : "memory");
 }
 // one value of exchange `seq` into every rank's region
 __device__ __forceinline__ void xchg_push1(const KParams& p, unsigned seq, int tok, int col, float v) {
@@ -565,21 +568,27 @@ __device__ __forceinline__ unsigned xchg_next(const Ctx& c) { return xchg_seq(c.
 // read as two 16-byte loads.
 // ------------------------------------------------------------------------------------
 __device__ __forceinline__ uint4 ld_gpu_words(const uint4* p) {
-  unsigned long long a, b;
-  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0,%1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
-  return split_words(a, b);
+  uint4 v;
+  asm volatile(
+      "{\n\t.reg .b64 a, b;\n\tld.relaxed.gpu.global.v2.b64 {a,b}, [%4];\n\tmov.b64 {%0,%1}, a;\n\tmov.b64 {%2,%3}, b;\n\t}"
+      : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+      : "l"(p)
+      : "memory");
+  return v;
 }
 __device__ __forceinline__ uint2 ld_gpu_word(const uint2* p) {
-  unsigned long long a;
-  asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(a) : "l"(p) : "memory");
-  return make_uint2((uint32_t)a, (uint32_t)(a >> 32));
+  uint2 v;
+  asm volatile("{\n\t.reg .b64 a;\n\tld.relaxed.gpu.global.b64 a, [%2];\n\tmov.b64 {%0,%1}, a;\n\t}" : "=r"(v.x), "=r"(v.y) : "l"(p) : "memory");
+  return v;
 }
 __device__ __forceinline__ void st_gpu_word(uint2* p, uint32_t value, uint32_t tag) {
-  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(join_word(value, tag)) : "memory");
+  asm volatile("{\n\t.reg .b64 a;\n\tmov.b64 a, {%1,%2};\n\tst.relaxed.gpu.global.b64 [%0], a;\n\t}" ::"l"(p), "r"(value), "r"(tag) : "memory");
 }
-// two words at once: a vector of 64-bit scalars, each of them single-copy atomic
+// two words at once, of the same number
 __device__ __forceinline__ void st_gpu_words(uint4* p, uint32_t a, uint32_t b, uint32_t tag) {
-  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1,%2};" ::"l"(p), "l"(join_word(a, tag)), "l"(join_word(b, tag)) : "memory");
+  asm volatile(
+      "{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%1,%3};\n\tmov.b64 b, {%2,%3};\n\tst.relaxed.gpu.global.v2.b64 [%0], {a,b};\n\t}" ::"l"(p), "r"(a), "r"(b), "r"(tag)
+      : "memory");
 }
 __device__ __forceinline__ bool ll_ok(const uint4& a, const uint4& b, unsigned tag) {
   return a.y == tag && a.w == tag && b.y == tag && b.w == tag;

@@ -479,5 +479,5 @@ def test_tagged_words_move_as_64_bit_scalars():
     found = set()
     for name in ("mk_kernel.cu", "mk_wide.cuh"):
         with open(os.path.join(csrc, name)) as f:
-            found |= set(re.findall(r"\b(?:ld|st)\.relaxed\.(?:gpu|sys)\.global\.[\w.]+", f.read()))
+            found |= set(re.findall(r"(?:ld|st)\.relaxed\.(?:gpu|sys)\.global\.[\w.]+", f.read()))
     assert found and all(re.fullmatch(r"(ld|st)\.relaxed\.(gpu|sys)\.global\.(v2\.)?b64", form) for form in found), found
