@@ -28,9 +28,10 @@
 // There are no calls in an instance: with one, its per-thread context lives in local memory, calls save
 // and restore registers there, and the register split of the warp roles (kConsumerRegs) has no effect.
 // A block then had 200 to 320 KB of local memory beside an L1 of 28 to 92 KB.  Without calls it has
-// none.  Measured against the same code with out-of-line functions, 12 layers of 8B width, us per step: one
-// request 1283 -> 1109, two 1468 -> 1166, eight of 300 tokens 1707 -> 1477, 32 of 100 1878 -> 1588, 64 of 100 2340 -> 1942;
-// four layers 1024 wide, one request 172 -> 134.
+// none (but for 80 and 8 bytes a thread in the tensor-parallel instances for one or two and for 33 to 128 tokens).  Measured
+// against the same code with out-of-line functions, 12 layers of 8B width, us per step: one request 1283 -> 1109, two
+// 1468 -> 1166, eight of 300 tokens 1707 -> 1477, 32 of 100 1878 -> 1588, 64 of 100 2340 -> 1942; four layers 1024 wide, one
+// request 172 -> 134.
 //   MK_NC             linear path: 0 the row-owner path, 8, 16 or 32 the wide path (token columns of a finishing thread)
 //   MK_VARIANT        inner namespace of this compilation: base | tp | hier | moe
 //   MK_WITH_XCHG      1: linear epilogues can push to / input staging can gather from the ranks' exchange regions
@@ -77,6 +78,9 @@ __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive_n(uint32_t bar, uint32_t n) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(n) : "memory");
+}
 __device__ __forceinline__ void mbar_arrive_expect_tx(uint32_t bar, uint32_t bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
@@ -120,6 +124,16 @@ __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, 256;
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   uint4 v;
   asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ uint2 lds64(uint32_t addr) {
+  uint2 v;
+  asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
   return v;
 }
 __device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
@@ -3021,6 +3035,10 @@ __device__ __forceinline__ void producer_loop(Ctx& c) {
   fl[1] = (int)issued;
 }
 
+// Arrivals that complete a stage's activation boxes: the 32 lanes of the norm warp where an instance has one (a box that needs no
+// norm is arrived at 32 times by its producer), else the producer's.
+constexpr uint32_t kBoxArrivals = MK_NC != 0 && 2 * MK_NC <= kNormBoxRows ? 32 : 1;
+
 // The activation producer of the wide path (warp 9, one lane).  It walks the same tile sequence
 // as the weight producer and adds the input boxes to every stage, but only after the consumers
 // have passed the op's barrier: unlike weights, activations are the previous op's output.
@@ -3062,6 +3080,7 @@ __device__ __forceinline__ void xproducer_loop(Ctx& c) {
         const uint32_t full = (raw ? bar_raw0 : bar_x0) + 8 * s;
         const uint32_t dst = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes + kStageBytes;
         mbar_arrive_expect_tx(full, 2 * x_sub);
+        if (kBoxArrivals > 1 && !raw) mbar_arrive_n(full, kBoxArrivals - 1);
         tma_load_2d(dst, tmap, full, lc.kt * kTileK, 0);
         tma_load_2d(dst + x_sub, tmap, full, lc.kt * kTileK + kBoxK, 0);
         xuse ^= 1u << s;
@@ -3130,7 +3149,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
     for (int s = 0; s < p.num_stages; ++s) {
       mbar_init(c.full_bar(s), 1);
       mbar_init(c.empty_bar(s), PATH == PATH_WIDE ? 1 : kNumConsumerWarps);  // the commit of the stage's MMAs, or every consumer warp
-      mbar_init(c.xfull_bar(s), 1);
+      mbar_init(c.xfull_bar(s), kBoxArrivals);
       if (PATH == PATH_WIDE) mbar_init(c.xraw_bar(s), 1);
     }
     mbar_init(c.done_bar(), 1);

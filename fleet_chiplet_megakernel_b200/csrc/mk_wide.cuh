@@ -269,27 +269,26 @@ __device__ __forceinline__ void wide_row_scales(Ctx& c, const OpDesc& op, int T)
 }
 
 // The norm warp (warp 11).  Lane l holds 16-byte column l & 15 of a stage's two boxes for token rows (l >> 4), + 2, ...
+// All it keeps has to fit the 56 registers of a service warp, or spills sit in the loop that has to keep up with the weight
+// stream (40 bytes of stack and 304 of spill loads a thread with four rows in flight and one lane arriving for the warp).  So two
+// rows are in flight ("mpk", which unpacks them to fp32: one), and every lane arrives by itself: a __syncwarp in front of a
+// single arrival costs registers in every loop around it.
 __device__ __forceinline__ void norm_loop(Ctx& c) {
   const KParams& p = c.p;
   const int S = p.num_stages;
   volatile int* fl = c.flags();
-  const bool torch_num = p.numerics == NUM_TORCH;
-  const uint32_t x_sub = (uint32_t)p.x_rows * 128u;
   const int col = c.lane & 15, row0 = c.lane >> 4;
-  const uint32_t scale = smem_u32(wide_tab(c).scale) + (uint32_t)row0 * (kNormBoxRows / 2) * 4u;
-  const uint32_t sub = kStageBytes + (uint32_t)(col >> 3) * x_sub + (uint32_t)row0 * 128u;
-  uint32_t at[4];  // rows row0, + 2, + 4 and + 6 of eight, in the swizzled box
-#pragma unroll
-  for (int u = 0; u < 4; ++u) at[u] = (uint32_t)(2 * u) * 128u + (uint32_t)(((col & 7) ^ (row0 + 2 * u)) << 4);
+  // rows row0 + 2 u of eight: 256 u bytes further, in the 16-byte column that the swizzle gives them
+  const uint32_t swz = (uint32_t)(((col & 7) ^ row0) << 4);
+  const uint32_t sub = kStageBytes + (uint32_t)(col >> 3) * (uint32_t)p.x_rows * 128u + (uint32_t)row0 * 128u;
   int s = 0;
   unsigned raw_phase = 0;  // per stage: parity of its next raw box
   unsigned lin_seq = 0;
-  bool dead = false;
-  for (int iter = 1; !dead; ++iter) {
+  for (int iter = 1;; ++iter) {
     int go;
-    if (!wait_go(c, fl, iter, go)) break;
+    if (!wait_go(c, fl, iter, go)) return;
     const int T = go & 255;
-    for (int oi = 0; oi < p.num_ops && !dead; ++oi) {
+    for (int oi = 0; oi < p.num_ops; ++oi) {
       const OpDesc& op = p.ops[oi];
       if (op.type != OP_LINEAR) continue;
       lin_seq += 1;
@@ -302,31 +301,32 @@ __device__ __forceinline__ void norm_loop(Ctx& c) {
       }
       // the weights of the first stages: they depend on nobody
       const uint4* nw = reinterpret_cast<const uint4*>(op.norm_w) + col;
-      const int kvec = op.k >> 3, nkt = op.nkt;
-      int kt = (int)(t0 % (unsigned)nkt);
-      auto weights = [&](int k) { return k * 16 + col < kvec ? __ldg(nw + k * 16) : make_uint4(0u, 0u, 0u, 0u); };
-      uint4 w = weights(kt);
-      if (!wait_lin(c, fl, 6, lin_seq)) { dead = true; break; }
+      const int kvec = (op.k >> 3) - col, k_end = op.nkt * 16;  // (16 vectors of eight columns per tile)
+      int kv = (int)(t0 % (unsigned)op.nkt) * 16;
+      auto weights = [&](int k) { return k < kvec ? __ldg(nw + k) : make_uint4(0u, 0u, 0u, 0u); };
+      uint4 w = weights(kv);
+      if (!wait_lin(c, fl, 6, lin_seq)) return;
       __threadfence_block();
-      for (unsigned tile = t0; tile < t1; ++tile) {
-        kt = kt + 1 == nkt ? 0 : kt + 1;
-        const uint4 w_next = weights(kt);
-        if (!mbar_wait(c, c.xraw_bar(s), (raw_phase >> s) & 1u, ST_TIMEOUT_FULL)) { dead = true; break; }
-        uint32_t box = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes + sub, sc = scale;
-        if (torch_num) {
-          // four rows at a time (rows past T, still inside the box, are nobody's): one by one, boxes of 32 rows took longer
-          // than their weight stage (1888 us per step)
+#pragma unroll 1
+      for (int left = (int)(t1 - t0); left > 0; --left) {
+        kv = kv + 16 == k_end ? 0 : kv + 16;
+        const uint4 w_next = weights(kv);
+        if (!mbar_wait(c, c.xraw_bar(s), (raw_phase >> s) & 1u, ST_TIMEOUT_FULL)) return;
+        uint32_t box = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes + sub;
+        uint32_t sc = smem_u32(wide_tab(c).scale) + (uint32_t)row0 * (kNormBoxRows / 2) * 4u;
+        // (rows past T, still inside the box, are nobody's)
+        if (p.numerics == NUM_TORCH) {
 #pragma unroll 1
           for (int t = 0; t < T; t += 8) {
-            uint4 x[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) x[u] = lds128(box + at[u]);
-            const uint4 r = lds128(sc);
-#pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const uint32_t ru = u == 0 ? r.x : (u == 1 ? r.y : (u == 2 ? r.z : r.w));
-              sts128(box + at[u], make_uint4(hmul2_bf16(w.x, hmul2_bf16(x[u].x, ru)), hmul2_bf16(w.y, hmul2_bf16(x[u].y, ru)),
-                                             hmul2_bf16(w.z, hmul2_bf16(x[u].z, ru)), hmul2_bf16(w.w, hmul2_bf16(x[u].w, ru))));
+            for (int u = 0; u < 4; u += 2) {
+              const uint32_t at0 = box + 256u * u + (swz ^ (32u * u)), at1 = box + 256u * (u + 1) + (swz ^ (32u * (u + 1)));
+              const uint4 x0 = lds128(at0), x1 = lds128(at1);
+              const uint2 r = lds64(sc + 4 * u);
+              sts128(at0, make_uint4(hmul2_bf16(w.x, hmul2_bf16(x0.x, r.x)), hmul2_bf16(w.y, hmul2_bf16(x0.y, r.x)),
+                                     hmul2_bf16(w.z, hmul2_bf16(x0.z, r.x)), hmul2_bf16(w.w, hmul2_bf16(x0.w, r.x))));
+              sts128(at1, make_uint4(hmul2_bf16(w.x, hmul2_bf16(x1.x, r.y)), hmul2_bf16(w.y, hmul2_bf16(x1.y, r.y)),
+                                     hmul2_bf16(w.z, hmul2_bf16(x1.z, r.y)), hmul2_bf16(w.w, hmul2_bf16(x1.w, r.y))));
             }
             box += 1024;
             sc += 16;
@@ -334,27 +334,25 @@ __device__ __forceinline__ void norm_loop(Ctx& c) {
         } else {
 #pragma unroll 1
           for (int t = 0; t < T; t += 8) {
-            const uint4 r = lds128(sc);
 #pragma unroll
-            for (int u = 0; u < 4; u += 2) {
-              const uint4 x0 = lds128(box + at[u]), x1 = lds128(box + at[u + 1]);
-              sts128(box + at[u], scale8(x0, w, __uint_as_float(u == 0 ? r.x : r.z), false));
-              sts128(box + at[u + 1], scale8(x1, w, __uint_as_float(u == 0 ? r.y : r.w), false));
-              if (t + 4 >= T) break;  // (rows t + 4 .. t + 7 are nobody's)
+            for (int u = 0; u < 4; ++u) {
+              const uint32_t at = box + 256u * u + (swz ^ (32u * u));
+              const uint4 x = lds128(at);
+              sts128(at, scale8(x, w, __uint_as_float(lds32(sc + 4 * u)), false));
+              if (u == 1 && t + 4 >= T) break;  // (rows t + 4 .. t + 7 are nobody's)
             }
             box += 1024;
             sc += 16;
           }
         }
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads the rows through the async proxy
-        __syncwarp();
-        if (c.lane == 0) mbar_arrive(c.xfull_bar(s));
+        mbar_arrive(c.xfull_bar(s));
         raw_phase ^= 1u << s;
         if (++s == S) s = 0;
         w = w_next;
       }
     }
-    if (p.mode == MODE_ONEPASS) break;
+    if (p.mode == MODE_ONEPASS) return;
   }
 }
 
