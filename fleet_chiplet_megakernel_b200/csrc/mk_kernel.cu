@@ -1755,7 +1755,15 @@ __device__ __forceinline__ void op_attention(Ctx& c, const OpDesc& op, int T) {
       if (a.nch == 1) {
         const float inv = __fdividef(1.0f, L);
         const uint2 y = make_uint2(pack2(O.x * inv, O.y * inv), pack2(O.z * inv, O.w * inv));
-        *reinterpret_cast<uint2*>(out + r * kHeadDim + d) = y;
+        if ((op.ld_out & 3) == 0) {
+          *reinterpret_cast<uint2*>(out + r * kHeadDim + d) = y;
+        } else {  // (rows of any pitch are accepted here)
+          unsigned short* dst = reinterpret_cast<unsigned short*>(out) + r * kHeadDim + d;
+          dst[0] = (unsigned short)y.x;
+          dst[1] = (unsigned short)(y.x >> 16);
+          dst[2] = (unsigned short)y.y;
+          dst[3] = (unsigned short)(y.y >> 16);
+        }
         if (ll_out != nullptr) st_gpu_words(reinterpret_cast<uint4*>(ll_out + ((r * kHeadDim + d) >> 1)), y.x, y.y, tag);
       } else if (ll_part) {
         uint4* dst = reinterpret_cast<uint4*>(partw + r * kHeadDim + d);

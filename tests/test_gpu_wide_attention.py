@@ -19,7 +19,7 @@ def _rand(shape, seed, scale=1.0):
 class Attention:
     """The paged attention layer over `requests`, (cached tokens, new tokens) each, with the pages scattered over the pool."""
 
-    def __init__(self, requests, n_q, n_kv, page, seed=1, edit=None):
+    def __init__(self, requests, n_q, n_kv, page, seed=1, edit=None, pitch=None):
         self.requests, self.n_q, self.n_kv, self.page = requests, n_q, n_kv, page
         R, T = len(requests), sum(n for _, n in requests)
         lens = [c + n for c, n in requests]
@@ -53,15 +53,21 @@ class Attention:
             mode="online_notoken", world_size=1, mpi_rank=0, num_workers=0, num_local_schedulers=0, num_remote_schedulers=0,
             max_seq_length=max(lens) + 1, max_num_batched_requests=R, max_num_batched_tokens=T, max_num_pages=pool, page_size=page,
             meta_tensors=meta, numerics="mpk")
+        out = k.attach_input(self.out, "o") if pitch is None else k.new_tensor(dims=(T, n_q * D), strides=(pitch, 1), name="o")
         k.paged_attention_layer(
             input=k.attach_input(self.qkv.to(dev), "qkv"), k_cache=k.attach_input(self.kcd, "kc"), v_cache=k.attach_input(self.vcd, "vc"),
             q_norm=k.attach_input(self.qn.to(dev), "qn"), k_norm=k.attach_input(self.kn.to(dev), "kn"),
             cos_pos_embed=k.attach_input(self.cos.to(dev), "cos"), sin_pos_embed=k.attach_input(self.sin.to(dev), "sin"),
-            output=k.attach_input(self.out, "o"), grid_dim=(R, n_kv, 1), block_dim=(128, 1, 1))
+            output=out, grid_dim=(R, n_kv, 1), block_dim=(128, 1, 1))
         k.compile()
         for _ in range(2):  # (the second launch finds the chunk counters as the first found them)
             k()
         torch.cuda.synchronize()
+        if pitch is not None:  # (the runtime's own rows, the last one without the columns behind it)
+            host = torch.zeros(T, pitch, dtype=BF)
+            n = ((T - 1) * pitch + n_q * D) * 2
+            assert k._lib.mk_tensor_read(k._h, out.id, host.data_ptr(), n) == 0
+            self.out.copy_(host[:, : n_q * D])
         k.finalize()
 
     def rows(self, r):
@@ -249,3 +255,10 @@ def test_infinite_values_of_one_or_two_tokens(requests, n_q, n_kv):
             assert torch.equal(ref[ref.isinf()], got[ref.isinf()])
             fin = ref.isfinite()
             assert float((got[fin] - ref[fin]).abs().max()) <= 1e-2 * float(ref[fin].abs().max())
+
+
+@pytest.mark.parametrize("more", [1, 2, 4])
+@pytest.mark.parametrize("requests", [[(0, 1), (40, 1)], [(700, 1), (384, 1)], [(30, 2)]])
+def test_output_rows_of_any_pitch_of_two_tokens(requests, more):
+    a, b = Attention(requests, 8, 2, 16, seed=9, pitch=8 * D + more), Attention(requests, 8, 2, 16, seed=9)
+    assert bool(b.out.any()) and torch.equal(a.out, b.out)
