@@ -52,7 +52,7 @@ def check_registers(instances):
     """The warp roles share out kLaunchRegs registers a thread (mk_types.h): an instance with fewer would wait for them for good."""
     with open(os.path.join(CSRC, "mk_types.h")) as f:
         need = int(re.search(r"kLaunchRegs = (\d+)", f.read())[1])
-    few = {name: r["registers"] for name, r in instances.items() if r["registers"] < need}
+    few = {name: r and r["registers"] for name, r in instances.items() if r is None or r["registers"] < need}  # (None: no kernel found)
     if few:
         raise RuntimeError(f"kernel instances with fewer than {need} registers a thread: {few}")
 

@@ -341,8 +341,7 @@ __device__ __forceinline__ void grid_arrive(Ctx& c) {
     else mbar_arrive_cluster(cluster_map(c.cl_arrive_bar(), 0));
   }
 }
-// The waiting half.  Inlined where values loaded ahead of the barrier must stay in registers
-// (a call would spill them, and a spill waits for the load).
+// The waiting half: values loaded ahead of the barrier stay in registers across it.
 __device__ __forceinline__ void grid_wait(Ctx& c) {
   c.arrived = false;
   if (c.tid == 0) {
@@ -399,8 +398,7 @@ __device__ __forceinline__ void grid_arrive(Ctx& c) {
   // arrive with a release reduction: nothing comes back, polling can start at once
   if (c.tid == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(c.p.grid_bar) : "memory");
 }
-// The waiting half.  Inlined where values loaded ahead of the barrier must stay in registers
-// (a call would spill them, and a spill waits for the load).
+// The waiting half: values loaded ahead of the barrier stay in registers across it.
 __device__ __forceinline__ void grid_wait(Ctx& c) {
   c.arrived = false;
   if (c.tid == 0) {
@@ -1361,11 +1359,14 @@ __device__ __forceinline__ F8 head_norm_rope(F8 xin, uint4 wv, uint4 csv, uint4 
 // Tiles of 16 positions that one CTA of the row-owner path takes alone, see op_attention.  Beyond, the chunks' merge (two round
 // trips) costs less than a third round of tiles.  12 layers of 8B width, one request, us per step with 8, 16, 24 and 32:
 // 1120, 1112, 1112, 1112 at 200 positions, 1118, 1118, 1135, 1135 at 300, 1124, 1126, 1125, 1163 at 440.
+// Outputs that are not the bf16 nearest to a float64 softmax, one and two requests behind 0 to 1200 positions, 1 to 8 q heads per
+// kv head, 19.7 million outputs: 0.0286 %; the scalar fp32 form before it 0.0290 %.  Us per layer of 8B width, scalar form and
+// this one: behind 100 positions 18.0 and 11.3, 4000 53 and 22, 30000 334 and 44; two requests behind 8000 153 and 30.
 constexpr int kAttnSoloTiles = 16;
 constexpr int kAttnLensMax = 128;  // requests (the host admits at most 128 batched tokens)
 
-// Merge of a (request, kv head)'s chunks by the CTA that arrived last: kept out of line, only a
-// handful of CTAs per layer ever run it.  One round of loads: every thread fetches, for its
+// Merge of a (request, kv head)'s chunks by the CTA that arrived last: only a handful of CTAs per layer ever run it.
+// One round of loads: every thread fetches, for its
 // output elements, the chunks' values together with their (max, sum) pairs and rescales as it
 // goes, eight chunks at a time (more loads in flight per thread measured slower).
 __device__ __forceinline__ void attn_merge(Ctx& c, const float* base, __nv_bfloat16* out, int nch, int qpk, int part_stride,
@@ -3119,7 +3120,8 @@ template <int PATH, int NC>
 __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_constant__ KParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // The parameters are read from shared memory: behind a reference they are generic loads, and the L1 left beside the
-  // ring (28 KB on the wide path) does not hold them from op to op.  Measured, 12 layers of 8B width: 1.765 -> 1.720 ms
+  // ring (28 KB when this was measured; 92 KB since the wide path keeps to the 164 KB carve-out) does not hold them from op
+  // to op.  Measured, 12 layers of 8B width: 1.765 -> 1.720 ms
   // at 8 requests, 2.364 -> 2.321 at 64; one request 0.3207 -> 0.3166 ms on a small model, no change at 8B width.
   __shared__ __align__(16) uint32_t skp[sizeof(KParams) / 4];
   for (int i = threadIdx.x; i < (int)(sizeof(KParams) / 4); i += blockDim.x) skp[i] = reinterpret_cast<const uint32_t*>(&p)[i];

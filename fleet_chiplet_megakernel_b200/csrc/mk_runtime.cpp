@@ -37,7 +37,8 @@ constexpr int kMaxSmem = 232448 - kParamSmem;  // 227 KB opt-in limit per CTA on
 constexpr int kRedBytes = 2048;    // small scratch (reductions, argmax, sequence lengths)
 constexpr int kFastSmem = 166912 - kParamSmem;  // 164 KB carve-out minus the 1 KB the system reserves per CTA
 constexpr int kRowsSumsBytes = mk::kNumConsumerWarps * mk::kChunkRows * 2 * 4;  // [warp][32 rows][2 tokens] floats
-// token rows a row-owner CTA may keep resident beside three 32 KB weight stages
+// Token rows a row-owner CTA may keep resident: 61,696 bytes, two rows of 15,360 columns.  They leave the ring four stages of
+// the 227 KB of a CTA, and five up to 60,672 bytes (one row in place of two would buy a stage for two passes over the weights).
 constexpr int kRowsXBudget = kFastSmem - 2048 - kRedBytes - kRowsSumsBytes - 3 * mk::kStageBytes;
 constexpr int kAttnMaxChunks = 32;
 constexpr int kGateUpUnit = 4;     // fused gate/up weights are laid out [4 gate | 4 up] per 8-row unit
@@ -45,7 +46,7 @@ constexpr int kMaxStepTimes = 16384;
 
 // The wide path's shared memory.  Ring: stages of 32 KB of weights and two activation boxes of x_rows token rows.  As many
 // stages as leave the CTA within the 164 KB carve-out (4 up to 16 token rows, 3 up to 64, 2 beyond; the attention's scratch
-// is 9 KB for that reason).  12 layers of 8B width, us per step: 8 requests with 3, 4 and 5 stages 1477, 1453, 1454; 32
+// is 9 KB for that reason): what the ring does not take is L1, and another stage brings nothing up to 64 token rows.  12 layers of 8B width, us per step: 8 requests with 3, 4 and 5 stages 1477, 1453, 1454; 32
 // requests 1588, 1562, 1566; 64 requests with 2, 3 and 4 1942, 1823, 1826; 2048 hidden, 8 requests with 3, 4 and 5 910, 893,
 // 904; more only pays from 65 token rows on (2 and 3: 2377 and 2243).
 constexpr int kWideFixed = 1024 /*alignment slack*/ + mk::kWideRedBytes + 2048 /*barriers and flags, op descriptors*/;
@@ -337,16 +338,12 @@ int plan_graph(mk_handle* h) {
       if (valid_tensor(h, op.t[i])) h->tensors[op.t[i]].readers++;
   }
   const bool fuse = cfg.fuse != 0;
-  // RMSNorm is fused into the activation staging of the next linear; batches above 8 tokens
-  // stream their activations by TMA instead, so the norm stays a task of its own there
-  // Fusing the norm into the next linear makes every CTA stage (and normalise) all token
-  // rows in its own shared memory: worth it for one or two tokens, beyond that the rows
-  // would push the CTA past the small shared-memory carve-out and a separate rmsnorm task
-  // with the linear reading activation boxes is faster.
+  // One or two tokens: RMSNorm is fused into the activation staging of the next linear, every CTA stages and normalises the
+  // token rows itself.  Wider programs read activation boxes by TMA: there the norm is planned as an op of its own, and
+  // lower_wide folds it into the boxes of the next linear where that pays.
   const bool fuse_norm = fuse && h->plan_tokens <= 2;
   // One or two tokens: linear layers run row-owner (every CTA owns whole output rows and keeps
-  // the token rows resident in shared memory), provided the widest input still leaves room
-  // for three weight stages inside the small carve-out.
+  // the token rows resident in shared memory), provided the widest input's rows stay within their budget.
   bool rows_mode = h->plan_tokens <= 2;
   for (const RecOp& op : h->nops) {
     if (!rows_mode || !is_linear(op.name)) continue;
@@ -1270,8 +1267,11 @@ static int lower_wide(mk_handle* h) {
   // A norm between two linears is applied to the second one's activation boxes (F_NORM_IN), from sums of squares that the
   // first one's epilogue leaves (F_ROW_SUMS), where nothing else reads the normalised rows and a box is no wider than what
   // one warp normalises in the time a weight stage takes to arrive.  The first norm of a graph (behind the embedding) stays.
-  // "mpk" multiplies in fp32, four times the instructions: up to 8 tokens (12 layers of 8B width: 4 requests 1343 -> 1277 us per
-  // step, 13 requests 1384 -> 1401).
+  // Us per step with a norm op and with the norm in the boxes: 12 layers of 8B width 4 requests 1337 and 1267, 16 1400 and 1336, 32
+  // 1535 and 1484; 12 of 2048 hidden 772 and 710, 825 and 770, 981 and 935; four of 1024 hidden 227 and 214, 238 and 219, 288
+  // and 276.  "mpk" multiplies in fp32, a row at a time: 8 requests 1347 and 1287, 775 and 724, 226 and 213; 32 of 8B width 1519 and
+  // 1889.  Its line at 8 tokens was drawn for a norm warp that spilled (13 requests 1384 and 1401); with the present one 9 to 16
+  // tokens would be faster in the boxes too (12 requests 1372 and 1311, 794 and 735, 227 and 213).
   const int norm_tokens = h->cfg.numerics == mk::NUM_TORCH ? mk::kNormBoxRows : 8;
   for (size_t i = 1; h->cfg.fuse && h->plan_tokens <= norm_tokens && i + 1 < h->plan.size(); ++i) {
     const PlanOp nrm = h->plan[i];
@@ -1336,7 +1336,7 @@ static int compile_program(mk_handle* h, bool first) {
   const int bar_bytes = rows_mode ? 1024 : 2048;  // barriers and flags, then the two op descriptors
   const int fixed0 = rows_mode ? kRowsFixed : kWideFixed;
   const int want_stages = cfg.max_stages > 0 ? std::min(cfg.max_stages, 16) : 4;
-  // (row-owner mode prefers two resident token rows and three stages to one row and four)
+  // (row-owner mode prefers two resident token rows to one row and a stage more)
   int x_budget = kRowsXBudget;
   int x_bytes = 0;
   int max_nblk = 1, n_linear = 0;
@@ -1345,7 +1345,7 @@ static int compile_program(mk_handle* h, bool first) {
     for (const PlanOp& p : h->plan) {
       if (p.type != mk::OP_LINEAR) continue;
       const int kp = (p.k + mk::kRowsStageK - 1) / mk::kRowsStageK * mk::kRowsStageK;
-      if ((x_budget - 16) / ((kp + 8) * 2) < 1) x_budget = kMaxSmem - fixed0 - 3 * stage_bytes;  // a wide fused norm: give up the small carve-out
+      if ((x_budget - 16) / ((kp + 8) * 2) < 1) x_budget = kMaxSmem - fixed0 - 3 * stage_bytes;  // a single row beyond the budget: what three stages leave
     }
   for (PlanOp& p : h->plan) {
     if (p.type == mk::OP_LINEAR) {

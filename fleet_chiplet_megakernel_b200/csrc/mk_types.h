@@ -29,7 +29,9 @@ constexpr int kServiceRegs = 56, kConsumerRegs = 224, kLaunchRegs = 168;
 static_assert(128 * kServiceRegs + kNumConsumers * kConsumerRegs == kNumThreads * kLaunchRegs, "a register split beyond the block's own would wait for good");
 constexpr int kWideRedBytes = 4096;              // scratch of the wide path: reductions and the iteration's token table
 constexpr int kHeadDim = 128;
-constexpr int kNormBoxRows = 32;                 // widest activation box that the norm is applied to in shared memory
+// Widest activation box that the norm is applied to in shared memory: what one warp normalises in the time a weight stage takes
+// to arrive (32 requests, 12 layers of 8B width, with a norm op and in the boxes: 1535 and 1484 us per step; 64 rows not built).
+constexpr int kNormBoxRows = 32;
 // Columns a stand-alone norm stages in shared memory (48 KB).  Wider rows are read twice instead: at 65 tokens and more,
 // where a ring stage is 64 KB, two stages would leave no room for rows of more than 46000 columns.
 constexpr int kNormStagedCols = 24576;

@@ -222,8 +222,8 @@ __device__ __forceinline__ void mma_loop(Ctx& c) {
 // 3.6 us per norm at 8 requests of 8B width.  The linear before it stores the sums of squares of its output
 // rows (F_ROW_SUMS), the consumers turn them into a scale per token at the start of the linear behind it while the first
 // raw boxes are on their way, and warp 11 normalises every box in place: w * bf16(x * r) or x * (r * w), the arithmetic of
-// the norm op.  Measured, us per step of 12 layers: 8B width, 4 requests 1343 -> 1285, 8 of 300 tokens 1442 -> 1381, 32 of
-// 100 1566 -> 1505; 2048 hidden, 8 requests 862 -> 806; four layers of 1024 hidden, 4 requests 202 -> 187.
+// the norm op.  Measured, us per step with a norm op and with the boxes, 12 layers: 8B width, 4 requests 1337 and 1267, 8 1353
+// and 1290, 32 1535 and 1484; 2048 hidden, 8 requests 785 and 725; four layers of 1024 hidden, 4 requests 227 and 214.
 __device__ __forceinline__ uint32_t hmul2_bf16(uint32_t a, uint32_t b) {  // both products rounded to bf16: exact in fp32 before that
   uint32_t d;
   asm("mul.rn.bf16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
@@ -371,8 +371,9 @@ __device__ __forceinline__ void norm_loop(Ctx& c) {
 //    before every launch, and a CTA's slot is written again only behind a grid barrier.
 //  * Beyond, twice the bytes cost more than the round trip: plain float4 of four tokens, [token / 4][row]; every warp
 //    publishes its share with a release of its own and the matching warp of the finisher waits for exactly those.
-// Both measured, us per step of 12 layers of 8B width (words, counters): 8 requests 1433, 1473; 32 1572, 1588; 64 1989,
-// 1942; 100 2488, 2377; 8 requests of 2048 hidden 855, 910; four layers of 1024 hidden, 4 requests 197, 209.
+// Both measured, us per step of 12 layers of 8B width (words, counters): 8 requests 1433, 1473; 20 1446, 1459; 32 1487, 1500; 64
+// 1989, 1942; 100 2488, 2377; 2048 hidden, 8 requests 855, 910; 20 893, 895; 32 942, 943; four layers of 1024 hidden, 4 requests
+// 197, 209; 20 263, 250; 32 276, 262; of 512 hidden, 20 215, 224; 32 226, 222.
 __device__ __forceinline__ uint32_t order_bf16(float v) {  // monotone 16-bit key of a bf16 value; 0 only for NaN
   const uint32_t b = __float_as_uint(v + 0.f) >> 16;       // (-0 counts as +0)
   const uint32_t k = (b & 0x8000u) ? (~b & 0xffffu) : (b | 0x8000u);

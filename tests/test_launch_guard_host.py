@@ -122,6 +122,8 @@ def test_the_build_refuses_an_instance_with_too_few_registers():
     assert _build.resources(PTXAS[PTXAS.index("init_state") - 60:]) is None
     with pytest.raises(RuntimeError, match="mk_kernel_8"):
         _build.check_registers({"mk_kernel_8": r, "mk_kernel_16": dict(r, registers=168)})
+    with pytest.raises(RuntimeError, match="mk_kernel_8"):
+        _build.check_registers({"mk_kernel_8": None})
     _build.check_registers({"mk_kernel_16": dict(r, registers=168)})
 
 
