@@ -26,7 +26,7 @@
 // hierarchical grid barrier (+2.0 %), and each instance holds one linear path.
 //
 // There are no calls in an instance: with one, its per-thread context lives in local memory, calls save
-// and restore registers there, and the register split of the warp roles (kConsumerRegs) has no effect.
+// and restore registers there, and the register split of the warp roles (consumer_regs) has no effect.
 // A block then had 200 to 320 KB of local memory beside an L1 of 28 to 92 KB.  Without calls it has
 // none (but for 80 and 8 bytes a thread in the tensor-parallel instances for one or two and for 33 to 128 tokens).  Measured
 // against the same code with out-of-line functions, 12 layers of 8B width, us per step: one request 1283 -> 1109, two
@@ -97,6 +97,34 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// Asks once, without the suspension of try_wait: for a thread that watches several barriers.
+__device__ __forceinline__ bool mbar_test_wait(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+// The same, suspended for no longer than about `ns`.
+__device__ __forceinline__ bool mbar_try_wait_for(uint32_t bar, uint32_t parity, uint32_t ns) {
+  uint32_t ok;
+  asm volatile(
+      "{\n"
+      ".reg .pred p;\n"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n"
+      "selp.u32 %0, 1, 0, p;\n"
+      "}\n"
+      : "=r"(ok)
+      : "r"(bar), "r"(parity), "r"(ns)
+      : "memory");
+  return ok != 0;
+}
 // 2-D tiled TMA load into this CTA only: box {64 k-elements, 128 rows} at (x = k, y = row).
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, uint32_t bar, int x, int y) {
   asm volatile(
@@ -120,6 +148,30 @@ __device__ __forceinline__ void tma_load_3d_hint(uint32_t dst, const void* tmap,
 __device__ __forceinline__ void tma_prefetch_2d(const void* tmap, int x, int y) {
   asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(tmap), "r"(x), "r"(y) : "memory");
 }
+// One lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t is;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}" : "=r"(is));
+  return is != 0u;
+}
+// ---- tcgen05: descriptors, completion, shared memory -> tensor memory
+__device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr) {
+  // start address >> 4 | leading offset (unused for swizzled K-major) 1 | stride between 8-row
+  // groups 1024 B >> 4 | descriptor version 1 | layout 2 = 128-byte swizzle
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ void umma_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// 128 rows x 64 k-elements of a swizzled stage (16 KB) -> 128 lanes x 32 columns of tensor memory: lane = row, column c = k-elements 2 c
+// and 2 c + 1.
+__device__ __forceinline__ void tmem_put_128x64(uint32_t tmem, uint32_t saddr) {
+  const uint64_t d = umma_smem_desc(saddr);
+#pragma unroll
+  for (int q = 0; q < 4; ++q)  // 16 k-elements = 32 bytes further inside the swizzle span
+    asm volatile("tcgen05.cp.cta_group::1.128x256b [%0], %1;" ::"r"(tmem + 8u * q), "l"(d + (uint64_t)(2 * q)) : "memory");
+}
+__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
 __device__ __forceinline__ uint4 lds128(uint32_t addr) {
   uint4 v;
@@ -176,7 +228,7 @@ struct Ctx {
   unsigned cons_idx;  // weight stages consumed
   bool arrived;       // this CTA has already arrived at the coming grid barrier
   int attn_iter;      // row-owner path: iteration whose attention metadata is cached in shared memory; wide path: head geometry planned
-  uint32_t tmem;      // wide path: base address of the CTA's tensor-memory columns
+  uint32_t tmem;      // base address of the CTA's tensor-memory columns
   unsigned acc_runs;  // wide path: accumulator runs finished
   int tid, lane, warp;
   int iter, cur_op;
@@ -198,28 +250,35 @@ struct Ctx {
     warp = tid >> 5;
     asm volatile("" : "+l"(smem), "+r"(smem_addr), "+r"(tmem));
   }
-  __device__ uint32_t full_bar(int s) const { return smem_addr + p.bar_off + 8 * s; }
-  __device__ uint32_t empty_bar(int s) const { return smem_addr + p.bar_off + 8 * (p.num_stages + s); }
-  __device__ uint32_t xfull_bar(int s) const { return smem_addr + p.bar_off + 8 * (2 * p.num_stages + s); }
-  __device__ volatile int* flags() const { return (volatile int*)(smem + p.bar_off + 24 * p.num_stages); }
-  // behind the flags: the end-of-work mbarrier of the tcgen05 path and the word tcgen05.alloc writes
-  __device__ uint32_t done_bar() const { return smem_addr + p.bar_off + 24 * p.num_stages + 64; }
-  __device__ uint32_t tmem_slot() const { return smem_addr + p.bar_off + 24 * p.num_stages + 72; }
+  // mbarriers, groups of kMaxStages: weights of a stage landed, and its shared memory free again; (wide path) activation boxes ready,
+  // their memory free, the raw rows of a box that still has to be normalised; a slot of the
+  // weight ring's part in tensor memory free again
+  __device__ uint32_t bar_of(int group, int s) const { return smem_addr + p.bar_off + 8 * (group * kMaxStages + s); }
+  __device__ uint32_t full_bar(int s) const { return bar_of(0, s); }
+  __device__ uint32_t empty_bar(int s) const { return bar_of(1, s); }
+  __device__ uint32_t xfull_bar(int s) const { return bar_of(2, s); }
+  __device__ uint32_t xempty_bar(int s) const { return bar_of(3, s); }
+  __device__ uint32_t xraw_bar(int s) const { return bar_of(4, s); }
+  __device__ uint32_t tfree_bar(int s) const { return bar_of(5, s); }
+  // wide path: the activation boxes of stage s, behind the weights of all stages
+  __device__ uint32_t xbox(int s) const { return smem_addr + (uint32_t)(p.num_stages * kStageBytes + s * (p.stage_bytes - kStageBytes)); }
+  __device__ volatile int* flags() const { return (volatile int*)(smem + p.bar_off + kFlagsOff); }
+  // behind the flags: the end-of-work mbarrier of the tcgen05 issuer and the word tcgen05.alloc writes
+  __device__ uint32_t done_bar() const { return smem_addr + p.bar_off + kFlagsOff + 64; }
+  __device__ uint32_t tmem_slot() const { return smem_addr + p.bar_off + kFlagsOff + 72; }
   // hierarchical grid barrier: arrivals of the cluster (used in its first CTA), release from the first CTA, its abort word
-  __device__ uint32_t cl_arrive_bar() const { return smem_addr + p.bar_off + 24 * p.num_stages + 80; }
-  __device__ uint32_t cl_open_bar() const { return smem_addr + p.bar_off + 24 * p.num_stages + 88; }
-  __device__ uint32_t cl_dead_word() const { return smem_addr + p.bar_off + 24 * p.num_stages + 96; }
+  __device__ uint32_t cl_arrive_bar() const { return smem_addr + p.bar_off + kFlagsOff + 80; }
+  __device__ uint32_t cl_open_bar() const { return smem_addr + p.bar_off + kFlagsOff + 88; }
+  __device__ uint32_t cl_dead_word() const { return smem_addr + p.bar_off + kFlagsOff + 96; }
   // wide path, per accumulator buffer: sums complete (tcgen05.commit), sums fetched (one arrival per finishing warp)
-  __device__ uint32_t acc_full_bar(unsigned b) const { return smem_addr + p.bar_off + 24 * p.num_stages + 104 + 8 * b; }
-  __device__ uint32_t acc_empty_bar(unsigned b) const { return smem_addr + p.bar_off + 24 * p.num_stages + 120 + 8 * b; }
-  // wide path, per stage: the raw rows of a box that still has to be normalised
-  __device__ uint32_t xraw_bar(int s) const { return smem_addr + p.bar_off + 24 * p.num_stages + 136 + 8 * s; }
+  __device__ uint32_t acc_full_bar(unsigned b) const { return smem_addr + p.bar_off + kFlagsOff + 104 + 8 * b; }
+  __device__ uint32_t acc_empty_bar(unsigned b) const { return smem_addr + p.bar_off + kFlagsOff + 120 + 8 * b; }
   __device__ float* sums() const { return (float*)(smem + p.sums_off); }
   __device__ float* red() const { return (float*)(smem + p.red_off); }  // small scratch: reductions, lengths
 };
 // flags(): [0] go word written by consumers, read by the producer
 //          [1] stages issued by the producer   [2] broadcast slot   [3] dead flag of the op
-//          [4] linear ops whose barrier the consumers have passed   [5] wide path: stages multiplied
+//          [4] linear ops whose barrier the consumers have passed   [5] stages taken from the ring by the tcgen05 issuer
 //          [6] wide path: linear ops whose row scales are in the token table
 
 #define MK_STAMP(c, k)                                             \
@@ -383,7 +442,7 @@ __device__ __forceinline__ void grid_wait(Ctx& c) {
       }
     } else {
       if (!cluster_bar_wait(c, c.cl_open_bar(), c.nbar & 1u)) dead = true;
-      else dead = *reinterpret_cast<volatile uint32_t*>(c.smem + c.p.bar_off + 24 * c.p.num_stages + 96) != 0u;
+      else dead = *reinterpret_cast<volatile uint32_t*>(c.smem + c.p.bar_off + kFlagsOff + 96) != 0u;
     }
     c.flags()[3] = dead ? 1 : 0;
   }
@@ -3022,7 +3081,7 @@ __device__ __forceinline__ void producer_loop(Ctx& c) {
           break;
         }
         const uint32_t full = bar_full0 + 8 * s;
-        const uint32_t dst = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes;
+        const uint32_t dst = c.smem_addr + (uint32_t)s * (uint32_t)kStageBytes;
         mbar_arrive_expect_tx(full, kStageBytes);
         tma_load_2d_hint(dst, lc.tmap, full, lc.kt * kTileK, lc.blk * kTileRows, pol_stream);
         tma_load_2d_hint(dst + kSubBytes, lc.tmap, full, lc.kt * kTileK + kBoxK, lc.blk * kTileRows, pol_stream);
@@ -3061,7 +3120,7 @@ __device__ __forceinline__ void xproducer_loop(Ctx& c) {
   // per stage: parity of its next use, whether its latest box is a plain one; raw boxes (for the norm warp) issued and
   // parity of the next one
   unsigned xuse = 0, last_plain = 0, issued_raw = 0, raw_phase = 0;
-  const uint32_t bar_x0 = c.xfull_bar(0), bar_raw0 = c.xraw_bar(0), bar_empty0 = c.empty_bar(0);
+  const uint32_t bar_x0 = c.xfull_bar(0), bar_raw0 = c.xraw_bar(0), bar_empty0 = c.xempty_bar(0);
   const uint32_t x_sub = (uint32_t)p.x_rows * 128u;
   for (int iter = 1;; ++iter) {
     int go;
@@ -3087,7 +3146,7 @@ __device__ __forceinline__ void xproducer_loop(Ctx& c) {
           break;
         }
         const uint32_t full = (raw ? bar_raw0 : bar_x0) + 8 * s;
-        const uint32_t dst = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes + kStageBytes;
+        const uint32_t dst = c.xbox(s);
         mbar_arrive_expect_tx(full, 2 * x_sub);
         if (kBoxArrivals > 1 && !raw) mbar_arrive_n(full, kBoxArrivals - 1);
         tma_load_2d(dst, tmap, full, lc.kt * kTileK, 0);
@@ -3156,11 +3215,13 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
   c.lin_seq = 0;
   volatile int* fl = c.flags();
   if (threadIdx.x == 0) {
-    for (int s = 0; s < p.num_stages; ++s) {
+    for (int s = 0; s < kMaxStages; ++s) {
       mbar_init(c.full_bar(s), 1);
-      mbar_init(c.empty_bar(s), PATH == PATH_WIDE ? 1 : kNumConsumerWarps);  // the commit of the stage's MMAs, or every consumer warp
+      mbar_init(c.empty_bar(s), PATH == PATH_WIDE ? 1 : kNumConsumerWarps);  // the commit behind what read the stage, or every consumer warp
       mbar_init(c.xfull_bar(s), kBoxArrivals);
-      if (PATH == PATH_WIDE) mbar_init(c.xraw_bar(s), 1);
+      mbar_init(c.xempty_bar(s), 1);
+      mbar_init(c.xraw_bar(s), 1);
+      mbar_init(c.tfree_bar(s), 1);
     }
     mbar_init(c.done_bar(), 1);
     for (int b = 0; b < 2; ++b) {
@@ -3188,24 +3249,27 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
 #endif
-  // Tensor memory for the tcgen05 linears: two buffers of x_rows columns of fp32 accumulators,
-  // allocated once by warp 0 and freed by it when the CTA leaves.
+  // All of the tensor memory (the CTA has its SM to itself), allocated once by warp 0 and freed by it when the CTA leaves: two
+  // buffers of x_rows columns of fp32 accumulators, then slots of the weight ring.
   constexpr bool use_tmem = PATH == PATH_WIDE;
   if (use_tmem) {
     if (c.warp == 0) {
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(c.tmem_slot()), "r"(2u * (uint32_t)p.x_rows) : "memory");
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(c.tmem_slot()), "n"(kTmemCols) : "memory");
       asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    c.tmem = *reinterpret_cast<volatile uint32_t*>(c.smem + p.bar_off + 24 * p.num_stages + 72);
+    c.tmem = *reinterpret_cast<volatile uint32_t*>(c.smem + p.bar_off + kFlagsOff + 72);
   }
 
   if (c.warp >= kNumConsumerWarps) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kServiceRegs));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(service_regs(NC)));
     if (c.warp == kNumConsumerWarps) {
-      if (c.lane == 0) producer_loop<PATH>(c);
+      // (one elected lane: the compiler then issues TMA and tcgen05 instructions from uniform registers, without moving their operands
+      // there one by one.  8 MoE layers, one request 582 -> 551 us per step, two 751 -> 676; one request of 12 dense layers of 8B
+      // width 1073 and 1081, and the wide instances spill)
+      if (MK_WITH_MOE ? elect_one() : c.lane == 0) producer_loop<PATH>(c);
     } else if (c.warp == kNumConsumerWarps + 1) {
       if constexpr (PATH == PATH_ROWS) {
         rows_prefetch_loop(c);
@@ -3214,14 +3278,14 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
       }
     } else if (PATH == PATH_WIDE && c.warp == kNumConsumerWarps + 2) {
       if constexpr (PATH == PATH_WIDE) {
-        if (c.lane == 0) mma_loop(c);
+        if (elect_one()) mma_loop(c);
       }
     } else {
       if constexpr (PATH == PATH_WIDE && 2 * NC <= kNormBoxRows) norm_loop(c);
     }
     __syncwarp();
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kConsumerRegs));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(consumer_regs(NC)));
     for (int iter = 1;; ++iter) {
       c.iter = iter;
       c.cur_op = -1;
@@ -3371,7 +3435,7 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
   if (use_tmem && c.warp == 0) {
     // (the MMA issuer has waited for everything it had in flight)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(c.tmem), "r"(2u * (uint32_t)p.x_rows) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(c.tmem), "n"(kTmemCols) : "memory");
   }
 #if MK_HIER_BARRIER
   if (c.cl_size > 1) {  // a peer may still be storing into this CTA's shared memory

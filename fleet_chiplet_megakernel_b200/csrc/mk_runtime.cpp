@@ -34,6 +34,7 @@ namespace {
 constexpr int kParamSmem = 768;  // static shared memory of the kernel: its copy of KParams
 static_assert(sizeof(mk::KParams) <= kParamSmem, "the kernel's parameter copy");
 constexpr int kMaxSmem = 232448 - kParamSmem;  // 227 KB opt-in limit per CTA on sm_100
+constexpr int kBarDescBytes = mk::kBarBytes + 2 * sizeof(mk::OpDesc);  // barriers and flags, then the two op descriptors
 constexpr int kRedBytes = 2048;    // small scratch (reductions, argmax, sequence lengths)
 constexpr int kFastSmem = 166912 - kParamSmem;  // 164 KB carve-out minus the 1 KB the system reserves per CTA
 constexpr int kRowsSumsBytes = mk::kNumConsumerWarps * mk::kChunkRows * 2 * 4;  // [warp][32 rows][2 tokens] floats
@@ -49,7 +50,7 @@ constexpr int kMaxStepTimes = 16384;
 // is 9 KB for that reason): what the ring does not take is L1, and another stage brings nothing up to 64 token rows.  12 layers of 8B width, us per step: 8 requests with 3, 4 and 5 stages 1477, 1453, 1454; 32
 // requests 1588, 1562, 1566; 64 requests with 2, 3 and 4 1942, 1823, 1826; 2048 hidden, 8 requests with 3, 4 and 5 910, 893,
 // 904; more only pays from 65 token rows on (2 and 3: 2377 and 2243).
-constexpr int kWideFixed = 1024 /*alignment slack*/ + mk::kWideRedBytes + 2048 /*barriers and flags, op descriptors*/;
+constexpr int kWideFixed = 1024 /*alignment slack*/ + mk::kWideRedBytes + kBarDescBytes;
 int wide_x_rows(int tokens) { return tokens <= 16 ? 16 : (tokens <= 32 ? 32 : (tokens <= 64 ? 64 : 128)); }
 int wide_stage_bytes(int tokens) { return mk::kStageBytes + 2 * wide_x_rows(tokens) * 128; }
 int wide_stages(int tokens, int x_bytes) {
@@ -59,7 +60,7 @@ int wide_stages(int tokens, int x_bytes) {
 
 // Row-owner path: five stages where they fit beside the resident rows.  12 layers of 8B width, us per step with 4 and 5 stages:
 // one request 1119 and 1109; two requests, 3, 4 and 5: 1238, 1172, 1166.
-constexpr int kRowsFixed = 1024 /*alignment slack*/ + kRowsSumsBytes + kRedBytes + 1024 /*barriers and flags, op descriptors*/;
+constexpr int kRowsFixed = 1024 /*alignment slack*/ + kRowsSumsBytes + kRedBytes + kBarDescBytes;
 int rows_stages(int x_bytes) { return std::min((kMaxSmem - kRowsFixed - x_bytes) / mk::kStageBytes, 5); }
 // Page numbers that the scheduler can keep in shared memory while it rewrites the page table: between two iterations the weight
 // ring in front of the x region is empty, so the table has both (MoE programs keep expert ids in the last 512 bytes).
@@ -1333,9 +1334,8 @@ static int compile_program(mk_handle* h, bool first) {
   const int stage_bytes = rows_mode ? mk::kStageBytes : wide_stage_bytes(nt);
   const int sums_bytes = rows_mode ? kRowsSumsBytes : 0;
   const int red_bytes = rows_mode ? kRedBytes : mk::kWideRedBytes;
-  const int bar_bytes = rows_mode ? 1024 : 2048;  // barriers and flags, then the two op descriptors
-  const int fixed0 = rows_mode ? kRowsFixed : kWideFixed;
-  const int want_stages = cfg.max_stages > 0 ? std::min(cfg.max_stages, 16) : 4;
+    const int fixed0 = rows_mode ? kRowsFixed : kWideFixed;
+  const int want_stages = cfg.max_stages > 0 ? std::min<int>(cfg.max_stages, mk::kMaxStages) : 4;
   // (row-owner mode prefers two resident token rows to one row and a stage more)
   int x_budget = kRowsXBudget;
   int x_bytes = 0;
@@ -1401,8 +1401,8 @@ static int compile_program(mk_handle* h, bool first) {
   kp.sums_stride = 2;
   kp.red_off = kp.x_off + x_bytes + sums_bytes;
   kp.bar_off = kp.red_off + red_bytes;
-  kp.desc_off = kp.bar_off + bar_bytes / 2;
-  h->smem_bytes = kp.bar_off + bar_bytes + 1024;
+  kp.desc_off = kp.bar_off + mk::kBarBytes;
+  h->smem_bytes = kp.bar_off + kBarDescBytes + 1024;
   kp.path = rows_mode ? mk::PATH_ROWS : mk::PATH_WIDE;
   kp.has_attn = has_attn ? 1 : 0;
   kp.rank = cfg.rank;

@@ -23,10 +23,14 @@ constexpr int kNumConsumerWarps = 8;
 constexpr int kNumConsumers = kNumConsumerWarps * 32;
 // + a warpgroup of service warps: the weight producer, the activation producer (or L2 look-ahead) and, on the wide path, the
 // MMA issuer and the norm warp.  The block starts with kLaunchRegs registers a thread; the service warps hand theirs to the
-// consumers (their sum is what the block was launched with; an instance that is compiled to fewer is not launched).
+// consumers (their sum is what the block was launched with; an instance that is compiled to fewer is not launched).  The
+// instances with a norm warp, up to 32 token rows, leave it 72: with 56 it has two rows in flight instead of four (12 layers of 8B
+// width, us per step: 32 requests 1520 and 1421, 8 requests 1249 and 1237); the others have consumers that would spill with 216.
 constexpr int kNumThreads = kNumConsumers + 128;
-constexpr int kServiceRegs = 56, kConsumerRegs = 224, kLaunchRegs = 168;
-static_assert(128 * kServiceRegs + kNumConsumers * kConsumerRegs == kNumThreads * kLaunchRegs, "a register split beyond the block's own would wait for good");
+constexpr int kLaunchRegs = 168;
+__host__ __device__ constexpr int service_regs(int nc) { return nc == 8 || nc == 16 ? 72 : 56; }  // (nc: MK_NC of the instance)
+__host__ __device__ constexpr int consumer_regs(int nc) { return (kNumThreads * kLaunchRegs - 128 * service_regs(nc)) / kNumConsumers; }
+static_assert(consumer_regs(0) == 224 && consumer_regs(8) == 216, "register counts in steps of eight, no more than the block has");
 constexpr int kWideRedBytes = 4096;              // scratch of the wide path: reductions and the iteration's token table
 constexpr int kHeadDim = 128;
 // Widest activation box that the norm is applied to in shared memory: what one warp normalises in the time a weight stage takes
@@ -41,6 +45,16 @@ constexpr int kNormStagedCols = 24576;
 constexpr int kUnitRows = 8;
 constexpr int kChunkRows = 32;
 constexpr int kRowsStageK = 512;
+// Tensor memory: 512 columns of 128 lanes x 4 bytes.  A slot holds a stage's 32 KB of weights.
+constexpr int kTmemCols = 512;
+constexpr int kSlotCols = 64;
+// Slots of the wide path's weight ring behind two accumulator buffers of x_rows columns: 7 up to 32 token rows, 6 up to 64, 4 beyond.
+__host__ __device__ constexpr int wide_slots(int x_rows) { return (kTmemCols - 2 * x_rows) / kSlotCols; }
+// mbarriers of a CTA: six groups of kMaxStages (see Ctx in mk_kernel.cu), then flags and the single ones
+constexpr int kMaxStages = 8;
+constexpr int kFlagsOff = 6 * kMaxStages * 8;
+constexpr int kBarBytes = kFlagsOff + 192;
+static_assert(wide_slots(16) <= kMaxStages, "a barrier per slot");
 
 enum OpType : int {
   OP_EMBED = 1,

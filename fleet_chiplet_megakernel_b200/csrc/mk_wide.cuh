@@ -2,8 +2,9 @@
 //
 // Linears are stream-K tiles on the 5th-generation tensor cores.  Five roles per CTA work side by side:
 //   warp 8   weight producer      TMA boxes of 128 rows x 64 k into the ring (producer_loop)
-//   warp 9   activation producer  the matching boxes of x_rows token rows x 64 k (xproducer_loop)
-//   warp 10  MMA issuer           tcgen05.mma over a stage's boxes, accumulators in tensor memory (mma_loop)
+//   warp 9   activation producer  the matching boxes of x_rows token rows x 64 k, in a ring of their own (xproducer_loop)
+//   warp 10  MMA issuer           tcgen05.mma over a tile's boxes, accumulators in tensor memory, where it also sets weights
+//                                 aside that have to wait for their activations (mma_loop)
 //   warp 11  norm warp            RMSNorm of the activation boxes, up to 32 token rows (norm_loop)
 //   warps 0-7                     finish: accumulators -> split-k exchange -> epilogue (linear_wide)
 // The accumulators are double-buffered, so the MMAs of the next row block run while the finishing warps
@@ -14,10 +15,13 @@
 // ------------------------------------------------------------------------------------
 // tcgen05
 // ------------------------------------------------------------------------------------
-__device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr) {
-  // start address >> 4 | leading offset (unused for swizzled K-major) 1 | stride between 8-row
-  // groups 1024 B >> 4 | descriptor version 1 | layout 2 = 128-byte swizzle
-  return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+// the same with A in tensor memory: 16 k-elements of 128 rows are eight columns
+__device__ __forceinline__ void umma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
 }
 __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
@@ -25,9 +29,6 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
-}
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 // NC (8, 16 or 32) accumulator columns of this warp's 32 lanes; the caller waits with tmem_wait_ld
 template <int NC>
@@ -56,7 +57,6 @@ __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[NC]) {
         : "memory");
   }
 }
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
 // This CTA's range of a stream-K linear's tiles (row block major, k minor); false: nothing for it.
 __device__ __forceinline__ bool wide_range(const KParams& p, const OpDesc& op, unsigned& total, int& G, unsigned& t0, unsigned& t1) {
@@ -117,7 +117,7 @@ __device__ __forceinline__ void wide_fill_tokens(Ctx& c, int T) {
 }
 
 // ------------------------------------------------------------------------------------
-// the MMA issuer (one lane of warp 10)
+// the MMA issuer (one elected lane of warp 10)
 // ------------------------------------------------------------------------------------
 // Waits for the consumers to publish iteration `iter`; false: the launch ends.
 __device__ __forceinline__ bool wait_go(const Ctx& c, volatile int* fl, int iter, int& go) {
@@ -153,17 +153,70 @@ __device__ __forceinline__ bool wait_lin(const Ctx& c, volatile int* fl, int wor
   return true;
 }
 
+// Weights depend on nobody, so between two ops the ring fills up and HBM would idle until the first activations arrive: split
+// sums, a barrier, a round trip for the boxes, 8 to 18 us around an attention op, of which three or four stages of the ring are 2 to
+// 3.  So when all stages of the ring have landed and there is nothing to multiply, the oldest goes into a slot of tensor memory
+// (tcgen05.cp, 0.27 us) and its stage is loaded again: 7 slots of 32 KB up to 32 token rows, 6 up to 64, 4 beyond.  Tiles are
+// multiplied in order, those set aside with A in tensor memory.  While boxes are there nothing is set aside: every tile through
+// tensor memory streams at 1.16 us a tile instead of 0.69 (copies and products take turns on the same pipe).
+// 12 layers of 8B width, us per step, without the slots and with them: 8 requests 1303 and 1249, 64 requests 1732 and 1680.
+//
+// The issuer is an elected lane, not lane 0: behind elect.sync the compiler issues tcgen05 from uniform registers.  Eight products
+// of a tile and a commit take 400 cycles instead of 920, of the 1350 in which HBM delivers a tile (128 x 16 x 16 each, the same up
+// to 64 columns); the step at 8 requests fell from 1392 to 1303 us with it, and setting aside pays only since.
 __device__ __forceinline__ void mma_loop(Ctx& c) {
   const KParams& p = c.p;
-  const int S = p.num_stages, N = p.x_rows;
+  const int S = p.num_stages, N = p.x_rows, slots = wide_slots(N);
   volatile int* fl = c.flags();
-  const uint32_t bar_full0 = c.full_bar(0), bar_empty0 = c.empty_bar(0), bar_x0 = c.xfull_bar(0);
   const uint32_t x_sub = (uint32_t)N * 128u;  // bytes of one activation box
+  const uint32_t slot0 = c.tmem + 2u * (uint32_t)N;
   // instruction descriptor: D = f32, A = B = bf16, both K-major, N >> 3, M >> 4
   const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((128u >> 4) << 24);
-  int s = 0;
-  uint32_t parity = 0;
-  unsigned consumed = 0, runs = 0;  // stages multiplied; accumulator runs started
+  int s = 0, xs = 0;               // next stage of weights, of activation boxes
+  uint32_t parity = 0, xparity = 0;
+  int head = 0, tail = 0, held = 0;  // slots: the oldest tile, the next to fill, tiles held
+  uint32_t tail_parity = 1;
+  unsigned taken = 0, runs = 0;  // stages taken from the ring; accumulator runs started
+  auto set_aside = [&]() {
+    const int newest = s == 0 ? S - 1 : s - 1;
+    // (the oldest and the newest stage: copies may land out of order)
+    if (held == slots || !mbar_test_wait(c.full_bar(s), parity) || !mbar_test_wait(c.full_bar(newest), s == 0 ? parity : parity ^ 1u) ||
+        !mbar_test_wait(c.tfree_bar(tail), tail_parity)) return;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t src = c.smem_addr + (uint32_t)s * (uint32_t)kStageBytes, dst = slot0 + (uint32_t)(tail * kSlotCols);
+    tmem_put_128x64(dst, src);
+    tmem_put_128x64(dst + 32u, src + kSubBytes);
+    umma_commit(c.empty_bar(s));
+    ++held;
+    ++taken;
+    if (++tail == slots) {
+      tail = 0;
+      tail_parity ^= 1u;
+    }
+    if (++s == S) {
+      s = 0;
+      parity ^= 1u;
+    }
+  };
+  // A bounded wait that sets tiles aside meanwhile.
+  auto ready = [&](uint32_t bar, uint32_t par, bool wait) {
+    unsigned long long since = 0;
+    unsigned polls = 0;
+    while (wait && !mbar_try_wait_for(bar, par, 200u)) {
+      set_aside();
+      if (((++polls) & 1023u) == 0) {
+        if (aborted(c)) return false;
+        const unsigned long long now = globaltimer();
+        if (since == 0) {
+          since = now;
+        } else if (now - since > 4 * p.timeout_ns) {
+          raise_abort(c, ST_TIMEOUT_FULL, (int)bar, (int)par);
+          return false;
+        }
+      }
+    }
+    return true;
+  };
   bool dead = false;
   for (int iter = 1; !dead; ++iter) {
     int go;
@@ -178,27 +231,48 @@ __device__ __forceinline__ void mma_loop(Ctx& c) {
       int kt = (int)(t0 % (unsigned)nkt);
       bool fresh = true;
       for (unsigned tile = t0; tile < t1; ++tile) {
-        const uint32_t d = c.tmem + (runs & 1u) * (uint32_t)N;
-        if (fresh && !mbar_wait(c, c.acc_empty_bar(runs & 1), ((runs >> 1) & 1u) ^ 1u, ST_TIMEOUT_EMPTY)) { dead = true; break; }
-        if (!mbar_wait(c, bar_full0 + 8 * s, parity, ST_TIMEOUT_FULL) || !mbar_wait(c, bar_x0 + 8 * s, parity, ST_TIMEOUT_FULL)) { dead = true; break; }
+        if (!ready(c.acc_empty_bar(runs & 1), ((runs >> 1) & 1u) ^ 1u, fresh) || !ready(c.xfull_bar(xs), xparity, true) ||
+            (held == 0 && !mbar_wait(c, c.full_bar(s), parity, ST_TIMEOUT_FULL))) {
+          dead = true;
+          break;
+        }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        const uint32_t st = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes;
-        const uint32_t xt = st + kStageBytes;
+        const uint32_t d = c.tmem + (runs & 1u) * (uint32_t)N, xt = c.xbox(xs);
+        if (held == 0) {  // straight from shared memory
+          const uint32_t st = c.smem_addr + (uint32_t)s * (uint32_t)kStageBytes;
 #pragma unroll
-        for (int sub = 0; sub < kSubTiles; ++sub) {
-          const uint64_t ad = umma_smem_desc(st + (uint32_t)sub * kSubBytes);
-          const uint64_t bd = umma_smem_desc(xt + (uint32_t)sub * x_sub);
+          for (int sub = 0; sub < kSubTiles; ++sub) {
+            const uint64_t ad = umma_smem_desc(st + (uint32_t)sub * kSubBytes);
+            const uint64_t bd = umma_smem_desc(xt + (uint32_t)sub * x_sub);
 #pragma unroll
-          for (int k16 = 0; k16 < 4; ++k16)  // 16 k-elements = 32 bytes further inside the swizzle span: +2 in the address field
-            umma_bf16(d, ad + (uint64_t)(2 * k16), bd + (uint64_t)(2 * k16), idesc, (fresh && sub == 0 && k16 == 0) ? 0u : 1u);
+            for (int k16 = 0; k16 < 4; ++k16)  // 16 k-elements = 32 bytes further inside the swizzle span: +2 in the address field
+              umma_bf16(d, ad + (uint64_t)(2 * k16), bd + (uint64_t)(2 * k16), idesc, (fresh && sub == 0 && k16 == 0) ? 0u : 1u);
+          }
+          umma_commit(c.empty_bar(s));
+          ++taken;
+          if (++s == S) {
+            s = 0;
+            parity ^= 1u;
+          }
+        } else {
+          const uint32_t at = slot0 + (uint32_t)(head * kSlotCols);
+#pragma unroll
+          for (int sub = 0; sub < kSubTiles; ++sub) {
+            const uint64_t bd = umma_smem_desc(xt + (uint32_t)sub * x_sub);
+#pragma unroll
+            for (int k16 = 0; k16 < 4; ++k16)
+              umma_bf16_ta(d, at + 32u * sub + 8u * k16, bd + (uint64_t)(2 * k16), idesc, (fresh && sub == 0 && k16 == 0) ? 0u : 1u);
+          }
+          umma_commit(c.tfree_bar(head));
+          if (++head == slots) head = 0;
+          --held;
         }
-        umma_commit(bar_empty0 + 8 * s);
+        umma_commit(c.xempty_bar(xs));
+        if (++xs == S) {
+          xs = 0;
+          xparity ^= 1u;
+        }
         fresh = false;
-        ++consumed;
-        if (++s == S) {
-          s = 0;
-          parity ^= 1u;
-        }
         if (++kt == nkt || tile + 1 == t1) {  // the run ends: its accumulators belong to the finishing warps
           umma_commit(c.acc_full_bar(runs & 1));
           ++runs;
@@ -212,7 +286,7 @@ __device__ __forceinline__ void mma_loop(Ctx& c) {
   // nothing of this thread may be in flight when the tensor memory is given back
   umma_commit(c.done_bar());
   mbar_wait(c, c.done_bar(), 0u, ST_TIMEOUT_FULL);
-  fl[5] = (int)consumed;
+  fl[5] = (int)taken;
 }
 
 // ------------------------------------------------------------------------------------
@@ -280,7 +354,7 @@ __device__ __forceinline__ void norm_loop(Ctx& c) {
   const int col = c.lane & 15, row0 = c.lane >> 4;
   // rows row0 + 2 u of eight: 256 u bytes further, in the 16-byte column that the swizzle gives them
   const uint32_t swz = (uint32_t)(((col & 7) ^ row0) << 4);
-  const uint32_t sub = kStageBytes + (uint32_t)(col >> 3) * (uint32_t)p.x_rows * 128u + (uint32_t)row0 * 128u;
+  const uint32_t sub = (uint32_t)(col >> 3) * (uint32_t)p.x_rows * 128u + (uint32_t)row0 * 128u;
   int s = 0;
   unsigned raw_phase = 0;  // per stage: parity of its next raw box
   unsigned lin_seq = 0;
@@ -312,21 +386,21 @@ __device__ __forceinline__ void norm_loop(Ctx& c) {
         kv = kv + 16 == k_end ? 0 : kv + 16;
         const uint4 w_next = weights(kv);
         if (!mbar_wait(c, c.xraw_bar(s), (raw_phase >> s) & 1u, ST_TIMEOUT_FULL)) return;
-        uint32_t box = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes + sub;
+        uint32_t box = c.xbox(s) + sub;
         uint32_t sc = smem_u32(wide_tab(c).scale) + (uint32_t)row0 * (kNormBoxRows / 2) * 4u;
         // (rows past T, still inside the box, are nobody's)
         if (p.numerics == NUM_TORCH) {
 #pragma unroll 1
           for (int t = 0; t < T; t += 8) {
+            uint4 x[4];
+            const uint4 r = lds128(sc);
 #pragma unroll
-            for (int u = 0; u < 4; u += 2) {
-              const uint32_t at0 = box + 256u * u + (swz ^ (32u * u)), at1 = box + 256u * (u + 1) + (swz ^ (32u * (u + 1)));
-              const uint4 x0 = lds128(at0), x1 = lds128(at1);
-              const uint2 r = lds64(sc + 4 * u);
-              sts128(at0, make_uint4(hmul2_bf16(w.x, hmul2_bf16(x0.x, r.x)), hmul2_bf16(w.y, hmul2_bf16(x0.y, r.x)),
-                                     hmul2_bf16(w.z, hmul2_bf16(x0.z, r.x)), hmul2_bf16(w.w, hmul2_bf16(x0.w, r.x))));
-              sts128(at1, make_uint4(hmul2_bf16(w.x, hmul2_bf16(x1.x, r.y)), hmul2_bf16(w.y, hmul2_bf16(x1.y, r.y)),
-                                     hmul2_bf16(w.z, hmul2_bf16(x1.z, r.y)), hmul2_bf16(w.w, hmul2_bf16(x1.w, r.y))));
+            for (int u = 0; u < 4; ++u) x[u] = lds128(box + 256u * u + (swz ^ (32u * u)));
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const uint32_t ru = u == 0 ? r.x : (u == 1 ? r.y : (u == 2 ? r.z : r.w));
+              sts128(box + 256u * u + (swz ^ (32u * u)), make_uint4(hmul2_bf16(w.x, hmul2_bf16(x[u].x, ru)), hmul2_bf16(w.y, hmul2_bf16(x[u].y, ru)),
+                                                                    hmul2_bf16(w.z, hmul2_bf16(x[u].z, ru)), hmul2_bf16(w.w, hmul2_bf16(x[u].w, ru))));
             }
             box += 1024;
             sc += 16;
@@ -335,11 +409,13 @@ __device__ __forceinline__ void norm_loop(Ctx& c) {
 #pragma unroll 1
           for (int t = 0; t < T; t += 8) {
 #pragma unroll
-            for (int u = 0; u < 4; ++u) {
-              const uint32_t at = box + 256u * u + (swz ^ (32u * u));
-              const uint4 x = lds128(at);
-              sts128(at, scale8(x, w, __uint_as_float(lds32(sc + 4 * u)), false));
-              if (u == 1 && t + 4 >= T) break;  // (rows t + 4 .. t + 7 are nobody's)
+            for (int u = 0; u < 4; u += 2) {
+              const uint32_t at0 = box + 256u * u + (swz ^ (32u * u)), at1 = box + 256u * (u + 1) + (swz ^ (32u * (u + 1)));
+              const uint4 x0 = lds128(at0), x1 = lds128(at1);
+              const uint2 r = lds64(sc + 4 * u);
+              sts128(at0, scale8(x0, w, __uint_as_float(r.x), false));
+              sts128(at1, scale8(x1, w, __uint_as_float(r.y), false));
+              if (u == 0 && t + 4 >= T) break;  // (rows t + 4 .. t + 7 are nobody's)
             }
             box += 1024;
             sc += 16;
