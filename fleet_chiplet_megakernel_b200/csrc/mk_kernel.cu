@@ -4,8 +4,8 @@
 // producer that streams this CTA's share of every linear layer's weights (boxes of 64 k-elements,
 // 128-byte swizzle) into a ring of shared-memory stages, running ahead of the consumers across op
 // boundaries (weights have no dependencies); the eight consumer warps walk the program: wait at a
-// grid barrier where an op reads what other CTAs wrote, do the op's share of work, go on.  The wide
-// path (mk_wide.cuh) has three more roles, an activation producer, an MMA issuer and a norm warp.  Every wait in
+// grid barrier where an op reads what other CTAs wrote, do the op's share of work, go on.  Warp 10 issues the
+// linears' tcgen05 instructions; the wide path (mk_wide.cuh) has two more roles, an activation producer and a norm warp.  Every wait in
 // the kernel is bounded: on expiry the waiter records a status and raises a sticky abort flag that
 // all other waits poll, and the kernel returns with an error code.
 //
@@ -155,10 +155,25 @@ __device__ __forceinline__ bool elect_one() {
   return is != 0u;
 }
 // ---- tcgen05: descriptors, completion, shared memory -> tensor memory
-__device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr) {
+__device__ __forceinline__ uint64_t umma_smem_desc(uint32_t saddr, uint32_t group_bytes = 1024u) {
   // start address >> 4 | leading offset (unused for swizzled K-major) 1 | stride between 8-row
-  // groups 1024 B >> 4 | descriptor version 1 | layout 2 = 128-byte swizzle
-  return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | (64ull << 32) | (1ull << 46) | (2ull << 61);
+  // groups >> 4 | descriptor version 1 | layout 2 = 128-byte swizzle
+  return (uint64_t)((saddr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(group_bytes >> 4) << 32) | (1ull << 46) | (2ull << 61);
+}
+__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// the same with A in tensor memory: 16 k-elements of 128 rows are eight columns
+__device__ __forceinline__ void umma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
 }
 __device__ __forceinline__ void umma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
@@ -170,6 +185,12 @@ __device__ __forceinline__ void tmem_put_128x64(uint32_t tmem, uint32_t saddr) {
 #pragma unroll
   for (int q = 0; q < 4; ++q)  // 16 k-elements = 32 bytes further inside the swizzle span
     asm volatile("tcgen05.cp.cta_group::1.128x256b [%0], %1;" ::"r"(tmem + 8u * q), "l"(d + (uint64_t)(2 * q)) : "memory");
+}
+// one accumulator column of this warp's 32 lanes; the caller waits with tmem_wait_ld
+__device__ __forceinline__ uint32_t tmem_ld1(uint32_t taddr) {
+  uint32_t r;
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(r) : "r"(taddr) : "memory");
+  return r;
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, 256;" ::: "memory"); }
@@ -225,11 +246,10 @@ struct Ctx {
   uint8_t* smem;
   uint32_t smem_addr;
   unsigned epoch;     // grid barriers passed
-  unsigned cons_idx;  // weight stages consumed
   bool arrived;       // this CTA has already arrived at the coming grid barrier
   int attn_iter;      // row-owner path: iteration whose attention metadata is cached in shared memory; wide path: head geometry planned
   uint32_t tmem;      // base address of the CTA's tensor-memory columns
-  unsigned acc_runs;  // wide path: accumulator runs finished
+  unsigned acc_runs;  // accumulator runs (row-owner path: chunks) finished
   int tid, lane, warp;
   int iter, cur_op;
   unsigned long long* dbg;  // inner-phase stamps of the traced op (thread 0), or null
@@ -333,6 +353,88 @@ __device__ __forceinline__ bool mbar_wait(const Ctx& c, uint32_t bar, uint32_t p
     if (mbar_try_wait(bar, parity)) return true;
   return mbar_wait_slow(&c.p, c.iter, c.cur_op, bar, parity, code);
 }
+
+// The weight ring as its tcgen05 issuer sees it: stages in shared memory, and slots of tensor memory for tiles that have to wait
+// for their activations.  Tiles are used in order, those in slots (the older ones) first.
+//
+// Weights depend on nobody, so between two ops the ring fills up and HBM would idle until the first activations are there: split
+// sums, words or a barrier, staging, 4 to 18 us, of which three to four stages are 2 to 3.  So while there is nothing to multiply,
+// the oldest stage goes into a slot (tcgen05.cp, 0.27 us) and is loaded again.  While there is, nothing goes into a slot: every tile
+// through tensor memory streams at 1.16 us a tile instead of 0.69 (copies and products take turns on the same pipe), and mma.sync
+// stands still while a copy is under way.  `flying`: loads that may still be under way when a stage goes into a slot, which is how
+// hard the stream goes on while words are polled and barriers are waited for: it slows them down.  All of them on the row-owner
+// path, one up to 32 token rows, none beyond.  12 layers of 8B width, us per step with none, one and all: one request 1057, 1032,
+// 1010; 4 requests 1190, 1167, 1213; 8 1245, 1220, 1270; 32 1419, 1408, 1425; 64 1668, 1685, 1734; 100 2215, 2228, 2220; without
+// slots: one request 1086, 8 1303, 64 1732.  With four slots instead of six one request takes 1031 instead of 1004.
+//
+// The issuer is an elected lane, not lane 0: behind elect.sync the compiler issues tcgen05 from uniform registers.  Eight products
+// (128 x 16 x 16 each, the same up to 64 columns) and a commit take 400 cycles instead of 920, of the 1350 in which HBM delivers
+// a tile; the step at 8 requests fell from 1392 to 1303 us with it.
+struct WeightRing {
+  const Ctx& c;
+  const int S, slots;
+  const uint32_t slot0;
+  int s = 0;                         // next stage
+  uint32_t parity = 0;
+  int head = 0, tail = 0, held = 0;  // slots: the oldest tile, the next to fill, tiles held
+  uint32_t tail_parity = 1;
+  unsigned taken = 0;                // stages taken from the ring
+  __device__ __forceinline__ WeightRing(const Ctx& c_, int slots_, uint32_t slot0_) : c(c_), S(c_.p.num_stages), slots(slots_), slot0(slot0_) {}
+  __device__ __forceinline__ uint32_t stage() const { return c.smem_addr + (uint32_t)(s * kStageBytes); }
+  __device__ __forceinline__ uint32_t slot() const { return slot0 + (uint32_t)(head * kSlotCols); }
+  // what reads the next stage, or the oldest slot, has been issued
+  __device__ __forceinline__ void free_stage() {
+    umma_commit(c.empty_bar(s));
+    ++taken;
+    if (++s == S) {
+      s = 0;
+      parity ^= 1u;
+    }
+  }
+  __device__ __forceinline__ void free_slot() {
+    umma_commit(c.tfree_bar(head));
+    if (++head == slots) head = 0;
+    --held;
+  }
+  // the oldest stage goes into a slot, when there is one and all stages but the `flying` newest have landed (both ends are looked
+  // at: copies may land out of order)
+  __device__ __forceinline__ void set_aside(int flying) {
+    const int last = s + S - 1 - flying, at = last >= S ? last - S : last;
+    if (held == slots || !mbar_test_wait(c.full_bar(s), parity) || !mbar_test_wait(c.full_bar(at), last >= S ? parity ^ 1u : parity) ||
+        !mbar_test_wait(c.tfree_bar(tail), tail_parity)) return;
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t src = stage(), dst = slot0 + (uint32_t)(tail * kSlotCols);
+    tmem_put_128x64(dst, src);
+    tmem_put_128x64(dst + 32u, src + kSubBytes);
+    ++held;
+    if (++tail == slots) {
+      tail = 0;
+      tail_parity ^= 1u;
+    }
+    free_stage();
+  }
+  // a bounded wait that sets tiles aside meanwhile
+  __device__ __forceinline__ bool wait(uint32_t bar, uint32_t par, int flying = 0) {
+    unsigned long long since = 0;
+    unsigned polls = 0;
+    while (!mbar_try_wait_for(bar, par, 200u)) {
+      set_aside(flying);
+      if (((++polls) & 1023u) == 0) {
+        if (aborted(c)) return false;
+        const unsigned long long now = globaltimer();
+        if (since == 0) {
+          since = now;
+        } else if (now - since > 4 * c.p.timeout_ns) {
+          raise_abort(c, ST_TIMEOUT_FULL, (int)bar, (int)par);
+          return false;
+        }
+      }
+    }
+    return true;
+  }
+  // a tile to multiply
+  __device__ __forceinline__ bool wait_tile() { return held > 0 || mbar_wait(c, c.full_bar(s), parity, ST_TIMEOUT_FULL); }
+};
 
 // Grid-wide barrier of the consumer warps.  The counter only grows within a launch: barrier
 // number e is passed when it reaches e * (arrivals per barrier), compared modulo 2^32 so
@@ -770,12 +872,13 @@ __device__ __forceinline__ float torch_rsqrt_bf16(float var, bool dbl);
 
 // activations -> shared memory, with the optional fused RMSNorm
 // ------------------------------------------------------------------------------------
-// Stages rows tok0 .. tok0+rows-1 of `in` as bf16 [rows][pitch] in the x region
-// (pitch = padded K + 8 elements, so that the 8 token rows of an ldmatrix hit 8
-// different banks), zero padded, followed by one 16-byte chunk of zeros that
-// stands in for the rows of absent tokens.
+// Row-owner path: token rows as the tensor core reads them (see linear_pass_rows), a row every x_pitch(kp) vectors of 16 bytes, kp
+// a multiple of 512 there: the 64 vectors of a 512-wide k stage are eight rows (the stage's 64-wide slices) of 128 bytes,
+// 128-byte swizzled.  Wide path (rows gathered from the ranks only): plain rows.
+__device__ __forceinline__ int x_pitch(int kp) { return kp >> 3; }
+__device__ __forceinline__ int x_vec(int v) { return MK_NC == 0 ? v ^ ((v >> 3) & 7) : v; }
 // Stage `rows` (at most 8) token rows (tokens tok0.. of T; absent ones zero) of a K-wide
-// bf16 input in shared memory, row pitch kp + 8, RMS-normalised when norm_w is given.  All
+// bf16 input in shared memory, RMS-normalised when norm_w is given.  All
 // rows are staged concurrently: the 8 consumer warps split into one group per row (8 warps
 // on a single row, 1 warp per row for 5 to 8 rows), a group's warps take interleaved
 // 512-byte pieces of the row and meet once to add up their sums of squares.  The loops are
@@ -908,7 +1011,7 @@ __device__ __forceinline__ void stage_row_regs(Ctx& c, const uint4* src, uint4* 
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int v = v0 + vstep * i;
-      if (v < nvec) dst[v] = scale8(raw[i], pre_w[i], r, torch_num);
+      if (v < nvec) dst[x_vec(v)] = scale8(raw[i], pre_w[i], r, torch_num);
     }
   }
   consumer_sync();
@@ -919,7 +1022,7 @@ __device__ __forceinline__ void stage_x(Ctx& c, const void* in, int ld_in, int K
                                      int rows, int T, const uint4* pre_w, bool gather = false, void* sums_out = nullptr) {
   if (!MK_WITH_XCHG) gather = false;  // (compiled out of the single-GPU build)
   uint4* xs = reinterpret_cast<uint4*>(c.smem + c.p.x_off);
-  const int pitch = (kp >> 3) + 1;  // uint4 per row
+  const int pitch = x_pitch(kp);  // uint4 per row
   const int nvec = kp >> 3, kvec = K >> 3;
   const bool torch_num = c.p.numerics == NUM_TORCH;
   const uint4* wv = reinterpret_cast<const uint4*>(norm_w);
@@ -931,8 +1034,6 @@ __device__ __forceinline__ void stage_x(Ctx& c, const void* in, int ld_in, int K
   uint4* dst = xs + tb * pitch;
   float* red = c.red();
   const int v0 = part * 32 + c.lane, vstep = 32 * wpr;
-  if (c.tid == 0) xs[rows * pitch] = make_uint4(0, 0, 0, 0);  // the chunk absent tokens point at
-  if (active && part == 0 && c.lane == 0) dst[nvec] = make_uint4(0, 0, 0, 0);  // the row's padding vector
   if (wv != nullptr && pre_w != nullptr && nvec <= 4 * vstep) {
     uint4* sum_row = (gather && sums_out != nullptr && valid) ? reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(sums_out) + (size_t)(tok0 + tb) * ld_in)
                                                               : nullptr;
@@ -963,7 +1064,7 @@ __device__ __forceinline__ void stage_x(Ctx& c, const void* in, int ld_in, int K
       for (int i = 0; i < 4; ++i) {
         const int v = vb + i * vstep;
         if (v < nvec) {
-          dst[v] = val[i];
+          dst[x_vec(v)] = val[i];
           if (wv != nullptr) ss = sumsq8(val[i], torch_num, ss);
         }
       }
@@ -978,26 +1079,24 @@ __device__ __forceinline__ void stage_x(Ctx& c, const void* in, int ld_in, int K
       const float r = row_rms_scale(red, tb * wpr, wpr, K, torch_num);
 #pragma unroll 2
       for (int v = v0; v < kvec; v += vstep)  // a lane re-reads only what it wrote itself
-        dst[v] = scale8(dst[v], __ldg(wv + v), r, torch_num);
+        dst[x_vec(v)] = scale8(dst[x_vec(v)], __ldg(wv + v), r, torch_num);
     }
   }
   consumer_sync();
 }
 
 // Staging for a row-owner linear WITHOUT a fused norm (one or two token rows, at most 24 stages
-// of 512 k): warp w multiplies only the w-th 64-wide slice of every stage, so it stages exactly
-// those slices of the row itself, all in one round of loads, and needs no CTA-wide sync before
-// its first tile.  Lane l takes the 16-byte chunk (l & 7) of the slices of stages (l >> 3) + 4 i.
+// of 512 k): warp w stages the w-th 64-wide slice of every stage, all in one round of loads and without a CTA-wide sync.  Lane
+// l takes the 16-byte chunk (l & 7) of the slices of stages (l >> 3) + 4 i.
 // (The same scheme with the norm fused in was 0.36 ms per step SLOWER: its unrolled scaling code
 // is several KB that every op would run once, out of a cold instruction cache.)
 __device__ __forceinline__ void stage_x_rows(Ctx& c, const void* in, int ld_in, int K, int kp, int tok0, int rows, int T) {
   constexpr int kMaxV = 6;  // 24 stages / 4 per round
   uint4* xs = reinterpret_cast<uint4*>(c.smem + c.p.x_off);
-  const int pitch = (kp >> 3) + 1;  // uint4 per row
+  const int pitch = x_pitch(kp);  // uint4 per row
   const int v0 = ((c.lane >> 3) * kRowsStageK + c.warp * 64 + (c.lane & 7) * 8) >> 3;  // vector of the first round
   constexpr int vstep = 4 * kRowsStageK / 8;                                           // vectors per round
   const int kvec = K >> 3, nvec = kp >> 3;
-  if (c.lane == 0) xs[rows * pitch] = make_uint4(0, 0, 0, 0);  // the chunk absent tokens point at (every warp writes the same zeros)
 #pragma unroll 1
   for (int t = 0; t < rows; ++t) {
     const uint4* src = reinterpret_cast<const uint4*>(reinterpret_cast<const __nv_bfloat16*>(in) + (size_t)(tok0 + t) * ld_in);
@@ -1011,7 +1110,7 @@ __device__ __forceinline__ void stage_x_rows(Ctx& c, const void* in, int ld_in, 
 #pragma unroll
     for (int i = 0; i < kMaxV; ++i) {
       const int v = v0 + i * vstep;
-      if (v < nvec) xs[t * pitch + v] = raw[i];
+      if (v < nvec) xs[t * pitch + x_vec(v)] = raw[i];
     }
   }
   __syncwarp();
@@ -1045,7 +1144,7 @@ __device__ __forceinline__ void stage_ll_regs(Ctx& c, const uint4* ll, uint4* ds
 #pragma unroll
     for (int i = 0; i < NV; ++i) {
       const int v = v0 + vstep * i;
-      if (v < nvec) dst[v] = scale8(raw[i], pre_w != nullptr ? pre_w[i] : (v < kvec ? __ldg(wv + v) : make_uint4(0, 0, 0, 0)), r, torch_num);
+      if (v < nvec) dst[x_vec(v)] = scale8(raw[i], pre_w != nullptr ? pre_w[i] : (v < kvec ? __ldg(wv + v) : make_uint4(0, 0, 0, 0)), r, torch_num);
     }
   }
   consumer_sync();
@@ -1054,7 +1153,7 @@ __device__ __forceinline__ void stage_ll_regs(Ctx& c, const uint4* ll, uint4* ds
 __device__ __forceinline__ void stage_x_ll(Ctx& c, const void* ll_in, int ld_in, int K, int kp, const void* norm_w, int tok0,
                                         int rows, int T, const uint4* pre_w, unsigned tag) {
   uint4* xs = reinterpret_cast<uint4*>(c.smem + c.p.x_off);
-  const int pitch = (kp >> 3) + 1;
+  const int pitch = x_pitch(kp);
   const int nvec = kp >> 3;
   const int wpr = stage_warps_per_row(rows);
   const int tb = c.warp / wpr, part = c.warp % wpr;
@@ -1063,21 +1162,18 @@ __device__ __forceinline__ void stage_x_ll(Ctx& c, const void* ll_in, int ld_in,
   const uint4* ll = reinterpret_cast<const uint4*>(ll_row(ll_in, ld_in, valid ? tok0 + tb : 0));
   uint4* dst = xs + tb * pitch;
   const int v0 = part * 32 + c.lane, vstep = 32 * wpr;
-  if (c.tid == 0) xs[rows * pitch] = make_uint4(0, 0, 0, 0);
-  if (active && part == 0 && c.lane == 0) dst[nvec] = make_uint4(0, 0, 0, 0);
   const uint4* wv = reinterpret_cast<const uint4*>(norm_w);
   if (nvec <= 2 * vstep) stage_ll_regs<2>(c, ll, dst, pre_w, wv, K, nvec, v0, vstep, active, valid, tb * wpr, wpr, tag);
   else stage_ll_regs<4>(c, ll, dst, pre_w, wv, K, nvec, v0, vstep, active, valid, tb * wpr, wpr, tag);
 }
-// no norm: every warp stages the k slices it multiplies (see stage_x_rows)
+// no norm: every warp stages its own k slices (see stage_x_rows)
 __device__ __forceinline__ void stage_rows_ll(Ctx& c, const void* ll_in, int ld_in, int K, int kp, int tok0, int rows, int T, unsigned tag) {
   constexpr int kMaxV = 6;
   uint4* xs = reinterpret_cast<uint4*>(c.smem + c.p.x_off);
-  const int pitch = (kp >> 3) + 1;
+  const int pitch = x_pitch(kp);
   const int v0 = ((c.lane >> 3) * kRowsStageK + c.warp * 64 + (c.lane & 7) * 8) >> 3;
   constexpr int vstep = 4 * kRowsStageK / 8;
   const int kvec = K >> 3, nvec = kp >> 3;
-  if (c.lane == 0) xs[rows * pitch] = make_uint4(0, 0, 0, 0);
 #pragma unroll 1
   for (int t = 0; t < rows; ++t) {
     const bool live = tok0 + t < T;
@@ -1089,7 +1185,7 @@ __device__ __forceinline__ void stage_rows_ll(Ctx& c, const void* ll_in, int ld_
     ll_take(c, ll, at, tag, raw);
 #pragma unroll
     for (int i = 0; i < kMaxV; ++i)
-      if (v0 + i * vstep < nvec) xs[t * pitch + v0 + i * vstep] = raw[i];
+      if (v0 + i * vstep < nvec) xs[t * pitch + x_vec(v0 + i * vstep)] = raw[i];
   }
   __syncwarp();
 }
@@ -1134,10 +1230,47 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 // more than the whole weight stream of a small layer, so every CTA takes whole output rows
 // instead: a contiguous range of 8-row units, walked in chunks of up to 32 rows over the
 // full K.  The token rows are resident in shared memory (stage_x, fused norm included).
-// Inside a chunk the 8 warps split k: warp w multiplies the w-th 64-wide k slice of every
-// 512-wide stage, 16 weight rows on the M side of the mma and the tokens on the N side, and
-// the eight partial sums of an output meet in shared memory when the chunk ends.
+//
+// A stage holds a chunk's rows for 512 k-elements as eight boxes of 32 rows x 64 k.  Four boxes are the 128 rows of a tcgen05.mma
+// whose lane 32 q + r is row r, slice q of the stage (q + 4 for the other four): the k slices of a row lie side by side on the M
+// side.  The B operand holds the eight slices of the token row as eight columns (and those of a second token as eight more), so of
+// a lane's columns only its own slice's means anything, which costs nothing (a 128 x 16 x 16 product takes as long as a 128 x 64 x
+// 16 one) and spares the finish over CTAs.  The issuer (rows_mma_loop) keeps even and odd k steps apart: four accumulators of 16
+// columns per chunk, two sets of them in turn, so that the next chunk is multiplied while the warps finish the last.  Warp w takes
+// slice w of its lanes' rows from them; the eight partial sums of an output meet in shared memory.  (These are the sums, in the
+// order, that mma.sync by the eight warps gave, and the same bits.  With it a stage was in shared memory until the slowest
+// warp had multiplied it, a chunk's finish stopped the stream's consumer, and stages could not go to tensor memory.  12 layers of
+// 8B width, us per step: one request 1086 -> 1006, two 1146 -> 1042; four layers 1024 wide 127 -> 119; 8 MoE layers 551 -> 552, two
+// requests 676 -> 697, whose chunks of two stages are too short to gain from it; 751 before the elected producer.)
 // ------------------------------------------------------------------------------------
+// The token rows of an op (or pass) are staged: the issuer may multiply.
+__device__ __forceinline__ void rows_x_ready(const Ctx& c) {
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads them through the async proxy
+  __syncwarp();
+  if (c.lane == 0) mbar_arrive(c.xfull_bar(0));
+}
+// This warp's slice of a chunk's sums -> the sums block: row = lane, `ntok` tokens to columns half, half + 1
+__device__ __forceinline__ void rows_take_sums(Ctx& c, int ntok, int half) {
+  const int TP = c.p.sums_stride;
+  mbar_wait(c, c.acc_full_bar(c.acc_runs & 1), (c.acc_runs >> 1) & 1u, ST_TIMEOUT_FULL);
+  __syncwarp();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t acc = c.tmem + (c.acc_runs & 1) * kRowsAccCols + (uint32_t)((c.warp >> 2) * 32 + c.warp) + ((uint32_t)(c.warp & 3) << 21);
+  const uint32_t even0 = tmem_ld1(acc), odd0 = tmem_ld1(acc + 16);
+  uint32_t even1 = 0u, odd1 = 0u;
+  if (ntok > 1) {
+    even1 = tmem_ld1(acc + 8);
+    odd1 = tmem_ld1(acc + 24);
+  }
+  tmem_wait_ld();
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncwarp();
+  if (c.lane == 0) mbar_arrive(c.acc_empty_bar(c.acc_runs & 1));
+  c.acc_runs += 1;
+  float* d = c.sums() + (c.warp * kChunkRows + c.lane) * TP + half;
+  d[0] = __uint_as_float(even0) + __uint_as_float(odd0);
+  if (ntok > 1) d[1] = __uint_as_float(even1) + __uint_as_float(odd1);
+}
 // Tokens one pass of a row-owner linear covers (aux3, fixed by the host from the shared-memory
 // budget) and the passes its weight stream makes for T active tokens.
 __device__ __forceinline__ int linear_passes(const OpDesc& op, int T) { return (T + op.aux3 - 1) / op.aux3; }
@@ -1171,24 +1304,9 @@ __device__ __forceinline__ void linear_pass_rows(Ctx& c, const OpDesc& op, int t
   } else if (nks <= 24 && ntok <= 2 && !(op.flags & F_NORM_IN) && !MK_XF(op, F_GATHER_IN)) stage_x_rows(c, op.in, op.ld_in, op.k, kp, tok0, ntok, T);
   else stage_x(c, op.in, op.ld_in, op.k, kp, (op.flags & F_NORM_IN) ? op.norm_w : nullptr, tok0, ntok, T, pre_w,
                MK_XF(op, F_GATHER_IN) != 0);
+  rows_x_ready(c);
   MK_STAMP(c, 1);
-  const int S = p.num_stages;
-  const int lane = c.lane, warp = c.warp;
-  const bool arith = !(p.debug_flags & 1);
-  // B operand (k x tokens): lane l addresses token (l & 7), 16-byte chunk (l >> 3) of a 32-wide k step
-  const int pitch_b = (kp + 8) * 2;
-  const uint32_t xs0 = c.smem_addr + p.x_off;
-  const bool a_real = (lane & 7) < ntok;
-  const uint32_t a_row = a_real ? xs0 + (uint32_t)((lane & 7) * pitch_b + (lane >> 3) * 16 + warp * 128)
-                                : xs0 + (uint32_t)(ntok * pitch_b);  // the zero chunk
-  // Weights sit on the M side of the mma (16 rows per tile, so a 32-row chunk is two tiles of
-  // four k steps: half the instructions of 8-row tiles on the N side) and the tokens on the N
-  // side.  Lane l addresses row (l & 15) of a tile and the 16-byte chunk 2 * step + (l >> 4)
-  // of the warp's 128-byte-swizzled box.
-  const uint32_t w_off = (uint32_t)(((lane & 7) + ((lane >> 3) & 1) * 8) * 128);
-  const uint32_t w_xor = (uint32_t)(lane & 7);
-  const uint32_t w_hi = (uint32_t)(lane >> 4);
-  const uint32_t bar_full0 = c.full_bar(0), bar_empty0 = c.empty_bar(0);
+  const int lane = c.lane;
   const int TP = p.sums_stride;  // token slots of the sums block: [warp][32 rows][TP]
   float* sums = c.sums();
   const bool with_res = (op.flags & F_RESIDUAL) && (!(op.flags & F_RES_RANK0) || p.rank == 0);
@@ -1199,15 +1317,11 @@ __device__ __forceinline__ void linear_pass_rows(Ctx& c, const OpDesc& op, int t
   ArgBest best;  // F_ARGMAX: lane 0 of warp t keeps the running best of token t over the CTA's rows
   best.v = -INFINITY;
   best.i = 0x7fffffff;
-  int s = (int)(c.cons_idx % (unsigned)S);
-  uint32_t parity = (c.cons_idx / (unsigned)S) & 1u;
-  unsigned consumed = 0;
   const int nch = rows_num_chunks(row0, row1);
 #pragma unroll 1
   for (int ci = 0; ci < nch; ++ci) {
     const int r0 = rows_chunk_begin(row0, row1, nch, ci);
     const int R = rows_chunk_begin(row0, row1, nch, ci + 1) - r0;
-    const int ntile = (R + 15) >> 4;  // a ragged last tile reads 8 rows of bytes behind the box: ignored rows
     // the residual of this thread's output is requested a whole chunk ahead of its use
     float res0 = 0.f;
     const bool e_live = e_row < R && e_tok < ntok && r0 + e_row < op.n;
@@ -1216,57 +1330,9 @@ __device__ __forceinline__ void linear_pass_rows(Ctx& c, const OpDesc& op, int t
       else res0 = MK_XF(op, F_GATHER_RES) ? xchg_gather1(c, xchg_cur(c), tok0 + e_tok, r0 + e_row)
                                             : __bfloat162float(__ldcg(res + (size_t)(tok0 + e_tok) * op.ld_res + r0 + e_row));
     }
-    float acc[4][4];  // [2 * tile + (k step & 1)]: two chains per tile, added up at the end
-#pragma unroll
-    for (int t = 0; t < 4; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
-    const uint32_t box_bytes = (uint32_t)R * 128u;
-#pragma unroll 1
-    for (int ks = 0; ks < nks; ++ks) {
-      if (ks == 0 && ci == 0) MK_STAMP(c, 2);
-      mbar_wait(c, bar_full0 + 8 * s, parity, ST_TIMEOUT_FULL);
-      if (arith) {
-        const uint32_t wb = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes + (uint32_t)warp * box_bytes + w_off;
-        const uint32_t xa = a_row + (a_real ? (uint32_t)(ks * kRowsStageK * 2) : 0u);
-        uint32_t x[2][4];  // x[h]: k chunks 4h .. 4h+3 of tokens 0..7: the B fragments of k steps 2h and 2h+1
-        ldmatrix_x4(xa, x[0][0], x[0][1], x[0][2], x[0][3]);
-        ldmatrix_x4(xa + (a_real ? 64u : 0u), x[1][0], x[1][1], x[1][2], x[1][3]);
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          if (t < ntile) {
-#pragma unroll
-            for (int st = 0; st < 4; ++st) {
-              uint32_t w0, w1, w2, w3;
-              ldmatrix_x4(wb + (uint32_t)t * 2048u + ((((uint32_t)(2 * st) + w_hi) ^ w_xor) << 4), w0, w1, w2, w3);
-              mma_bf16(acc[2 * t + (st & 1)], w0, w1, w2, w3, x[st >> 1][2 * (st & 1)], x[st >> 1][2 * (st & 1) + 1]);
-            }
-          }
-        }
-      }
-      __syncwarp();
-      if (lane == 0) mbar_arrive(bar_empty0 + 8 * s);
-      ++consumed;
-      if (++s == S) {
-        s = 0;
-        parity ^= 1u;
-      }
-    }
+    if (ci == 0) MK_STAMP(c, 2);
+    rows_take_sums(c, ntok, 0);
     if (ci == nch - 1) MK_STAMP(c, 3);
-    // the chunk's partial sums of this warp: rows 16t + (lane >> 2) and + 8, tokens 2 * (lane & 3) + {0, 1}
-    {
-      const int tk = 2 * (lane & 3);
-      if (tk < TP) {
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          float* d = sums + ((warp * kChunkRows + 16 * t + (lane >> 2)) * TP + tk);
-          d[0] = acc[2 * t][0] + acc[2 * t + 1][0];
-          d[8 * TP] = acc[2 * t][2] + acc[2 * t + 1][2];
-          if (tk + 1 < TP) {
-            d[1] = acc[2 * t][1] + acc[2 * t + 1][1];
-            d[8 * TP + 1] = acc[2 * t][3] + acc[2 * t + 1][3];
-          }
-        }
-      }
-    }
     consumer_sync();
     if (op.flags & F_SILU_MUL) {
       // units are [4 gate rows | 4 up rows]: the thread of a gate row also adds up its partner
@@ -1324,7 +1390,6 @@ __device__ __forceinline__ void linear_pass_rows(Ctx& c, const OpDesc& op, int t
     op.amax_idx[(size_t)(tok0 + e_tok) * op.amax_n + blockIdx.x] = best.i;
   }
   MK_STAMP(c, 4);
-  c.cons_idx += consumed;
 }
 
 __device__ __forceinline__ void op_linear_rows(Ctx& c, const OpDesc& op, int T) {
@@ -1971,7 +2036,7 @@ __device__ __forceinline__ void op_rmsnorm(Ctx& c, const OpDesc& op, int T) {
                  pre ? pre_w : nullptr);
     const uint4* xs = reinterpret_cast<const uint4*>(c.smem + c.p.x_off);
     uint4* dst = reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(op.out) + (size_t)tok * op.ld_out);
-    for (int v = c.tid; v < (op.n >> 3); v += kNumConsumers) dst[v] = xs[v];
+    for (int v = c.tid; v < (op.n >> 3); v += kNumConsumers) dst[v] = xs[x_vec(v)];
     consumer_sync();
   }
 }
@@ -2256,12 +2321,11 @@ __device__ __forceinline__ MoeWalk moe_walk(const OpDesc& op, int pairs) {
 __device__ __forceinline__ int* moe_route_ids(const Ctx& c) { return reinterpret_cast<int*>(c.smem + c.p.x_off + c.p.x_bytes - 512); }
 __device__ __forceinline__ float* moe_route_weights(const Ctx& c) { return reinterpret_cast<float*>(moe_route_ids(c) + 64); }
 
-// `rows` tagged rows of K columns -> shared memory rows of pitch kp + 8, zero padded, by all consumers: four 8-column
+// `rows` tagged rows of K columns -> rows in shared memory, zero padded, by all consumers: four 8-column
 // pieces of a thread in flight, then whatever has not arrived is polled.
 __device__ __forceinline__ void stage_ll_pairs(Ctx& c, const uint2* base, int ld, int rows, int K, int kp, unsigned tag) {
   uint4* xs = reinterpret_cast<uint4*>(c.smem + c.p.x_off);
-  const int pitch = (kp >> 3) + 1, nvec = kp >> 3, kvec = K >> 3, total = rows * nvec;
-  if (c.tid == 0) xs[rows * pitch] = make_uint4(0, 0, 0, 0);  // the chunk absent columns of the mma point at
+  const int pitch = x_pitch(kp), nvec = kp >> 3, kvec = K >> 3, total = rows * nvec;
 #pragma unroll 1
   for (int i0 = c.tid; i0 < total; i0 += 4 * kNumConsumers) {
     uint4 got[4];
@@ -2269,7 +2333,7 @@ __device__ __forceinline__ void stage_ll_pairs(Ctx& c, const uint2* base, int ld
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int i = i0 + u * kNumConsumers, r = i / nvec, v = i - r * nvec;
-      dst[u] = i < total ? r * pitch + v : -1;
+      dst[u] = i < total ? r * pitch + x_vec(v) : -1;
       at[u] = i < total && v < kvec ? r * (ld >> 3) + v : -1;
     }
     ll_take(c, reinterpret_cast<const uint4*>(base), at, tag, got);
@@ -2347,78 +2411,23 @@ __device__ __forceinline__ void op_moe_linear(Ctx& c, const OpDesc& op, int T) {
   if (!ll)
     stage_x(c, reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)in_first * op.ld_in, op.ld_in, op.k, kp,
             (op.flags & F_NORM_IN) ? op.norm_w : nullptr, 0, nrows, nrows, nullptr);
-  const int S = p.num_stages;
-  const int lane = c.lane, warp = c.warp;
-  const int pitch_b = (kp + 8) * 2;
-  const uint32_t xs0 = c.smem_addr + p.x_off;
-  const uint32_t x_zero = xs0 + (uint32_t)(nrows * pitch_b);
-  const uint32_t w_off = (uint32_t)(((lane & 7) + ((lane >> 3) & 1) * 8) * 128);
-  const uint32_t w_xor = (uint32_t)(lane & 7);
-  const uint32_t w_hi = (uint32_t)(lane >> 4);
-  const uint32_t bar_full0 = c.full_bar(0), bar_empty0 = c.empty_bar(0);
+  rows_x_ready(c);
   const int TP = p.sums_stride;
   float* sums = c.sums();
   __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out);
   const int e_row = c.tid & 31;
-  int s = (int)(c.cons_idx % (unsigned)S);
-  uint32_t parity = (c.cons_idx / (unsigned)S) & 1u;
   int half = 0;
-  unsigned consumed = 0;
 #pragma unroll 1
   for (int pr = p_first; pr <= p_last; ++pr) {
     const int seg0 = max(wk.row0, pr * wk.n), seg1 = min(wk.row1, (pr + 1) * wk.n);
     const int nch = rows_num_chunks(seg0, seg1);
-    // the B operand of the mma: column 0 = the pair's input row, the other seven columns zero
-    const int xrow = (pair_in ? pr : pr / topk) - in_first;
-    const bool a_real = (lane & 7) == 0;
-    const uint32_t a_row = a_real ? xs0 + (uint32_t)(xrow * pitch_b + (lane >> 3) * 16 + warp * 128) : x_zero;
 #pragma unroll 1
     for (int ci = 0; ci < nch; ++ci) {
       const int r0 = rows_chunk_begin(seg0, seg1, nch, ci);
       const int R = rows_chunk_begin(seg0, seg1, nch, ci + 1) - r0;
-      const int ntile = (R + 15) >> 4;
-      float acc[4][4];
-#pragma unroll
-      for (int t = 0; t < 4; ++t) acc[t][0] = acc[t][1] = acc[t][2] = acc[t][3] = 0.f;
-      const uint32_t box_bytes = (uint32_t)R * 128u;
-#pragma unroll 1
-      for (int ks = 0; ks < nks; ++ks) {
-        mbar_wait(c, bar_full0 + 8 * s, parity, ST_TIMEOUT_FULL);
-        const uint32_t wb = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes + (uint32_t)warp * box_bytes + w_off;
-        const uint32_t xa = a_row + (a_real ? (uint32_t)(ks * kRowsStageK * 2) : 0u);
-        uint32_t x[2][4];
-        ldmatrix_x4(xa, x[0][0], x[0][1], x[0][2], x[0][3]);
-        ldmatrix_x4(xa + (a_real ? 64u : 0u), x[1][0], x[1][1], x[1][2], x[1][3]);
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          if (t < ntile) {
-#pragma unroll
-            for (int st = 0; st < 4; ++st) {
-              uint32_t w0, w1, w2, w3;
-              ldmatrix_x4(wb + (uint32_t)t * 2048u + ((((uint32_t)(2 * st) + w_hi) ^ w_xor) << 4), w0, w1, w2, w3);
-              mma_bf16(acc[2 * t + (st & 1)], w0, w1, w2, w3, x[st >> 1][2 * (st & 1)], x[st >> 1][2 * (st & 1) + 1]);
-            }
-          }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(bar_empty0 + 8 * s);
-        ++consumed;
-        if (++s == S) {
-          s = 0;
-          parity ^= 1u;
-        }
-      }
-      // column 0 of the accumulators (lanes with (lane & 3) == 0): rows 16t + (lane >> 2) and + 8.  Consecutive chunks
-      // take turns in the two token slots of the sums block: one CTA-wide sync per chunk.
+      // Consecutive chunks take turns in the two token slots of the sums block: one CTA-wide sync per chunk.
       half ^= 1;
-      if ((lane & 3) == 0) {
-#pragma unroll
-        for (int t = 0; t < 2; ++t) {
-          float* d = sums + ((warp * kChunkRows + 16 * t + (lane >> 2)) * TP) + half;
-          d[0] = acc[2 * t][0] + acc[2 * t + 1][0];
-          d[8 * TP] = acc[2 * t][2] + acc[2 * t + 1][2];
-        }
-      }
+      rows_take_sums(c, 1, half);
       consumer_sync();
       if (c.warp == 0) {
         float v = 0.f;
@@ -2446,7 +2455,6 @@ __device__ __forceinline__ void op_moe_linear(Ctx& c, const OpDesc& op, int T) {
       }
     }
   }
-  c.cons_idx += consumed;
 }
 
 // The down projection of the experts with the weighted sum folded in (F_MOE_COMBINE).  A CTA owns a range of the n
@@ -2464,15 +2472,6 @@ __device__ __forceinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, in
   if (!any || row0 >= row1) return;
   const int nks = op.nkt;
   const int kp = nks * kRowsStageK;
-  const int S = p.num_stages;
-  const int lane = c.lane, warp = c.warp;
-  const int pitch_b = (kp + 8) * 2;
-  const uint32_t xs0 = c.smem_addr + p.x_off;
-  const uint32_t x_zero = xs0 + (uint32_t)(topk * pitch_b);
-  const uint32_t w_off = (uint32_t)(((lane & 7) + ((lane >> 3) & 1) * 8) * 128);
-  const uint32_t w_xor = (uint32_t)(lane & 7);
-  const uint32_t w_hi = (uint32_t)(lane >> 4);
-  const uint32_t bar_full0 = c.full_bar(0), bar_empty0 = c.empty_bar(0);
   const int TP = p.sums_stride;  // 2
   float* sums = c.sums();
   const bool torch_num = p.numerics == NUM_TORCH;
@@ -2480,20 +2479,16 @@ __device__ __forceinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, in
   const __nv_bfloat16* res = reinterpret_cast<const __nv_bfloat16*>(op.res);
   __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out);
   const int e_row = c.tid & 31;
-  int s = (int)(c.cons_idx % (unsigned)S);
-  uint32_t parity = (c.cons_idx / (unsigned)S) & 1u;
-  unsigned consumed = 0;
   const int nch = rows_num_chunks(row0, row1);
 #pragma unroll 1
   for (int t = 0; t < T; ++t) {
     if (ll) stage_ll_pairs(c, reinterpret_cast<const uint2*>(op.ll_in) + (size_t)t * topk * (size_t)(op.ld_in >> 1), op.ld_in, topk, op.k, kp, ll_tag_of(c, op.ll_in_op));
     else stage_x(c, reinterpret_cast<const __nv_bfloat16*>(op.in) + (size_t)t * topk * op.ld_in, op.ld_in, op.k, kp, nullptr, 0, topk, topk, nullptr);
+    rows_x_ready(c);
 #pragma unroll 1
     for (int ci = 0; ci < nch; ++ci) {
       const int r0 = rows_chunk_begin(row0, row1, nch, ci);
       const int R = rows_chunk_begin(row0, row1, nch, ci + 1) - r0;
-      const int ntile = (R + 15) >> 4;
-      const uint32_t box_bytes = (uint32_t)R * 128u;
       float comb = 0.f;  // (threads 0..R-1: the running weighted sum of output row r0 + tid)
       float rr = 0.f;
       if (c.tid < R && res != nullptr)
@@ -2501,47 +2496,8 @@ __device__ __forceinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, in
                                    : __bfloat162float(__ldcg(res + (size_t)t * op.ld_res + r0 + e_row));
 #pragma unroll 1
       for (int sl = 0; sl < topk; ++sl) {
-        const bool a_real = (lane & 7) == 0;
-        const uint32_t a_row = a_real ? xs0 + (uint32_t)(sl * pitch_b + (lane >> 3) * 16 + warp * 128) : x_zero;
-        float acc[4][4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) acc[q][0] = acc[q][1] = acc[q][2] = acc[q][3] = 0.f;
-#pragma unroll 1
-        for (int ks = 0; ks < nks; ++ks) {
-          mbar_wait(c, bar_full0 + 8 * s, parity, ST_TIMEOUT_FULL);
-          const uint32_t wb = c.smem_addr + (uint32_t)s * (uint32_t)p.stage_bytes + (uint32_t)warp * box_bytes + w_off;
-          const uint32_t xa = a_row + (a_real ? (uint32_t)(ks * kRowsStageK * 2) : 0u);
-          uint32_t x[2][4];
-          ldmatrix_x4(xa, x[0][0], x[0][1], x[0][2], x[0][3]);
-          ldmatrix_x4(xa + (a_real ? 64u : 0u), x[1][0], x[1][1], x[1][2], x[1][3]);
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            if (q < ntile) {
-#pragma unroll
-              for (int st = 0; st < 4; ++st) {
-                uint32_t w0, w1, w2, w3;
-                ldmatrix_x4(wb + (uint32_t)q * 2048u + ((((uint32_t)(2 * st) + w_hi) ^ w_xor) << 4), w0, w1, w2, w3);
-                mma_bf16(acc[2 * q + (st & 1)], w0, w1, w2, w3, x[st >> 1][2 * (st & 1)], x[st >> 1][2 * (st & 1) + 1]);
-              }
-            }
-          }
-          __syncwarp();
-          if (lane == 0) mbar_arrive(bar_empty0 + 8 * s);
-          ++consumed;
-          if (++s == S) {
-            s = 0;
-            parity ^= 1u;
-          }
-        }
         const int half = sl & 1;
-        if ((lane & 3) == 0) {
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            float* d = sums + ((warp * kChunkRows + 16 * q + (lane >> 2)) * TP) + half;
-            d[0] = acc[2 * q][0] + acc[2 * q + 1][0];
-            d[8 * TP] = acc[2 * q][2] + acc[2 * q + 1][2];
-          }
-        }
+        rows_take_sums(c, 1, half);
         consumer_sync();
         if (c.tid < R) {
           float v = 0.f;
@@ -2567,7 +2523,6 @@ __device__ __forceinline__ void op_moe_down_combine(Ctx& c, const OpDesc& op, in
       consumer_sync();  // (the next chunk's or token's first slot writes the half the last slot may still be read from)
     }
   }
-  c.cons_idx += consumed;
 }
 
 // aux0 = top-k.  in: [T * top-k, n] bf16, amax_val: routing weights [T, top-k], res: [T, n] (may be null), out: [T, n].
@@ -2977,7 +2932,7 @@ __device__ __forceinline__ void producer_loop(Ctx& c) {
                     mbar_arrive_expect_tx(full, 8u * box_bytes);
 #pragma unroll
                     for (int j = 0; j < 8; ++j)
-                      tma_load_2d_hint(dst + (uint32_t)j * box_bytes, tmap, full, ks * kRowsStageK + j * kBoxK, wrow, pol_stream);
+                      tma_load_2d_hint(dst + (uint32_t)(j * kRowsBoxBytes), tmap, full, ks * kRowsStageK + j * kBoxK, wrow, pol_stream);
                     issued += 1;
                     fl[1] = (int)issued;
                     if (++s == S) {
@@ -3013,8 +2968,8 @@ __device__ __forceinline__ void producer_loop(Ctx& c) {
                 mbar_arrive_expect_tx(full, 8u * box_bytes);
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
-                  if (silu) tma_load_3d_hint(dst + (uint32_t)j * box_bytes, tmap, full, ks * kRowsStageK + j * kBoxK, (r0 - pr * wk.n) >> 1, 2 * expert, pol_stream);
-                  else tma_load_2d_hint(dst + (uint32_t)j * box_bytes, tmap, full, ks * kRowsStageK + j * kBoxK, wrow, pol_stream);
+                  if (silu) tma_load_3d_hint(dst + (uint32_t)(j * kRowsBoxBytes), tmap, full, ks * kRowsStageK + j * kBoxK, (r0 - pr * wk.n) >> 1, 2 * expert, pol_stream);
+                  else tma_load_2d_hint(dst + (uint32_t)(j * kRowsBoxBytes), tmap, full, ks * kRowsStageK + j * kBoxK, wrow, pol_stream);
                 issued += 1;
                 fl[1] = (int)issued;
                 if (++s == S) {
@@ -3053,7 +3008,7 @@ __device__ __forceinline__ void producer_loop(Ctx& c) {
               mbar_arrive_expect_tx(full, 8u * box_bytes);
 #pragma unroll
               for (int j = 0; j < 8; ++j)
-                tma_load_2d_hint(dst + (uint32_t)j * box_bytes, tmap, full, ks * kRowsStageK + j * kBoxK, r0, pol_stream);
+                tma_load_2d_hint(dst + (uint32_t)(j * kRowsBoxBytes), tmap, full, ks * kRowsStageK + j * kBoxK, r0, pol_stream);
               issued += 1;
               fl[1] = (int)issued;
               if (++s == S) {
@@ -3102,6 +3057,117 @@ __device__ __forceinline__ void producer_loop(Ctx& c) {
   }
   fl[1] = (int)issued;
 }
+
+#if MK_NC == 0
+// ------------------------------------------------------------------------------------
+// the MMA issuer of the row-owner path (one elected lane of warp 10)
+// ------------------------------------------------------------------------------------
+// Walks the chunks in the consumers' order; see linear_pass_rows for the operands and WeightRing for what happens while the token
+// rows are not there.
+__device__ __forceinline__ void rows_mma_loop(Ctx& c) {
+  const KParams& p = c.p;
+  volatile int* fl = c.flags();
+  WeightRing ring(c, kRowsSlots, c.tmem + 2 * kRowsAccCols);
+  // instruction descriptor: D = f32, A = B = bf16, both K-major, N = 16, M = 128
+  const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((16u >> 3) << 17) | ((128u >> 4) << 24);
+  unsigned runs = 0;  // chunks started
+  uint32_t x_parity = 0;
+  const uint32_t x0 = c.smem_addr + p.x_off;
+  const bool arith = !(p.debug_flags & 1);
+  bool dead = false;
+  // one chunk: the token row (or two, `second` bytes apart) at x
+  auto chunk = [&](uint32_t x, uint32_t second, int nks) {
+    if (!ring.wait(c.acc_empty_bar(runs & 1), ((runs >> 1) & 1u) ^ 1u)) return false;
+    const uint32_t d0 = c.tmem + (runs & 1u) * kRowsAccCols;
+    uint64_t bd = umma_smem_desc(x, second);
+#pragma unroll 1
+    for (int ks = 0; ks < nks; ++ks) {
+      if (!ring.wait_tile()) return false;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t more = ks > 0 ? 1u : 0u;
+      if (ring.held == 0) {
+        const uint64_t ad = umma_smem_desc(ring.stage());
+        if (arith)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int k16 = 0; k16 < 4; ++k16)
+              umma_bf16(d0 + 32 * h + 16 * (k16 & 1), ad + (uint64_t)(h * (kSubBytes >> 4) + 2 * k16), bd + (uint64_t)(2 * k16), idesc, k16 < 2 ? more : 1u);
+        ring.free_stage();
+      } else {
+        const uint32_t at = ring.slot();
+        if (arith)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int k16 = 0; k16 < 4; ++k16)
+              umma_bf16_ta(d0 + 32 * h + 16 * (k16 & 1), at + 32 * h + 8 * k16, bd + (uint64_t)(2 * k16), idesc, k16 < 2 ? more : 1u);
+        ring.free_slot();
+      }
+      bd += 1024 >> 4;
+    }
+    umma_commit(c.acc_full_bar(runs & 1));
+    ++runs;
+    return true;
+  };
+  for (int iter = 1; !dead; ++iter) {
+    int go;
+    if (!wait_go(c, fl, iter, go)) break;
+    const int T = go & 255;
+    for (int oi = 0; oi < p.num_ops && !dead; ++oi) {
+      const OpDesc& op = p.ops[oi];
+      const int nks = op.nkt;
+      const uint32_t row_bytes = (uint32_t)nks * 1024u;
+      // groups of chunks on the same staged rows; chunks of a group (in a MoE linear: of each of its pairs, on the pair's row or its
+      // token's); the down projection goes chunk by chunk, slot by slot
+      int groups, chunks = 0, first = 0, last = 0;
+#if MK_WITH_MOE
+      MoeWalk wk;
+      const bool pairs = op.type == OP_MOE_LINEAR && !(op.flags & F_MOE_COMBINE), slots = op.type == OP_MOE_LINEAR && !pairs;
+      if (pairs) {
+        wk = moe_walk(op, T * op.aux0);
+        if (!wk.any || wk.row0 >= wk.row1) continue;
+        groups = 1;
+        first = wk.row0 / wk.n;
+        last = (wk.row1 - 1) / wk.n;
+      } else
+#else
+      constexpr bool slots = false;
+#endif
+      {
+        if (op.type != OP_LINEAR && !slots) continue;
+        int row0, row1;
+        bool any;
+        rows_range(op, row0, row1, any);
+        if (!any) continue;
+        chunks = rows_num_chunks(row0, row1) * (slots ? op.aux0 : 1);
+        groups = slots ? T : linear_passes(op, T);
+      }
+      for (int g = 0; g < groups && !dead; ++g) {
+        dead = !ring.wait(c.xfull_bar(0), x_parity, ring.S - 1);
+        x_parity ^= 1u;
+        // (of one token the columns of a second hold whatever lies behind the stage's slices)
+        const uint32_t second = op.type == OP_LINEAR && min(op.aux3, T - g * op.aux3) > 1 ? row_bytes : 1024u;
+        for (int pr = first; pr <= last && !dead; ++pr) {
+          uint32_t x = x0;
+#if MK_WITH_MOE
+          if (pairs) {
+            chunks = rows_num_chunks(max(wk.row0, pr * wk.n), min(wk.row1, (pr + 1) * wk.n));
+            x += (uint32_t)((op.flags & F_MOE_PAIR_IN) ? pr - first : pr / op.aux0 - first / op.aux0) * row_bytes;
+          }
+#endif
+          for (int i = 0; i < chunks && !dead; ++i) dead = !chunk(slots ? x + (uint32_t)(i % op.aux0) * row_bytes : x, second, nks);
+        }
+      }
+    }
+    if (p.mode == MODE_ONEPASS) break;
+  }
+  // nothing of this thread may be in flight when the tensor memory is given back
+  umma_commit(c.done_bar());
+  mbar_wait(c, c.done_bar(), 0u, ST_TIMEOUT_FULL);
+  fl[5] = (int)ring.taken;
+}
+#endif
 
 // Arrivals that complete a stage's activation boxes: the 32 lanes of the norm warp where an instance has one (a box that needs no
 // norm is arrived at 32 times by its producer), else the producer's.
@@ -3198,7 +3264,6 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
   c.cl_rank = 0;
   if (c.cl_size > 1) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(c.cl_rank));
 #endif
-  c.cons_idx = 0;
   c.arrived = false;
   c.attn_iter = -1;
   c.tmem = 0u;
@@ -3217,8 +3282,8 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
   if (threadIdx.x == 0) {
     for (int s = 0; s < kMaxStages; ++s) {
       mbar_init(c.full_bar(s), 1);
-      mbar_init(c.empty_bar(s), PATH == PATH_WIDE ? 1 : kNumConsumerWarps);  // the commit behind what read the stage, or every consumer warp
-      mbar_init(c.xfull_bar(s), kBoxArrivals);
+      mbar_init(c.empty_bar(s), 1);  // the commit behind what read the stage
+      mbar_init(c.xfull_bar(s), PATH == PATH_WIDE ? kBoxArrivals : kNumConsumerWarps);
       mbar_init(c.xempty_bar(s), 1);
       mbar_init(c.xraw_bar(s), 1);
       mbar_init(c.tfree_bar(s), 1);
@@ -3250,18 +3315,15 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
   }
 #endif
   // All of the tensor memory (the CTA has its SM to itself), allocated once by warp 0 and freed by it when the CTA leaves: two
-  // buffers of x_rows columns of fp32 accumulators, then slots of the weight ring.
-  constexpr bool use_tmem = PATH == PATH_WIDE;
-  if (use_tmem) {
-    if (c.warp == 0) {
-      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(c.tmem_slot()), "n"(kTmemCols) : "memory");
-      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    c.tmem = *reinterpret_cast<volatile uint32_t*>(c.smem + p.bar_off + kFlagsOff + 72);
+  // sets of fp32 accumulators, then slots of the weight ring.
+  if (c.warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(c.tmem_slot()), "n"(kTmemCols) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  c.tmem = *reinterpret_cast<volatile uint32_t*>(c.smem + p.bar_off + kFlagsOff + 72);
 
   if (c.warp >= kNumConsumerWarps) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(service_regs(NC)));
@@ -3276,10 +3338,12 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
       } else {
         if (c.lane == 0) xproducer_loop(c);
       }
-    } else if (PATH == PATH_WIDE && c.warp == kNumConsumerWarps + 2) {
-      if constexpr (PATH == PATH_WIDE) {
-        if (elect_one()) mma_loop(c);
-      }
+    } else if (c.warp == kNumConsumerWarps + 2) {
+#if MK_NC == 0
+      if (elect_one()) rows_mma_loop(c);
+#else
+      if (elect_one()) mma_loop(c);
+#endif
     } else {
       if constexpr (PATH == PATH_WIDE && 2 * NC <= kNormBoxRows) norm_loop(c);
     }
@@ -3428,12 +3492,12 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
   // no CTA may exit with a bulk copy still writing its shared memory
   if (threadIdx.x == 0) {
     const unsigned issued = (unsigned)fl[1];
-    for (unsigned i = PATH == PATH_WIDE ? (unsigned)fl[5] : c.cons_idx; i < issued; ++i)
+    for (unsigned i = (unsigned)fl[5]; i < issued; ++i)
       mbar_wait(c, c.full_bar(i % p.num_stages), (i / p.num_stages) & 1, ST_TIMEOUT_FULL);
   }
   __syncthreads();
-  if (use_tmem && c.warp == 0) {
-    // (the MMA issuer has waited for everything it had in flight)
+  if (c.warp == 0) {
+    // (the tcgen05 issuer has waited for everything it had in flight)
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(c.tmem), "n"(kTmemCols) : "memory");
   }

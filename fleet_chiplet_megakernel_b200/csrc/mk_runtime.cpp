@@ -39,7 +39,7 @@ constexpr int kRedBytes = 2048;    // small scratch (reductions, argmax, sequenc
 constexpr int kFastSmem = 166912 - kParamSmem;  // 164 KB carve-out minus the 1 KB the system reserves per CTA
 constexpr int kRowsSumsBytes = mk::kNumConsumerWarps * mk::kChunkRows * 2 * 4;  // [warp][32 rows][2 tokens] floats
 // Token rows a row-owner CTA may keep resident: 61,696 bytes, two rows of 15,360 columns.  They leave the ring four stages of
-// the 227 KB of a CTA, and five up to 60,672 bytes (one row in place of two would buy a stage for two passes over the weights).
+// the 227 KB of a CTA.
 constexpr int kRowsXBudget = kFastSmem - 2048 - kRedBytes - kRowsSumsBytes - 3 * mk::kStageBytes;
 constexpr int kAttnMaxChunks = 32;
 constexpr int kGateUpUnit = 4;     // fused gate/up weights are laid out [4 gate | 4 up] per 8-row unit
@@ -58,10 +58,11 @@ int wide_stages(int tokens, int x_bytes) {
   return fast >= 2 ? fast : std::min(2, (kMaxSmem - kWideFixed - x_bytes) / wide_stage_bytes(tokens));
 }
 
-// Row-owner path: five stages where they fit beside the resident rows.  12 layers of 8B width, us per step with 4 and 5 stages:
-// one request 1119 and 1109; two requests, 3, 4 and 5: 1238, 1172, 1166.
+// Row-owner path: four stages.  What a fifth and a sixth take is L1, and the slots of tensor memory hold six more.  Us per step with
+// 3, 4 and 5: one request of 12 layers of 8B width 1050, 1020, 1025, two 1089, 1055, 1062; 2048 hidden 500, 489, 493; 8 MoE
+// layers 554, 554, 565, two requests 700, 693, 713.  With 6 one request as with 5, 2048 hidden 505, 8 MoE layers 577.
 constexpr int kRowsFixed = 1024 /*alignment slack*/ + kRowsSumsBytes + kRedBytes + kBarDescBytes;
-int rows_stages(int x_bytes) { return std::min((kMaxSmem - kRowsFixed - x_bytes) / mk::kStageBytes, 5); }
+int rows_stages(int x_bytes) { return std::min((kMaxSmem - kRowsFixed - x_bytes) / mk::kStageBytes, 4); }
 // Page numbers that the scheduler can keep in shared memory while it rewrites the page table: between two iterations the weight
 // ring in front of the x region is empty, so the table has both (MoE programs keep expert ids in the last 512 bytes).
 int page_entries(int ring_bytes, int x_bytes, bool moe) { return (ring_bytes + x_bytes - (moe ? 512 : 0)) / 4; }

@@ -25,12 +25,13 @@ constexpr int kNumConsumers = kNumConsumerWarps * 32;
 // MMA issuer and the norm warp.  The block starts with kLaunchRegs registers a thread; the service warps hand theirs to the
 // consumers (their sum is what the block was launched with; an instance that is compiled to fewer is not launched).  The
 // instances with a norm warp, up to 32 token rows, leave it 72: with 56 it has two rows in flight instead of four (12 layers of 8B
-// width, us per step: 32 requests 1520 and 1421, 8 requests 1249 and 1237); the others have consumers that would spill with 216.
+// width, us per step: 32 requests 1520 and 1421, 8 requests 1249 and 1237).  On the row-owner path the MoE build's issuer would
+// spill with 56, beyond 32 token rows the consumers with 216.
 constexpr int kNumThreads = kNumConsumers + 128;
 constexpr int kLaunchRegs = 168;
-__host__ __device__ constexpr int service_regs(int nc) { return nc == 8 || nc == 16 ? 72 : 56; }  // (nc: MK_NC of the instance)
+__host__ __device__ constexpr int service_regs(int nc) { return nc == 32 ? 56 : 72; }  // (nc: MK_NC of the instance)
 __host__ __device__ constexpr int consumer_regs(int nc) { return (kNumThreads * kLaunchRegs - 128 * service_regs(nc)) / kNumConsumers; }
-static_assert(consumer_regs(0) == 224 && consumer_regs(8) == 216, "register counts in steps of eight, no more than the block has");
+static_assert(consumer_regs(32) == 224 && consumer_regs(8) == 216, "register counts in steps of eight, no more than the block has");
 constexpr int kWideRedBytes = 4096;              // scratch of the wide path: reductions and the iteration's token table
 constexpr int kHeadDim = 128;
 // Widest activation box that the norm is applied to in shared memory: what one warp normalises in the time a weight stage takes
@@ -48,13 +49,17 @@ constexpr int kRowsStageK = 512;
 // Tensor memory: 512 columns of 128 lanes x 4 bytes.  A slot holds a stage's 32 KB of weights.
 constexpr int kTmemCols = 512;
 constexpr int kSlotCols = 64;
+constexpr int kRowsBoxBytes = kChunkRows * kBoxK * 2;  // row-owner path: boxes of a stage lie 4 KB apart, however many of their 32 rows there are
+// Row-owner path: two sets of four accumulators of 16 columns, then slots.
+constexpr int kRowsAccCols = 64;
+constexpr int kRowsSlots = (kTmemCols - 2 * kRowsAccCols) / kSlotCols;
 // Slots of the wide path's weight ring behind two accumulator buffers of x_rows columns: 7 up to 32 token rows, 6 up to 64, 4 beyond.
 __host__ __device__ constexpr int wide_slots(int x_rows) { return (kTmemCols - 2 * x_rows) / kSlotCols; }
 // mbarriers of a CTA: six groups of kMaxStages (see Ctx in mk_kernel.cu), then flags and the single ones
 constexpr int kMaxStages = 8;
 constexpr int kFlagsOff = 6 * kMaxStages * 8;
 constexpr int kBarBytes = kFlagsOff + 192;
-static_assert(wide_slots(16) <= kMaxStages, "a barrier per slot");
+static_assert(wide_slots(16) <= kMaxStages && kRowsSlots <= kMaxStages, "a barrier per slot");
 
 enum OpType : int {
   OP_EMBED = 1,

@@ -15,21 +15,6 @@
 // ------------------------------------------------------------------------------------
 // tcgen05
 // ------------------------------------------------------------------------------------
-// the same with A in tensor memory: 16 k-elements of 128 rows are eight columns
-__device__ __forceinline__ void umma_bf16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-__device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // NC (8, 16 or 32) accumulator columns of this warp's 32 lanes; the caller waits with tmem_wait_ld
 template <int NC>
 __device__ __forceinline__ void tmem_ld(uint32_t taddr, uint32_t (&r)[NC]) {
@@ -153,70 +138,19 @@ __device__ __forceinline__ bool wait_lin(const Ctx& c, volatile int* fl, int wor
   return true;
 }
 
-// Weights depend on nobody, so between two ops the ring fills up and HBM would idle until the first activations arrive: split
-// sums, a barrier, a round trip for the boxes, 8 to 18 us around an attention op, of which three or four stages of the ring are 2 to
-// 3.  So when all stages of the ring have landed and there is nothing to multiply, the oldest goes into a slot of tensor memory
-// (tcgen05.cp, 0.27 us) and its stage is loaded again: 7 slots of 32 KB up to 32 token rows, 6 up to 64, 4 beyond.  Tiles are
-// multiplied in order, those set aside with A in tensor memory.  While boxes are there nothing is set aside: every tile through
-// tensor memory streams at 1.16 us a tile instead of 0.69 (copies and products take turns on the same pipe).
-// 12 layers of 8B width, us per step, without the slots and with them: 8 requests 1303 and 1249, 64 requests 1732 and 1680.
-//
-// The issuer is an elected lane, not lane 0: behind elect.sync the compiler issues tcgen05 from uniform registers.  Eight products
-// of a tile and a commit take 400 cycles instead of 920, of the 1350 in which HBM delivers a tile (128 x 16 x 16 each, the same up
-// to 64 columns); the step at 8 requests fell from 1392 to 1303 us with it, and setting aside pays only since.
+// See WeightRing for the tiles that wait in tensor memory, 7 up to 32 token rows, 6 up to 64, 4 beyond.
 __device__ __forceinline__ void mma_loop(Ctx& c) {
   const KParams& p = c.p;
-  const int S = p.num_stages, N = p.x_rows, slots = wide_slots(N);
+  const int S = p.num_stages, N = p.x_rows;
+  WeightRing ring(c, wide_slots(N), c.tmem + 2u * (uint32_t)N);
   volatile int* fl = c.flags();
   const uint32_t x_sub = (uint32_t)N * 128u;  // bytes of one activation box
-  const uint32_t slot0 = c.tmem + 2u * (uint32_t)N;
   // instruction descriptor: D = f32, A = B = bf16, both K-major, N >> 3, M >> 4
   const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((128u >> 4) << 24);
-  int s = 0, xs = 0;               // next stage of weights, of activation boxes
-  uint32_t parity = 0, xparity = 0;
-  int head = 0, tail = 0, held = 0;  // slots: the oldest tile, the next to fill, tiles held
-  uint32_t tail_parity = 1;
-  unsigned taken = 0, runs = 0;  // stages taken from the ring; accumulator runs started
-  auto set_aside = [&]() {
-    const int newest = s == 0 ? S - 1 : s - 1;
-    // (the oldest and the newest stage: copies may land out of order)
-    if (held == slots || !mbar_test_wait(c.full_bar(s), parity) || !mbar_test_wait(c.full_bar(newest), s == 0 ? parity : parity ^ 1u) ||
-        !mbar_test_wait(c.tfree_bar(tail), tail_parity)) return;
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t src = c.smem_addr + (uint32_t)s * (uint32_t)kStageBytes, dst = slot0 + (uint32_t)(tail * kSlotCols);
-    tmem_put_128x64(dst, src);
-    tmem_put_128x64(dst + 32u, src + kSubBytes);
-    umma_commit(c.empty_bar(s));
-    ++held;
-    ++taken;
-    if (++tail == slots) {
-      tail = 0;
-      tail_parity ^= 1u;
-    }
-    if (++s == S) {
-      s = 0;
-      parity ^= 1u;
-    }
-  };
-  // A bounded wait that sets tiles aside meanwhile.
-  auto ready = [&](uint32_t bar, uint32_t par, bool wait) {
-    unsigned long long since = 0;
-    unsigned polls = 0;
-    while (wait && !mbar_try_wait_for(bar, par, 200u)) {
-      set_aside();
-      if (((++polls) & 1023u) == 0) {
-        if (aborted(c)) return false;
-        const unsigned long long now = globaltimer();
-        if (since == 0) {
-          since = now;
-        } else if (now - since > 4 * p.timeout_ns) {
-          raise_abort(c, ST_TIMEOUT_FULL, (int)bar, (int)par);
-          return false;
-        }
-      }
-    }
-    return true;
-  };
+  const int flying = N <= 32 ? 1 : 0;
+  int xs = 0;  // next stage of activation boxes
+  uint32_t xparity = 0;
+  unsigned runs = 0;  // accumulator runs started
   bool dead = false;
   for (int iter = 1; !dead; ++iter) {
     int go;
@@ -231,15 +165,14 @@ __device__ __forceinline__ void mma_loop(Ctx& c) {
       int kt = (int)(t0 % (unsigned)nkt);
       bool fresh = true;
       for (unsigned tile = t0; tile < t1; ++tile) {
-        if (!ready(c.acc_empty_bar(runs & 1), ((runs >> 1) & 1u) ^ 1u, fresh) || !ready(c.xfull_bar(xs), xparity, true) ||
-            (held == 0 && !mbar_wait(c, c.full_bar(s), parity, ST_TIMEOUT_FULL))) {
+        if ((fresh && !ring.wait(c.acc_empty_bar(runs & 1), ((runs >> 1) & 1u) ^ 1u)) || !ring.wait(c.xfull_bar(xs), xparity, flying) || !ring.wait_tile()) {
           dead = true;
           break;
         }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t d = c.tmem + (runs & 1u) * (uint32_t)N, xt = c.xbox(xs);
-        if (held == 0) {  // straight from shared memory
-          const uint32_t st = c.smem_addr + (uint32_t)s * (uint32_t)kStageBytes;
+        if (ring.held == 0) {  // straight from shared memory
+          const uint32_t st = ring.stage();
 #pragma unroll
           for (int sub = 0; sub < kSubTiles; ++sub) {
             const uint64_t ad = umma_smem_desc(st + (uint32_t)sub * kSubBytes);
@@ -248,14 +181,9 @@ __device__ __forceinline__ void mma_loop(Ctx& c) {
             for (int k16 = 0; k16 < 4; ++k16)  // 16 k-elements = 32 bytes further inside the swizzle span: +2 in the address field
               umma_bf16(d, ad + (uint64_t)(2 * k16), bd + (uint64_t)(2 * k16), idesc, (fresh && sub == 0 && k16 == 0) ? 0u : 1u);
           }
-          umma_commit(c.empty_bar(s));
-          ++taken;
-          if (++s == S) {
-            s = 0;
-            parity ^= 1u;
-          }
+          ring.free_stage();
         } else {
-          const uint32_t at = slot0 + (uint32_t)(head * kSlotCols);
+          const uint32_t at = ring.slot();
 #pragma unroll
           for (int sub = 0; sub < kSubTiles; ++sub) {
             const uint64_t bd = umma_smem_desc(xt + (uint32_t)sub * x_sub);
@@ -263,9 +191,7 @@ __device__ __forceinline__ void mma_loop(Ctx& c) {
             for (int k16 = 0; k16 < 4; ++k16)
               umma_bf16_ta(d, at + 32u * sub + 8u * k16, bd + (uint64_t)(2 * k16), idesc, (fresh && sub == 0 && k16 == 0) ? 0u : 1u);
           }
-          umma_commit(c.tfree_bar(head));
-          if (++head == slots) head = 0;
-          --held;
+          ring.free_slot();
         }
         umma_commit(c.xempty_bar(xs));
         if (++xs == S) {
@@ -286,7 +212,7 @@ __device__ __forceinline__ void mma_loop(Ctx& c) {
   // nothing of this thread may be in flight when the tensor memory is given back
   umma_commit(c.done_bar());
   mbar_wait(c, c.done_bar(), 0u, ST_TIMEOUT_FULL);
-  fl[5] = (int)taken;
+  fl[5] = (int)ring.taken;
 }
 
 // ------------------------------------------------------------------------------------

@@ -9,9 +9,11 @@ pytestmark = pytest.mark.gpu
 BF = torch.bfloat16
 
 
-# 48 x 48 tiles are 15 or 16 for each of 148 CTAs; ring and slots hold 11 up to 16 token rows, 10 up to 32, 9 up to 64, 6 beyond
-@pytest.mark.parametrize("T", [3, 16, 17, 32, 33, 64, 65, 128])
-@pytest.mark.parametrize("N,K", [(6144, 6144), (6152, 6120)])
+# 48 x 48 tiles are 15 or 16 for each of 148 CTAs; ring and slots hold 11 up to 16 token rows, 10 up to 32, 9 up to 64, 6 beyond.
+# One and two tokens: a CTA's 8-row units make chunks of 8 to 32 rows (1 to 5 units and more), stages of 512 k are whole, ragged and
+# one; two rows of 16384 columns go in two passes.
+@pytest.mark.parametrize("T,N,K", [(T, N, K) for T in (3, 16, 17, 32, 33, 64, 65, 128) for N, K in ((6144, 6144), (6152, 6120))] +
+                         [(T, N, K) for T in (1, 2) for N, K in ((6144, 6144), (6152, 6120), (8, 512), (1192, 136), (2376, 520), (3560, 1096), (16384, 512), (4736, 4744))])
 def test_chained_linears_multiply_their_tiles_in_order(T, N, K):
     """Small whole numbers: every sum is exact in fp32, in any order, and so is its rounding to bf16; a tile out of place or
     overwritten early changes the outputs."""
