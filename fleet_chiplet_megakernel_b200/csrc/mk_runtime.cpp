@@ -1589,15 +1589,15 @@ static int compile_program(mk_handle* h, bool first) {
   if (words) ll_bytes += (size_t)h->grid * mk::kTileRows * x_rows * 8;
   h->ll_buf = nullptr;
   h->ll_bytes = ll_bytes;
-  // behind the words: the counters of the attention chunks and of the split-k pieces
+  // behind the words: the counters of the attention chunks and the flags of the split-k pieces
   int count_hkv = 1;
   for (const PlanOp& po : h->plan)
     if (po.type == mk::OP_ATTN) count_hkv = std::max(count_hkv, po.aux0);
   const size_t count_off = (ll_bytes + 255) / 256 * 256, attn_counts = (size_t)h->plan_tokens * count_hkv;
-  h->clear_bytes = count_off + (attn_counts + (rows_mode ? 1 : (size_t)max_nblk * mk::kNumConsumerWarps)) * 4;
+  h->clear_bytes = count_off + (attn_counts + (rows_mode ? 1 : (size_t)h->grid * 2 * mk::kNumConsumerWarps)) * 4;
   if (int e = h->dmalloc(&h->ll_buf, h->clear_bytes)) return e;
   kp.attn_count = (unsigned*)((char*)h->ll_buf + count_off);
-  kp.piece_count = kp.attn_count + attn_counts;
+  kp.piece_flag = kp.attn_count + attn_counts;
   kp.partial = words ? (uint4*)((char*)h->ll_buf + partial_off) : nullptr;
   kp.attn_part_ll = ll_part ? (uint2*)((char*)h->ll_buf + ll_part_off) : nullptr;
 
@@ -1605,7 +1605,7 @@ static int compile_program(mk_handle* h, bool first) {
   const int G = h->grid;
   void* p = nullptr;
   if (!rows_mode && !words) {
-    if (int e = h->dmalloc(&p, (size_t)G * mk::kTileRows * x_rows * 4)) return e;
+    if (int e = h->dmalloc(&p, (size_t)G * 2 * mk::kTileRows * x_rows * 4)) return e;
     kp.partial = (uint4*)p;
   }
   int max_hkv = 1, max_qpk = 2;

@@ -226,9 +226,9 @@ struct KParams {
   int max_iters;      // 0 = unlimited
   unsigned long long timeout_ns;
   // split-k scratch shared by all linear ops of the wide path
-  uint4* partial;         // [grid][...][128 rows]: a CTA's sums of the block that an earlier CTA finishes.  Up to 32 token rows
-                          // [x_rows / 2] words {sum, tag, sum of the next token, tag}, beyond [x_rows / 4] float4
-  unsigned* piece_count;  // [max nblk][8 warps]: shares published (beyond 32 token rows)
+  uint4* partial;         // sums of blocks that several CTAs share.  Up to 32 token rows [grid][x_rows / 2][128 rows] words {sum, tag,
+                          // sum of the next token, tag}, beyond [grid][2][x_rows / 4][128 rows] float4
+  unsigned* piece_flag;   // [grid][2][8 warps]: tag of the op whose piece is there (beyond 32 token rows)
   // attention scratch
   float* attn_part;       // [tokens][kv heads][max chunks][qpk*(128+2)]
   unsigned* attn_count;   // [tokens][kv heads]
@@ -304,6 +304,11 @@ __host__ __device__ inline int wide_ctas(int grid, int nblk, int nkt) {
   const unsigned total = (unsigned)nblk * (unsigned)nkt;
   return total < (unsigned)grid ? (int)total : grid;
 }
+
+// Beyond 32 token rows: whether the CTAs of a row block share its finish (see mk_wide.cuh).  With more blocks than half the CTAs a
+// CTA has about a block to finish either way, and two shares in turn take longer than one block at once: 8B width, 64 requests,
+// gate/up (192 blocks) 39.8 us shared and 36.4 by one CTA; QKV (48) 18.9 and 20.2, O and down (32) 13.2 and 16.0, 22.5 and 26.5.
+__host__ __device__ inline bool wide_shares(int nblk, int ctas) { return 2 * nblk <= ctas; }
 
 static_assert(sizeof(OpDesc) % 16 == 0 && sizeof(OpDesc) <= 256, "OpDesc is copied to shared memory in 16-byte pieces");
 

@@ -364,18 +364,17 @@ __device__ __forceinline__ void norm_loop(Ctx& c) {
 // Warp w reads accumulator lanes 32 (w & 3) .. + 31 (weight rows of the tile) and one half of the token columns;
 // a thread holds one output row for up to 32 tokens in registers, from tensor memory to the store.
 //
-// When several CTAs hold k-ranges of a row block, the CTA with the block's FIRST k-range finishes it (that range
-// is the tail of its own tile range, so it is computed last anyway); a thread adds the other pieces of its output row up in
-// CTA order.  No CTA-wide sync and no shared memory on the way.
-//  * Up to 32 token rows the others store their sums as words that carry a tag, two tokens per 16 bytes, [token / 2][row],
-//    and the finisher polls them, several pieces at once: data and "ready" arrive in one load, with no release behind the
-//    stores, no counter and no second round trip.  The tag differs in every op of every iteration, the words are cleared
-//    before every launch, and a CTA's slot is written again only behind a grid barrier.
-//  * Beyond, twice the bytes cost more than the round trip: plain float4 of four tokens, [token / 4][row]; every warp
-//    publishes its share with a release of its own and the matching warp of the finisher waits for exactly those.
-// Both measured, us per step of 12 layers of 8B width (words, counters): 8 requests 1433, 1473; 20 1446, 1459; 32 1487, 1500; 64
-// 1989, 1942; 100 2488, 2377; 2048 hidden, 8 requests 855, 910; 20 893, 895; 32 942, 943; four layers of 1024 hidden, 4 requests
-// 197, 209; 20 263, 250; 32 276, 262; of 512 hidden, 20 215, 224; 32 226, 222.
+// Several CTAs hold k-ranges of a row block; their sums are added up in CTA order.  No CTA-wide sync and no shared memory on the way.
+//  * Up to 32 token rows (linear_wide) the CTA with the block's FIRST k-range finishes it (that range is the tail of its own tile
+//    range, so it is computed last anyway).  The others store their sums as words that carry a tag, two tokens per 16 bytes,
+//    [token / 2][row], and a finishing thread polls those of its own output row, several pieces at once: data and "ready" arrive in one
+//    load, with no release behind the stores, no flag and no second round trip.  The tag differs in every op of every
+//    iteration, the words are cleared before every launch, and a CTA's slot is written again only behind a grid barrier.
+//  * Beyond (linear_wide_shared) the bytes cost more than the round trip, and one CTA per block would read four to six pieces of
+//    32 KB and more in turn, 7 us of a linear's end.  So every CTA of a block finishes its share of the tokens: all of them store their
+//    sums, plain float4 of four tokens, [token / 4][row], every warp publishes its share with a release of its own (a flag that holds the
+//    op's tag), and behind the op's last tile a warp waits for the matching warps of the block's CTAs.
+//    MEASURED_SHARED
 __device__ __forceinline__ uint32_t order_bf16(float v) {  // monotone 16-bit key of a bf16 value; 0 only for NaN
   const uint32_t b = __float_as_uint(v + 0.f) >> 16;       // (-0 counts as +0)
   const uint32_t k = (b & 0x8000u) ? (~b & 0xffffu) : (b | 0x8000u);
@@ -419,9 +418,11 @@ __device__ __forceinline__ void wide_store_head(const Ctx& c, const OpDesc& op, 
   }
 }
 
+// `cc`, `l0`: where the running best of the first token is kept (pair, lane)
 template <int NC>
 __device__ __forceinline__ void wide_epilogue(Ctx& c, const OpDesc& op, int blk, int row, int tok0, int nlive, const float (&v)[NC],
-                                              const uint32_t (&res)[NC / 2], WideBest& best, int cc) {
+                                              const uint32_t (&res)[NC / 2], WideBest& best, int cc = 0, int l0 = 0) {
+  constexpr bool kSums = 2 * MK_NC <= kNormBoxRows;
   const KParams& p = c.p;
   const int col = blk * kTileRows + row;
   __nv_bfloat16* out = reinterpret_cast<__nv_bfloat16*>(op.out);
@@ -465,7 +466,7 @@ __device__ __forceinline__ void wide_epilogue(Ctx& c, const OpDesc& op, int blk,
   const bool okc = col < op.n;
   const bool push = MK_XF(op, F_PUSH) != 0;
   const bool with_res = (op.flags & F_RESIDUAL) && (!(op.flags & F_RES_RANK0) || p.rank == 0);
-  float sq[2 * NC <= kNormBoxRows ? NC : 1];
+  float sq[kSums ? NC : 1];
   const bool rnd = p.numerics == NUM_TORCH && !push;  // (pushed partial sums stay fp32: rounded once, after the ranks are added up)
 #pragma unroll
   for (int i = 0; i < NC; ++i) {
@@ -479,12 +480,12 @@ __device__ __forceinline__ void wide_epilogue(Ctx& c, const OpDesc& op, int blk,
       if (push) xchg_push1(p, xchg_next(c), tok0 + i, col, y);
       else out[(size_t)(tok0 + i) * op.ld_out + col] = __float2bfloat16_rn(y);
     }
-    if constexpr (2 * NC <= kNormBoxRows) {
+    if constexpr (kSums) {
       y = okc ? rbf(y) : 0.f;
       sq[i] = p.numerics == NUM_TORCH ? rbf(y * y) : y * y;
     }
   }
-  if constexpr (2 * NC <= kNormBoxRows) {
+  if constexpr (kSums) {
     if (op.flags & F_ROW_SUMS) {
       // NC sums over the warp's 32 rows: halves change places until a lane is left with one token, then the rest is added up
       int tok = 0;
@@ -510,14 +511,15 @@ __device__ __forceinline__ void wide_epilogue(Ctx& c, const OpDesc& op, int blk,
       // larger value wins, ties go to the lower index: one 32-bit maximum over the warp's rows
       const uint32_t k = okc ? (order_bf16(rbf(v[i])) << 16) | (uint32_t)(0xffff - row) : 0u;
       const uint32_t m = __reduce_max_sync(0xffffffffu, k);
-      // (blocks come in ascending order: an equal value keeps the lower index; indexed by cc, the pairs would live in local memory)
-      if (c.lane == i && (m >> 16) > (cc == 0 ? best.key[0] : best.key[1])) {
-        const int at = blk * kTileRows + 0xffff - (int)(m & 0xffffu);
+      // (an equal value keeps the lower index; indexed by cc, the pairs would live in local memory)
+      const uint32_t key = m >> 16, had = cc == 0 ? best.key[0] : best.key[1];
+      const int at = blk * kTileRows + 0xffff - (int)(m & 0xffffu);
+      if (c.lane == l0 + i && key != 0u && (key > had || (key == had && at < (cc == 0 ? best.idx[0] : best.idx[1])))) {
         if (cc == 0) {
-          best.key[0] = m >> 16;
+          best.key[0] = key;
           best.idx[0] = at;
         } else {
-          best.key[1] = m >> 16;
+          best.key[1] = key;
           best.idx[1] = at;
         }
       }
@@ -525,52 +527,218 @@ __device__ __forceinline__ void wide_epilogue(Ctx& c, const OpDesc& op, int blk,
   }
 }
 
-// A finisher's warp waits until the `want` other pieces of its block have published their share (bounded).
-__device__ __forceinline__ void wide_wait_pieces(const Ctx& c, unsigned* cnt, unsigned want, int blk) {
-  if (c.lane == 0) {
-    unsigned long long t0 = 0;
-    unsigned spins = 0;
-    while (ld_acquire_u32(cnt) < want) {
-      if (((++spins) & 1023u) == 0) {
-        if (aborted(c)) break;
-        const unsigned long long now = globaltimer();
-        if (t0 == 0) {
-          t0 = now;
-        } else if (now - t0 > 2 * c.p.timeout_ns) {
-          raise_abort(c, ST_TIMEOUT_PEER, blk, (int)ld_acquire_u32(cnt));
-          break;
-        }
-      }
-    }
-    *cnt = 0u;  // (its next use lies behind a grid barrier)
+// The residual of NC tokens from col0 on, pairs of bf16 (zeros where there is none)
+template <int NC>
+__device__ __forceinline__ void wide_residual(const OpDesc& op, bool with_res, int col, int col0, int nlive, uint32_t (&res)[NC / 2]) {
+#pragma unroll
+  for (int i = 0; i < NC / 2; ++i) res[i] = 0u;
+  if (!with_res || col >= op.n) return;
+  const unsigned short* rp = reinterpret_cast<const unsigned short*>(op.res) + (size_t)col0 * op.ld_res + col;
+#pragma unroll
+  for (int i = 0; i < NC / 2; ++i) {
+    uint32_t lo = 0u, hi = 0u;
+    if (2 * i < nlive) lo = __ldcg(rp + (size_t)(2 * i) * op.ld_res);
+    if (2 * i + 1 < nlive) hi = __ldcg(rp + (size_t)(2 * i + 1) * op.ld_res);
+    res[i] = lo | (hi << 16);
   }
-  __syncwarp();
+}
+__device__ __forceinline__ bool wide_with_res(const Ctx& c, const OpDesc& op) {
+  return (op.flags & F_RESIDUAL) && !MK_XF(op, F_GATHER_RES) && (!(op.flags & F_RES_RANK0) || c.p.rank == 0);
+}
+// one (max, index) partial per token, CTA and row quarter; NC token columns per pair of `best`
+template <int NC>
+__device__ __forceinline__ void wide_store_best(const Ctx& c, const OpDesc& op, int T, int G, int pairs, const WideBest& best) {
+#pragma unroll
+  for (int cc = 0; cc < 2; ++cc) {
+    const int t = (c.warp >> 2) * (c.p.x_rows >> 1) + cc * NC + c.lane;
+    if (cc < pairs && c.lane < NC && t < T && (int)blockIdx.x < G) {
+      const size_t o = (size_t)t * op.amax_n + blockIdx.x * 4 + (c.warp & 3);
+      op.amax_val[o] = best.key[cc] != 0u ? unorder_bf16(best.key[cc]) : -INFINITY;
+      op.amax_idx[o] = best.idx[cc];
+    }
+  }
 }
 
-// NC: token columns of a thread per round: x_rows / 2, at most 32 (128 token rows: two rounds)
+// Up to 32 token rows.  NC: token columns of a thread, x_rows / 2
 template <int NC>
 __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
   const KParams& p = c.p;
   const int N = p.x_rows, nkt = op.nkt;
   const int q = c.warp & 3, half = c.warp >> 2, row = 32 * q + c.lane;
-  const int nround = N > 2 * NC ? 2 : 1;
   WideBest best;
   best.key[0] = best.key[1] = 0u;
   best.idx[0] = best.idx[1] = 0x7fffffff;
   unsigned total, t0, t1;
   int G;
   if (wide_range(p, op, total, G, t0, t1)) {
-    const bool with_res = (op.flags & F_RESIDUAL) && !MK_XF(op, F_GATHER_RES) && (!(op.flags & F_RES_RANK0) || p.rank == 0);
-    constexpr bool kWords = NC < 32;
-    const size_t slot_vec = (size_t)kTileRows * N / (kWords ? 2 : 4);  // 16-byte vectors of a CTA's sums
+    const bool with_res = wide_with_res(c, op);
+    const size_t slot_vec = (size_t)kTileRows * N / 2;  // 16-byte vectors of a CTA's sums
     const unsigned tag = ll_tag_of(c, c.cur_op);
+    const int col0 = half * (N >> 1);     // first token column of this thread
+    const int nlive = min(NC, T - col0);  // may be negative: nothing but padding
 #pragma unroll 1
     for (unsigned tile = t0; tile < t1;) {
       const int blk = (int)(tile / (unsigned)nkt);
       const unsigned blk0 = (unsigned)blk * (unsigned)nkt, blk1 = blk0 + (unsigned)nkt;
       const bool finisher = tile == blk0;  // (only the first run of a range can belong to another CTA's block)
       const int c_last = tile_owner(blk1 - 1, total, G);
-      unsigned* cnt = p.piece_count + (size_t)blk * kNumConsumerWarps + c.warp;
+      const uint32_t acc = c.tmem + (c.acc_runs & 1u) * (uint32_t)N + ((uint32_t)(32 * q) << 16);
+      // the residual does not depend on the sums: requested first
+      uint32_t res[NC / 2];
+      wide_residual<NC>(op, with_res && finisher, blk * kTileRows + row, col0, nlive, res);
+      mbar_wait(c, c.acc_full_bar(c.acc_runs & 1), (c.acc_runs >> 1) & 1u, ST_TIMEOUT_FULL);
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      if (tile == t0) MK_STAMP(c, 0);
+      __syncwarp();
+      uint32_t raw[NC];
+      tmem_ld<NC>(acc + (uint32_t)col0, raw);
+      tmem_wait_ld();
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (c.lane == 0) mbar_arrive(c.acc_empty_bar(c.acc_runs & 1));  // the accumulators may be overwritten
+      c.acc_runs += 1;
+      tile = min(blk1, t1);
+      float v[NC];
+#pragma unroll
+      for (int i = 0; i < NC; ++i) v[i] = __uint_as_float(raw[i]);
+      if (!finisher) {
+        uint4* mine = p.partial + (size_t)blockIdx.x * slot_vec + (size_t)(col0 >> 1) * kTileRows + row;
+#pragma unroll
+        for (int i = 0; i < NC / 2; ++i)
+          if (2 * i < nlive) st_gpu_words(mine + (size_t)i * kTileRows, __float_as_uint(v[2 * i]), __float_as_uint(v[2 * i + 1]), tag);
+        MK_STAMP(c, 1);
+        continue;
+      }
+      MK_STAMP(c, 2);
+      if (c_last > (int)blockIdx.x) {
+        const uint4* src0 = p.partial + (size_t)(col0 >> 1) * kTileRows + row;
+        // Several pieces in flight per round (registers allowing): a block of a small layer has up to `nkt` of them.
+        constexpr int PB = NC == 8 ? 4 : 2;
+#pragma unroll 1
+        for (int cta = (int)blockIdx.x + 1; cta <= c_last; cta += PB) {
+          uint4 w[PB][NC / 2];
+#pragma unroll
+          for (int u = 0; u < PB; ++u)
+#pragma unroll
+            for (int i = 0; i < NC / 2; ++i) {
+              const unsigned t = (cta + u <= c_last && 2 * i < nlive) ? ~tag : tag;  // (nothing to wait for: zeros)
+              w[u][i] = make_uint4(0u, t, 0u, t);
+            }
+          PollLimit limit;
+          while (true) {
+#pragma unroll
+            for (int u = 0; u < PB; ++u)
+#pragma unroll
+              for (int i = 0; i < NC / 2; ++i)
+                if (w[u][i].y != tag || w[u][i].w != tag) w[u][i] = ld_gpu_words(src0 + (size_t)(cta + u) * slot_vec + (size_t)i * kTileRows);
+            bool here = true;
+#pragma unroll
+            for (int u = 0; u < PB; ++u)
+#pragma unroll
+              for (int i = 0; i < NC / 2; ++i) here = here && w[u][i].y == tag && w[u][i].w == tag;
+            if (here || limit.expired(c, tag, w[0][0].y)) break;
+          }
+#pragma unroll
+          for (int u = 0; u < PB; ++u)
+#pragma unroll
+            for (int i = 0; i < NC / 2; ++i) {
+              v[2 * i] += __uint_as_float(w[u][i].x);
+              v[2 * i + 1] += __uint_as_float(w[u][i].z);
+            }
+        }
+        MK_STAMP(c, 3);
+      }
+      __syncwarp();  // (lanes leave the poll at different times; the epilogue shuffles)
+      MK_STAMP(c, 4);
+      wide_epilogue<NC>(c, op, blk, row, col0, nlive, v, res, best);
+      MK_STAMP(c, 5);
+    }
+  }
+  if (op.flags & F_ARGMAX) wide_store_best<NC>(c, op, T, G, 1, best);
+}
+
+// Beyond 32 token rows: where a piece of a block lies.  A CTA has two slots: the block its range begins in, and the one it ends in.
+__device__ __forceinline__ float4* wide_piece(const KParams& p, int cta, int slot) {
+  return reinterpret_cast<float4*>(p.partial) + ((size_t)cta * 2 + slot) * (size_t)(kTileRows * p.x_rows / 4);
+}
+__device__ __forceinline__ unsigned* wide_flag(const KParams& p, int cta, int slot) { return p.piece_flag + ((size_t)cta * 2 + slot) * kNumConsumerWarps; }
+// Waits until the matching warps of CTAs c0 .. c1 have published their pieces; `slot`: the one of c0 (the others open their ranges).
+__device__ __forceinline__ void wide_wait_pieces(const Ctx& c, int c0, int c1, int slot, unsigned tag) {
+  for (int cta = c0 + c.lane; cta <= c1; cta += 32) {
+    const unsigned* flag = wide_flag(c.p, cta, cta == c0 ? slot : 0) + c.warp;
+    PollLimit limit;
+    unsigned got;
+    while ((got = ld_acquire_u32(flag)) != tag && !limit.expired(c, tag, got)) {
+    }
+  }
+  __syncwarp();
+}
+// This CTA's share of a block's tokens: of the eight-token groups of each half, as many as there are CTAs to share them, in CTA order.
+__device__ __forceinline__ void wide_finish_share(Ctx& c, const OpDesc& op, int T, int blk, unsigned total, int G, WideBest& best) {
+  const KParams& p = c.p;
+  const int N = p.x_rows, half = c.warp >> 2, row = 32 * (c.warp & 3) + c.lane, col = blk * kTileRows + row;
+  const unsigned blk0 = (unsigned)blk * (unsigned)op.nkt;
+  const int c_first = tile_owner(blk0, total, G), P = tile_owner(blk0 + (unsigned)op.nkt - 1u, total, G) - c_first + 1, me = (int)blockIdx.x - c_first;
+  const int groups = max(0, min(N >> 4, (T - half * (N >> 1) + 7) >> 3));
+  const int g0 = (me * groups + P - 1) / P, g1 = ((me + 1) * groups + P - 1) / P;
+  if (g0 >= g1) return;  // (the same in all four warps of a half)
+  const unsigned tag = ll_tag_of(c, c.cur_op);
+  const int slot = tile_begin((unsigned)c_first, total, (unsigned)G) == blk0 ? 0 : 1;  // of the first piece; the others open their CTA's range
+  const bool with_res = wide_with_res(c, op);
+#pragma unroll 1
+  for (int g = g0; g < g1; ++g) {
+    const int tok0 = half * (N >> 1) + 8 * g, nlive = min(8, T - tok0);
+    uint32_t res[4];
+    wide_residual<8>(op, with_res, col, tok0, nlive, res);  // (does not depend on the sums: requested first)
+    if (g == g0) wide_wait_pieces(c, c_first, c_first + P - 1, slot, tag);
+    float v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = 0.f;
+    constexpr int PB = 4;  // pieces in flight per round
+#pragma unroll 1
+    for (int i0 = 0; i0 < P; i0 += PB) {
+      float4 w[PB][2];
+#pragma unroll
+      for (int u = 0; u < PB; ++u) {
+        const int i = min(i0 + u, P - 1);
+        const float4* src = wide_piece(p, c_first + i, i == 0 ? slot : 0) + (size_t)(tok0 >> 2) * kTileRows + row;
+        w[u][0] = i0 + u < P ? __ldcg(src) : make_float4(0.f, 0.f, 0.f, 0.f);
+        w[u][1] = i0 + u < P && nlive > 4 ? __ldcg(src + kTileRows) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < PB; ++u)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          v[4 * i] += w[u][i].x;
+          v[4 * i + 1] += w[u][i].y;
+          v[4 * i + 2] += w[u][i].z;
+          v[4 * i + 3] += w[u][i].w;
+        }
+    }
+    wide_epilogue<8>(c, op, blk, row, tok0, nlive, v, res, best, g >> 2, 8 * (g & 3));
+  }
+}
+__device__ __forceinline__ void linear_wide_shared(Ctx& c, const OpDesc& op, int T) {
+  constexpr int NC = 32;  // token columns of a thread per round (128 token rows: two rounds)
+  const KParams& p = c.p;
+  const int N = p.x_rows, nkt = op.nkt, nround = N > 2 * NC ? 2 : 1;
+  const int q = c.warp & 3, half = c.warp >> 2, row = 32 * q + c.lane;
+  WideBest best;
+  best.key[0] = best.key[1] = 0u;
+  best.idx[0] = best.idx[1] = 0x7fffffff;
+  unsigned total, t0, t1;
+  int G;
+  if (wide_range(p, op, total, G, t0, t1)) {
+    const bool with_res = wide_with_res(c, op), share = wide_shares(op.nblk, G);
+    const unsigned tag = ll_tag_of(c, c.cur_op);
+    int shared[2] = {-1, -1};  // blocks to finish with others: the one the range begins in, the one it ends in
+#pragma unroll 1
+    for (unsigned tile = t0; tile < t1;) {
+      const int blk = (int)(tile / (unsigned)nkt);
+      const unsigned blk0 = (unsigned)blk * (unsigned)nkt, blk1 = blk0 + (unsigned)nkt;
+      const bool first = tile == t0, begins = tile == blk0;
+      const int c_last = tile_owner(blk1 - 1, total, G);
+      const bool finisher = begins && (!share || c_last == (int)blockIdx.x);
       const uint32_t acc = c.tmem + (c.acc_runs & 1u) * (uint32_t)N + ((uint32_t)(32 * q) << 16);
 #pragma unroll 1
       for (int cc = 0; cc < nround; ++cc) {
@@ -578,23 +746,12 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
         const int nlive = min(NC, T - col0);          // may be negative: nothing but padding
         // the residual does not depend on the sums: requested first
         uint32_t res[NC / 2];
-#pragma unroll
-        for (int i = 0; i < NC / 2; ++i) res[i] = 0u;
-        if (with_res && finisher && blk * kTileRows + row < op.n) {
-          const unsigned short* rp = reinterpret_cast<const unsigned short*>(op.res) + (size_t)col0 * op.ld_res + blk * kTileRows + row;
-#pragma unroll
-          for (int i = 0; i < NC / 2; ++i) {
-            uint32_t lo = 0u, hi = 0u;
-            if (2 * i < nlive) lo = __ldcg(rp + (size_t)(2 * i) * op.ld_res);
-            if (2 * i + 1 < nlive) hi = __ldcg(rp + (size_t)(2 * i + 1) * op.ld_res);
-            res[i] = lo | (hi << 16);
-          }
-        }
+        wide_residual<NC>(op, with_res && finisher, blk * kTileRows + row, col0, nlive, res);
         if (cc == 0) {
           mbar_wait(c, c.acc_full_bar(c.acc_runs & 1), (c.acc_runs >> 1) & 1u, ST_TIMEOUT_FULL);
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         }
-        if (tile == t0) MK_STAMP(c, 0);
+        if (first) MK_STAMP(c, 0);
         __syncwarp();
         uint32_t raw[NC];
         tmem_ld<NC>(acc + (uint32_t)col0, raw);
@@ -608,89 +765,47 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
 #pragma unroll
         for (int i = 0; i < NC; ++i) v[i] = __uint_as_float(raw[i]);
         if (!finisher) {
-          if constexpr (kWords) {
-            uint4* mine = p.partial + (size_t)blockIdx.x * slot_vec + (size_t)(col0 >> 1) * kTileRows + row;
+          float4* mine = wide_piece(p, (int)blockIdx.x, first ? 0 : 1) + (size_t)(col0 >> 2) * kTileRows + row;
 #pragma unroll
-            for (int i = 0; i < NC / 2; ++i)
-              if (2 * i < nlive) st_gpu_words(mine + (size_t)i * kTileRows, __float_as_uint(v[2 * i]), __float_as_uint(v[2 * i + 1]), tag);
-          } else {
-            float4* mine = reinterpret_cast<float4*>(p.partial) + (size_t)blockIdx.x * slot_vec + (size_t)(col0 >> 2) * kTileRows + row;
-#pragma unroll
-            for (int i = 0; i < NC / 4; ++i)
-              if (4 * i < nlive) mine[(size_t)i * kTileRows] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-            if (cc == nround - 1) {
-              __syncwarp();  // lane 0's release covers what the warp wrote before
-              if (c.lane == 0) asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(cnt) : "memory");
-            }
+          for (int i = 0; i < NC / 4; ++i)
+            if (4 * i < nlive) mine[(size_t)i * kTileRows] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+          if (cc == nround - 1) {
+            __syncwarp();  // lane 0's release covers what the warp wrote before
+            if (c.lane == 0)
+              asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(wide_flag(p, (int)blockIdx.x, first ? 0 : 1) + c.warp), "r"(tag) : "memory");
+            if (share) (first ? shared[0] : shared[1]) = blk;
           }
-          if (tile == t0) MK_STAMP(c, 1);
+          if (first) MK_STAMP(c, 1);
           continue;
         }
         MK_STAMP(c, 2);
         if (c_last > (int)blockIdx.x) {
-          if constexpr (kWords) {
-            const uint4* src0 = p.partial + (size_t)(col0 >> 1) * kTileRows + row;
-            // Several pieces in flight per round (registers allowing): a block of a small layer has up to `nkt` of them.
-            constexpr int PB = NC == 8 ? 4 : 2;
+          if (cc == 0) wide_wait_pieces(c, (int)blockIdx.x + 1, c_last, 0, tag);
+          const float4* src0 = wide_piece(p, 0, 0) + (size_t)(col0 >> 2) * kTileRows + row;
+          const size_t stride = (size_t)kTileRows * N / 2;  // from a CTA's first piece to the next one's
+          constexpr int PB = 2;  // pieces in flight per round
 #pragma unroll 1
-            for (int cta = (int)blockIdx.x + 1; cta <= c_last; cta += PB) {
-              uint4 w[PB][NC / 2];
+          for (int cta = (int)blockIdx.x + 1; cta <= c_last; cta += PB) {
+            float4 w[PB][NC / 4];
 #pragma unroll
-              for (int u = 0; u < PB; ++u)
+            for (int u = 0; u < PB; ++u)
 #pragma unroll
-                for (int i = 0; i < NC / 2; ++i) {
-                  const unsigned t = (cta + u <= c_last && 2 * i < nlive) ? ~tag : tag;  // (nothing to wait for: zeros)
-                  w[u][i] = make_uint4(0u, t, 0u, t);
-                }
-              PollLimit limit;
-              while (true) {
+              for (int i = 0; i < NC / 4; ++i)
+                w[u][i] = (cta + u <= c_last && 4 * i < nlive) ? __ldcg(src0 + (size_t)(cta + u) * stride + (size_t)i * kTileRows)
+                                                               : make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-                for (int u = 0; u < PB; ++u)
+            for (int u = 0; u < PB; ++u)
 #pragma unroll
-                  for (int i = 0; i < NC / 2; ++i)
-                    if (w[u][i].y != tag || w[u][i].w != tag) w[u][i] = ld_gpu_words(src0 + (size_t)(cta + u) * slot_vec + (size_t)i * kTileRows);
-                bool here = true;
-#pragma unroll
-                for (int u = 0; u < PB; ++u)
-#pragma unroll
-                  for (int i = 0; i < NC / 2; ++i) here = here && w[u][i].y == tag && w[u][i].w == tag;
-                if (here || limit.expired(c, tag, w[0][0].y)) break;
+              for (int i = 0; i < NC / 4; ++i) {
+                v[4 * i] += w[u][i].x;
+                v[4 * i + 1] += w[u][i].y;
+                v[4 * i + 2] += w[u][i].z;
+                v[4 * i + 3] += w[u][i].w;
               }
-#pragma unroll
-              for (int u = 0; u < PB; ++u)
-#pragma unroll
-                for (int i = 0; i < NC / 2; ++i) {
-                  v[2 * i] += __uint_as_float(w[u][i].x);
-                  v[2 * i + 1] += __uint_as_float(w[u][i].z);
-                }
-            }
-          } else {
-            if (cc == 0) wide_wait_pieces(c, cnt, (unsigned)(c_last - (int)blockIdx.x), blk);
-            const float4* src0 = reinterpret_cast<const float4*>(p.partial) + (size_t)(col0 >> 2) * kTileRows + row;
-            constexpr int PB = 2;  // pieces in flight per round
-#pragma unroll 1
-            for (int cta = (int)blockIdx.x + 1; cta <= c_last; cta += PB) {
-              float4 w[PB][NC / 4];
-#pragma unroll
-              for (int u = 0; u < PB; ++u)
-#pragma unroll
-                for (int i = 0; i < NC / 4; ++i)
-                  w[u][i] = (cta + u <= c_last && 4 * i < nlive) ? __ldcg(src0 + (size_t)(cta + u) * slot_vec + (size_t)i * kTileRows)
-                                                                 : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-              for (int u = 0; u < PB; ++u)
-#pragma unroll
-                for (int i = 0; i < NC / 4; ++i) {
-                  v[4 * i] += w[u][i].x;
-                  v[4 * i + 1] += w[u][i].y;
-                  v[4 * i + 2] += w[u][i].z;
-                  v[4 * i + 3] += w[u][i].w;
-                }
-            }
           }
           MK_STAMP(c, 3);
         }
-        __syncwarp();  // (lanes leave the poll at different times; the epilogue shuffles)
+        __syncwarp();
         MK_STAMP(c, 4);
         wide_epilogue<NC>(c, op, blk, row, col0, nlive, v, res, best, cc);
         MK_STAMP(c, 5);
@@ -698,18 +813,15 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
       c.acc_runs += 1;
       tile = min(blk1, t1);
     }
-  }
-  if (op.flags & F_ARGMAX) {  // one (max, index) partial per token, CTA and row quarter
-#pragma unroll
-    for (int cc = 0; cc < 2; ++cc) {
-      const int t = half * (N >> 1) + cc * NC + c.lane;
-      if (cc < nround && c.lane < NC && t < T && (int)blockIdx.x < G) {
-        const size_t o = (size_t)t * op.amax_n + blockIdx.x * 4 + q;
-        op.amax_val[o] = best.key[cc] != 0u ? unorder_bf16(best.key[cc]) : -INFINITY;
-        op.amax_idx[o] = best.idx[cc];
-      }
+    // the block the range ends in first: its other CTAs began with it
+#pragma unroll 1
+    for (int i = 1; i >= 0; --i) {
+      const int blk = i == 1 ? shared[1] : shared[0];
+      if (blk >= 0) wide_finish_share(c, op, T, blk, total, G, best);
     }
+    MK_STAMP(c, 6);
   }
+  if (op.flags & F_ARGMAX) wide_store_best<NC>(c, op, T, G, nround, best);
 }
 
 template <int NC>
@@ -720,7 +832,8 @@ __device__ __forceinline__ void op_linear_wide(Ctx& c, const OpDesc& op, int T) 
   if constexpr (2 * NC <= kNormBoxRows) {
     if (op.flags & F_NORM_IN) wide_row_scales(c, op, T);
   }
-  linear_wide<NC>(c, op, T);
+  if constexpr (2 * NC <= kNormBoxRows) linear_wide<NC>(c, op, T);
+  else linear_wide_shared(c, op, T);
   if (MK_XF(op, F_PUSH)) c.ar_seq += 1;  // every CTA counts the exchange, with or without rows of its own
 }
 
