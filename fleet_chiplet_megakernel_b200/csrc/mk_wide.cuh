@@ -545,13 +545,20 @@ __device__ __forceinline__ void wide_residual(const OpDesc& op, bool with_res, i
 __device__ __forceinline__ bool wide_with_res(const Ctx& c, const OpDesc& op) {
   return (op.flags & F_RESIDUAL) && !MK_XF(op, F_GATHER_RES) && (!(op.flags & F_RES_RANK0) || c.p.rank == 0);
 }
+// The live token columns are split evenly over the two halves of the warps: the upper half's first column.  In steps of the two
+// tokens of a word, beyond 32 token rows of the eight that a share is made of.
+template <int NC>
+__device__ __forceinline__ int wide_split(int T) {
+  constexpr int step = NC < 32 ? 2 : 8;
+  return (T + 2 * step - 1) / (2 * step) * step;
+}
 // one (max, index) partial per token, CTA and row quarter; NC token columns per pair of `best`
 template <int NC>
 __device__ __forceinline__ void wide_store_best(const Ctx& c, const OpDesc& op, int T, int G, int pairs, const WideBest& best) {
 #pragma unroll
   for (int cc = 0; cc < 2; ++cc) {
-    const int t = (c.warp >> 2) * (c.p.x_rows >> 1) + cc * NC + c.lane;
-    if (cc < pairs && c.lane < NC && t < T && (int)blockIdx.x < G) {
+    const int half = c.warp >> 2, t0 = wide_split<NC>(T), t = half * t0 + cc * NC + c.lane;
+    if (cc < pairs && c.lane < NC && t < (half == 0 ? min(t0, T) : T) && (int)blockIdx.x < G) {
       const size_t o = (size_t)t * op.amax_n + blockIdx.x * 4 + (c.warp & 3);
       op.amax_val[o] = best.key[cc] != 0u ? unorder_bf16(best.key[cc]) : -INFINITY;
       op.amax_idx[o] = best.idx[cc];
@@ -574,8 +581,8 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
     const bool with_res = wide_with_res(c, op);
     const size_t slot_vec = (size_t)kTileRows * N / 2;  // 16-byte vectors of a CTA's sums
     const unsigned tag = ll_tag_of(c, c.cur_op);
-    const int col0 = half * (N >> 1);     // first token column of this thread
-    const int nlive = min(NC, T - col0);  // may be negative: nothing but padding
+    const int col0 = half * wide_split<NC>(T);  // first token column of this thread
+    const int nlive = half == 0 ? min(wide_split<NC>(T), T) : T - col0;  // may be none: nothing but padding
 #pragma unroll 1
     for (unsigned tile = t0; tile < t1;) {
       const int blk = (int)(tile / (unsigned)nkt);
@@ -676,10 +683,11 @@ __device__ __forceinline__ void wide_wait_pieces(const Ctx& c, int c0, int c1, i
 // This CTA's share of a block's tokens: of the eight-token groups of each half, as many as there are CTAs to share them, in CTA order.
 __device__ __forceinline__ void wide_finish_share(Ctx& c, const OpDesc& op, int T, int blk, unsigned total, int G, WideBest& best) {
   const KParams& p = c.p;
-  const int N = p.x_rows, half = c.warp >> 2, row = 32 * (c.warp & 3) + c.lane, col = blk * kTileRows + row;
+  const int half = c.warp >> 2, row = 32 * (c.warp & 3) + c.lane, col = blk * kTileRows + row;
   const unsigned blk0 = (unsigned)blk * (unsigned)op.nkt;
   const int c_first = tile_owner(blk0, total, G), P = tile_owner(blk0 + (unsigned)op.nkt - 1u, total, G) - c_first + 1, me = (int)blockIdx.x - c_first;
-  const int groups = max(0, min(N >> 4, (T - half * (N >> 1) + 7) >> 3));
+  const int split = wide_split<32>(T), end = half == 0 ? min(split, T) : T;
+  const int groups = max(0, (end - half * split + 7) >> 3);
   const int g0 = (me * groups + P - 1) / P, g1 = ((me + 1) * groups + P - 1) / P;
   if (g0 >= g1) return;  // (the same in all four warps of a half)
   const unsigned tag = ll_tag_of(c, c.cur_op);
@@ -687,7 +695,7 @@ __device__ __forceinline__ void wide_finish_share(Ctx& c, const OpDesc& op, int 
   const bool with_res = wide_with_res(c, op);
 #pragma unroll 1
   for (int g = g0; g < g1; ++g) {
-    const int tok0 = half * (N >> 1) + 8 * g, nlive = min(8, T - tok0);
+    const int tok0 = half * split + 8 * g, nlive = min(8, end - tok0);
     uint32_t res[4];
     wide_residual<8>(op, with_res, col, tok0, nlive, res);  // (does not depend on the sums: requested first)
     if (g == g0) wide_wait_pieces(c, c_first, c_first + P - 1, slot, tag);
@@ -721,7 +729,7 @@ __device__ __forceinline__ void wide_finish_share(Ctx& c, const OpDesc& op, int 
 __device__ __forceinline__ void linear_wide_shared(Ctx& c, const OpDesc& op, int T) {
   constexpr int NC = 32;  // token columns of a thread per round (128 token rows: two rounds)
   const KParams& p = c.p;
-  const int N = p.x_rows, nkt = op.nkt, nround = N > 2 * NC ? 2 : 1;
+  const int N = p.x_rows, nkt = op.nkt, split = wide_split<NC>(T), nround = split > NC ? 2 : 1;
   const int q = c.warp & 3, half = c.warp >> 2, row = 32 * q + c.lane;
   WideBest best;
   best.key[0] = best.key[1] = 0u;
@@ -742,8 +750,8 @@ __device__ __forceinline__ void linear_wide_shared(Ctx& c, const OpDesc& op, int
       const uint32_t acc = c.tmem + (c.acc_runs & 1u) * (uint32_t)N + ((uint32_t)(32 * q) << 16);
 #pragma unroll 1
       for (int cc = 0; cc < nround; ++cc) {
-        const int col0 = half * (N >> 1) + cc * NC;   // first token column of this thread's round
-        const int nlive = min(NC, T - col0);          // may be negative: nothing but padding
+        const int col0 = half * split + cc * NC;  // first token column of this thread's round
+        const int nlive = min(NC, (half == 0 ? min(split, T) : T) - col0);  // may be none or less: nothing but padding
         // the residual does not depend on the sums: requested first
         uint32_t res[NC / 2];
         wide_residual<NC>(op, with_res && finisher, blk * kTileRows + row, col0, nlive, res);
