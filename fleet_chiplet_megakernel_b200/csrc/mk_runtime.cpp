@@ -1586,7 +1586,7 @@ static int compile_program(mk_handle* h, bool first) {
   }
   const size_t partial_off = ll_bytes;  // wide path up to 32 token rows: the split sums of a CTA, as tagged words
   const bool words = !rows_mode && x_rows <= 32;
-  if (words) ll_bytes += (size_t)h->grid * mk::kTileRows * x_rows * 8;
+  if (words) ll_bytes += (size_t)h->grid * mk::kTileRows * x_rows * (x_rows > 16 ? 16 : 8);  // (two slots a CTA beyond 16 token rows)
   h->ll_buf = nullptr;
   h->ll_bytes = ll_bytes;
   // behind the words: the counters of the attention chunks and the flags of the split-k pieces

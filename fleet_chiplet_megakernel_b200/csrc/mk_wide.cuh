@@ -566,7 +566,70 @@ __device__ __forceinline__ void wide_store_best(const Ctx& c, const OpDesc& op, 
   }
 }
 
-// Up to 32 token rows.  NC: token columns of a thread, x_rows / 2
+// Up to 32 token rows: where a piece of a block lies.  Beyond 16 a CTA has two slots, for the block its range begins in and the one it
+// ends in.
+__device__ __forceinline__ uint4* wide_words(const KParams& p, int cta, int slot) {
+  return p.partial + ((size_t)cta * (MK_NC == 16 ? 2 : 1) + slot) * (size_t)(kTileRows * p.x_rows / 2);
+}
+// This CTA's share of a block's tokens, 17 to 32 token rows: of the four-token groups of each half, as many as there are CTAs to
+// share them, in CTA order.
+__device__ __forceinline__ void wide_finish_words(Ctx& c, const OpDesc& op, int T, int blk, unsigned total, int G, WideBest& best) {
+  const KParams& p = c.p;
+  const int half = c.warp >> 2, row = 32 * (c.warp & 3) + c.lane, col = blk * kTileRows + row;
+  const unsigned blk0 = (unsigned)blk * (unsigned)op.nkt;
+  const int c_first = tile_owner(blk0, total, G), P = tile_owner(blk0 + (unsigned)op.nkt - 1u, total, G) - c_first + 1, me = (int)blockIdx.x - c_first;
+  const int split = wide_split<16>(T), end = half == 0 ? min(split, T) : T;
+  const int groups = max(0, (end - half * split + 3) >> 2);
+  const int g0 = (me * groups + P - 1) / P, g1 = ((me + 1) * groups + P - 1) / P;
+  if (g0 >= g1) return;  // (the same in all four warps of a half)
+  const unsigned tag = ll_tag_of(c, c.cur_op);
+  const int slot = tile_begin((unsigned)c_first, total, (unsigned)G) == blk0 ? 0 : 1;  // of the first piece; the others open their CTA's range
+  const bool with_res = wide_with_res(c, op);
+#pragma unroll 1
+  for (int g = g0; g < g1; ++g) {
+    const int tok0 = half * split + 4 * g, nlive = min(4, end - tok0);
+    uint32_t res[2];
+    wide_residual<4>(op, with_res, col, tok0, nlive, res);  // (does not depend on the sums: requested first)
+    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    constexpr int PB = 6;  // pieces in flight per round
+#pragma unroll 1
+    for (int i0 = 0; i0 < P; i0 += PB) {
+      uint4 w[PB][2];
+#pragma unroll
+      for (int u = 0; u < PB; ++u)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const unsigned t = (i0 + u < P && 2 * i < nlive) ? ~tag : tag;  // (nothing to wait for: zeros)
+          w[u][i] = make_uint4(0u, t, 0u, t);
+        }
+      PollLimit limit;
+      while (true) {
+#pragma unroll
+        for (int u = 0; u < PB; ++u)
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            if (w[u][i].y != tag || w[u][i].w != tag)
+              w[u][i] = ld_gpu_words(wide_words(p, c_first + i0 + u, i0 + u == 0 ? slot : 0) + (size_t)((tok0 >> 1) + i) * kTileRows + row);
+        bool here = true;
+#pragma unroll
+        for (int u = 0; u < PB; ++u)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) here = here && w[u][i].y == tag && w[u][i].w == tag;
+        if (here || limit.expired(c, tag, w[0][0].y)) break;
+      }
+#pragma unroll
+      for (int u = 0; u < PB; ++u)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          v[2 * i] += __uint_as_float(w[u][i].x);
+          v[2 * i + 1] += __uint_as_float(w[u][i].z);
+        }
+    }
+    __syncwarp();  // (lanes leave the poll at different times; the epilogue shuffles)
+    wide_epilogue<4>(c, op, blk, row, tok0, nlive, v, res, best, 0, 4 * g);
+  }
+}
+// NC: token columns of a thread, x_rows / 2
 template <int NC>
 __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
   const KParams& p = c.p;
@@ -578,8 +641,8 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
   unsigned total, t0, t1;
   int G;
   if (wide_range(p, op, total, G, t0, t1)) {
-    const bool with_res = wide_with_res(c, op);
-    const size_t slot_vec = (size_t)kTileRows * N / 2;  // 16-byte vectors of a CTA's sums
+    const bool with_res = wide_with_res(c, op), share = NC == 16 && wide_shares(op.nblk, G);
+    int shared[2] = {-1, -1};  // blocks to finish with others: the one the range begins in, the one it ends in
     const unsigned tag = ll_tag_of(c, c.cur_op);
     const int col0 = half * wide_split<NC>(T);  // first token column of this thread
     const int nlive = half == 0 ? min(wide_split<NC>(T), T) : T - col0;  // may be none: nothing but padding
@@ -587,15 +650,15 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
     for (unsigned tile = t0; tile < t1;) {
       const int blk = (int)(tile / (unsigned)nkt);
       const unsigned blk0 = (unsigned)blk * (unsigned)nkt, blk1 = blk0 + (unsigned)nkt;
-      const bool finisher = tile == blk0;  // (only the first run of a range can belong to another CTA's block)
       const int c_last = tile_owner(blk1 - 1, total, G);
+      const bool first = tile == t0, finisher = tile == blk0 && (!share || c_last == (int)blockIdx.x);
       const uint32_t acc = c.tmem + (c.acc_runs & 1u) * (uint32_t)N + ((uint32_t)(32 * q) << 16);
       // the residual does not depend on the sums: requested first
       uint32_t res[NC / 2];
       wide_residual<NC>(op, with_res && finisher, blk * kTileRows + row, col0, nlive, res);
       mbar_wait(c, c.acc_full_bar(c.acc_runs & 1), (c.acc_runs >> 1) & 1u, ST_TIMEOUT_FULL);
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      if (tile == t0) MK_STAMP(c, 0);
+      if (first) MK_STAMP(c, 0);
       __syncwarp();
       uint32_t raw[NC];
       tmem_ld<NC>(acc + (uint32_t)col0, raw);
@@ -609,16 +672,18 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
 #pragma unroll
       for (int i = 0; i < NC; ++i) v[i] = __uint_as_float(raw[i]);
       if (!finisher) {
-        uint4* mine = p.partial + (size_t)blockIdx.x * slot_vec + (size_t)(col0 >> 1) * kTileRows + row;
+        uint4* mine = wide_words(p, (int)blockIdx.x, first ? 0 : 1) + (size_t)(col0 >> 1) * kTileRows + row;
 #pragma unroll
         for (int i = 0; i < NC / 2; ++i)
           if (2 * i < nlive) st_gpu_words(mine + (size_t)i * kTileRows, __float_as_uint(v[2 * i]), __float_as_uint(v[2 * i + 1]), tag);
+        if (share) (first ? shared[0] : shared[1]) = blk;
         MK_STAMP(c, 1);
         continue;
       }
       MK_STAMP(c, 2);
       if (c_last > (int)blockIdx.x) {
-        const uint4* src0 = p.partial + (size_t)(col0 >> 1) * kTileRows + row;
+        const uint4* src0 = wide_words(p, 0, 0) + (size_t)(col0 >> 1) * kTileRows + row;
+        const size_t stride = (size_t)(wide_words(p, 1, 0) - wide_words(p, 0, 0));
         // Several pieces in flight per round (registers allowing): a block of a small layer has up to `nkt` of them.
         constexpr int PB = NC == 8 ? 4 : 2;
 #pragma unroll 1
@@ -637,7 +702,7 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
             for (int u = 0; u < PB; ++u)
 #pragma unroll
               for (int i = 0; i < NC / 2; ++i)
-                if (w[u][i].y != tag || w[u][i].w != tag) w[u][i] = ld_gpu_words(src0 + (size_t)(cta + u) * slot_vec + (size_t)i * kTileRows);
+                if (w[u][i].y != tag || w[u][i].w != tag) w[u][i] = ld_gpu_words(src0 + (size_t)(cta + u) * stride + (size_t)i * kTileRows);
             bool here = true;
 #pragma unroll
             for (int u = 0; u < PB; ++u)
@@ -659,6 +724,15 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
       MK_STAMP(c, 4);
       wide_epilogue<NC>(c, op, blk, row, col0, nlive, v, res, best);
       MK_STAMP(c, 5);
+    }
+    if constexpr (NC == 16) {
+      // the block the range ends in first: its other CTAs began with it
+#pragma unroll 1
+      for (int i = 1; i >= 0; --i) {
+        const int blk = i == 1 ? shared[1] : shared[0];
+        if (blk >= 0) wide_finish_words(c, op, T, blk, total, G, best);
+      }
+      MK_STAMP(c, 6);
     }
   }
   if (op.flags & F_ARGMAX) wide_store_best<NC>(c, op, T, G, 1, best);
