@@ -770,14 +770,14 @@ __device__ __forceinline__ bool ll_ok(const uint4& a, const uint4& b, unsigned t
 struct PollLimit {
   unsigned spins = 0;
   unsigned long long t0 = 0;
-  __device__ __forceinline__ bool expired(const Ctx& c, unsigned tag, unsigned got) {
+  __device__ __forceinline__ bool expired(const Ctx& c, unsigned tag, unsigned got, int code = ST_TIMEOUT_DATA) {
     if (((++spins) & 63u) != 0) return false;
     if (aborted(c)) return true;
     const unsigned long long now = globaltimer();
     if (t0 == 0) {
       t0 = now;
     } else if (now - t0 > 2 * c.p.timeout_ns) {
-      raise_abort(c, ST_TIMEOUT_DATA, (int)tag, (int)got);
+      raise_abort(c, code, (int)tag, (int)got);
       return true;
     }
     return false;

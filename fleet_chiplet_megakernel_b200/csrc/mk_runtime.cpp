@@ -139,7 +139,6 @@ struct Program {
   mk::KParams kp{};
   int smem_bytes = 0;
   int64_t weight_bytes = 0;
-  int max_nblk = 1;
   void* ll_buf = nullptr;  // tagged words of the program, then its arrival counters: cleared before every kernel launch
   size_t clear_bytes = 0;
   size_t ll_bytes = 0;
@@ -153,7 +152,7 @@ struct mk_handle {
   std::vector<PlanOp> plan;
   bool planned = false, compiled = false, meta_set = false;
   bool rows_mode = false;  // linear layers run row-owner (F_ROWS)
-  // plan / rows_mode / kp / smem_bytes / weight_bytes / max_nblk above and below are the program being
+  // plan / rows_mode / kp / smem_bytes / weight_bytes above and below are the program being
   // built or, after compile, a copy of the primary program (what the introspection calls describe)
   Program prog[2];
   int nprog = 0;
@@ -166,7 +165,6 @@ struct mk_handle {
   int grid = 0, smem_bytes = 0;
   mk::KParams kp{};
   std::vector<void*> allocs;
-  int max_nblk = 1;
   int64_t weight_bytes = 0;
   bool launched = false;
   void* prof_ptr = nullptr;
@@ -1340,7 +1338,7 @@ static int compile_program(mk_handle* h, bool first) {
   // (row-owner mode prefers two resident token rows to one row and a stage more)
   int x_budget = kRowsXBudget;
   int x_bytes = 0;
-  int max_nblk = 1, n_linear = 0;
+  int n_linear = 0;
   bool has_moe = false, has_attn = false;
   if (rows_mode)
     for (const PlanOp& p : h->plan) {
@@ -1350,7 +1348,6 @@ static int compile_program(mk_handle* h, bool first) {
     }
   for (PlanOp& p : h->plan) {
     if (p.type == mk::OP_LINEAR) {
-      max_nblk = std::max(max_nblk, (p.n + mk::kTileRows - 1) / mk::kTileRows);
       ++n_linear;
       if (!rows_mode) continue;  // the input arrives as activation boxes that ride with the weight stages
       const int kp = (p.k + mk::kRowsStageK - 1) / mk::kRowsStageK * mk::kRowsStageK;
@@ -1428,7 +1425,6 @@ static int compile_program(mk_handle* h, bool first) {
     return h->fail(MK_E_INVALID, "cluster_size must be 0, 1, 2 or 4");
   }
   kp.bar_epoch0 = cfg.test_barrier_epoch;
-  h->max_nblk = max_nblk;
   // row-owner LM head: one (max, index) partial per CTA that owns rows
   for (size_t i = 0; i < h->plan.size(); ++i) {
     PlanOp& po = h->plan[i];
@@ -1586,7 +1582,7 @@ static int compile_program(mk_handle* h, bool first) {
   }
   const size_t partial_off = ll_bytes;  // wide path up to 32 token rows: the split sums of a CTA, as tagged words
   const bool words = !rows_mode && x_rows <= 32;
-  if (words) ll_bytes += (size_t)h->grid * mk::kTileRows * x_rows * (x_rows > 16 ? 16 : 8);  // (two slots a CTA beyond 16 token rows)
+  if (words) ll_bytes += (size_t)h->grid * mk::kTileRows * x_rows * 2 * 8;
   h->ll_buf = nullptr;
   h->ll_bytes = ll_bytes;
   // behind the words: the counters of the attention chunks and the flags of the split-k pieces
@@ -1966,7 +1962,6 @@ int mk_compile(mk_handle* h) {
   if (int e = compile_program(h, true)) return e;
   h->prog[0].plan = h->plan; h->prog[0].rows_mode = h->rows_mode; h->prog[0].max_tokens = h->plan_tokens;
   h->prog[0].kp = h->kp; h->prog[0].smem_bytes = h->smem_bytes; h->prog[0].weight_bytes = h->weight_bytes;
-  h->prog[0].max_nblk = h->max_nblk;
   h->prog[0].ll_buf = h->ll_buf; h->prog[0].ll_bytes = h->ll_bytes; h->prog[0].clear_bytes = h->clear_bytes;
   h->nprog = 1;
   if (two) {
@@ -1975,8 +1970,7 @@ int mk_compile(mk_handle* h) {
     if (int e = compile_program(h, false)) return e;
     h->prog[1].plan = h->plan; h->prog[1].rows_mode = h->rows_mode; h->prog[1].max_tokens = h->plan_tokens;
     h->prog[1].kp = h->kp; h->prog[1].smem_bytes = h->smem_bytes; h->prog[1].weight_bytes = h->weight_bytes;
-    h->prog[1].max_nblk = h->max_nblk;
-      h->prog[1].ll_buf = h->ll_buf; h->prog[1].ll_bytes = h->ll_bytes; h->prog[1].clear_bytes = h->clear_bytes;
+    h->prog[1].ll_buf = h->ll_buf; h->prog[1].ll_bytes = h->ll_bytes; h->prog[1].clear_bytes = h->clear_bytes;
     h->nprog = 2;
     h->prog[0].kp.tok_lo = 1;
     h->prog[0].kp.tok_hi = h->prog[0].max_tokens;
@@ -1984,7 +1978,7 @@ int mk_compile(mk_handle* h) {
     h->prog[1].kp.tok_hi = h->prog[1].max_tokens;
     // the handle's own copies describe the primary program again
     h->plan = h->prog[0].plan; h->rows_mode = h->prog[0].rows_mode; h->kp = h->prog[0].kp;
-    h->smem_bytes = h->prog[0].smem_bytes; h->weight_bytes = h->prog[0].weight_bytes; h->max_nblk = h->prog[0].max_nblk;
+    h->smem_bytes = h->prog[0].smem_bytes; h->weight_bytes = h->prog[0].weight_bytes;
     h->plan_tokens = h->prog[0].max_tokens;
   } else {
     h->prog[0].kp.tok_lo = 1;

@@ -305,10 +305,14 @@ __host__ __device__ inline int wide_ctas(int grid, int nblk, int nkt) {
   return total < (unsigned)grid ? (int)total : grid;
 }
 
-// Beyond 32 token rows: whether the CTAs of a row block share its finish (see mk_wide.cuh).  With more blocks than half the CTAs a
-// CTA has about a block to finish either way, and two shares in turn take longer than one block at once: 8B width, 64 requests,
+// Whether the CTAs of a row block share its finish (see mk_wide.cuh); x_rows: token rows of a box.  With more blocks than half the
+// CTAs a CTA has about a block to finish either way, and two shares in turn take longer than one block at once: 8B width, 64 requests,
 // gate/up (192 blocks) 39.8 us shared and 36.4 by one CTA; QKV (48) 18.9 and 20.2, O and down (32) 13.2 and 16.0, 22.5 and 26.5.
-__host__ __device__ inline bool wide_shares(int nblk, int ctas) { return 2 * nblk <= ctas; }
+// Up to 16 token rows shares are of two tokens, and the line lies between QKV of 8B width, which is finished a head vector at a
+// time, and its O and down: 16 requests without any of them, with O and down and with all three 1237, 1221 and 1239 us per step.  12 layers
+// of 2048 hidden, 4 and 16 requests without any shares 674 and 708, now 652 and 682; four of 1024 185 and 207, now 172 and 200; six of
+// 512, 16 requests 247 and 234.
+__host__ __device__ inline bool wide_shares(int nblk, int ctas, int x_rows) { return (x_rows <= 16 ? 4 : 2) * nblk <= ctas; }
 
 static_assert(sizeof(OpDesc) % 16 == 0 && sizeof(OpDesc) <= 256, "OpDesc is copied to shared memory in 16-byte pieces");
 

@@ -365,16 +365,17 @@ __device__ __forceinline__ void norm_loop(Ctx& c) {
 // a thread holds one output row for up to 32 tokens in registers, from tensor memory to the store.
 //
 // Several CTAs hold k-ranges of a row block; their sums are added up in CTA order.  No CTA-wide sync and no shared memory on the way.
-//  * Up to 32 token rows (linear_wide) the CTA with the block's FIRST k-range finishes it (that range is the tail of its own tile
-//    range, so it is computed last anyway).  The others store their sums as words that carry a tag, two tokens per 16 bytes,
-//    [token / 2][row], and a finishing thread polls those of its own output row, several pieces at once: data and "ready" arrive in one
-//    load, with no release behind the stores, no flag and no second round trip.  The tag differs in every op of every
-//    iteration, the words are cleared before every launch, and a CTA's slot is written again only behind a grid barrier.
-//  * Beyond (linear_wide_shared) the bytes cost more than the round trip, and one CTA per block would read four to six pieces of
-//    32 KB and more in turn, 7 us of a linear's end.  So every CTA of a block finishes its share of the tokens: all of them store their
-//    sums, plain float4 of four tokens, [token / 4][row], every warp publishes its share with a release of its own (a flag that holds the
-//    op's tag), and behind the op's last tile a warp waits for the matching warps of the block's CTAs.
-//    MEASURED_SHARED
+//  * A block is finished by the CTA with its FIRST k-range (that range is the tail of its own tile range, so it is computed last
+//    anyway), or, where there are few blocks (wide_shares), by all of its CTAs, each a share of the tokens, behind the op's last tile: one
+//    CTA would read up to six pieces and more in turn, 5 to 7 us of a linear's end.
+//  * Up to 32 token rows (linear_wide) sums travel as words that carry a tag, two tokens per 16 bytes, [token / 2][row], and
+//    a finishing thread polls those of its own output row, several pieces at once: data and "ready" arrive in one load, with no
+//    release behind the stores, no flag and no second round trip.  The tag differs in every op of every iteration, the words are
+//    cleared before every launch, and a CTA's slot is written again only behind a grid barrier.
+//  * Beyond (linear_wide_shared), twice the bytes cost more than the round trip: plain float4 of four tokens, [token / 4][row]; every
+//    warp publishes its share with a release of its own, a flag that holds the op's tag, for the matching warps of the other CTAs.
+// 12 layers of 8B width, us per step with one finishing CTA per block and with shares: 64 requests 1671 and 1573, 100 2193 and
+// 2053; 17 1324 and 1294, 32 1400 and 1391; 2048 hidden, 32 requests 890 and 811.
 __device__ __forceinline__ uint32_t order_bf16(float v) {  // monotone 16-bit key of a bf16 value; 0 only for NaN
   const uint32_t b = __float_as_uint(v + 0.f) >> 16;       // (-0 counts as +0)
   const uint32_t k = (b & 0x8000u) ? (~b & 0xffffu) : (b | 0x8000u);
@@ -566,20 +567,21 @@ __device__ __forceinline__ void wide_store_best(const Ctx& c, const OpDesc& op, 
   }
 }
 
-// Up to 32 token rows: where a piece of a block lies.  Beyond 16 a CTA has two slots, for the block its range begins in and the one it
-// ends in.
+// Up to 32 token rows: where a piece of a block lies.  A CTA has two slots: the block its range begins in, and the one it ends in.
 __device__ __forceinline__ uint4* wide_words(const KParams& p, int cta, int slot) {
-  return p.partial + ((size_t)cta * (MK_NC == 16 ? 2 : 1) + slot) * (size_t)(kTileRows * p.x_rows / 2);
+  return p.partial + ((size_t)cta * 2 + slot) * (size_t)(kTileRows * p.x_rows / 2);
 }
-// This CTA's share of a block's tokens, 17 to 32 token rows: of the four-token groups of each half, as many as there are CTAs to
-// share them, in CTA order.
+// This CTA's share of a block's tokens: of the groups of NC / 4 tokens of each half, as many as there are CTAs to share them, in CTA
+// order.
+template <int NC>
 __device__ __forceinline__ void wide_finish_words(Ctx& c, const OpDesc& op, int T, int blk, unsigned total, int G, WideBest& best) {
+  constexpr int NT = NC / 4;
   const KParams& p = c.p;
   const int half = c.warp >> 2, row = 32 * (c.warp & 3) + c.lane, col = blk * kTileRows + row;
   const unsigned blk0 = (unsigned)blk * (unsigned)op.nkt;
   const int c_first = tile_owner(blk0, total, G), P = tile_owner(blk0 + (unsigned)op.nkt - 1u, total, G) - c_first + 1, me = (int)blockIdx.x - c_first;
-  const int split = wide_split<16>(T), end = half == 0 ? min(split, T) : T;
-  const int groups = max(0, (end - half * split + 3) >> 2);
+  const int split = wide_split<NC>(T), end = half == 0 ? min(split, T) : T;
+  const int groups = max(0, (end - half * split + NT - 1) / NT);
   const int g0 = (me * groups + P - 1) / P, g1 = ((me + 1) * groups + P - 1) / P;
   if (g0 >= g1) return;  // (the same in all four warps of a half)
   const unsigned tag = ll_tag_of(c, c.cur_op);
@@ -587,18 +589,20 @@ __device__ __forceinline__ void wide_finish_words(Ctx& c, const OpDesc& op, int 
   const bool with_res = wide_with_res(c, op);
 #pragma unroll 1
   for (int g = g0; g < g1; ++g) {
-    const int tok0 = half * split + 4 * g, nlive = min(4, end - tok0);
-    uint32_t res[2];
-    wide_residual<4>(op, with_res, col, tok0, nlive, res);  // (does not depend on the sums: requested first)
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
+    const int tok0 = half * split + NT * g, nlive = min(NT, end - tok0);
+    uint32_t res[NT / 2];
+    wide_residual<NT>(op, with_res, col, tok0, nlive, res);  // (does not depend on the sums: requested first)
+    float v[NT];
+#pragma unroll
+    for (int i = 0; i < NT; ++i) v[i] = 0.f;
     constexpr int PB = 6;  // pieces in flight per round
 #pragma unroll 1
     for (int i0 = 0; i0 < P; i0 += PB) {
-      uint4 w[PB][2];
+      uint4 w[PB][NT / 2];
 #pragma unroll
       for (int u = 0; u < PB; ++u)
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < NT / 2; ++i) {
           const unsigned t = (i0 + u < P && 2 * i < nlive) ? ~tag : tag;  // (nothing to wait for: zeros)
           w[u][i] = make_uint4(0u, t, 0u, t);
         }
@@ -607,26 +611,26 @@ __device__ __forceinline__ void wide_finish_words(Ctx& c, const OpDesc& op, int 
 #pragma unroll
         for (int u = 0; u < PB; ++u)
 #pragma unroll
-          for (int i = 0; i < 2; ++i)
+          for (int i = 0; i < NT / 2; ++i)
             if (w[u][i].y != tag || w[u][i].w != tag)
               w[u][i] = ld_gpu_words(wide_words(p, c_first + i0 + u, i0 + u == 0 ? slot : 0) + (size_t)((tok0 >> 1) + i) * kTileRows + row);
         bool here = true;
 #pragma unroll
         for (int u = 0; u < PB; ++u)
 #pragma unroll
-          for (int i = 0; i < 2; ++i) here = here && w[u][i].y == tag && w[u][i].w == tag;
+          for (int i = 0; i < NT / 2; ++i) here = here && w[u][i].y == tag && w[u][i].w == tag;
         if (here || limit.expired(c, tag, w[0][0].y)) break;
       }
 #pragma unroll
       for (int u = 0; u < PB; ++u)
 #pragma unroll
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < NT / 2; ++i) {
           v[2 * i] += __uint_as_float(w[u][i].x);
           v[2 * i + 1] += __uint_as_float(w[u][i].z);
         }
     }
     __syncwarp();  // (lanes leave the poll at different times; the epilogue shuffles)
-    wide_epilogue<4>(c, op, blk, row, tok0, nlive, v, res, best, 0, 4 * g);
+    wide_epilogue<NT>(c, op, blk, row, tok0, nlive, v, res, best, 0, NT * g);
   }
 }
 // NC: token columns of a thread, x_rows / 2
@@ -641,7 +645,7 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
   unsigned total, t0, t1;
   int G;
   if (wide_range(p, op, total, G, t0, t1)) {
-    const bool with_res = wide_with_res(c, op), share = NC == 16 && wide_shares(op.nblk, G);
+    const bool with_res = wide_with_res(c, op), share = wide_shares(op.nblk, G, N);
     int shared[2] = {-1, -1};  // blocks to finish with others: the one the range begins in, the one it ends in
     const unsigned tag = ll_tag_of(c, c.cur_op);
     const int col0 = half * wide_split<NC>(T);  // first token column of this thread
@@ -725,15 +729,13 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
       wide_epilogue<NC>(c, op, blk, row, col0, nlive, v, res, best);
       MK_STAMP(c, 5);
     }
-    if constexpr (NC == 16) {
-      // the block the range ends in first: its other CTAs began with it
+    // the block the range ends in first: its other CTAs began with it
 #pragma unroll 1
-      for (int i = 1; i >= 0; --i) {
-        const int blk = i == 1 ? shared[1] : shared[0];
-        if (blk >= 0) wide_finish_words(c, op, T, blk, total, G, best);
-      }
-      MK_STAMP(c, 6);
+    for (int i = 1; i >= 0; --i) {
+      const int blk = i == 1 ? shared[1] : shared[0];
+      if (blk >= 0) wide_finish_words<NC>(c, op, T, blk, total, G, best);
     }
+    MK_STAMP(c, 6);
   }
   if (op.flags & F_ARGMAX) wide_store_best<NC>(c, op, T, G, 1, best);
 }
@@ -749,7 +751,7 @@ __device__ __forceinline__ void wide_wait_pieces(const Ctx& c, int c0, int c1, i
     const unsigned* flag = wide_flag(c.p, cta, cta == c0 ? slot : 0) + c.warp;
     PollLimit limit;
     unsigned got;
-    while ((got = ld_acquire_u32(flag)) != tag && !limit.expired(c, tag, got)) {
+    while ((got = ld_acquire_u32(flag)) != tag && !limit.expired(c, tag, got, ST_TIMEOUT_PEER)) {
     }
   }
   __syncwarp();
@@ -811,7 +813,7 @@ __device__ __forceinline__ void linear_wide_shared(Ctx& c, const OpDesc& op, int
   unsigned total, t0, t1;
   int G;
   if (wide_range(p, op, total, G, t0, t1)) {
-    const bool with_res = wide_with_res(c, op), share = wide_shares(op.nblk, G);
+    const bool with_res = wide_with_res(c, op), share = wide_shares(op.nblk, G, N);
     const unsigned tag = ll_tag_of(c, c.cur_op);
     int shared[2] = {-1, -1};  // blocks to finish with others: the one the range begins in, the one it ends in
 #pragma unroll 1
