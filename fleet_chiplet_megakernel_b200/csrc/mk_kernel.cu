@@ -2604,113 +2604,196 @@ __device__ __forceinline__ void op_allreduce(Ctx& c, const OpDesc& op, int T) {
 }
 
 // ------------------------------------------------------------------------------------
-// continuous-batching bookkeeping between iterations (CTA 0, one thread)
+// continuous-batching bookkeeping between iterations (the consumers of CTA 0)
 // ------------------------------------------------------------------------------------
-// Same protocol as the reference's offline mode (persistent_kernel.cuh:380-536):
-// append the sampled tokens, retire finished requests and free their pages,
-// compact the survivors, give each one more token, admit new requests, and
-// leave the number of active tokens in qo_indptr[max_reqs].  It is split in two so
-// that a launch bounded by max_iters still appends its last tokens before it ends.
-// Part 1, after an iteration: append the sampled tokens, advance step[], retire
-// finished requests and return their pages.
-__device__ __forceinline__ void bookkeep_finish(const KParams& p) {
-  const int R = p.max_reqs;
-  int tail = p.sched[1];
-  for (int i = 0; i < R; ++i) {
-    const int rid = p.request_ids[i];
-    if (rid < 0) continue;
-    int st = p.step[rid];
-    const int q0 = p.qo_indptr[i];
-    const int n = p.qo_indptr[i + 1] - q0;
-    const int pl = p.prompt_lengths[rid];
-    for (int j = 0; j < n; ++j) {
-      const int pos = st + j + 1;
-      if (pos >= pl && pos < p.max_seq_len) p.tokens[(size_t)rid * p.max_seq_len + pos] = p.output_tokens[q0 + j];
+// Same protocol as the reference's offline mode (persistent_kernel.cuh:380-536): append the sampled tokens, retire finished
+// requests and free their pages (`finish`: skipped when there are none to append, alone when a launch bounded by max_iters ends);
+// compact the survivors, give each one more token, or a chunk of its prompt as far as the iteration's budget goes, and the pages
+// it needs, admit new requests (`prepare`).  Returns the active tokens.
+//
+// All requests at once, thread i for request i (the host admits at most 128): what used to run on along the list are prefix sums, tokens
+// cut off at the budget.  Lists of pages and prompt chunks are copied by warps.  One thread took three dependent round trips
+// a request: us between two iterations at 1, 8, 32 and 64 requests 7.9, 14, 42 and 90, now 3, 6, 14 and 11.
+struct Sum3 {
+  int a, b, c;
+};
+// Sums over the threads before this one; `all`: over all of them.
+__device__ __forceinline__ Sum3 book_sums(Ctx& c, Sum3 v, Sum3& all) {
+  int* r = reinterpret_cast<int*>(c.red());  // 8 warps x 3
+  const Sum3 own = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int a = __shfl_up_sync(0xffffffffu, v.a, o), b = __shfl_up_sync(0xffffffffu, v.b, o), d = __shfl_up_sync(0xffffffffu, v.c, o);
+    if (c.lane >= o) {
+      v.a += a;
+      v.b += b;
+      v.c += d;
     }
+  }
+  if (c.lane == 31) {
+    r[c.warp * 3] = v.a;
+    r[c.warp * 3 + 1] = v.b;
+    r[c.warp * 3 + 2] = v.c;
+  }
+  consumer_sync();
+  all.a = all.b = all.c = 0;
+#pragma unroll
+  for (int w = 0; w < kNumConsumerWarps; ++w) {
+    if (w == c.warp) {
+      v.a += all.a;
+      v.b += all.b;
+      v.c += all.c;
+    }
+    all.a += r[w * 3];
+    all.b += r[w * 3 + 1];
+    all.c += r[w * 3 + 2];
+  }
+  consumer_sync();
+  v.a -= own.a;
+  v.b -= own.b;
+  v.c -= own.c;
+  return v;
+}
+constexpr int kBookReqs = 128;
+static_assert(kBookReqs <= kNumConsumers, "a thread per request");
+// What a warp copies of a request: n of a list (of row `row`) from `from` on, to `to`.  In the scratch region behind the sums: one for
+// each request, on the row-owner path at most two.
+struct BookList {
+  int row, from, to, n;
+};
+static_assert(256 + kBookReqs * sizeof(BookList) <= kWideRedBytes, "the lists fit the scratch region");
+__device__ __forceinline__ BookList* book_lists(const Ctx& c) { return reinterpret_cast<BookList*>(c.smem + c.p.red_off + 256); }
+
+// Prompt chunks, but for their first tokens
+__device__ __forceinline__ void book_chunks(Ctx& c, bool any, bool mine, int i, int rid, int from, int to, int n) {
+  if (!any) return;
+  const KParams& p = c.p;
+  BookList* list = book_lists(c);
+  if (i < p.max_reqs) list[i] = {rid, from, to, mine ? n : 0};
+  consumer_sync();
+#pragma unroll 1
+  for (int r = c.warp; r < p.max_reqs; r += kNumConsumerWarps)
+    for (int j = 1 + c.lane; j < list[r].n; j += 32) p.input_tokens[list[r].to + j] = __ldcg(p.tokens + (size_t)list[r].row * p.max_seq_len + list[r].from + j);
+  consumer_sync();
+}
+__device__ __forceinline__ int bookkeep(Ctx& c, bool finish, bool prepare, int* table) {
+  const KParams& p = c.p;
+  BookList* list = book_lists(c);
+  const int R = p.max_reqs, i = c.tid, page = p.page_size;
+  const bool slot = i < R;
+  int rid = slot ? __ldcg(p.request_ids + i) : -1;
+  const int q0 = slot ? __ldcg(p.qo_indptr + i) : 0, q1 = slot ? __ldcg(p.qo_indptr + i + 1) : 0;
+  const int k0 = slot ? __ldcg(p.kv_indptr + i) : 0, k1 = slot ? __ldcg(p.kv_indptr + i + 1) : 0;
+  const int n_old = __ldcg(p.kv_indptr + R), next = __ldcg(p.sched + 2);
+  int head = __ldcg(p.sched), tail = __ldcg(p.sched + 1);
+  int st = 0, pl = 0;
+  if (rid >= 0) {
+    st = __ldcg(p.step + rid);
+    pl = __ldcg(p.prompt_lengths + rid);
+  }
+  long long* row = p.tokens + (size_t)max(rid, 0) * p.max_seq_len;
+  int freed = 0;
+  if (finish && rid >= 0) {
+    const int n = q1 - q0;
+    for (int j = max(0, pl - st - 1); j < n; ++j)
+      if (st + j + 1 < p.max_seq_len) row[st + j + 1] = __ldcg(p.output_tokens + q0 + j);
     st += n;
     p.step[rid] = st;
-    const bool done = (st + 1 >= p.max_seq_len) ||
-                      (st >= pl && p.tokens[(size_t)rid * p.max_seq_len + st] == p.eos);
-    if (done) {
-      p.request_ids[i] = -1;
-      const int k0 = p.kv_indptr[i], k1 = p.kv_indptr[i + 1];
-      for (int j = k0; j < k1; ++j) {
-        p.page_queue[tail % p.max_pages] = p.kv_indices[j];
-        ++tail;
-      }
+    if (st + 1 >= p.max_seq_len || (st >= pl && __ldcg(row + st) == p.eos)) {
+      freed = k1 - k0;
+      rid = -1;
+      if (!prepare) p.request_ids[i] = -1;
     }
   }
-  p.sched[1] = tail;
-}
-
-// Part 2, before an iteration: compact the surviving requests, give each one more
-// token and the page it needs, admit new requests.  Returns the active tokens.
-__device__ __forceinline__ int bookkeep_prepare(const KParams& p, int* table, int iter) {
-  const int R = p.max_reqs;
-  int head = p.sched[0], tail = p.sched[1];
-  const int n_old = p.kv_indptr[R];
-  int* old_idx = n_old <= p.page_entries ? table : p.page_scratch;
-  for (int i = 0; i < n_old; ++i) old_idx[i] = p.kv_indices[i];
-  int nreq = 0, ntok = 0, npages = 0;
-  for (int i = 0; i < R; ++i) {
-    const int rid = p.request_ids[i];
-    if (rid < 0) continue;
-    const int k0 = p.kv_indptr[i];
-    const int have = p.kv_indptr[i + 1] - k0;
-    p.request_ids[nreq] = rid;
-    p.qo_indptr[nreq] = ntok;
-    p.kv_indptr[nreq] = npages;
-    const int st = p.step[rid];
-    // a request still inside its prompt gets a chunk of it (as many tokens as the budget allows), a
-    // decoding one its single token; either may get nothing when the iteration's budget is spent
-    const int left = p.prompt_lengths[rid] - st;
-    const int budget = p.max_tokens - ntok;
-    const int nnew = left > 0 ? min(left, min(p.max_tokens_per_req, budget)) : min(1, budget);
-    for (int j = 0; j < nnew; ++j) p.input_tokens[ntok + j] = p.tokens[(size_t)rid * p.max_seq_len + st + j];
-    const int need = (st + nnew + p.page_size - 1) / p.page_size;
-    const int last = (st + nnew) % p.page_size;
-    p.kv_last_page_len[nreq] = last == 0 ? p.page_size : last;
-    for (int j = 0; j < have; ++j) p.kv_indices[npages + j] = old_idx[k0 + j];
-    for (int j = have; j < need; ++j) {
-      if (tail - head <= 0) {
-        raise_abort_at(&p, iter, -1, ST_OUT_OF_PAGES, rid, need);
-        return 0;
-      }
-      p.kv_indices[npages + j] = p.page_queue[head % p.max_pages];
-      ++head;
-    }
-    npages += need > have ? need : have;
-    ntok += nnew;
-    ++nreq;
+  // a request still inside its prompt gets a chunk of it (as many tokens as the budget allows), a decoding one its single
+  // token; either may get nothing when the iteration's budget is spent
+  const bool alive = rid >= 0;
+  const int left = pl - st, want = alive ? (left > 0 ? min(left, p.max_tokens_per_req) : 1) : 0;
+  Sum3 all;
+  const Sum3 at = book_sums(c, {freed, alive ? 1 : 0, want}, all);
+  const int nrun = all.b;
+  int ntok = min(all.c, p.max_tokens);
+  if (all.a > 0) {  // pages that are free again, behind the others
+    if (slot) list[i] = {0, k0, tail + at.a, freed};
+    consumer_sync();
+#pragma unroll 1
+    for (int r = c.warp; r < R; r += kNumConsumerWarps)
+      for (int j = c.lane; j < list[r].n; j += 32) p.page_queue[(list[r].to + j) % p.max_pages] = __ldcg(p.kv_indices + list[r].from + j);
+    tail += all.a;
+    consumer_sync();
   }
-  while (nreq < R && ntok < p.max_tokens) {
-    const int rid = p.sched[2];
-    if (rid >= p.total_requests) break;
-    const int nnew = max(1, min(p.prompt_lengths[rid], min(p.max_tokens_per_req, p.max_tokens - ntok)));
-    const int need = (nnew + p.page_size - 1) / p.page_size;
-    if (tail - head < need) break;  // no pages for a new request yet: admit it later
-    p.request_ids[nreq] = rid;
-    p.qo_indptr[nreq] = ntok;
-    p.kv_indptr[nreq] = npages;
-    for (int j = 0; j < nnew; ++j) p.input_tokens[ntok + j] = p.tokens[(size_t)rid * p.max_seq_len + j];
-    const int last = nnew % p.page_size;
-    p.kv_last_page_len[nreq] = last == 0 ? p.page_size : last;
-    for (int j = 0; j < need; ++j) {
-      p.kv_indices[npages + j] = p.page_queue[head % p.max_pages];
-      ++head;
-    }
-    npages += need;
-    ntok += nnew;
-    ++nreq;
-    p.sched[2] = rid + 1;
+  if (!prepare) {
+    if (c.tid == 0) p.sched[1] = tail;
+    return 0;
   }
-  for (int i = nreq; i < R; ++i) p.request_ids[i] = -1;
-  for (int i = nreq; i <= R; ++i) {
+  const int t0 = min(at.c, p.max_tokens), nnew = min(want, p.max_tokens - t0);
+  const int have = alive ? k1 - k0 : 0, pages = alive ? max(have, (st + nnew + page - 1) / page) : 0;
+  const Sum3 pg = book_sums(c, {pages, pages - have, nnew > 1 ? 1 : 0}, all);
+  if (all.b > tail - head) {
+    if (pg.b <= tail - head && pg.b + pages - have > tail - head)  // (the first that gets none)
+      raise_abort_at(&p, c.iter, -1, ST_OUT_OF_PAGES, rid, pages);
+    return 0;
+  }
+  int npages = all.a;
+  if (all.b > 0 || npages != n_old) {  // lists change their places: all of them out of the table first
+    int* old_idx = n_old <= p.page_entries ? table : p.page_scratch;
+#pragma unroll 1
+    for (int j = c.tid; j < n_old; j += kNumConsumers) old_idx[j] = __ldcg(p.kv_indices + j);
+    if (slot) list[i] = {0, k0, pg.a, have};
+    consumer_sync();
+#pragma unroll 1
+    for (int r = c.warp; r < R; r += kNumConsumerWarps)
+      for (int j = c.lane; j < list[r].n; j += 32) p.kv_indices[list[r].to + j] = old_idx[list[r].from + j];
+    for (int j = have; j < pages; ++j) p.kv_indices[pg.a + j] = __ldcg(p.page_queue + (head + pg.b + j - have) % p.max_pages);
+    head += all.b;
+    consumer_sync();
+  }
+  if (alive) {
+    p.request_ids[at.b] = rid;
+    p.qo_indptr[at.b] = t0;
+    p.kv_indptr[at.b] = pg.a;
+    const int last = (st + nnew) % page;
+    p.kv_last_page_len[at.b] = last == 0 ? page : last;
+    if (nnew > 0) p.input_tokens[t0] = __ldcg(row + st);
+  }
+  book_chunks(c, all.c > 0, alive, i, rid, st, t0, nnew);
+  // new requests: as many of the next ones as there are places, tokens of the budget and pages for
+  int nreq = nrun;
+  if (nreq < R && ntok < p.max_tokens && next < p.total_requests) {
+    const int r = next + i;
+    const bool may = i < R - nreq && r < p.total_requests;
+    const int w = may ? max(1, min(__ldcg(p.prompt_lengths + r), p.max_tokens_per_req)) : 0;
+    const Sum3 s = book_sums(c, {w, 0, 0}, all);
+    const int q = ntok + s.a, n = may && q < p.max_tokens ? min(w, p.max_tokens - q) : 0, pgs = (n + page - 1) / page;
+    const Sum3 u = book_sums(c, {pgs, 0, 0}, all);
+    const bool ok = n > 0 && u.a + pgs <= tail - head;  // (where one has to wait for pages, the later ones do too: the sums grow)
+    if (ok) {
+      p.request_ids[nreq + i] = r;
+      p.qo_indptr[nreq + i] = q;
+      p.kv_indptr[nreq + i] = npages + u.a;
+      const int last = n % page;
+      p.kv_last_page_len[nreq + i] = last == 0 ? page : last;
+      for (int j = 0; j < pgs; ++j) p.kv_indices[npages + u.a + j] = __ldcg(p.page_queue + (head + u.a + j) % p.max_pages);
+      p.input_tokens[q] = __ldcg(p.tokens + (size_t)r * p.max_seq_len);
+    }
+    const Sum3 got = book_sums(c, {ok ? 1 : 0, ok ? n : 0, ok ? pgs : 0}, all);
+    (void)got;
+    book_chunks(c, all.b > all.a, ok, i, r, 0, q, n);
+    nreq += all.a;
+    ntok += all.b;
+    npages += all.c;
+    head += all.c;
+  }
+  if (slot && i >= nreq) p.request_ids[i] = -1;
+  if (i <= R && i >= nreq) {
     p.qo_indptr[i] = ntok;
     p.kv_indptr[i] = npages;
   }
-  p.sched[0] = head;
-  p.sched[1] = tail;
+  if (c.tid == 0) {
+    p.sched[0] = head;
+    p.sched[1] = tail;
+    p.sched[2] = next + nreq - nrun;
+  }
   return ntok;
 }
 
@@ -3358,35 +3441,29 @@ __global__ void __launch_bounds__(kNumThreads, 1) megakernel(const __grid_consta
       if (prof && c.tid == 0) prof[((size_t)p.num_ops * gridDim.x + blockIdx.x) * 4 + 0] = globaltimer();
       if (p.mode == MODE_OFFLINE) {
         if (blockIdx.x == 0) {
-          consumer_sync();
-          if (c.tid == 0) {
-            int n = 0;
-            const int done_before = p.sched[7];  // iterations completed by earlier kernels of this generation call
-            const int git = done_before + iter;  // this iteration's number within the call
-            bool hand_over = false;
-            if (!aborted(c)) {
-              if (iter == 1 && p.sched[5] > 0) {
-                // prepared by the kernel that handed this iteration over
-                n = p.sched[5];
-                p.sched[5] = 0;
-              } else {
-                // sched[4] != 0: the last iteration's outputs have not been appended yet
-                if (p.sched[4] != 0) bookkeep_finish(c.p);
-                p.sched[4] = 0;
-                if (p.max_iters == 0 || git <= p.max_iters) {
-                  // (the page table goes through the weight ring: no stage is under way between two iterations)
-                  n = bookkeep_prepare(c.p, reinterpret_cast<int*>(c.smem), iter);
-                  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // TMA writes there next
-                  if (n > 0) p.sched[4] = 1;
-                }
-              }
-              if (n > 0 && (n < p.tok_lo || n > p.tok_hi)) {
-                // not an iteration for this program: leave it prepared and let the host launch the other one
-                p.sched[5] = n;
-                p.sched[7] = git - 1;
-                hand_over = true;
-              }
+          const int prepared = __ldcg(p.sched + 5), appended = __ldcg(p.sched + 4);
+          const int git = __ldcg(p.sched + 7) + iter;  // this iteration's number within the call (sched[7]: of earlier kernels)
+          int n = 0;
+          bool hand_over = false;
+          if (!bar_any(1, kNumConsumers, c.tid == 0 && aborted(c))) {  // (all threads take thread 0's view)
+            if (iter == 1 && prepared > 0) {
+              n = prepared;  // by the kernel that handed this iteration over
+            } else {
+              // sched[4] != 0: the last iteration's outputs have not been appended yet
+              const bool prepare = p.max_iters == 0 || git <= p.max_iters;
+              // (the page table goes through the weight ring: no stage is under way between two iterations)
+              if (appended != 0 || prepare) n = bookkeep(c, appended != 0, prepare, reinterpret_cast<int*>(c.smem));
+              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // TMA writes there next
+              if (c.tid == 0) p.sched[4] = n > 0 ? 1 : 0;
             }
+            // not an iteration for this program: leave it prepared and let the host launch the other one
+            hand_over = n > 0 && (n < p.tok_lo || n > p.tok_hi);
+            if (c.tid == 0) {
+              p.sched[5] = hand_over ? n : 0;
+              if (hand_over) p.sched[7] = git - 1;
+            }
+          }
+          if (c.tid == 0) {
             if (!hand_over && git - 1 < p.max_step_times) {
               p.step_times[2 * (git - 1)] = globaltimer();
               p.step_times[2 * (git - 1) + 1] = (unsigned long long)n;

@@ -1,0 +1,99 @@
+"""The scheduler between two iterations (admission, prompt chunks under a token budget, pages, retirement), against the same rules
+followed request by request on the host."""
+import pytest
+import torch
+
+import fleet_chiplet_megakernel_b200 as mk
+from oracle import qwen3_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+class _Host:
+    """One request after the other, as the reference's offline mode does it."""
+
+    def __init__(self, lens, slots, budget, cap, page, pool, seq):
+        self.lens, self.slots, self.budget, self.cap, self.page, self.pool, self.seq = lens, slots, budget, cap, page, pool, seq
+        self.queue, self.head, self.tail = list(range(pool)), 0, pool
+        self.next, self.running = 0, []  # running: [request, step, tokens of the iteration, pages]
+
+    def finish(self):
+        left = []
+        for q in self.running:
+            q[1] += q[2]
+            if q[1] + 1 < self.seq:
+                left.append(q)
+            else:
+                for pg in q[3]:
+                    self.queue[self.tail % self.pool] = pg
+                    self.tail += 1
+        self.running = left
+
+    def _pages(self, q):
+        while len(q[3]) < -(-(q[1] + q[2]) // self.page):
+            assert self.tail > self.head
+            q[3].append(self.queue[self.head % self.pool])
+            self.head += 1
+
+    def prepare(self):
+        used = 0
+        for q in self.running:
+            left = self.lens[q[0]] - q[1]
+            q[2] = min(left, self.cap, self.budget - used) if left > 0 else min(1, self.budget - used)
+            used += q[2]
+            self._pages(q)
+        while len(self.running) < self.slots and used < self.budget and self.next < len(self.lens):
+            n = max(1, min(self.lens[self.next], self.cap, self.budget - used))
+            if self.tail - self.head < -(-n // self.page):
+                break
+            q = [self.next, 0, n, []]
+            self._pages(q)
+            self.running.append(q)
+            self.next += 1
+            used += n
+        return used
+
+
+@pytest.mark.parametrize("slots,total,budget,cap,page,pool,seq,iterations", [
+    (1, 3, 1, 0, 4, 8, 24, 5), (2, 7, 64, 0, 4, 20, 30, 3), (3, 3, 3, 0, 16, 9, 40, 4), (8, 24, 64, 0, 4, 80, 33, 7), (8, 20, 20, 9, 8, 40, 37, 4),
+    (13, 40, 20, 0, 2, 200, 30, 6), (64, 64, 128, 0, 16, 200, 45, 5), (33, 90, 40, 1, 4, 264, 31, 9), (128, 300, 128, 16, 4, 1024, 29, 11)])
+def test_every_iteration_is_prepared_as_one_request_after_the_other(slots, total, budget, cap, page, pool, seq, iterations):
+    geom = O.TINY
+    g = mk.Qwen3Geometry(hidden=geom.hidden, n_q=geom.n_q, n_kv=geom.n_kv, mlp=geom.mlp, layers=1, vocab=geom.vocab)
+    w = {k: v.cuda() for k, v in O.make_weights(geom, 0).items() if not k.startswith("l") or k.startswith(("l0.", "lm_head"))}
+    gen = torch.Generator().manual_seed(total * slots)
+    lens = torch.randint(1, seq - 3, (total,), generator=gen).tolist()
+    prompts = [torch.randint(0, geom.vocab, (n,), generator=gen) for n in lens]
+    dec = mk.Qwen3Decoder(g, w, max_seq_length=seq, max_requests=slots, total_requests=total, page_size=page, max_num_pages=pool,
+                          max_num_batched_tokens=budget, max_tokens_per_request=cap, max_iterations=iterations)
+    dec.set_prompts(prompts)
+    host = _Host(lens, slots, max(slots, budget), cap or max(slots, budget), page, pool, seq)
+    for _ in range(200):
+        used = 0
+        for _ in range(iterations):
+            used = host.prepare()
+            if used == 0:
+                break
+            want = [list(map(list, (q[:3] for q in host.running))), [list(q[3]) for q in host.running]]
+            host.finish()
+        dec.run()
+        if used == 0:
+            break
+        state, pages = want
+        n = len(state)
+        qo = [0]
+        kv = [0]
+        for q, pg in zip(state, pages):
+            qo.append(qo[-1] + q[2])
+            kv.append(kv[-1] + len(pg))
+        assert dec.qo_indptr.tolist() == qo + [qo[-1]] * (slots - n)
+        assert dec.kv_indptr.tolist() == kv + [kv[-1]] * (slots - n)
+        assert dec.kv_indices[:kv[-1]].tolist() == [p for pg in pages for p in pg]
+        assert dec.kv_last_page_len[:n].tolist() == [(q[1] + q[2] - 1) % page + 1 for q in state]
+        tokens, fed = dec.tokens.cpu(), dec.input_tokens[:, 0].cpu()
+        for q, at in zip(state, qo):
+            assert torch.equal(fed[at:at + q[2]], tokens[q[0], q[1]:q[1] + q[2]]), q
+    assert used == 0 and dec.step.tolist() == [seq - 1] * total
+    for r, p in enumerate(prompts):
+        assert torch.equal(dec.tokens[r, :len(p)].cpu(), p)
+    dec.finalize()
