@@ -45,11 +45,11 @@ constexpr int kAttnMaxChunks = 32;
 constexpr int kGateUpUnit = 4;     // fused gate/up weights are laid out [4 gate | 4 up] per 8-row unit
 constexpr int kMaxStepTimes = 16384;
 
-// The wide path's shared memory.  Ring: stages of 32 KB of weights and two activation boxes of x_rows token rows.  As many
-// stages as leave the CTA within the 164 KB carve-out (4 up to 16 token rows, 3 up to 64, 2 beyond; the attention's scratch
-// is 9 KB for that reason): what the ring does not take is L1, and another stage brings nothing up to 64 token rows.  12 layers of 8B width, us per step: 8 requests with 3, 4 and 5 stages 1477, 1453, 1454; 32
-// requests 1588, 1562, 1566; 64 requests with 2, 3 and 4 1942, 1823, 1826; 2048 hidden, 8 requests with 3, 4 and 5 910, 893,
-// 904; more only pays from 65 token rows on (2 and 3: 2377 and 2243).
+// The wide path's shared memory.  Stages of 32 KB of weights and two activation boxes of x_rows token rows, each in a ring of its own.  As
+// many as leave the CTA within the 164 KB carve-out (4 up to 16 token rows, 3 up to 64, 2 beyond; the attention's scratch is 9 KB for that
+// reason): what the ring does not take is L1, and the ring goes on in tensor memory.  12 layers of 8B width, us per step: 8 requests
+// with 2, 3, 4, 5 and 6 stages 1331, 1267, 1249, 1270, 1269; 2048 hidden, 8 requests with 3, 4 and 5 685, 683, 691.  A stage more would pay
+// beyond 16 token rows: 32 requests with 3 and 4 1422 and 1394, 64 1682 and 1671, 100 with 2 and 3 2215 and 2137.
 constexpr int kWideFixed = 1024 /*alignment slack*/ + mk::kWideRedBytes + kBarDescBytes;
 int wide_x_rows(int tokens) { return tokens <= 16 ? 16 : (tokens <= 32 ? 32 : (tokens <= 64 ? 64 : 128)); }
 int wide_stage_bytes(int tokens) { return mk::kStageBytes + 2 * wide_x_rows(tokens) * 128; }
@@ -1269,9 +1269,9 @@ static int lower_wide(mk_handle* h) {
   // one warp normalises in the time a weight stage takes to arrive.  The first norm of a graph (behind the embedding) stays.
   // Us per step with a norm op and with the norm in the boxes: 12 layers of 8B width 4 requests 1337 and 1267, 16 1400 and 1336, 32
   // 1535 and 1484; 12 of 2048 hidden 772 and 710, 825 and 770, 981 and 935; four of 1024 hidden 227 and 214, 238 and 219, 288
-  // and 276.  "mpk" multiplies in fp32, a row at a time: 8 requests 1347 and 1287, 775 and 724, 226 and 213; 32 of 8B width 1519 and
-  // 1889.  Its line at 8 tokens was drawn for a norm warp that spilled (13 requests 1384 and 1401); with the present one 9 to 16
-  // tokens would be faster in the boxes too (12 requests 1372 and 1311, 794 and 735, 227 and 213).
+  // and 276.  "mpk" multiplies in fp32, two rows at a time: 8 requests 1347 and 1287, 775 and 724, 226 and 213; 20 of 8B width 1406 and
+  // 1450.  Its line at 8 tokens was drawn for a norm warp of 56 registers; with the present one 9 to 16 tokens would be faster in the
+  // boxes too (13 requests 1294 and 1254, 16 1307 and 1267).
   const int norm_tokens = h->cfg.numerics == mk::NUM_TORCH ? mk::kNormBoxRows : 8;
   for (size_t i = 1; h->cfg.fuse && h->plan_tokens <= norm_tokens && i + 1 < h->plan.size(); ++i) {
     const PlanOp nrm = h->plan[i];
