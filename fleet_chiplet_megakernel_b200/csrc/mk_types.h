@@ -49,6 +49,7 @@ constexpr int kRowsStageK = 512;
 // Tensor memory: 512 columns of 128 lanes x 4 bytes.  A slot holds a stage's 32 KB of weights.
 constexpr int kTmemCols = 512;
 constexpr int kSlotCols = 64;
+constexpr int kRowsCombineBytes = kNumConsumerWarps * 4 * kHeadDim * 4;  // row-owner attention: four rows of sums of every warp
 constexpr int kRowsBoxBytes = kChunkRows * kBoxK * 2;  // row-owner path: boxes of a stage lie 4 KB apart, however many of their 32 rows there are
 // Row-owner path: two sets of four accumulators of 16 columns, then slots.
 constexpr int kRowsAccCols = 64;
