@@ -2754,7 +2754,7 @@ __device__ __forceinline__ int bookkeep(Ctx& c, bool finish, bool prepare, int* 
     if (st + 1 >= p.max_seq_len || (st >= pl && __ldcg(row + st) == p.eos)) {
       freed = k1 - k0;
       rid = -1;
-      if (!prepare) p.request_ids[i] = -1;
+      p.request_ids[i] = -1;
     }
   }
   // a request still inside its prompt gets a chunk of it (as many tokens as the budget allows), a decoding one its single
@@ -2784,6 +2784,7 @@ __device__ __forceinline__ int bookkeep(Ctx& c, bool finish, bool prepare, int* 
   if (all.b > tail - head) {
     if (pg.b <= tail - head && pg.b + pages - have > tail - head)  // (the first that gets none)
       raise_abort_at(&p, c.iter, -1, ST_OUT_OF_PAGES, rid, pages);
+    if (c.tid == 0) p.sched[1] = tail;  // who has ended stays so, their pages free: another launch may follow
     return 0;
   }
   int npages = all.a;
