@@ -119,6 +119,36 @@ def test_every_iteration_is_prepared_as_one_request_after_the_other(slots, total
     dec.finalize()
 
 
+# Pools that hold fewer requests than there are places: some wait while others run, with places and budget to spare.  All of a
+# request's pages are there when it is admitted (seq - 1 positions after a prompt of seq - 4 or more), so none runs out later.
+@pytest.mark.parametrize("slots,total,budget,cap,page,pool,seq,iterations", [
+    (2, 7, 64, 0, 4, 9, 24, 3), (8, 24, 64, 0, 4, 20, 24, 1), (8, 24, 128, 0, 4, 33, 24, 4), (33, 70, 128, 0, 2, 42, 17, 2), (128, 200, 128, 0, 16, 11, 16, 5)])
+def test_requests_wait_for_pages(slots, total, budget, cap, page, pool, seq, iterations):
+    gen = torch.Generator().manual_seed(pool)
+    lens = torch.randint((seq - 2) // page * page + 1, seq - 1, (total,), generator=gen).tolist()
+    dec, prompts, host = _decoder(slots, total, budget, cap, page, pool, seq, iterations, lens)
+    _follow(dec, prompts, host, slots, page, iterations)
+    assert host.waited > 0 and dec.step.tolist() == [seq - 1] * total
+    dec.finalize()
+
+
+@pytest.mark.parametrize("slots,total,budget,page,pool,seq", [(5, 17, 5, 4, 60, 40), (13, 40, 30, 4, 140, 40), (70, 130, 128, 8, 400, 40)])
+def test_requests_that_end_early_make_room_in_the_middle_of_the_list(slots, total, budget, page, pool, seq):
+    lens = [1 + (5 * r) % 11 for r in range(total)]
+    dec, _, _ = _decoder(slots, total, budget, 0, page, pool, seq, 0, lens)
+    dec.run()
+    made = [dec.tokens[r, lens[r]:].tolist() for r in range(total)]
+    dec.finalize()
+    # the end token: the one that would end requests at the most different lengths
+    eos = max({t for m in made for t in m}, key=lambda t: len({m.index(t) + n for m, n in zip(made, lens) if t in m}))
+    dec, prompts, host = _decoder(slots, total, budget, 0, page, pool, seq, 1, lens, eos)
+    _follow(dec, prompts, host, slots, page, 1, eos)
+    # (the step of a request that has ended is the position of its last token)
+    ends = [n + m.index(eos) if eos in m else seq - 1 for n, m in zip(lens, made)]
+    assert len(set(ends)) > 2 and dec.step.tolist() == ends
+    dec.finalize()
+
+
 def test_a_pool_that_runs_dry_is_reported_and_nobody_is_lost():
     """Request 0 ends when the five others all need their second page: its two pages go to the first two, the third gets none.  A
     second launch finds the same: request 0 has ended and its pages are free."""
