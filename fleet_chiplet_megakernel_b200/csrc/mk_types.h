@@ -306,14 +306,24 @@ __host__ __device__ inline int wide_ctas(int grid, int nblk, int nkt) {
   return total < (unsigned)grid ? (int)total : grid;
 }
 
-// Whether the CTAs of a row block share its finish (see mk_wide.cuh); x_rows: token rows of a box.  With more blocks than half the
-// CTAs a CTA has about a block to finish either way, and two shares in turn take longer than one block at once: 8B width, 64 requests,
-// gate/up (192 blocks) 39.8 us shared and 36.4 by one CTA; QKV (48) 18.9 and 20.2, O and down (32) 13.2 and 16.0, 22.5 and 26.5.
+// Whether the CTAs of a row block share its finish (see mk_wide.cuh); x_rows: token rows of a box, T: tokens there are.  It pays
+// where no CTA has two groups of tokens to finish in turn: a half's tokens make T / 8 groups up to 32 token rows and T / 16 beyond, and
+// a block has ctas / nblk CTAs.  So the line follows the tokens; beyond 64 one CTA takes the block in two rounds, and three
+// groups in turn still pay.  Linears in a row (barrier each), us by one CTA and shared, 48 blocks (6144 rows) of 1024 columns: 24 tokens
+// 8.1 and 7.6, 32 8.3 and 9.5; 48 9.7 and 9.5, 64 10.4 and 11.8; 80 13.9 and 13.6; 64 blocks: 24 tokens 8.2 and 9.4, 48
+// 10.1 and 11.8, 80 14.2 and 14.6; 32 blocks: 32 tokens 7.9 and 7.3, 64 9.8 and 9.3, 128 15.0 and 14.6.
+// Head vectors and the argmax take longer to finish than to fetch: shared up to half as many blocks as CTAs.  12 layers of 8B
+// width, 64 requests, QKV (48 blocks) by one CTA and shared 1549 and 1537 us per step; four of 1024, LM head (64 blocks), 17 and 48
+// requests 207.5 and 205.5, 238.3 and 234.8.
 // Up to 16 token rows shares are of two tokens, and the line lies between QKV of 8B width, which is finished a head vector at a
 // time, and its O and down: 16 requests without any of them, with O and down and with all three 1237, 1221 and 1239 us per step.  12 layers
 // of 2048 hidden, 4 and 16 requests without any shares 674 and 708, now 652 and 682; four of 1024 185 and 207, now 172 and 200; six of
 // 512, 16 requests 247 and 234.
-__host__ __device__ inline bool wide_shares(int nblk, int ctas, int x_rows) { return (x_rows <= 16 ? 4 : 2) * nblk <= ctas; }
+__host__ __device__ inline bool wide_shares(const OpDesc& op, int ctas, int x_rows, int T) {
+  int line = x_rows <= 16 ? 4 : 2;
+  if (x_rows > 16 && !(op.flags & (F_QKV_PREP | F_ARGMAX))) line = x_rows <= 32 ? (T <= 16 ? 2 : (T + 7) / 8) : (T > 48 && T <= 64 ? 4 : 3);
+  return line * op.nblk <= ctas;
+}
 
 static_assert(sizeof(OpDesc) % 16 == 0 && sizeof(OpDesc) <= 256, "OpDesc is copied to shared memory in 16-byte pieces");
 

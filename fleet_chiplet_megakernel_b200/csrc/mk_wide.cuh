@@ -645,7 +645,7 @@ __device__ __forceinline__ void linear_wide(Ctx& c, const OpDesc& op, int T) {
   unsigned total, t0, t1;
   int G;
   if (wide_range(p, op, total, G, t0, t1)) {
-    const bool with_res = wide_with_res(c, op), share = wide_shares(op.nblk, G, N);
+    const bool with_res = wide_with_res(c, op), share = wide_shares(op, G, N, T);
     int shared[2] = {-1, -1};  // blocks to finish with others: the one the range begins in, the one it ends in
     const unsigned tag = ll_tag_of(c, c.cur_op);
     const int col0 = half * wide_split<NC>(T);  // first token column of this thread
@@ -813,7 +813,7 @@ __device__ __forceinline__ void linear_wide_shared(Ctx& c, const OpDesc& op, int
   unsigned total, t0, t1;
   int G;
   if (wide_range(p, op, total, G, t0, t1)) {
-    const bool with_res = wide_with_res(c, op), share = wide_shares(op.nblk, G, N);
+    const bool with_res = wide_with_res(c, op), share = wide_shares(op, G, N, T);
     const unsigned tag = ll_tag_of(c, c.cur_op);
     int shared[2] = {-1, -1};  // blocks to finish with others: the one the range begins in, the one it ends in
 #pragma unroll 1

@@ -97,6 +97,30 @@ def test_wide_lm_head_picks_the_lowest_index_of_ties(T):
 # Share of outputs that are not the bf16 nearest to the float64 product.  An mma chain truncates to 2^-23 of its sum at each
 # of its steps of 16: over 8 tiles of 128 that is 64 steps, 2^-18 of the sum on average and 0.06 % of the values; a tile per
 # CTA, with the tiles added up in fp32, is 8 steps, 2^-21 and 0.01 %.
+@pytest.mark.parametrize("N,K", [(4736, 1032), (6136, 520), (6144, 1152), (8184, 1032), (9472, 512)])
+def test_a_block_finished_by_several_ctas_holds_the_bits_of_one_finished_by_one(N, K):
+    """How many CTAs finish a row block follows the tokens (37, 48, 64 and 74 blocks over 148 CTAs lie on both sides of every line);
+    the sums are the same, in the same order, and so are the bits of a token's row at any number of tokens."""
+    gen = torch.Generator(device="cuda").manual_seed(N + K)
+    x, w, res = (torch.randn(*s, generator=gen, device="cuda").to(BF) for s in ((128, K), (N, K), (128, N)))
+    exact = x.double() @ w.double().T + res.double()
+    want = None
+    for T in (128, 3, 8, 16, 17, 24, 25, 32, 33, 48, 49, 64, 65, 100):
+        k, _, _ = onepass_kernel(T)
+        out = torch.zeros(T, N, dtype=BF, device="cuda")
+        k.linear_with_residual_layer(input=k.attach_input(x[:T].contiguous(), "x"), weight=k.attach_input(w, "w"),
+                                     residual=k.attach_input(res[:T].contiguous(), "res"), output=k.attach_input(out, "out"), grid_dim=(8, 1, 1),
+                                     block_dim=(128, 1, 1))
+        k.compile()
+        k()
+        if want is None:
+            want = out
+            # K fp32 products and sums of about sqrt(K), one bf16 rounding
+            assert bool(((out.double() - exact).abs() <= exact.abs() * 2 ** -8 + K ** 0.5 * K * 2 ** -24).all())
+        assert torch.equal(out, want[:T]), T
+        k.finalize()
+
+
 @pytest.mark.parametrize("T", [24, 40, 64, 100])
 @pytest.mark.parametrize("N,K", [(1024, 1024), (1024, 512), (640, 1152)])
 def test_sums_of_few_tiles_keep_fp32(T, N, K):
