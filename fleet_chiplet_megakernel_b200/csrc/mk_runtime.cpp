@@ -1582,7 +1582,14 @@ static int compile_program(mk_handle* h, bool first) {
   }
   const size_t partial_off = ll_bytes;  // wide path up to 32 token rows: the split sums of a CTA, as tagged words
   const bool words = !rows_mode && x_rows <= 32;
-  if (words) ll_bytes += (size_t)h->grid * mk::kTileRows * x_rows * 2 * 8;
+  // CTAs that may hold a piece of a block: none where k is one tile, as many as there are tiles in a small graph.  (What is not used need
+  // not be cleared: a call of one linear of 128 x 128 at 33 to 128 tokens took 40.3 to 41.7 us with the flags of all CTAs.)
+  size_t piece_ctas = 0;
+  if (!rows_mode)
+    for (const PlanOp& po : h->plan)
+      if (po.type == mk::OP_LINEAR && po.k > mk::kTileK)
+        piece_ctas = std::max(piece_ctas, (size_t)mk::wide_ctas(h->grid, (po.n + mk::kTileRows - 1) / mk::kTileRows, (po.k + mk::kTileK - 1) / mk::kTileK));
+  if (words) ll_bytes += piece_ctas * mk::kTileRows * x_rows * 2 * 8;
   h->ll_buf = nullptr;
   h->ll_bytes = ll_bytes;
   // behind the words: the counters of the attention chunks and the flags of the split-k pieces
@@ -1590,7 +1597,7 @@ static int compile_program(mk_handle* h, bool first) {
   for (const PlanOp& po : h->plan)
     if (po.type == mk::OP_ATTN) count_hkv = std::max(count_hkv, po.aux0);
   const size_t count_off = (ll_bytes + 255) / 256 * 256, attn_counts = (size_t)h->plan_tokens * count_hkv;
-  h->clear_bytes = count_off + (attn_counts + (rows_mode ? 1 : (size_t)h->grid * 2 * mk::kNumConsumerWarps)) * 4;
+  h->clear_bytes = count_off + (attn_counts + (words ? 0 : piece_ctas * 2 * mk::kNumConsumerWarps)) * 4;
   if (int e = h->dmalloc(&h->ll_buf, h->clear_bytes)) return e;
   kp.attn_count = (unsigned*)((char*)h->ll_buf + count_off);
   kp.piece_flag = kp.attn_count + attn_counts;
@@ -1601,7 +1608,7 @@ static int compile_program(mk_handle* h, bool first) {
   const int G = h->grid;
   void* p = nullptr;
   if (!rows_mode && !words) {
-    if (int e = h->dmalloc(&p, (size_t)G * 2 * mk::kTileRows * x_rows * 4)) return e;
+    if (int e = h->dmalloc(&p, std::max<size_t>(16, piece_ctas * 2 * mk::kTileRows * x_rows * 4))) return e;
     kp.partial = (uint4*)p;
   }
   int max_hkv = 1, max_qpk = 2;
