@@ -204,11 +204,6 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
   asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
   return v;
 }
-__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-  return v;
-}
 __device__ __forceinline__ void sts128(uint32_t addr, const uint4& v) {
   asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
@@ -609,20 +604,6 @@ __device__ __forceinline__ bool op_barrier(Ctx& c, const OpDesc& op) {
   if (c.pr != nullptr && c.tid == 0) c.pr[1] = globaltimer();
   c.dead = c.flags()[3] != 0;
   return c.dead;
-}
-
-// Sum over the 256 consumer threads; every thread gets the result.
-__device__ __forceinline__ float block_sum(Ctx& c, float v) {
-  float* r = c.red();  // scratch behind the 128x4 accumulator block
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if (c.lane == 0) r[c.warp] = v;
-  consumer_sync();
-  float s = 0.f;
-#pragma unroll
-  for (int i = 0; i < kNumConsumerWarps; ++i) s += r[i];
-  consumer_sync();
-  return s;
 }
 
 // ------------------------------------------------------------------------------------
@@ -1211,11 +1192,6 @@ __device__ __forceinline__ ArgBest warp_argmax(ArgBest a) {
     a = arg_better(a, b);
   }
   return a;
-}
-__device__ __forceinline__ void ldmatrix_x4(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-               : "r"(addr));
 }
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1) {
@@ -2829,8 +2805,7 @@ __device__ __forceinline__ int bookkeep(Ctx& c, bool finish, bool prepare, int* 
       for (int j = 0; j < pgs; ++j) p.kv_indices[npages + u.a + j] = __ldcg(p.page_queue + (head + u.a + j) % p.max_pages);
       p.input_tokens[q] = __ldcg(p.tokens + (size_t)r * p.max_seq_len);
     }
-    const Sum3 got = book_sums(c, {ok ? 1 : 0, ok ? n : 0, ok ? pgs : 0}, all);
-    (void)got;
+    book_sums(c, {ok ? 1 : 0, ok ? n : 0, ok ? pgs : 0}, all);  // (the totals)
     book_chunks(c, all.b > all.a, ok, i, r, 0, q, n);
     nreq += all.a;
     ntok += all.b;

@@ -1333,7 +1333,7 @@ static int compile_program(mk_handle* h, bool first) {
   const int stage_bytes = rows_mode ? mk::kStageBytes : wide_stage_bytes(nt);
   const int sums_bytes = rows_mode ? kRowsSumsBytes : 0;
   const int red_bytes = rows_mode ? kRedBytes : mk::kWideRedBytes;
-    const int fixed0 = rows_mode ? kRowsFixed : kWideFixed;
+  const int fixed0 = rows_mode ? kRowsFixed : kWideFixed;
   const int want_stages = cfg.max_stages > 0 ? std::min<int>(cfg.max_stages, mk::kMaxStages) : 4;
   // (row-owner mode prefers two resident token rows to one row and a stage more)
   int x_budget = kRowsXBudget;
