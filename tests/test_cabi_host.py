@@ -385,8 +385,9 @@ def test_mpk_wrapper_builds_the_same_program(native_lib):
 @pytest.mark.parametrize("tokens,depth", [(3, 4), (16, 4), (17, 3), (32, 3), (33, 3), (64, 3), (65, 2), (128, 2)])
 def test_wide_ring_leaves_the_l1_its_share(native_lib, tokens, depth):
     """The ring beside the attention's scratch, as the product builds it: as many stages as stay within the 164 KB carve-out (with
-    the 1 KB that the system adds).  A stage more brings nothing up to 64 token rows (3, 4 and 5 stages at 8 requests 1477, 1453 and
-    1454 us per step), and what the ring does not take is L1.  From 65 rows on three would be faster and need 210 KB."""
+    the 1 KB that the system adds): what the ring does not take is L1.  12 layers of 8B width, us per step: a stage more brings
+    nothing up to 16 token rows (8 requests with 4, 5 and 6 stages 1249, 1270, 1269) and would be faster beyond (32 requests with 3
+    and 4 1422, 1394; 64 1682, 1671; 100 with 2 and 3 2215, 2137, which need 210 KB); this is the depth that is built."""
     smem = C.c_int(0)
     attention = 8192 + 8 * 8 * 8  # the attention scratch: 8 KB to combine the warps' sums, (max, sum) pairs
     attention = (attention + 1023) // 1024 * 1024

@@ -52,21 +52,19 @@ def test_wide_gate_up_matches_oracle(T, K, inter):
     k.finalize()
 
 
-@pytest.mark.parametrize("T", [3, 17, 64, 65, 128])
-def test_wide_lm_head_picks_the_lowest_index_of_ties(T):
+def _lm_head_ties(T, V, far, span, K=512):
     """The argmax in the epilogue of the LM head, on whole numbers (every sum and its bf16 rounding is exact): two equal best
     rows within a warp's rows, within a block, in two blocks and far apart; logits that are all negative; logits that are
     all zero, of either sign."""
-    V, K = 20008, 512
     gen = torch.Generator().manual_seed(3)
     w = torch.randint(-1, 2, (V, K), generator=gen).float()
     x = torch.randint(0, 2, (T, K), generator=gen).float() * 2 - 1
     w[:, 0], x[:, 0] = 1.0, 0.0
     tied = 0
     for t in range(T):
-        a = (t * 151 + 7) % (V - 9000)
+        a = (t * 151 + 7) % span
         if t % 6 < 4:
-            for row in (a, a + (5, 70, 128, 8000)[t % 6]):
+            for row in (a, a + (5, 70, 128, far)[t % 6]):
                 w[row, 1:] = x[t, 1:]
         elif t % 6 == 4:
             x[t, 0] = -600.0
@@ -97,6 +95,18 @@ def test_wide_lm_head_picks_the_lowest_index_of_ties(T):
 # Share of outputs that are not the bf16 nearest to the float64 product.  An mma chain truncates to 2^-23 of its sum at each
 # of its steps of 16: over 8 tiles of 128 that is 64 steps, 2^-18 of the sum on average and 0.06 % of the values; a tile per
 # CTA, with the tiles added up in fp32, is 8 steps, 2^-21 and 0.01 %.
+@pytest.mark.parametrize("T", [3, 17, 64, 65, 128])
+def test_wide_lm_head_picks_the_lowest_index_of_ties(T):
+    _lm_head_ties(T, 20008, 8000, 20008 - 9000)
+
+
+# 16 and 60 row blocks over 148 CTAs: several CTAs finish a block, each some of its tokens, and one CTA parts of two blocks
+@pytest.mark.parametrize("T", [3, 16, 17, 32, 33, 64, 65, 128])
+@pytest.mark.parametrize("V", [2040, 7672])
+def test_ties_in_blocks_that_several_ctas_finish(T, V):
+    _lm_head_ties(T, V, V // 2, V // 2 - 8)
+
+
 @pytest.mark.parametrize("N,K", [(4736, 1032), (6136, 520), (6144, 1152), (8184, 1032), (9472, 512)])
 def test_a_block_finished_by_several_ctas_holds_the_bits_of_one_finished_by_one(N, K):
     """How many CTAs finish a row block follows the tokens (37, 48, 64 and 74 blocks over 148 CTAs lie on both sides of every line);
