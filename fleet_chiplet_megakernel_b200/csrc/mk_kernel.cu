@@ -28,7 +28,7 @@
 // There are no calls in an instance: with one, its per-thread context lives in local memory, calls save
 // and restore registers there, and the register split of the warp roles (consumer_regs) has no effect.
 // A block then had 200 to 320 KB of local memory beside an L1 of 28 to 92 KB.  Without calls it has
-// none (but for 80 and 8 bytes a thread in the tensor-parallel instances for one or two and for 33 to 128 tokens).  Measured
+// none (but for 88 and 16 bytes a thread in the tensor-parallel instances for one or two and for 33 to 128 tokens).  Measured
 // against the same code with out-of-line functions, 12 layers of 8B width, us per step: one request 1283 -> 1109, two
 // 1468 -> 1166, eight of 300 tokens 1707 -> 1477, 32 of 100 1878 -> 1588, 64 of 100 2340 -> 1942; four layers 1024 wide, one
 // request 172 -> 134.
@@ -1217,7 +1217,8 @@ __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1
 // order, that mma.sync by the eight warps gave, and the same bits.  With it a stage was in shared memory until the slowest
 // warp had multiplied it, a chunk's finish stopped the stream's consumer, and stages could not go to tensor memory.  12 layers of
 // 8B width, us per step: one request 1086 -> 1006, two 1146 -> 1042; four layers 1024 wide 127 -> 119; 8 MoE layers 551 -> 552, two
-// requests 676 -> 697, whose chunks of two stages are too short to gain from it; 751 before the elected producer.)
+// requests 676 -> 697, whose chunks of two stages are too short to gain from it: now 540 and 679, 582 and 751 before the elected
+// producer.)
 // ------------------------------------------------------------------------------------
 // The token rows of an op (or pass) are staged: the issuer may multiply.
 __device__ __forceinline__ void rows_x_ready(const Ctx& c) {
@@ -3296,8 +3297,8 @@ __device__ __forceinline__ void rows_mma_loop(Ctx& c) {
 constexpr uint32_t kBoxArrivals = MK_NC != 0 && 2 * MK_NC <= kNormBoxRows ? 32 : 1;
 
 // The activation producer of the wide path (warp 9, one lane).  It walks the same tile sequence
-// as the weight producer and adds the input boxes to every stage, but only after the consumers
-// have passed the op's barrier: unlike weights, activations are the previous op's output.
+// as the weight producer and loads the input boxes of every tile into a ring of their own, but only after the
+// consumers have passed the op's barrier: unlike weights, activations are the previous op's output.
 __device__ __forceinline__ void xproducer_loop(Ctx& c) {
   const KParams& p = c.p;
   const int S = p.num_stages;

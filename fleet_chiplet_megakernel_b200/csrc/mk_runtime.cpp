@@ -178,7 +178,7 @@ struct mk_handle {
   unsigned xchg_total = 0;      // cross-rank exchanges executed by all completed launches (all ranks advance alike)
   bool in_flight = false;       // launched and not yet waited for
   bool poisoned = false;        // a tensor-parallel launch aborted: the ranks' exchange sequences may differ
-  size_t clear_bytes = 0;       // of ll_buf: the words and the arrival counters behind them
+  size_t clear_bytes = 0;       // of ll_buf: the words, and the counters and flags behind them
   void* launch_stream = nullptr;
   void* ll_buf = nullptr;       // tagged activation words of the program being compiled
   size_t ll_bytes = 0;
@@ -1324,8 +1324,8 @@ static int compile_program(mk_handle* h, bool first) {
       if (t.owned && !t.ptr)
         if (int e = h->dmalloc(&t.ptr, t.alloc_bytes())) return e;
   }
-  // 2. shared-memory carve-up: [weight ring: stages x (32 KB of weights + two activation
-  // boxes of x_rows token rows)][x region: resident token rows (row-owner path), attention
+  // 2. shared-memory carve-up: [weight ring: stages x 32 KB][wide path, ring of activation boxes:
+  // stages x two boxes of x_rows token rows][x region: resident token rows (row-owner path), attention
   // scratch][row-owner path: sums block][small scratch][barriers, flags, op descriptors].
   const int nt = h->plan_tokens;
   const bool rows_mode = h->rows_mode;  // row-owner linears: resident token rows, no activation boxes
@@ -1349,7 +1349,7 @@ static int compile_program(mk_handle* h, bool first) {
   for (PlanOp& p : h->plan) {
     if (p.type == mk::OP_LINEAR) {
       ++n_linear;
-      if (!rows_mode) continue;  // the input arrives as activation boxes that ride with the weight stages
+      if (!rows_mode) continue;  // the input arrives as activation boxes, in their own ring
       const int kp = (p.k + mk::kRowsStageK - 1) / mk::kRowsStageK * mk::kRowsStageK;
       const int row_bytes = (kp + 8) * 2;
       int tpp = std::min(std::min(2, nt), (x_budget - 16) / row_bytes);
@@ -2024,8 +2024,8 @@ static int launch_program(mk_handle* h, int idx, void* stream, bool first) {
     ce = cudaMemcpyAsync(P.kp.grid_bar, &start, 4, cudaMemcpyHostToDevice, s);
     if (ce != cudaSuccess) return h->cuda_fail(ce, "state reset");
   }
-  // Tags restart with every kernel: no word of an earlier one may look valid.  And a launch that aborted may have left
-  // arrival counters half-way: a finisher that gave up clears its counter while late pieces still add to it.
+  // Tags restart with every kernel: no word and no flag of an earlier one may look valid.  And a launch that aborted may have left
+  // the arrival counters of attention chunks half-way.
   ce = cudaMemsetAsync(P.ll_buf, 0, P.clear_bytes, s);
   if (ce != cudaSuccess) return h->cuda_fail(ce, "state reset");
   // exchange sequence numbers continue where the last kernel stopped (mk_wait adds what it executed)

@@ -227,9 +227,10 @@ struct KParams {
   int max_iters;      // 0 = unlimited
   unsigned long long timeout_ns;
   // split-k scratch shared by all linear ops of the wide path
-  uint4* partial;         // sums of blocks that several CTAs share.  Up to 32 token rows [grid][x_rows / 2][128 rows] words {sum, tag,
-                          // sum of the next token, tag}, beyond [grid][2][x_rows / 4][128 rows] float4
-  unsigned* piece_flag;   // [grid][2][8 warps]: tag of the op whose piece is there (beyond 32 token rows)
+  uint4* partial;         // sums of blocks that several CTAs hold, two slots a CTA (for the CTAs that may hold any: see the host).  Up to
+                          // 32 token rows [CTAs][2][x_rows / 2][128 rows] words {sum, tag, sum of the next token, tag}, beyond
+                          // [CTAs][2][x_rows / 4][128 rows] float4
+  unsigned* piece_flag;   // [CTAs][2][8 warps]: tag of the op whose piece is there (beyond 32 token rows)
   // attention scratch
   float* attn_part;       // [tokens][kv heads][max chunks][qpk*(128+2)]
   unsigned* attn_count;   // [tokens][kv heads]
@@ -257,7 +258,7 @@ struct KParams {
   int has_moe;         // the program holds mixture-of-experts ops: the host launches the build of the kernel that has them
   // shared-memory carve-up (bytes from the 1024-aligned base)
   int num_stages;
-  int stage_bytes;  // weights (kStageBytes) + the activation boxes of a wide-batch stage
+  int stage_bytes;  // weights (kStageBytes) + on the wide path a stage of the activation boxes' ring
   int x_rows;       // token rows of an activation box (wide path: 16, 32, 64 or 128; row-owner path: 0)
   int sums_off;     // per-(row, token) sums of a run of tiles: [128][sums_stride] floats
   int sums_stride;

@@ -269,10 +269,10 @@ __device__ __forceinline__ void wide_row_scales(Ctx& c, const OpDesc& op, int T)
 }
 
 // The norm warp (warp 11).  Lane l holds 16-byte column l & 15 of a stage's two boxes for token rows (l >> 4), + 2, ...
-// All it keeps has to fit the 56 registers of a service warp, or spills sit in the loop that has to keep up with the weight
-// stream (40 bytes of stack and 304 of spill loads a thread with four rows in flight and one lane arriving for the warp).  So two
-// rows are in flight ("mpk", which unpacks them to fp32: one), and every lane arrives by itself: a __syncwarp in front of a
-// single arrival costs registers in every loop around it.
+// All it keeps has to fit the registers of a service warp, or spills sit in the loop that has to keep up with the weight stream.  With
+// the 72 it has here four rows are in flight ("mpk", which unpacks them to fp32: two); with 56 it was half as many (32 requests 1520 us
+// per step of 12 layers of 8B width instead of 1421).  Every lane arrives by itself: a __syncwarp in front of a single arrival costs
+// registers in every loop around it.
 __device__ __forceinline__ void norm_loop(Ctx& c) {
   const KParams& p = c.p;
   const int S = p.num_stages;
