@@ -1304,9 +1304,10 @@ __device__ __forceinline__ void attend_combine(const Ctx& c, int W, int gi, int 
   }
 }
 
-// One task by W warps.  `reg`: the group's shared memory (W KB), `ml`: [warps of the CTA][8] (max, sum) pairs.  `loaded`: the
-// first tile's K and V rows are in kr and vr already, but for the rows that this iteration writes.
-__device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTask& a, int W, int gi, uint8_t* reg, float2* ml, bool loaded,
+// One task by W warps.  `loaded`: the first tile's K and V rows are in kr and vr already, but for the rows that this iteration writes.
+// (What is only used behind the tiles is worked out there: held in registers across their loop it cost 0.5 to 1.5 % behind 8000
+// positions at 33 and more tokens.)
+__device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const WideTask& a, int W, bool loaded,
                                             uint4 (&kr)[2][4], uint4 (&vr)[4][2]) {
   const KParams& p = c.p;
   const int lane = c.lane, g = lane >> 2, j = lane & 3;
@@ -1374,6 +1375,9 @@ __device__ __forceinline__ void wide_attend(Ctx& c, const OpDesc& op, const Wide
     if (__any_sync(0xffffffffu, chk != 0.f)) attend_exact(p, op, a, W, q, op.ld_out2, kHeadDim, store);
     return;
   }
+  const int gi = c.warp / W;
+  uint8_t* reg = c.smem + p.x_off + (size_t)gi * W * 1024;          // the group's shared memory, W KB
+  float2* ml = reinterpret_cast<float2*>(c.smem + p.x_off + 8192);  // [warps of the CTA][8] (max, sum) pairs
   const uint32_t nbar = (uint32_t)(2 + gi);
   attend_combine(c, W, gi, rows, reg, ml, m, l, oacc, [&](int, int r, int d, const float4& O, float M, float L) {
     chk = fmaf(O.x, 0.f, fmaf(O.y, 0.f, fmaf(O.z, 0.f, fmaf(O.w, 0.f, chk))));
@@ -1456,8 +1460,6 @@ __device__ __forceinline__ void op_attention_wide(Ctx& c, const OpDesc& op, int 
   const int W = tab.plan[1], nch = tab.plan[2], CS = tab.plan[3];
   const int ntasks = tab.plan[0] * HKV * nch, per = kNumConsumerWarps / W;
   const int gi = c.warp / W;
-  uint8_t* reg = c.smem + p.x_off + (size_t)gi * W * 1024;
-  float2* ml = reinterpret_cast<float2*>(c.smem + p.x_off + 8192);
   uint4 kr[2][4], vr[4][2];
   bool loaded = false;
 #pragma unroll 1
@@ -1500,6 +1502,6 @@ __device__ __forceinline__ void op_attention_wide(Ctx& c, const OpDesc& op, int 
       MK_STAMP(c, 0);
     }
     if (task >= ntasks) break;
-    if (live) wide_attend(c, op, a, W, gi, reg, ml, first && loaded, kr, vr);
+    if (live) wide_attend(c, op, a, W, first && loaded, kr, vr);
   }
 }
