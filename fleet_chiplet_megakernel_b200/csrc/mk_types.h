@@ -311,9 +311,10 @@ __host__ __device__ inline int wide_ctas(int grid, int nblk, int nkt) {
 // where no CTA has two groups of tokens to finish in turn: a half's tokens make T / 8 groups up to 32 token rows and T / 16 beyond, and
 // a block has ctas / nblk CTAs.  So the line follows the tokens; beyond 64 one CTA takes the block in two rounds, and three
 // groups in turn still pay.  Where the CTAs come out even, none is in two blocks, and half as many do beyond 32 rows (74 blocks of 512
-// columns: 48 tokens 9.2 and 8.7, 128 13.9 and 12.6; but 24 tokens 7.4 and 8.0).  Linears in a row (barrier each), us by one CTA and shared, 48 blocks (6144 rows) of 1024 columns: 24 tokens
-// 8.1 and 7.6, 32 8.3 and 9.5; 48 9.7 and 9.5, 64 10.4 and 11.8; 80 13.9 and 13.6; 64 blocks: 24 tokens 8.2 and 9.4, 48
-// 10.1 and 11.8, 80 14.2 and 14.6; 32 blocks: 32 tokens 7.9 and 7.3, 64 9.8 and 9.3, 128 15.0 and 14.6.
+// columns: 48 tokens 9.2 and 8.7, 128 13.9 and 12.6; but 24 tokens 7.4 and 8.0).  Linears in a row (barrier each), us by one CTA and
+// shared, 48 blocks (6144 rows) of 1024 columns: 24 tokens 8.1 and 7.6, 32 8.3 and 9.5; 48 9.7 and 9.5, 64 10.4 and 11.8; 80 13.9 and
+// 13.6; 64 blocks: 24 tokens 8.2 and 9.4, 48 10.1 and 11.8, 80 14.2 and 14.6; 32 blocks: 32 tokens 7.9 and 7.3, 64 9.8 and 9.3, 128
+// 15.0 and 14.6.
 // Head vectors and the argmax take longer to finish than to fetch: shared up to half as many blocks as CTAs.  12 layers of 8B
 // width, 64 requests, QKV (48 blocks) by one CTA and shared 1549 and 1537 us per step; four of 1024, LM head (64 blocks), 17 and 48
 // requests 207.5 and 205.5, 238.3 and 234.8.

@@ -558,3 +558,28 @@ def test_page_tables_wider_than_the_ring(requests, length, budget):
         dec.finalize()
     assert all(torch.equal(a, b) for a, b in zip(got[0][0], got[1][0]))
     assert torch.equal(got[0][1], got[1][1])
+
+
+@pytest.mark.parametrize("requests,budget", [(1, 1), (2, 2), (5, 5), (24, 24), (40, 40), (100, 100), (1, 64), (3, 20)])
+def test_a_generation_behind_one_that_was_given_up(requests, budget):
+    """A token id out of range ends a launch in its fourth iteration (its first, where prompts come in chunks), with weights under
+    way, in shared memory and in tensor memory; the handle generates as a new one does afterwards."""
+    geom, n_new = O.TINY, 8
+    w = _cuda(O.make_weights(geom, 0, norm_jitter=0.25))
+    prompts = [O.make_prompt(geom, 6, r) for r in range(requests)]
+    bad = [p.clone() for p in prompts]
+    bad[-1][3] = geom.vocab
+    got = []
+    for spoil in (True, False):
+        dec = mk.Qwen3Decoder(_geom(geom), w, max_seq_length=6 + n_new, max_requests=requests, page_size=16, max_num_batched_tokens=budget,
+                              numerics="mpk", keep_logits=True)
+        for _ in range(2 if spoil else 0):
+            dec.set_prompts(bad)
+            with pytest.raises(RuntimeError, match="token id out of range"):
+                dec.run()
+        dec.set_prompts(prompts)
+        dec.run()
+        got.append(([dec.generated(r).cpu() for r in range(requests)], dec.logits[:requests].cpu()))
+        dec.finalize()
+    assert all(torch.equal(a, b) for a, b in zip(got[0][0], got[1][0]))
+    assert torch.equal(got[0][1], got[1][1])
